@@ -169,11 +169,13 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constant
     // ------------------------------ producer ------------------------------
     if (lane == 0 && nmax > 0) {
       uint32_t bytes = 0;
+      // a tile without keys has no use for Q, and its warps stage zeros for O in that place at once
+      const int n_t[2] = {n0, n1};
       for (int t = 0; t < 2; ++t)
-        if (tile_valid[t]) bytes += L::QT;
+        if (n_t[t] > 0) bytes += L::QT;
       mbar_expect_tx(q_full, bytes);
       for (int t = 0; t < 2; ++t) {
-        if (!tile_valid[t]) continue;
+        if (n_t[t] == 0) continue;
 #pragma unroll
         for (int hf = 0; hf < HALVES; ++hf)
           tma_load_4d(smem + L::OFF_Q + t * L::QT + hf * 16384, &map_q, q_full, hf * 64, h, q0 + t * 128, b);

@@ -69,6 +69,27 @@ def test_matches_oracle(cuda_lib, d, hq, hkv, layout):
     assert cuda_lib.device_status() == (0, 0, 0, 0)
 
 
+@pytest.mark.parametrize("side", ["right", "left"])
+@pytest.mark.parametrize("d", [128, 64])
+def test_query_tile_of_padding_beside_a_tile_with_keys(cuda_lib, d, side):
+    """One of the two 128-query tiles of a CTA is all padding, the other is not: its output is exactly
+    zero however its (unneeded) queries and the other tile's work are timed."""
+    b, s, hq, hkv = 4, 512, 16, 4
+    seg = torch.ones(b, s, dtype=torch.int32, device="cuda")
+    if side == "right":
+        seg[:, 128:256] = 0
+        seg[:, 384:] = 0
+    else:
+        seg[:, :128] = 0
+        seg[:, 256:384] = 0
+    pad = seg == 0
+    for seed in range(8):
+        _, (o, lse, dq, dk, dv) = _run(b, s, hq, hkv, d, seg, seed=seed)
+        for t in (o, dq, dk, dv, lse.permute(0, 2, 1)):
+            assert torch.all(t[pad] == 0)
+    assert cuda_lib.device_status() == (0, 0, 0, 0)
+
+
 def test_matches_oracle_at_the_training_shape(cuda_lib):
     """32 query / 8 key-value heads, 4096 tokens packed from six documents (the benchmark's layer
     shape), forward and all three gradients against the fp32 PyTorch attention."""
