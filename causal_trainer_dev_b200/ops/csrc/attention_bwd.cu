@@ -1,23 +1,36 @@
 // Flash attention backward for sm_100a, two kernels from one template, no atomics:
 //
-//   MODE_DKV  KV-tile-owned: a CTA owns 128 keys of one KV head and walks every query
-//             block (64 rows) of every query head of the GQA group that can see them.
+//   MODE_DKV  KV-tile-owned: a CTA owns 128 keys of one KV head and walks the 64-row query blocks
+//             of every query head of the GQA group that can see them, two blocks per iteration.
 //                 S^T = K Q^T          dP^T = V dO^T            (tcgen05, TMEM)
 //                 P^T = exp2(S^T c - lse),  dS^T = P^T (dP^T - delta)   (registers; the per-query
 //                 statistics arrive negated and in log2 units, ready for packed fma / add)
 //                 dV += P^T dO         dK += dS^T Q             (tcgen05, TMEM accumulators)
 //             The reduction over the group's query heads happens in the TMEM accumulators.
 //   MODE_DQ   Q-tile-owned: a CTA owns 128 query rows of one query head and walks the
-//             64-key blocks it can see:  S = Q K^T, dP = dO V^T, dS = P (dP - delta),
-//             dQ += dS K.
+//             64-key blocks it can see, two per iteration:  S = Q K^T, dP = dO V^T,
+//             dS = P (dP - delta), dQ += dS K.
 //
-// Structure of both: resident operand pair X (K,V or Q,dO), streamed pair Y (Q,dO or K,V)
-// through a 4-stage TMA ring, four compute warpgroups that share every Y block (16 of its 64
-// columns each) over two alternating S / dP buffers, so the tensor core works on block i+1 and
-// on the accumulate MMAs of block i-1 while block i is exponentiated.  P^T / dS go back into TMEM
-// as bf16 pairs over the scores they were computed from and are the TMEM A operands of the
-// accumulate MMAs (they never cross shared memory); the Y tiles are reused in place as MN-major
-// B operands.
+// Structure of both: resident operand pair X (K,V or Q,dO), streamed pair Y (Q,dO or K,V) of
+// 128 rows through TMA rings (three slots of Y1 = Q or K, two of Y2 = dO or V), four compute warpgroups that share every iteration
+// (32 of its 128 columns each).  An iteration is two independent 64-row blocks, so block ranges and
+// work lists keep their 64-row granularity.  P^T / dS go back into TMEM as bf16 pairs over the scores
+// they were computed from and are the TMEM A operands of the accumulate MMAs (they never cross
+// shared memory); the Y tiles are reused in place as MN-major B operands.
+//
+// What bounds it.  A 128 x 128 iteration costs the tensor core 4 x 518 cycles (dQ: 3 x 518; measured, a
+// 128 x 64 score tile takes 390 and not 259: it is bound by its operands' shared memory reads), the
+// exponentials 1024 cycles (16 / clk / SM).  So two 64-row blocks share a 128-column tile, and the fixed
+// costs (barrier round trips, masks, TMEM latency) are paid once per 32 columns of a thread.  S and dP have
+// separate barriers, so that the exponentials overlap the dP product and dS overlaps dV and the next S
+// (order of the tensor core: dV(i) S(i+1) dK(i) dP(i+1); with room in TMEM for a second S buffer:
+// S(i+1) dV(i) dK(i) dP(i+1)), and each of P and dS is published in two halves of 16 columns per
+// thread, so that the accumulate MMAs start on the first half.  Y1 has three slots because S(i+1) wants its
+// operand early while dK(i) still reads the one before (with two joint slots the products waited 1200
+// cycles per iteration for copies).  One document of 16384 tokens, 8 / 2 heads, D = 128, cycles per
+// iteration of a CTA: dK/dV 4509 with joint slots, 3840 with three, 2615 with the warp-uniform issue
+// of elect_one() (64-column tiles: 2 x 2700); dQ 3540, 3032, 2047.  Whole kernels 1.24 -> 0.79 ms and
+// 0.88 -> 0.56 ms.  Now the compute warps are the longer side (P 1300, dS 420, masks 400 cycles).
 //
 // Reference counterparts: causal_trainer_attention_dq / _dkv
 // (src/causal_trainer/kernels/efficient_attention.py:985-1173, 1270-1436); the psum that
@@ -31,7 +44,9 @@ namespace ctb {
 namespace attn {
 
 constexpr int BWD_THREADS = 640;   // 4 service warps + 4 compute warpgroups
-constexpr int Y_STAGES = 4;
+constexpr int Y1_SLOTS = 3;        // Q (DKV) or K (DQ): needed first, released last
+constexpr int Y2_SLOTS = 2;        // dO (DKV) or V (DQ)
+constexpr int COMPUTE_WARPS = 16;
 
 enum : unsigned {
   SITE_B_PROD = 0x0301,
@@ -40,18 +55,27 @@ enum : unsigned {
   SITE_B_MMA_T = 0x0304,
   SITE_B_CW_S = 0x0305,
   SITE_B_CW_ACC = 0x0307,
+  SITE_B_BASE = 0x0308,
 };
 
 template <int D>
 struct BwdSmem {
   static constexpr int HALVES = D / 64;
   static constexpr int XT = HALVES * 16384;   // 128-row resident tile
-  static constexpr int YT = HALVES * 8192;    // 64-row streamed tile
+  static constexpr int YT = HALVES * 16384;   // streamed tile: two 64-row blocks
   static constexpr int OFF_X = 0;             // X1, X2
-  static constexpr int OFF_Y = 2 * XT;        // stages of (Y1, Y2)
-  static constexpr int OFF_BAR = OFF_Y + Y_STAGES * 2 * YT;
-  static constexpr int OFF_STAT = OFF_BAR + 256;   // per Y stage: 64 x -lse*log2(e), 64 x -delta of the block's queries (DKV)
-  static constexpr int BYTES = OFF_STAT + Y_STAGES * 512 + 1024;
+  static constexpr int OFF_Y1 = 2 * XT;
+  static constexpr int OFF_Y2 = OFF_Y1 + Y1_SLOTS * YT;
+  // statistics of the streamed queries (DKV): 128 x -delta beside each Y1 slot, 128 x -lse*log2(e)
+  // beside each Y2 slot (dS is read after dV has released Y2, so -delta cannot live there)
+  static constexpr int OFF_DELTA = OFF_Y2 + Y2_SLOTS * YT;
+  static constexpr int OFF_LSE = OFF_DELTA + Y1_SLOTS * 512;
+  static constexpr int OFF_BAR = OFF_LSE + Y2_SLOTS * 512;
+  static constexpr int BYTES = OFF_BAR + 256;       // no slack: the tiles need a 1024-byte aligned base (checked)
+  static_assert(BYTES <= 232448, "shared memory of one CTA");
+  // TMEM columns: S buffers, dP, accumulators.  A second S buffer where it fits into 512 columns.
+  static constexpr int S_BUFS_DKV = 2 * 128 + 128 + 2 * D <= 512 ? 2 : 1;
+  static constexpr int S_BUFS_DQ = 2;
 };
 
 template <int D, int MODE>
@@ -63,18 +87,26 @@ attn_bwd_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constant
   using L = BwdSmem<D>;
   constexpr int HALVES = L::HALVES;
   constexpr bool DKV = (MODE == MODE_DKV);
-  extern __shared__ uint8_t smem_raw[];
-  uint8_t* smem = smem_raw + ((1024u - (smem_u32(smem_raw) & 1023u)) & 1023u);
+  constexpr int S_BUFS = DKV ? L::S_BUFS_DKV : L::S_BUFS_DQ;
+  extern __shared__ __align__(1024) uint8_t smem[];
+  if ((smem_u32(smem) & 1023u) != 0u) {              // (uniform) the swizzled tiles would not be where TMA writes them
+    if (threadIdx.x == 0) report_failure(args.status, SITE_B_BASE, smem_u32(smem), 0u);
+    return;
+  }
   uint64_t* x_full = reinterpret_cast<uint64_t*>(smem + L::OFF_BAR);
-  uint64_t* y_full = x_full + 1;
-  uint64_t* y_empty = y_full + Y_STAGES;
-  uint64_t* s_full = y_empty + Y_STAGES;   // [2] S and dP of buffer u ready
-  uint64_t* t_full = s_full + 2;           // [2] P^T / dS tiles of buffer u written
-  uint64_t* acc_full = t_full + 2;
+  uint64_t* y1_full = x_full + 1;
+  uint64_t* y1_empty = y1_full + Y1_SLOTS;
+  uint64_t* y2_full = y1_empty + Y1_SLOTS;
+  uint64_t* y2_empty = y2_full + Y2_SLOTS;
+  uint64_t* s_full = y2_empty + Y2_SLOTS;   // [2] S of buffer u ready
+  uint64_t* dp_full = s_full + 2;          // dP ready
+  uint64_t* p_full = dp_full + 1;          // [2][2] S buffer u: half h (columns [16 h, 16 h + 16) of every 32) of P^T written
+  uint64_t* ds_full = p_full + 4;          // [2] half h of dS written
+  uint64_t* acc_full = ds_full + 2;
   uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(acc_full + 1);
   volatile uint32_t* abort_flag = tmem_slot + 1;
 
-  const int warp = threadIdx.x >> 5;
+  const int warp = uniform_warp_index();
   const int lane = threadIdx.x & 31;
   DeviceStatus* st = args.status;
   const long long budget = args.spin_budget;
@@ -125,7 +157,7 @@ attn_bwd_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constant
     y_n64 = khi > klo ? (khi + 63) / 64 - y_lo64 : 0;
     heads_in_loop = 1;
   }
-  int n_iter = y_n64 * heads_in_loop;
+  int n_entry = y_n64 * heads_in_loop;      // 64-row blocks to visit
   const int hkv = grouped ? (gd.x >> 16) : (DKV ? head : head / group);
   const int kbatch = grouped ? (gd.x & 0xffff) : b;     // batch of the K / V / dK / dV tensors
   const int y_base = grouped ? (DKV ? gd.z : gd.y) : 0; // first row (dK/dV) or key (dQ) of the streamed operand
@@ -134,26 +166,35 @@ attn_bwd_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constant
   const int* it_list = nullptr;
   if (sparse) {
     int base;
-    sparse_list(args.sp, blockIdx.x, base, n_iter);
+    sparse_list(args.sp, blockIdx.x, base, n_entry);
     it_list = args.sp.it_list + base;
   }
-  // iteration -> (64-row block of the streamed operand, query head)
-  auto y_block = [&](int it) -> int { return sparse ? (__ldg(it_list + it) & 0xffffff) : y_lo64 + it % y_n64; };
-  auto y_head = [&](int it) -> int {
+  const int n_iter = (n_entry + 1) / 2;
+  // entry -> (64-row block of the streamed operand, query head).  Iteration i holds entries 2i and
+  // 2i + 1 in the two halves of its tile; an odd last half repeats the last entry, fully masked.
+  auto y_block = [&](int e) -> int { return sparse ? (__ldg(it_list + e) & 0xffffff) : y_lo64 + e % y_n64; };
+  auto y_head = [&](int e) -> int {
     if (grouped) return 0;
     if (!DKV) return head;
-    return hkv * group + (sparse ? (__ldg(it_list + it) >> 24) : it / y_n64);
+    return hkv * group + (sparse ? (__ldg(it_list + e) >> 24) : e / y_n64);
   };
 
   if (threadIdx.x == 0) {
     mbar_init(x_full, 1);
-    for (int s = 0; s < Y_STAGES; ++s) {
-      mbar_init(&y_full[s], 1);
-      mbar_init(&y_empty[s], 1);
+    for (int s = 0; s < Y1_SLOTS; ++s) {
+      mbar_init(&y1_full[s], 1);
+      mbar_init(&y1_empty[s], 1);
     }
+    for (int s = 0; s < Y2_SLOTS; ++s) {
+      mbar_init(&y2_full[s], 1);
+      mbar_init(&y2_empty[s], 1);
+    }
+    mbar_init(dp_full, 1);
     for (int u = 0; u < 2; ++u) {
       mbar_init(&s_full[u], 1);
-      mbar_init(&t_full[u], 512);
+      mbar_init(&p_full[2 * u], COMPUTE_WARPS);
+      mbar_init(&p_full[2 * u + 1], COMPUTE_WARPS);
+      mbar_init(&ds_full[u], COMPUTE_WARPS);
     }
     mbar_init(acc_full, 1);
     *abort_flag = 0u;
@@ -167,120 +208,143 @@ attn_bwd_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constant
   __syncthreads();
   tc_fence_after();
   const uint32_t tmem_base = *tmem_slot;
-  // S^T / dP^T (or S / dP) of block buffer u: 64 columns each (address arithmetic, not arrays: a
-  // runtime index into a local array would go through local memory)
-  auto tmem_s = [&](int u) -> uint32_t { return tmem_base + static_cast<uint32_t>(u) * 64u; };
-  auto tmem_dp = [&](int u) -> uint32_t { return tmem_base + 128u + static_cast<uint32_t>(u) * 64u; };
-  const uint32_t tmem_acc1 = tmem_base + 256;       // dV (DKV) or dQ (DQ)
-  const uint32_t tmem_acc2 = tmem_base + 256 + D;   // dK (DKV)
+  // address arithmetic, not arrays: a runtime index into a local array would go through local memory
+  auto tmem_s = [&](int u) -> uint32_t { return tmem_base + static_cast<uint32_t>(u) * 128u; };
+  const uint32_t tmem_dp = tmem_base + S_BUFS * 128u;
+  const uint32_t tmem_acc1 = tmem_dp + 128u;        // dV (DKV) or dQ (DQ)
+  const uint32_t tmem_acc2 = tmem_acc1 + D;   // dK (DKV)
 
   if (warp == 0) {
     // ------------------------------ producer ------------------------------
-    if (lane == 0 && n_iter > 0) {
-      mbar_expect_tx(x_full, 2 * L::XT);
+    if (n_iter > 0) {
+      const uint32_t on = elect_one();            // the whole warp walks, one lane issues
+      mbar_expect_tx_if(on, x_full, 2 * L::XT);
       const CUtensorMap* mx1 = DKV ? &map_k : &map_q;
       const CUtensorMap* mx2 = DKV ? &map_v : &map_do;
       const int xh = DKV ? hkv : head;
       const int xb = DKV ? kbatch : b;
 #pragma unroll
       for (int hf = 0; hf < HALVES; ++hf) {
-        tma_load_4d(smem + L::OFF_X + hf * 16384, mx1, x_full, hf * 64, xh, x0, xb);
-        tma_load_4d(smem + L::OFF_X + L::XT + hf * 16384, mx2, x_full, hf * 64, xh, x0, xb);
+        tma_load_4d_if(on, smem + L::OFF_X + hf * 16384, mx1, x_full, hf * 64, xh, x0, xb);
+        tma_load_4d_if(on, smem + L::OFF_X + L::XT + hf * 16384, mx2, x_full, hf * 64, xh, x0, xb);
       }
       const CUtensorMap* my1 = DKV ? &map_q : &map_k;
       const CUtensorMap* my2 = DKV ? &map_do : &map_v;
-      uint32_t stage = 0, phase = 0;
+      uint32_t slot1 = 0, phase1 = 0;
+      const int ybatch = DKV ? b * (grouped ? 0 : 1) : kbatch;
       for (int it = 0; it < n_iter; ++it) {
-        const int yh = DKV ? y_head(it) : hkv;
-        const int ybatch = DKV ? b * (grouped ? 0 : 1) : kbatch;
-        const int y0 = y_base + y_block(it) * 64 - (DKV ? args.q_off : 0);   // streamed queries are stored locally
-        if (!mbar_wait(&y_empty[stage], phase ^ 1u, abort_flag, st, SITE_B_PROD, budget)) break;
-        mbar_expect_tx(&y_full[stage], 2 * L::YT + (DKV ? 512 : 0));
-        uint8_t* dst = smem + L::OFF_Y + stage * 2 * L::YT;
-        if (DKV) {
-          // the per-query statistics of the block travel with it (256 B each, 256 B aligned)
-          const size_t stat = grouped ? static_cast<size_t>(y0) : (static_cast<size_t>(b) * args.Hq + yh) * args.Sq + y0;
-          tma_load_1d(smem + L::OFF_STAT + stage * 512, args.neg_lse2 + stat, 256, &y_full[stage]);
-          tma_load_1d(smem + L::OFF_STAT + stage * 512 + 256, args.neg_delta + stat, 256, &y_full[stage]);
-        }
+        const uint32_t slot2 = it & 1, phase2 = (it >> 1) & 1;
+        int y0[2], yh[2];
+        size_t stat[2];
 #pragma unroll
-        for (int hf = 0; hf < HALVES; ++hf) {
-          tma_load_4d(dst + hf * 8192, my1, &y_full[stage], hf * 64, yh, y0, ybatch);
-          tma_load_4d(dst + L::YT + hf * 8192, my2, &y_full[stage], hf * 64, yh, y0, ybatch);
+        for (int q = 0; q < 2; ++q) {              // the two 64-row halves of the tile
+          const int e = min(2 * it + q, n_entry - 1);
+          yh[q] = DKV ? y_head(e) : hkv;
+          y0[q] = y_base + y_block(e) * 64 - (DKV ? args.q_off : 0);   // streamed queries are stored locally
+          stat[q] = grouped ? static_cast<size_t>(y0[q])
+                            : (static_cast<size_t>(b) * args.Hq + yh[q]) * args.Sq + y0[q];
         }
-        if (++stage == Y_STAGES) {
-          stage = 0;
-          phase ^= 1u;
+        auto load = [&](uint8_t* dst, const CUtensorMap* map, uint64_t* bar, float* stat_dst, const float* stat_src) {
+          mbar_expect_tx_if(on, bar, L::YT + (DKV ? 512 : 0));
+#pragma unroll
+          for (int q = 0; q < 2; ++q) {
+            // the per-query statistics of the block travel with it (256 B each, 256 B aligned)
+            if (DKV) tma_load_1d_if(on, stat_dst + q * 64, stat_src + stat[q], 256, bar);
+#pragma unroll
+            for (int hf = 0; hf < HALVES; ++hf)
+              tma_load_4d_if(on, dst + hf * 16384 + q * 8192, map, bar, hf * 64, yh[q], y0[q], ybatch);
+          }
+        };
+        if (!mbar_wait_warp(&y1_empty[slot1], phase1 ^ 1u, abort_flag, st, SITE_B_PROD, budget)) break;
+        load(smem + L::OFF_Y1 + slot1 * L::YT, my1, &y1_full[slot1],
+             reinterpret_cast<float*>(smem + L::OFF_DELTA + slot1 * 512), args.neg_delta);
+        if (!mbar_wait_warp(&y2_empty[slot2], phase2 ^ 1u, abort_flag, st, SITE_B_PROD, budget)) break;
+        load(smem + L::OFF_Y2 + slot2 * L::YT, my2, &y2_full[slot2],
+             reinterpret_cast<float*>(smem + L::OFF_LSE + slot2 * 512), args.neg_lse2);
+        if (++slot1 == Y1_SLOTS) {
+          slot1 = 0;
+          phase1 ^= 1u;
         }
       }
     }
   } else if (warp == 1) {
     // ------------------------------ MMA issuer ------------------------------
-    if (lane == 0 && n_iter > 0) {
-      constexpr uint32_t idesc_s = make_idesc_bf16(128, 64, false, false);
+    if (n_iter > 0) {
+      const uint32_t on = elect_one();            // the whole warp walks, one lane issues
+      constexpr uint32_t idesc_s = make_idesc_bf16(128, 128, false, false);
       constexpr uint32_t idesc_acc = make_idesc_bf16(128, D, false, true);
       const uint32_t x1 = smem_u32(smem + L::OFF_X);
       const uint32_t x2 = smem_u32(smem + L::OFF_X + L::XT);
-      bool ok = mbar_wait(x_full, 0, abort_flag, st, SITE_B_MMA_X, budget);
-      uint32_t stage = 0, phase = 0;       // stage of the block whose S/dP is issued next
-      uint32_t astage = 0;                 // stage of the block whose accumulate MMAs come next
-      uint32_t tph[2] = {0, 0};
-      auto accumulate_block = [&](int k) -> bool {
-        const int u = k & 1;
-        if (!mbar_wait(&t_full[u], tph[u], abort_flag, st, SITE_B_MMA_T, budget)) return false;
-        tph[u] ^= 1u;
-        tc_fence_after();
-        const uint32_t y1 = smem_u32(smem + L::OFF_Y + astage * 2 * L::YT);
-        const uint32_t y2 = y1 + L::YT;
-        // P^T / dS are bf16 pairs in TMEM: the 16 columns of group kk sit in the first 8 columns of
-        // the group's own 16-column slice of the S / dP buffer (written over the scores it read)
+      const uint32_t y1_at = smem_u32(smem + L::OFF_Y1);
+      const uint32_t y2_at = smem_u32(smem + L::OFF_Y2);
+      // S or dP of the tile in `y`: both operands K-major
+      auto product = [&](uint32_t d, uint32_t x, uint32_t y) {
 #pragma unroll
-        for (int kk = 0; kk < 4; ++kk) {
-          if (DKV) {
-            umma_bf16_ts(tmem_acc1, tmem_s(u) + 16 * kk, desc_mnmajor(y2, kk, 8192), idesc_acc, (k | kk) != 0 ? 1u : 0u);
-            umma_bf16_ts(tmem_acc2, tmem_dp(u) + 16 * kk, desc_mnmajor(y1, kk, 8192), idesc_acc, (k | kk) != 0 ? 1u : 0u);
-          } else {
-            umma_bf16_ts(tmem_acc1, tmem_dp(u) + 16 * kk, desc_mnmajor(y1, kk, 8192), idesc_acc, (k | kk) != 0 ? 1u : 0u);
-          }
+        for (int k = 0; k < D / 16; ++k)
+          umma_bf16_if(on, d, desc_kmajor(x + (k / 4) * 16384, k % 4), desc_kmajor(y + (k / 4) * 16384, k % 4), idesc_s,
+                    k != 0 ? 1u : 0u);
+      };
+      // accumulator += (P^T or dS) Y as its halves arrive.  The bf16 pairs of the 16 columns of group kk
+      // sit in the first 8 columns of the group's own 16-column slice of the fp32 buffer
+      auto accumulate = [&](uint64_t* full, uint32_t parity, uint32_t acc, uint32_t a, uint32_t y, int it) -> bool {
+#pragma unroll
+        for (int half = 0; half < 2; ++half) {
+          if (!mbar_wait_warp(&full[half], parity, abort_flag, st, SITE_B_MMA_T, budget)) return false;
+          tc_fence_after();
+#pragma unroll
+          for (int kk = half; kk < 8; kk += 2)
+            umma_bf16_ts_if(on, acc, a + 16 * kk, desc_mnmajor(y, kk, 16384), idesc_acc, (it | kk) != 0 ? 1u : 0u);
         }
-        umma_commit(&y_empty[astage]);
-        if (++astage == Y_STAGES) astage = 0;
         return true;
       };
-      for (int it = 0; ok && it < n_iter; ++it) {
-        const int u = it & 1;
-        if (!mbar_wait(&y_full[stage], phase, abort_flag, st, SITE_B_MMA_Y, budget)) {
-          ok = false;
-          break;
-        }
+      bool ok = mbar_wait_warp(x_full, 0, abort_flag, st, SITE_B_MMA_X, budget);
+      uint32_t slot_s = 0, phase_s = 0;        // Y1 slot of the next S
+      uint32_t slot_a = 0;                     // Y1 slot of the next dK / dQ
+      auto next_s = [&](int it) -> bool {
+        if (!mbar_wait_warp(&y1_full[slot_s], phase_s, abort_flag, st, SITE_B_MMA_Y, budget)) return false;
         tc_fence_after();
-        const uint32_t y1 = smem_u32(smem + L::OFF_Y + stage * 2 * L::YT);
-        const uint32_t y2 = y1 + L::YT;
-#pragma unroll
-        for (int k = 0; k < D / 16; ++k)
-          umma_bf16(tmem_s(u), desc_kmajor(x1 + (k / 4) * 16384, k % 4), desc_kmajor(y1 + (k / 4) * 8192, k % 4),
-                    idesc_s, k != 0 ? 1u : 0u);
-#pragma unroll
-        for (int k = 0; k < D / 16; ++k)
-          umma_bf16(tmem_dp(u), desc_kmajor(x2 + (k / 4) * 16384, k % 4), desc_kmajor(y2 + (k / 4) * 8192, k % 4),
-                    idesc_s, k != 0 ? 1u : 0u);
-        umma_commit(&s_full[u]);
-        if (++stage == Y_STAGES) {
-          stage = 0;
-          phase ^= 1u;
+        product(tmem_s(it % S_BUFS), x1, y1_at + slot_s * L::YT);
+        umma_commit_if(on, &s_full[it % S_BUFS]);
+        if (++slot_s == Y1_SLOTS) {
+          slot_s = 0;
+          phase_s ^= 1u;
         }
-        if (it > 0) ok = accumulate_block(it - 1);
+        return true;
+      };
+      auto next_dp = [&](int it) -> bool {
+        if (!mbar_wait_warp(&y2_full[it & 1], static_cast<uint32_t>(it >> 1) & 1u, abort_flag, st, SITE_B_MMA_Y, budget))
+          return false;
+        tc_fence_after();
+        product(tmem_dp, x2, y2_at + (it & 1) * L::YT);
+        umma_commit_if(on, dp_full);
+        if (!DKV) umma_commit_if(on, &y2_empty[it & 1]);          // V is read by this product alone
+        return true;
+      };
+      ok = ok && next_s(0) && next_dp(0);
+      for (int it = 0; ok && it < n_iter; ++it) {
+        const bool more = it + 1 < n_iter;
+        // with one S buffer the next scores overwrite P, which dV reads: in issue order, so no wait
+        if (S_BUFS == 2 && more && !next_s(it + 1)) break;
+        if (DKV) {
+          if (!accumulate(p_full + 2 * (it % S_BUFS), static_cast<uint32_t>(it / S_BUFS) & 1u, tmem_acc1,
+                          tmem_s(it % S_BUFS), y2_at + (it & 1) * L::YT, it))
+            break;
+          umma_commit_if(on, &y2_empty[it & 1]);
+        }
+        if (S_BUFS == 1 && more && !next_s(it + 1)) break;
+        if (!accumulate(ds_full, static_cast<uint32_t>(it) & 1u, DKV ? tmem_acc2 : tmem_acc1, tmem_dp,
+                        y1_at + slot_a * L::YT, it))
+          break;
+        umma_commit_if(on, &y1_empty[slot_a]);
+        if (++slot_a == Y1_SLOTS) slot_a = 0;
+        if (more) ok = next_dp(it + 1);
+        else umma_commit_if(on, acc_full);
       }
-      if (ok) ok = accumulate_block(n_iter - 1);
-      if (ok) umma_commit(acc_full);
     }
   } else if (warp >= 4) {
     // ------------------------------ compute warpgroups ------------------------------
-    // Four compute warpgroups work on every block together: warpgroup wg takes columns
-    // [16 wg, 16 wg + 16) of the 64-column block, so one block costs a single short pass (one TMEM
-    // round trip, 16 exponentials per thread).  The S / dP buffers alternate from block to block:
-    // the tensor core fills buffer 1 - u and runs the accumulate MMAs of the previous block while
-    // buffer u is exponentiated.
+    // Four compute warpgroups work on every iteration together: warpgroup wg takes columns
+    // [32 wg, 32 wg + 32) of the tile, i.e. 32 columns of entry 2 it + wg / 2.
     const int wg = (warp - 4) >> 2;
     const int quad = warp & 3;
     const int r = quad * 32 + lane;
@@ -311,110 +375,117 @@ attn_bwd_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constant
       neg_delta = args.neg_delta[at];
     }
     bool ok = true;
-    uint32_t sph = 0;                      // bit u: phase parity of s_full[u]
     const uint64_t scale2 = pack_f32x2(args.scale_log2, args.scale_log2);
-    // dense walk: (block, head) advance without a division per iteration
+    const int mine = wg >> 1;               // half of the tile this warpgroup works on
+    // dense walk: (block, head) advance without a division per iteration (the first step moves by one
+    // entry for the warpgroups of the second half, the others by two)
     int walk_block = 0, walk_head = 0;
-    uint32_t ystage = 0, yphase = 0;        // stage of the Y ring that holds block `it` (and its statistics)
+    auto advance = [&](int n) {
+      walk_block += n;
+      while (walk_block >= y_n64) {
+        walk_block -= y_n64;
+        ++walk_head;
+      }
+    };
+    if (!sparse && n_entry > 0) advance(mine);
+    uint32_t y1_slot = 0, y1_phase = 0;       // Y1 slot of iteration `it`
     for (int it = 0; it < n_iter; ++it) {
-      const int u = it & 1;
+      const int entry_at = 2 * it + mine;
+      const bool real = entry_at < n_entry;
       int yb, hq;
       if (sparse) {
-        const int entry = __ldg(it_list + it);
+        const int entry = __ldg(it_list + min(entry_at, n_entry - 1));
         yb = entry & 0xffffff;
         hq = DKV ? hkv * group + (entry >> 24) : head;
       } else {
         yb = y_lo64 + walk_block;
         hq = DKV ? hkv * group + walk_head : head;
-        if (++walk_block == y_n64) {
-          walk_block = 0;
-          ++walk_head;
-        }
+        advance(2);
       }
       const int y0 = yb * 64;                   // (grouped: relative to the group, and nothing is masked)
-      const int base = y0 + 16 * wg;            // first column of this thread
-      // ---- visibility of this row against its 16 columns, as a bit mask.  The keys a query sees
+      const int base = y0 + 32 * (wg & 1);      // first column of this thread
+      // ---- visibility of this row against its 32 columns, as a bit mask.  The keys a query sees
       // and the queries that see a key are both contiguous intervals (runs are contiguous):
       //   DQ   row = query xi,  columns = keys     [start[xi], lim[xi]]
       //   DKV  row = key xi,    columns = queries  [first_q[xi], end[xi]]
-      unsigned vis = (row_seg == 0) ? 0u : (bits_from(row_a - base) & bits_upto(row_b - base) & 0xffffu);
-      if (sparse && vis != 0u) {
-        if (DKV) {
-          if ((row_blk >> 5) >= args.sp.words) {
-            vis = 0u;
-          } else {
-            // when every query of the block selected this key's block the selection adds nothing
-            const unsigned aw = __ldg(args.sp.allsel + ((static_cast<size_t>(b) * args.Hq + hq) * nb64 + yb) * args.sp.words +
-                                      (row_blk >> 5));
-            if (!((aw >> (row_blk & 31)) & 1u)) {
-              // per-query selection bit of this key's block, for the 16 columns of this thread
-              const unsigned* col_sel = args.sp.sel + ((static_cast<size_t>(b) * args.Hq + hq) * args.S + base) * args.sp.words +
-                                        (row_blk >> 5);
-              const int bit = row_blk & 31;
-              unsigned selbits = 0u;
+      // Most tiles are wholly visible: two compares, the mask itself only where some row needs it.
+      unsigned vis = 0xffffffffu;
+      const bool inside = real && row_seg != 0 && row_a <= base && row_b >= base + 31;
+      if (sparse || !__all_sync(0xffffffffu, inside)) {
+        vis = (row_seg == 0 || !real) ? 0u : (bits_from(row_a - base) & bits_upto(row_b - base));
+        if (sparse && vis != 0u) {
+          if (DKV) {
+            if ((row_blk >> 5) >= args.sp.words) {
+              vis = 0u;
+            } else {
+              // when every query of the block selected this key's block the selection adds nothing
+              const unsigned aw = __ldg(args.sp.allsel + ((static_cast<size_t>(b) * args.Hq + hq) * nb64 + yb) * args.sp.words +
+                                        (row_blk >> 5));
+              if (!((aw >> (row_blk & 31)) & 1u)) {
+                // per-query selection bit of this key's block, for the 32 columns of this thread
+                const unsigned* col_sel = args.sp.sel + ((static_cast<size_t>(b) * args.Hq + hq) * args.S + base) * args.sp.words +
+                                          (row_blk >> 5);
+                const int bit = row_blk & 31;
+                unsigned selbits = 0u;
 #pragma unroll 4
-              for (int e = 0; e < 16; ++e)
-                selbits |= ((__ldg(col_sel + static_cast<size_t>(e) * args.sp.words) >> bit) & 1u) << e;
-              vis &= selbits;
+                for (int e = 0; e < 32; ++e)
+                  selbits |= ((__ldg(col_sel + static_cast<size_t>(e) * args.sp.words) >> bit) & 1u) << e;
+                vis &= selbits;
+              }
             }
+          } else {
+            const SparseRow sr = sparse_row(args.sp, b, head, args.Hq, args.S, xi, row_start, y0, 64);
+            const unsigned above = bits_from(sr.bound - base);               // keys >= bound
+            vis &= (sr.v0 ? ~above : 0u) | (sr.v1 ? above : 0u);
           }
-        } else {
-          const SparseRow sr = sparse_row(args.sp, b, head, args.Hq, args.S, xi, row_start, y0, 64);
-          const unsigned above = bits_from(sr.bound - base);               // keys >= bound
-          vis &= (sr.v0 ? ~above : 0u) | (sr.v1 ? above : 0u);
         }
       }
-      const bool all = vis == 0xffffu;
-      // DKV: per-query statistics of this thread's 16 columns, staged beside the block by the producer
-      const float4* lse_col = reinterpret_cast<const float4*>(smem + L::OFF_STAT + ystage * 512) + 4 * wg;
-      const float4* delta_col = lse_col + 16;
-      if (!mbar_wait(&s_full[u], (sph >> u) & 1u, abort_flag, st, SITE_B_CW_S, budget)) {
-        ok = false;
-        break;
-      }
-      sph ^= 1u << u;
+      const bool warp_all = __all_sync(0xffffffffu, vis == 0xffffffffu);
+      // DKV: per-query statistics of this thread's 32 columns, staged beside the tile by the producer
+      const ulonglong2* lse_col = reinterpret_cast<const ulonglong2*>(smem + L::OFF_LSE + (it & 1) * 512) + 8 * wg;
+      const ulonglong2* delta_col = reinterpret_cast<const ulonglong2*>(smem + L::OFF_DELTA + y1_slot * 512) + 8 * wg;
+      const uint32_t s_at = tmem_s(it % S_BUFS) + lane_off + 32 * wg;
+      const uint32_t dp_at = tmem_dp + lane_off + 32 * wg;
       if (DKV) {
-        // S was computed from this stage, so its bytes have landed; the wait makes the statistics
-        // written by the bulk copy visible to this thread
-        if (!mbar_wait(&y_full[ystage], yphase, abort_flag, st, SITE_B_CW_S, budget)) {
+        // (the statistics were written by bulk copies: these waits make them visible to the thread)
+        if (!mbar_wait(&y1_full[y1_slot], y1_phase, abort_flag, st, SITE_B_CW_S, budget) ||
+            !mbar_wait(&y2_full[it & 1], static_cast<uint32_t>(it >> 1) & 1u, abort_flag, st, SITE_B_CW_S, budget)) {
           ok = false;
           break;
         }
       }
-      // (the accumulate MMAs of block it - 2 read P^T / dS from this buffer; they were issued before
-      // the S / dP MMAs of this block and the tensor core completes MMAs in issue order)
+      if (!mbar_wait(&s_full[it % S_BUFS], static_cast<uint32_t>(it / S_BUFS) & 1u, abort_flag, st, SITE_B_CW_S, budget)) {
+        ok = false;
+        break;
+      }
+      // (the accumulate MMAs that read P^T / dS of the previous iteration from these buffers were issued
+      // before the products that refilled them, and the tensor core completes MMAs in issue order)
       tc_fence_after();
-      uint32_t rs[16], rd[16];
-      tmem_ld16(tmem_s(u) + lane_off + 16 * wg, rs);
-      tmem_ld16(tmem_dp(u) + lane_off + 16 * wg, rd);
-      tmem_ld_wait();
-      // Eight columns at a time: probabilities and dS are packed and stored as soon as they exist.
-      // MASKED = false is the path of a warp whose rows all see all 16 columns: no selects.
-      auto compute16 = [&](auto masked_tag) {
+      // MASKED = false is the path of a warp whose rows all see all 32 columns: no selects.
+      float p[32];
+      auto probabilities = [&](auto masked_tag) {
         constexpr bool MASKED = decltype(masked_tag)::value;
+        uint32_t sc[32];
+        tmem_ld32(s_at, sc);
+        tmem_ld_wait();
 #pragma unroll
-        for (int gg = 0; gg < 2; ++gg) {
-          uint32_t pw[4], dw[4];
+        for (int half = 0; half < 2; ++half) {
+          uint32_t pw[8];
 #pragma unroll
-          for (int h4 = 0; h4 < 2; ++h4) {
-            const int e4 = gg * 2 + h4;                  // group of four of the 16 columns
-            uint64_t l2[2], dl[2];                       // negated statistics, two columns per word
+          for (int e4 = 0; e4 < 4; ++e4) {                 // groups of four columns
+            uint64_t l2[2];                                // negated statistics, two columns per word
             if (DKV) {
-              const float4 lv = lse_col[e4];
-              const float4 dv = delta_col[e4];
-              l2[0] = pack_f32x2(lv.x, lv.y);
-              l2[1] = pack_f32x2(lv.z, lv.w);
-              dl[0] = pack_f32x2(dv.x, dv.y);
-              dl[1] = pack_f32x2(dv.z, dv.w);
+              const ulonglong2 lv = lse_col[half * 4 + e4];
+              l2[0] = lv.x;
+              l2[1] = lv.y;
             } else {
               l2[0] = l2[1] = pack_f32x2(neg_lse2, neg_lse2);
-              dl[0] = dl[1] = pack_f32x2(neg_delta, neg_delta);
             }
-            // p = exp2(s * scale - lse), dS = p * (dP - delta): two columns per packed instruction
+            // p = exp2(s * scale - lse): two columns per packed instruction
 #pragma unroll
             for (int pr = 0; pr < 2; ++pr) {
-              const int e = e4 * 4 + pr * 2;
-              const uint64_t x2 = fma_f32x2(pack_f32x2(__uint_as_float(rs[e]), __uint_as_float(rs[e + 1])), scale2, l2[pr]);
+              const int e = half * 16 + e4 * 4 + pr * 2;
+              const uint64_t x2 = fma_f32x2(pack_f32x2(__uint_as_float(sc[e]), __uint_as_float(sc[e + 1])), scale2, l2[pr]);
               float xa, xb;
               unpack_f32x2(x2, xa, xb);
               float pa = fast_exp2(xa), pb = fast_exp2(xb);
@@ -422,26 +493,63 @@ attn_bwd_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constant
                 if (!((vis >> e) & 1u)) pa = 0.f;
                 if (!((vis >> (e + 1)) & 1u)) pb = 0.f;
               }
-              const uint64_t d2 = add_f32x2(pack_f32x2(__uint_as_float(rd[e]), __uint_as_float(rd[e + 1])), dl[pr]);
-              const uint64_t ds2 = mul_f32x2(pack_f32x2(pa, pb), d2);
-              float da, db;
-              unpack_f32x2(ds2, da, db);
-              pw[h4 * 2 + pr] = pack_bf16(pa, pb);
-              dw[h4 * 2 + pr] = pack_bf16(da, db);
+              p[e] = pa;
+              p[e + 1] = pb;
+              if (DKV) pw[e4 * 2 + pr] = pack_bf16(pa, pb);
             }
           }
-          if (DKV) tmem_st4(tmem_s(u) + lane_off + 16 * wg + 4 * gg, pw);
-          tmem_st4(tmem_dp(u) + lane_off + 16 * wg + 4 * gg, dw);
+          if (DKV) {
+            tmem_st8(s_at + 16 * half, pw);
+            tmem_st_wait();
+            tc_fence_before();
+            __syncwarp();
+            if (lane == 0) mbar_arrive(&p_full[2 * (it % S_BUFS) + half]);
+          }
         }
       };
-      if (__all_sync(0xffffffffu, all)) compute16(std::false_type{});
-      else compute16(std::true_type{});
-      tmem_st_wait();
-      tc_fence_before();
-      mbar_arrive(&t_full[u]);
-      if (++ystage == Y_STAGES) {
-        ystage = 0;
-        yphase ^= 1u;
+      if (warp_all) probabilities(std::false_type{});
+      else probabilities(std::true_type{});
+      if (!mbar_wait(dp_full, static_cast<uint32_t>(it) & 1u, abort_flag, st, SITE_B_CW_S, budget)) {
+        ok = false;
+        break;
+      }
+      tc_fence_after();
+      uint32_t rd[32];
+      tmem_ld32(dp_at, rd);
+      tmem_ld_wait();
+      // dS = p * (dP - delta)
+#pragma unroll
+      for (int half = 0; half < 2; ++half) {
+        uint32_t dw[8];
+#pragma unroll
+        for (int e4 = 0; e4 < 4; ++e4) {
+          uint64_t dl[2];
+          if (DKV) {
+            const ulonglong2 dv = delta_col[half * 4 + e4];
+            dl[0] = dv.x;
+            dl[1] = dv.y;
+          } else {
+            dl[0] = dl[1] = pack_f32x2(neg_delta, neg_delta);
+          }
+#pragma unroll
+          for (int pr = 0; pr < 2; ++pr) {
+            const int e = half * 16 + e4 * 4 + pr * 2;
+            const uint64_t d2 = add_f32x2(pack_f32x2(__uint_as_float(rd[e]), __uint_as_float(rd[e + 1])), dl[pr]);
+            const uint64_t ds2 = mul_f32x2(pack_f32x2(p[e], p[e + 1]), d2);
+            float da, db;
+            unpack_f32x2(ds2, da, db);
+            dw[e4 * 2 + pr] = pack_bf16(da, db);
+          }
+        }
+        tmem_st8(dp_at + 16 * half, dw);
+        tmem_st_wait();
+        tc_fence_before();
+        __syncwarp();
+        if (lane == 0) mbar_arrive(&ds_full[half]);
+      }
+      if (++y1_slot == Y1_SLOTS) {
+        y1_slot = 0;
+        y1_phase ^= 1u;
       }
     }
     // the epilogue pairs the warpgroups: pair u converts accumulator u, each warpgroup half of it

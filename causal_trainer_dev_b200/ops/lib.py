@@ -92,6 +92,7 @@ _SITES = {
     0x0304: "attention backward mma: P^T / dS never published",
     0x0305: "attention backward compute: S / dP never completed",
     0x0307: "attention backward compute: accumulators never completed",
+    0x0308: "attention backward: shared memory base not 1024-byte aligned (nothing written)",
     0x0401: "fsdp reduce-scatter: a peer's gradients never arrived",
     0x0402: "fsdp: flags never published",
     0x0501: "tensor-parallel all-gather: a peer's rows never became ready",
