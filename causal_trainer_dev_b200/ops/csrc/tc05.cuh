@@ -458,6 +458,31 @@ __device__ __forceinline__ uint64_t mul_f32x2(uint64_t a, uint64_t b) {
   asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(d) : "l"(a), "l"(b));
   return d;
 }
+// exp2 of a packed pair on the FMA pipe, for a share of the exponentials of kernels whose ex2 unit (16 a
+// clock per SM) is the busiest pipe.  x = n + f with n = round(x) by the 1.5 * 2^23 addition, 2^f on
+// [-1/2, 1/2] by the degree-5 minimax polynomial of the relative error (Remez; 7.7e-8, 2.1e-7 with the
+// rounding of its fp32 steps, where ex2.approx allows 2.4e-7), times 2^n built in the exponent field.
+// Arguments below -125 count as -125 (no zero result), above 127 are not meant; NaN stays NaN.
+__device__ __forceinline__ void poly_exp2_x2(uint64_t x2, float& ya, float& yb) {
+  const uint64_t magic = pack_f32x2(12582912.f, 12582912.f), minus = pack_f32x2(-1.f, -1.f);
+  float xa, xb, ta, tb;
+  unpack_f32x2(x2, xa, xb);
+  asm("max.NaN.f32 %0, %0, %1;" : "+f"(xa) : "f"(-125.f));
+  asm("max.NaN.f32 %0, %0, %1;" : "+f"(xb) : "f"(-125.f));
+  x2 = pack_f32x2(xa, xb);
+  const uint64_t t2 = add_f32x2(x2, magic);
+  const uint64_t f2 = add_f32x2(x2, fma_f32x2(t2, minus, magic));
+  uint64_t p2 = fma_f32x2(pack_f32x2(0.0013277939287945628f, 0.0013277939287945628f), f2,
+                          pack_f32x2(0.009675757959485054f, 0.009675757959485054f));
+  p2 = fma_f32x2(p2, f2, pack_f32x2(0.05550709739327431f, 0.05550709739327431f));
+  p2 = fma_f32x2(p2, f2, pack_f32x2(0.24022114276885986f, 0.24022114276885986f));
+  p2 = fma_f32x2(p2, f2, pack_f32x2(0.6931469440460205f, 0.6931469440460205f));
+  p2 = fma_f32x2(p2, f2, pack_f32x2(1.0000001192092896f, 1.0000001192092896f));
+  unpack_f32x2(t2, ta, tb);
+  const uint64_t n2 = pack_f32x2(__uint_as_float((__float_as_uint(ta) << 23) + 0x3f800000u),
+                                 __uint_as_float((__float_as_uint(tb) << 23) + 0x3f800000u));
+  unpack_f32x2(mul_f32x2(p2, n2), ya, yb);
+}
 __device__ __forceinline__ float fmax3(float a, float b, float c) {
   float d;
   asm("max.f32 %0, %1, %2, %3;" : "=f"(d) : "f"(a), "f"(b), "f"(c));
