@@ -368,6 +368,50 @@ __global__ void attn_bwd_stats_kernel(const __nv_bfloat16* __restrict__ o, const
   }
 }
 
+// The same for D = 64 or 128 and 16-byte aligned rows.  Bound by reading O and dO once.  The kernel
+// above reads 4 bytes per lane and access and stores one float per warp, S floats apart; here a
+// group of D / 8 lanes reads a (token, head) row as 16-byte vectors, a block takes STAT_TOKENS tokens
+// x 8 heads (2 KiB contiguous per token at D = 128) and turns the sums round in shared memory, so that
+// lse is read and both statistics are written 128 bytes at a time.
+constexpr int STAT_TOKENS = 32;
+constexpr int STAT_HEADS = 8;
+template <int D>
+__global__ void __launch_bounds__(256)
+attn_bwd_stats_vec_kernel(const __nv_bfloat16* __restrict__ o, const __nv_bfloat16* __restrict__ dout,
+                          const float* __restrict__ lse, float* __restrict__ neg_lse2,
+                          float* __restrict__ neg_delta, int S, int H, long tokens, long o_rs, long do_rs) {
+  constexpr int LANES = D / 8;                   // lanes per (token, head) row
+  constexpr int ROWS = 256 / LANES;              // rows per pass of the block
+  constexpr int PASSES = STAT_TOKENS * STAT_HEADS / ROWS;
+  __shared__ float sums[STAT_HEADS][STAT_TOKENS + 1];
+  const long t0 = static_cast<long>(blockIdx.x) * STAT_TOKENS;
+  const int h0 = blockIdx.y * STAT_HEADS;
+  const int sub = threadIdx.x / LANES, c = (threadIdx.x % LANES) * 8;
+#pragma unroll 4
+  for (int p = 0; p < PASSES; ++p) {
+    const int row = p * ROWS + sub, hl = row % STAT_HEADS, tl = row / STAT_HEADS;
+    float acc = 0.f;
+    if (t0 + tl < tokens && h0 + hl < H) {
+      const long at = static_cast<long>(h0 + hl) * D + c;
+      float a[8], b[8];
+      unpack8(__ldg(reinterpret_cast<const uint4*>(o + (t0 + tl) * o_rs + at)), a);
+      unpack8(__ldg(reinterpret_cast<const uint4*>(dout + (t0 + tl) * do_rs + at)), b);
+#pragma unroll
+      for (int e = 0; e < 8; ++e) acc += a[e] * b[e];
+    }
+#pragma unroll
+    for (int m = LANES / 2; m > 0; m >>= 1) acc += __shfl_xor_sync(0xffffffffu, acc, m);
+    if (c == 0) sums[hl][tl] = acc;
+  }
+  __syncthreads();
+  const int hl = threadIdx.x >> 5, tl = threadIdx.x & 31;
+  const long t = t0 + tl;
+  if (t >= tokens || h0 + hl >= H) return;
+  const long i = (t / S * H + h0 + hl) * S + t % S;
+  neg_delta[i] = -sums[hl][tl];
+  neg_lse2[i] = -lse[i] * 1.4426950408889634f;
+}
+
 // ------------------------------------------------------------------------------------------
 // Cut-CE combine: merges per-slab (max, sumexp) into lse[row], emits the weighted NLL per
 // row, the backward coefficient coef[row] = weight * grad_scale, and block partial sums of
@@ -831,6 +875,20 @@ CTB_API int ctb_attn_delta(const void* o, const void* dout, float* delta, int B,
 // o, dout: [B,S,H,D] bf16 views (row strides in elements); lse, neg_lse2, neg_delta: [B,H,S] fp32.
 CTB_API int ctb_attn_bwd_stats(const void* o, const void* dout, const float* lse, float* neg_lse2, float* neg_delta,
                                int B, int S, int H, int D, long o_rs, long do_rs, void* stream) {
+  // 16-byte rows of the two head sizes the flash kernels take (anything else: one warp per row, below)
+  const bool wide = (D == 64 || D == 128) && o_rs % 8 == 0 && do_rs % 8 == 0 &&
+                    (reinterpret_cast<uintptr_t>(o) | reinterpret_cast<uintptr_t>(dout)) % 16 == 0;
+  const long tokens = static_cast<long>(B) * S;
+  const int head_blocks = (H + STAT_HEADS - 1) / STAT_HEADS;
+  if (wide && tokens > 0 && H > 0 && head_blocks <= 65535) {
+    const dim3 grid(static_cast<unsigned>((tokens + STAT_TOKENS - 1) / STAT_TOKENS), head_blocks);
+    auto kern = D == 128 ? attn_bwd_stats_vec_kernel<128> : attn_bwd_stats_vec_kernel<64>;
+    kern<<<grid, 256, 0, static_cast<cudaStream_t>(stream)>>>(
+        static_cast<const __nv_bfloat16*>(o), static_cast<const __nv_bfloat16*>(dout), lse, neg_lse2, neg_delta, S, H,
+        tokens, o_rs, do_rs);
+    CTB_CUDA_OK(cudaGetLastError());
+    return 0;
+  }
   const long warps = static_cast<long>(B) * S * H;
   const int threads = 256;
   const long blocks = (warps * 32 + threads - 1) / threads;
