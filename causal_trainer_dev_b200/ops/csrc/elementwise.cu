@@ -183,13 +183,26 @@ rmsnorm_bwd_kernel(const __nv_bfloat16* __restrict__ dy, const __nv_bfloat16* __
   }
 }
 
-// dw[c] (+)= sum_p partial[p][c]; out dtype bf16 or fp32.
-__global__ void rmsnorm_dw_reduce_kernel(const float* __restrict__ partial, int parts, int d, void* __restrict__ dw,
-                                         int out_f32, int accumulate) {
-  const int c = blockIdx.x * blockDim.x + threadIdx.x;
-  if (c >= d) return;
+// dw[c] (+)= sum_p partial[p][c]; out dtype bf16 or fp32.  A block takes 32 columns, its warps take
+// every 8th partial row (128 bytes a row) and join through shared memory in a fixed order: with one
+// thread per column walking all rows, the 16 blocks of d = 4096 were a chain of 296 loads.
+constexpr int DW_WARPS = 8;
+__global__ void __launch_bounds__(DW_WARPS * 32)
+rmsnorm_dw_reduce_kernel(const float* __restrict__ partial, int parts, int d, void* __restrict__ dw, int out_f32,
+                         int accumulate) {
+  __shared__ float sums[DW_WARPS][32];
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  const int c = blockIdx.x * 32 + lane;
   float s = 0.f;
-  for (int p = 0; p < parts; ++p) s += partial[static_cast<size_t>(p) * d + c];
+  if (c < d) {
+#pragma unroll 8
+    for (int p = warp; p < parts; p += DW_WARPS) s += __ldg(partial + static_cast<size_t>(p) * d + c);
+  }
+  sums[warp][lane] = s;
+  __syncthreads();
+  if (warp != 0 || c >= d) return;
+#pragma unroll
+  for (int k = 1; k < DW_WARPS; ++k) s += sums[k][lane];
   if (out_f32) {
     float* o = static_cast<float*>(dw);
     o[c] = accumulate ? o[c] + s : s;
@@ -225,6 +238,59 @@ __global__ void rope_kernel(__nv_bfloat16* __restrict__ x, const float* __restri
     const float b = __bfloat162float(base[i1]);
     base[i0] = __float2bfloat16(a * c - b * s);
     base[i1] = __float2bfloat16(b * c + a * s);
+  }
+}
+
+// The same on 16-byte vectors: a warp owns a token, a lane keeps the cos / sin of its channels in
+// registers and walks the heads, so the table is read once per token instead of once per head and
+// the projection moves in whole 128-byte segments.  Bound by reading and writing the rotated heads once.
+//   gpt-neox: a lane holds channels [8 p, 8 p + 8) of both halves;  gpt-j: four adjacent pairs.
+template <int STYLE>
+__global__ void __launch_bounds__(256)
+rope_vec_kernel(__nv_bfloat16* __restrict__ x, const float* __restrict__ cosv, const float* __restrict__ sinv,
+                long row_stride, int T, int heads, int D, int rot, float sign) {
+  constexpr int N = STYLE == 0 ? 4 : 8;          // angles per lane
+  const int half = rot / 2;
+  const int per_head = half / N;                 // lanes per head (<= 32)
+  const int lane = threadIdx.x & 31;
+  const int together = 32 / per_head;            // heads a warp rotates at once
+  const int p = lane % per_head, first = lane / per_head;
+  if (first >= together) return;
+  const long warps = (static_cast<long>(gridDim.x) * blockDim.x) >> 5;
+  for (long t = (static_cast<long>(blockIdx.x) * blockDim.x + threadIdx.x) >> 5; t < T; t += warps) {
+    float c[N], s[N];
+#pragma unroll
+    for (int e = 0; e < N; e += 4) {
+      *reinterpret_cast<float4*>(c + e) = __ldg(reinterpret_cast<const float4*>(cosv + t * half + p * N + e));
+      *reinterpret_cast<float4*>(s + e) = __ldg(reinterpret_cast<const float4*>(sinv + t * half + p * N + e));
+    }
+#pragma unroll
+    for (int e = 0; e < N; ++e) s[e] *= sign;
+    __nv_bfloat16* row = x + t * row_stride + 8 * p;
+#pragma unroll 4
+    for (int h = first; h < heads; h += together) {
+      uint4* at = reinterpret_cast<uint4*>(row + static_cast<long>(h) * D);
+      float a[8], b[8], o[8];
+      unpack8(at[0], a);
+      if (STYLE == 0) {
+#pragma unroll
+        for (int e = 0; e < 4; ++e) {
+          o[2 * e] = a[2 * e] * c[e] - a[2 * e + 1] * s[e];
+          o[2 * e + 1] = a[2 * e + 1] * c[e] + a[2 * e] * s[e];
+        }
+      } else {
+        uint4* up = reinterpret_cast<uint4*>(row + static_cast<long>(h) * D + half);
+        unpack8(up[0], b);
+        float q[8];
+#pragma unroll
+        for (int e = 0; e < 8; ++e) {
+          o[e] = a[e] * c[e] - b[e] * s[e];
+          q[e] = b[e] * c[e] + a[e] * s[e];
+        }
+        up[0] = pack8(q);
+      }
+      at[0] = pack8(o);
+    }
   }
 }
 
@@ -812,7 +878,7 @@ CTB_API int ctb_rmsnorm_bwd(const void* dy, const void* x, const void* w, const 
 #undef CTB_NORM_BWD
   CTB_CUDA_OK(cudaGetLastError());
   if (dw != nullptr) {
-    rmsnorm_dw_reduce_kernel<<<(d + 255) / 256, 256, 0, s>>>(dw_partial, parts, d, dw, dw_f32, dw_accumulate);
+    rmsnorm_dw_reduce_kernel<<<(d + 31) / 32, DW_WARPS * 32, 0, s>>>(dw_partial, parts, d, dw, dw_f32, dw_accumulate);
     CTB_CUDA_OK(cudaGetLastError());
   }
   return 0;
@@ -829,6 +895,17 @@ CTB_API int ctb_rope_table(const int* pos, const float* inv_freq, float* cosv, f
 CTB_API int ctb_rope(void* x, const float* cosv, const float* sinv, long row_stride, int T, int heads, int D, int rot,
                      int style, int inverse, void* stream) {
   if (rot % 2 || rot > D) return fail("rope: rotary_dim must be even and <= head_dim");
+  // whole 16-byte vectors per lane: 8 channels of each half (gpt-neox) or 4 pairs (gpt-j), at most 32 lanes a head
+  const int angles = style == 0 ? 4 : 8;
+  const int per_head = rot / 2 / angles;
+  if (rot % (2 * angles) == 0 && per_head >= 1 && per_head <= 32 && D % 8 == 0 && row_stride % 8 == 0 && T > 0 &&
+      (reinterpret_cast<uintptr_t>(x) | reinterpret_cast<uintptr_t>(cosv) | reinterpret_cast<uintptr_t>(sinv)) % 16 == 0) {
+    auto kern = style == 0 ? rope_vec_kernel<0> : rope_vec_kernel<1>;
+    kern<<<grid_for(static_cast<long>(T) * 32, 256), 256, 0, static_cast<cudaStream_t>(stream)>>>(
+        static_cast<__nv_bfloat16*>(x), cosv, sinv, row_stride, T, heads, D, rot, inverse ? -1.f : 1.f);
+    CTB_CUDA_OK(cudaGetLastError());
+    return 0;
+  }
   rope_kernel<<<grid_for(static_cast<long>(T) * heads * (rot / 2), 256), 256, 0, static_cast<cudaStream_t>(stream)>>>(
       static_cast<__nv_bfloat16*>(x), cosv, sinv, row_stride, T, heads, D, rot, style, inverse ? -1.f : 1.f);
   CTB_CUDA_OK(cudaGetLastError());
