@@ -103,7 +103,7 @@ def cut_ce_forward(hidden, head, targets, weights, grad_scale: float | torch.Ten
         return nll, wsum, lse, coef
     lse = torch.empty(rows, dtype=torch.float32, device=dev)
     coef = torch.empty(rows, dtype=torch.float32, device=dev)
-    nblk = (rows + 255) // 256
+    nblk = (rows + 31) // 32          # partial sums of 32 rows each (csrc/elementwise.cu: CE_ROWS)
     bn = torch.empty(nblk, dtype=torch.float32, device=dev)
     bw = torch.empty(nblk, dtype=torch.float32, device=dev)
     code = L.ctb_ce_combine(_lib.ptr(pmax), _lib.ptr(psum), slabs, _lib.ptr(tlogit), _lib.ptr(w),

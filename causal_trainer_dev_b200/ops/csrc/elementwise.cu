@@ -117,56 +117,95 @@ rmsnorm_fwd_kernel(const __nv_bfloat16* __restrict__ x, const __nv_bfloat16* __r
 // partial sums of dw = sum_rows dy * xhat into `dw_partial[gridDim.x][d]` (fp32 scratch),
 // reduced by rmsnorm_dw_reduce_kernel.  No atomics: the result is deterministic.
 // ------------------------------------------------------------------------------------------
+// The loads of the next row are issued before the current row is reduced (d <= 4096: wider rows have no
+// registers for it), and the row sum takes one
+// barrier (two alternating sets of warp sums): with the loads, two barriers and the residual load in
+// one chain per row, two CTAs per SM kept too little in flight.
 template <int NV>
 __global__ void __launch_bounds__(NORM_THREADS)
 rmsnorm_bwd_kernel(const __nv_bfloat16* __restrict__ dy, const __nv_bfloat16* __restrict__ x,
                    const __nv_bfloat16* __restrict__ w, const float* __restrict__ rstd,
                    const __nv_bfloat16* __restrict__ dres, __nv_bfloat16* __restrict__ dx,
                    float* __restrict__ dw_partial, int rows, int d) {
-  __shared__ float scratch[33];
+  constexpr int WARPS = NORM_THREADS / 32;
+  constexpr bool AHEAD = NV <= 2;
+  constexpr bool HOLD = NV <= 4;          // w and the residual gradient in registers (else read where they are used)
+  __shared__ float sums[2][WARPS];
   const int nvec = d / 8;
   float dw_acc[NV][8];
+  uint4 wv[NV], dyv[NV], xv[NV], rv[NV];
+  const uint4 zero = make_uint4(0u, 0u, 0u, 0u);
 #pragma unroll
-  for (int i = 0; i < NV; ++i)
+  for (int i = 0; i < NV; ++i) {
+    const int v = threadIdx.x + i * NORM_THREADS;
+    if (HOLD) wv[i] = v < nvec ? reinterpret_cast<const uint4*>(w)[v] : zero;
+    rv[i] = zero;
 #pragma unroll
     for (int e = 0; e < 8; ++e) dw_acc[i][e] = 0.f;
-  for (int row = blockIdx.x; row < rows; row += gridDim.x) {
-    const float rs = rstd[row];
-    const uint4* dyr = reinterpret_cast<const uint4*>(dy + static_cast<size_t>(row) * d);
-    const uint4* xr = reinterpret_cast<const uint4*>(x + static_cast<size_t>(row) * d);
-    float gx[NV][8], xh[NV][8];
+  }
+  float rs = 0.f;
+  auto fetch = [&](int row) {
+    const size_t at = static_cast<size_t>(row) * nvec;
+    rs = rstd[row];
+#pragma unroll
+    for (int i = 0; i < NV; ++i) {
+      const int v = threadIdx.x + i * NORM_THREADS;
+      if (v < nvec) {
+        dyv[i] = reinterpret_cast<const uint4*>(dy)[at + v];
+        xv[i] = reinterpret_cast<const uint4*>(x)[at + v];
+        if (HOLD && dres) rv[i] = reinterpret_cast<const uint4*>(dres)[at + v];
+      } else {
+        dyv[i] = xv[i] = zero;
+      }
+    }
+  };
+  if (AHEAD && blockIdx.x < rows) fetch(blockIdx.x);
+  int parity = 0;
+  for (int row = blockIdx.x; row < rows; row += gridDim.x, parity ^= 1) {
+    if (!AHEAD) fetch(row);
+    const float r_now = rs;
+    uint4 dy_now[NV], x_now[NV], res_now[NV];
+#pragma unroll
+    for (int i = 0; i < NV; ++i) {
+      dy_now[i] = dyv[i];
+      x_now[i] = xv[i];
+      res_now[i] = rv[i];
+    }
+    if (AHEAD && row + static_cast<int>(gridDim.x) < rows) fetch(row + gridDim.x);
     float dot = 0.f;
 #pragma unroll
     for (int i = 0; i < NV; ++i) {
+      float a[8], b[8], c[8];
+      unpack8(dy_now[i], a);
+      unpack8(x_now[i], b);
       const int v = threadIdx.x + i * NORM_THREADS;
-      if (v < nvec) {
-        float a[8], b[8], c[8];
-        unpack8(dyr[v], a);
-        unpack8(xr[v], b);
-        unpack8(reinterpret_cast<const uint4*>(w)[v], c);
+      unpack8(HOLD ? wv[i] : (v < nvec ? __ldg(reinterpret_cast<const uint4*>(w) + v) : zero), c);
 #pragma unroll
-        for (int e = 0; e < 8; ++e) {
-          xh[i][e] = b[e] * rs;
-          gx[i][e] = a[e] * c[e];
-          dot += gx[i][e] * xh[i][e];
-          dw_acc[i][e] += a[e] * xh[i][e];
-        }
+      for (int e = 0; e < 8; ++e) {
+        const float xh = b[e] * r_now;
+        dot += a[e] * c[e] * xh;
+        dw_acc[i][e] += a[e] * xh;
       }
     }
-    const float mean = block_sum(dot, scratch) / d;
+    dot = warp_sum(dot);
+    if ((threadIdx.x & 31) == 0) sums[parity][threadIdx.x >> 5] = dot;
+    __syncthreads();
+    float mean = 0.f;
+#pragma unroll
+    for (int k = 0; k < WARPS; ++k) mean += sums[parity][k];
+    mean /= d;
 #pragma unroll
     for (int i = 0; i < NV; ++i) {
       const int v = threadIdx.x + i * NORM_THREADS;
       if (v < nvec) {
-        float o[8];
+        float a[8], b[8], c[8], r[8], o[8];
+        unpack8(dy_now[i], a);
+        unpack8(x_now[i], b);
+        unpack8(HOLD ? wv[i] : __ldg(reinterpret_cast<const uint4*>(w) + v), c);
+        if (!HOLD && dres) res_now[i] = reinterpret_cast<const uint4*>(dres)[static_cast<size_t>(row) * nvec + v];
+        unpack8(res_now[i], r);
 #pragma unroll
-        for (int e = 0; e < 8; ++e) o[e] = rs * (gx[i][e] - xh[i][e] * mean);
-        if (dres) {
-          float r[8];
-          unpack8(reinterpret_cast<const uint4*>(dres + static_cast<size_t>(row) * d)[v], r);
-#pragma unroll
-          for (int e = 0; e < 8; ++e) o[e] += r[e];
-        }
+        for (int e = 0; e < 8; ++e) o[e] = r_now * (a[e] * c[e] - b[e] * r_now * mean) + r[e];
         reinterpret_cast<uint4*>(dx + static_cast<size_t>(row) * d)[v] = pack8(o);
       }
     }
@@ -315,48 +354,74 @@ __global__ void rope_table_kernel(const int* __restrict__ pos, const float* __re
 // SwiGLU on the packed projection gu[T][2f] = [gate | up]:  h = silu(gate) * up.
 // Backward writes d(gate|up) in the same packed layout.
 // ------------------------------------------------------------------------------------------
-__global__ void swiglu_fwd_kernel(const __nv_bfloat16* __restrict__ gu, __nv_bfloat16* __restrict__ h, long T, int f) {
-  const int nvec = f / 8;
-  const long total = T * nvec;
-  for (long i = blockIdx.x * static_cast<long>(blockDim.x) + threadIdx.x; i < total;
-       i += static_cast<long>(gridDim.x) * blockDim.x) {
-    const long t = i / nvec;
-    const int v = static_cast<int>(i % nvec);
-    const uint4* row = reinterpret_cast<const uint4*>(gu + t * 2 * f);
-    float g[8], u[8], o[8];
-    unpack8(row[v], g);
-    unpack8(row[nvec + v], u);
+// A thread keeps its column vector and walks the rows (blockIdx.y, two at a time), so there is no
+// division per vector; the quotient of the sigmoid is the fast one (2 ulp, the result is rounded to
+// bf16): with the IEEE division the forward kernel was bound by instructions, 345 us for the 1.41 GB
+// of 16384 x 14336, not by memory.
+constexpr int SWIGLU_ROWS = 2;
+__global__ void __launch_bounds__(256)
+swiglu_fwd_kernel(const __nv_bfloat16* __restrict__ gu, __nv_bfloat16* __restrict__ h, long T, int f) {
+  const int nvec = f / 8, v = blockIdx.x * blockDim.x + threadIdx.x;
+  if (v >= nvec) return;
+  const long step = static_cast<long>(gridDim.y) * SWIGLU_ROWS;
+  for (long t0 = static_cast<long>(blockIdx.y) * SWIGLU_ROWS; t0 < T; t0 += step) {
+    uint4 gv[SWIGLU_ROWS], uv[SWIGLU_ROWS];
 #pragma unroll
-    for (int e = 0; e < 8; ++e) {
-      const float act = __bfloat162float(__float2bfloat16(g[e] / (1.f + __expf(-g[e]))));
-      o[e] = act * u[e];
-    }
-    reinterpret_cast<uint4*>(h + t * f)[v] = pack8(o);
+    for (int k = 0; k < SWIGLU_ROWS; ++k)
+      if (t0 + k < T) {
+        const uint4* row = reinterpret_cast<const uint4*>(gu) + static_cast<size_t>(t0 + k) * 2 * nvec;
+        gv[k] = row[v];
+        uv[k] = row[nvec + v];
+      }
+#pragma unroll
+    for (int k = 0; k < SWIGLU_ROWS; ++k)
+      if (t0 + k < T) {
+        float g[8], u[8], o[8];
+        unpack8(gv[k], g);
+        unpack8(uv[k], u);
+#pragma unroll
+        for (int e = 0; e < 8; ++e) {
+          const float act = __bfloat162float(__float2bfloat16(__fdividef(g[e], 1.f + __expf(-g[e]))));
+          o[e] = act * u[e];
+        }
+        reinterpret_cast<uint4*>(h)[static_cast<size_t>(t0 + k) * nvec + v] = pack8(o);
+      }
   }
 }
-__global__ void swiglu_bwd_kernel(const __nv_bfloat16* __restrict__ gu, const __nv_bfloat16* __restrict__ dh,
-                                  __nv_bfloat16* __restrict__ dgu, long T, int f) {
-  const int nvec = f / 8;
-  const long total = T * nvec;
-  for (long i = blockIdx.x * static_cast<long>(blockDim.x) + threadIdx.x; i < total;
-       i += static_cast<long>(gridDim.x) * blockDim.x) {
-    const long t = i / nvec;
-    const int v = static_cast<int>(i % nvec);
-    const uint4* row = reinterpret_cast<const uint4*>(gu + t * 2 * f);
-    float g[8], u[8], d[8], dg[8], du[8];
-    unpack8(row[v], g);
-    unpack8(row[nvec + v], u);
-    unpack8(reinterpret_cast<const uint4*>(dh + t * f)[v], d);
+__global__ void __launch_bounds__(256)
+swiglu_bwd_kernel(const __nv_bfloat16* __restrict__ gu, const __nv_bfloat16* __restrict__ dh,
+                  __nv_bfloat16* __restrict__ dgu, long T, int f) {
+  const int nvec = f / 8, v = blockIdx.x * blockDim.x + threadIdx.x;
+  if (v >= nvec) return;
+  const long step = static_cast<long>(gridDim.y) * SWIGLU_ROWS;
+  for (long t0 = static_cast<long>(blockIdx.y) * SWIGLU_ROWS; t0 < T; t0 += step) {
+    uint4 gv[SWIGLU_ROWS], uv[SWIGLU_ROWS], dv[SWIGLU_ROWS];
 #pragma unroll
-    for (int e = 0; e < 8; ++e) {
-      const float sg = 1.f / (1.f + __expf(-g[e]));
-      const float act = g[e] * sg;
-      du[e] = d[e] * act;
-      dg[e] = d[e] * u[e] * sg * (1.f + g[e] * (1.f - sg));
-    }
-    uint4* orow = reinterpret_cast<uint4*>(dgu + t * 2 * f);
-    orow[v] = pack8(dg);
-    orow[nvec + v] = pack8(du);
+    for (int k = 0; k < SWIGLU_ROWS; ++k)
+      if (t0 + k < T) {
+        const uint4* row = reinterpret_cast<const uint4*>(gu) + static_cast<size_t>(t0 + k) * 2 * nvec;
+        gv[k] = row[v];
+        uv[k] = row[nvec + v];
+        dv[k] = reinterpret_cast<const uint4*>(dh)[static_cast<size_t>(t0 + k) * nvec + v];
+      }
+#pragma unroll
+    for (int k = 0; k < SWIGLU_ROWS; ++k)
+      if (t0 + k < T) {
+        float g[8], u[8], d[8], dg[8], du[8];
+        unpack8(gv[k], g);
+        unpack8(uv[k], u);
+        unpack8(dv[k], d);
+#pragma unroll
+        for (int e = 0; e < 8; ++e) {
+          const float sg = __fdividef(1.f, 1.f + __expf(-g[e]));
+          const float act = g[e] * sg;
+          du[e] = d[e] * act;
+          dg[e] = d[e] * u[e] * sg * (1.f + g[e] * (1.f - sg));
+        }
+        uint4* orow = reinterpret_cast<uint4*>(dgu) + static_cast<size_t>(t0 + k) * 2 * nvec;
+        orow[v] = pack8(dg);
+        orow[nvec + v] = pack8(du);
+      }
   }
 }
 
@@ -483,32 +548,56 @@ attn_bwd_stats_vec_kernel(const __nv_bfloat16* __restrict__ o, const __nv_bfloat
 // row, the backward coefficient coef[row] = weight * grad_scale, and block partial sums of
 // (nll, weight) which the host-side wrapper adds up (fp32, fixed order: deterministic).
 // ------------------------------------------------------------------------------------------
-__global__ void ce_combine_kernel(const float* __restrict__ pmax, const float* __restrict__ psum, int slabs,
-                                  const float* __restrict__ target_logit, const float* __restrict__ weights,
-                                  float grad_scale, float* __restrict__ lse, float* __restrict__ coef,
-                                  float* __restrict__ block_nll, float* __restrict__ block_w, int rows) {
-  __shared__ float scratch[33];
-  const int row = blockIdx.x * blockDim.x + threadIdx.x;
-  float nll = 0.f, w = 0.f;
-  if (row < rows) {
-    float m = -INFINITY;
-    for (int s = 0; s < slabs; ++s) m = fmaxf(m, pmax[static_cast<size_t>(s) * rows + row]);
-    float acc = 0.f;
-    for (int s = 0; s < slabs; ++s) {
+// A block takes CE_ROWS rows (one per lane); its warps share the slabs and join through shared memory in a
+// fixed order.  With a thread walking all slabs of its row, the 16 blocks of 4096 rows were a chain of
+// 2 x 501 loads (129 us).
+constexpr int CE_ROWS = 32, CE_WARPS = 8;
+__global__ void __launch_bounds__(CE_ROWS * CE_WARPS)
+ce_combine_kernel(const float* __restrict__ pmax, const float* __restrict__ psum, int slabs,
+                  const float* __restrict__ target_logit, const float* __restrict__ weights, float grad_scale,
+                  float* __restrict__ lse, float* __restrict__ coef, float* __restrict__ block_nll,
+                  float* __restrict__ block_w, int rows) {
+  __shared__ float part[CE_WARPS][CE_ROWS];
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  const int row = blockIdx.x * CE_ROWS + lane;
+  const bool live = row < rows;
+  float m = -INFINITY;
+  if (live) {
+#pragma unroll 8
+    for (int s = warp; s < slabs; s += CE_WARPS) m = fmaxf(m, __ldg(pmax + static_cast<size_t>(s) * rows + row));
+  }
+  part[warp][lane] = m;
+  __syncthreads();
+#pragma unroll
+  for (int k = 0; k < CE_WARPS; ++k) m = fmaxf(m, part[k][lane]);
+  float acc = 0.f;
+  if (live) {
+#pragma unroll 8
+    for (int s = warp; s < slabs; s += CE_WARPS) {
       const size_t i = static_cast<size_t>(s) * rows + row;
-      acc += psum[i] * __expf(pmax[i] - m);
+      acc += __ldg(psum + i) * __expf(__ldg(pmax + i) - m);
     }
+  }
+  __syncthreads();
+  part[warp][lane] = acc;
+  __syncthreads();
+  if (warp != 0) return;
+  acc = 0.f;
+#pragma unroll
+  for (int k = 0; k < CE_WARPS; ++k) acc += part[k][lane];
+  float nll = 0.f, w = 0.f;
+  if (live) {
     const float l = m + logf(acc);
     lse[row] = l;
     w = weights[row];
     coef[row] = w * grad_scale;
     nll = (w != 0.f) ? (l - target_logit[row]) * w : 0.f;
   }
-  const float bn = block_sum(nll, scratch);
-  const float bw = block_sum(w, scratch);
-  if (threadIdx.x == 0) {
-    block_nll[blockIdx.x] = bn;
-    block_w[blockIdx.x] = bw;
+  nll = warp_sum(nll);
+  w = warp_sum(w);
+  if (lane == 0) {
+    block_nll[blockIdx.x] = nll;
+    block_w[blockIdx.x] = w;
   }
 }
 
@@ -597,16 +686,45 @@ logits_ce_backward_kernel(__nv_bfloat16* __restrict__ logits, long ld, int vocab
 // ------------------------------------------------------------------------------------------
 // Sum of squares (fp32) of a bf16 / fp32 vector into per-block partials.
 // ------------------------------------------------------------------------------------------
+// 16-byte loads, four in flight per thread (with one element per load: 3.0 TB/s on 872 MB of fp32); a
+// vector whose base is not 16-byte aligned is read element by element.
+__device__ __forceinline__ float square_of(float v, int round_bf16) {
+  if (round_bf16) v = __bfloat162float(__float2bfloat16(v));
+  return v * v;
+}
 template <typename T>
-__global__ void sumsq_kernel(const T* __restrict__ x, long n, float* __restrict__ partial, int round_bf16) {
+__global__ void __launch_bounds__(256)
+sumsq_kernel(const T* __restrict__ x, long n, float* __restrict__ partial, int round_bf16) {
+  constexpr int N = 16 / sizeof(T), UNROLL = 4;
   __shared__ float scratch[33];
+  const long first = blockIdx.x * static_cast<long>(blockDim.x) + threadIdx.x;
+  const long stride = static_cast<long>(gridDim.x) * blockDim.x;
   float acc = 0.f;
-  for (long i = blockIdx.x * static_cast<long>(blockDim.x) + threadIdx.x; i < n;
-       i += static_cast<long>(gridDim.x) * blockDim.x) {
-    float v = static_cast<float>(x[i]);
-    if (round_bf16) v = __bfloat162float(__float2bfloat16(v));
-    acc += v * v;
+  auto add = [&](const uint4& raw) {
+    if (sizeof(T) == 4) {
+      acc += square_of(__uint_as_float(raw.x), round_bf16);
+      acc += square_of(__uint_as_float(raw.y), round_bf16);
+      acc += square_of(__uint_as_float(raw.z), round_bf16);
+      acc += square_of(__uint_as_float(raw.w), round_bf16);
+    } else {
+      float f[8];
+      unpack8(raw, f);
+#pragma unroll
+      for (int e = 0; e < 8; ++e) acc += f[e] * f[e];
+    }
+  };
+  const long nvec = reinterpret_cast<uintptr_t>(x) % 16 == 0 ? n / N : 0;
+  const uint4* xv = reinterpret_cast<const uint4*>(x);
+  long i = first;
+  for (; i + (UNROLL - 1) * stride < nvec; i += UNROLL * stride) {
+    uint4 raw[UNROLL];
+#pragma unroll
+    for (int k = 0; k < UNROLL; ++k) raw[k] = __ldg(xv + i + k * stride);
+#pragma unroll
+    for (int k = 0; k < UNROLL; ++k) add(raw[k]);
   }
+  for (; i < nvec; i += stride) add(__ldg(xv + i));
+  for (long j = nvec * N + first; j < n; j += stride) acc += square_of(static_cast<float>(x[j]), round_bf16);
   const float t = block_sum(acc, scratch);
   if (threadIdx.x == 0) partial[blockIdx.x] = t;
 }
@@ -912,9 +1030,20 @@ CTB_API int ctb_rope(void* x, const float* cosv, const float* sinv, long row_str
   return 0;
 }
 
+// Column blocks x row blocks, about eight CTAs per SM.
+static inline dim3 swiglu_grid(long T, int f) {
+  const long cols = (f / 8 + 255) / 256;
+  long rows = (T + SWIGLU_ROWS - 1) / SWIGLU_ROWS;
+  const long cap = (static_cast<long>(sm_count()) * 8 + cols - 1) / cols;
+  if (rows > cap) rows = cap;
+  if (rows > 65535) rows = 65535;
+  return dim3(static_cast<unsigned>(cols), static_cast<unsigned>(rows));
+}
+
 CTB_API int ctb_swiglu_fwd(const void* gu, void* h, long T, int f, void* stream) {
   if (f % 8) return fail("swiglu: intermediate size must be a multiple of 8");
-  swiglu_fwd_kernel<<<grid_for(T * (f / 8), 256), 256, 0, static_cast<cudaStream_t>(stream)>>>(
+  if (T <= 0 || f <= 0) return 0;
+  swiglu_fwd_kernel<<<swiglu_grid(T, f), 256, 0, static_cast<cudaStream_t>(stream)>>>(
       static_cast<const __nv_bfloat16*>(gu), static_cast<__nv_bfloat16*>(h), T, f);
   CTB_CUDA_OK(cudaGetLastError());
   return 0;
@@ -922,7 +1051,8 @@ CTB_API int ctb_swiglu_fwd(const void* gu, void* h, long T, int f, void* stream)
 
 CTB_API int ctb_swiglu_bwd(const void* gu, const void* dh, void* dgu, long T, int f, void* stream) {
   if (f % 8) return fail("swiglu: intermediate size must be a multiple of 8");
-  swiglu_bwd_kernel<<<grid_for(T * (f / 8), 256), 256, 0, static_cast<cudaStream_t>(stream)>>>(
+  if (T <= 0 || f <= 0) return 0;
+  swiglu_bwd_kernel<<<swiglu_grid(T, f), 256, 0, static_cast<cudaStream_t>(stream)>>>(
       static_cast<const __nv_bfloat16*>(gu), static_cast<const __nv_bfloat16*>(dh), static_cast<__nv_bfloat16*>(dgu),
       T, f);
   CTB_CUDA_OK(cudaGetLastError());
@@ -976,11 +1106,11 @@ CTB_API int ctb_attn_bwd_stats(const void* o, const void* dout, const float* lse
   return 0;
 }
 
-// block_nll / block_w must hold ceil(rows / 256) floats each.
+// block_nll / block_w must hold ceil(rows / 32) floats each.
 CTB_API int ctb_ce_combine(const float* pmax, const float* psum, int slabs, const float* target_logit,
                            const float* weights, float grad_scale, float* lse, float* coef, float* block_nll,
                            float* block_w, int rows, void* stream) {
-  ce_combine_kernel<<<(rows + 255) / 256, 256, 0, static_cast<cudaStream_t>(stream)>>>(
+  ce_combine_kernel<<<(rows + CE_ROWS - 1) / CE_ROWS, CE_ROWS * CE_WARPS, 0, static_cast<cudaStream_t>(stream)>>>(
       pmax, psum, slabs, target_logit, weights, grad_scale, lse, coef, block_nll, block_w, rows);
   CTB_CUDA_OK(cudaGetLastError());
   return 0;
