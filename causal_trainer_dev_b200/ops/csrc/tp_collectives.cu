@@ -322,28 +322,94 @@ __global__ void embed_push_kernel(const int* __restrict__ ids, const __nv_bfloat
 // stable sort of the ids (one CTA per run, fixed order, fp32) and added to the gradient table.
 // Rows outside [vocab_lo, vocab_lo + vocab_rows) and the padding row are skipped.
 // ------------------------------------------------------------------------------------------
-template <typename G>
-__global__ void embedding_backward_kernel(const int* __restrict__ sorted_ids, const int* __restrict__ perm,
-                                          const int* __restrict__ run_start, int n_runs, long tokens,
-                                          const __nv_bfloat16* __restrict__ dout, G* __restrict__ grad, int d,
-                                          int vocab_lo, int vocab_rows, int pad_id) {
-  for (int run = blockIdx.x; run < n_runs; run += gridDim.x) {
-    const long s0 = run_start[run];
-    const long s1 = (run + 1 < n_runs) ? run_start[run + 1] : tokens;
-    const int id = sorted_ids[s0];
-    const int local = id - vocab_lo;
-    if (id == pad_id || local < 0 || local >= vocab_rows) continue;
-    for (int c = threadIdx.x * 2; c < d; c += blockDim.x * 2) {
-      float a0 = 0.f, a1 = 0.f;
-      for (long s = s0; s < s1; ++s) {
-        const float2 f = __bfloat1622float2(
-            *reinterpret_cast<const __nv_bfloat162*>(dout + static_cast<long>(perm[s]) * d + c));
-        a0 += f.x;
-        a1 += f.y;
+// `sorted_ids` holds the token ids in order, `perm` where each came from; a run is a stretch of one id.  A CTA
+// looks at EMB_WARPS positions and takes the runs that begin there, 32 * V columns a warp: short runs one
+// per warp, runs longer than LONG_RUN (a mask token, a newline) by all eight warps together, whose partial sums
+// are added in warp order, so the result does not depend on timing.  Finding the runs here instead of in a
+// list spares the host a read back of their number.  With one CTA walking a run row by row, 4 bytes per
+// load, 4000 repeats of one token were a chain of 4000 loads (968 us of a step).
+constexpr int LONG_RUN = 16;
+constexpr int EMB_WARPS = 8;
+template <int V> struct EmbRaw;
+template <> struct EmbRaw<8> { using T = uint4; };
+template <> struct EmbRaw<2> { using T = uint32_t; };
+template <typename G, int V>
+__global__ void __launch_bounds__(EMB_WARPS * 32)
+embedding_backward_kernel(const int* __restrict__ sorted_ids, const int* __restrict__ perm, int tokens,
+                          const __nv_bfloat16* __restrict__ dout, G* __restrict__ grad, int d, int vocab_lo,
+                          int vocab_rows, int pad_id) {
+  using Raw = typename EmbRaw<V>::T;
+  __shared__ float part[EMB_WARPS][32 * V];
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  const int c = (blockIdx.y * 32 + lane) * V;
+  const bool live = c < d;
+  // acc += rows perm[s0], perm[s0 + step], ... of dout, eight loads in flight
+  auto gather = [&](int s0, int s1, int step, float (&acc)[V]) {
+    constexpr int U = 8;
+    for (int s = s0; s < s1; s += U * step) {
+      Raw raw[U];
+#pragma unroll
+      for (int k = 0; k < U; ++k) {
+        // past the end: the run's last row again, not added (unconditional loads stay in flight together)
+        const int at = min(s + k * step, s1 - 1);
+        raw[k] = __ldg(reinterpret_cast<const Raw*>(dout + static_cast<long>(__ldg(perm + at)) * d + (live ? c : 0)));
       }
-      G* g = grad + static_cast<long>(local) * d + c;
-      g[0] = static_cast<G>(static_cast<float>(g[0]) + a0);
-      g[1] = static_cast<G>(static_cast<float>(g[1]) + a1);
+#pragma unroll
+      for (int k = 0; k < U; ++k) {
+        if (s + k * step < s1) {
+          const __nv_bfloat162* h = reinterpret_cast<const __nv_bfloat162*>(&raw[k]);
+#pragma unroll
+          for (int e = 0; e < V / 2; ++e) {
+            const float2 f = __bfloat1622float2(h[e]);
+            acc[2 * e] += f.x;
+            acc[2 * e + 1] += f.y;
+          }
+        }
+      }
+    }
+  };
+  auto add_row = [&](int local, const float (&acc)[V]) {
+    G* g = grad + static_cast<long>(local) * d + c;
+#pragma unroll
+    for (int e = 0; e < V; ++e) g[e] = static_cast<G>(static_cast<float>(g[e]) + acc[e]);
+  };
+  for (int first = blockIdx.x * EMB_WARPS; first < tokens; first += gridDim.x * EMB_WARPS) {
+    for (int k = 0; k < EMB_WARPS && first + k < tokens; ++k) {       // (uniform over the CTA up to `shared_run`)
+      const int s0 = first + k;
+      const int id = __ldg(sorted_ids + s0), local = id - vocab_lo;
+      if (s0 > 0 && __ldg(sorted_ids + s0 - 1) == id) continue;
+      if (id == pad_id || local < 0 || local >= vocab_rows) continue;
+      const bool shared_run = s0 + LONG_RUN < tokens && __ldg(sorted_ids + s0 + LONG_RUN) == id;
+      if (!shared_run && k != warp) continue;
+      int s1 = s0 + 1;
+      float acc[V];
+#pragma unroll
+      for (int e = 0; e < V; ++e) acc[e] = 0.f;
+      if (!shared_run) {
+        while (s1 < tokens && __ldg(sorted_ids + s1) == id) ++s1;
+        gather(s0, s1, 1, acc);
+        if (live) add_row(local, acc);
+        continue;
+      }
+      int hi = tokens;                     // first position past the run, by bisection
+      s1 = s0 + LONG_RUN + 1;
+      while (s1 < hi) {
+        const int mid = s1 + (hi - s1) / 2;
+        if (__ldg(sorted_ids + mid) == id) s1 = mid + 1;
+        else hi = mid;
+      }
+      gather(s0 + warp, s1, EMB_WARPS, acc);
+#pragma unroll
+      for (int e = 0; e < V; ++e) part[warp][e * 32 + lane] = acc[e];
+      __syncthreads();
+      if (warp == 0 && live) {
+#pragma unroll 1
+        for (int w = 1; w < EMB_WARPS; ++w)
+#pragma unroll
+          for (int e = 0; e < V; ++e) acc[e] += part[w][e * 32 + lane];
+        add_row(local, acc);
+      }
+      __syncthreads();
     }
   }
 }
@@ -423,21 +489,30 @@ CTB_API int ctb_embed_push(const int* ids, const void* table, void* const* out_p
   return 0;
 }
 
-CTB_API int ctb_embedding_backward(const int* sorted_ids, const int* perm, const int* run_start, int n_runs,
-                                   long tokens, const void* dout, void* grad, int grad_f32, int d, int vocab_lo,
-                                   int vocab_rows, int pad_id, void* stream) {
-  if (n_runs <= 0) return 0;
+CTB_API int ctb_embedding_backward(const int* sorted_ids, const int* perm, long tokens, const void* dout, void* grad,
+                                   int grad_f32, int d, int vocab_lo, int vocab_rows, int pad_id, void* stream) {
+  if (tokens <= 0) return 0;
   if (d % 2) return fail("embedding_backward: hidden size must be even");
-  const int grid = n_runs < 148 * 8 ? n_runs : 148 * 8;
+  if (tokens > 0x7fff0000L) return fail("embedding_backward: too many tokens");
   cudaStream_t s = static_cast<cudaStream_t>(stream);
-  if (grad_f32)
-    embedding_backward_kernel<float><<<grid, 256, 0, s>>>(sorted_ids, perm, run_start, n_runs, tokens,
-                                                         static_cast<const __nv_bfloat16*>(dout),
-                                                         static_cast<float*>(grad), d, vocab_lo, vocab_rows, pad_id);
-  else
-    embedding_backward_kernel<__nv_bfloat16><<<grid, 256, 0, s>>>(
-        sorted_ids, perm, run_start, n_runs, tokens, static_cast<const __nv_bfloat16*>(dout),
-        static_cast<__nv_bfloat16*>(grad), d, vocab_lo, vocab_rows, pad_id);
+  const auto* src = static_cast<const __nv_bfloat16*>(dout);
+  const int n = static_cast<int>(tokens);
+  const bool wide = d % 8 == 0 && reinterpret_cast<uintptr_t>(dout) % 16 == 0;     // whole 16-byte vectors
+  const int width = wide ? 256 : 64, chunks = (d + width - 1) / width;
+  if (chunks > 65535) return fail("embedding_backward: hidden size too large");
+  const int blocks = (n + EMB_WARPS - 1) / EMB_WARPS, cap = (148 * 32 + chunks - 1) / chunks;
+  const dim3 grid(static_cast<unsigned>(blocks < cap ? blocks : cap), static_cast<unsigned>(chunks));
+#define CTB_EMB(G, V)                                                                                          \
+  embedding_backward_kernel<G, V><<<grid, EMB_WARPS * 32, 0, s>>>(sorted_ids, perm, n, src, static_cast<G*>(grad), d, \
+                                                                  vocab_lo, vocab_rows, pad_id)
+  if (grad_f32) {
+    if (wide) CTB_EMB(float, 8);
+    else CTB_EMB(float, 2);
+  } else {
+    if (wide) CTB_EMB(__nv_bfloat16, 8);
+    else CTB_EMB(__nv_bfloat16, 2);
+  }
+#undef CTB_EMB
   CTB_CUDA_OK(cudaGetLastError());
   return 0;
 }

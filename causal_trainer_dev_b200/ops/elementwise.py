@@ -161,15 +161,10 @@ def embedding_backward(ids: torch.Tensor, dout: torch.Tensor, grad: torch.Tensor
     """
     flat = ids.reshape(-1).to(torch.int32)
     order = torch.sort(flat, stable=True)
-    sorted_ids = order.values.contiguous()
-    perm = order.indices.to(torch.int32).contiguous()
-    change = torch.ones_like(sorted_ids, dtype=torch.bool)
-    change[1:] = sorted_ids[1:] != sorted_ids[:-1]
-    starts = torch.nonzero(change).reshape(-1).to(torch.int32).contiguous()
-    code = _lib.lib().ctb_embedding_backward(_lib.ptr(sorted_ids), _lib.ptr(perm), _lib.ptr(starts), starts.numel(),
-                                             _l(flat.numel()), _lib.ptr(dout), _lib.ptr(grad),
-                                             int(grad.dtype == torch.float32), dout.shape[1], vocab_lo, grad.shape[0],
-                                             pad_id, _lib.stream_ptr())
+    perm = order.indices.to(torch.int32)
+    code = _lib.lib().ctb_embedding_backward(_lib.ptr(order.values), _lib.ptr(perm), _l(flat.numel()), _lib.ptr(dout),
+                                             _lib.ptr(grad), int(grad.dtype == torch.float32), dout.shape[1], vocab_lo,
+                                             grad.shape[0], pad_id, _lib.stream_ptr())
     _lib.check(code, "ctb_embedding_backward")
 
 
