@@ -742,6 +742,8 @@ int run_gemm(const GemmCall& c) {
   const bool needs_c = (c.epi != EPI_CE_STATS) && !c.push.enabled;
   if (needs_c && (c.ldc % (c.out_f32 ? 4 : 8))) return fail("gemm: ldc must be a multiple of 16 bytes");
   if (gemm_pair_eligible(c)) return launch_gemm_pair(c);       // two-CTA 256 x 256 tiles (gemm_pair.cu)
+  int split_width = 0, split_slices = 0;
+  if (gemm_split_plan(c, &split_width, &split_slices)) return launch_gemm_split(c, split_width, split_slices);
   const CUtensorMap* ma = c.a_mn ? get_tensor_map_2d(c.A, Elt::BF16, c.M, c.K, c.lda, 64, 64, true)
                                  : get_tensor_map_2d(c.A, Elt::BF16, c.K, c.M, c.lda, 64, BM, true);
   if (!ma) return 1;

@@ -107,4 +107,9 @@ int run_gemm(const GemmCall& call);
 bool gemm_pair_eligible(const GemmCall& c);
 int launch_gemm_pair(const GemmCall& c);
 
+// Products with too few output tiles to fill the GPU (gemm_split.cu): the K range of a tile cut over the
+// CTAs of a cluster.  The plan is false where the persistent kernel is the better one.
+bool gemm_split_plan(const GemmCall& c, int* width, int* splits);
+int launch_gemm_split(const GemmCall& c, int width, int splits);
+
 }  // namespace ctb

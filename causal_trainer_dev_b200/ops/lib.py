@@ -105,6 +105,10 @@ _SITES = {
     0x0802: "two-CTA gemm mma: operands never arrived",
     0x0803: "two-CTA gemm mma: accumulator never drained",
     0x0804: "two-CTA gemm epilogue: accumulator never completed",
+    0x0901: "split-K gemm producer: stage never freed",
+    0x0902: "split-K gemm mma: operands never arrived",
+    0x0903: "split-K gemm epilogue: accumulator never completed",
+    0x0904: "split-K gemm producer: copy still in flight at teardown",
 }
 
 
