@@ -25,6 +25,10 @@ _f = ctypes.c_float
 _l = ctypes.c_long
 
 
+def _at(t: torch.Tensor | None) -> int | None:
+    return None if t is None else t.data_ptr()
+
+
 # ------------------------------------------------------------------------------ RMSNorm
 def rmsnorm_reference(x: torch.Tensor, w: torch.Tensor, eps: float) -> torch.Tensor:
     xf = x.float()
@@ -39,8 +43,8 @@ def rmsnorm_forward(x, w, eps, residual=None, out=None):
     rstd = torch.empty(rows, dtype=torch.float32, device=x.device)
     h = torch.empty_like(x) if residual is not None else x
     code = _lib.lib().ctb_rmsnorm_fwd(
-        _lib.ptr(x), _lib.ptr(residual), _lib.ptr(w), _lib.ptr(y), _lib.ptr(h if residual is not None else None),
-        _lib.ptr(rstd), rows, d, _f(eps), _lib.stream_ptr(),
+        x.data_ptr(), _at(residual), w.data_ptr(), y.data_ptr(), _at(h if residual is not None else None),
+        rstd.data_ptr(), rows, d, eps, _lib.raw_stream(),
     )
     _lib.check(code, "ctb_rmsnorm_fwd")
     return y, rstd, h
@@ -64,8 +68,8 @@ def rmsnorm_backward(dy, x, w, rstd, dres=None, dw_out=None, dw_accumulate=False
         dw_out = torch.empty(d, dtype=torch.float32, device=x.device)
         dw_accumulate = False
     code = L.ctb_rmsnorm_bwd(
-        _lib.ptr(dy), _lib.ptr(x), _lib.ptr(w), _lib.ptr(rstd), _lib.ptr(dres), _lib.ptr(dx), _lib.ptr(scratch),
-        _lib.ptr(dw_out), int(dw_out.dtype == torch.float32), int(dw_accumulate), rows, d, _lib.stream_ptr(),
+        dy.data_ptr(), x.data_ptr(), w.data_ptr(), rstd.data_ptr(), _at(dres), dx.data_ptr(), scratch.data_ptr(),
+        dw_out.data_ptr(), dw_out.dtype == torch.float32, bool(dw_accumulate), rows, d, _lib.raw_stream(),
     )
     _lib.check(code, "ctb_rmsnorm_bwd")
     return dx, dw_out
@@ -115,8 +119,8 @@ def rope_inplace(x2d: torch.Tensor, cos, sin, heads: int, head_dim: int, rotary_
     t = x2d.shape[0]
     base = x2d[:, col_offset:]
     code = _lib.lib().ctb_rope(
-        _lib.ptr(base), _lib.ptr(cos), _lib.ptr(sin), _l(x2d.stride(0)), t, heads, head_dim, rotary_dim,
-        0 if style == "gpt-j" else 1, int(inverse), _lib.stream_ptr(),
+        base.data_ptr(), cos.data_ptr(), sin.data_ptr(), x2d.stride(0), t, heads, head_dim, rotary_dim,
+        0 if style == "gpt-j" else 1, bool(inverse), _lib.raw_stream(),
     )
     _lib.check(code, "ctb_rope")
 
@@ -131,14 +135,14 @@ def swiglu_reference(gu: torch.Tensor) -> torch.Tensor:
 def swiglu_forward(gu: torch.Tensor) -> torch.Tensor:
     t, f2 = gu.shape
     h = torch.empty((t, f2 // 2), dtype=gu.dtype, device=gu.device)
-    _lib.check(_lib.lib().ctb_swiglu_fwd(_lib.ptr(gu), _lib.ptr(h), _l(t), f2 // 2, _lib.stream_ptr()), "ctb_swiglu_fwd")
+    _lib.check(_lib.lib().ctb_swiglu_fwd(gu.data_ptr(), h.data_ptr(), t, f2 // 2, _lib.raw_stream()), "ctb_swiglu_fwd")
     return h
 
 
 def swiglu_backward(gu: torch.Tensor, dh: torch.Tensor, out: torch.Tensor | None = None) -> torch.Tensor:
     t, f2 = gu.shape
     dgu = torch.empty_like(gu) if out is None else out
-    _lib.check(_lib.lib().ctb_swiglu_bwd(_lib.ptr(gu), _lib.ptr(dh), _lib.ptr(dgu), _l(t), f2 // 2, _lib.stream_ptr()),
+    _lib.check(_lib.lib().ctb_swiglu_bwd(gu.data_ptr(), dh.data_ptr(), dgu.data_ptr(), t, f2 // 2, _lib.raw_stream()),
                "ctb_swiglu_bwd")
     return dgu
 

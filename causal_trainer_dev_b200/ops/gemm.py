@@ -134,10 +134,9 @@ def gemm(
         _lib.check(code, "ctb_gemm_flagged")
         return out
     code = _lib.lib().ctb_gemm(
-        _lib.ptr(a), _lib.ptr(b), _lib.ptr(out), m, n, k,
-        ctypes.c_long(a.stride(0)), ctypes.c_long(b.stride(0)), ctypes.c_long(out.stride(0)),
-        int(a_mn), int(b_mn), int(out.dtype == torch.float32), int(accumulate), ctypes.c_float(alpha),
-        _lib.ptr(bias), max_ctas, _lib.stream_ptr(),
+        a.data_ptr(), b.data_ptr(), out.data_ptr(), m, n, k, a.stride(0), b.stride(0), out.stride(0),
+        a_mn, b_mn, out.dtype == torch.float32, accumulate, alpha, None if bias is None else bias.data_ptr(), max_ctas,
+        _lib.raw_stream(),
     )
     _lib.check(code, "ctb_gemm")
     return out

@@ -14,6 +14,21 @@ import torch
 from .build import LIB_PATH
 
 
+# Argument kinds of the launchers that every layer calls several times (p pointer, i int, l long, f float,
+# q long long): with them ctypes converts plain Python numbers itself, and a call needs no wrapper object per
+# argument.  Launchers that are not listed take wrapped arguments (:func:`ptr` and the ctypes types).
+_KINDS = {"p": ctypes.c_void_p, "i": ctypes.c_int, "l": ctypes.c_long, "f": ctypes.c_float, "q": ctypes.c_longlong}
+_SIGNATURES = {
+    "ctb_gemm": "pppiiillliiiifpip",
+    "ctb_rmsnorm_fwd": "ppppppiifp",
+    "ctb_rmsnorm_bwd": "ppppppppiiiip",
+    "ctb_rope": "pppliiiiiip",
+    "ctb_swiglu_fwd": "pplip",
+    "ctb_swiglu_bwd": "ppplip",
+    "ctb_attn_bwd_stats": "pppppiiiillp",
+}
+
+
 class KernelError(RuntimeError):
     """A launcher refused its arguments, a CUDA call failed, or a bounded wait ran out."""
 
@@ -24,6 +39,8 @@ def _load() -> ctypes.CDLL | None:
         return None
     lib = ctypes.CDLL(str(LIB_PATH))
     lib.ctb_last_error.restype = ctypes.c_char_p
+    for name, kinds in _SIGNATURES.items():
+        getattr(lib, name).argtypes = [_KINDS[k] for k in kinds]
     return lib
 
 
@@ -63,7 +80,13 @@ def check(code: int, what: str) -> None:
 
 
 def stream_ptr() -> ctypes.c_void_p:
-    return ctypes.c_void_p(torch.cuda.current_stream().cuda_stream)
+    return ctypes.c_void_p(raw_stream())
+
+
+def raw_stream() -> int:
+    """Address of the current stream of the current device (``torch.cuda.current_stream()`` builds a
+    Stream object and resolves the device by name on every call: 10 us against 0.3)."""
+    return torch._C._cuda_getCurrentRawStream(torch.cuda.current_device())
 
 
 def ptr(t: torch.Tensor | None) -> ctypes.c_void_p:
