@@ -346,10 +346,11 @@ class LayerwiseEngine:
 
         per_layer = layer_activation_bytes(cfg, tokens)
         free, _ = torch.cuda.mem_get_info()
-        held = torch.cuda.memory_stats_as_nested_dict()       # one look, without memory_stats()'s flattening
-        cached = held["reserved_bytes"]["all"]["current"] - held["allocated_bytes"]["all"]["current"]
         working_set = backward_working_set_bytes(cfg, tokens, self.options.cut_chunk_rows)
-        budget = free + cached - working_set - self.options.memory_reserve_bytes
+        budget = free - working_set - self.options.memory_reserve_bytes
+        if budget < cfg.num_hidden_layers * per_layer:
+            # what the allocator holds without using it counts too (asking takes 0.1 ms: only where it matters)
+            budget += torch.cuda.memory_reserved() - torch.cuda.memory_allocated()
         return max(0, min(cfg.num_hidden_layers, int(budget // per_layer)))
 
     # ------------------------------------------------------------------ step context
