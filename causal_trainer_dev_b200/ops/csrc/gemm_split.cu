@@ -343,6 +343,7 @@ bool gemm_split_plan(const GemmCall& c, int* width, int* splits) {
       c.max_ctas > 0)
     return false;
   if (reinterpret_cast<uintptr_t>(c.C) % 16 != 0) return false;
+  if (c.bias != nullptr && c.out_f32) return false;      // the fp32 store of the persistent kernel takes no bias
   const long num_m = (c.M + 127) / 128, num_k = (c.K + 63) / 64, sms = sm_count();
   const long tiles = num_m * ((c.N + 255) / 256);
   if (tiles > sms) return false;
