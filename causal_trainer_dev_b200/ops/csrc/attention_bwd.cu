@@ -595,7 +595,12 @@ attn_bwd_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constant
         const int oh = DKV ? hkv : head;
         const int ob = DKV ? kbatch : b;
 #pragma unroll
-        for (int hf = 0; hf < HALVES; ++hf) tma_store_4d(mo, stage_buf + hf * 16384, hf * 64, oh, x0, ob);
+        for (int hf = 0; hf < HALVES; ++hf) {
+          // grouped dK / dV: the history part joins what the own-block pass stored (one CTA per tile, so the sum
+          // does not depend on timing)
+          if (DKV && grouped) tma_reduce_add_4d(mo, stage_buf + hf * 16384, hf * 64, oh, x0, ob);
+          else tma_store_4d(mo, stage_buf + hf * 16384, hf * 64, oh, x0, ob);
+        }
         tma_commit_group();
         tma_wait_group<0>();
       }
@@ -746,8 +751,8 @@ CTB_API int ctb_attn_bwd_sparse(int mode, const void* q, const void* k, const vo
 }
 
 // Grouped MoBA backward (see GroupArgs).  mode 0 (dK/dV): one CTA per (group, 128-key tile), `ctas`
-// descriptors; dk / dv are [B,S,Hkv,D] views that receive the history part (tiles of groups without
-// rows are not written: clear the buffers first).  mode 1 (dQ): one CTA per 128 gathered rows,
+// descriptors; dk / dv are [B,S,Hkv,D] views that hold the own-block gradients, and the history part is
+// added to them (tiles of groups without rows are left alone).  mode 1 (dQ): one CTA per 128 gathered rows,
 // gathered_rows / 128 descriptors; dqg is [gathered_rows, D].  qg / dog / the statistics are the
 // gathered rows ([gathered_rows, D] contiguous, [gathered_rows] fp32, padding rows zero).
 CTB_API int ctb_attn_bwd_grouped(int mode, const void* qg, const void* k, const void* v, const void* dog, void* dqg,

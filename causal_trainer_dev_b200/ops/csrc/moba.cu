@@ -144,6 +144,80 @@ moba_route_kernel(const __nv_bfloat16* __restrict__ q, long q_row_stride, const 
   }
 }
 
+// The same for top_k <= 9: a warp routes four consecutive tokens of one head, eight lanes each, lane r of the
+// eight holding the r-th best block.  A warp per token spent most of its instructions on 32-lane shuffles for
+// a reduction of 128 products and a list of three (32768 tokens, 32 heads, 8 blocks: 585 us; reading q takes
+// 40).  Lane j holds the channels that lanes j, j + 8, j + 16 and j + 24 hold above and adds them up in the
+// same order, so the scores and with them the routing are the same bit for bit.
+template <int D>
+__global__ void __launch_bounds__(256)
+moba_route4_kernel(const __nv_bfloat16* __restrict__ q, long q_row_stride, const float* __restrict__ pooled,
+                   const int* __restrict__ pool_start, const int* __restrict__ seg,
+                   const int* __restrict__ doc_start, int B, int S, int Hq, int Hkv, int block, int top_k, int words,
+                   unsigned* __restrict__ sel) {
+  const long warp_id = (blockIdx.x * static_cast<long>(blockDim.x) + threadIdx.x) >> 5;
+  const int lane = threadIdx.x & 31, j = lane & 7, g = lane >> 3;
+  if (warp_id >= static_cast<long>(B) * (S / 4) * Hq) return;
+  const int h = static_cast<int>(warp_id % Hq);
+  const long t = warp_id / Hq * 4 + g;               // S is a multiple of 128: the four tokens share their row
+  const int b = static_cast<int>(t / S), i = static_cast<int>(t % S);
+  const bool live = seg[t] != 0;
+  const int start = doc_start[t];
+  const int cur = live ? (i - start) / block : 0;
+  const int hkv = h / (Hq / Hkv), ntile = S / 128;
+  constexpr int PER = D / 32;
+  float qv[4][PER];
+  const __nv_bfloat16* qp = q + t * q_row_stride + static_cast<long>(h) * D + j * PER;
+#pragma unroll
+  for (int r = 0; r < 4; ++r)
+#pragma unroll
+    for (int e = 0; e < PER; e += 2) {
+      const float2 f = __bfloat1622float2(*reinterpret_cast<const __nv_bfloat162*>(qp + r * 8 * PER + e));
+      qv[r][e] = f.x;
+      qv[r][e + 1] = f.y;
+    }
+  float held = -INFINITY;
+  int held_id = -1;
+  const int keep = top_k - 1;
+  const int most = __reduce_max_sync(0xffffffffu, cur);
+  for (int c = 0; c < most && keep > 0; ++c) {
+    float part[4] = {0.f, 0.f, 0.f, 0.f};
+    const int p = start + c * block, tile = p >> 7;
+    if (c < cur && pool_start[b * ntile + tile] == p) {
+      const float* pk = pooled + ((static_cast<size_t>(b) * ntile + tile) * Hkv + hkv) * D + j * PER;
+#pragma unroll
+      for (int r = 0; r < 4; ++r)
+#pragma unroll
+        for (int e = 0; e < PER; ++e) part[r] += qv[r][e] * pk[r * 8 * PER + e];
+    }
+    float s = (part[0] + part[2]) + (part[1] + part[3]);
+#pragma unroll
+    for (int o = 4; o > 0; o >>= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
+    const unsigned ahead = __ballot_sync(0xffffffffu, j < keep && held >= s);
+    const int pos = __popc((ahead >> (8 * g)) & 0xffu);
+    const float up = __shfl_up_sync(0xffffffffu, held, 1, 8);
+    const int up_id = __shfl_up_sync(0xffffffffu, held_id, 1, 8);
+    if (c < cur) {
+      if (j > pos) {
+        held = up;
+        held_id = up_id;
+      } else if (j == pos) {
+        held = s;
+        held_id = c;
+      }
+    }
+  }
+  unsigned* out = sel + ((static_cast<size_t>(b) * Hq + h) * S + i) * words;
+  for (int w = 0; w < words; ++w) {
+    unsigned bits = 0u;
+    if (j < keep && held_id >= 0 && (held_id >> 5) == w) bits = 1u << (held_id & 31);
+#pragma unroll
+    for (int o = 4; o > 0; o >>= 1) bits |= __shfl_xor_sync(0xffffffffu, bits, o);
+    if (live && (cur >> 5) == w) bits |= 1u << (cur & 31);
+    if (j == 0) out[w] = bits;
+  }
+}
+
 }  // namespace moba
 }  // namespace ctb
 
@@ -179,6 +253,16 @@ CTB_API int ctb_moba_route(const void* q, long q_row_stride, const float* pooled
   const long blocks = (warps * 32 + 255) / 256;
   cudaStream_t s = static_cast<cudaStream_t>(stream);
   const __nv_bfloat16* qp = static_cast<const __nv_bfloat16*>(q);
+  // eight lanes hold the list of kept blocks; rows of 4-byte aligned channel pairs, four tokens of one row a warp
+  if (top_k <= 9 && (D == 128 || D == 64) && S % 4 == 0 && q_row_stride % 2 == 0 &&
+      reinterpret_cast<uintptr_t>(q) % 4 == 0) {
+    const long quads = static_cast<long>(B) * (S / 4) * Hq;
+    auto kern = D == 128 ? moba::moba_route4_kernel<128> : moba::moba_route4_kernel<64>;
+    kern<<<static_cast<unsigned>((quads * 32 + 255) / 256), 256, 0, s>>>(qp, q_row_stride, pooled, pool_start, seg,
+                                                                        doc_start, B, S, Hq, Hkv, block, top_k, words, sel);
+    CTB_CUDA_OK(cudaGetLastError());
+    return 0;
+  }
   if (D == 128)
     moba::moba_route_kernel<128><<<static_cast<unsigned>(blocks), 256, 0, s>>>(
         qp, q_row_stride, pooled, pool_start, seg, doc_start, B, S, Hq, Hkv, block, top_k, words, sel);

@@ -381,7 +381,7 @@ def moba_grouped_backward(q, k, v, out, dout, lse, meta: AttentionMeta, groups: 
     """Backward of :func:`moba_grouped_forward`.  Every pass uses the statistics of the merged
     softmax (total LSE, ``delta = sum O dO``), so the partial gradients simply add: own-block dQ / dK
     / dV from the dense kernels, history dQ per gathered row (scattered back and added), history
-    dK / dV per key block over its group's rows (grouped_moba.py:177-272)."""
+    dK / dV per key block over its group's rows, added in place by the kernel (grouped_moba.py:177-272)."""
     from .attention import flash_attention_backward
 
     b, s, hq, d = q.shape
@@ -393,21 +393,17 @@ def moba_grouped_backward(q, k, v, out, dout, lse, meta: AttentionMeta, groups: 
     qg, _, _ = _gather(groups, q, None, s, hq, d)
     dog, lse_g, delta_g = _gather(groups, dout, stats, s, hq, d)
     dqg = torch.empty_like(qg)
-    dkh = torch.zeros((b, s, hkv, d), dtype=torch.bfloat16, device=q.device)
-    dvh = torch.zeros_like(dkh)
     L = _lib.lib()
     for mode, desc in ((0, groups.dkv_desc), (1, groups.dq_desc)):
         code = L.ctb_attn_bwd_grouped(
-            mode, _lib.ptr(qg), _lib.ptr(k), _lib.ptr(v), _lib.ptr(dog), _lib.ptr(dqg), _lib.ptr(dkh), _lib.ptr(dvh),
+            mode, _lib.ptr(qg), _lib.ptr(k), _lib.ptr(v), _lib.ptr(dog), _lib.ptr(dqg), _lib.ptr(dk), _lib.ptr(dv),
             _lib.ptr(lse_g), _lib.ptr(delta_g), _lib.ptr(desc), desc.shape[0], groups.rows_cap, groups.block, b, s, hkv,
-            d, ctypes.c_long(_row_stride(k)), ctypes.c_long(_row_stride(v)), ctypes.c_long(_row_stride(dkh)),
-            ctypes.c_long(_row_stride(dvh)), ctypes.c_float(scale), ctypes.c_longlong(spin_budget), _lib.stream_ptr())
+            d, ctypes.c_long(_row_stride(k)), ctypes.c_long(_row_stride(v)), ctypes.c_long(_row_stride(dk)),
+            ctypes.c_long(_row_stride(dv)), ctypes.c_float(scale), ctypes.c_longlong(spin_budget), _lib.stream_ptr())
         _lib.check(code, "ctb_attn_bwd_grouped")
     code = L.ctb_moba_merge_dq(_lib.ptr(dq), ctypes.c_long(_row_stride(dq)), _lib.ptr(dqg), _lib.ptr(groups.pos_of), b, s,
                                hq, d, groups.picks, _lib.stream_ptr())
     _lib.check(code, "ctb_moba_merge_dq")
-    dk.add_(dkh)
-    dv.add_(dvh)
     return dq, dk, dv
 
 
