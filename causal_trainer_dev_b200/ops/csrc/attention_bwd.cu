@@ -199,6 +199,19 @@ attn_bwd_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constant
     mbar_init(acc_full, 1);
     *abort_flag = 0u;
     mbar_fence_init();
+    if (n_iter > 0) {
+      // the resident tiles are on their way while TMEM is allocated
+      mbar_expect_tx(x_full, 2 * L::XT);
+      const CUtensorMap* mx1 = DKV ? &map_k : &map_q;
+      const CUtensorMap* mx2 = DKV ? &map_v : &map_do;
+      const int xh = DKV ? hkv : head;
+      const int xb = DKV ? kbatch : b;
+#pragma unroll
+      for (int hf = 0; hf < HALVES; ++hf) {
+        tma_load_4d(smem + L::OFF_X + hf * 16384, mx1, x_full, hf * 64, xh, x0, xb);
+        tma_load_4d(smem + L::OFF_X + L::XT + hf * 16384, mx2, x_full, hf * 64, xh, x0, xb);
+      }
+    }
   }
   if (warp == 1) {
     tmem_alloc(tmem_slot, 512);
@@ -218,16 +231,6 @@ attn_bwd_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constant
     // ------------------------------ producer ------------------------------
     if (n_iter > 0) {
       const uint32_t on = elect_one();            // the whole warp walks, one lane issues
-      mbar_expect_tx_if(on, x_full, 2 * L::XT);
-      const CUtensorMap* mx1 = DKV ? &map_k : &map_q;
-      const CUtensorMap* mx2 = DKV ? &map_v : &map_do;
-      const int xh = DKV ? hkv : head;
-      const int xb = DKV ? kbatch : b;
-#pragma unroll
-      for (int hf = 0; hf < HALVES; ++hf) {
-        tma_load_4d_if(on, smem + L::OFF_X + hf * 16384, mx1, x_full, hf * 64, xh, x0, xb);
-        tma_load_4d_if(on, smem + L::OFF_X + L::XT + hf * 16384, mx2, x_full, hf * 64, xh, x0, xb);
-      }
       const CUtensorMap* my1 = DKV ? &map_q : &map_k;
       const CUtensorMap* my2 = DKV ? &map_do : &map_v;
       uint32_t slot1 = 0, phase1 = 0;

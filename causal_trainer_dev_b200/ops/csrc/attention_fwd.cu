@@ -164,6 +164,17 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constant
     }
     *abort_flag = 0u;
     mbar_fence_init();
+    if (nmax > 0) {
+      // Q is on its way while TMEM is allocated.  A tile without keys has no use for it, and its warps stage
+      // zeros for O in that place at once
+      mbar_expect_tx(q_full, ((n0 > 0 ? 1u : 0u) + (n1 > 0 ? 1u : 0u)) * L::QT);
+      for (int t = 0; t < 2; ++t) {
+        if ((t == 0 ? n0 : n1) == 0) continue;
+#pragma unroll
+        for (int hf = 0; hf < HALVES; ++hf)
+          tma_load_4d(smem + L::OFF_Q + t * L::QT + hf * 16384, &map_q, q_full, hf * 64, h, q0 + t * 128, b);
+      }
+    }
   }
   if (warp == 1) {
     tmem_alloc(tmem_slot, 512);
@@ -184,18 +195,6 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constant
     // ------------------------------ producer ------------------------------
     if (nmax > 0) {
       const uint32_t on = elect_one();            // the whole warp walks, one lane issues
-      uint32_t bytes = 0;
-      // a tile without keys has no use for Q, and its warps stage zeros for O in that place at once
-      const int n_t[2] = {n0, n1};
-      for (int t = 0; t < 2; ++t)
-        if (n_t[t] > 0) bytes += L::QT;
-      mbar_expect_tx_if(on, q_full, bytes);
-      for (int t = 0; t < 2; ++t) {
-        if (n_t[t] == 0) continue;
-#pragma unroll
-        for (int hf = 0; hf < HALVES; ++hf)
-          tma_load_4d_if(on, smem + L::OFF_Q + t * L::QT + hf * 16384, &map_q, q_full, hf * 64, h, q0 + t * 128, b);
-      }
       uint32_t slot = 0, phase = 0;
       bool ok = true;
       for (int i = 0; ok && i < nmax; ++i) {
