@@ -93,10 +93,11 @@ __device__ __forceinline__ bool mbar_wait(uint64_t* bar, uint32_t parity, volati
 // One issuing lane of a converged warp
 // ---------------------------------------------------------------------------------------
 // The single-thread instructions (tcgen05.mma, its commit, TMA copies) take their operands from uniform
-// registers.  Inside an `if (lane == 0)` the compiler has to move every operand there one by one: 134
-// cycles per MMA, whatever its shape, measured on B200, where a 128 x 128 x 16 product takes 64.  So the
-// whole warp walks the loop with warp-uniform values and only the instruction itself is predicated with
-// the lane that elect_one() chose: the *_if functions below.
+// registers.  Inside an `if (lane == 0)` the compiler cannot keep loop-dependent operands there and moves
+// them one by one: 134 cycles per MMA, whatever its shape, in a loop that chose its operands at run time,
+// where a 128 x 128 x 16 product takes 65 with constant ones; four boxes of a 32 KB tile took 426 cycles to
+// issue from one lane and 264 this way.  So the whole warp walks the loop with warp-uniform values and
+// only the instruction itself is predicated with the lane that elect_one() chose: the *_if functions below.
 __device__ __forceinline__ uint32_t elect_one() {
   uint32_t on;
   asm volatile(
