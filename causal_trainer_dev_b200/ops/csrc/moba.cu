@@ -58,6 +58,7 @@ moba_pool_kernel(const __nv_bfloat16* __restrict__ k, long k_row_stride, const i
 #pragma unroll
   for (int e = 0; e < 8; ++e) acc[e] = 0.f;
   const __nv_bfloat16* base = k + (static_cast<size_t>(b) * S + p) * k_row_stride + static_cast<size_t>(hkv) * D + v * 8;
+#pragma unroll 16                                // (64 CTAs with work at 32768 tokens: loads in flight are what counts)
   for (int r = rg; r < block; r += ROWS) {
     const uint4 raw = *reinterpret_cast<const uint4*>(base + static_cast<size_t>(r) * k_row_stride);
     const __nv_bfloat162* h2 = reinterpret_cast<const __nv_bfloat162*>(&raw);
@@ -447,9 +448,10 @@ CTB_API int ctb_moba_lists(int mode, const unsigned* touch, int B, int S, int Hq
 //
 //   moba_rank    gives every row that selected block c of its document its rank among such rows of
 //                the same (document, head) and leaves the count in cnt[group][head in group]:
-//                moba_rank_scan_kernel, one CTA per (batch, head, c), a segmented scan over the
-//                sequence (default); moba_rank_kernel, one warp per (batch, head, c) walking the
-//                sequence (CTB_MOBA_RANK=walk; same result, kept for comparison).
+//                moba_rank_bits_kernel, one CTA per (batch, head, c), from a bit per token (rows of up
+//                to 192512 tokens); moba_rank_scan_kernel, a segmented scan over the sequence (longer
+//                rows); moba_rank_kernel, one warp per (batch, head, c) walking the sequence
+//                (CTB_MOBA_RANK=walk; same result, kept for comparison).
 //   moba_groups  one CTA: exclusive scan of the padded group sizes -> first row of every group,
 //                offsets of the heads inside a group, the compact list of non-empty groups.
 //   moba_desc    descriptors of the CTAs of the grouped flash kernels.
@@ -504,6 +506,85 @@ moba_rank_kernel(const unsigned* __restrict__ sel, const int* __restrict__ seg, 
     const int add = __popc(last_mates);
     carry_count = (last_start == carry_start ? carry_count : 0) + add;
     carry_start = last_start;
+  }
+}
+
+// The same ranks by one CTA per (batch, head, block index) from a bit per token: the tokens of a document are
+// adjacent, so the rank of a picked row is the number of picks before it in the sequence less the number
+// before its document, two look-ups in a prefix sum over 32-token words.  Every load is coalesced and the
+// words stay in shared memory (S / 4 bytes); with a contiguous span per thread and a segmented scan, as
+// below, 32768 tokens, 32 heads and 8 blocks took 255-307 us of strided loads.
+constexpr int RANK_MAX_SEQ = 47 * 1024 * 4;         // beside the 128 static bytes within 48 KB
+__global__ void __launch_bounds__(1024)
+moba_rank_bits_kernel(const unsigned* __restrict__ sel, const int* __restrict__ seg, const int* __restrict__ doc_start,
+                      int S, int Hq, int Hkv, int block, int words, int nblk, int picks, int* __restrict__ rank,
+                      int* __restrict__ cnt) {
+  extern __shared__ unsigned rank_smem[];
+  __shared__ int s_warp[32];
+  const int chunks = S / 32;
+  unsigned* bits = rank_smem;                            // [chunks] picked rows of 32 tokens
+  int* before = reinterpret_cast<int*>(rank_smem + chunks);   // [chunks] picks left of the chunk
+  const int c = static_cast<int>(blockIdx.x % nblk);
+  const int h = static_cast<int>((blockIdx.x / nblk) % Hq);
+  const int b = static_cast<int>(blockIdx.x / nblk / Hq);
+  const int gsize = Hq / Hkv, hkv = h / gsize, hg = h % gsize, nt128 = S / 128;
+  const int word = c >> 5;
+  const unsigned below = (1u << (c & 31)) - 1u;
+  const int t = threadIdx.x, lane = t & 31, warp = t >> 5;
+  const size_t row_base = (static_cast<size_t>(b) * Hq + h) * S;
+  for (int k = warp; k < chunks; k += 32) {
+    const int i = k * 32 + lane;
+    const int st = doc_start[b * S + i];
+    const unsigned w = word < words ? __ldg(sel + (row_base + i) * words + word) : 0u;
+    const bool picked = seg[b * S + i] != 0 && ((w >> (c & 31)) & 1u) && c < (i - st) / block;
+    const unsigned m = __ballot_sync(0xffffffffu, picked);
+    if (lane == 0) bits[k] = m;
+  }
+  __syncthreads();
+  // exclusive prefix sum over the chunks, a contiguous stretch per thread
+  const int per = (chunks + 1023) / 1024, k0 = min(chunks, t * per), k1 = min(chunks, k0 + per);
+  int mine = 0;
+  for (int k = k0; k < k1; ++k) mine += __popc(bits[k]);
+  int incl = mine;
+#pragma unroll
+  for (int d = 1; d < 32; d <<= 1) {
+    const int up = __shfl_up_sync(0xffffffffu, incl, d);
+    if (lane >= d) incl += up;
+  }
+  if (lane == 31) s_warp[warp] = incl;
+  __syncthreads();
+  if (warp == 0) {
+    int v = s_warp[lane];
+#pragma unroll
+    for (int d = 1; d < 32; d <<= 1) {
+      const int up = __shfl_up_sync(0xffffffffu, v, d);
+      if (lane >= d) v += up;
+    }
+    s_warp[lane] = v;
+  }
+  __syncthreads();
+  int run = incl - mine + (warp > 0 ? s_warp[warp - 1] : 0);
+  for (int k = k0; k < k1; ++k) {
+    before[k] = run;
+    run += __popc(bits[k]);
+  }
+  __syncthreads();
+  for (int k = warp; k < chunks; k += 32) {
+    const unsigned m = bits[k];
+    if (m == 0u) continue;                               // (the same for the whole warp)
+    const int i = k * 32 + lane;
+    const bool picked = (m >> lane) & 1u;
+    const int st = picked ? doc_start[b * S + i] : -1;
+    const unsigned mates = __match_any_sync(0xffffffffu, st);
+    if (!picked) continue;
+    const int doc = before[st >> 5] + __popc(bits[st >> 5] & ((1u << (st & 31)) - 1u));
+    const int r = before[k] + __popc(m & ((1u << lane) - 1u)) - doc;
+    const unsigned* mine_sel = sel + (row_base + i) * words;
+    int j = __popc(__ldg(mine_sel + word) & below);      // earlier picks of this row: its slot for block c
+    for (int x = 0; x < word; ++x) j += __popc(__ldg(mine_sel + x));
+    if (j < picks) rank[(row_base + i) * picks + j] = r;
+    if ((mates >> lane) == 1u)                           // last picked row of its document in the chunk
+      atomicMax(cnt + ((b * Hkv + hkv) * nt128 + ((st + c * block) >> 7)) * gsize + hg, r + 1);
   }
 }
 
@@ -956,6 +1037,9 @@ CTB_API int ctb_moba_group(const unsigned* sel, const int* seg, const int* doc_s
   if (walk || warps > 0x7fffffffL)
     moba::moba_rank_kernel<<<static_cast<unsigned>((warps * 32 + 255) / 256), 256, 0, s>>>(
         sel, seg, doc_start, B, S, Hq, Hkv, block, words, nblk, picks, rank, cnt);
+  else if (S <= moba::RANK_MAX_SEQ)                      // its words and counts fit into 48 KB
+    moba::moba_rank_bits_kernel<<<static_cast<unsigned>(warps), 1024, S / 4, s>>>(
+        sel, seg, doc_start, S, Hq, Hkv, block, words, nblk, picks, rank, cnt);
   else
     moba::moba_rank_scan_kernel<<<static_cast<unsigned>(warps), 1024, 0, s>>>(
         sel, seg, doc_start, B, S, Hq, Hkv, block, words, nblk, picks, rank, cnt);
