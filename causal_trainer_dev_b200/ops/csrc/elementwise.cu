@@ -251,6 +251,40 @@ rmsnorm_dw_reduce_kernel(const float* __restrict__ partial, int parts, int d, vo
   }
 }
 
+// Column sums of a bf16 matrix (the gradient of a projection's bias) into per-CTA partial rows, which
+// rmsnorm_dw_reduce_kernel adds up.  Bound by reading the matrix once: a warp reads 512 bytes of a row, eight
+// rows a CTA and four in flight a warp; the cast to fp32 and the strided sum that did this wrote and read
+// twice the matrix in between.
+__global__ void __launch_bounds__(256)
+column_sum_kernel(const __nv_bfloat16* __restrict__ x, long ld, int rows, int n, float* __restrict__ partial) {
+  __shared__ float sums[8][256 + 8];
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  const int c = blockIdx.x * 256 + lane * 8;
+  const bool live = c < n;
+  const int step = gridDim.y * 8;
+  float acc[8] = {0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f};
+  if (live) {
+#pragma unroll 4
+    for (int r = blockIdx.y * 8 + warp; r < rows; r += step) {
+      float f[8];
+      unpack8(__ldg(reinterpret_cast<const uint4*>(x + static_cast<long>(r) * ld + c)), f);
+#pragma unroll
+      for (int e = 0; e < 8; ++e) acc[e] += f[e];
+    }
+  }
+#pragma unroll
+  for (int e = 0; e < 8; ++e) sums[warp][e * 33 + lane] = acc[e];
+  __syncthreads();
+  // thread t: column t of the block's 256
+  const int col = blockIdx.x * 256 + threadIdx.x;
+  if (col >= n) return;
+  const int at = (threadIdx.x & 7) * 33 + (threadIdx.x >> 3);
+  float t = 0.f;
+#pragma unroll
+  for (int w = 0; w < 8; ++w) t += sums[w][at];
+  partial[static_cast<size_t>(blockIdx.y) * n + col] = t;
+}
+
 // ------------------------------------------------------------------------------------------
 // RoPE, in place on `heads` consecutive heads of a packed projection row.
 //   x: [T][row_stride] with head h at columns h*D..h*D+D-1; cos/sin: [T][rot/2] fp32.
@@ -999,6 +1033,27 @@ CTB_API int ctb_rmsnorm_bwd(const void* dy, const void* x, const void* w, const 
     rmsnorm_dw_reduce_kernel<<<(d + 31) / 32, DW_WARPS * 32, 0, s>>>(dw_partial, parts, d, dw, dw_f32, dw_accumulate);
     CTB_CUDA_OK(cudaGetLastError());
   }
+  return 0;
+}
+
+// Rows of partial sums that ctb_column_sum writes for a matrix of `rows` rows and `n` columns.
+CTB_API int ctb_column_sum_parts(int rows, int n) {
+  const int cols = (n + 255) / 256;
+  const int want = (sm_count() * 4 + cols - 1) / cols, most = (rows + 31) / 32;
+  return want < most ? want : (most < 1 ? 1 : most);
+}
+// out[c] (+)= sum over rows of x[r][c]; n and ld multiples of 8 elements, x 16-byte aligned; partial holds
+// ctb_column_sum_parts(rows, n) * n floats.
+CTB_API int ctb_column_sum(const void* x, long ld, int rows, int n, float* partial, void* out, int out_f32, int accumulate,
+                           void* stream) {
+  if (n % 8 || ld % 8 || reinterpret_cast<uintptr_t>(x) % 16) return fail("column_sum: rows must be whole 16-byte vectors");
+  if (n <= 0) return 0;
+  cudaStream_t s = static_cast<cudaStream_t>(stream);
+  const int parts = ctb_column_sum_parts(rows, n);
+  column_sum_kernel<<<dim3((n + 255) / 256, parts), 256, 0, s>>>(static_cast<const __nv_bfloat16*>(x), ld, rows, n, partial);
+  CTB_CUDA_OK(cudaGetLastError());
+  rmsnorm_dw_reduce_kernel<<<(n + 31) / 32, DW_WARPS * 32, 0, s>>>(partial, parts, n, out, out_f32, accumulate);
+  CTB_CUDA_OK(cudaGetLastError());
   return 0;
 }
 

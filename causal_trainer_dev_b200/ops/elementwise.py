@@ -75,6 +75,17 @@ def rmsnorm_backward(dy, x, w, rstd, dres=None, dw_out=None, dw_accumulate=False
     return dx, dw_out
 
 
+def column_sum(x: torch.Tensor, out: torch.Tensor, accumulate: bool = False) -> None:
+    """``out (+)= x.sum(0)`` for a bf16 matrix with unit inner stride (fp32 sums, rounded once to ``out``'s
+    dtype, bf16 or fp32): the gradient of a projection's bias."""
+    rows, n = x.shape
+    L = _lib.lib()
+    partial = torch.empty(L.ctb_column_sum_parts(rows, n) * n, dtype=torch.float32, device=x.device)
+    code = L.ctb_column_sum(_lib.ptr(x), _l(x.stride(0)), rows, n, _lib.ptr(partial), _lib.ptr(out),
+                            int(out.dtype == torch.float32), int(accumulate), _lib.stream_ptr())
+    _lib.check(code, "ctb_column_sum")
+
+
 # ------------------------------------------------------------------------------ RoPE
 def inverse_frequencies(rotary_dim: int, theta: float, device=None) -> torch.Tensor:
     channels = torch.arange(0, rotary_dim, 2, dtype=torch.float32, device=device)

@@ -169,11 +169,7 @@ class LayerwiseEngine:
     def _bias_grad(self, dy: torch.Tensor, gview: torch.Tensor | None, accumulate: bool) -> None:
         if gview is None:
             return
-        s = dy.float().sum(0)
-        if accumulate:
-            gview.add_(s.to(gview.dtype))
-        else:
-            gview.copy_(s.to(gview.dtype))
+        ew.column_sum(dy, gview, accumulate)
         self._count(2)
 
     # ------------------------------------------------------------------ attention (dense or MoBA)

@@ -138,6 +138,20 @@ def test_sum_of_squares_tails_and_alignment(cuda_lib, dtype, n, offset):
         assert abs(float(E.sum_of_squares(x, round_bf16=True)) / float(rounded) - 1) < 1e-5
 
 
+@pytest.mark.parametrize("rows,n", [(1, 8), (7, 264), (1000, 2048), (5000, 72)])
+@pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float32])
+def test_column_sums(cuda_lib, rows, n, dtype):
+    from causal_trainer_dev_b200.ops import elementwise as E
+
+    x = _bf16(rows, n + 8, seed=1)[:, :n]
+    first = _bf16(n, seed=2).to(dtype)
+    for accumulate in (False, True):
+        out = first.clone()
+        E.column_sum(x, out, accumulate)
+        want = x.double().sum(0) + (first.double() if accumulate else 0)
+        assert _rel(out, want) < (BF16 if dtype == torch.bfloat16 else 1e-5)
+
+
 @pytest.mark.parametrize("rows", [1, 31, 33, 300])
 @pytest.mark.parametrize("vocab", [128, 2056, 16400])
 def test_cross_entropy_statistics_over_slabs(cuda_lib, rows, vocab):
