@@ -44,7 +44,7 @@ def rmsnorm_forward(x, w, eps, residual=None, out=None):
     h = torch.empty_like(x) if residual is not None else x
     code = _lib.lib().ctb_rmsnorm_fwd(
         x.data_ptr(), _at(residual), w.data_ptr(), y.data_ptr(), _at(h if residual is not None else None),
-        rstd.data_ptr(), rows, d, eps, _lib.raw_stream(),
+        rstd.data_ptr(), rows, d, float(eps), _lib.raw_stream(),
     )
     _lib.check(code, "ctb_rmsnorm_fwd")
     return y, rstd, h

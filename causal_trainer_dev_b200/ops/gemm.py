@@ -135,8 +135,8 @@ def gemm(
         return out
     code = _lib.lib().ctb_gemm(
         a.data_ptr(), b.data_ptr(), out.data_ptr(), m, n, k, a.stride(0), b.stride(0), out.stride(0),
-        a_mn, b_mn, out.dtype == torch.float32, accumulate, alpha, None if bias is None else bias.data_ptr(), max_ctas,
-        _lib.raw_stream(),
+        bool(a_mn), bool(b_mn), out.dtype == torch.float32, bool(accumulate), float(alpha),
+        None if bias is None else bias.data_ptr(), max_ctas, _lib.raw_stream(),
     )
     _lib.check(code, "ctb_gemm")
     return out
