@@ -389,9 +389,10 @@ __global__ void rope_table_kernel(const int* __restrict__ pos, const float* __re
 // Backward writes d(gate|up) in the same packed layout.
 // ------------------------------------------------------------------------------------------
 // A thread keeps its column vector and walks the rows (blockIdx.y, two at a time), so there is no
-// division per vector; the quotient of the sigmoid is the fast one (2 ulp, the result is rounded to
-// bf16): with the IEEE division the forward kernel was bound by instructions, 345 us for the 1.41 GB
-// of 16384 x 14336, not by memory.
+// division per vector.  The quotient of the sigmoid is the correctly rounded one: the fast division takes
+// 246 us where this takes 325 (forward, 16384 x 14336; 339 with a division per vector as well; backward 398 and
+// 408), but returns zero for denominators above 2^126, i.e. for gates between -88.7 and -87.4.  So the forward
+// kernel is bound by the instructions of that division (1.41 GB at 4.3 TB/s), the backward one by memory.
 constexpr int SWIGLU_ROWS = 2;
 __global__ void __launch_bounds__(256)
 swiglu_fwd_kernel(const __nv_bfloat16* __restrict__ gu, __nv_bfloat16* __restrict__ h, long T, int f) {
@@ -415,7 +416,7 @@ swiglu_fwd_kernel(const __nv_bfloat16* __restrict__ gu, __nv_bfloat16* __restric
         unpack8(uv[k], u);
 #pragma unroll
         for (int e = 0; e < 8; ++e) {
-          const float act = __bfloat162float(__float2bfloat16(__fdividef(g[e], 1.f + __expf(-g[e]))));
+          const float act = __bfloat162float(__float2bfloat16(g[e] / (1.f + __expf(-g[e]))));
           o[e] = act * u[e];
         }
         reinterpret_cast<uint4*>(h)[static_cast<size_t>(t0 + k) * nvec + v] = pack8(o);
@@ -447,7 +448,7 @@ swiglu_bwd_kernel(const __nv_bfloat16* __restrict__ gu, const __nv_bfloat16* __r
         unpack8(dv[k], d);
 #pragma unroll
         for (int e = 0; e < 8; ++e) {
-          const float sg = __fdividef(1.f, 1.f + __expf(-g[e]));
+          const float sg = 1.f / (1.f + __expf(-g[e]));
           const float act = g[e] * sg;
           du[e] = d[e] * act;
           dg[e] = d[e] * u[e] * sg * (1.f + g[e] * (1.f - sg));

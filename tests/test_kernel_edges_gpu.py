@@ -125,6 +125,25 @@ def test_swiglu_ragged(cuda_lib, rows, f):
     assert _rel(E.swiglu_backward(gu, dh), gd.grad) < BF16
 
 
+def test_swiglu_of_large_negative_gates(cuda_lib):
+    """Every bf16 gate from -88.5 to -64 has a result that bf16 can hold, also where 1 + exp(-gate) is above
+    2^126.  (Below -88.7 exp(-gate) is infinite in fp32 and the result zero.)"""
+    from causal_trainer_dev_b200.ops import elementwise as E
+
+    gate = -torch.arange(64, 89, 0.5).bfloat16()
+    gate = torch.cat([gate, gate.new_zeros(-gate.numel() % 8)]).cuda()
+    up, dh = torch.full_like(gate, 3.0), torch.full_like(gate, 0.5)
+    gd, ud = gate.double().requires_grad_(), up.double().requires_grad_()
+    want = torch.nn.functional.silu(gd) * ud
+    want.backward(dh.double())
+    gu = torch.cat([gate, up])[None]
+    # element by element; __expf is off by up to 2 + 1.2 |x| units in the last place of fp32: 1.3e-5 at 88
+    near = lambda got, ref, roundings: bool(((got.double() - ref).abs() <= (roundings * BF16 + 2e-5) * ref.abs()).all())  # noqa: E731
+    assert near(E.swiglu_forward(gu)[0], want.detach(), 2)                    # silu is rounded before the product
+    dgate, dup = E.swiglu_backward(gu, dh[None])[0].chunk(2)
+    assert near(dgate, gd.grad, 1) and near(dup, ud.grad, 1)
+
+
 @pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float32])
 @pytest.mark.parametrize("n,offset", [(1, 0), (7, 0), (4099, 0), (4099, 1), (1 << 20, 0), ((1 << 20) + 5, 3)])
 def test_sum_of_squares_tails_and_alignment(cuda_lib, dtype, n, offset):
