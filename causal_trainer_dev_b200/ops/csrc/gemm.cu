@@ -685,6 +685,25 @@ inline int& tail_split_mode() {
   return mode;
 }
 
+// Dynamic tile claiming measured slightly slower than the static walk on B200 (0-4 % on the
+// projection shapes, alone and under communication), so it is opt-in.
+inline bool dynamic_tiles_mode() {
+  static const bool on = [] {
+    const char* e = std::getenv("CTB_GEMM_DYNAMIC_TILES");
+    return e != nullptr && e[0] == '1';
+  }();
+  return on;
+}
+
+// 1 or 2: CTB_GEMM_TM forces the 128 x 256 or the 256 x 256 tile; 0: chosen by size.
+inline int forced_tile_mode() {
+  static const int tm = [] {
+    const char* e = std::getenv("CTB_GEMM_TM");
+    return (e != nullptr && (e[0] == '1' || e[0] == '2')) ? e[0] - '0' : 0;
+  }();
+  return tm;
+}
+
 // Host copy of tile_coord: first row / column of output tile `tile`.
 template <int TM>
 inline void host_tile_origin(int tile, int num_m, int num_n, int n_rotate, int m_rotate, int* m0, int* n0) {
@@ -735,6 +754,13 @@ int launch(const CUtensorMap* ma, const CUtensorMap* mb, const CUtensorMap* mc, 
 
 }  // namespace gemm
 
+// Whether the product goes to the cluster split-K kernel (gemm_split.cu).  A switch that asks for one form of
+// the persistent kernel (its tile, its own split-K, dynamic tiles) is obeyed for every size.
+static bool gemm_splits(const GemmCall& c, int* width, int* slices) {
+  if (gemm::forced_tile_mode() != 0 || gemm::dynamic_tiles_mode() || gemm::split_k_mode() != 0) return false;
+  return gemm_split_plan(c, width, slices);
+}
+
 int run_gemm(const GemmCall& c) {
   using namespace gemm;
   if (c.M <= 0 || c.N <= 0 || c.K <= 0) return fail("gemm: M, N, K must be positive");
@@ -743,7 +769,7 @@ int run_gemm(const GemmCall& c) {
   if (needs_c && (c.ldc % (c.out_f32 ? 4 : 8))) return fail("gemm: ldc must be a multiple of 16 bytes");
   if (gemm_pair_eligible(c)) return launch_gemm_pair(c);       // two-CTA 256 x 256 tiles (gemm_pair.cu)
   int split_width = 0, split_slices = 0;
-  if (gemm_split_plan(c, &split_width, &split_slices)) return launch_gemm_split(c, split_width, split_slices);
+  if (gemm_splits(c, &split_width, &split_slices)) return launch_gemm_split(c, split_width, split_slices);
   const CUtensorMap* ma = c.a_mn ? get_tensor_map_2d(c.A, Elt::BF16, c.M, c.K, c.lda, 64, 64, true)
                                  : get_tensor_map_2d(c.A, Elt::BF16, c.K, c.M, c.lda, 64, BM, true);
   if (!ma) return 1;
@@ -790,12 +816,7 @@ int run_gemm(const GemmCall& c) {
   a.ce_lse = c.ce_lse;
   a.ce_coef = c.ce_coef;
   a.push = c.push;
-  // Dynamic tile claiming measured slightly slower than the static walk on B200 (0-4 % on the
-  // projection shapes, alone and under communication), so it is opt-in.
-  static const bool dynamic_tiles = [] {
-    const char* e = std::getenv("CTB_GEMM_DYNAMIC_TILES");
-    return e != nullptr && e[0] == '1';
-  }();
+  const bool dynamic_tiles = dynamic_tiles_mode();
   a.dynamic_tiles = dynamic_tiles ? 1 : 0;
   a.tile_counter = nullptr;
   if (dynamic_tiles) {
@@ -809,10 +830,7 @@ int run_gemm(const GemmCall& c) {
   }
   // Tile shape: 256 x 256 when there are enough of them to fill the machine a few times over,
   // 128 x 256 for small problems (CTB_GEMM_TM=1|2 forces one).
-  static const int forced_tm = [] {
-    const char* e = std::getenv("CTB_GEMM_TM");
-    return (e != nullptr && (e[0] == '1' || e[0] == '2')) ? e[0] - '0' : 0;
-  }();
+  const int forced_tm = forced_tile_mode();
   const int num_n = (c.N + BN - 1) / BN;
   const int tiles2 = ((c.M + 2 * BM - 1) / (2 * BM)) * num_n;
   // (the push epilogue copies every block out with the epilogue threads themselves and keeps its
@@ -1003,7 +1021,16 @@ CTB_API int ctb_ce_dlogits(const void* hidden, const void* head, void* g, int ro
   return ctb::run_gemm(c);
 }
 
-// 0: never split K; 1: split K when it fills the last wave (see launch_gemm).  Returns the previous mode.
+// Which kernel a plain product with a 16-byte aligned bf16 output takes: 1 and the tile width and number of K
+// slices of the cluster kernel, or 0 for the persistent kernel.
+CTB_API int ctb_gemm_split_choice(int M, int N, int K, int* width, int* slices) {
+  ctb::GemmCall c{};
+  c.M = M; c.N = N; c.K = K; c.alpha = 1.f; c.epi = ctb::EPI_STORE;
+  return ctb::gemm_splits(c, width, slices) ? 1 : 0;
+}
+
+// Split-K in the persistent kernel.  0: never; 1: split K when it fills the last wave (see run_gemm), and no
+// product goes to the cluster kernel.  Returns the previous mode.
 CTB_API int ctb_gemm_set_split_k(int mode) {
   int& m = ctb::gemm::split_k_mode();
   const int before = m;
