@@ -3,7 +3,7 @@
 //
 // A down projection or an input gradient of a short batch (M = 1000, N = 1536, K = 17920) has 48
 // tiles of 128 x 256: a third of the SMs work, each on a chain of K / 64 = 280 k-blocks, and nothing
-// but K is left to divide.  Here a cluster of S = 1, 2, 4 or 8 CTAs owns a tile; CTA s multiplies the
+// but K is left to divide.  Here a cluster of S = 2, 4 or 8 CTAs owns a tile; CTA s multiplies the
 // k-blocks [s K/S, (s+1) K/S) into its own TMEM accumulator, writes the fp32 partial tile into its own
 // shared memory (the operand ring is dead by then), and after one cluster barrier every CTA adds up 1/S
 // of the rows over distributed shared memory and stores them.  No workspace, no atomics: the partial
@@ -99,7 +99,7 @@ gemm_split_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_consta
   const int warp = uniform_warp_index();
   const int lane = threadIdx.x & 31;
   const int S = args.splits;
-  const int slice = S > 1 ? static_cast<int>(cluster_rank()) : 0;
+  const int slice = static_cast<int>(cluster_rank());
   const int tile = blockIdx.x / S;
   const int num_m = (args.M + BM - 1) / BM;
   const int m0 = (tile % num_m) * BM, n0 = (tile / num_m) * BN;   // tiles that share B are neighbours
@@ -228,7 +228,7 @@ gemm_split_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_consta
     tmem_dealloc(tmem_base, BN);
   }
   __syncwarp();
-  if (S > 1) cluster_barrier();          // every slice's partial tile is in its CTA's shared memory
+  cluster_barrier();                     // every slice's partial tile is in its CTA's shared memory
 
   // ------------------------------ sum of the slices, 1 / S of the rows per CTA ------------------------------
   constexpr int CHUNKS = BN / 4;
@@ -246,7 +246,7 @@ gemm_split_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_consta
         const uint32_t at = base + partial_offset(slice * rows + item / CHUNKS, item % CHUNKS, BN * 4);
 #pragma unroll
         for (int s = 0; s < MAX_SPLITS; ++s)
-          if (s < S) part[u][s] = S > 1 ? ld_peer(at, s) : *reinterpret_cast<const float4*>(smem + (at - base));
+          if (s < S) part[u][s] = ld_peer(at, s);
       }
 #pragma unroll
       for (int u = 0; u < U; ++u) {
@@ -292,7 +292,7 @@ gemm_split_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_consta
     }
   }
   __syncwarp();
-  if (S > 1) cluster_barrier();          // nobody leaves while a peer still reads its partial tile
+  cluster_barrier();                     // nobody leaves while a peer still reads its partial tile
 }
 
 template <int BN, bool A_MN, bool B_MN>
@@ -316,7 +316,7 @@ int launch(const CUtensorMap* ma, const CUtensorMap* mb, const SplitArgs& a, int
   attr[0].val.clusterDim.y = 1;
   attr[0].val.clusterDim.z = 1;
   cfg.attrs = attr;
-  cfg.numAttrs = a.splits > 1 ? 1 : 0;
+  cfg.numAttrs = 1;
   CTB_CUDA_OK(cudaLaunchKernelEx(&cfg, kern, *ma, *mb, a));
   return 0;
 }
@@ -335,7 +335,7 @@ int dispatch(const GemmCall& c, const CUtensorMap* ma, const CUtensorMap* mb, co
 // Chooses tile width and slices from estimated cycles and compares with the persistent kernel.  The figures
 // are fits to a sweep of 100 shapes on B200: a k-block takes about 700 cycles at either tile width (operand
 // latency, not the tensor core, once few CTAs run), a launch 6000 beside its k-blocks with the persistent
-// kernel, 9000 here and 14000 with an exchange of slices.  Clusters of 8, 4 and 2 leave some SMs of a 148-SM
+// kernel and 14000 here, where the slices are exchanged.  Clusters of 8, 4 and 2 leave some SMs of a 148-SM
 // part unused: 14, 32 and 72 of them run at a time.  Examples (us, persistent -> here): 64 x 1536 x 8960
 // 49 -> 15, 333 x 1536 x 32000 199 -> 60, 1000 x 1536 x 17920 107 -> 62; 2000 x 1536 x 17920 stays (112, 111).
 bool gemm_split_plan(const GemmCall& c, int* width, int* splits) {
@@ -351,12 +351,12 @@ bool gemm_split_plan(const GemmCall& c, int* width, int* splits) {
   bool found = false;
   for (int bn = 128; bn <= 256; bn += 128) {
     const long t = num_m * ((c.N + bn - 1) / bn);
-    for (int s = 1; s <= gemm3::MAX_SPLITS; s *= 2) {
+    for (int s = 2; s <= gemm3::MAX_SPLITS; s *= 2) {
       if (num_k < 4 * s) break;      // a slice shorter than the ring is all ramp
-      const long at_once = s == 1 ? sms : (s == 2 ? sms * 72 / 148 : (s == 4 ? sms * 32 / 148 : sms * 14 / 148));
+      const long at_once = s == 2 ? sms * 72 / 148 : (s == 4 ? sms * 32 / 148 : sms * 14 / 148);
       if (at_once < 1) break;
       const long waves = (t + at_once - 1) / at_once;
-      const double cycles = waves * (static_cast<double>((num_k + s - 1) / s) * 700.0 + (s == 1 ? 9000.0 : 14000.0));
+      const double cycles = waves * (static_cast<double>((num_k + s - 1) / s) * 700.0 + 14000.0);
       if (cycles < best) {
         best = cycles;
         *width = bn;
