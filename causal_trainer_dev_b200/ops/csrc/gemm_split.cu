@@ -390,3 +390,24 @@ int launch_gemm_split(const GemmCall& c, int width, int splits) {
 }
 
 }  // namespace ctb
+
+// The cluster kernel at a given tile width (128 or 256) and number of slices (2, 4 or 8), whatever the plan would
+// say: for tests of every form that the plan may choose and for measurements of the plan.
+CTB_API int ctb_gemm_split(const void* A, const void* B, void* C, int M, int N, int K, long lda, long ldb, long ldc,
+                           int a_mn, int b_mn, int out_f32, float alpha, const void* bias, int width, int slices,
+                           void* stream) {
+  using ctb::fail;
+  if (M <= 0 || N <= 0 || K <= 0) return fail("gemm_split: M, N, K must be positive");
+  if (lda % 8 || ldb % 8) return fail("gemm_split: lda and ldb must be multiples of 8 elements (16 bytes)");
+  if (ldc % (out_f32 ? 4 : 8) || reinterpret_cast<uintptr_t>(C) % 16)
+    return fail("gemm_split: rows of C must be 16-byte aligned");
+  if (bias != nullptr && out_f32) return fail("gemm_split: a biased product is stored as bf16");
+  if ((width != 128 && width != 256) || (slices != 2 && slices != 4 && slices != 8))
+    return fail("gemm_split: width 128 or 256, 2, 4 or 8 slices");
+  if ((K + 63) / 64 < slices) return fail("gemm_split: every slice needs a k-block");
+  ctb::GemmCall c{};
+  c.A = A; c.B = B; c.C = C; c.M = M; c.N = N; c.K = K; c.lda = lda; c.ldb = ldb; c.ldc = ldc;
+  c.a_mn = a_mn; c.b_mn = b_mn; c.out_f32 = out_f32; c.alpha = alpha; c.bias = bias;
+  c.epi = ctb::EPI_STORE; c.stream = stream;
+  return ctb::launch_gemm_split(c, width, slices);
+}

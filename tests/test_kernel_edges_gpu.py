@@ -5,6 +5,7 @@ Each is compared with a 64-bit PyTorch statement of the same operation.  ``BF16`
 relative error of one rounding to bf16 (half a unit in the last of its 8 bits, 2^-8): a result rounded once
 is within it, one that is built from an intermediate rounded once within twice that.
 """
+import ctypes
 import math
 
 import pytest
@@ -221,9 +222,13 @@ def test_embedding_gradient_of_long_and_short_runs(cuda_lib, d, dtype):
                                    (64, 1000, 640), (500, 96, 5000), (1000, 1536, 3000)])
 @pytest.mark.parametrize("a_mn,b_mn", [(False, False), (False, True), (True, True), (True, False)])
 def test_products_with_few_tiles(cuda_lib, m, n, k, a_mn, b_mn):
-    """Against 64 bits and against the persistent kernel (which a call that limits its CTAs always gets)."""
+    """Against 64 bits and against the persistent kernel (which a call that limits its CTAs always gets).  Two of
+    the shapes are just too short for the cluster kernel."""
     from causal_trainer_dev_b200.ops.gemm import gemm
 
+    form = ctypes.c_int(), ctypes.c_int()
+    planned = cuda_lib.lib().ctb_gemm_split_choice(m, n, k, ctypes.byref(form[0]), ctypes.byref(form[1]))
+    assert planned == int((m, n, k) not in [(128, 256, 1024), (64, 1000, 640)])
     pad = lambda x: -(-x // 8) * 8  # noqa: E731
     a = _bf16(k, pad(m), seed=1)[:, :m] if a_mn else _bf16(m, pad(k), seed=1)[:, :k]
     b = _bf16(k, pad(n), seed=2)[:, :n] if b_mn else _bf16(n, pad(k), seed=2)[:, :k]
@@ -239,6 +244,31 @@ def test_products_with_few_tiles(cuda_lib, m, n, k, a_mn, b_mn):
     assert _rel(biased, (want + bias.double()) * 0.5) < BF16
     full = torch.empty(m, pad(n), dtype=torch.float32, device="cuda")[:, :n]
     assert _rel(gemm(a, b, a_mn=a_mn, b_mn=b_mn, out=full, alpha=0.5), want * 0.5) < 1e-5     # fp32 sums of 9000 products
+    assert cuda_lib.device_status() == (0, 0, 0, 0)
+
+
+@pytest.mark.parametrize("width,slices", [(w, s) for w in (128, 256) for s in (2, 4, 8)])
+@pytest.mark.parametrize("m,n,k", [(1, 8, 512), (130, 270, 1000), (257, 512, 520), (300, 131, 4104)])
+@pytest.mark.parametrize("a_mn,b_mn", [(False, False), (False, True), (True, True), (True, False)])
+def test_every_form_of_the_cluster_kernel(cuda_lib, width, slices, m, n, k, a_mn, b_mn):
+    """Slices of unequal length, the last k-block, rows and columns cut off, and slices of a single k-block."""
+    pad = lambda x: -(-x // 8) * 8  # noqa: E731
+    a = _bf16(k, pad(m), seed=1)[:, :m] if a_mn else _bf16(m, pad(k), seed=1)[:, :k]
+    b = _bf16(k, pad(n), seed=2)[:, :n] if b_mn else _bf16(n, pad(k), seed=2)[:, :k]
+    want = (a.double().t() if a_mn else a.double()) @ (b.double() if b_mn else b.double().t())
+    bias, p, ln = _bf16(n, seed=3), cuda_lib.ptr, ctypes.c_long
+
+    def run(dtype, alpha, bias):
+        out = torch.full((m, pad(n) + 8), 7.0, dtype=dtype, device="cuda")
+        cuda_lib.check(cuda_lib.lib().ctb_gemm_split(
+            p(a), p(b), p(out), m, n, k, ln(a.stride(0)), ln(b.stride(0)), ln(out.stride(0)), int(a_mn), int(b_mn),
+            int(dtype == torch.float32), ctypes.c_float(alpha), p(bias), width, slices, cuda_lib.stream_ptr()), "ctb_gemm_split")
+        assert torch.all(out[:, n:] == 7.0)                                   # nothing beyond column n
+        return out[:, :n]
+
+    assert _rel(run(torch.bfloat16, 1.0, None), want) < BF16
+    assert _rel(run(torch.bfloat16, 0.5, bias), (want + bias.double()) * 0.5) < BF16
+    assert _rel(run(torch.float32, 0.5, None), want * 0.5) < 1e-5             # fp32 sums of 4104 products
     assert cuda_lib.device_status() == (0, 0, 0, 0)
 
 
