@@ -53,8 +53,7 @@ def test_attention_gradients_with_odd_numbers_of_blocks(cuda_lib, d, hq, hkv, le
 
 
 def test_attention_keeps_nan_and_stays_finite_elsewhere(cuda_lib):
-    """A NaN query makes its own output row NaN and no other: the exponentials that run on the FMA pipe pass
-    NaN on like the ex2 unit."""
+    """A NaN query makes its own output row NaN and no other."""
     from causal_trainer_dev_b200.ops import attention as A
 
     q, k, v = (_bf16(1, 512, h, 128, seed=i) for i, h in enumerate((2, 1, 1)))
@@ -63,6 +62,22 @@ def test_attention_keeps_nan_and_stays_finite_elsewhere(cuda_lib):
     bad = torch.isnan(o).any(-1)
     assert bad[0, 300, 1] and int(bad.sum()) == 1
     assert bool(torch.isnan(o[0, 300, 1]).all())
+
+
+@pytest.mark.parametrize("d", [128, 64])
+@pytest.mark.parametrize("key", [6, 7, 14, 79, 126, 127, 5, 128 + 54])
+def test_a_nan_key_reaches_every_query_that_sees_it(cuda_lib, d, key):
+    """The scores of one key are NaN, the maxima of the rows stay finite, so query tiles that see the key's whole tile
+    take the path whose exponentials of columns 6 and 7 of every 8 run on the FMA pipe (both halves of a pair are
+    here, and columns of the ex2 unit): NaN passes through either, and only to queries at or behind the key."""
+    from causal_trainer_dev_b200.ops import attention as A
+
+    s = 640
+    q, k, v = (_bf16(1, s, h, d, seed=i) for i, h in enumerate((2, 1, 1)))
+    k[0, key, 0, 3] = math.nan
+    o, _ = A.flash_attention_forward(q, k, v, A.build_attention_meta(torch.ones(1, s, dtype=torch.int32, device="cuda")))
+    sees = (torch.arange(s, device="cuda") >= key)[None, :, None]
+    assert torch.equal(torch.isnan(o).any(-1), sees.expand(1, s, 2)) and torch.equal(torch.isnan(o).all(-1), sees.expand(1, s, 2))
 
 
 @pytest.mark.parametrize("d", [128, 64, 96])
