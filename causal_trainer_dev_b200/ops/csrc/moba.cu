@@ -450,8 +450,8 @@ CTB_API int ctb_moba_lists(int mode, const unsigned* touch, int B, int S, int Hq
 //                the same (document, head) and leaves the count in cnt[group][head in group]:
 //                moba_rank_bits_kernel, one CTA per (batch, head, c), from a bit per token (rows of up
 //                to 192512 tokens); moba_rank_scan_kernel, a segmented scan over the sequence (longer
-//                rows); moba_rank_kernel, one warp per (batch, head, c) walking the sequence
-//                (CTB_MOBA_RANK=walk; same result, kept for comparison).
+//                rows, CTB_MOBA_RANK=scan); moba_rank_kernel, one warp per (batch, head, c) walking the
+//                sequence (CTB_MOBA_RANK=walk).  The same ranks from all three.
 //   moba_groups  one CTA: exclusive scan of the padded group sizes -> first row of every group,
 //                offsets of the heads inside a group, the compact list of non-empty groups.
 //   moba_desc    descriptors of the CTAs of the grouped flash kernels.
@@ -1029,15 +1029,14 @@ CTB_API int ctb_moba_group(const unsigned* sel, const int* seg, const int* doc_s
   CTB_CUDA_OK(cudaMemsetAsync(cnt, 0, sizeof(int) * static_cast<size_t>(G) * gsize, s));
   CTB_CUDA_OK(cudaMemsetAsync(row_of, 0xff, sizeof(int) * static_cast<size_t>(rows_cap), s));
   const long warps = static_cast<long>(B) * Hq * nblk;
-  // CTB_MOBA_RANK=walk selects the one-warp-per-(head, block) walk; the default is the CTA-wide scan
-  static const bool walk = [] {
-    const char* e = std::getenv("CTB_MOBA_RANK");
-    return e != nullptr && e[0] == 'w';
-  }();
-  if (walk || warps > 0x7fffffffL)
+  // the ranks from a bit per token where its words and counts fit into 48 KB, else by the CTA-wide scan;
+  // CTB_MOBA_RANK=walk|scan|bits asks for one of the three (bits only where they fit)
+  const char* wish = std::getenv("CTB_MOBA_RANK");
+  const char kind = wish != nullptr ? wish[0] : 'b';
+  if (kind == 'w' || warps > 0x7fffffffL)
     moba::moba_rank_kernel<<<static_cast<unsigned>((warps * 32 + 255) / 256), 256, 0, s>>>(
         sel, seg, doc_start, B, S, Hq, Hkv, block, words, nblk, picks, rank, cnt);
-  else if (S <= moba::RANK_MAX_SEQ)                      // its words and counts fit into 48 KB
+  else if (kind != 's' && S <= moba::RANK_MAX_SEQ)
     moba::moba_rank_bits_kernel<<<static_cast<unsigned>(warps), 1024, S / 4, s>>>(
         sel, seg, doc_start, S, Hq, Hkv, block, words, nblk, picks, rank, cnt);
   else

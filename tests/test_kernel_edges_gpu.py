@@ -324,3 +324,36 @@ def test_router_picks_the_best_blocks(cuda_lib, d, hq, hkv, top_k):
         assert bool((left <= worst + 1e-5).all())
         at += n
     assert not bits[:, at:].any()
+
+
+@pytest.mark.parametrize("s,block,top_k,kinds", [(4096, 128, 3, "bits scan walk"), (1024, 256, 2, "bits scan walk"),
+                                                 (192512, 4096, 4, "bits scan"), (192640, 4096, 4, "bits scan walk")])
+def test_rank_kernels_group_alike(cuda_lib, monkeypatch, s, block, top_k, kinds):
+    """Ranks from a bit per token (rows of up to 192512 tokens), by the scan (longer rows) and by the walk give the same
+    grouping bit for bit: documents that begin anywhere, padding between and behind them."""
+    from causal_trainer_dev_b200.ops import attention as A
+    from causal_trainer_dev_b200.ops import moba as M
+
+    seg = torch.zeros(2, s, dtype=torch.int32, device="cuda")
+    for row, cuts in enumerate(([0, s // 37, s // 3 + 5, s - 77], [13, s // 2 + 1, s])):
+        for i, (lo, hi) in enumerate(zip(cuts[:-1], cuts[1:])):
+            seg[row, lo:hi] = i + 1
+    seg[0, s // 3 - 40:s // 3 + 5] = 0                                        # padding between two documents
+    q, k = _bf16(2, s, 2, 64, seed=1), _bf16(2, s, 1, 64, seed=2)
+    meta = A.build_attention_meta(seg)
+    seen = []
+    for kind in kinds.split():
+        monkeypatch.setenv("CTB_MOBA_RANK", kind)
+        g = M.build_groups(q, k, meta, block, top_k)
+        seen.append((g.totals, g.row_of, g.pos_of, g.fwd_desc, g.dq_desc, g.dkv_desc))
+    assert int(seen[0][0][0]) > 0
+    for other in seen[1:]:
+        assert all(torch.equal(a, b) for a, b in zip(seen[0], other))
+    # ranks: the rows of a (document, head, block) in the order of their tokens
+    rows = int(seen[0][0][0])
+    token = (seen[0][1][:rows] // 2).long()
+    pos = seen[0][2]
+    for h in range(2):
+        for j in range(top_k - 1):
+            mine = pos[0, h, :, j]
+            assert torch.equal(token[mine[mine >= 0].long()], torch.nonzero(mine >= 0)[:, 0])
