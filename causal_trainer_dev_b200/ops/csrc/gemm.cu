@@ -955,7 +955,8 @@ CTB_API int ctb_gemm(const void* A, const void* B, void* C, int M, int N, int K,
 
 // Same GEMM family whose B operand lives in a buffer that another kernel (the all-gather
 // pull) is still filling: flags[i] >= epoch means elements [i*chunk, (i+1)*chunk) of that
-// buffer are complete; `flag_base` is the element offset of B inside the buffer.
+// buffer are complete; `flag_base` is the element offset of B inside the buffer.  Flags may be null once
+// the pull is known to be done: the product takes the same kernel either way, so its bits do not depend on that.
 CTB_API int ctb_gemm_flagged(const void* A, const void* B, void* C, int M, int N, int K, long lda, long ldb, long ldc,
                              int a_mn, int b_mn, int out_f32, int accumulate, float alpha, const void* bias,
                              const unsigned* flags, long flag_chunk, long flag_base, unsigned epoch, int wait_all,
@@ -968,7 +969,7 @@ CTB_API int ctb_gemm_flagged(const void* A, const void* B, void* C, int M, int N
   c.b_flags = flags; c.b_flag_chunk = flag_chunk; c.b_flag_base = flag_base; c.b_flag_epoch = epoch;
   c.b_wait_all = wait_all; c.spin_budget = spin_budget; c.n_rotate = n_rotate;
   c.a_flags = a_flags; c.a_flag_chunk = a_flag_chunk; c.a_flag_base = a_flag_base; c.a_flag_epoch = a_epoch;
-  c.m_rotate = m_rotate;
+  c.m_rotate = m_rotate; c.gathered = 1;
   return ctb::run_gemm(c);
 }
 

@@ -89,6 +89,7 @@ struct GemmCall {
   long a_flag_chunk = 0;
   long a_flag_base = 0;
   unsigned a_flag_epoch = 0;
+  int gathered = 0;       // an operand lies in a gathered buffer (its flags may be left out once the pull is done)
   long long spin_budget = 0;
   const int* ce_targets = nullptr;
   float* ce_max = nullptr;

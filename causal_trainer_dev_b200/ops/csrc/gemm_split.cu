@@ -339,9 +339,10 @@ int dispatch(const GemmCall& c, const CUtensorMap* ma, const CUtensorMap* mb, co
 // part unused: 14, 32 and 72 of them run at a time.  Examples (us, persistent -> here): 64 x 1536 x 8960
 // 49 -> 15, 333 x 1536 x 32000 199 -> 60, 1000 x 1536 x 17920 107 -> 62; 2000 x 1536 x 17920 stays (112, 111).
 bool gemm_split_plan(const GemmCall& c, int* width, int* splits) {
-  if (c.epi != EPI_STORE || c.accumulate || c.push.enabled || c.a_flags != nullptr || c.b_flags != nullptr ||
-      c.max_ctas > 0)
-    return false;
+  if (c.epi != EPI_STORE || c.accumulate || c.push.enabled || c.max_ctas > 0) return false;
+  // a gathered operand: with flags only the persistent kernel will do, and without them (the pull was done
+  // before the call) the product must come out the same
+  if (c.gathered || c.a_flags != nullptr || c.b_flags != nullptr) return false;
   if (reinterpret_cast<uintptr_t>(c.C) % 16 != 0) return false;
   if (c.bias != nullptr && c.out_f32) return false;      // the fp32 store of the persistent kernel takes no bias
   const long num_m = (c.M + 127) / 128, num_k = (c.K + 63) / 64, sms = sm_count();

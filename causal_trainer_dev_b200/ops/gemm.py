@@ -46,14 +46,20 @@ def unregister_flag_source(src: FlagSource) -> None:
         _FLAG_SOURCES.remove(src)
 
 
-def flag_source_of(t: torch.Tensor) -> tuple[FlagSource, int] | None:
+def _source_of(t: torch.Tensor) -> FlagSource | None:
+    """The gathered buffer that ``t`` lies in, whether or not its pull has completed."""
     p = t.data_ptr()
     for src in _FLAG_SOURCES:
         if src.start <= p < src.end and src.epoch > 0:
-            if src.complete is not None and src.complete.query():
-                return None
-            return src, (p - src.start) // t.element_size()
+            return src
     return None
+
+
+def flag_source_of(t: torch.Tensor) -> tuple[FlagSource, int] | None:
+    src = _source_of(t)
+    if src is None or (src.complete is not None and src.complete.query()):
+        return None
+    return src, (t.data_ptr() - src.start) // t.element_size()
 
 
 def _flag_args(hit):
@@ -118,9 +124,10 @@ def gemm(
         raise ValueError("out must be [M,N] bf16/fp32 with unit inner stride")
     if bias is not None and (bias.dtype != torch.bfloat16 or bias.numel() != n):
         raise ValueError("bias must be bf16 of length N")
-    hit = flag_source_of(b) if _FLAG_SOURCES else None
-    hit_a = flag_source_of(a) if _FLAG_SOURCES else None
-    if hit is not None or hit_a is not None:
+    if _FLAG_SOURCES and (_source_of(b) is not None or _source_of(a) is not None):
+        # (a finished pull needs no flags, but the same kernel: how far a pull has come must not decide the
+        # order of the sums)
+        hit, hit_a = flag_source_of(b), flag_source_of(a)
         n_rotate, m_rotate = _rotations(hit, hit_a, a, b, a_mn, b_mn, m, n)
         bf = _flag_args(hit)
         af = _flag_args(hit_a)

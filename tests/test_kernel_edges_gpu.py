@@ -287,6 +287,30 @@ def test_every_form_of_the_cluster_kernel(cuda_lib, width, slices, m, n, k, a_mn
     assert cuda_lib.device_status() == (0, 0, 0, 0)
 
 
+@pytest.mark.parametrize("side", ["weight", "activation"])
+@pytest.mark.parametrize("m,n,k", [(64, 1536, 8960), (512, 512, 8192)])
+def test_a_product_of_a_gathered_operand_does_not_depend_on_how_far_its_gather_has_come(cuda_lib, side, m, n, k):
+    """With chunk flags (the gather may still run) and without (it was seen to be done) the bits are the same."""
+    from causal_trainer_dev_b200.ops import gemm as G
+
+    a, b = _bf16(m, k, seed=1), _bf16(n, k, seed=2)
+    buffer = b if side == "weight" else a
+    src = G.FlagSource(buffer, torch.ones(buffer.numel() // 65536 + 1, dtype=torch.int32, device="cuda"), 65536)
+    src.epoch = 1
+    G.register_flag_source(src)
+    try:
+        running = G.gemm(a, b)
+        src.complete = torch.cuda.Event()
+        src.complete.record()
+        src.complete.synchronize()
+        done = G.gemm(a, b)
+    finally:
+        G.unregister_flag_source(src)
+    assert torch.equal(running, done)
+    assert _rel(done, a.double() @ b.double().t()) < BF16
+    assert cuda_lib.device_status() == (0, 0, 0, 0)
+
+
 # ------------------------------------------------------------------------------ MoBA router
 @pytest.mark.parametrize("d,hq,hkv", [(128, 4, 2), (64, 3, 1)])
 @pytest.mark.parametrize("top_k", [1, 2, 9, 10])
