@@ -199,9 +199,9 @@ def attention_backward_stats(o: torch.Tensor, dout: torch.Tensor, lse: torch.Ten
     b, s, h, d = o.shape
     neg_lse2 = torch.empty((b, h, s), dtype=torch.float32, device=o.device)
     neg_delta = torch.empty_like(neg_lse2)
-    code = _lib.lib().ctb_attn_bwd_stats(_lib.ptr(o), _lib.ptr(dout), _lib.ptr(lse), _lib.ptr(neg_lse2),
-                                         _lib.ptr(neg_delta), b, s, h, d, _l(o.stride(1)), _l(dout.stride(1)),
-                                         _lib.stream_ptr())
+    code = _lib.lib().ctb_attn_bwd_stats(o.data_ptr(), dout.data_ptr(), lse.data_ptr(), neg_lse2.data_ptr(),
+                                         neg_delta.data_ptr(), b, s, h, d, o.stride(1), dout.stride(1),
+                                         _lib.raw_stream())
     _lib.check(code, "ctb_attn_bwd_stats")
     return neg_lse2, neg_delta
 

@@ -14,10 +14,11 @@ import torch
 from .build import LIB_PATH
 
 
-# Argument kinds of the launchers that every layer calls several times (p pointer, i int, l long, f float,
-# q long long): with them ctypes converts plain Python numbers itself, and a call needs no wrapper object per
-# argument.  Launchers that are not listed take wrapped arguments (:func:`ptr` and the ctypes types).
-_KINDS = {"p": ctypes.c_void_p, "i": ctypes.c_int, "l": ctypes.c_long, "f": ctypes.c_float, "q": ctypes.c_longlong}
+# Argument kinds of the projections, norms, rotary embedding, activation and backward statistics (p pointer,
+# i int, l long, f float): with them ctypes converts plain Python numbers itself, and a call needs no wrapper object
+# per argument.  All other launchers, the attention kernels among them, take wrapped arguments (:func:`ptr` and the
+# ctypes types).
+_KINDS = {"p": ctypes.c_void_p, "i": ctypes.c_int, "l": ctypes.c_long, "f": ctypes.c_float}
 _SIGNATURES = {
     "ctb_gemm": "pppiiillliiiifpip",
     "ctb_rmsnorm_fwd": "ppppppiifp",
