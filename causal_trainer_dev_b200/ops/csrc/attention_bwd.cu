@@ -200,7 +200,8 @@ attn_bwd_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constant
     *abort_flag = 0u;
     mbar_fence_init();
     if (n_iter > 0) {
-      // the resident tiles are on their way while TMEM is allocated
+      // the resident tiles are on their way while TMEM is allocated (with Q in the forward kernel, a layer's forward
+      // and backward: 8.00 -> 7.77 ms on one document of 32768 tokens, 1096 -> 1047 us on 8 image rows of 4096)
       mbar_expect_tx(x_full, 2 * L::XT);
       const CUtensorMap* mx1 = DKV ? &map_k : &map_q;
       const CUtensorMap* mx2 = DKV ? &map_v : &map_do;
