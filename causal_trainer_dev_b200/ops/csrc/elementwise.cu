@@ -1138,12 +1138,16 @@ CTB_API int ctb_attn_delta(const void* o, const void* dout, float* delta, int B,
 // o, dout: [B,S,H,D] bf16 views (row strides in elements); lse, neg_lse2, neg_delta: [B,H,S] fp32.
 CTB_API int ctb_attn_bwd_stats(const void* o, const void* dout, const float* lse, float* neg_lse2, float* neg_delta,
                                int B, int S, int H, int D, long o_rs, long do_rs, void* stream) {
-  // 16-byte rows of the two head sizes the flash kernels take (anything else: one warp per row, below)
-  const bool wide = (D == 64 || D == 128) && o_rs % 8 == 0 && do_rs % 8 == 0 &&
-                    (reinterpret_cast<uintptr_t>(o) | reinterpret_cast<uintptr_t>(dout)) % 16 == 0;
+  // 16-byte rows of the two head sizes the flash kernels take, and enough of them: a block of the wide kernel takes
+  // 256 rows one after the other, 4.0 us at D = 64 and 6.4 at D = 128 however few there are, where a warp per row
+  // (below) takes 2.0 and grows with the rows.  They meet at 192 D rows (us, warp per row and wide: D = 64 8192 rows
+  // 3.5 and 4.0, 12288 rows 4.2 and 4.0, 16384 rows 5.0 and 4.1; D = 128 16384 rows 5.3 and 6.5, 24576 rows 7.0
+  // and 6.6, 32768 rows 8.6 and 6.9).
   const long tokens = static_cast<long>(B) * S;
+  const bool wide = (D == 64 || D == 128) && o_rs % 8 == 0 && do_rs % 8 == 0 && tokens * H >= 192l * D &&
+                    (reinterpret_cast<uintptr_t>(o) | reinterpret_cast<uintptr_t>(dout)) % 16 == 0;
   const int head_blocks = (H + STAT_HEADS - 1) / STAT_HEADS;
-  if (wide && tokens > 0 && H > 0 && head_blocks <= 65535) {
+  if (wide && head_blocks <= 65535) {
     const dim3 grid(static_cast<unsigned>((tokens + STAT_TOKENS - 1) / STAT_TOKENS), head_blocks);
     auto kern = D == 128 ? attn_bwd_stats_vec_kernel<128> : attn_bwd_stats_vec_kernel<64>;
     kern<<<grid, 256, 0, static_cast<cudaStream_t>(stream)>>>(
