@@ -388,29 +388,60 @@ __global__ void rope_table_kernel(const int* __restrict__ pos, const float* __re
 // SwiGLU on the packed projection gu[T][2f] = [gate | up]:  h = silu(gate) * up.
 // Backward writes d(gate|up) in the same packed layout.
 // ------------------------------------------------------------------------------------------
-// A thread keeps its column vector and walks the rows (blockIdx.y, two at a time), so there is no
-// division per vector.  The quotient of the sigmoid is the correctly rounded one: the fast division takes
-// 246 us where this takes 325 (forward, 16384 x 14336; 339 with a division per vector as well; backward 398 and
-// 408), but returns zero for denominators above 2^126, i.e. for gates between -88.7 and -87.4.  So the forward
-// kernel is bound by the instructions of that division (1.41 GB at 4.3 TB/s), the backward one by memory.
-constexpr int SWIGLU_ROWS = 2;
+// A thread takes every gridDim * blockDim-th 16-byte vector of h and steps its row along instead of dividing for
+// it, so no thread idles whatever the width (a column per thread and rows over blockIdx.y left 224 of 256 idle at
+// f = 256: 100000 x 256 82 us forward where this takes 36).  The forward kernel keeps two vectors in flight where
+// a thread has ten or more (16384 x 14336: 279 us against 300; 333 x 8960: 5.7 against 5.1), the backward kernel one (389 us
+// against 465 with two, for their 92 registers).
+// The quotient of the sigmoid is the correctly rounded one: the fast division takes 228 and 371 us at 16384 x 14336
+// where this takes 279 and 389, but returns zero for denominators above 2^126, i.e. for gates between -88.7 and
+// -87.4.  So the forward kernel is bound by the instructions of that division (1.41 GB at 5.0 TB/s), the
+// backward one by memory (6.0 TB/s).
+struct SwigluWalk {
+  long i, total, stride;      // vector of h; number of them; step
+  long row_at, row_step;      // (row of i) * nvec: the gate vector of i is i + row_at, its up vector nvec further
+  int v, v_step, nvec;        // column of i
+  __device__ __forceinline__ SwigluWalk(long T, int f) {
+    nvec = f / 8;
+    total = T * nvec;
+    const unsigned first = blockIdx.x * blockDim.x + threadIdx.x, all = gridDim.x * blockDim.x;   // (a few hundred thousand)
+    i = first;
+    stride = all;
+    v = static_cast<int>(first % nvec);
+    row_at = i - v;
+    v_step = static_cast<int>(all % nvec);
+    row_step = stride - v_step;
+  }
+  __device__ __forceinline__ void step() {
+    i += stride;
+    v += v_step;
+    row_at += row_step;
+    if (v >= nvec) {
+      v -= nvec;
+      row_at += nvec;
+    }
+  }
+};
+template <int AHEAD>      // vectors in flight
 __global__ void __launch_bounds__(256)
 swiglu_fwd_kernel(const __nv_bfloat16* __restrict__ gu, __nv_bfloat16* __restrict__ h, long T, int f) {
-  const int nvec = f / 8, v = blockIdx.x * blockDim.x + threadIdx.x;
-  if (v >= nvec) return;
-  const long step = static_cast<long>(gridDim.y) * SWIGLU_ROWS;
-  for (long t0 = static_cast<long>(blockIdx.y) * SWIGLU_ROWS; t0 < T; t0 += step) {
-    uint4 gv[SWIGLU_ROWS], uv[SWIGLU_ROWS];
+  const uint4* src = reinterpret_cast<const uint4*>(gu);
+  SwigluWalk w(T, f);
+  while (w.i < w.total) {
+    uint4 gv[AHEAD], uv[AHEAD];
+    long to[AHEAD];
 #pragma unroll
-    for (int k = 0; k < SWIGLU_ROWS; ++k)
-      if (t0 + k < T) {
-        const uint4* row = reinterpret_cast<const uint4*>(gu) + static_cast<size_t>(t0 + k) * 2 * nvec;
-        gv[k] = row[v];
-        uv[k] = row[nvec + v];
+    for (int k = 0; k < AHEAD; ++k) {
+      to[k] = w.i;
+      if (w.i < w.total) {
+        gv[k] = src[w.i + w.row_at];
+        uv[k] = src[w.i + w.row_at + w.nvec];
       }
+      w.step();
+    }
 #pragma unroll
-    for (int k = 0; k < SWIGLU_ROWS; ++k)
-      if (t0 + k < T) {
+    for (int k = 0; k < AHEAD; ++k)
+      if (to[k] < w.total) {
         float g[8], u[8], o[8];
         unpack8(gv[k], g);
         unpack8(uv[k], u);
@@ -419,44 +450,31 @@ swiglu_fwd_kernel(const __nv_bfloat16* __restrict__ gu, __nv_bfloat16* __restric
           const float act = __bfloat162float(__float2bfloat16(g[e] / (1.f + __expf(-g[e]))));
           o[e] = act * u[e];
         }
-        reinterpret_cast<uint4*>(h)[static_cast<size_t>(t0 + k) * nvec + v] = pack8(o);
+        reinterpret_cast<uint4*>(h)[to[k]] = pack8(o);
       }
   }
 }
 __global__ void __launch_bounds__(256)
 swiglu_bwd_kernel(const __nv_bfloat16* __restrict__ gu, const __nv_bfloat16* __restrict__ dh,
                   __nv_bfloat16* __restrict__ dgu, long T, int f) {
-  const int nvec = f / 8, v = blockIdx.x * blockDim.x + threadIdx.x;
-  if (v >= nvec) return;
-  const long step = static_cast<long>(gridDim.y) * SWIGLU_ROWS;
-  for (long t0 = static_cast<long>(blockIdx.y) * SWIGLU_ROWS; t0 < T; t0 += step) {
-    uint4 gv[SWIGLU_ROWS], uv[SWIGLU_ROWS], dv[SWIGLU_ROWS];
+  const uint4* src = reinterpret_cast<const uint4*>(gu);
+  uint4* dst = reinterpret_cast<uint4*>(dgu);
+  for (SwigluWalk w(T, f); w.i < w.total; w.step()) {
+    const long at = w.i + w.row_at;
+    const uint4 gv = src[at], uv = src[at + w.nvec], dv = reinterpret_cast<const uint4*>(dh)[w.i];
+    float g[8], u[8], d[8], dg[8], du[8];
+    unpack8(gv, g);
+    unpack8(uv, u);
+    unpack8(dv, d);
 #pragma unroll
-    for (int k = 0; k < SWIGLU_ROWS; ++k)
-      if (t0 + k < T) {
-        const uint4* row = reinterpret_cast<const uint4*>(gu) + static_cast<size_t>(t0 + k) * 2 * nvec;
-        gv[k] = row[v];
-        uv[k] = row[nvec + v];
-        dv[k] = reinterpret_cast<const uint4*>(dh)[static_cast<size_t>(t0 + k) * nvec + v];
-      }
-#pragma unroll
-    for (int k = 0; k < SWIGLU_ROWS; ++k)
-      if (t0 + k < T) {
-        float g[8], u[8], d[8], dg[8], du[8];
-        unpack8(gv[k], g);
-        unpack8(uv[k], u);
-        unpack8(dv[k], d);
-#pragma unroll
-        for (int e = 0; e < 8; ++e) {
-          const float sg = 1.f / (1.f + __expf(-g[e]));
-          const float act = g[e] * sg;
-          du[e] = d[e] * act;
-          dg[e] = d[e] * u[e] * sg * (1.f + g[e] * (1.f - sg));
-        }
-        uint4* orow = reinterpret_cast<uint4*>(dgu) + static_cast<size_t>(t0 + k) * 2 * nvec;
-        orow[v] = pack8(dg);
-        orow[nvec + v] = pack8(du);
-      }
+    for (int e = 0; e < 8; ++e) {
+      const float sg = 1.f / (1.f + __expf(-g[e]));
+      const float act = g[e] * sg;
+      du[e] = d[e] * act;
+      dg[e] = d[e] * u[e] * sg * (1.f + g[e] * (1.f - sg));
+    }
+    dst[at] = pack8(dg);
+    dst[at + w.nvec] = pack8(du);
   }
 }
 
@@ -1086,20 +1104,13 @@ CTB_API int ctb_rope(void* x, const float* cosv, const float* sinv, long row_str
   return 0;
 }
 
-// Column blocks x row blocks, about eight CTAs per SM.
-static inline dim3 swiglu_grid(long T, int f) {
-  const long cols = (f / 8 + 255) / 256;
-  long rows = (T + SWIGLU_ROWS - 1) / SWIGLU_ROWS;
-  const long cap = (static_cast<long>(sm_count()) * 8 + cols - 1) / cols;
-  if (rows > cap) rows = cap;
-  if (rows > 65535) rows = 65535;
-  return dim3(static_cast<unsigned>(cols), static_cast<unsigned>(rows));
-}
-
 CTB_API int ctb_swiglu_fwd(const void* gu, void* h, long T, int f, void* stream) {
   if (f % 8) return fail("swiglu: intermediate size must be a multiple of 8");
   if (T <= 0 || f <= 0) return 0;
-  swiglu_fwd_kernel<<<swiglu_grid(T, f), 256, 0, static_cast<cudaStream_t>(stream)>>>(
+  const long total = T * (f / 8);
+  const int grid = grid_for(total, 256);
+  auto kern = total >= 10l * 256 * grid ? swiglu_fwd_kernel<2> : swiglu_fwd_kernel<1>;
+  kern<<<grid, 256, 0, static_cast<cudaStream_t>(stream)>>>(
       static_cast<const __nv_bfloat16*>(gu), static_cast<__nv_bfloat16*>(h), T, f);
   CTB_CUDA_OK(cudaGetLastError());
   return 0;
@@ -1108,7 +1119,7 @@ CTB_API int ctb_swiglu_fwd(const void* gu, void* h, long T, int f, void* stream)
 CTB_API int ctb_swiglu_bwd(const void* gu, const void* dh, void* dgu, long T, int f, void* stream) {
   if (f % 8) return fail("swiglu: intermediate size must be a multiple of 8");
   if (T <= 0 || f <= 0) return 0;
-  swiglu_bwd_kernel<<<swiglu_grid(T, f), 256, 0, static_cast<cudaStream_t>(stream)>>>(
+  swiglu_bwd_kernel<<<grid_for(T * (f / 8), 256), 256, 0, static_cast<cudaStream_t>(stream)>>>(
       static_cast<const __nv_bfloat16*>(gu), static_cast<const __nv_bfloat16*>(dh), static_cast<__nv_bfloat16*>(dgu),
       T, f);
   CTB_CUDA_OK(cudaGetLastError());

@@ -129,7 +129,7 @@ def test_rmsnorm_backward_widths(cuda_lib, rows, d):
         assert _rel(dw, wd.grad) < 1e-5                                       # fp32 sums over the rows
 
 
-@pytest.mark.parametrize("rows,f", [(1, 8), (2, 2048), (7, 2056), (1301, 688)])
+@pytest.mark.parametrize("rows,f", [(1, 8), (2, 2048), (7, 2056), (1301, 688), (40003, 24), (4099, 6008)])
 def test_swiglu_ragged(cuda_lib, rows, f):
     from causal_trainer_dev_b200.ops import elementwise as E
 
