@@ -317,11 +317,12 @@ __global__ void rope_kernel(__nv_bfloat16* __restrict__ x, const float* __restri
 // The same on 16-byte vectors: a warp owns a token, a lane keeps the cos / sin of its channels in
 // registers and walks the heads, so the table is read once per token instead of once per head and
 // the projection moves in whole 128-byte segments.  Bound by reading and writing the rotated heads once.
+// Where there are too few tokens to fill the GPU, 2^share warps share the heads of a token.
 //   gpt-neox: a lane holds channels [8 p, 8 p + 8) of both halves;  gpt-j: four adjacent pairs.
-template <int STYLE>
+template <int STYLE, bool SHARED>
 __global__ void __launch_bounds__(256)
 rope_vec_kernel(__nv_bfloat16* __restrict__ x, const float* __restrict__ cosv, const float* __restrict__ sinv,
-                long row_stride, int T, int heads, int D, int rot, float sign) {
+                long row_stride, int T, int heads, int D, int rot, float sign, int share) {
   constexpr int N = STYLE == 0 ? 4 : 8;          // angles per lane
   const int half = rot / 2;
   const int per_head = half / N;                 // lanes per head (<= 32)
@@ -329,8 +330,11 @@ rope_vec_kernel(__nv_bfloat16* __restrict__ x, const float* __restrict__ cosv, c
   const int together = 32 / per_head;            // heads a warp rotates at once
   const int p = lane % per_head, first = lane / per_head;
   if (first >= together) return;
-  const long warps = (static_cast<long>(gridDim.x) * blockDim.x) >> 5;
-  for (long t = (static_cast<long>(blockIdx.x) * blockDim.x + threadIdx.x) >> 5; t < T; t += warps) {
+  if (!SHARED) share = 0;
+  const long warps = ((static_cast<long>(gridDim.x) * blockDim.x) >> 5) >> share;
+  const long warp = (static_cast<long>(blockIdx.x) * blockDim.x + threadIdx.x) >> 5;
+  const int stride = together << share, h0 = first + (static_cast<int>(warp) & ((1 << share) - 1)) * together;
+  for (long t = warp >> share; t < T; t += warps) {
     float c[N], s[N];
 #pragma unroll
     for (int e = 0; e < N; e += 4) {
@@ -341,7 +345,7 @@ rope_vec_kernel(__nv_bfloat16* __restrict__ x, const float* __restrict__ cosv, c
     for (int e = 0; e < N; ++e) s[e] *= sign;
     __nv_bfloat16* row = x + t * row_stride + 8 * p;
 #pragma unroll 4
-    for (int h = first; h < heads; h += together) {
+    for (int h = h0; h < heads; h += stride) {
       uint4* at = reinterpret_cast<uint4*>(row + static_cast<long>(h) * D);
       float a[8], b[8], o[8];
       unpack8(at[0], a);
@@ -1087,14 +1091,22 @@ CTB_API int ctb_rope_table(const int* pos, const float* inv_freq, float* cosv, f
 CTB_API int ctb_rope(void* x, const float* cosv, const float* sinv, long row_stride, int T, int heads, int D, int rot,
                      int style, int inverse, void* stream) {
   if (rot % 2 || rot > D) return fail("rope: rotary_dim must be even and <= head_dim");
-  // whole 16-byte vectors per lane: 8 channels of each half (gpt-neox) or 4 pairs (gpt-j), at most 32 lanes a head
+  // Whole 16-byte vectors per lane: 8 channels of each half (gpt-neox) or 4 pairs (gpt-j), at most 32 lanes a head.
+  // A warp with fewer than 8 lanes in use, or fewer than 10000 vectors in all, is no faster than a thread per pair (us,
+  // pair and vector: 8192 tokens, 4 lanes of a warp 3.2 and 4.0; 2048 tokens, 8 lanes 2.7 and 2.4; 64 tokens, 24 lanes
+  // 1.9 and 1.9; 333 tokens, 4 heads of 128 2.2 and 2.0).
   const int angles = style == 0 ? 4 : 8;
   const int per_head = rot / 2 / angles;
-  if (rot % (2 * angles) == 0 && per_head >= 1 && per_head <= 32 && D % 8 == 0 && row_stride % 8 == 0 && T > 0 &&
+  if (rot % (2 * angles) == 0 && per_head >= 1 && per_head <= 32 && D % 8 == 0 && row_stride % 8 == 0 &&
+      heads * per_head >= 8 && static_cast<long>(T) * heads * per_head >= 10000 &&
       (reinterpret_cast<uintptr_t>(x) | reinterpret_cast<uintptr_t>(cosv) | reinterpret_cast<uintptr_t>(sinv)) % 16 == 0) {
-    auto kern = style == 0 ? rope_vec_kernel<0> : rope_vec_kernel<1>;
-    kern<<<grid_for(static_cast<long>(T) * 32, 256), 256, 0, static_cast<cudaStream_t>(stream)>>>(
-        static_cast<__nv_bfloat16*>(x), cosv, sinv, row_stride, T, heads, D, rot, inverse ? -1.f : 1.f);
+    const int together = 32 / per_head, walk = (heads + together - 1) / together;
+    int share = 0;                 // at most the eight warps of a block (333 tokens, 40 heads of 128: 5.9 us alone, 3.1)
+    while (share < 3 && (2 << share) <= walk && (static_cast<long>(T) << share) < sm_count() * 8l) ++share;
+    auto kern = style == 0 ? (share ? rope_vec_kernel<0, true> : rope_vec_kernel<0, false>)
+                           : (share ? rope_vec_kernel<1, true> : rope_vec_kernel<1, false>);
+    kern<<<grid_for((static_cast<long>(T) << share) * 32, 256), 256, 0, static_cast<cudaStream_t>(stream)>>>(
+        static_cast<__nv_bfloat16*>(x), cosv, sinv, row_stride, T, heads, D, rot, inverse ? -1.f : 1.f, share);
     CTB_CUDA_OK(cudaGetLastError());
     return 0;
   }

@@ -98,10 +98,12 @@ def test_attention_backward_statistics(cuda_lib, d, shape):
 # ------------------------------------------------------------------------------ memory-bound kernels
 @pytest.mark.parametrize("style", ["gpt-neox", "gpt-j"])
 @pytest.mark.parametrize("d,rot", [(128, 128), (64, 64), (128, 32), (128, 48), (80, 40), (128, 8), (128, 4)])
-def test_rope_of_whole_and_partial_vectors(cuda_lib, style, d, rot):
+@pytest.mark.parametrize("t,heads", [(37, 5), (2051, 5), (601, 29), (16500, 1)])
+def test_rope_of_whole_and_partial_vectors(cuda_lib, style, d, rot, t, heads):
+    """A thread per pair for few vectors, lanes that walk the heads of a token for many, and warps that share a token's
+    heads where there are few tokens."""
     from causal_trainer_dev_b200.ops import elementwise as E
 
-    t, heads = 37, 5
     x = _bf16(t, (heads + 1) * d, seed=3)
     pos = torch.randint(0, 5000, (t,), device="cuda")
     cos, sin = E.rope_table(pos, E.inverse_frequencies(rot, 1e4, device="cuda"))
