@@ -1092,13 +1092,14 @@ CTB_API int ctb_rope(void* x, const float* cosv, const float* sinv, long row_str
                      int style, int inverse, void* stream) {
   if (rot % 2 || rot > D) return fail("rope: rotary_dim must be even and <= head_dim");
   // Whole 16-byte vectors per lane: 8 channels of each half (gpt-neox) or 4 pairs (gpt-j), at most 32 lanes a head.
-  // A warp with fewer than 8 lanes in use, or fewer than 10000 vectors in all, is no faster than a thread per pair (us,
-  // pair and vector: 8192 tokens, 4 lanes of a warp 3.2 and 4.0; 2048 tokens, 8 lanes 2.7 and 2.4; 64 tokens, 24 lanes
-  // 1.9 and 1.9; 333 tokens, 4 heads of 128 2.2 and 2.0).
+  // A warp with fewer than 8 lanes in use, or fewer than 10000 vectors in all (16384 where a walk over the heads is
+  // long for the number of tokens), is no faster than a thread per pair (us, pair and vector: 8192 tokens, 4 lanes of a warp
+  // 3.2 and 4.0; 2048 tokens, 8 lanes 2.7 and 2.4; 333 tokens, 4 heads of 128 2.2 and 2.0; 128 tokens, 10 heads of 128 2.3 and
+  // 2.5, 40 heads 3.7 and 2.6).
   const int angles = style == 0 ? 4 : 8;
   const int per_head = rot / 2 / angles;
   if (rot % (2 * angles) == 0 && per_head >= 1 && per_head <= 32 && D % 8 == 0 && row_stride % 8 == 0 &&
-      heads * per_head >= 8 && static_cast<long>(T) * heads * per_head >= 10000 &&
+      heads * per_head >= 8 && static_cast<long>(T) * heads * per_head >= (T < 256 ? 16384 : 10000) &&
       (reinterpret_cast<uintptr_t>(x) | reinterpret_cast<uintptr_t>(cosv) | reinterpret_cast<uintptr_t>(sinv)) % 16 == 0) {
     const int together = 32 / per_head, walk = (heads + together - 1) / together;
     int share = 0;                 // at most the eight warps of a block (333 tokens, 40 heads of 128: 5.9 us alone, 3.1)
