@@ -328,6 +328,10 @@ __global__ void embed_push_kernel(const int* __restrict__ ids, const __nv_bfloat
 // are added in warp order, so the result does not depend on timing.  Finding the runs here instead of in a
 // list spares the host a read back of their number.  With one CTA walking a run row by row, 4 bytes per
 // load, 4000 repeats of one token were a chain of 4000 loads (968 us of a step).
+// Bound by memory latency where runs are short: the ids and sources of the 8 positions and of the 23 behind them come in
+// one load per lane, begins, lengths and sources of the runs are votes and shuffles, and the gradient row is requested
+// with the first rows of the run.  With the positions tried one after the other, each a chain of loads, 8192 tokens of a
+// 1536-wide table took 41 us for ids that occur once or twice and 32 for runs of 12; now 19 and 19.
 constexpr int LONG_RUN = 16;
 constexpr int EMB_WARPS = 8;
 template <int V> struct EmbRaw;
@@ -339,78 +343,115 @@ embedding_backward_kernel(const int* __restrict__ sorted_ids, const int* __restr
                           const __nv_bfloat16* __restrict__ dout, G* __restrict__ grad, int d, int vocab_lo,
                           int vocab_rows, int pad_id) {
   using Raw = typename EmbRaw<V>::T;
+  constexpr unsigned ALL = 0xffffffffu;
   __shared__ float part[EMB_WARPS][32 * V];
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   const int c = (blockIdx.y * 32 + lane) * V;
   const bool live = c < d;
-  // acc += rows perm[s0], perm[s0 + step], ... of dout, eight loads in flight
-  auto gather = [&](int s0, int s1, int step, float (&acc)[V]) {
+  const __nv_bfloat16* src = dout + (live ? c : 0);
+  auto add = [&](const Raw& raw, float (&acc)[V]) {
+    const __nv_bfloat162* h = reinterpret_cast<const __nv_bfloat162*>(&raw);
+#pragma unroll
+    for (int e = 0; e < V / 2; ++e) {
+      const float2 f = __bfloat1622float2(h[e]);
+      acc[2 * e] += f.x;
+      acc[2 * e + 1] += f.y;
+    }
+  };
+  // this thread's columns of a gradient row, moved as whole 16-byte vectors where V = 8 (the launcher checks)
+  constexpr int WORDS = V * static_cast<int>(sizeof(G)) / 4;
+  auto row_at = [&](int local) { return grad + static_cast<long>(local) * d + c; };
+  auto load_row = [&](const G* g, uint32_t (&w)[WORDS]) {
+    if constexpr (WORDS % 4 == 0) {
+#pragma unroll
+      for (int i = 0; i < WORDS; i += 4) *reinterpret_cast<uint4*>(w + i) = *reinterpret_cast<const uint4*>(reinterpret_cast<const uint32_t*>(g) + i);
+    } else {
+#pragma unroll
+      for (int e = 0; e < V; ++e) reinterpret_cast<G*>(w)[e] = g[e];
+    }
+  };
+  auto add_row = [&](G* g, uint32_t (&w)[WORDS], const float (&acc)[V]) {
+    G* v = reinterpret_cast<G*>(w);
+#pragma unroll
+    for (int e = 0; e < V; ++e) v[e] = static_cast<G>(static_cast<float>(v[e]) + acc[e]);
+    if constexpr (WORDS % 4 == 0) {
+#pragma unroll
+      for (int i = 0; i < WORDS; i += 4) *reinterpret_cast<uint4*>(reinterpret_cast<uint32_t*>(g) + i) = *reinterpret_cast<const uint4*>(w + i);
+    } else {
+#pragma unroll
+      for (int e = 0; e < V; ++e) g[e] = v[e];
+    }
+  };
+  // lane l: position first - 1 + l.  Lanes 1 to 8 are the positions of this CTA
+  const int first = blockIdx.x * EMB_WARPS, p = first - 1 + lane;
+  const bool in = p >= 0 && p < tokens;
+  const int id = in ? __ldg(sorted_ids + p) : 0, from = in ? __ldg(perm + p) : 0;
+  const int before = __shfl_up_sync(ALL, id, 1), beyond = __shfl_down_sync(ALL, id, LONG_RUN);
+  const bool begins = in && lane >= 1 && lane <= EMB_WARPS && (p == 0 || before != id) && id != pad_id &&
+                      id >= vocab_lo && id - vocab_lo < vocab_rows;
+  const unsigned starts = __ballot_sync(ALL, begins);
+  const unsigned longs = __ballot_sync(ALL, begins && p + LONG_RUN < tokens && beyond == id);
+  if (((starts & ~longs) >> (warp + 1)) & 1u) {                  // (uniform in the warp)
+    const int mine = __shfl_sync(ALL, id, warp + 1);
+    const int n = __popc(__ballot_sync(ALL, in && id == mine));  // 1 to LONG_RUN, all of them in the window
+    G* g = row_at(mine - vocab_lo);
+    uint32_t old[WORDS];
+    if (live) load_row(g, old);
+    float acc[V];
+#pragma unroll
+    for (int e = 0; e < V; ++e) acc[e] = 0.f;
     constexpr int U = 8;
-    for (int s = s0; s < s1; s += U * step) {
+    for (int j = 0; j < n; j += U) {
+      Raw raw[U];
+#pragma unroll
+      for (int k = 0; k < U; ++k) {
+        const int row = __shfl_sync(ALL, from, warp + 1 + j + k);
+        if (j + k < n) raw[k] = __ldg(reinterpret_cast<const Raw*>(src + static_cast<long>(row) * d));
+      }
+#pragma unroll
+      for (int k = 0; k < U; ++k)
+        if (j + k < n) add(raw[k], acc);
+    }
+    if (live) add_row(g, old, acc);
+  }
+  for (unsigned left = longs; left != 0u; left &= left - 1u) {   // (uniform in the CTA: every warp holds the same window)
+    const int at = __ffs(left) - 1, mine = __shfl_sync(ALL, id, at), s0 = first - 1 + at;
+    int s1 = s0 + LONG_RUN + 1, hi = tokens;                     // first position past the run, by bisection
+    while (s1 < hi) {
+      const int mid = s1 + (hi - s1) / 2;
+      if (__ldg(sorted_ids + mid) == mine) s1 = mid + 1;
+      else hi = mid;
+    }
+    float acc[V];
+#pragma unroll
+    for (int e = 0; e < V; ++e) acc[e] = 0.f;
+    constexpr int U = 8;                                         // rows in flight; every eighth row of the run is this warp's
+    for (int s = s0 + warp; s < s1; s += U * EMB_WARPS) {
       Raw raw[U];
 #pragma unroll
       for (int k = 0; k < U; ++k) {
         // past the end: the run's last row again, not added (unconditional loads stay in flight together)
-        const int at = min(s + k * step, s1 - 1);
-        raw[k] = __ldg(reinterpret_cast<const Raw*>(dout + static_cast<long>(__ldg(perm + at)) * d + (live ? c : 0)));
+        const int row = __ldg(perm + min(s + k * EMB_WARPS, s1 - 1));
+        raw[k] = __ldg(reinterpret_cast<const Raw*>(src + static_cast<long>(row) * d));
       }
 #pragma unroll
-      for (int k = 0; k < U; ++k) {
-        if (s + k * step < s1) {
-          const __nv_bfloat162* h = reinterpret_cast<const __nv_bfloat162*>(&raw[k]);
-#pragma unroll
-          for (int e = 0; e < V / 2; ++e) {
-            const float2 f = __bfloat1622float2(h[e]);
-            acc[2 * e] += f.x;
-            acc[2 * e + 1] += f.y;
-          }
-        }
-      }
+      for (int k = 0; k < U; ++k)
+        if (s + k * EMB_WARPS < s1) add(raw[k], acc);
     }
-  };
-  auto add_row = [&](int local, const float (&acc)[V]) {
-    G* g = grad + static_cast<long>(local) * d + c;
 #pragma unroll
-    for (int e = 0; e < V; ++e) g[e] = static_cast<G>(static_cast<float>(g[e]) + acc[e]);
-  };
-  for (int first = blockIdx.x * EMB_WARPS; first < tokens; first += gridDim.x * EMB_WARPS) {
-    for (int k = 0; k < EMB_WARPS && first + k < tokens; ++k) {       // (uniform over the CTA up to `shared_run`)
-      const int s0 = first + k;
-      const int id = __ldg(sorted_ids + s0), local = id - vocab_lo;
-      if (s0 > 0 && __ldg(sorted_ids + s0 - 1) == id) continue;
-      if (id == pad_id || local < 0 || local >= vocab_rows) continue;
-      const bool shared_run = s0 + LONG_RUN < tokens && __ldg(sorted_ids + s0 + LONG_RUN) == id;
-      if (!shared_run && k != warp) continue;
-      int s1 = s0 + 1;
-      float acc[V];
-#pragma unroll
-      for (int e = 0; e < V; ++e) acc[e] = 0.f;
-      if (!shared_run) {
-        while (s1 < tokens && __ldg(sorted_ids + s1) == id) ++s1;
-        gather(s0, s1, 1, acc);
-        if (live) add_row(local, acc);
-        continue;
-      }
-      int hi = tokens;                     // first position past the run, by bisection
-      s1 = s0 + LONG_RUN + 1;
-      while (s1 < hi) {
-        const int mid = s1 + (hi - s1) / 2;
-        if (__ldg(sorted_ids + mid) == id) s1 = mid + 1;
-        else hi = mid;
-      }
-      gather(s0 + warp, s1, EMB_WARPS, acc);
-#pragma unroll
-      for (int e = 0; e < V; ++e) part[warp][e * 32 + lane] = acc[e];
-      __syncthreads();
-      if (warp == 0 && live) {
+    for (int e = 0; e < V; ++e) part[warp][e * 32 + lane] = acc[e];
+    __syncthreads();
+    if (warp == 0 && live) {
 #pragma unroll 1
-        for (int w = 1; w < EMB_WARPS; ++w)
+      for (int w = 1; w < EMB_WARPS; ++w)
 #pragma unroll
-          for (int e = 0; e < V; ++e) acc[e] += part[w][e * 32 + lane];
-        add_row(local, acc);
-      }
-      __syncthreads();
+        for (int e = 0; e < V; ++e) acc[e] += part[w][e * 32 + lane];
+      G* g = row_at(mine - vocab_lo);
+      uint32_t old[WORDS];
+      load_row(g, old);
+      add_row(g, old, acc);
     }
+    __syncthreads();
   }
 }
 
@@ -497,11 +538,11 @@ CTB_API int ctb_embedding_backward(const int* sorted_ids, const int* perm, long 
   cudaStream_t s = static_cast<cudaStream_t>(stream);
   const auto* src = static_cast<const __nv_bfloat16*>(dout);
   const int n = static_cast<int>(tokens);
-  const bool wide = d % 8 == 0 && reinterpret_cast<uintptr_t>(dout) % 16 == 0;     // whole 16-byte vectors
+  // whole 16-byte vectors of dout and of the table
+  const bool wide = d % 8 == 0 && (reinterpret_cast<uintptr_t>(dout) | reinterpret_cast<uintptr_t>(grad)) % 16 == 0;
   const int width = wide ? 256 : 64, chunks = (d + width - 1) / width;
   if (chunks > 65535) return fail("embedding_backward: hidden size too large");
-  const int blocks = (n + EMB_WARPS - 1) / EMB_WARPS, cap = (148 * 32 + chunks - 1) / chunks;
-  const dim3 grid(static_cast<unsigned>(blocks < cap ? blocks : cap), static_cast<unsigned>(chunks));
+  const dim3 grid(static_cast<unsigned>((n + EMB_WARPS - 1) / EMB_WARPS), static_cast<unsigned>(chunks));
 #define CTB_EMB(G, V)                                                                                          \
   embedding_backward_kernel<G, V><<<grid, EMB_WARPS * 32, 0, s>>>(sorted_ids, perm, n, src, static_cast<G*>(grad), d, \
                                                                   vocab_lo, vocab_rows, pad_id)
