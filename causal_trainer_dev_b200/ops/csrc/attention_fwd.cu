@@ -59,13 +59,20 @@ struct FwdSmem {
   static constexpr int BYTES = OFF_BAR + 256 + 1024;
 };
 
-template <int D>
+// SPARSE: the key tiles come from a routing list.  Nearly every warp then has rows that do not see a tile, so that
+// kernel has no second copy of the exponentials for wholly visible ones; in one kernel with the dense walk the two
+// copies cost it up to 12 % of its time at D = 64 (8192 tokens, 8 heads, block 1024: 184 us, apart 140).
+template <int D, bool SPARSE>
 __global__ void __launch_bounds__(FWD_THREADS, 1)
 attn_fwd_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constant__ CUtensorMap map_k,
                 const __grid_constant__ CUtensorMap map_v, const __grid_constant__ CUtensorMap map_o,
                 const FwdArgs args) {
   using L = FwdSmem<D>;
   constexpr int HALVES = L::HALVES;
+  // P published in two halves, except where the rows of a warp see different key tiles and the products are
+  // short: there the softmax alone is the longer side (SPARSE, D = 64: 16384 tokens, 4 heads, block 512 299 us
+  // against 331)
+  constexpr bool HALVED = !(SPARSE && D == 64);
   extern __shared__ uint8_t smem_raw[];
   uint8_t* smem = smem_raw + ((1024u - (smem_u32(smem_raw) & 1023u)) & 1023u);
   uint64_t* q_full = reinterpret_cast<uint64_t*>(smem + L::OFF_BAR);
@@ -125,7 +132,7 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constant
   int n1 = (hi_t[1] > lo_t[1]) ? hi_t[1] - lo : 0;
   // Block-sparse routing: both query tiles walk the listed key tiles (rows that selected nothing in
   // a tile see it fully masked).
-  const bool sparse = args.sp.it_list != nullptr;
+  constexpr bool sparse = SPARSE;
   const int* kv_list = nullptr;
   if (sparse) {
     int base, cnt;
@@ -447,15 +454,18 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constant
             pw[jj] = pack_bf16(pa, pb);
           }
           tmem_st8(tmem_s_of(t) + lane_off + qt * 8, pw);
-          if (qt % 4 == 3) {
+          if (qt == 7 || (qt == 3 && HALVED)) {
             tmem_st_wait();
             tc_fence_before();
             __syncwarp();
-            if (lane == 0) mbar_arrive(&p_full[2 * t + qt / 4]);
+            if (lane == 0) {
+              if (!HALVED) mbar_arrive(&p_full[2 * t]);
+              mbar_arrive(&p_full[2 * t + qt / 4]);
+            }
           }
         }
       };
-      if (__all_sync(0xffffffffu, all && m_ref > -INFINITY)) exponentials(std::true_type{});
+      if (!SPARSE && __all_sync(0xffffffffu, all && m_ref > -INFINITY)) exponentials(std::true_type{});
       else exponentials(std::false_type{});
       float rs_a, rs_b;
       unpack_f32x2(rs2, rs_a, rs_b);
@@ -510,8 +520,8 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constant
   }
 }
 
-template <int D>
-int launch_fwd(const FwdCall& c) {
+template <int D, bool SPARSE>
+int launch_fwd_as(const FwdCall& c) {
   using L = FwdSmem<D>;
   const bool grouped = c.grp.desc != nullptr;
   const int Sq = grouped ? c.gathered_rows : (c.Sq > 0 ? c.Sq : c.S);
@@ -545,7 +555,7 @@ int launch_fwd(const FwdCall& c) {
   a.kvf = c.kvf;
   a.status = device_status();
   a.spin_budget = c.spin_budget > 0 ? c.spin_budget : CTB_SPIN_BUDGET;
-  auto kern = attn_fwd_kernel<D>;
+  auto kern = attn_fwd_kernel<D, SPARSE>;
   static int configured_dev = -1;
   int dev = 0;
   cudaGetDevice(&dev);
@@ -557,6 +567,11 @@ int launch_fwd(const FwdCall& c) {
   kern<<<grid, FWD_THREADS, L::BYTES, static_cast<cudaStream_t>(c.stream)>>>(*mq, *mk, *mv, *mo, a);
   CTB_CUDA_OK(cudaGetLastError());
   return 0;
+}
+
+template <int D>
+int launch_fwd(const FwdCall& c) {
+  return c.sp.it_list != nullptr ? launch_fwd_as<D, true>(c) : launch_fwd_as<D, false>(c);
 }
 
 }  // namespace attn
