@@ -58,7 +58,6 @@ moba_pool_kernel(const __nv_bfloat16* __restrict__ k, long k_row_stride, const i
 #pragma unroll
   for (int e = 0; e < 8; ++e) acc[e] = 0.f;
   const __nv_bfloat16* base = k + (static_cast<size_t>(b) * S + p) * k_row_stride + static_cast<size_t>(hkv) * D + v * 8;
-#pragma unroll 16                                // (64 CTAs with work at 32768 tokens: loads in flight are what counts)
   for (int r = rg; r < block; r += ROWS) {
     const uint4 raw = *reinterpret_cast<const uint4*>(base + static_cast<size_t>(r) * k_row_stride);
     const __nv_bfloat162* h2 = reinterpret_cast<const __nv_bfloat162*>(&raw);
