@@ -235,6 +235,28 @@ def test_embedding_gradient_of_long_and_short_runs(cuda_lib, d, dtype):
     assert torch.equal(first, again)
 
 
+@pytest.mark.parametrize("tokens", [1, 7, 8, 9, 16, 17, 18, 24, 25, 33, 100])
+@pytest.mark.parametrize("kind", ["one", "distinct", "pairs", "tail"])
+def test_embedding_gradient_at_the_ends_of_a_block(cuda_lib, tokens, kind):
+    """Runs that end with the tokens, fill a block of 8 positions or cross into the next; and a table whose base is not
+    16-byte aligned, which the kernel takes two columns at a time."""
+    from causal_trainer_dev_b200.ops import elementwise as E
+
+    at = torch.arange(tokens, device="cuda")
+    ids = {"one": at * 0 + 3, "distinct": at, "pairs": at // 2, "tail": (at - (tokens - 17)).clamp(max=0) + 20}[kind]
+    ids = ids[torch.randperm(tokens, generator=torch.Generator(device="cuda").manual_seed(2), device="cuda")]
+    keep = (ids >= 1) & (ids < 65)
+    dout = _bf16(tokens, 40, seed=1)
+    for offset in (0, 4):
+        flat = _bf16(64 * 40 + offset, seed=2)
+        grad = flat[offset:].view(64, 40)
+        want = grad.double()
+        want.index_add_(0, ids[keep] - 1, dout[keep].double())
+        E.embedding_backward(ids, dout, grad, -1, 1)
+        assert _rel(grad, want) < BF16
+        assert torch.equal(flat[:offset], _bf16(64 * 40 + offset, seed=2)[:offset])
+
+
 # ------------------------------------------------------------------------------ split-K products
 @pytest.mark.parametrize("m,n,k", [(1, 8, 2048), (128, 256, 1024), (129, 264, 4104), (70, 130, 9000), (333, 1536, 8200),
                                    (64, 1000, 640), (500, 96, 5000), (1000, 1536, 3000)])
