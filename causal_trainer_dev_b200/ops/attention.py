@@ -14,7 +14,6 @@ Reference counterparts: ``vanilla_attention`` (src/causal_trainer/modeling/atten
 """
 from __future__ import annotations
 
-import ctypes
 import math
 from dataclasses import dataclass
 
@@ -170,10 +169,15 @@ def vanilla_attention(
 
 def _row_stride(t: torch.Tensor) -> int:
     # [B,S,H,D] view: D contiguous, heads D apart, batches S rows apart.
-    b, s, h, d = t.shape
-    if t.stride(3) != 1 or t.stride(2) != d or (b > 1 and t.stride(0) != t.stride(1) * s):
+    b, s, _, d = t.shape
+    batch, row, head, channel = t.stride()
+    if channel != 1 or head != d or (b > 1 and batch != row * s):
         raise ValueError("attention operands must be [B,S,H,D] views with contiguous heads")
-    return t.stride(1)
+    return row
+
+
+def _at(t: torch.Tensor | None) -> int | None:
+    return None if t is None else t.data_ptr()
 
 
 def flash_attention_forward(
@@ -196,17 +200,16 @@ def flash_attention_forward(
     if out is None:
         out = torch.empty((b, sq, hq, d), dtype=torch.bfloat16, device=q.device)
     lse = torch.empty((b, hq, sq), dtype=torch.float32, device=q.device)
-    common = (_lib.ptr(q), _lib.ptr(k), _lib.ptr(v), _lib.ptr(out), _lib.ptr(lse), _lib.ptr(meta.seg), _lib.ptr(meta.lim),
-              _lib.ptr(meta.start), _lib.ptr(meta.kv_lo), _lib.ptr(meta.kv_hi),
-              b, s, sq, q_offset, hq, hkv, d, ctypes.c_long(_row_stride(q)), ctypes.c_long(_row_stride(k)),
-              ctypes.c_long(_row_stride(v)), ctypes.c_long(_row_stride(out)), ctypes.c_float(scale))
+    common = (q.data_ptr(), k.data_ptr(), v.data_ptr(), out.data_ptr(), lse.data_ptr(), meta.seg.data_ptr(), _at(meta.lim),
+              _at(meta.start), meta.kv_lo.data_ptr(), meta.kv_hi.data_ptr(), b, s, sq, q_offset, hq, hkv, d,
+              _row_stride(q), _row_stride(k), _row_stride(v), _row_stride(out), float(scale))
     if kv_flags is None:
-        code = _lib.lib().ctb_attn_fwd_range(*common, ctypes.c_longlong(spin_budget), _lib.stream_ptr())
+        code = _lib.lib().ctb_attn_fwd_range(*common, spin_budget, _lib.raw_stream())
         _lib.check(code, "ctb_attn_fwd_range")
     else:
         flags, chunk, row_elems, epoch = kv_flags
-        code = _lib.lib().ctb_attn_fwd_gathered(*common, _lib.ptr(flags), ctypes.c_long(chunk), ctypes.c_long(row_elems),
-                                                ctypes.c_uint(epoch), ctypes.c_longlong(spin_budget), _lib.stream_ptr())
+        code = _lib.lib().ctb_attn_fwd_gathered(*common, flags.data_ptr(), chunk, row_elems, epoch, spin_budget,
+                                                _lib.raw_stream())
         _lib.check(code, "ctb_attn_fwd_gathered")
     return out, lse
 
@@ -217,7 +220,7 @@ def flash_attention_backward(
     dq: torch.Tensor | None = None, dk: torch.Tensor | None = None, dv: torch.Tensor | None = None,
     q_offset: int = 0, stats: tuple[torch.Tensor, torch.Tensor] | None = None,
 ) -> tuple[torch.Tensor, torch.Tensor, torch.Tensor]:
-    """dQ (query-tile-owned kernel) and dK/dV (key-tile-owned kernel, group reduced in TMEM).
+    """dQ (query-tile-owned work items) and dK/dV (key-tile-owned ones, group reduced in TMEM), in one launch.
 
     With a query range (``q_offset``, ``Sq < S``) dK / dV are this rank's partial sums over its
     queries, for all ``S`` keys.
@@ -226,26 +229,25 @@ def flash_attention_backward(
     s = k.shape[1]
     hkv = k.shape[2]
     scale = 1.0 / math.sqrt(d) if scale is None else scale
-    from .elementwise import attention_backward_stats
-
-    _row_stride(out), _row_stride(dout)
-    # [B,Hq,Sq] fp32; a caller that splits one softmax over several passes hands in the shared ones
-    neg_lse2, neg_delta = attention_backward_stats(out, dout, lse) if stats is None else stats
+    out_stride, dout_stride = _row_stride(out), _row_stride(dout)
+    # [B,Hq,Sq] fp32 each; a caller that splits one softmax over several passes hands in the shared ones
+    if stats is None:
+        both = torch.empty(2 * b * hq * sq, dtype=torch.float32, device=q.device)
+        neg_lse2 = both.data_ptr()
+        neg_delta = neg_lse2 + 4 * b * hq * sq
+    else:
+        neg_lse2, neg_delta = stats[0].data_ptr(), stats[1].data_ptr()
     dq = torch.empty((b, sq, hq, d), dtype=torch.bfloat16, device=q.device) if dq is None else dq
     dk = torch.empty((b, s, hkv, d), dtype=torch.bfloat16, device=q.device) if dk is None else dk
     dv = torch.empty((b, s, hkv, d), dtype=torch.bfloat16, device=q.device) if dv is None else dv
-    L = _lib.lib()
-    for mode in (0, 1):
-        code = L.ctb_attn_bwd_range(
-            mode, _lib.ptr(q), _lib.ptr(k), _lib.ptr(v), _lib.ptr(dout), _lib.ptr(dq), _lib.ptr(dk), _lib.ptr(dv),
-            _lib.ptr(neg_lse2), _lib.ptr(neg_delta), _lib.ptr(meta.seg), _lib.ptr(meta.lim), _lib.ptr(meta.kv_lo),
-            _lib.ptr(meta.kv_hi), _lib.ptr(meta.q_lo), _lib.ptr(meta.q_hi), _lib.ptr(meta.start), _lib.ptr(meta.end), _lib.ptr(meta.first_q),
-            b, s, sq, q_offset, hq, hkv, d,
-            ctypes.c_long(_row_stride(q)), ctypes.c_long(_row_stride(k)), ctypes.c_long(_row_stride(v)),
-            ctypes.c_long(_row_stride(dout)), ctypes.c_long(_row_stride(dq)), ctypes.c_long(_row_stride(dk)),
-            ctypes.c_long(_row_stride(dv)), ctypes.c_float(scale), ctypes.c_longlong(spin_budget), _lib.stream_ptr(),
-        )
-        _lib.check(code, "ctb_attn_bwd_range")
+    code = _lib.lib().ctb_attn_bwd_range(
+        q.data_ptr(), k.data_ptr(), v.data_ptr(), out.data_ptr() if stats is None else None, dout.data_ptr(), lse.data_ptr(),
+        dq.data_ptr(), dk.data_ptr(), dv.data_ptr(), neg_lse2, neg_delta, meta.seg.data_ptr(),
+        _at(meta.lim), meta.kv_lo.data_ptr(), meta.kv_hi.data_ptr(), meta.q_lo.data_ptr(), meta.q_hi.data_ptr(),
+        _at(meta.start), _at(meta.end), _at(meta.first_q), b, s, sq, q_offset, hq, hkv, d, _row_stride(q), _row_stride(k),
+        _row_stride(v), out_stride, dout_stride, _row_stride(dq), _row_stride(dk), _row_stride(dv), float(scale), spin_budget,
+        _lib.raw_stream())
+    _lib.check(code, "ctb_attn_bwd_range", 1 if stats is not None else 2)
     return dq, dk, dv
 
 

@@ -2,6 +2,10 @@
 #pragma once
 #include "host_common.h"
 
+// elementwise.cu
+CTB_API int ctb_attn_bwd_stats(const void* o, const void* dout, const float* lse, float* neg_lse2, float* neg_delta, int B,
+                               int S, int H, int D, long o_rs, long do_rs, void* stream);
+
 namespace ctb {
 namespace attn {
 

@@ -1,4 +1,4 @@
-// Flash attention backward for sm_100a, two kernels from one template, no atomics:
+// Flash attention backward for sm_100a, two kinds of work items from one template, no atomics:
 //
 //   MODE_DKV  KV-tile-owned: a CTA owns 128 keys of one KV head and walks the 64-row query blocks
 //             of every query head of the GQA group that can see them, two blocks per iteration.
@@ -78,12 +78,13 @@ struct BwdSmem {
   static constexpr int S_BUFS_DQ = 2;
 };
 
+struct BwdMaps {
+  CUtensorMap q, k, v, dout, out1, out2;     // out1: dV (DKV) or dQ (DQ), out2: dK (DKV)
+};
+
+// Work item `cta` of one mode.
 template <int D, int MODE>
-__global__ void __launch_bounds__(BWD_THREADS, 1)
-attn_bwd_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constant__ CUtensorMap map_k,
-                const __grid_constant__ CUtensorMap map_v, const __grid_constant__ CUtensorMap map_do,
-                const __grid_constant__ CUtensorMap map_out1, const __grid_constant__ CUtensorMap map_out2,
-                const BwdArgs args) {
+__device__ __forceinline__ void bwd_cta(const BwdMaps& maps, const BwdArgs& args, const int cta) {
   using L = BwdSmem<D>;
   constexpr int HALVES = L::HALVES;
   constexpr bool DKV = (MODE == MODE_DKV);
@@ -119,17 +120,17 @@ attn_bwd_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constant
   const bool grouped = args.grp.desc != nullptr;
   int4 gd = make_int4(0, 0, 0, 0);
   if (grouped) {
-    gd = __ldg(args.grp.desc + blockIdx.x);
+    gd = __ldg(args.grp.desc + cta);
     if (gd.w <= 0) return;                       // unused capacity: the whole CTA leaves
   }
-  int idx = blockIdx.x;
+  int idx = cta;
   int b, head, x0, y_lo64, y_n64, heads_in_loop;
   if (grouped) {
     // X = this CTA's resident tile: 128 keys of the block (dK/dV) or 128 gathered rows (dQ);
     // Y = 64-row blocks of the group's gathered rows (dK/dV) or of the block's keys (dQ).
     b = DKV ? (gd.x & 0xffff) : 0;
     head = DKV ? (gd.x >> 16) : 0;
-    x0 = DKV ? gd.y : static_cast<int>(blockIdx.x) * 128;
+    x0 = DKV ? gd.y : cta * 128;
     y_lo64 = 0;
     y_n64 = DKV ? gd.w / 64 : args.grp.block / 64;
     heads_in_loop = 1;
@@ -166,7 +167,7 @@ attn_bwd_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constant
   const int* it_list = nullptr;
   if (sparse) {
     int base;
-    sparse_list(args.sp, blockIdx.x, base, n_entry);
+    sparse_list(args.sp, cta, base, n_entry);
     it_list = args.sp.it_list + base;
   }
   const int n_iter = (n_entry + 1) / 2;
@@ -203,8 +204,8 @@ attn_bwd_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constant
       // the resident tiles are on their way while TMEM is allocated (with Q in the forward kernel, a layer's forward
       // and backward: 8.00 -> 7.77 ms on one document of 32768 tokens, 1096 -> 1047 us on 8 image rows of 4096)
       mbar_expect_tx(x_full, 2 * L::XT);
-      const CUtensorMap* mx1 = DKV ? &map_k : &map_q;
-      const CUtensorMap* mx2 = DKV ? &map_v : &map_do;
+      const CUtensorMap* mx1 = DKV ? &maps.k : &maps.q;
+      const CUtensorMap* mx2 = DKV ? &maps.v : &maps.dout;
       const int xh = DKV ? hkv : head;
       const int xb = DKV ? kbatch : b;
 #pragma unroll
@@ -232,8 +233,8 @@ attn_bwd_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constant
     // ------------------------------ producer ------------------------------
     if (n_iter > 0) {
       const uint32_t on = elect_one();            // the whole warp walks, one lane issues
-      const CUtensorMap* my1 = DKV ? &map_q : &map_k;
-      const CUtensorMap* my2 = DKV ? &map_do : &map_v;
+      const CUtensorMap* my1 = DKV ? &maps.q : &maps.k;
+      const CUtensorMap* my2 = DKV ? &maps.dout : &maps.v;
       uint32_t slot1 = 0, phase1 = 0;
       const int ybatch = DKV ? b * (grouped ? 0 : 1) : kbatch;
       for (int it = 0; it < n_iter; ++it) {
@@ -595,7 +596,7 @@ attn_bwd_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constant
       fence_proxy_async_smem();
       named_bar_sync(4 + u, 256);
       if (r == 0 && half == 0) {
-        const CUtensorMap* mo = (DKV && u == 1) ? &map_out2 : &map_out1;
+        const CUtensorMap* mo = (DKV && u == 1) ? &maps.out2 : &maps.out1;
         const int oh = DKV ? hkv : head;
         const int ob = DKV ? kbatch : b;
 #pragma unroll
@@ -620,8 +621,26 @@ attn_bwd_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constant
 }
 
 template <int D, int MODE>
-int launch_bwd(const BwdCall& c) {
-  using L = BwdSmem<D>;
+__global__ void __launch_bounds__(BWD_THREADS, 1)
+attn_bwd_kernel(const __grid_constant__ BwdMaps maps, const __grid_constant__ BwdArgs args) {
+  bwd_cta<D, MODE>(maps, args, static_cast<int>(blockIdx.x));
+}
+
+// Both modes in one launch: neither reads what the other writes, so the dQ work items fill the SMs that the last, long
+// dK/dV items leave idle, and a short call pays for one launch less (8 image rows of 4096 tokens, 12 / 2 heads, forward and
+// backward: 1014 -> 969 us; 2 rows of 256 tokens, with the launches' host side: 76 -> 38 us).
+template <int D>
+__global__ void __launch_bounds__(BWD_THREADS, 1)
+attn_bwd_both_kernel(const __grid_constant__ BwdMaps dkv_maps, const __grid_constant__ BwdMaps dq_maps,
+                     const __grid_constant__ BwdArgs dkv, const __grid_constant__ BwdArgs dq, const int dkv_items) {
+  const int cta = static_cast<int>(blockIdx.x);
+  if (cta < dkv_items) bwd_cta<D, MODE_DKV>(dkv_maps, dkv, cta);
+  else bwd_cta<D, MODE_DQ>(dq_maps, dq, cta - dkv_items);
+}
+
+// Maps, arguments and number of work items of one mode.
+template <int D, int MODE>
+int prepare_bwd(const BwdCall& c, BwdMaps* maps, BwdArgs* args, int* items) {
   const bool grouped = c.grp.desc != nullptr;
   const int Sq = grouped ? c.gathered_rows : (c.Sq > 0 ? c.Sq : c.S);
   auto make = [&](const void* base, int heads, long row_stride, int rows, int seq, int batches) -> const CUtensorMap* {
@@ -656,17 +675,54 @@ int launch_bwd(const BwdCall& c) {
   a.grp = c.grp;
   a.status = device_status();
   a.spin_budget = c.spin_budget > 0 ? c.spin_budget : CTB_SPIN_BUDGET;
-  auto kern = attn_bwd_kernel<D, MODE>;
-  static int configured_dev = -1;
+  *maps = BwdMaps{*mq, *mk, *mv, *mdo, *mo1, *mo2};
+  *args = a;
+  *items = grouped ? c.ctas : (DKV ? c.B * c.Hkv * (c.S / 128) : c.B * c.Hq * (Sq / 128));
+  return 0;
+}
+
+template <int D, typename Kernel>
+int configure_bwd(Kernel kern, int* configured_dev) {
   int dev = 0;
   cudaGetDevice(&dev);
-  if (configured_dev != dev) {
-    CTB_CUDA_OK(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, L::BYTES));
-    configured_dev = dev;
+  if (*configured_dev != dev) {
+    CTB_CUDA_OK(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, BwdSmem<D>::BYTES));
+    *configured_dev = dev;
   }
-  const int grid = grouped ? c.ctas : (DKV ? c.B * c.Hkv * (c.S / 128) : c.B * c.Hq * (Sq / 128));
-  if (grid <= 0) return 0;
-  kern<<<grid, BWD_THREADS, L::BYTES, static_cast<cudaStream_t>(c.stream)>>>(*mq, *mk, *mv, *mdo, *mo1, *mo2, a);
+  return 0;
+}
+
+template <int D, int MODE>
+int launch_bwd(const BwdCall& c) {
+  BwdMaps maps;
+  BwdArgs args{};
+  int items = 0;
+  if (prepare_bwd<D, MODE>(c, &maps, &args, &items)) return 1;
+  if (items <= 0) return 0;
+  auto kern = attn_bwd_kernel<D, MODE>;
+  static int configured_dev = -1;
+  if (configure_bwd<D>(kern, &configured_dev)) return 1;
+  kern<<<items, BWD_THREADS, BwdSmem<D>::BYTES, static_cast<cudaStream_t>(c.stream)>>>(maps, args);
+  CTB_CUDA_OK(cudaGetLastError());
+  return 0;
+}
+
+// dK/dV as described by `dkv` and dQ as described by `dq`, in one launch.
+template <int D>
+int launch_bwd_both(const BwdCall& dkv, const BwdCall& dq) {
+  BwdMaps dkv_maps, dq_maps;
+  BwdArgs dkv_args{}, dq_args{};
+  int dkv_items = 0, dq_items = 0;
+  if (prepare_bwd<D, MODE_DKV>(dkv, &dkv_maps, &dkv_args, &dkv_items)) return 1;
+  if (prepare_bwd<D, MODE_DQ>(dq, &dq_maps, &dq_args, &dq_items)) return 1;
+  dkv_items = max(dkv_items, 0);
+  dq_items = max(dq_items, 0);
+  if (dkv_items + dq_items == 0) return 0;
+  auto kern = attn_bwd_both_kernel<D>;
+  static int configured_dev = -1;
+  if (configure_bwd<D>(kern, &configured_dev)) return 1;
+  kern<<<dkv_items + dq_items, BWD_THREADS, BwdSmem<D>::BYTES, static_cast<cudaStream_t>(dkv.stream)>>>(
+      dkv_maps, dq_maps, dkv_args, dq_args, dkv_items);
   CTB_CUDA_OK(cudaGetLastError());
   return 0;
 }
@@ -697,17 +753,24 @@ CTB_API int ctb_attn_bwd(int mode, const void* q, const void* k, const void* v, 
   return ctb::fail("attention: head_dim must be 64 or 128");
 }
 
-// Sequence-parallel backward: q / dout / dq, neg_lse2 and neg_delta hold the Sq queries [q_off, q_off + Sq)
-// of every row; k / v / dk / dv cover all S keys (dk / dv are this rank's partial sums).
-CTB_API int ctb_attn_bwd_range(int mode, const void* q, const void* k, const void* v, const void* dout, void* dq,
-                               void* dk, void* dv, const float* neg_lse2, const float* neg_delta, const int* seg,
-                               const int* lim, const int* kv_lo, const int* kv_hi, const int* q_lo, const int* q_hi,
-                               const int* run_start, const int* run_end, const int* first_q, int B, int S, int Sq, int q_off, int Hq, int Hkv, int D,
-                               long q_rs, long k_rs, long v_rs, long do_rs, long dq_rs, long dk_rs, long dv_rs,
-                               float scale, long long spin_budget, void* stream) {
+// Whole backward of the queries [q_off, q_off + Sq) of every row (all of them: q_off 0, Sq = S): q / out / dout / dq, lse,
+// neg_lse2 and neg_delta hold those queries; k / v / dk / dv cover all S keys (with fewer queries dk / dv are partial sums).
+// The statistics are computed from out and lse first, unless out is null: then the caller hands them in.
+CTB_API int ctb_attn_bwd_range(const void* q, const void* k, const void* v, const void* out, const void* dout,
+                               const float* lse, void* dq, void* dk, void* dv, float* neg_lse2, float* neg_delta,
+                               const int* seg, const int* lim, const int* kv_lo, const int* kv_hi, const int* q_lo,
+                               const int* q_hi, const int* run_start, const int* run_end, const int* first_q, int B, int S,
+                               int Sq, int q_off, int Hq, int Hkv, int D, long q_rs, long k_rs, long v_rs, long o_rs,
+                               long do_rs, long dq_rs, long dk_rs, long dv_rs, float scale, long long spin_budget,
+                               void* stream) {
   if (S % 128 || Sq % 128 || q_off % 128 || q_off < 0 || q_off + Sq > S)
     return ctb::fail("attention: S, Sq and q_off must be multiples of 128 with q_off + Sq <= S");
   if (Hq % Hkv) return ctb::fail("attention: Hq must be a multiple of Hkv");
+  if (D != 64 && D != 128) return ctb::fail("attention: head_dim must be 64 or 128");
+  if (out != nullptr) {
+    const int rc = ctb_attn_bwd_stats(out, dout, lse, neg_lse2, neg_delta, B, Sq, Hq, D, o_rs, do_rs, stream);
+    if (rc != 0) return rc;
+  }
   ctb::attn::BwdCall c{};
   c.q = q; c.k = k; c.v = v; c.dout = dout; c.dq = dq; c.dk = dk; c.dv = dv; c.neg_lse2 = neg_lse2; c.neg_delta = neg_delta;
   c.seg = seg; c.lim = lim; c.kv_lo = kv_lo; c.kv_hi = kv_hi; c.q_lo = q_lo; c.q_hi = q_hi;
@@ -716,10 +779,7 @@ CTB_API int ctb_attn_bwd_range(int mode, const void* q, const void* k, const voi
   c.q_row_stride = q_rs; c.k_row_stride = k_rs; c.v_row_stride = v_rs; c.do_row_stride = do_rs;
   c.dq_row_stride = dq_rs; c.dk_row_stride = dk_rs; c.dv_row_stride = dv_rs;
   c.scale = scale; c.spin_budget = spin_budget; c.stream = stream;
-  using namespace ctb::attn;
-  if (D == 128) return mode == 0 ? launch_bwd<128, MODE_DKV>(c) : launch_bwd<128, MODE_DQ>(c);
-  if (D == 64) return mode == 0 ? launch_bwd<64, MODE_DKV>(c) : launch_bwd<64, MODE_DQ>(c);
-  return ctb::fail("attention: head_dim must be 64 or 128");
+  return D == 128 ? ctb::attn::launch_bwd_both<128>(c, c) : ctb::attn::launch_bwd_both<64>(c, c);
 }
 
 // Block-sparse (MoBA) backward: `it_off` has one entry per CTA plus one, in grid order
@@ -754,16 +814,15 @@ CTB_API int ctb_attn_bwd_sparse(int mode, const void* q, const void* k, const vo
   return ctb::fail("attention: head_dim must be 64 or 128");
 }
 
-// Grouped MoBA backward (see GroupArgs).  mode 0 (dK/dV): one CTA per (group, 128-key tile), `ctas`
-// descriptors; dk / dv are [B,S,Hkv,D] views that hold the own-block gradients, and the history part is
-// added to them (tiles of groups without rows are left alone).  mode 1 (dQ): one CTA per 128 gathered rows,
-// gathered_rows / 128 descriptors; dqg is [gathered_rows, D].  qg / dog / the statistics are the
-// gathered rows ([gathered_rows, D] contiguous, [gathered_rows] fp32, padding rows zero).
-CTB_API int ctb_attn_bwd_grouped(int mode, const void* qg, const void* k, const void* v, const void* dog, void* dqg,
+// Grouped MoBA backward (see GroupArgs).  dK/dV: one CTA per (group, 128-key tile), `dkv_ctas` descriptors; dk / dv are
+// [B,S,Hkv,D] views that hold the own-block gradients, and the history part is added to them (tiles of groups without
+// rows are left alone).  dQ: one CTA per 128 gathered rows, gathered_rows / 128 descriptors; dqg is [gathered_rows, D].
+// qg / dog / the statistics are the gathered rows ([gathered_rows, D] contiguous, [gathered_rows] fp32, padding rows zero).
+CTB_API int ctb_attn_bwd_grouped(const void* qg, const void* k, const void* v, const void* dog, void* dqg,
                                  void* dk, void* dv, const float* neg_lse2_g, const float* neg_delta_g,
-                                 const void* desc, int ctas, int gathered_rows, int block, int B, int S, int Hkv, int D,
-                                 long k_rs, long v_rs, long dk_rs, long dv_rs, float scale, long long spin_budget,
-                                 void* stream) {
+                                 const void* dkv_desc, int dkv_ctas, const void* dq_desc, int gathered_rows, int block, int B,
+                                 int S, int Hkv, int D, long k_rs, long v_rs, long dk_rs, long dv_rs, float scale,
+                                 long long spin_budget, void* stream) {
   if (S % 128 || block % 128 || block < 128) return ctb::fail("grouped attention: S and the block must be multiples of 128");
   if (gathered_rows <= 0 || gathered_rows % 256) return ctb::fail("grouped attention: gathered rows must be a positive multiple of 256");
   ctb::attn::BwdCall c{};
@@ -773,10 +832,14 @@ CTB_API int ctb_attn_bwd_grouped(int mode, const void* qg, const void* k, const 
   c.q_row_stride = D; c.do_row_stride = D; c.dq_row_stride = D;
   c.k_row_stride = k_rs; c.v_row_stride = v_rs; c.dk_row_stride = dk_rs; c.dv_row_stride = dv_rs;
   c.scale = scale; c.spin_budget = spin_budget; c.stream = stream;
-  c.grp.desc = static_cast<const int4*>(desc); c.grp.block = block; c.gathered_rows = gathered_rows;
-  c.ctas = mode == 0 ? ctas : gathered_rows / 128;
+  c.grp.block = block; c.gathered_rows = gathered_rows;
+  ctb::attn::BwdCall dkv = c, dq = c;
+  dkv.grp.desc = static_cast<const int4*>(dkv_desc);
+  dkv.ctas = dkv_ctas;
+  dq.grp.desc = static_cast<const int4*>(dq_desc);
+  dq.ctas = gathered_rows / 128;
   using namespace ctb::attn;
-  if (D == 128) return mode == 0 ? launch_bwd<128, MODE_DKV>(c) : launch_bwd<128, MODE_DQ>(c);
-  if (D == 64) return mode == 0 ? launch_bwd<64, MODE_DKV>(c) : launch_bwd<64, MODE_DQ>(c);
+  if (D == 128) return launch_bwd_both<128>(dkv, dq);
+  if (D == 64) return launch_bwd_both<64>(dkv, dq);
   return ctb::fail("attention: head_dim must be 64 or 128");
 }

@@ -14,11 +14,11 @@ import torch
 from .build import LIB_PATH
 
 
-# Argument kinds of the projections, norms, rotary embedding, activation and backward statistics (p pointer,
-# i int, l long, f float): with them ctypes converts plain Python numbers itself, and a call needs no wrapper object
-# per argument.  All other launchers, the attention kernels among them, take wrapped arguments (:func:`ptr` and the
-# ctypes types).
-_KINDS = {"p": ctypes.c_void_p, "i": ctypes.c_int, "l": ctypes.c_long, "f": ctypes.c_float}
+# Argument kinds of the projections, norms, rotary embedding, activation and attention (p pointer, i int, l long and
+# long long, u unsigned, f float): with them ctypes converts plain Python numbers itself, and a call needs no wrapper
+# object per argument.  All other launchers, block-sparse attention among them, take wrapped arguments (:func:`ptr` and
+# the ctypes types).
+_KINDS = {"p": ctypes.c_void_p, "i": ctypes.c_int, "l": ctypes.c_long, "u": ctypes.c_uint, "f": ctypes.c_float}
 _SIGNATURES = {
     "ctb_gemm": "pppiiillliiiifpip",
     "ctb_rmsnorm_fwd": "ppppppiifp",
@@ -27,6 +27,9 @@ _SIGNATURES = {
     "ctb_swiglu_fwd": "pplip",
     "ctb_swiglu_bwd": "ppplip",
     "ctb_attn_bwd_stats": "pppppiiiillp",
+    "ctb_attn_fwd_range": "pppppppppp" "iiiiiii" "llll" "flp",
+    "ctb_attn_fwd_gathered": "pppppppppp" "iiiiiii" "llll" "f" "pllu" "lp",
+    "ctb_attn_bwd_range": "ppppppppppp" "ppppppppp" "iiiiiii" "llllllll" "flp",
 }
 
 
@@ -73,9 +76,9 @@ def launch_count() -> int:
     return _LAUNCHES
 
 
-def check(code: int, what: str) -> None:
+def check(code: int, what: str, launches: int = 1) -> None:
     global _LAUNCHES
-    _LAUNCHES += 1
+    _LAUNCHES += launches
     if code != 0:
         raise KernelError(f"{what}: {lib().ctb_last_error().decode()}")
 

@@ -394,13 +394,13 @@ def moba_grouped_backward(q, k, v, out, dout, lse, meta: AttentionMeta, groups: 
     dog, lse_g, delta_g = _gather(groups, dout, stats, s, hq, d)
     dqg = torch.empty_like(qg)
     L = _lib.lib()
-    for mode, desc in ((0, groups.dkv_desc), (1, groups.dq_desc)):
-        code = L.ctb_attn_bwd_grouped(
-            mode, _lib.ptr(qg), _lib.ptr(k), _lib.ptr(v), _lib.ptr(dog), _lib.ptr(dqg), _lib.ptr(dk), _lib.ptr(dv),
-            _lib.ptr(lse_g), _lib.ptr(delta_g), _lib.ptr(desc), desc.shape[0], groups.rows_cap, groups.block, b, s, hkv,
-            d, ctypes.c_long(_row_stride(k)), ctypes.c_long(_row_stride(v)), ctypes.c_long(_row_stride(dk)),
-            ctypes.c_long(_row_stride(dv)), ctypes.c_float(scale), ctypes.c_longlong(spin_budget), _lib.stream_ptr())
-        _lib.check(code, "ctb_attn_bwd_grouped")
+    code = L.ctb_attn_bwd_grouped(
+        _lib.ptr(qg), _lib.ptr(k), _lib.ptr(v), _lib.ptr(dog), _lib.ptr(dqg), _lib.ptr(dk), _lib.ptr(dv), _lib.ptr(lse_g),
+        _lib.ptr(delta_g), _lib.ptr(groups.dkv_desc), groups.dkv_desc.shape[0], _lib.ptr(groups.dq_desc), groups.rows_cap,
+        groups.block, b, s, hkv, d, ctypes.c_long(_row_stride(k)), ctypes.c_long(_row_stride(v)),
+        ctypes.c_long(_row_stride(dk)), ctypes.c_long(_row_stride(dv)), ctypes.c_float(scale), ctypes.c_longlong(spin_budget),
+        _lib.stream_ptr())
+    _lib.check(code, "ctb_attn_bwd_grouped")
     code = L.ctb_moba_merge_dq(_lib.ptr(dq), ctypes.c_long(_row_stride(dq)), _lib.ptr(dqg), _lib.ptr(groups.pos_of), b, s,
                                hq, d, groups.picks, _lib.stream_ptr())
     _lib.check(code, "ctb_moba_merge_dq")
