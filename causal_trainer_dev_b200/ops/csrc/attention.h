@@ -99,7 +99,7 @@ struct FwdCall {
   KvFlags kvf{};
 };
 
-enum : int { MODE_DKV = 0, MODE_DQ = 1 };
+enum : int { MODE_DKV = 0, MODE_DQ = 1, MODE_BOTH = 2 };
 
 // Extra metadata of the backward kernels, per token [B,S]:
 //   run_start / run_end   first / last token of the token's run

@@ -32,6 +32,9 @@
 // of elect_one() (64-column tiles: 2 x 2700); dQ 3540, 3032, 2047.  Whole kernels 1.24 -> 0.79 ms and
 // 0.88 -> 0.56 ms.  Now the compute warps are the longer side (P 1300, dS 420, masks 400 cycles).
 //
+// The results of an item are staged in ring slots (the producer leaves it one of Y1, and for dK / dV one of Y2) and not in
+// the resident tiles' place, which the next item's tiles take as soon as the last dP is done.
+//
 // Reference counterparts: causal_trainer_attention_dq / _dkv
 // (src/causal_trainer/kernels/efficient_attention.py:985-1173, 1270-1436); the psum that
 // follows the reference's dK/dV kernel is not needed on one GPU because the group is reduced
@@ -56,6 +59,7 @@ enum : unsigned {
   SITE_B_CW_S = 0x0305,
   SITE_B_CW_ACC = 0x0307,
   SITE_B_BASE = 0x0308,
+  SITE_B_ITEM = 0x0309,
 };
 
 template <int D>
@@ -71,7 +75,8 @@ struct BwdSmem {
   static constexpr int OFF_DELTA = OFF_Y2 + Y2_SLOTS * YT;
   static constexpr int OFF_LSE = OFF_DELTA + Y1_SLOTS * 512;
   static constexpr int OFF_BAR = OFF_LSE + Y2_SLOTS * 512;
-  static constexpr int BYTES = OFF_BAR + 256;       // no slack: the tiles need a 1024-byte aligned base (checked)
+  static constexpr int OFF_ITEMS = OFF_BAR + 256;   // answer of the work request, two work items
+  static constexpr int BYTES = OFF_BAR + 512;       // no slack: the tiles need a 1024-byte aligned base (checked)
   static_assert(BYTES <= 232448, "shared memory of one CTA");
   // TMEM columns: S buffers, dP, accumulators.  A second S buffer where it fits into 512 columns.
   static constexpr int S_BUFS_DKV = 2 * 128 + 128 + 2 * D <= 512 ? 2 : 1;
@@ -82,137 +87,684 @@ struct BwdMaps {
   CUtensorMap q, k, v, dout, out1, out2;     // out1: dV (DKV) or dQ (DQ), out2: dK (DKV)
 };
 
-// Work item `cta` of one mode.
-template <int D, int MODE>
-__device__ __forceinline__ void bwd_cta(const BwdMaps& maps, const BwdArgs& args, const int cta) {
-  using L = BwdSmem<D>;
-  constexpr int HALVES = L::HALVES;
-  constexpr bool DKV = (MODE == MODE_DKV);
-  constexpr int S_BUFS = DKV ? L::S_BUFS_DKV : L::S_BUFS_DQ;
-  extern __shared__ __align__(1024) uint8_t smem[];
-  if ((smem_u32(smem) & 1023u) != 0u) {              // (uniform) the swizzled tiles would not be where TMA writes them
-    if (threadIdx.x == 0) report_failure(args.status, SITE_B_BASE, smem_u32(smem), 0u);
-    return;
-  }
-  uint64_t* x_full = reinterpret_cast<uint64_t*>(smem + L::OFF_BAR);
-  uint64_t* y1_full = x_full + 1;
-  uint64_t* y1_empty = y1_full + Y1_SLOTS;
-  uint64_t* y2_full = y1_empty + Y1_SLOTS;
-  uint64_t* y2_empty = y2_full + Y2_SLOTS;
-  uint64_t* s_full = y2_empty + Y2_SLOTS;   // [2] S of buffer u ready
-  uint64_t* dp_full = s_full + 2;          // dP ready
-  uint64_t* p_full = dp_full + 1;          // [2][2] S buffer u: half h (columns [16 h, 16 h + 16) of every 32) of P^T written
-  uint64_t* ds_full = p_full + 4;          // [2] half h of dS written
-  uint64_t* acc_full = ds_full + 2;
-  uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(acc_full + 1);
-  volatile uint32_t* abort_flag = tmem_slot + 1;
+// One work item, resolved once by the producer warp and handed to the other roles through shared memory.
+struct alignas(16) BwdItem {
+  int mode;          // MODE_DKV, MODE_DQ, or -1: no more work
+  int b, head;       // batch and head of X (kv head for DKV, query head for DQ; 0 for the gathered rows of grouped DQ)
+  int hkv, kbatch;   // kv head and batch of the K / V / dK / dV tensors
+  int x0;            // first row of the resident tiles
+  int y_lo64;        // first 64-row block of the streamed operand
+  int y_n64;         // their number (per head)
+  int y_base;        // grouped: first row (DKV) or key (DQ) of the streamed operand
+  int n_entry;       // 64-row blocks to visit
+  int list;          // block-sparse: offset of the item's entries in it_list
+  int pad;
+};
+static_assert(sizeof(BwdItem) == 48, "three 16-byte reads");
 
-  const int warp = uniform_warp_index();
-  const int lane = threadIdx.x & 31;
-  DeviceStatus* st = args.status;
-  const long long budget = args.spin_budget;
+template <int MODE>
+__device__ __forceinline__ BwdItem bwd_item(const BwdArgs& args, const int cta) {
+  constexpr bool DKV = (MODE == MODE_DKV);
   const int group = args.Hq / args.Hkv;
   const int nb128 = args.S / 128;
-  const int nb64 = args.S / 64;
-
-  // ---- work item ----
-  // grouped MoBA (see GroupArgs): gathered rows of one group against the keys of its block, no masks
-  const bool grouped = args.grp.desc != nullptr;
-  int4 gd = make_int4(0, 0, 0, 0);
-  if (grouped) {
-    gd = __ldg(args.grp.desc + cta);
-    if (gd.w <= 0) return;                       // unused capacity: the whole CTA leaves
+  BwdItem w;
+  w.mode = MODE;
+  w.y_base = 0;
+  w.list = 0;
+  w.pad = 0;
+  if (args.grp.desc != nullptr) {
+    // grouped MoBA (see GroupArgs): gathered rows of one group against the keys of its block, no masks.
+    // X = the item's resident tile: 128 keys of the block (dK/dV) or 128 gathered rows (dQ);
+    // Y = 64-row blocks of the group's gathered rows (dK/dV) or of the block's keys (dQ).
+    const int4 gd = __ldg(args.grp.desc + cta);
+    w.hkv = gd.x >> 16;
+    w.kbatch = gd.x & 0xffff;
+    w.b = DKV ? w.kbatch : 0;
+    w.head = DKV ? w.hkv : 0;
+    w.x0 = DKV ? gd.y : cta * 128;
+    w.y_lo64 = 0;
+    w.y_n64 = gd.w <= 0 ? 0 : (DKV ? gd.w / 64 : args.grp.block / 64);
+    w.y_base = DKV ? gd.z : gd.y;
+    w.n_entry = w.y_n64;
+    if (gd.w <= 0) w.mode = -2;                        // unused capacity: nothing is written
+    return w;
   }
   int idx = cta;
-  int b, head, x0, y_lo64, y_n64, heads_in_loop;
-  if (grouped) {
-    // X = this CTA's resident tile: 128 keys of the block (dK/dV) or 128 gathered rows (dQ);
-    // Y = 64-row blocks of the group's gathered rows (dK/dV) or of the block's keys (dQ).
-    b = DKV ? (gd.x & 0xffff) : 0;
-    head = DKV ? (gd.x >> 16) : 0;
-    x0 = DKV ? gd.y : cta * 128;
-    y_lo64 = 0;
-    y_n64 = DKV ? gd.w / 64 : args.grp.block / 64;
-    heads_in_loop = 1;
-  } else if (DKV) {
-    head = idx % args.Hkv;      // kv head
+  if (DKV) {
+    w.head = idx % args.Hkv;      // kv head
     idx /= args.Hkv;
-    b = idx % args.B;
+    w.b = idx % args.B;
     const int kb = idx / args.B;  // ascending: key blocks near the start see the most queries
-    x0 = kb * 128;
+    w.x0 = kb * 128;
     // only the queries this rank holds, [q_off, q_off + Sq), are walked
-    const int qlo = max(args.q_lo[b * nb128 + kb], args.q_off);
-    const int qhi = min(args.q_hi[b * nb128 + kb], args.q_off + args.Sq);
-    y_lo64 = qlo / 64;
-    y_n64 = qhi > qlo ? (qhi + 63) / 64 - y_lo64 : 0;
-    heads_in_loop = group;
+    const int qlo = max(args.q_lo[w.b * nb128 + kb], args.q_off);
+    const int qhi = min(args.q_hi[w.b * nb128 + kb], args.q_off + args.Sq);
+    w.y_lo64 = qlo / 64;
+    w.y_n64 = qhi > qlo ? (qhi + 63) / 64 - w.y_lo64 : 0;
+    w.n_entry = w.y_n64 * group;
+    w.hkv = w.head;
   } else {
-    head = idx % args.Hq;       // query head
+    w.head = idx % args.Hq;       // query head
     idx /= args.Hq;
-    b = idx % args.B;
+    w.b = idx % args.B;
     const int qb = args.Sq / 128 - 1 - idx / args.B;  // descending: late query blocks see the most keys
-    x0 = qb * 128;                                    // row of the local Q / dO / dQ
-    const int klo = args.kv_lo[b * nb128 + args.q_off / 128 + qb];
-    const int khi = args.kv_hi[b * nb128 + args.q_off / 128 + qb];
-    y_lo64 = klo / 64;
-    y_n64 = khi > klo ? (khi + 63) / 64 - y_lo64 : 0;
-    heads_in_loop = 1;
+    w.x0 = qb * 128;                                  // row of the local Q / dO / dQ
+    const int klo = args.kv_lo[w.b * nb128 + args.q_off / 128 + qb];
+    const int khi = args.kv_hi[w.b * nb128 + args.q_off / 128 + qb];
+    w.y_lo64 = klo / 64;
+    w.y_n64 = khi > klo ? (khi + 63) / 64 - w.y_lo64 : 0;
+    w.n_entry = w.y_n64;
+    w.hkv = w.head / group;
   }
-  int n_entry = y_n64 * heads_in_loop;      // 64-row blocks to visit
-  const int hkv = grouped ? (gd.x >> 16) : (DKV ? head : head / group);
-  const int kbatch = grouped ? (gd.x & 0xffff) : b;     // batch of the K / V / dK / dV tensors
-  const int y_base = grouped ? (DKV ? gd.z : gd.y) : 0; // first row (dK/dV) or key (dQ) of the streamed operand
+  w.kbatch = w.b;
   // Block-sparse routing: the (64-row block, head) pairs come from a list instead of a range.
-  const bool sparse = args.sp.it_list != nullptr;
-  const int* it_list = nullptr;
-  if (sparse) {
-    int base;
-    sparse_list(args.sp, cta, base, n_entry);
-    it_list = args.sp.it_list + base;
-  }
-  const int n_iter = (n_entry + 1) / 2;
-  // entry -> (64-row block of the streamed operand, query head).  Iteration i holds entries 2i and
-  // 2i + 1 in the two halves of its tile; an odd last half repeats the last entry, fully masked.
-  auto y_block = [&](int e) -> int { return sparse ? (__ldg(it_list + e) & 0xffffff) : y_lo64 + e % y_n64; };
-  auto y_head = [&](int e) -> int {
-    if (grouped) return 0;
-    if (!DKV) return head;
-    return hkv * group + (sparse ? (__ldg(it_list + e) >> 24) : e / y_n64);
-  };
+  if (args.sp.it_list != nullptr) sparse_list(args.sp, cta, w.list, w.n_entry);
+  return w;
+}
 
-  if (threadIdx.x == 0) {
-    mbar_init(x_full, 1);
-    for (int s = 0; s < Y1_SLOTS; ++s) {
-      mbar_init(&y1_full[s], 1);
-      mbar_init(&y1_empty[s], 1);
+// entry -> (64-row block of the streamed operand, query head).  Iteration i holds entries 2i and
+// 2i + 1 in the two halves of its tile; an odd last half repeats the last entry, fully masked.
+template <int MODE>
+__device__ __forceinline__ void bwd_entry(const BwdArgs& args, const BwdItem& w, int e, int& block, int& head) {
+  const bool sparse = args.sp.it_list != nullptr;
+  const int entry = sparse ? __ldg(args.sp.it_list + w.list + e) : 0;
+  block = sparse ? (entry & 0xffffff) : w.y_lo64 + e % w.y_n64;
+  if (args.grp.desc != nullptr) head = 0;
+  else if (MODE == MODE_DQ) head = w.head;
+  else head = w.hkv * (args.Hq / args.Hkv) + (sparse ? (entry >> 24) : e / w.y_n64);
+}
+
+// What every role needs to find its way, besides the work item.
+struct BwdShared {
+  uint8_t* smem;
+  uint64_t *x_full, *x_empty, *y1_full, *y1_empty, *y2_full, *y2_empty, *s_full, *dp_full, *p_full, *ds_full, *acc_full, *acc_empty;
+  volatile uint32_t* abort_flag;
+  DeviceStatus* st;
+  long long budget;
+  uint32_t tmem_base;
+};
+
+// Positions that go on from one work item to the next.  The two rings and the barriers of the iterations keep their
+// phases; `items` counts the items with work.
+struct BwdWalk {
+  uint32_t y1_slot = 0, y1_phase = 0;     // Y1 ring
+  uint32_t y2 = 0;                        // uses of the Y2 ring: slot y2 & 1, phase (y2 >> 1) & 1
+  uint32_t iterations = 0;                // dP and dS
+  uint32_t s_phase = 0;                   // bit u: phase of S buffer u (MMA warp: of its P, which dQ items have not)
+  uint32_t items = 0;
+
+  __device__ __forceinline__ void next_y1() {
+    if (++y1_slot == Y1_SLOTS) {
+      y1_slot = 0;
+      y1_phase ^= 1u;
     }
-    for (int s = 0; s < Y2_SLOTS; ++s) {
-      mbar_init(&y2_full[s], 1);
-      mbar_init(&y2_empty[s], 1);
-    }
-    mbar_init(dp_full, 1);
-    for (int u = 0; u < 2; ++u) {
-      mbar_init(&s_full[u], 1);
-      mbar_init(&p_full[2 * u], COMPUTE_WARPS);
-      mbar_init(&p_full[2 * u + 1], COMPUTE_WARPS);
-      mbar_init(&ds_full[u], COMPUTE_WARPS);
-    }
-    mbar_init(acc_full, 1);
-    *abort_flag = 0u;
-    mbar_fence_init();
-    if (n_iter > 0) {
-      // the resident tiles are on their way while TMEM is allocated (with Q in the forward kernel, a layer's forward
-      // and backward: 8.00 -> 7.77 ms on one document of 32768 tokens, 1096 -> 1047 us on 8 image rows of 4096)
-      mbar_expect_tx(x_full, 2 * L::XT);
-      const CUtensorMap* mx1 = DKV ? &maps.k : &maps.q;
-      const CUtensorMap* mx2 = DKV ? &maps.v : &maps.dout;
-      const int xh = DKV ? hkv : head;
-      const int xb = DKV ? kbatch : b;
+  }
+  __device__ __forceinline__ uint32_t y2_slot() const { return y2 & 1u; }
+  __device__ __forceinline__ uint32_t y2_phase() const { return (y2 >> 1) & 1u; }
+};
+
+template <int D, int MODE>
+struct BwdTmem {
+  static constexpr int S_BUFS = MODE == MODE_DKV ? BwdSmem<D>::S_BUFS_DKV : BwdSmem<D>::S_BUFS_DQ;
+  static constexpr uint32_t DP = S_BUFS * 128;
+  static constexpr uint32_t ACC1 = DP + 128;       // dV (DKV) or dQ (DQ)
+  static constexpr uint32_t ACC2 = ACC1 + D;       // dK (DKV)
+};
+
+// Resident tiles of an item (one lane).
+template <int D, int MODE>
+__device__ __forceinline__ void bwd_load_x(uint32_t on, const BwdShared& sh, const BwdMaps& maps, const BwdItem& w) {
+  using L = BwdSmem<D>;
+  constexpr bool DKV = (MODE == MODE_DKV);
+  mbar_expect_tx_if(on, sh.x_full, 2 * L::XT);
+  const CUtensorMap* mx1 = DKV ? &maps.k : &maps.q;
+  const CUtensorMap* mx2 = DKV ? &maps.v : &maps.dout;
+  const int xh = DKV ? w.hkv : w.head;
+  const int xb = DKV ? w.kbatch : w.b;
 #pragma unroll
-      for (int hf = 0; hf < HALVES; ++hf) {
-        tma_load_4d(smem + L::OFF_X + hf * 16384, mx1, x_full, hf * 64, xh, x0, xb);
-        tma_load_4d(smem + L::OFF_X + L::XT + hf * 16384, mx2, x_full, hf * 64, xh, x0, xb);
+  for (int hf = 0; hf < L::HALVES; ++hf) {
+    tma_load_4d_if(on, sh.smem + L::OFF_X + hf * 16384, mx1, sh.x_full, hf * 64, xh, w.x0, xb);
+    tma_load_4d_if(on, sh.smem + L::OFF_X + L::XT + hf * 16384, mx2, sh.x_full, hf * 64, xh, w.x0, xb);
+  }
+}
+
+// ------------------------------ producer ------------------------------
+// The streamed tiles of an item, then the ring slots that its epilogue stages its results in: a slot whose full barrier
+// completes without a copy belongs to the epilogue, which frees it when the results have left.
+template <int D, int MODE>
+__device__ __forceinline__ bool bwd_produce(uint32_t on, const BwdShared& sh, const BwdMaps& maps, const BwdArgs& args,
+                                            const BwdItem& w, BwdWalk& at) {
+  using L = BwdSmem<D>;
+  constexpr bool DKV = (MODE == MODE_DKV);
+  const bool grouped = args.grp.desc != nullptr;
+  const int n_iter = (w.n_entry + 1) / 2;
+  const CUtensorMap* my1 = DKV ? &maps.q : &maps.k;
+  const CUtensorMap* my2 = DKV ? &maps.dout : &maps.v;
+  const int ybatch = DKV ? w.b * (grouped ? 0 : 1) : w.kbatch;
+  for (int it = 0; it < n_iter; ++it) {
+    int y0[2], yh[2];
+    size_t stat[2];
+#pragma unroll
+    for (int q = 0; q < 2; ++q) {              // the two 64-row halves of the tile
+      int block;
+      bwd_entry<MODE>(args, w, min(2 * it + q, w.n_entry - 1), block, yh[q]);
+      if (!DKV) yh[q] = w.hkv;
+      y0[q] = w.y_base + block * 64 - (DKV ? args.q_off : 0);   // streamed queries are stored locally
+      stat[q] = grouped ? static_cast<size_t>(y0[q])
+                        : (static_cast<size_t>(w.b) * args.Hq + yh[q]) * args.Sq + y0[q];
+    }
+    auto load = [&](uint8_t* dst, const CUtensorMap* map, uint64_t* bar, float* stat_dst, const float* stat_src) {
+      mbar_expect_tx_if(on, bar, L::YT + (DKV ? 512 : 0));
+#pragma unroll
+      for (int q = 0; q < 2; ++q) {
+        // the per-query statistics of the block travel with it (256 B each, 256 B aligned)
+        if (DKV) tma_load_1d_if(on, stat_dst + q * 64, stat_src + stat[q], 256, bar);
+#pragma unroll
+        for (int hf = 0; hf < L::HALVES; ++hf)
+          tma_load_4d_if(on, dst + hf * 16384 + q * 8192, map, bar, hf * 64, yh[q], y0[q], ybatch);
       }
+    };
+    if (!mbar_wait_warp(&sh.y1_empty[at.y1_slot], at.y1_phase ^ 1u, sh.abort_flag, sh.st, SITE_B_PROD, sh.budget)) return false;
+    load(sh.smem + L::OFF_Y1 + at.y1_slot * L::YT, my1, &sh.y1_full[at.y1_slot],
+         reinterpret_cast<float*>(sh.smem + L::OFF_DELTA + at.y1_slot * 512), args.neg_delta);
+    at.next_y1();
+    const uint32_t slot2 = at.y2_slot();
+    if (!mbar_wait_warp(&sh.y2_empty[slot2], at.y2_phase() ^ 1u, sh.abort_flag, sh.st, SITE_B_PROD, sh.budget)) return false;
+    load(sh.smem + L::OFF_Y2 + slot2 * L::YT, my2, &sh.y2_full[slot2],
+         reinterpret_cast<float*>(sh.smem + L::OFF_LSE + slot2 * 512), args.neg_lse2);
+    ++at.y2;
+  }
+  if (!mbar_wait_warp(&sh.y1_empty[at.y1_slot], at.y1_phase ^ 1u, sh.abort_flag, sh.st, SITE_B_PROD, sh.budget)) return false;
+  if (on) mbar_arrive(&sh.y1_full[at.y1_slot]);
+  at.next_y1();
+  if (DKV) {
+    if (!mbar_wait_warp(&sh.y2_empty[at.y2_slot()], at.y2_phase() ^ 1u, sh.abort_flag, sh.st, SITE_B_PROD, sh.budget)) return false;
+    if (on) mbar_arrive(&sh.y2_full[at.y2_slot()]);
+    ++at.y2;
+  }
+  return true;
+}
+
+// ------------------------------ MMA issuer ------------------------------
+// `switched`: the item before was of the other mode, whose accumulators lie where this one keeps its dP.
+template <int D, int MODE>
+__device__ __forceinline__ bool bwd_issue(uint32_t on, const BwdShared& sh, const BwdItem& w, BwdWalk& at, bool switched) {
+  using L = BwdSmem<D>;
+  using T = BwdTmem<D, MODE>;
+  constexpr bool DKV = (MODE == MODE_DKV);
+  constexpr int S_BUFS = T::S_BUFS;
+  const int n_iter = (w.n_entry + 1) / 2;
+  bool ok = true;
+  if (n_iter > 0) {
+    constexpr uint32_t idesc_s = make_idesc_bf16(128, 128, false, false);
+    constexpr uint32_t idesc_acc = make_idesc_bf16(128, D, false, true);
+    const uint32_t x1 = smem_u32(sh.smem + L::OFF_X);
+    const uint32_t x2 = smem_u32(sh.smem + L::OFF_X + L::XT);
+    const uint32_t y1_at = smem_u32(sh.smem + L::OFF_Y1);
+    const uint32_t y2_at = smem_u32(sh.smem + L::OFF_Y2);
+    // address arithmetic, not arrays: a runtime index into a local array would go through local memory
+    auto tmem_s = [&](int u) -> uint32_t { return sh.tmem_base + static_cast<uint32_t>(u) * 128u; };
+    const uint32_t tmem_dp = sh.tmem_base + T::DP;
+    // S or dP of the tile in `y`: both operands K-major
+    auto product = [&](uint32_t d, uint32_t x, uint32_t y) {
+#pragma unroll
+      for (int k = 0; k < D / 16; ++k)
+        umma_bf16_if(on, d, desc_kmajor(x + (k / 4) * 16384, k % 4), desc_kmajor(y + (k / 4) * 16384, k % 4), idesc_s,
+                     k != 0 ? 1u : 0u);
+    };
+    // accumulator += (P^T or dS) Y as its halves arrive.  The bf16 pairs of the 16 columns of group kk
+    // sit in the first 8 columns of the group's own 16-column slice of the fp32 buffer
+    auto accumulate = [&](uint64_t* full, uint32_t parity, uint32_t acc, uint32_t a, uint32_t y, int it) -> bool {
+#pragma unroll
+      for (int half = 0; half < 2; ++half) {
+        if (!mbar_wait_warp(&full[half], parity, sh.abort_flag, sh.st, SITE_B_MMA_T, sh.budget)) return false;
+        tc_fence_after();
+#pragma unroll
+        for (int kk = half; kk < 8; kk += 2)
+          umma_bf16_ts_if(on, acc, a + 16 * kk, desc_mnmajor(y, kk, 16384), idesc_acc, (it | kk) != 0 ? 1u : 0u);
+      }
+      return true;
+    };
+    // the epilogue of the last item with work has read the accumulators
+    const uint32_t acc_parity = (at.items & 1u) ^ 1u;
+    if (switched) ok = mbar_wait_warp(sh.acc_empty, acc_parity, sh.abort_flag, sh.st, SITE_B_MMA_T, sh.budget);
+    ok = ok && mbar_wait_warp(sh.x_full, at.items & 1u, sh.abort_flag, sh.st, SITE_B_MMA_X, sh.budget);
+    uint32_t slot_a = at.y1_slot;            // Y1 slot of the next dK / dQ (at.y1_slot: of the next S)
+    uint32_t y2_a = at.y2;                   // Y2 use of the next dV (at.y2: of the next dP)
+    auto next_s = [&](int it) -> bool {
+      if (!mbar_wait_warp(&sh.y1_full[at.y1_slot], at.y1_phase, sh.abort_flag, sh.st, SITE_B_MMA_Y, sh.budget)) return false;
+      tc_fence_after();
+      product(tmem_s(it % S_BUFS), x1, y1_at + at.y1_slot * L::YT);
+      umma_commit_if(on, &sh.s_full[it % S_BUFS]);
+      at.next_y1();
+      return true;
+    };
+    auto next_dp = [&](bool last) -> bool {
+      const uint32_t slot = at.y2_slot();
+      if (!mbar_wait_warp(&sh.y2_full[slot], at.y2_phase(), sh.abort_flag, sh.st, SITE_B_MMA_Y, sh.budget)) return false;
+      tc_fence_after();
+      product(tmem_dp, x2, y2_at + slot * L::YT);
+      umma_commit_if(on, sh.dp_full);
+      if (!DKV) umma_commit_if(on, &sh.y2_empty[slot]);          // V is read by this product alone
+      if (last) umma_commit_if(on, sh.x_empty);                  // the resident tiles may be replaced
+      ++at.y2;
+      return true;
+    };
+    ok = ok && next_s(0) && next_dp(n_iter == 1);
+    for (int it = 0; ok && it < n_iter; ++it) {
+      const bool more = it + 1 < n_iter;
+      const int u = it % S_BUFS;
+      // with one S buffer the next scores overwrite P, which dV reads: in issue order, so no wait
+      if (S_BUFS == 2 && more && !next_s(it + 1)) return false;
+      if (it == 0 && !switched &&
+          !mbar_wait_warp(sh.acc_empty, acc_parity, sh.abort_flag, sh.st, SITE_B_MMA_T, sh.budget))
+        return false;
+      if (DKV) {
+        if (!accumulate(sh.p_full + 2 * u, (at.s_phase >> u) & 1u, sh.tmem_base + T::ACC1, tmem_s(u),
+                        y2_at + (y2_a & 1u) * L::YT, it))
+          return false;
+        umma_commit_if(on, &sh.y2_empty[y2_a & 1u]);
+        ++y2_a;
+        at.s_phase ^= 1u << u;
+      }
+      if (S_BUFS == 1 && more && !next_s(it + 1)) return false;
+      if (!accumulate(sh.ds_full, at.iterations & 1u, sh.tmem_base + (DKV ? T::ACC2 : T::ACC1), tmem_dp,
+                      y1_at + slot_a * L::YT, it))
+        return false;
+      ++at.iterations;
+      umma_commit_if(on, &sh.y1_empty[slot_a]);
+      if (++slot_a == Y1_SLOTS) slot_a = 0;
+      if (more) ok = next_dp(it + 2 == n_iter);
+      else umma_commit_if(on, sh.acc_full);
+    }
+    ++at.items;
+  }
+  at.next_y1();              // the slots that the epilogue stages in
+  if (DKV) ++at.y2;
+  return ok;
+}
+
+// ------------------------------ compute warpgroups ------------------------------
+// Four compute warpgroups work on every iteration together: warpgroup wg takes columns
+// [32 wg, 32 wg + 32) of the tile, i.e. 32 columns of entry 2 it + wg / 2.
+template <int D, int MODE>
+__device__ __forceinline__ bool bwd_compute(const BwdShared& sh, const BwdMaps& maps, const BwdArgs& args, const BwdItem& w,
+                                            BwdWalk& at) {
+  using L = BwdSmem<D>;
+  using T = BwdTmem<D, MODE>;
+  constexpr bool DKV = (MODE == MODE_DKV);
+  constexpr int S_BUFS = T::S_BUFS;
+  const int warp = uniform_warp_index(), lane = threadIdx.x & 31;
+  const bool grouped = args.grp.desc != nullptr, sparse = args.sp.it_list != nullptr;
+  const int b = w.b, head = w.head, hkv = w.hkv, x0 = w.x0;
+  const int group = args.Hq / args.Hkv, nb64 = args.S / 64;
+  const int n_entry = w.n_entry, n_iter = (n_entry + 1) / 2;
+  const int* it_list = sparse ? args.sp.it_list + w.list : nullptr;
+  const int wg = (warp - 4) >> 2;
+  const int quad = warp & 3;
+  const int r = quad * 32 + lane;
+  const uint32_t lane_off = static_cast<uint32_t>(quad * 32) << 16;
+  // position in the whole sequence of this thread's row: a key (DKV) or a local query (DQ)
+  const int xi = x0 + r + (DKV ? 0 : args.q_off);
+  const int xi_local = x0 + r;
+  const int row_seg = grouped ? 1 : args.seg[b * args.S + xi];
+  // interval of visible columns (whole-sequence positions): see the mask below
+  int row_a, row_b;
+  if (grouped) {
+    row_a = -(1 << 30);       // everything is visible: padding rows hold zeros and contribute zero
+    row_b = 1 << 30;
+  } else if (DKV) {
+    row_a = args.first_q[b * args.S + xi];
+    row_b = args.run_end[b * args.S + xi];
+  } else {
+    row_a = args.run_start[b * args.S + xi];
+    row_b = (args.lim != nullptr) ? args.lim[b * args.S + xi] : xi;
+  }
+  const int row_start = sparse ? args.sp.doc_start[b * args.S + xi] : 0;
+  // DKV: the document-relative block of this key is the bit every query column is tested for
+  const int row_blk = (sparse && DKV) ? (xi - row_start) / args.sp.block : 0;
+  float neg_lse2 = 0.f, neg_delta = 0.f;      // DQ: per-row statistics (stored negated, lse in log2 units)
+  if (!DKV) {
+    const size_t row = grouped ? static_cast<size_t>(xi_local) : (static_cast<size_t>(b) * args.Hq + head) * args.Sq + xi_local;
+    neg_lse2 = args.neg_lse2[row];
+    neg_delta = args.neg_delta[row];
+  }
+  bool ok = true;
+  const uint64_t scale2 = pack_f32x2(args.scale_log2, args.scale_log2);
+  const int mine = wg >> 1;               // half of the tile this warpgroup works on
+  // dense walk: (block, head) advance without a division per iteration (the first step moves by one
+  // entry for the warpgroups of the second half, the others by two)
+  int walk_block = 0, walk_head = 0;
+  auto advance = [&](int n) {
+    walk_block += n;
+    while (walk_block >= w.y_n64) {
+      walk_block -= w.y_n64;
+      ++walk_head;
+    }
+  };
+  if (!sparse && n_entry > 0) advance(mine);
+  for (int it = 0; it < n_iter; ++it) {
+    const int entry_at = 2 * it + mine;
+    const bool real = entry_at < n_entry;
+    int yb, hq;
+    if (sparse) {
+      const int entry = __ldg(it_list + min(entry_at, n_entry - 1));
+      yb = entry & 0xffffff;
+      hq = DKV ? hkv * group + (entry >> 24) : head;
+    } else {
+      yb = w.y_lo64 + walk_block;
+      hq = DKV ? hkv * group + walk_head : head;
+      advance(2);
+    }
+    const int y0 = yb * 64;                   // (grouped: relative to the group, and nothing is masked)
+    const int base = y0 + 32 * (wg & 1);      // first column of this thread
+    // ---- visibility of this row against its 32 columns, as a bit mask.  The keys a query sees
+    // and the queries that see a key are both contiguous intervals (runs are contiguous):
+    //   DQ   row = query xi,  columns = keys     [start[xi], lim[xi]]
+    //   DKV  row = key xi,    columns = queries  [first_q[xi], end[xi]]
+    // Most tiles are wholly visible: two compares, the mask itself only where some row needs it.
+    unsigned vis = 0xffffffffu;
+    const bool inside = real && row_seg != 0 && row_a <= base && row_b >= base + 31;
+    if (sparse || !__all_sync(0xffffffffu, inside)) {
+      vis = (row_seg == 0 || !real) ? 0u : (bits_from(row_a - base) & bits_upto(row_b - base));
+      if (sparse && vis != 0u) {
+        if (DKV) {
+          if ((row_blk >> 5) >= args.sp.words) {
+            vis = 0u;
+          } else {
+            // when every query of the block selected this key's block the selection adds nothing
+            const unsigned aw = __ldg(args.sp.allsel + ((static_cast<size_t>(b) * args.Hq + hq) * nb64 + yb) * args.sp.words +
+                                      (row_blk >> 5));
+            if (!((aw >> (row_blk & 31)) & 1u)) {
+              // per-query selection bit of this key's block, for the 32 columns of this thread
+              const unsigned* col_sel = args.sp.sel + ((static_cast<size_t>(b) * args.Hq + hq) * args.S + base) * args.sp.words +
+                                        (row_blk >> 5);
+              const int bit = row_blk & 31;
+              unsigned selbits = 0u;
+#pragma unroll 4
+              for (int e = 0; e < 32; ++e)
+                selbits |= ((__ldg(col_sel + static_cast<size_t>(e) * args.sp.words) >> bit) & 1u) << e;
+              vis &= selbits;
+            }
+          }
+        } else {
+          const SparseRow sr = sparse_row(args.sp, b, head, args.Hq, args.S, xi, row_start, y0, 64);
+          const unsigned above = bits_from(sr.bound - base);               // keys >= bound
+          vis &= (sr.v0 ? ~above : 0u) | (sr.v1 ? above : 0u);
+        }
+      }
+    }
+    const bool warp_all = __all_sync(0xffffffffu, vis == 0xffffffffu);
+    // DKV: per-query statistics of this thread's 32 columns, staged beside the tile by the producer
+    const ulonglong2* lse_col = reinterpret_cast<const ulonglong2*>(sh.smem + L::OFF_LSE + at.y2_slot() * 512) + 8 * wg;
+    const ulonglong2* delta_col = reinterpret_cast<const ulonglong2*>(sh.smem + L::OFF_DELTA + at.y1_slot * 512) + 8 * wg;
+    const int u = it % S_BUFS;
+    const uint32_t s_at = sh.tmem_base + static_cast<uint32_t>(u) * 128u + lane_off + 32 * wg;
+    const uint32_t dp_at = sh.tmem_base + T::DP + lane_off + 32 * wg;
+    if (DKV) {
+      // (the statistics were written by bulk copies: these waits make them visible to the thread)
+      if (!mbar_wait(&sh.y1_full[at.y1_slot], at.y1_phase, sh.abort_flag, sh.st, SITE_B_CW_S, sh.budget) ||
+          !mbar_wait(&sh.y2_full[at.y2_slot()], at.y2_phase(), sh.abort_flag, sh.st, SITE_B_CW_S, sh.budget)) {
+        ok = false;
+        break;
+      }
+    }
+    if (!mbar_wait(&sh.s_full[u], (at.s_phase >> u) & 1u, sh.abort_flag, sh.st, SITE_B_CW_S, sh.budget)) {
+      ok = false;
+      break;
+    }
+    // (the accumulate MMAs that read P^T / dS of the previous iteration from these buffers were issued
+    // before the products that refilled them, and the tensor core completes MMAs in issue order)
+    tc_fence_after();
+    // MASKED = false is the path of a warp whose rows all see all 32 columns: no selects.
+    float p[32];
+    auto probabilities = [&](auto masked_tag) {
+      constexpr bool MASKED = decltype(masked_tag)::value;
+      uint32_t sc[32];
+      tmem_ld32(s_at, sc);
+      tmem_ld_wait();
+#pragma unroll
+      for (int half = 0; half < 2; ++half) {
+        uint32_t pw[8];
+#pragma unroll
+        for (int e4 = 0; e4 < 4; ++e4) {                 // groups of four columns
+          uint64_t l2[2];                                // negated statistics, two columns per word
+          if (DKV) {
+            const ulonglong2 lv = lse_col[half * 4 + e4];
+            l2[0] = lv.x;
+            l2[1] = lv.y;
+          } else {
+            l2[0] = l2[1] = pack_f32x2(neg_lse2, neg_lse2);
+          }
+          // p = exp2(s * scale - lse): two columns per packed instruction
+#pragma unroll
+          for (int pr = 0; pr < 2; ++pr) {
+            const int e = half * 16 + e4 * 4 + pr * 2;
+            const uint64_t x2 = fma_f32x2(pack_f32x2(__uint_as_float(sc[e]), __uint_as_float(sc[e + 1])), scale2, l2[pr]);
+            float xa, xb;
+            unpack_f32x2(x2, xa, xb);
+            float pa = fast_exp2(xa), pb = fast_exp2(xb);
+            if (MASKED) {
+              if (!((vis >> e) & 1u)) pa = 0.f;
+              if (!((vis >> (e + 1)) & 1u)) pb = 0.f;
+            }
+            p[e] = pa;
+            p[e + 1] = pb;
+            if (DKV) pw[e4 * 2 + pr] = pack_bf16(pa, pb);
+          }
+        }
+        if (DKV) {
+          tmem_st8(s_at + 16 * half, pw);
+          tmem_st_wait();
+          tc_fence_before();
+          __syncwarp();
+          if (lane == 0) mbar_arrive(&sh.p_full[2 * u + half]);
+        }
+      }
+    };
+    if (warp_all) probabilities(std::false_type{});
+    else probabilities(std::true_type{});
+    if (!mbar_wait(sh.dp_full, at.iterations & 1u, sh.abort_flag, sh.st, SITE_B_CW_S, sh.budget)) {
+      ok = false;
+      break;
+    }
+    tc_fence_after();
+    uint32_t rd[32];
+    tmem_ld32(dp_at, rd);
+    tmem_ld_wait();
+    // dS = p * (dP - delta)
+#pragma unroll
+    for (int half = 0; half < 2; ++half) {
+      uint32_t dw[8];
+#pragma unroll
+      for (int e4 = 0; e4 < 4; ++e4) {
+        uint64_t dl[2];
+        if (DKV) {
+          const ulonglong2 dv = delta_col[half * 4 + e4];
+          dl[0] = dv.x;
+          dl[1] = dv.y;
+        } else {
+          dl[0] = dl[1] = pack_f32x2(neg_delta, neg_delta);
+        }
+#pragma unroll
+        for (int pr = 0; pr < 2; ++pr) {
+          const int e = half * 16 + e4 * 4 + pr * 2;
+          const uint64_t d2 = add_f32x2(pack_f32x2(__uint_as_float(rd[e]), __uint_as_float(rd[e + 1])), dl[pr]);
+          const uint64_t ds2 = mul_f32x2(pack_f32x2(p[e], p[e + 1]), d2);
+          float da, db;
+          unpack_f32x2(ds2, da, db);
+          dw[e4 * 2 + pr] = pack_bf16(da, db);
+        }
+      }
+      tmem_st8(dp_at + 16 * half, dw);
+      tmem_st_wait();
+      tc_fence_before();
+      __syncwarp();
+      if (lane == 0) mbar_arrive(&sh.ds_full[half]);
+    }
+    at.next_y1();
+    ++at.y2;
+    ++at.iterations;
+    at.s_phase ^= 1u << u;
+  }
+  // the epilogue pairs the warpgroups: pair u converts accumulator u, each warpgroup half of it
+  const int u = wg & 1;
+  const int half = wg >> 1;
+  const bool writes = DKV || (u == 0);
+  // ---- epilogue: accumulators -> bf16 -> staging -> TMA store ----
+  if (ok && n_iter > 0) {
+    ok = mbar_wait(sh.acc_full, at.items & 1u, sh.abort_flag, sh.st, SITE_B_CW_ACC, sh.budget);
+    tc_fence_after();
+  }
+  // pair 0 stages in the Y1 slot, pair 1 in the Y2 slot that the producer leaves to the epilogue
+  const uint32_t slot = u == 0 ? at.y1_slot : at.y2_slot();
+  if (ok && writes)
+    ok = mbar_wait(u == 0 ? &sh.y1_full[slot] : &sh.y2_full[slot], u == 0 ? at.y1_phase : at.y2_phase(), sh.abort_flag, sh.st,
+                   SITE_B_CW_ACC, sh.budget);
+  const bool any_bad = named_bar_or(2 + u, 256, !ok);
+  if (!any_bad && writes) {
+    // DKV: warpgroup 0 stores dV, warpgroup 1 stores dK (scaled); DQ: warpgroup 0 stores dQ (scaled).
+    const uint32_t acc = sh.tmem_base + ((DKV && u == 1) ? T::ACC2 : T::ACC1);
+    const float mul = (DKV && u == 0) ? 1.f : args.scale;
+    uint8_t* stage_buf = sh.smem + (u == 0 ? L::OFF_Y1 : L::OFF_Y2) + slot * L::YT;      // [HALVES][128 rows][128 B]
+    // the two warpgroups of the pair convert half of the head dimension each
+#pragma unroll 1
+    for (int c = half * (D / 64); c < (half + 1) * (D / 64); ++c) {
+      uint32_t rr[32];
+      if (n_iter > 0) {
+        tmem_ld32(acc + lane_off + c * 32, rr);
+        tmem_ld_wait();
+      } else {
+#pragma unroll
+        for (int e = 0; e < 32; ++e) rr[e] = 0u;
+      }
+#pragma unroll
+      for (int jj = 0; jj < 4; ++jj) {
+        uint4 v;
+        v.x = pack_bf16(__uint_as_float(rr[jj * 8 + 0]) * mul, __uint_as_float(rr[jj * 8 + 1]) * mul);
+        v.y = pack_bf16(__uint_as_float(rr[jj * 8 + 2]) * mul, __uint_as_float(rr[jj * 8 + 3]) * mul);
+        v.z = pack_bf16(__uint_as_float(rr[jj * 8 + 4]) * mul, __uint_as_float(rr[jj * 8 + 5]) * mul);
+        v.w = pack_bf16(__uint_as_float(rr[jj * 8 + 6]) * mul, __uint_as_float(rr[jj * 8 + 7]) * mul);
+        *reinterpret_cast<uint4*>(stage_buf + (c / 2) * 16384 + sw128_offset(r, (c % 2) * 4 + jj)) = v;
+      }
+    }
+    tc_fence_before();
+    fence_proxy_async_smem();
+    named_bar_sync(4 + u, 256);
+    if (r == 0 && half == 0) {
+      const CUtensorMap* mo = (DKV && u == 1) ? &maps.out2 : &maps.out1;
+      const int oh = DKV ? hkv : head;
+      const int ob = DKV ? w.kbatch : b;
+#pragma unroll
+      for (int hf = 0; hf < L::HALVES; ++hf) {
+        // grouped dK / dV: the history part joins what the own-block pass stored (one CTA per tile, so the sum
+        // does not depend on timing)
+        if (DKV && grouped) tma_reduce_add_4d(mo, stage_buf + hf * 16384, hf * 64, oh, x0, ob);
+        else tma_store_4d(mo, stage_buf + hf * 16384, hf * 64, oh, x0, ob);
+      }
+      tma_commit_group();
+    }
+  }
+  if (n_iter > 0) {
+    tc_fence_before();
+    __syncwarp();
+    if (lane == 0) mbar_arrive(sh.acc_empty);      // the next item may accumulate
+    ++at.items;
+  }
+  if (!any_bad && writes && r == 0 && half == 0) {
+    tma_wait_group_read<0>();
+    mbar_arrive(u == 0 ? &sh.y1_empty[slot] : &sh.y2_empty[slot]);
+  }
+  at.next_y1();
+  if (DKV) ++at.y2;
+  return !any_bad;
+}
+
+// MODES: MODE_DKV, MODE_DQ, or MODE_BOTH: work items [0, dkv_items) of the first kind, then those of the second.
+//
+// A CTA stays on its SM and takes over work items of the grid that have not started (cluster launch control): the
+// resident tiles, the first scores and the results of neighbouring items overlap, where a CTA of its own for each pays for
+// its start, its first copies and its last stores one after the other (about 7000 cycles, a quarter of the dQ item of a
+// packed row).  The next item is requested when the last copies of the current one are issued, not earlier: an item
+// that waits behind a long one could have run elsewhere.
+template <int D, int MODES>
+__global__ void __launch_bounds__(BWD_THREADS, 1)
+attn_bwd_kernel(const __grid_constant__ BwdMaps dkv_maps, const __grid_constant__ BwdMaps dq_maps,
+                const __grid_constant__ BwdArgs dkv, const __grid_constant__ BwdArgs dq, const int dkv_items) {
+  using L = BwdSmem<D>;
+  extern __shared__ __align__(1024) uint8_t smem[];
+  const BwdArgs& any = MODES == MODE_DQ ? dq : dkv;
+  if ((smem_u32(smem) & 1023u) != 0u) {              // (uniform) the swizzled tiles would not be where TMA writes them
+    if (threadIdx.x == 0) report_failure(any.status, SITE_B_BASE, smem_u32(smem), 0u);
+    return;
+  }
+  BwdShared sh;
+  sh.smem = smem;
+  sh.x_full = reinterpret_cast<uint64_t*>(smem + L::OFF_BAR);
+  sh.x_empty = sh.x_full + 1;
+  sh.y1_full = sh.x_empty + 1;
+  sh.y1_empty = sh.y1_full + Y1_SLOTS;
+  sh.y2_full = sh.y1_empty + Y1_SLOTS;
+  sh.y2_empty = sh.y2_full + Y2_SLOTS;
+  sh.s_full = sh.y2_empty + Y2_SLOTS;       // [2] S of buffer u ready
+  sh.dp_full = sh.s_full + 2;              // dP ready
+  sh.p_full = sh.dp_full + 1;              // [2][2] S buffer u: half h (columns [16 h, 16 h + 16) of every 32) of P^T written
+  sh.ds_full = sh.p_full + 4;              // [2] half h of dS written
+  sh.acc_full = sh.ds_full + 2;
+  sh.acc_empty = sh.acc_full + 1;
+  uint64_t* item_full = sh.acc_empty + 1;  // [2] work item u resolved
+  uint64_t* item_empty = item_full + 2;    // [2] and read by the MMA warp and the compute warps
+  uint64_t* answer_full = item_empty + 2;
+  uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(answer_full + 1);
+  sh.abort_flag = tmem_slot + 1;
+  static_assert((1 + 1 + 2 * Y1_SLOTS + 2 * Y2_SLOTS + 2 + 1 + 4 + 2 + 2 + 2 + 2 + 1) * 8 + 8 <= 256, "barrier block");
+  const uint32_t answer = smem_u32(smem + L::OFF_ITEMS);
+  BwdItem* items = reinterpret_cast<BwdItem*>(smem + L::OFF_ITEMS + 16);
+  sh.st = any.status;
+  sh.budget = any.spin_budget;
+  const int warp = uniform_warp_index();
+  const int lane = threadIdx.x & 31;
+
+  auto resolve = [&](int cta) -> BwdItem {
+    if (MODES == MODE_DKV || (MODES == MODE_BOTH && cta < dkv_items)) return bwd_item<MODE_DKV>(dkv, cta);
+    return bwd_item<MODE_DQ>(dq, MODES == MODE_BOTH ? cta - dkv_items : cta);
+  };
+  BwdItem w;
+  if (threadIdx.x < 32) {
+    if (lane == 0) {
+      mbar_init(sh.x_full, 1);
+      mbar_init(sh.x_empty, 1);
+      for (int s = 0; s < Y1_SLOTS; ++s) {
+        mbar_init(&sh.y1_full[s], 1);
+        mbar_init(&sh.y1_empty[s], 1);
+      }
+      for (int s = 0; s < Y2_SLOTS; ++s) {
+        mbar_init(&sh.y2_full[s], 1);
+        mbar_init(&sh.y2_empty[s], 1);
+      }
+      mbar_init(sh.dp_full, 1);
+      for (int u = 0; u < 2; ++u) {
+        mbar_init(&sh.s_full[u], 1);
+        mbar_init(&sh.p_full[2 * u], COMPUTE_WARPS);
+        mbar_init(&sh.p_full[2 * u + 1], COMPUTE_WARPS);
+        mbar_init(&sh.ds_full[u], COMPUTE_WARPS);
+        mbar_init(&item_full[u], 1);
+        mbar_init(&item_empty[u], 1 + COMPUTE_WARPS);
+      }
+      mbar_init(sh.acc_full, 1);
+      mbar_init(sh.acc_empty, COMPUTE_WARPS);
+      mbar_init(answer_full, 1);
+      *sh.abort_flag = 0u;
+      mbar_fence_init();
+    }
+    __syncwarp();
+    w = resolve(static_cast<int>(blockIdx.x));
+    // the resident tiles are on their way while TMEM is allocated (with Q in the forward kernel, a layer's forward
+    // and backward: 8.00 -> 7.77 ms on one document of 32768 tokens, 1096 -> 1047 us on 8 image rows of 4096)
+    if (w.mode >= 0 && w.n_entry > 0) {
+      const uint32_t on = elect_one();
+      if (w.mode == MODE_DKV) bwd_load_x<D, MODE_DKV>(on, sh, dkv_maps, w);
+      else bwd_load_x<D, MODE_DQ>(on, sh, dq_maps, w);
     }
   }
   if (warp == 1) {
@@ -222,420 +774,95 @@ __device__ __forceinline__ void bwd_cta(const BwdMaps& maps, const BwdArgs& args
   tc_fence_before();
   __syncthreads();
   tc_fence_after();
-  const uint32_t tmem_base = *tmem_slot;
-  // address arithmetic, not arrays: a runtime index into a local array would go through local memory
-  auto tmem_s = [&](int u) -> uint32_t { return tmem_base + static_cast<uint32_t>(u) * 128u; };
-  const uint32_t tmem_dp = tmem_base + S_BUFS * 128u;
-  const uint32_t tmem_acc1 = tmem_dp + 128u;        // dV (DKV) or dQ (DQ)
-  const uint32_t tmem_acc2 = tmem_acc1 + D;   // dK (DKV)
+  sh.tmem_base = *tmem_slot;
+
+  // the next work item, for the roles that are told of it
+  uint32_t turn = 0;
+  auto take = [&](BwdItem& item) -> bool {
+    const uint32_t u = turn & 1u;
+    const bool got = mbar_wait_warp(&item_full[u], (turn >> 1) & 1u, sh.abort_flag, sh.st, SITE_B_ITEM, sh.budget);
+    if (!got) return false;
+    const int4* from = reinterpret_cast<const int4*>(&items[u]);
+    int4* to = reinterpret_cast<int4*>(&item);
+#pragma unroll
+    for (int i = 0; i < 3; ++i) to[i] = from[i];
+    __syncwarp();
+    if (lane == 0) mbar_arrive(&item_empty[u]);
+    ++turn;
+    return item.mode >= 0;
+  };
 
   if (warp == 0) {
-    // ------------------------------ producer ------------------------------
-    if (n_iter > 0) {
-      const uint32_t on = elect_one();            // the whole warp walks, one lane issues
-      const CUtensorMap* my1 = DKV ? &maps.q : &maps.k;
-      const CUtensorMap* my2 = DKV ? &maps.dout : &maps.v;
-      uint32_t slot1 = 0, phase1 = 0;
-      const int ybatch = DKV ? b * (grouped ? 0 : 1) : kbatch;
-      for (int it = 0; it < n_iter; ++it) {
-        const uint32_t slot2 = it & 1, phase2 = (it >> 1) & 1;
-        int y0[2], yh[2];
-        size_t stat[2];
-#pragma unroll
-        for (int q = 0; q < 2; ++q) {              // the two 64-row halves of the tile
-          const int e = min(2 * it + q, n_entry - 1);
-          yh[q] = DKV ? y_head(e) : hkv;
-          y0[q] = y_base + y_block(e) * 64 - (DKV ? args.q_off : 0);   // streamed queries are stored locally
-          stat[q] = grouped ? static_cast<size_t>(y0[q])
-                            : (static_cast<size_t>(b) * args.Hq + yh[q]) * args.Sq + y0[q];
+    const uint32_t on = elect_one();            // the whole warp walks, one lane issues
+    BwdWalk at;
+    uint32_t requests = 0;
+    bool ok = true, loaded = true;              // the first item's resident tiles are on their way
+    while (ok) {
+      if (w.mode != -2) {                       // (unused capacity of a grouped launch is not passed on)
+        const uint32_t u = turn & 1u;
+        ok = mbar_wait_warp(&item_empty[u], ((turn >> 1) & 1u) ^ 1u, sh.abort_flag, sh.st, SITE_B_ITEM, sh.budget);
+        if (!ok) break;
+        if (lane == 0) {
+          items[u] = w;
+          mbar_arrive(&item_full[u]);
         }
-        auto load = [&](uint8_t* dst, const CUtensorMap* map, uint64_t* bar, float* stat_dst, const float* stat_src) {
-          mbar_expect_tx_if(on, bar, L::YT + (DKV ? 512 : 0));
-#pragma unroll
-          for (int q = 0; q < 2; ++q) {
-            // the per-query statistics of the block travel with it (256 B each, 256 B aligned)
-            if (DKV) tma_load_1d_if(on, stat_dst + q * 64, stat_src + stat[q], 256, bar);
-#pragma unroll
-            for (int hf = 0; hf < HALVES; ++hf)
-              tma_load_4d_if(on, dst + hf * 16384 + q * 8192, map, bar, hf * 64, yh[q], y0[q], ybatch);
+        ++turn;
+        if (w.mode < 0) break;
+        if (w.n_entry > 0) {
+          if (!loaded) {
+            ok = mbar_wait_warp(sh.x_empty, (at.items & 1u) ^ 1u, sh.abort_flag, sh.st, SITE_B_PROD, sh.budget);
+            if (!ok) break;
+            if (w.mode == MODE_DKV) bwd_load_x<D, MODE_DKV>(on, sh, dkv_maps, w);
+            else bwd_load_x<D, MODE_DQ>(on, sh, dq_maps, w);
           }
-        };
-        if (!mbar_wait_warp(&y1_empty[slot1], phase1 ^ 1u, abort_flag, st, SITE_B_PROD, budget)) break;
-        load(smem + L::OFF_Y1 + slot1 * L::YT, my1, &y1_full[slot1],
-             reinterpret_cast<float*>(smem + L::OFF_DELTA + slot1 * 512), args.neg_delta);
-        if (!mbar_wait_warp(&y2_empty[slot2], phase2 ^ 1u, abort_flag, st, SITE_B_PROD, budget)) break;
-        load(smem + L::OFF_Y2 + slot2 * L::YT, my2, &y2_full[slot2],
-             reinterpret_cast<float*>(smem + L::OFF_LSE + slot2 * 512), args.neg_lse2);
-        if (++slot1 == Y1_SLOTS) {
-          slot1 = 0;
-          phase1 ^= 1u;
+          ++at.items;
         }
+        if (MODES != MODE_DQ && w.mode == MODE_DKV) ok = bwd_produce<D, MODE_DKV>(on, sh, dkv_maps, dkv, w, at);
+        else if (MODES != MODE_DKV) ok = bwd_produce<D, MODE_DQ>(on, sh, dq_maps, dq, w, at);
+        if (!ok) break;
       }
+      loaded = false;
+      // a work item of the grid that has not started, if there is one
+      mbar_expect_tx_if(on, answer_full, 16);
+      work_request_if(on, answer, answer_full);
+      ok = mbar_wait_warp(answer_full, requests & 1u, sh.abort_flag, sh.st, SITE_B_ITEM, sh.budget);
+      if (!ok) break;
+      ++requests;
+      const int cta = work_answer(answer);
+      fence_proxy_async_smem();                 // the next answer is written after this one is read
+      __syncwarp();
+      if (cta >= 0) w = resolve(cta);
+      else w.mode = -1;
     }
   } else if (warp == 1) {
-    // ------------------------------ MMA issuer ------------------------------
-    if (n_iter > 0) {
-      const uint32_t on = elect_one();            // the whole warp walks, one lane issues
-      constexpr uint32_t idesc_s = make_idesc_bf16(128, 128, false, false);
-      constexpr uint32_t idesc_acc = make_idesc_bf16(128, D, false, true);
-      const uint32_t x1 = smem_u32(smem + L::OFF_X);
-      const uint32_t x2 = smem_u32(smem + L::OFF_X + L::XT);
-      const uint32_t y1_at = smem_u32(smem + L::OFF_Y1);
-      const uint32_t y2_at = smem_u32(smem + L::OFF_Y2);
-      // S or dP of the tile in `y`: both operands K-major
-      auto product = [&](uint32_t d, uint32_t x, uint32_t y) {
-#pragma unroll
-        for (int k = 0; k < D / 16; ++k)
-          umma_bf16_if(on, d, desc_kmajor(x + (k / 4) * 16384, k % 4), desc_kmajor(y + (k / 4) * 16384, k % 4), idesc_s,
-                    k != 0 ? 1u : 0u);
-      };
-      // accumulator += (P^T or dS) Y as its halves arrive.  The bf16 pairs of the 16 columns of group kk
-      // sit in the first 8 columns of the group's own 16-column slice of the fp32 buffer
-      auto accumulate = [&](uint64_t* full, uint32_t parity, uint32_t acc, uint32_t a, uint32_t y, int it) -> bool {
-#pragma unroll
-        for (int half = 0; half < 2; ++half) {
-          if (!mbar_wait_warp(&full[half], parity, abort_flag, st, SITE_B_MMA_T, budget)) return false;
-          tc_fence_after();
-#pragma unroll
-          for (int kk = half; kk < 8; kk += 2)
-            umma_bf16_ts_if(on, acc, a + 16 * kk, desc_mnmajor(y, kk, 16384), idesc_acc, (it | kk) != 0 ? 1u : 0u);
-        }
-        return true;
-      };
-      bool ok = mbar_wait_warp(x_full, 0, abort_flag, st, SITE_B_MMA_X, budget);
-      uint32_t slot_s = 0, phase_s = 0;        // Y1 slot of the next S
-      uint32_t slot_a = 0;                     // Y1 slot of the next dK / dQ
-      auto next_s = [&](int it) -> bool {
-        if (!mbar_wait_warp(&y1_full[slot_s], phase_s, abort_flag, st, SITE_B_MMA_Y, budget)) return false;
-        tc_fence_after();
-        product(tmem_s(it % S_BUFS), x1, y1_at + slot_s * L::YT);
-        umma_commit_if(on, &s_full[it % S_BUFS]);
-        if (++slot_s == Y1_SLOTS) {
-          slot_s = 0;
-          phase_s ^= 1u;
-        }
-        return true;
-      };
-      auto next_dp = [&](int it) -> bool {
-        if (!mbar_wait_warp(&y2_full[it & 1], static_cast<uint32_t>(it >> 1) & 1u, abort_flag, st, SITE_B_MMA_Y, budget))
-          return false;
-        tc_fence_after();
-        product(tmem_dp, x2, y2_at + (it & 1) * L::YT);
-        umma_commit_if(on, dp_full);
-        if (!DKV) umma_commit_if(on, &y2_empty[it & 1]);          // V is read by this product alone
-        return true;
-      };
-      ok = ok && next_s(0) && next_dp(0);
-      for (int it = 0; ok && it < n_iter; ++it) {
-        const bool more = it + 1 < n_iter;
-        // with one S buffer the next scores overwrite P, which dV reads: in issue order, so no wait
-        if (S_BUFS == 2 && more && !next_s(it + 1)) break;
-        if (DKV) {
-          if (!accumulate(p_full + 2 * (it % S_BUFS), static_cast<uint32_t>(it / S_BUFS) & 1u, tmem_acc1,
-                          tmem_s(it % S_BUFS), y2_at + (it & 1) * L::YT, it))
-            break;
-          umma_commit_if(on, &y2_empty[it & 1]);
-        }
-        if (S_BUFS == 1 && more && !next_s(it + 1)) break;
-        if (!accumulate(ds_full, static_cast<uint32_t>(it) & 1u, DKV ? tmem_acc2 : tmem_acc1, tmem_dp,
-                        y1_at + slot_a * L::YT, it))
-          break;
-        umma_commit_if(on, &y1_empty[slot_a]);
-        if (++slot_a == Y1_SLOTS) slot_a = 0;
-        if (more) ok = next_dp(it + 1);
-        else umma_commit_if(on, acc_full);
-      }
+    const uint32_t on = elect_one();
+    BwdWalk at;
+    int mode = -1;
+    while (take(w)) {
+      const bool switched = mode >= 0 && mode != w.mode;
+      bool ok = true;
+      if (MODES != MODE_DQ && w.mode == MODE_DKV) ok = bwd_issue<D, MODE_DKV>(on, sh, w, at, switched);
+      else if (MODES != MODE_DKV) ok = bwd_issue<D, MODE_DQ>(on, sh, w, at, switched);
+      if (!ok) break;
+      if (w.n_entry > 0) mode = w.mode;
     }
   } else if (warp >= 4) {
-    // ------------------------------ compute warpgroups ------------------------------
-    // Four compute warpgroups work on every iteration together: warpgroup wg takes columns
-    // [32 wg, 32 wg + 32) of the tile, i.e. 32 columns of entry 2 it + wg / 2.
-    const int wg = (warp - 4) >> 2;
-    const int quad = warp & 3;
-    const int r = quad * 32 + lane;
-    const uint32_t lane_off = static_cast<uint32_t>(quad * 32) << 16;
-    // position in the whole sequence of this thread's row: a key (DKV) or a local query (DQ)
-    const int xi = x0 + r + (DKV ? 0 : args.q_off);
-    const int xi_local = x0 + r;
-    const int row_seg = grouped ? 1 : args.seg[b * args.S + xi];
-    // interval of visible columns (whole-sequence positions): see the mask below
-    int row_a, row_b;
-    if (grouped) {
-      row_a = -(1 << 30);       // everything is visible: padding rows hold zeros and contribute zero
-      row_b = 1 << 30;
-    } else if (DKV) {
-      row_a = args.first_q[b * args.S + xi];
-      row_b = args.run_end[b * args.S + xi];
-    } else {
-      row_a = args.run_start[b * args.S + xi];
-      row_b = (args.lim != nullptr) ? args.lim[b * args.S + xi] : xi;
+    BwdWalk at;
+    while (take(w)) {
+      bool ok = true;
+      if (MODES != MODE_DQ && w.mode == MODE_DKV) ok = bwd_compute<D, MODE_DKV>(sh, dkv_maps, dkv, w, at);
+      else if (MODES != MODE_DKV) ok = bwd_compute<D, MODE_DQ>(sh, dq_maps, dq, w, at);
+      if (!ok) break;
     }
-    const int row_start = sparse ? args.sp.doc_start[b * args.S + xi] : 0;
-    // DKV: the document-relative block of this key is the bit every query column is tested for
-    const int row_blk = (sparse && DKV) ? (xi - row_start) / args.sp.block : 0;
-    float neg_lse2 = 0.f, neg_delta = 0.f;      // DQ: per-row statistics (stored negated, lse in log2 units)
-    if (!DKV) {
-      const size_t at = grouped ? static_cast<size_t>(xi_local) : (static_cast<size_t>(b) * args.Hq + head) * args.Sq + xi_local;
-      neg_lse2 = args.neg_lse2[at];
-      neg_delta = args.neg_delta[at];
-    }
-    bool ok = true;
-    const uint64_t scale2 = pack_f32x2(args.scale_log2, args.scale_log2);
-    const int mine = wg >> 1;               // half of the tile this warpgroup works on
-    // dense walk: (block, head) advance without a division per iteration (the first step moves by one
-    // entry for the warpgroups of the second half, the others by two)
-    int walk_block = 0, walk_head = 0;
-    auto advance = [&](int n) {
-      walk_block += n;
-      while (walk_block >= y_n64) {
-        walk_block -= y_n64;
-        ++walk_head;
-      }
-    };
-    if (!sparse && n_entry > 0) advance(mine);
-    uint32_t y1_slot = 0, y1_phase = 0;       // Y1 slot of iteration `it`
-    for (int it = 0; it < n_iter; ++it) {
-      const int entry_at = 2 * it + mine;
-      const bool real = entry_at < n_entry;
-      int yb, hq;
-      if (sparse) {
-        const int entry = __ldg(it_list + min(entry_at, n_entry - 1));
-        yb = entry & 0xffffff;
-        hq = DKV ? hkv * group + (entry >> 24) : head;
-      } else {
-        yb = y_lo64 + walk_block;
-        hq = DKV ? hkv * group + walk_head : head;
-        advance(2);
-      }
-      const int y0 = yb * 64;                   // (grouped: relative to the group, and nothing is masked)
-      const int base = y0 + 32 * (wg & 1);      // first column of this thread
-      // ---- visibility of this row against its 32 columns, as a bit mask.  The keys a query sees
-      // and the queries that see a key are both contiguous intervals (runs are contiguous):
-      //   DQ   row = query xi,  columns = keys     [start[xi], lim[xi]]
-      //   DKV  row = key xi,    columns = queries  [first_q[xi], end[xi]]
-      // Most tiles are wholly visible: two compares, the mask itself only where some row needs it.
-      unsigned vis = 0xffffffffu;
-      const bool inside = real && row_seg != 0 && row_a <= base && row_b >= base + 31;
-      if (sparse || !__all_sync(0xffffffffu, inside)) {
-        vis = (row_seg == 0 || !real) ? 0u : (bits_from(row_a - base) & bits_upto(row_b - base));
-        if (sparse && vis != 0u) {
-          if (DKV) {
-            if ((row_blk >> 5) >= args.sp.words) {
-              vis = 0u;
-            } else {
-              // when every query of the block selected this key's block the selection adds nothing
-              const unsigned aw = __ldg(args.sp.allsel + ((static_cast<size_t>(b) * args.Hq + hq) * nb64 + yb) * args.sp.words +
-                                        (row_blk >> 5));
-              if (!((aw >> (row_blk & 31)) & 1u)) {
-                // per-query selection bit of this key's block, for the 32 columns of this thread
-                const unsigned* col_sel = args.sp.sel + ((static_cast<size_t>(b) * args.Hq + hq) * args.S + base) * args.sp.words +
-                                          (row_blk >> 5);
-                const int bit = row_blk & 31;
-                unsigned selbits = 0u;
-#pragma unroll 4
-                for (int e = 0; e < 32; ++e)
-                  selbits |= ((__ldg(col_sel + static_cast<size_t>(e) * args.sp.words) >> bit) & 1u) << e;
-                vis &= selbits;
-              }
-            }
-          } else {
-            const SparseRow sr = sparse_row(args.sp, b, head, args.Hq, args.S, xi, row_start, y0, 64);
-            const unsigned above = bits_from(sr.bound - base);               // keys >= bound
-            vis &= (sr.v0 ? ~above : 0u) | (sr.v1 ? above : 0u);
-          }
-        }
-      }
-      const bool warp_all = __all_sync(0xffffffffu, vis == 0xffffffffu);
-      // DKV: per-query statistics of this thread's 32 columns, staged beside the tile by the producer
-      const ulonglong2* lse_col = reinterpret_cast<const ulonglong2*>(smem + L::OFF_LSE + (it & 1) * 512) + 8 * wg;
-      const ulonglong2* delta_col = reinterpret_cast<const ulonglong2*>(smem + L::OFF_DELTA + y1_slot * 512) + 8 * wg;
-      const uint32_t s_at = tmem_s(it % S_BUFS) + lane_off + 32 * wg;
-      const uint32_t dp_at = tmem_dp + lane_off + 32 * wg;
-      if (DKV) {
-        // (the statistics were written by bulk copies: these waits make them visible to the thread)
-        if (!mbar_wait(&y1_full[y1_slot], y1_phase, abort_flag, st, SITE_B_CW_S, budget) ||
-            !mbar_wait(&y2_full[it & 1], static_cast<uint32_t>(it >> 1) & 1u, abort_flag, st, SITE_B_CW_S, budget)) {
-          ok = false;
-          break;
-        }
-      }
-      if (!mbar_wait(&s_full[it % S_BUFS], static_cast<uint32_t>(it / S_BUFS) & 1u, abort_flag, st, SITE_B_CW_S, budget)) {
-        ok = false;
-        break;
-      }
-      // (the accumulate MMAs that read P^T / dS of the previous iteration from these buffers were issued
-      // before the products that refilled them, and the tensor core completes MMAs in issue order)
-      tc_fence_after();
-      // MASKED = false is the path of a warp whose rows all see all 32 columns: no selects.
-      float p[32];
-      auto probabilities = [&](auto masked_tag) {
-        constexpr bool MASKED = decltype(masked_tag)::value;
-        uint32_t sc[32];
-        tmem_ld32(s_at, sc);
-        tmem_ld_wait();
-#pragma unroll
-        for (int half = 0; half < 2; ++half) {
-          uint32_t pw[8];
-#pragma unroll
-          for (int e4 = 0; e4 < 4; ++e4) {                 // groups of four columns
-            uint64_t l2[2];                                // negated statistics, two columns per word
-            if (DKV) {
-              const ulonglong2 lv = lse_col[half * 4 + e4];
-              l2[0] = lv.x;
-              l2[1] = lv.y;
-            } else {
-              l2[0] = l2[1] = pack_f32x2(neg_lse2, neg_lse2);
-            }
-            // p = exp2(s * scale - lse): two columns per packed instruction
-#pragma unroll
-            for (int pr = 0; pr < 2; ++pr) {
-              const int e = half * 16 + e4 * 4 + pr * 2;
-              const uint64_t x2 = fma_f32x2(pack_f32x2(__uint_as_float(sc[e]), __uint_as_float(sc[e + 1])), scale2, l2[pr]);
-              float xa, xb;
-              unpack_f32x2(x2, xa, xb);
-              float pa = fast_exp2(xa), pb = fast_exp2(xb);
-              if (MASKED) {
-                if (!((vis >> e) & 1u)) pa = 0.f;
-                if (!((vis >> (e + 1)) & 1u)) pb = 0.f;
-              }
-              p[e] = pa;
-              p[e + 1] = pb;
-              if (DKV) pw[e4 * 2 + pr] = pack_bf16(pa, pb);
-            }
-          }
-          if (DKV) {
-            tmem_st8(s_at + 16 * half, pw);
-            tmem_st_wait();
-            tc_fence_before();
-            __syncwarp();
-            if (lane == 0) mbar_arrive(&p_full[2 * (it % S_BUFS) + half]);
-          }
-        }
-      };
-      if (warp_all) probabilities(std::false_type{});
-      else probabilities(std::true_type{});
-      if (!mbar_wait(dp_full, static_cast<uint32_t>(it) & 1u, abort_flag, st, SITE_B_CW_S, budget)) {
-        ok = false;
-        break;
-      }
-      tc_fence_after();
-      uint32_t rd[32];
-      tmem_ld32(dp_at, rd);
-      tmem_ld_wait();
-      // dS = p * (dP - delta)
-#pragma unroll
-      for (int half = 0; half < 2; ++half) {
-        uint32_t dw[8];
-#pragma unroll
-        for (int e4 = 0; e4 < 4; ++e4) {
-          uint64_t dl[2];
-          if (DKV) {
-            const ulonglong2 dv = delta_col[half * 4 + e4];
-            dl[0] = dv.x;
-            dl[1] = dv.y;
-          } else {
-            dl[0] = dl[1] = pack_f32x2(neg_delta, neg_delta);
-          }
-#pragma unroll
-          for (int pr = 0; pr < 2; ++pr) {
-            const int e = half * 16 + e4 * 4 + pr * 2;
-            const uint64_t d2 = add_f32x2(pack_f32x2(__uint_as_float(rd[e]), __uint_as_float(rd[e + 1])), dl[pr]);
-            const uint64_t ds2 = mul_f32x2(pack_f32x2(p[e], p[e + 1]), d2);
-            float da, db;
-            unpack_f32x2(ds2, da, db);
-            dw[e4 * 2 + pr] = pack_bf16(da, db);
-          }
-        }
-        tmem_st8(dp_at + 16 * half, dw);
-        tmem_st_wait();
-        tc_fence_before();
-        __syncwarp();
-        if (lane == 0) mbar_arrive(&ds_full[half]);
-      }
-      if (++y1_slot == Y1_SLOTS) {
-        y1_slot = 0;
-        y1_phase ^= 1u;
-      }
-    }
-    // the epilogue pairs the warpgroups: pair u converts accumulator u, each warpgroup half of it
-    const int u = wg & 1;
-    const int half = wg >> 1;
-    // ---- epilogue: accumulators -> bf16 -> staging -> TMA store ----
-    if (ok && n_iter > 0) {
-      ok = mbar_wait(acc_full, 0, abort_flag, st, SITE_B_CW_ACC, budget);
-      tc_fence_after();
-    }
-    const bool any_bad = named_bar_or(2 + u, 256, !ok);
-    const bool writes = DKV || (u == 0);
-    if (!any_bad && writes) {
-      // DKV: warpgroup 0 stores dV, warpgroup 1 stores dK (scaled); DQ: warpgroup 0 stores dQ (scaled).
-      const uint32_t acc = (DKV && u == 1) ? tmem_acc2 : tmem_acc1;
-      const float mul = (DKV && u == 0) ? 1.f : args.scale;
-      uint8_t* stage_buf = smem + L::OFF_X + u * L::XT;      // the resident tile u is dead now: [HALVES][128 rows][128 B]
-      // the two warpgroups of the pair convert half of the head dimension each
-#pragma unroll 1
-      for (int c = half * (D / 64); c < (half + 1) * (D / 64); ++c) {
-        uint32_t rr[32];
-        if (n_iter > 0) {
-          tmem_ld32(acc + lane_off + c * 32, rr);
-          tmem_ld_wait();
-        } else {
-#pragma unroll
-          for (int e = 0; e < 32; ++e) rr[e] = 0u;
-        }
-#pragma unroll
-        for (int jj = 0; jj < 4; ++jj) {
-          uint4 v;
-          v.x = pack_bf16(__uint_as_float(rr[jj * 8 + 0]) * mul, __uint_as_float(rr[jj * 8 + 1]) * mul);
-          v.y = pack_bf16(__uint_as_float(rr[jj * 8 + 2]) * mul, __uint_as_float(rr[jj * 8 + 3]) * mul);
-          v.z = pack_bf16(__uint_as_float(rr[jj * 8 + 4]) * mul, __uint_as_float(rr[jj * 8 + 5]) * mul);
-          v.w = pack_bf16(__uint_as_float(rr[jj * 8 + 6]) * mul, __uint_as_float(rr[jj * 8 + 7]) * mul);
-          *reinterpret_cast<uint4*>(stage_buf + (c / 2) * 16384 + sw128_offset(r, (c % 2) * 4 + jj)) = v;
-        }
-      }
-      fence_proxy_async_smem();
-      named_bar_sync(4 + u, 256);
-      if (r == 0 && half == 0) {
-        const CUtensorMap* mo = (DKV && u == 1) ? &maps.out2 : &maps.out1;
-        const int oh = DKV ? hkv : head;
-        const int ob = DKV ? kbatch : b;
-#pragma unroll
-        for (int hf = 0; hf < HALVES; ++hf) {
-          // grouped dK / dV: the history part joins what the own-block pass stored (one CTA per tile, so the sum
-          // does not depend on timing)
-          if (DKV && grouped) tma_reduce_add_4d(mo, stage_buf + hf * 16384, hf * 64, oh, x0, ob);
-          else tma_store_4d(mo, stage_buf + hf * 16384, hf * 64, oh, x0, ob);
-        }
-        tma_commit_group();
-        tma_wait_group<0>();
-      }
-    }
+    tma_wait_group<0>();
   }
 
   tc_fence_before();
   __syncthreads();
   if (warp == 1) {
     tc_fence_after();
-    tmem_dealloc(tmem_base, 512);
+    tmem_dealloc(sh.tmem_base, 512);
   }
-}
-
-template <int D, int MODE>
-__global__ void __launch_bounds__(BWD_THREADS, 1)
-attn_bwd_kernel(const __grid_constant__ BwdMaps maps, const __grid_constant__ BwdArgs args) {
-  bwd_cta<D, MODE>(maps, args, static_cast<int>(blockIdx.x));
-}
-
-// Both modes in one launch: neither reads what the other writes, so the dQ work items fill the SMs that the last, long
-// dK/dV items leave idle, and a short call pays for one launch less (8 image rows of 4096 tokens, 12 / 2 heads, forward and
-// backward: 1014 -> 969 us; 2 rows of 256 tokens, with the launches' host side: 76 -> 38 us).
-template <int D>
-__global__ void __launch_bounds__(BWD_THREADS, 1)
-attn_bwd_both_kernel(const __grid_constant__ BwdMaps dkv_maps, const __grid_constant__ BwdMaps dq_maps,
-                     const __grid_constant__ BwdArgs dkv, const __grid_constant__ BwdArgs dq, const int dkv_items) {
-  const int cta = static_cast<int>(blockIdx.x);
-  if (cta < dkv_items) bwd_cta<D, MODE_DKV>(dkv_maps, dkv, cta);
-  else bwd_cta<D, MODE_DQ>(dq_maps, dq, cta - dkv_items);
 }
 
 // Maps, arguments and number of work items of one mode.
@@ -681,14 +908,22 @@ int prepare_bwd(const BwdCall& c, BwdMaps* maps, BwdArgs* args, int* items) {
   return 0;
 }
 
-template <int D, typename Kernel>
-int configure_bwd(Kernel kern, int* configured_dev) {
+template <int D, int MODES>
+int launch_items(const BwdMaps& dkv_maps, const BwdMaps& dq_maps, const BwdArgs& dkv, const BwdArgs& dq, int dkv_items,
+                 int dq_items, void* stream) {
+  const int items = max(dkv_items, 0) + max(dq_items, 0);
+  if (items == 0) return 0;
+  auto kern = attn_bwd_kernel<D, MODES>;
+  static int configured_dev = -1;
   int dev = 0;
   cudaGetDevice(&dev);
-  if (*configured_dev != dev) {
+  if (configured_dev != dev) {
     CTB_CUDA_OK(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, BwdSmem<D>::BYTES));
-    *configured_dev = dev;
+    configured_dev = dev;
   }
+  kern<<<items, BWD_THREADS, BwdSmem<D>::BYTES, static_cast<cudaStream_t>(stream)>>>(dkv_maps, dq_maps, dkv, dq,
+                                                                                   max(dkv_items, 0));
+  CTB_CUDA_OK(cudaGetLastError());
   return 0;
 }
 
@@ -698,16 +933,13 @@ int launch_bwd(const BwdCall& c) {
   BwdArgs args{};
   int items = 0;
   if (prepare_bwd<D, MODE>(c, &maps, &args, &items)) return 1;
-  if (items <= 0) return 0;
-  auto kern = attn_bwd_kernel<D, MODE>;
-  static int configured_dev = -1;
-  if (configure_bwd<D>(kern, &configured_dev)) return 1;
-  kern<<<items, BWD_THREADS, BwdSmem<D>::BYTES, static_cast<cudaStream_t>(c.stream)>>>(maps, args);
-  CTB_CUDA_OK(cudaGetLastError());
-  return 0;
+  return launch_items<D, MODE>(maps, maps, args, args, items, 0, c.stream);
 }
 
-// dK/dV as described by `dkv` and dQ as described by `dq`, in one launch.
+// dK/dV as described by `dkv` and dQ as described by `dq`, in one launch: neither reads what the other writes, so the dQ
+// work items fill the SMs that the last, long dK/dV items leave idle, and a short call pays for one launch less (8 image
+// rows of 4096 tokens, 12 / 2 heads, forward and backward: 1014 -> 969 us; 2 rows of 256 tokens, with the launches' host
+// side: 76 -> 38 us).
 template <int D>
 int launch_bwd_both(const BwdCall& dkv, const BwdCall& dq) {
   BwdMaps dkv_maps, dq_maps;
@@ -715,43 +947,11 @@ int launch_bwd_both(const BwdCall& dkv, const BwdCall& dq) {
   int dkv_items = 0, dq_items = 0;
   if (prepare_bwd<D, MODE_DKV>(dkv, &dkv_maps, &dkv_args, &dkv_items)) return 1;
   if (prepare_bwd<D, MODE_DQ>(dq, &dq_maps, &dq_args, &dq_items)) return 1;
-  dkv_items = max(dkv_items, 0);
-  dq_items = max(dq_items, 0);
-  if (dkv_items + dq_items == 0) return 0;
-  auto kern = attn_bwd_both_kernel<D>;
-  static int configured_dev = -1;
-  if (configure_bwd<D>(kern, &configured_dev)) return 1;
-  kern<<<dkv_items + dq_items, BWD_THREADS, BwdSmem<D>::BYTES, static_cast<cudaStream_t>(dkv.stream)>>>(
-      dkv_maps, dq_maps, dkv_args, dq_args, dkv_items);
-  CTB_CUDA_OK(cudaGetLastError());
-  return 0;
+  return launch_items<D, MODE_BOTH>(dkv_maps, dq_maps, dkv_args, dq_args, dkv_items, dq_items, dkv.stream);
 }
 
 }  // namespace attn
 }  // namespace ctb
-
-// mode 0: dK/dV kernel, mode 1: dQ kernel.  All tensors are [B,S,H,D] views with a row
-// stride; neg_lse2 = -lse * log2(e) and neg_delta = -sum_d O dO are [B,Hq,S] fp32 (ctb_attn_bwd_stats).
-CTB_API int ctb_attn_bwd(int mode, const void* q, const void* k, const void* v, const void* dout, void* dq, void* dk,
-                         void* dv, const float* neg_lse2, const float* neg_delta, const int* seg, const int* lim,
-                         const int* kv_lo, const int* kv_hi, const int* q_lo, const int* q_hi, const int* run_start, const int* run_end, const int* first_q, int B, int S, int Hq,
-                         int Hkv, int D, long q_rs, long k_rs, long v_rs, long do_rs, long dq_rs, long dk_rs,
-                         long dv_rs, float scale, long long spin_budget, void* stream) {
-  if (S % 128) return ctb::fail("attention: sequence length must be a multiple of 128");
-  if (Hq % Hkv) return ctb::fail("attention: Hq must be a multiple of Hkv");
-  ctb::attn::BwdCall c{};
-  c.q = q; c.k = k; c.v = v; c.dout = dout; c.dq = dq; c.dk = dk; c.dv = dv; c.neg_lse2 = neg_lse2; c.neg_delta = neg_delta;
-  c.seg = seg; c.lim = lim; c.kv_lo = kv_lo; c.kv_hi = kv_hi; c.q_lo = q_lo; c.q_hi = q_hi;
-  c.run_start = run_start; c.run_end = run_end; c.first_q = first_q;
-  c.B = B; c.S = S; c.Hq = Hq; c.Hkv = Hkv;
-  c.q_row_stride = q_rs; c.k_row_stride = k_rs; c.v_row_stride = v_rs; c.do_row_stride = do_rs;
-  c.dq_row_stride = dq_rs; c.dk_row_stride = dk_rs; c.dv_row_stride = dv_rs;
-  c.scale = scale; c.spin_budget = spin_budget; c.stream = stream;
-  using namespace ctb::attn;
-  if (D == 128) return mode == 0 ? launch_bwd<128, MODE_DKV>(c) : launch_bwd<128, MODE_DQ>(c);
-  if (D == 64) return mode == 0 ? launch_bwd<64, MODE_DKV>(c) : launch_bwd<64, MODE_DQ>(c);
-  return ctb::fail("attention: head_dim must be 64 or 128");
-}
 
 // Whole backward of the queries [q_off, q_off + Sq) of every row (all of them: q_off 0, Sq = S): q / out / dout / dq, lse,
 // neg_lse2 and neg_delta hold those queries; k / v / dk / dv cover all S keys (with fewer queries dk / dv are partial sums).

@@ -3,7 +3,7 @@
 //
 //   key j is visible to query i  <=>  seg[j] == seg[i] != 0  and  j <= max(i, attention_end[i])
 //
-// One CTA owns 256 consecutive query rows of one (batch, query head): two 128-row tiles
+// A work item is 256 consecutive query rows of one (batch, query head): two 128-row tiles
 // that ping-pong so the tensor core computes one tile's S = Q K^T / O += P V while the
 // other tile's softmax runs.
 //   warp 0      TMA producer (Q tiles once, then K(j), V(j) through a 5-slot ring)
@@ -23,6 +23,15 @@
 // the FMA pipe (the ex2 unit alone takes 1024 cycles per 128 x 128 tile).  The issuing warps run converged
 // (elect_one).  A tile joins the walk at its own first key tile, not at its neighbour's.  One document of
 // 16384 tokens, 8 / 2 heads, D = 128: 0.483 -> 0.430 ms (1280 TFLOP/s causal).
+//
+// A CTA stays on its SM and takes over work items of the grid that have not started (cluster launch control), so that
+// the next item's Q, keys and first scores overlap this one's last product and its results.  A CTA of its own for each item
+// paid for its start, its first copies and its last stores one after the other: 15000 cycles of the 55000 of an item of
+// packed rows, 20000 of the 49000 of one of image rows (next to 1684 per pair of tiles on a long document).  The next item
+// is asked for when this one's last copies are issued, not earlier: an item that waits behind a long one could have run
+// elsewhere.  O is staged in two slots of the K / V ring, which leaves Q's place to the next item.  With the same change
+// to the backward, forward and backward: 4 packed rows of 4096 (32 / 8 heads) 1578 -> 1504 us under the power cap, 8 image
+// rows of 4096 (12 / 2 heads) 969 -> 935 us, one document of 32768 unchanged.
 // KV blocks outside [kv_lo, kv_hi) of a query block are never visited (block skipping from
 // segment summaries); rows without any visible key produce O = 0 and LSE = 0.
 //
@@ -47,6 +56,7 @@ enum : unsigned {
   SITE_F_SM_S = 0x0205,
   SITE_F_SM_PV = 0x0206,
   SITE_F_KV_FLAG = 0x0207,
+  SITE_F_ITEM = 0x0208,
 };
 
 template <int D>
@@ -56,8 +66,97 @@ struct FwdSmem {
   static constexpr int OFF_Q = 0;                  // two Q tiles; each doubles as the staging tile of its O
   static constexpr int OFF_KV = 2 * QT;
   static constexpr int OFF_BAR = OFF_KV + KV_SLOTS * QT;
-  static constexpr int BYTES = OFF_BAR + 256 + 1024;
+  static constexpr int OFF_ITEMS = OFF_BAR + 320;  // answer of the work request, two work items
+  static constexpr int BYTES = OFF_BAR + 512 + 1024;
 };
+
+// One work item (256 query rows of one head), resolved once by the producer warp and handed to the other roles through
+// shared memory.  Query tile t walks the key tiles [s[t], n[t]) of the item's walk.
+struct alignas(16) FwdItem {
+  int state;         // 0: work, -1: no more work, -2: unused capacity of a grouped launch
+  int b, h;          // batch and head of Q / O (0 for gathered rows)
+  int hkv, kb;       // kv head and batch of the keys
+  int q0;            // first row of Q / O
+  int lo;            // first key tile of the walk
+  int first_key;     // grouped: first key of the group's block
+  int n[2], s[2];
+  int valid;         // bit t: query tile t exists
+  int real;          // grouped: rows that are real
+  int list;          // block-sparse: offset of the item's key tiles in it_list
+  int pad;
+};
+static_assert(sizeof(FwdItem) == 64, "four 16-byte reads");
+
+template <bool SPARSE>
+__device__ __forceinline__ FwdItem fwd_item(const FwdArgs& args, const int cta) {
+  const bool grouped = args.grp.desc != nullptr;
+  FwdItem w;
+  int4 gd = make_int4(0, 0, 0, 0);
+  if (grouped) gd = __ldg(args.grp.desc + cta);      // this item's 256 gathered rows against one key block (see GroupArgs)
+  w.state = grouped && gd.w <= 0 ? -2 : 0;           // capacity beyond the rows in use
+  const int nqp = (args.Sq + 255) / 256;
+  int idx = cta;
+  w.h = grouped ? 0 : idx % args.Hq;
+  idx /= args.Hq;
+  w.b = grouped ? 0 : idx % args.B;
+  const int pair = grouped ? cta : nqp - 1 - idx / args.B;
+  w.q0 = pair * 256;
+  w.hkv = grouped ? (gd.x >> 16) : w.h / (args.Hq / args.Hkv);
+  w.kb = grouped ? (gd.x & 0xffff) : w.b;
+  w.first_key = gd.y;
+  w.real = gd.w;
+  w.list = 0;
+  w.pad = 0;
+  w.valid = 0;
+  const int nqb = args.S / 128;
+  int lo_t[2], hi_t[2];
+#pragma unroll
+  for (int t = 0; t < 2; ++t) {
+    const bool valid = grouped ? (t * 128 < gd.w) : (w.q0 + t * 128) < args.Sq;
+    w.valid |= valid ? 1 << t : 0;
+    lo_t[t] = 0;
+    hi_t[t] = 0;
+    if (valid && !grouped) {
+      const int qb = (args.q_off + w.q0) / 128 + t;      // query block in the whole sequence
+      const int lo_tok = args.kv_lo[w.b * nqb + qb];
+      const int hi_tok = args.kv_hi[w.b * nqb + qb];
+      if (hi_tok > lo_tok) {
+        lo_t[t] = lo_tok / 128;
+        hi_t[t] = (hi_tok + 127) / 128;
+      }
+    }
+  }
+  w.lo = 0;
+  if (hi_t[0] > lo_t[0] && hi_t[1] > lo_t[1]) w.lo = min(lo_t[0], lo_t[1]);
+  else if (hi_t[0] > lo_t[0]) w.lo = lo_t[0];
+  else if (hi_t[1] > lo_t[1]) w.lo = lo_t[1];
+#pragma unroll
+  for (int t = 0; t < 2; ++t) {
+    w.n[t] = (hi_t[t] > lo_t[t]) ? hi_t[t] - w.lo : 0;
+    // iteration at which a tile joins the walk: key tiles before its own range are masked for all its rows
+    w.s[t] = (!SPARSE && w.n[t] > 0) ? lo_t[t] - w.lo : 0;
+  }
+  // Block-sparse routing: both query tiles walk the listed key tiles (rows that selected nothing in
+  // a tile see it fully masked).
+  if (SPARSE) {
+    int cnt;
+    sparse_list(args.sp, cta, w.list, cnt);
+    w.n[0] = (w.valid & 1) ? cnt : 0;
+    w.n[1] = (w.valid & 2) ? cnt : 0;
+  }
+  if (grouped) {
+    w.n[0] = args.grp.block / 128;
+    w.n[1] = (w.valid & 2) ? w.n[0] : 0;
+  }
+  return w;
+}
+
+// first key of the i-th key tile that an item visits
+template <bool SPARSE>
+__device__ __forceinline__ int fwd_key(const FwdArgs& args, const FwdItem& w, int i) {
+  if (args.grp.desc != nullptr) return w.first_key + i * 128;
+  return (SPARSE ? __ldg(args.sp.it_list + w.list + i) : w.lo + i) * 128;
+}
 
 // SPARSE: the key tiles come from a routing list.  Nearly every warp then has rows that do not see a tile, so that
 // kernel has no second copy of the exponentials for wholly visible ones; in one kernel with the dense walk the two
@@ -76,112 +175,67 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constant
   extern __shared__ uint8_t smem_raw[];
   uint8_t* smem = smem_raw + ((1024u - (smem_u32(smem_raw) & 1023u)) & 1023u);
   uint64_t* q_full = reinterpret_cast<uint64_t*>(smem + L::OFF_BAR);
-  uint64_t* kv_full = q_full + 1;
+  uint64_t* q_empty = q_full + 1;
+  uint64_t* kv_full = q_empty + 1;
   uint64_t* kv_empty = kv_full + KV_SLOTS;
   uint64_t* s_full = kv_empty + KV_SLOTS;
   uint64_t* p_full = s_full + 2;           // [2][2] tile t: half of the columns of P written
-  uint64_t* pv_done = p_full + 4;
-  uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(pv_done + 2);
+  uint64_t* pv_done = p_full + 4;          // [2]
+  uint64_t* o_empty = pv_done + 2;         // [2] the results of tile t have been read
+  uint64_t* o_slot = o_empty + 2;          // [KV_SLOTS] the slot is left to the results of a tile
+  uint64_t* item_full = o_slot + KV_SLOTS; // [2] work item u resolved
+  uint64_t* item_empty = item_full + 2;    // [2] and read by the MMA warp and the softmax warps
+  uint64_t* answer_full = item_empty + 2;
+  uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(answer_full + 1);
   volatile uint32_t* abort_flag = tmem_slot + 1;
+  static_assert((2 + 3 * KV_SLOTS + 2 + 4 + 2 + 2 + 4 + 1) * 8 + 8 <= 320, "barrier block");
+  const uint32_t answer = smem_u32(smem + L::OFF_ITEMS);
+  FwdItem* items = reinterpret_cast<FwdItem*>(smem + L::OFF_ITEMS + 16);
 
   const int warp = uniform_warp_index();
   const int lane = threadIdx.x & 31;
   DeviceStatus* st = args.status;
   const long long budget = args.spin_budget;
-
-  // ---- work item ----
-  // grouped MoBA: this CTA's 256 gathered rows against one key block (see GroupArgs)
   const bool grouped = args.grp.desc != nullptr;
-  int4 gd = make_int4(0, 0, 0, 0);
-  if (grouped) {
-    gd = __ldg(args.grp.desc + blockIdx.x);
-    if (gd.w <= 0) return;                       // capacity beyond the rows in use: the whole CTA leaves
-  }
-  const int nqp = (args.Sq + 255) / 256;
-  int idx = blockIdx.x;
-  const int h = grouped ? 0 : idx % args.Hq;
-  idx /= args.Hq;
-  const int b = grouped ? 0 : idx % args.B;
-  const int pair = grouped ? static_cast<int>(blockIdx.x) : nqp - 1 - idx / args.B;
-  const int q0 = pair * 256;
-  const int hkv = grouped ? (gd.x >> 16) : h / (args.Hq / args.Hkv);
-  const int kb = grouped ? (gd.x & 0xffff) : b;  // batch of the keys
-  const int nqb = args.S / 128;
-  bool tile_valid[2];
-  int lo_t[2], hi_t[2];
-#pragma unroll
-  for (int t = 0; t < 2; ++t) {
-    tile_valid[t] = grouped ? (t * 128 < gd.w) : (q0 + t * 128) < args.Sq;
-    lo_t[t] = 0;
-    hi_t[t] = 0;
-    if (tile_valid[t] && !grouped) {
-      const int qb = (args.q_off + q0) / 128 + t;      // query block in the whole sequence
-      const int lo_tok = args.kv_lo[b * nqb + qb];
-      const int hi_tok = args.kv_hi[b * nqb + qb];
-      if (hi_tok > lo_tok) {
-        lo_t[t] = lo_tok / 128;
-        hi_t[t] = (hi_tok + 127) / 128;
-      }
-    }
-  }
-  int lo = 0;
-  if (hi_t[0] > lo_t[0] && hi_t[1] > lo_t[1]) lo = min(lo_t[0], lo_t[1]);
-  else if (hi_t[0] > lo_t[0]) lo = lo_t[0];
-  else if (hi_t[1] > lo_t[1]) lo = lo_t[1];
-  int n0 = (hi_t[0] > lo_t[0]) ? hi_t[0] - lo : 0;
-  int n1 = (hi_t[1] > lo_t[1]) ? hi_t[1] - lo : 0;
-  // Block-sparse routing: both query tiles walk the listed key tiles (rows that selected nothing in
-  // a tile see it fully masked).
   constexpr bool sparse = SPARSE;
-  const int* kv_list = nullptr;
-  if (sparse) {
-    int base, cnt;
-    sparse_list(args.sp, blockIdx.x, base, cnt);
-    kv_list = args.sp.it_list + base;
-    n0 = tile_valid[0] ? cnt : 0;
-    n1 = tile_valid[1] ? cnt : 0;
-  }
-  if (grouped) {
-    n0 = args.grp.block / 128;
-    n1 = tile_valid[1] ? n0 : 0;
-  }
-  const int nmax = max(n0, n1);
-  // iteration at which a tile joins the walk: key tiles before its own range are masked for all its rows
-  int s0 = 0, s1 = 0;
-  if (!grouped && !sparse) {
-    if (n0 > 0) s0 = lo_t[0] - lo;
-    if (n1 > 0) s1 = lo_t[1] - lo;
-  }
-  // first key of the i-th key tile this CTA visits
-  auto kv_pos = [&](int i) -> int {
-    return grouped ? gd.y + i * 128 : (sparse ? __ldg(kv_list + i) : lo + i) * 128;
+
+  // Q tiles of an item.  A tile without keys has no use for it
+  auto load_q = [&](uint32_t on, const FwdItem& w) {
+    mbar_expect_tx_if(on, q_full, ((w.n[0] > 0 ? 1u : 0u) + (w.n[1] > 0 ? 1u : 0u)) * L::QT);
+    for (int t = 0; t < 2; ++t) {
+      if (w.n[t] == 0) continue;
+#pragma unroll
+      for (int hf = 0; hf < HALVES; ++hf)
+        tma_load_4d_if(on, smem + L::OFF_Q + t * L::QT + hf * 16384, &map_q, q_full, hf * 64, w.h, w.q0 + t * 128, w.b);
+    }
   };
 
-  if (threadIdx.x == 0) {
-    mbar_init(q_full, 1);
-    for (int s = 0; s < KV_SLOTS; ++s) {
-      mbar_init(&kv_full[s], 1);
-      mbar_init(&kv_empty[s], 1);
-    }
-    for (int t = 0; t < 2; ++t) {
-      mbar_init(&s_full[t], 1);
-      mbar_init(&p_full[2 * t], 4);        // one arrival per warp
-      mbar_init(&p_full[2 * t + 1], 4);
-      mbar_init(&pv_done[t], 1);
-    }
-    *abort_flag = 0u;
-    mbar_fence_init();
-    if (nmax > 0) {
-      // Q is on its way while TMEM is allocated.  A tile without keys has no use for it, and its warps stage
-      // zeros for O in that place at once
-      mbar_expect_tx(q_full, ((n0 > 0 ? 1u : 0u) + (n1 > 0 ? 1u : 0u)) * L::QT);
-      for (int t = 0; t < 2; ++t) {
-        if ((t == 0 ? n0 : n1) == 0) continue;
-#pragma unroll
-        for (int hf = 0; hf < HALVES; ++hf)
-          tma_load_4d(smem + L::OFF_Q + t * L::QT + hf * 16384, &map_q, q_full, hf * 64, h, q0 + t * 128, b);
+  FwdItem w;
+  if (warp == 0) {
+    if (lane == 0) {
+      mbar_init(q_full, 1);
+      mbar_init(q_empty, 1);
+      for (int s = 0; s < KV_SLOTS; ++s) {
+        mbar_init(&kv_full[s], 1);
+        mbar_init(&kv_empty[s], 1);
+        mbar_init(&o_slot[s], 1);
       }
+      for (int t = 0; t < 2; ++t) {
+        mbar_init(&s_full[t], 1);
+        mbar_init(&p_full[2 * t], 4);        // one arrival per warp
+        mbar_init(&p_full[2 * t + 1], 4);
+        mbar_init(&pv_done[t], 1);
+        mbar_init(&o_empty[t], 4);
+        mbar_init(&item_full[t], 1);
+        mbar_init(&item_empty[t], 1 + 8);
+      }
+      mbar_init(answer_full, 1);
+      *abort_flag = 0u;
+      mbar_fence_init();
     }
+    __syncwarp();
+    w = fwd_item<SPARSE>(args, static_cast<int>(blockIdx.x));
+    if (w.state == 0 && max(w.n[0], w.n[1]) > 0) load_q(elect_one(), w);      // on its way while TMEM is allocated
   }
   if (warp == 1) {
     tmem_alloc(tmem_slot, 512);
@@ -194,134 +248,222 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constant
   auto tmem_s_of = [&](int t) -> uint32_t { return tmem_base + static_cast<uint32_t>(t) * 128u; };
   auto tmem_o_of = [&](int t) -> uint32_t { return tmem_base + 256u + static_cast<uint32_t>(t) * D; };
 
+  // the next work item, for the roles that are told of it
+  uint32_t turn = 0;
+  auto take = [&]() -> bool {
+    const uint32_t u = turn & 1u;
+    if (!mbar_wait_warp(&item_full[u], (turn >> 1) & 1u, abort_flag, st, SITE_F_ITEM, budget)) return false;
+    const int4* from = reinterpret_cast<const int4*>(&items[u]);
+    int4* to = reinterpret_cast<int4*>(&w);
+#pragma unroll
+    for (int i = 0; i < 4; ++i) to[i] = from[i];
+    __syncwarp();
+    if (lane == 0) mbar_arrive(&item_empty[u]);
+    ++turn;
+    return w.state == 0;
+  };
+
   if (warp < 4) {
   // the service warpgroup hands most of its registers to the two softmax warpgroups, which hold a
   // whole 128-column score row per thread
   asm volatile("setmaxnreg.dec.sync.aligned.u32 72;" ::: "memory");
   if (warp == 0) {
     // ------------------------------ producer ------------------------------
-    if (nmax > 0) {
-      const uint32_t on = elect_one();            // the whole warp walks, one lane issues
-      uint32_t slot = 0, phase = 0;
-      bool ok = true;
-      for (int i = 0; ok && i < nmax; ++i) {
-        const int k0 = kv_pos(i);
-        if (args.kvf.flags != nullptr) {
-          // gathered K / V (see KvFlags): the rows [k0, k0 + 128) of batch kb must have landed
-          const long e0 = (static_cast<long>(kb) * args.S + k0) * args.kvf.row_elems;
-          const long e1 = e0 + 128 * args.kvf.row_elems - 1;
-          for (long f = e0 / args.kvf.chunk; ok && f <= e1 / args.kvf.chunk; ++f) {
-            const long long t0 = clock64();
-            while (true) {
-              unsigned got;
-              asm volatile("ld.acquire.gpu.global.u32 %0, [%1];" : "=r"(got) : "l"(args.kvf.flags + f) : "memory");
-              if (got >= args.kvf.epoch) break;
-              if (*abort_flag || clock64() - t0 > budget) {
-                *abort_flag = 1u;
-                report_failure(st, SITE_F_KV_FLAG, static_cast<unsigned>(f), args.kvf.epoch);
-                ok = false;
-                break;
-              }
-              __nanosleep(64);
-            }
-          }
-          ok = __all_sync(0xffffffffu, ok);
-          if (!ok) break;
-          fence_proxy_async_all();   // generic-proxy writes of the pull CTAs -> async-proxy reads below
-        }
-#pragma unroll 1
-        for (int which = 0; which < 2; ++which) {
-          if (!mbar_wait_warp(&kv_empty[slot], phase ^ 1u, abort_flag, st, SITE_F_PROD, budget)) {
-            ok = false;
-            break;
-          }
-          mbar_expect_tx_if(on, &kv_full[slot], L::QT);
-          uint8_t* dst = smem + L::OFF_KV + slot * L::QT;
-          const CUtensorMap* m = which == 0 ? &map_k : &map_v;
-#pragma unroll
-          for (int hf = 0; hf < HALVES; ++hf) tma_load_4d_if(on, dst + hf * 16384, m, &kv_full[slot], hf * 64, hkv, k0, kb);
-          if (++slot == KV_SLOTS) {
-            slot = 0;
-            phase ^= 1u;
-          }
-        }
+    const uint32_t on = elect_one();            // the whole warp walks, one lane issues
+    uint32_t slot = 0, phase = 0, loads = 0, requests = 0;
+    bool ok = true, loaded = true;              // the first item's Q is on its way
+    auto next_slot = [&]() {
+      if (++slot == KV_SLOTS) {
+        slot = 0;
+        phase ^= 1u;
       }
+    };
+    while (ok) {
+      if (w.state != -2) {                      // (unused capacity is not passed on)
+        const uint32_t u = turn & 1u;
+        ok = mbar_wait_warp(&item_empty[u], ((turn >> 1) & 1u) ^ 1u, abort_flag, st, SITE_F_ITEM, budget);
+        if (!ok) break;
+        if (lane == 0) {
+          items[u] = w;
+          mbar_arrive(&item_full[u]);
+        }
+        ++turn;
+        if (w.state < 0) break;
+        const int nmax = max(w.n[0], w.n[1]);
+        if (nmax > 0) {
+          if (!loaded) {
+            ok = mbar_wait_warp(q_empty, (loads & 1u) ^ 1u, abort_flag, st, SITE_F_PROD, budget);
+            if (!ok) break;
+            load_q(on, w);
+          }
+          ++loads;
+        }
+        for (int i = 0; ok && i < nmax; ++i) {
+          const int k0 = fwd_key<SPARSE>(args, w, i);
+          if (args.kvf.flags != nullptr) {
+            // gathered K / V (see KvFlags): the rows [k0, k0 + 128) of batch kb must have landed
+            const long e0 = (static_cast<long>(w.kb) * args.S + k0) * args.kvf.row_elems;
+            const long e1 = e0 + 128 * args.kvf.row_elems - 1;
+            for (long f = e0 / args.kvf.chunk; ok && f <= e1 / args.kvf.chunk; ++f) {
+              const long long t0 = clock64();
+              while (true) {
+                unsigned got;
+                asm volatile("ld.acquire.gpu.global.u32 %0, [%1];" : "=r"(got) : "l"(args.kvf.flags + f) : "memory");
+                if (got >= args.kvf.epoch) break;
+                if (*abort_flag || clock64() - t0 > budget) {
+                  *abort_flag = 1u;
+                  report_failure(st, SITE_F_KV_FLAG, static_cast<unsigned>(f), args.kvf.epoch);
+                  ok = false;
+                  break;
+                }
+                __nanosleep(64);
+              }
+            }
+            ok = __all_sync(0xffffffffu, ok);
+            if (!ok) break;
+            fence_proxy_async_all();   // generic-proxy writes of the pull CTAs -> async-proxy reads below
+          }
+#pragma unroll 1
+          for (int which = 0; which < 2; ++which) {
+            if (!mbar_wait_warp(&kv_empty[slot], phase ^ 1u, abort_flag, st, SITE_F_PROD, budget)) {
+              ok = false;
+              break;
+            }
+            mbar_expect_tx_if(on, &kv_full[slot], L::QT);
+            uint8_t* dst = smem + L::OFF_KV + slot * L::QT;
+            const CUtensorMap* m = which == 0 ? &map_k : &map_v;
+#pragma unroll
+            for (int hf = 0; hf < HALVES; ++hf) tma_load_4d_if(on, dst + hf * 16384, m, &kv_full[slot], hf * 64, w.hkv, k0, w.kb);
+            next_slot();
+          }
+        }
+        if (!ok) break;
+        // The two slots that O is staged in: they belong to the softmax warpgroups, which free them when the results have
+        // left.  (Their full barriers complete without a copy, so that every use of a slot is a phase of both barriers.)
+        for (int t = 0; ok && t < 2; ++t) {
+          ok = mbar_wait_warp(&kv_empty[slot], phase ^ 1u, abort_flag, st, SITE_F_PROD, budget);
+          if (!ok) break;
+          if (on) {
+            mbar_arrive(&kv_full[slot]);
+            mbar_arrive(&o_slot[slot]);
+          }
+          next_slot();
+        }
+        if (!ok) break;
+      }
+      loaded = false;
+      // a work item of the grid that has not started, if there is one
+      mbar_expect_tx_if(on, answer_full, 16);
+      work_request_if(on, answer, answer_full);
+      ok = mbar_wait_warp(answer_full, requests & 1u, abort_flag, st, SITE_F_ITEM, budget);
+      if (!ok) break;
+      ++requests;
+      const int cta = work_answer(answer);
+      fence_proxy_async_smem();                 // the next answer is written after this one is read
+      __syncwarp();
+      if (cta >= 0) w = fwd_item<SPARSE>(args, cta);
+      else w.state = -1;
     }
   } else if (warp == 1) {
     // ------------------------------ MMA issuer ------------------------------
-    if (nmax > 0) {
-      const uint32_t on = elect_one();            // the whole warp walks, one lane issues
-      constexpr uint32_t idesc_s = make_idesc_bf16(128, 128, false, false);
-      constexpr uint32_t idesc_o = make_idesc_bf16(128, D, false, true);
-      uint32_t slot = 0, phase = 0;
-      uint32_t pph = 0;                      // bit t: phase parity of p_full of tile t
-      bool ok = mbar_wait_warp(q_full, 0, abort_flag, st, SITE_F_MMA_Q, budget);
-      auto issue_s = [&](int t, uint32_t kslot) {
-        const uint32_t qa = smem_u32(smem + L::OFF_Q + t * L::QT);
-        const uint32_t ka = smem_u32(smem + L::OFF_KV + kslot * L::QT);
-#pragma unroll
-        for (int k = 0; k < D / 16; ++k) {
-          const uint64_t da = desc_kmajor(qa + (k / 4) * 16384, k % 4);
-          const uint64_t db = desc_kmajor(ka + (k / 4) * 16384, k % 4);
-          umma_bf16_if(on, tmem_s_of(t), da, db, idesc_s, k != 0 ? 1u : 0u);
-        }
-        umma_commit_if(on, &s_full[t]);
-      };
-      uint32_t kslot = 0;
-      if (ok) {
-        ok = mbar_wait_warp(&kv_full[slot], phase, abort_flag, st, SITE_F_MMA_KV, budget);
-        if (ok) {
-          tc_fence_after();
-          kslot = slot;
-          if (++slot == KV_SLOTS) { slot = 0; phase ^= 1u; }
-          for (int t = 0; t < 2; ++t)
-            if ((t == 0 ? n0 : n1) > 0 && (t == 0 ? s0 : s1) == 0) issue_s(t, kslot);
-          umma_commit_if(on, &kv_empty[kslot]);
-        }
+    const uint32_t on = elect_one();            // the whole warp walks, one lane issues
+    constexpr uint32_t idesc_s = make_idesc_bf16(128, 128, false, false);
+    constexpr uint32_t idesc_o = make_idesc_bf16(128, D, false, true);
+    uint32_t slot = 0, phase = 0, loads = 0;
+    uint32_t pph = 0;                      // bit t: phase parity of p_full of tile t
+    uint32_t oph = 0;                      // bit t: parity of the items of tile t
+    bool ok = true;
+    auto next_slot = [&]() {
+      if (++slot == KV_SLOTS) {
+        slot = 0;
+        phase ^= 1u;
       }
-      for (int i = 0; ok && i < nmax; ++i) {
-        if (!mbar_wait_warp(&kv_full[slot], phase, abort_flag, st, SITE_F_MMA_KV, budget)) break;
-        const uint32_t vslot = slot;
-        if (++slot == KV_SLOTS) { slot = 0; phase ^= 1u; }
-        const bool has_next = (i + 1 < nmax);
-        if (has_next) {
-          if (!mbar_wait_warp(&kv_full[slot], phase, abort_flag, st, SITE_F_MMA_KV, budget)) break;
-          kslot = slot;
-          if (++slot == KV_SLOTS) { slot = 0; phase ^= 1u; }
+    };
+    auto issue_s = [&](int t, uint32_t kslot) {
+      const uint32_t qa = smem_u32(smem + L::OFF_Q + t * L::QT);
+      const uint32_t ka = smem_u32(smem + L::OFF_KV + kslot * L::QT);
+#pragma unroll
+      for (int k = 0; k < D / 16; ++k) {
+        const uint64_t da = desc_kmajor(qa + (k / 4) * 16384, k % 4);
+        const uint64_t db = desc_kmajor(ka + (k / 4) * 16384, k % 4);
+        umma_bf16_if(on, tmem_s_of(t), da, db, idesc_s, k != 0 ? 1u : 0u);
+      }
+      umma_commit_if(on, &s_full[t]);
+    };
+    while (ok && take()) {
+      const int n0 = w.n[0], n1 = w.n[1], s0 = w.s[0], s1 = w.s[1];
+      const int nmax = max(n0, n1);
+      if (nmax > 0) {
+        ok = mbar_wait_warp(q_full, loads & 1u, abort_flag, st, SITE_F_MMA_Q, budget);
+        uint32_t kslot = 0;
+        if (ok) {
+          ok = mbar_wait_warp(&kv_full[slot], phase, abort_flag, st, SITE_F_MMA_KV, budget);
+          if (ok) {
+            tc_fence_after();
+            kslot = slot;
+            next_slot();
+            for (int t = 0; t < 2; ++t)
+              if ((t == 0 ? n0 : n1) > 0 && (t == 0 ? s0 : s1) == 0) issue_s(t, kslot);
+            umma_commit_if(on, &kv_empty[kslot]);
+            if (nmax == 1) umma_commit_if(on, q_empty);      // the Q tiles may be replaced
+          }
         }
-        tc_fence_after();
-        const uint32_t va = smem_u32(smem + L::OFF_KV + vslot * L::QT);
+        for (int i = 0; ok && i < nmax; ++i) {
+          if (!mbar_wait_warp(&kv_full[slot], phase, abort_flag, st, SITE_F_MMA_KV, budget)) break;
+          const uint32_t vslot = slot;
+          next_slot();
+          const bool has_next = (i + 1 < nmax);
+          if (has_next) {
+            if (!mbar_wait_warp(&kv_full[slot], phase, abort_flag, st, SITE_F_MMA_KV, budget)) break;
+            kslot = slot;
+            next_slot();
+          }
+          tc_fence_after();
+          const uint32_t va = smem_u32(smem + L::OFF_KV + vslot * L::QT);
 #pragma unroll
-        for (int t = 0; t < 2; ++t) {
-          if (i >= (t == 0 ? n0 : n1)) continue;
-          if (i >= (t == 0 ? s0 : s1)) {
-            // P is read from TMEM (bf16 pairs in the first 64 columns of the tile's score region): it
-            // never crosses shared memory, whose bandwidth the operand fetches of the MMAs saturate.
-            // It comes in two halves, so that the first products overlap the second half's exponentials.
-#pragma unroll
-            for (int half = 0; half < 2; ++half) {
-              if (!mbar_wait_warp(&p_full[2 * t + half], (pph >> t) & 1u, abort_flag, st, SITE_F_MMA_P, budget)) {
+          for (int t = 0; t < 2; ++t) {
+            if (i >= (t == 0 ? n0 : n1)) continue;
+            if (i >= (t == 0 ? s0 : s1)) {
+              // the results of the item before have been read
+              if (i == (t == 0 ? s0 : s1) &&
+                  !mbar_wait_warp(&o_empty[t], ((oph >> t) & 1u) ^ 1u, abort_flag, st, SITE_F_MMA_P, budget)) {
                 ok = false;
                 break;
               }
-              tc_fence_after();
+              // P is read from TMEM (bf16 pairs in the first 64 columns of the tile's score region): it
+              // never crosses shared memory, whose bandwidth the operand fetches of the MMAs saturate.
+              // It comes in two halves, so that the first products overlap the second half's exponentials.
 #pragma unroll
-              for (int k = half * 4; k < half * 4 + 4; ++k) {
-                const uint64_t db = desc_mnmajor(va, k, 16384);
-                umma_bf16_ts_if(on, tmem_o_of(t), tmem_s_of(t) + k * 8, db, idesc_o,
-                                (i > (t == 0 ? s0 : s1) || k != 0) ? 1u : 0u);
+              for (int half = 0; half < 2; ++half) {
+                if (!mbar_wait_warp(&p_full[2 * t + half], (pph >> t) & 1u, abort_flag, st, SITE_F_MMA_P, budget)) {
+                  ok = false;
+                  break;
+                }
+                tc_fence_after();
+#pragma unroll
+                for (int k = half * 4; k < half * 4 + 4; ++k) {
+                  const uint64_t db = desc_mnmajor(va, k, 16384);
+                  umma_bf16_ts_if(on, tmem_o_of(t), tmem_s_of(t) + k * 8, db, idesc_o,
+                                  (i > (t == 0 ? s0 : s1) || k != 0) ? 1u : 0u);
+                }
               }
+              if (!ok) break;
+              pph ^= 1u << t;
+              umma_commit_if(on, &pv_done[t]);
             }
-            if (!ok) break;
-            pph ^= 1u << t;
-            umma_commit_if(on, &pv_done[t]);
+            if (i + 1 < (t == 0 ? n0 : n1) && i + 1 >= (t == 0 ? s0 : s1)) issue_s(t, kslot);
           }
-          if (i + 1 < (t == 0 ? n0 : n1) && i + 1 >= (t == 0 ? s0 : s1)) issue_s(t, kslot);
+          if (!ok) break;
+          umma_commit_if(on, &kv_empty[vslot]);
+          if (has_next) umma_commit_if(on, &kv_empty[kslot]);
+          if (i + 2 == nmax) umma_commit_if(on, q_empty);
         }
         if (!ok) break;
-        umma_commit_if(on, &kv_empty[vslot]);
-        if (has_next) umma_commit_if(on, &kv_empty[kslot]);
+        oph ^= (n0 > 0 ? 1u : 0u) | (n1 > 0 ? 2u : 0u);
+        ++loads;
       }
+      next_slot();              // the slots that O is staged in
+      next_slot();
     }
   }
   } else {
@@ -330,186 +472,208 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constant
     const int t = (warp - 4) >> 2;
     const int quad = warp & 3;
     const int r = quad * 32 + lane;
-    const int n_mine = t == 0 ? n0 : n1;
-    const int s_mine = t == 0 ? s0 : s1;
     const uint32_t lane_off = static_cast<uint32_t>(quad * 32) << 16;
-    uint8_t* obuf = smem + L::OFF_Q + t * L::QT;       // staging of O: the Q tile is dead after the last S MMA
-    bool ok = true;
-    float m_ref = -INFINITY, l_sum = 0.f;
-    const int qi_local = q0 + t * 128 + r;             // row of Q / O / LSE held by this rank
-    const int qi = args.q_off + qi_local;              // its position in the whole sequence
-    int my_seg = 0, my_lim = qi, my_start = 0, my_first = 0;
-    if (tile_valid[t] && grouped) {
-      // a real gathered row sees every key of the block; a padding row sees none
-      my_seg = (t * 128 + r < gd.w) ? 1 : 0;
-      my_first = -(1 << 30);
-      my_lim = 1 << 30;
-    } else if (tile_valid[t]) {
-      my_seg = args.seg[b * args.S + qi];
-      my_first = args.row_start[b * args.S + qi];
-      if (args.lim != nullptr) my_lim = args.lim[b * args.S + qi];
-      if (sparse) my_start = args.sp.doc_start[b * args.S + qi];
-    }
-    uint32_t sph = 0;
     const uint64_t scale2 = pack_f32x2(args.scale_log2, args.scale_log2);
-    for (int i = s_mine; i < n_mine; ++i) {
-      const int k0 = kv_pos(i);
-      // ---- visible columns of this row inside the key tile: the keys of a row's run are
-      // contiguous, so they form one interval [c_lo, c_hi] (tile-relative, may lie outside) ----
-      const int c_lo = my_first - k0;
-      const int c_hi = my_lim - k0;
-      bool none = (my_seg == 0) || (c_hi < 0) || (c_lo > 127);
-      int bound = 0x7fffffff;     // keys below it need v0, keys from it on need v1
-      bool v0 = true, v1 = true;
-      if (sparse && !none) {
-        const SparseRow sr = sparse_row(args.sp, b, h, args.Hq, args.S, qi, my_start, k0, 128);
-        bound = sr.bound; v0 = sr.v0; v1 = sr.v1;
-        none = !v0 && !v1;
+    uint32_t sph = 0, pv = 0;              // parity of the scores, products so far
+    uint32_t slot = 0;                     // KV ring
+    uint32_t left = 0;                     // bit s: parity of the times that slot s was left to a tile
+    while (take()) {
+      const int n_mine = t == 0 ? w.n[0] : w.n[1];
+      const int s_mine = t == 0 ? w.s[0] : w.s[1];
+      const bool tile_valid = (w.valid >> t) & 1;
+      bool ok = true;
+      float m_ref = -INFINITY, l_sum = 0.f;
+      const int qi_local = w.q0 + t * 128 + r;             // row of Q / O / LSE held by this rank
+      const int qi = args.q_off + qi_local;              // its position in the whole sequence
+      int my_seg = 0, my_lim = qi, my_start = 0, my_first = 0;
+      if (tile_valid && grouped) {
+        // a real gathered row sees every key of the block; a padding row sees none
+        my_seg = (t * 128 + r < w.real) ? 1 : 0;
+        my_first = -(1 << 30);
+        my_lim = 1 << 30;
+      } else if (tile_valid) {
+        my_seg = args.seg[w.b * args.S + qi];
+        my_first = args.row_start[w.b * args.S + qi];
+        if (args.lim != nullptr) my_lim = args.lim[w.b * args.S + qi];
+        if (sparse) my_start = args.sp.doc_start[w.b * args.S + qi];
       }
-      const bool all = !none && (c_lo <= 0) && (c_hi >= 127) && v0 && v1;
-      if (!mbar_wait(&s_full[t], sph, abort_flag, st, SITE_F_SM_S, budget)) {
-        ok = false;
-        break;
-      }
-      sph ^= 1u;
-      tc_fence_after();
-      // ---- the whole score row in registers: one TMEM round trip ----
-      uint32_t sc[128];
-      tmem_ld32x4(tmem_s_of(t) + lane_off, sc);
-      tmem_ld_wait();
-      if (!all) {
+      for (int i = s_mine; i < n_mine; ++i) {
+        const int k0 = fwd_key<SPARSE>(args, w, i);
+        // ---- visible columns of this row inside the key tile: the keys of a row's run are
+        // contiguous, so they form one interval [c_lo, c_hi] (tile-relative, may lie outside) ----
+        const int c_lo = my_first - k0;
+        const int c_hi = my_lim - k0;
+        bool none = (my_seg == 0) || (c_hi < 0) || (c_lo > 127);
+        int bound = 0x7fffffff;     // keys below it need v0, keys from it on need v1
+        bool v0 = true, v1 = true;
+        if (sparse && !none) {
+          const SparseRow sr = sparse_row(args.sp, w.b, w.h, args.Hq, args.S, qi, my_start, k0, 128);
+          bound = sr.bound; v0 = sr.v0; v1 = sr.v1;
+          none = !v0 && !v1;
+        }
+        const bool all = !none && (c_lo <= 0) && (c_hi >= 127) && v0 && v1;
+        if (!mbar_wait(&s_full[t], sph, abort_flag, st, SITE_F_SM_S, budget)) {
+          ok = false;
+          break;
+        }
+        sph ^= 1u;
+        tc_fence_after();
+        // ---- the whole score row in registers: one TMEM round trip ----
+        uint32_t sc[128];
+        tmem_ld32x4(tmem_s_of(t) + lane_off, sc);
+        tmem_ld_wait();
+        if (!all) {
+#pragma unroll
+          for (int c = 0; c < 4; ++c) {
+            unsigned vis = none ? 0u : (bits_from(c_lo - 32 * c) & bits_upto(c_hi - 32 * c));
+            if (sparse) {
+              const unsigned above = bits_from(bound - k0 - 32 * c);      // keys >= bound
+              vis &= (v0 ? ~above : 0u) | (v1 ? above : 0u);
+            }
+            if (vis != 0xffffffffu) {
+#pragma unroll
+              for (int e = 0; e < 32; ++e)
+                if (!((vis >> e) & 1u)) sc[c * 32 + e] = 0xff800000u;     // -inf
+            }
+          }
+        }
+        // ---- row maximum of the raw scores (the scale is positive), four independent chains ----
+        float mq[4];
 #pragma unroll
         for (int c = 0; c < 4; ++c) {
-          unsigned vis = none ? 0u : (bits_from(c_lo - 32 * c) & bits_upto(c_hi - 32 * c));
-          if (sparse) {
-            const unsigned above = bits_from(bound - k0 - 32 * c);      // keys >= bound
-            vis &= (v0 ? ~above : 0u) | (v1 ? above : 0u);
-          }
-          if (vis != 0xffffffffu) {
+          mq[c] = __uint_as_float(sc[c * 32]);
 #pragma unroll
-            for (int e = 0; e < 32; ++e)
-              if (!((vis >> e) & 1u)) sc[c * 32 + e] = 0xff800000u;     // -inf
-          }
+          for (int e = 1; e < 31; e += 2)
+            mq[c] = fmax3(mq[c], __uint_as_float(sc[c * 32 + e]), __uint_as_float(sc[c * 32 + e + 1]));
+          mq[c] = fmaxf(mq[c], __uint_as_float(sc[c * 32 + 31]));
         }
-      }
-      // ---- row maximum of the raw scores (the scale is positive), four independent chains ----
-      float mq[4];
-#pragma unroll
-      for (int c = 0; c < 4; ++c) {
-        mq[c] = __uint_as_float(sc[c * 32]);
-#pragma unroll
-        for (int e = 1; e < 31; e += 2)
-          mq[c] = fmax3(mq[c], __uint_as_float(sc[c * 32 + e]), __uint_as_float(sc[c * 32 + e + 1]));
-        mq[c] = fmaxf(mq[c], __uint_as_float(sc[c * 32 + 31]));
-      }
-      const float mx = fmaxf(fmaxf(mq[0], mq[1]), fmaxf(mq[2], mq[3])) * args.scale_log2;
-      // ---- lazy running maximum ----
-      const bool need = (mx > m_ref + 8.f) || (m_ref == -INFINITY && mx > -INFINITY);
-      float alpha = 1.f;
-      if (need) {
-        alpha = (m_ref == -INFINITY) ? 0.f : fast_exp2(m_ref - mx);
-        m_ref = mx;
-        l_sum *= alpha;
-      }
-      // PV(i-1) was issued before S(i) and the tensor core completes MMAs in issue order, so the
-      // scores of this tile being ready means O holds every earlier tile: no separate wait.
-      if (i > s_mine && __any_sync(0xffffffffu, need)) {
+        const float mx = fmaxf(fmaxf(mq[0], mq[1]), fmaxf(mq[2], mq[3])) * args.scale_log2;
+        // ---- lazy running maximum ----
+        const bool need = (mx > m_ref + 8.f) || (m_ref == -INFINITY && mx > -INFINITY);
+        float alpha = 1.f;
+        if (need) {
+          alpha = (m_ref == -INFINITY) ? 0.f : fast_exp2(m_ref - mx);
+          m_ref = mx;
+          l_sum *= alpha;
+        }
+        // PV(i-1) was issued before S(i) and the tensor core completes MMAs in issue order, so the
+        // scores of this tile being ready means O holds every earlier tile: no separate wait.
+        if (i > s_mine && __any_sync(0xffffffffu, need)) {
 #pragma unroll 1
-        for (int c = 0; c < D / 8; ++c) {      // narrow chunks: the score row stays in registers
-          uint32_t rr[8];
-          tmem_ld8(tmem_o_of(t) + lane_off + c * 8, rr);
-          tmem_ld_wait();
+          for (int c = 0; c < D / 8; ++c) {      // narrow chunks: the score row stays in registers
+            uint32_t rr[8];
+            tmem_ld8(tmem_o_of(t) + lane_off + c * 8, rr);
+            tmem_ld_wait();
 #pragma unroll
-          for (int e = 0; e < 8; ++e) rr[e] = __float_as_uint(__uint_as_float(rr[e]) * alpha);
-          tmem_st8(tmem_o_of(t) + lane_off + c * 8, rr);
-        }
-        tmem_st_wait();
-      }
-      // ---- P = exp2(s * scale - m): packed fma / add on pairs; P goes back into TMEM as bf16 pairs
-      // over the first 64 columns of the score row this thread already holds in registers ----
-      const float m_use = (m_ref == -INFINITY) ? 0.f : m_ref;
-      const uint64_t neg_m2 = pack_f32x2(-m_use, -m_use);
-      uint64_t rs2 = pack_f32x2(0.f, 0.f);
-      // FAST: the whole row is visible and has a maximum, so every fourth pair of exponentials can go to the
-      // FMA pipe (poly_exp2_x2 never returns zero; masked scores need one)
-      auto exponentials = [&](auto fast_tag) {
-        constexpr bool FAST = decltype(fast_tag)::value;
-#pragma unroll
-        for (int qt = 0; qt < 8; ++qt) {           // 16 scores -> 8 packed columns per store
-          uint32_t pw[8];
-#pragma unroll
-          for (int jj = 0; jj < 8; ++jj) {
-            const int e = qt * 16 + jj * 2;
-            const uint64_t x2 = fma_f32x2(pack_f32x2(__uint_as_float(sc[e]), __uint_as_float(sc[e + 1])), scale2, neg_m2);
-            float pa, pb;
-            if (FAST && jj % POLY_PERIOD == POLY_PERIOD - 1) {
-              poly_exp2_x2(x2, pa, pb);
-            } else {
-              float xa, xb;
-              unpack_f32x2(x2, xa, xb);
-              pa = fast_exp2(xa);
-              pb = fast_exp2(xb);
-            }
-            rs2 = add_f32x2(rs2, pack_f32x2(pa, pb));
-            pw[jj] = pack_bf16(pa, pb);
+            for (int e = 0; e < 8; ++e) rr[e] = __float_as_uint(__uint_as_float(rr[e]) * alpha);
+            tmem_st8(tmem_o_of(t) + lane_off + c * 8, rr);
           }
-          tmem_st8(tmem_s_of(t) + lane_off + qt * 8, pw);
-          if (qt == 7 || (qt == 3 && HALVED)) {
-            tmem_st_wait();
-            tc_fence_before();
-            __syncwarp();
-            if (lane == 0) {
-              if (!HALVED) mbar_arrive(&p_full[2 * t]);
-              mbar_arrive(&p_full[2 * t + qt / 4]);
+          tmem_st_wait();
+        }
+        // ---- P = exp2(s * scale - m): packed fma / add on pairs; P goes back into TMEM as bf16 pairs
+        // over the first 64 columns of the score row this thread already holds in registers ----
+        const float m_use = (m_ref == -INFINITY) ? 0.f : m_ref;
+        const uint64_t neg_m2 = pack_f32x2(-m_use, -m_use);
+        uint64_t rs2 = pack_f32x2(0.f, 0.f);
+        // FAST: the whole row is visible and has a maximum, so every fourth pair of exponentials can go to the
+        // FMA pipe (poly_exp2_x2 never returns zero; masked scores need one)
+        auto exponentials = [&](auto fast_tag) {
+          constexpr bool FAST = decltype(fast_tag)::value;
+#pragma unroll
+          for (int qt = 0; qt < 8; ++qt) {           // 16 scores -> 8 packed columns per store
+            uint32_t pw[8];
+#pragma unroll
+            for (int jj = 0; jj < 8; ++jj) {
+              const int e = qt * 16 + jj * 2;
+              const uint64_t x2 = fma_f32x2(pack_f32x2(__uint_as_float(sc[e]), __uint_as_float(sc[e + 1])), scale2, neg_m2);
+              float pa, pb;
+              if (FAST && jj % POLY_PERIOD == POLY_PERIOD - 1) {
+                poly_exp2_x2(x2, pa, pb);
+              } else {
+                float xa, xb;
+                unpack_f32x2(x2, xa, xb);
+                pa = fast_exp2(xa);
+                pb = fast_exp2(xb);
+              }
+              rs2 = add_f32x2(rs2, pack_f32x2(pa, pb));
+              pw[jj] = pack_bf16(pa, pb);
+            }
+            tmem_st8(tmem_s_of(t) + lane_off + qt * 8, pw);
+            if (qt == 7 || (qt == 3 && HALVED)) {
+              tmem_st_wait();
+              tc_fence_before();
+              __syncwarp();
+              if (lane == 0) {
+                if (!HALVED) mbar_arrive(&p_full[2 * t]);
+                mbar_arrive(&p_full[2 * t + qt / 4]);
+              }
             }
           }
-        }
-      };
-      if (!SPARSE && __all_sync(0xffffffffu, all && m_ref > -INFINITY)) exponentials(std::true_type{});
-      else exponentials(std::false_type{});
-      float rs_a, rs_b;
-      unpack_f32x2(rs2, rs_a, rs_b);
-      l_sum += rs_a + rs_b;
-    }
-    // ---- finalize ----
-    if (ok && n_mine > 0) {
-      ok = mbar_wait(&pv_done[t], static_cast<uint32_t>(n_mine - s_mine - 1) & 1u, abort_flag, st, SITE_F_SM_PV, budget);
-      tc_fence_after();
-    }
-    const bool any_bad = named_bar_or(2 + t, 128, !ok);
-    if (!any_bad && tile_valid[t]) {
-      const float inv = (l_sum > 0.f) ? 1.f / l_sum : 0.f;
-#pragma unroll 1
-      for (int c = 0; c < D / 32; ++c) {
-        uint32_t rr[32];
-        if (n_mine > 0) {
-          tmem_ld32(tmem_o_of(t) + lane_off + c * 32, rr);
-          tmem_ld_wait();
-        } else {
-#pragma unroll
-          for (int e = 0; e < 32; ++e) rr[e] = 0u;
-        }
-#pragma unroll
-        for (int jj = 0; jj < 4; ++jj) {
-          uint4 v;
-          v.x = pack_bf16(__uint_as_float(rr[jj * 8 + 0]) * inv, __uint_as_float(rr[jj * 8 + 1]) * inv);
-          v.y = pack_bf16(__uint_as_float(rr[jj * 8 + 2]) * inv, __uint_as_float(rr[jj * 8 + 3]) * inv);
-          v.z = pack_bf16(__uint_as_float(rr[jj * 8 + 4]) * inv, __uint_as_float(rr[jj * 8 + 5]) * inv);
-          v.w = pack_bf16(__uint_as_float(rr[jj * 8 + 6]) * inv, __uint_as_float(rr[jj * 8 + 7]) * inv);
-          *reinterpret_cast<uint4*>(obuf + (c / 2) * 16384 + sw128_offset(r, (c % 2) * 4 + jj)) = v;
-        }
+        };
+        if (!SPARSE && __all_sync(0xffffffffu, all && m_ref > -INFINITY)) exponentials(std::true_type{});
+        else exponentials(std::false_type{});
+        float rs_a, rs_b;
+        unpack_f32x2(rs2, rs_a, rs_b);
+        l_sum += rs_a + rs_b;
       }
-      fence_proxy_async_smem();
-      named_bar_sync(4 + t, 128);
+      // ---- finalize ----
+      if (ok && n_mine > 0) {
+        pv += static_cast<uint32_t>(n_mine - s_mine);
+        ok = mbar_wait(&pv_done[t], (pv - 1u) & 1u, abort_flag, st, SITE_F_SM_PV, budget);
+        tc_fence_after();
+      }
+      // tile t stages in the t-th of the slots that the producer leaves to O
+      // (all that it left to earlier items it did before it handed over this one, so no phase is mistaken for another)
+      const uint32_t first = (slot + static_cast<uint32_t>(2 * max(w.n[0], w.n[1]))) % KV_SLOTS;
+      const uint32_t second = first + 1 < KV_SLOTS ? first + 1 : 0;
+      slot = t == 0 ? first : second;
+      ok = ok && mbar_wait(&o_slot[slot], (left >> slot) & 1u, abort_flag, st, SITE_F_SM_PV, budget);
+      left ^= (1u << first) | (1u << second);
+      uint8_t* obuf = smem + L::OFF_KV + slot * L::QT;
+      const bool any_bad = named_bar_or(2 + t, 128, !ok);
+      if (any_bad) break;
+      if (tile_valid) {
+        const float inv = (l_sum > 0.f) ? 1.f / l_sum : 0.f;
+#pragma unroll 1
+        for (int c = 0; c < D / 32; ++c) {
+          uint32_t rr[32];
+          if (n_mine > 0) {
+            tmem_ld32(tmem_o_of(t) + lane_off + c * 32, rr);
+            tmem_ld_wait();
+          } else {
+#pragma unroll
+            for (int e = 0; e < 32; ++e) rr[e] = 0u;
+          }
+#pragma unroll
+          for (int jj = 0; jj < 4; ++jj) {
+            uint4 v;
+            v.x = pack_bf16(__uint_as_float(rr[jj * 8 + 0]) * inv, __uint_as_float(rr[jj * 8 + 1]) * inv);
+            v.y = pack_bf16(__uint_as_float(rr[jj * 8 + 2]) * inv, __uint_as_float(rr[jj * 8 + 3]) * inv);
+            v.z = pack_bf16(__uint_as_float(rr[jj * 8 + 4]) * inv, __uint_as_float(rr[jj * 8 + 5]) * inv);
+            v.w = pack_bf16(__uint_as_float(rr[jj * 8 + 6]) * inv, __uint_as_float(rr[jj * 8 + 7]) * inv);
+            *reinterpret_cast<uint4*>(obuf + (c / 2) * 16384 + sw128_offset(r, (c % 2) * 4 + jj)) = v;
+          }
+        }
+        tc_fence_before();
+        fence_proxy_async_smem();
+        named_bar_sync(4 + t, 128);
+        if (r == 0) {
+#pragma unroll
+          for (int hf = 0; hf < HALVES; ++hf) tma_store_4d(&map_o, obuf + hf * 16384, hf * 64, w.h, w.q0 + t * 128, w.b);
+          tma_commit_group();
+        }
+        const float lse = (l_sum > 0.f) ? (m_ref + log2f(l_sum)) * 0.6931471805599453f : 0.f;
+        args.lse[(static_cast<size_t>(w.b) * args.Hq + w.h) * args.Sq + qi_local] = lse;
+      }
+      __syncwarp();
+      if (n_mine > 0 && lane == 0) mbar_arrive(&o_empty[t]);      // the next item may write its results
       if (r == 0) {
-#pragma unroll
-        for (int hf = 0; hf < HALVES; ++hf) tma_store_4d(&map_o, obuf + hf * 16384, hf * 64, h, q0 + t * 128, b);
-        tma_commit_group();
-        tma_wait_group<0>();
+        tma_wait_group_read<0>();
+        mbar_arrive(&kv_empty[slot]);
       }
-      const float lse = (l_sum > 0.f) ? (m_ref + log2f(l_sum)) * 0.6931471805599453f : 0.f;
-      args.lse[(static_cast<size_t>(b) * args.Hq + h) * args.Sq + qi_local] = lse;
+      slot = second + 1;
     }
+    tma_wait_group<0>();
   }
 
   tc_fence_before();

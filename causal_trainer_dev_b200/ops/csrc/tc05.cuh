@@ -240,6 +240,32 @@ __device__ __forceinline__ void tma_wait_group() {
 }
 
 // ---------------------------------------------------------------------------------------
+// Cluster launch control: a CTA takes over a work item (CTA) of its grid that has not started
+// ---------------------------------------------------------------------------------------
+// Asks for one; the 16-byte answer is credited to `bar`.  Not to be asked again after a refusal.
+__device__ __forceinline__ void work_request_if(uint32_t on, uint32_t answer, uint64_t* bar) {
+  asm volatile(
+      "{\n\t.reg .pred q;\n\tsetp.ne.b32 q, %2, 0;\n\t"
+      "@q clusterlaunchcontrol.try_cancel.async.shared::cta.mbarrier::complete_tx::bytes.b128 [%0], [%1];\n\t}" ::"r"(answer),
+      "r"(smem_u32(bar)), "r"(on)
+      : "memory");
+}
+// blockIdx.x of the work item taken over, -1: there is none left.
+__device__ __forceinline__ int work_answer(uint32_t answer) {
+  int index;
+  asm volatile(
+      "{\n\t.reg .b128 r;\n\t.reg .pred p;\n\t"
+      "ld.shared.b128 r, [%1];\n\t"
+      "mov.s32 %0, -1;\n\t"
+      "clusterlaunchcontrol.query_cancel.is_canceled.pred.b128 p, r;\n\t"
+      "@p clusterlaunchcontrol.query_cancel.get_first_ctaid::x.b32.b128 %0, r;\n\t}"
+      : "=r"(index)
+      : "r"(answer)
+      : "memory");
+  return index;
+}
+
+// ---------------------------------------------------------------------------------------
 // TMEM allocation (one warp, all lanes)
 // ---------------------------------------------------------------------------------------
 __device__ __forceinline__ void tmem_alloc(uint32_t* smem_result, uint32_t ncols) {

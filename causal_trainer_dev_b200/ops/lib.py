@@ -113,6 +113,7 @@ _SITES = {
     0x0205: "attention forward softmax: scores never completed",
     0x0206: "attention forward softmax: P V never completed",
     0x0207: "attention forward producer: gathered K/V flag never published",
+    0x0208: "attention forward: work item never handed over",
     0x0301: "attention backward producer: streamed stage never freed",
     0x0302: "attention backward mma: resident tiles never arrived",
     0x0303: "attention backward mma: streamed block never arrived",
@@ -120,6 +121,7 @@ _SITES = {
     0x0305: "attention backward compute: S / dP never completed",
     0x0307: "attention backward compute: accumulators never completed",
     0x0308: "attention backward: shared memory base not 1024-byte aligned (nothing written)",
+    0x0309: "attention backward: work item never handed over",
     0x0401: "fsdp reduce-scatter: a peer's gradients never arrived",
     0x0402: "fsdp: flags never published",
     0x0501: "tensor-parallel all-gather: a peer's rows never became ready",
