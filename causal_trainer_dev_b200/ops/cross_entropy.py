@@ -87,14 +87,15 @@ def cut_ce_forward(hidden, head, targets, weights, grad_scale: float | torch.Ten
     tgt = targets.to(torch.int32).contiguous()
     w = weights.to(torch.float32).contiguous()
     L = _lib.lib()
-    from .gemm import _FLAG_SOURCES, _flag_args, _rotations, flag_source_of
+    from .gemm import _FLAG_SOURCES, _flag_args, _rotations, flag_source_of, in_gathered_buffer
 
     hit = flag_source_of(head) if _FLAG_SOURCES else None
     hit_a = flag_source_of(hidden) if _FLAG_SOURCES else None
     _, m_rotate = _rotations(None, hit_a, hidden, head, False, False, rows, vocab)
     code = L.ctb_ce_stats(_lib.ptr(hidden), _lib.ptr(head), rows, vocab, d, ctypes.c_long(hidden.stride(0)),
                           ctypes.c_long(head.stride(0)), _lib.ptr(tgt), _lib.ptr(pmax), _lib.ptr(psum),
-                          _lib.ptr(tlogit), *_flag_args(hit), *_flag_args(hit_a), m_rotate, _lib.stream_ptr())
+                          _lib.ptr(tlogit), *_flag_args(hit), *_flag_args(hit_a), m_rotate,
+                          int(in_gathered_buffer(hidden, head)), _lib.stream_ptr())
     _lib.check(code, "ctb_ce_stats")
     if exchange is not None:
         nll, wsum, lse, coef = exchange.ce_exchange(pmax, psum, slabs, tlogit, w, grad_scale)
@@ -137,6 +138,9 @@ def cut_ce_backward(hidden, head, targets, lse, coef, *, chunk_rows: int = 4096,
         chunk_rows = max(128, chunk_rows // 128 * 128)
     slab = torch.empty((chunk_rows, vocab), dtype=torch.bfloat16, device=dev)
     L = _lib.lib()
+    from .gemm import in_gathered_buffer
+
+    gathered = int(in_gathered_buffer(hidden, head))
     first = True
     for start in range(0, rows, chunk_rows):
         n = min(chunk_rows, rows - start)
@@ -145,7 +149,7 @@ def cut_ce_backward(hidden, head, targets, lse, coef, *, chunk_rows: int = 4096,
         code = L.ctb_ce_dlogits(_lib.ptr(h), _lib.ptr(head), _lib.ptr(g), n, vocab, d, ctypes.c_long(h.stride(0)),
                                 ctypes.c_long(head.stride(0)), ctypes.c_long(g.stride(0)),
                                 _lib.ptr(tgt[start:start + n]), _lib.ptr(lse[start:start + n]),
-                                _lib.ptr(coef[start:start + n]), _lib.stream_ptr())
+                                _lib.ptr(coef[start:start + n]), gathered, _lib.stream_ptr())
         _lib.check(code, "ctb_ce_dlogits")
         if push is None:
             gemm(g, head, b_mn=True, out=dhidden[start:start + n])              # dH = G @ W

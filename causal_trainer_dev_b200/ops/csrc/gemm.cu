@@ -23,7 +23,7 @@
 // Counterpart in the reference: XLA dot_general behind `linear`
 // (src/causal_trainer/modeling/architecture.py:186-202) and the Pallas cut-CE kernels
 // (src/causal_trainer/kernels/cut_cross_entropy.py:85-156, 225-278).
-#include "gemm.h"
+#include "gemm_epilogue.cuh"
 
 #include <algorithm>
 #include <cstdlib>
@@ -35,11 +35,8 @@
 namespace ctb {
 namespace gemm {
 
-constexpr int BM = 128;            // rows of one UMMA accumulator (one TMEM slot)
-constexpr int BN = 256;
 constexpr int BK = 64;
 constexpr int B_STAGE = BN * BK * 2;   // 32 KiB
-constexpr int EPI_BUF = 128 * 128;     // 128 rows x 128 B
 constexpr int TQ = 4;                  // depth of the tile-index queue
 
 // Cycles producer warps spent waiting for chunk flags of gathered operands, summed over CTAs
@@ -140,24 +137,6 @@ __device__ __forceinline__ TileCoord tile_coord(int tile, int num_m, int num_n, 
   c.m0 = m * Cfg<TM>::BMT;
   c.n0 = n * BN;
   return c;
-}
-
-// Copies a staged 128 x 128 B block (128-byte swizzle) to `out` (row stride `ld` elements) with
-// 16-byte stores: thread -> (row etid/8 + 16*i, 16-byte column etid%8), so a warp writes four
-// full 128 B rows per step.  Kept out of line so its address arithmetic does not raise the
-// register count of the whole kernel.
-__device__ __noinline__ void push_block(const uint8_t* buf, __nv_bfloat16* out, long ld, int etid, int rows_left,
-                                        int cols_left) {
-  const int j = etid & 7;
-  if (j * 8 >= cols_left) return;
-  out += static_cast<long>(etid >> 3) * ld + j * 8;
-#pragma unroll 4
-  for (int i = 0; i < 8; ++i) {
-    const int r = (etid >> 3) + i * 16;
-    if (r < rows_left)
-      *reinterpret_cast<uint4*>(out + static_cast<long>(i) * 16 * ld) =
-          *reinterpret_cast<const uint4*>(buf + sw128_offset(r, j));
-  }
 }
 
 template <int TM, bool A_MN, bool B_MN, int EPI>
@@ -462,7 +441,7 @@ gemm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ C
     const uint32_t bar_stage = 1 + wg;       // named barriers of this warpgroup
     const uint32_t bar_vote = 3 + wg;
     uint32_t uses[2] = {0, 0};
-    uint32_t next_slot = 0, buf_idx = 0;
+    uint32_t next_slot = 0, staged = 0;
     uint8_t* epi = smem + C::OFF_EPI + wg * EPI_BUF;
     uint32_t tq = 0, tq_phase = 0;
     while (true) {
@@ -489,171 +468,12 @@ gemm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ C
       tc_fence_after();
       const uint32_t taddr = tmem_base + slot * BN + (static_cast<uint32_t>(q * 32) << 16);
       const int m_sub = tc.m0 + wg * BM;     // first row of this warpgroup's sub-tile
-      const int grow = m_sub + row;
-
-      if (EPI == EPI_CE_STATS) {
-        // Online softmax statistics of this 256-column slab for one row per thread.
-        const int target = (grow < args.M) ? args.ce_targets[grow] : -1;
-        float vmax = -INFINITY, vsum = 0.f, tlogit = 0.f;
-        bool has_target = false;
-#pragma unroll 1
-        for (int c = 0; c < BN / 32; ++c) {
-          const int col0 = tc.n0 + c * 32;
-          if (col0 >= args.N) break;
-          uint32_t r[32];
-          tmem_ld32(taddr + c * 32, r);
-          tmem_ld_wait();
-          float cmax = -INFINITY;
-#pragma unroll
-          for (int j = 0; j < 32; ++j) {
-            const float v = (col0 + j < args.N) ? __uint_as_float(r[j]) : -INFINITY;
-            r[j] = __float_as_uint(v);
-            cmax = fmaxf(cmax, v);
-            if (col0 + j == target) {
-              tlogit = v;
-              has_target = true;
-            }
-          }
-          const float nmax = fmaxf(vmax, cmax);
-          float s = 0.f;
-#pragma unroll
-          for (int j = 0; j < 32; ++j) s += __expf(__uint_as_float(r[j]) - nmax);
-          vsum = vsum * __expf(vmax - nmax) + s;
-          vmax = nmax;
-        }
-        if (grow < args.M) {
-          const int slab = tc.n0 / BN;
-          args.ce_max[static_cast<size_t>(slab) * args.M + grow] = vmax;
-          args.ce_sum[static_cast<size_t>(slab) * args.M + grow] = vsum;
-          if (has_target) args.ce_target_logit[grow] = tlogit;
-        }
-      } else if (args.out_f32) {
-#pragma unroll 1
-        for (int c = 0; c < BN / 32; ++c) {
-          const int col0 = tc.n0 + c * 32;
-          if (col0 >= args.N) break;
-          uint32_t r[32];
-          tmem_ld32(taddr + c * 32, r);
-          tmem_ld_wait();
-          uint8_t* buf = epi + (C::EPI_BUFS == 2 ? (buf_idx & 1u) * EPI_BUF : 0u);
-          if (etid == 0) tma_wait_group_read<C::EPI_BUFS - 1>();
-          named_bar_sync(bar_stage, 128);
-#pragma unroll
-          for (int j = 0; j < 8; ++j) {
-            float4 v;
-            v.x = __uint_as_float(r[4 * j + 0]) * args.alpha;
-            v.y = __uint_as_float(r[4 * j + 1]) * args.alpha;
-            v.z = __uint_as_float(r[4 * j + 2]) * args.alpha;
-            v.w = __uint_as_float(r[4 * j + 3]) * args.alpha;
-            *reinterpret_cast<float4*>(buf + sw128_offset(row, j)) = v;
-          }
-          fence_proxy_async_smem();
-          named_bar_sync(bar_stage, 128);
-          if (etid == 0 && m_sub < args.M) {
-            if (add_into_c) tma_reduce_add_2d(&map_c, buf, col0, m_sub);
-            else tma_store_2d(&map_c, buf, col0, m_sub);
-            tma_commit_group();
-          }
-          ++buf_idx;
-        }
-      } else {
-        float lse = 0.f, coef = 0.f;
-        int target = -1;
-        if (EPI == EPI_CE_DLOGITS && grow < args.M) {
-          lse = args.ce_lse[grow];
-          coef = args.ce_coef[grow];
-          target = args.ce_targets[grow];
-        }
-#pragma unroll 1
-        for (int c = 0; c < BN / 64; ++c) {
-          const int col0 = tc.n0 + c * 64;
-          if (col0 >= args.N) break;
-          uint8_t* buf = epi + (C::EPI_BUFS == 2 ? (buf_idx & 1u) * EPI_BUF : 0u);
-          // 64 output columns per staged block, converted 32 at a time to keep registers low
-#pragma unroll
-          for (int hh = 0; hh < 2; ++hh) {
-            uint32_t r[32];
-            tmem_ld32(taddr + c * 64 + hh * 32, r);
-            tmem_ld_wait();
-            const int cb = col0 + hh * 32;
-            if (EPI == EPI_CE_DLOGITS) {
-#pragma unroll
-              for (int j = 0; j < 32; ++j) {
-                float pv = __expf(__uint_as_float(r[j]) - lse);
-                if (cb + j == target) pv -= 1.f;
-                r[j] = __float_as_uint(pv * coef);
-              }
-            } else if (args.bias != nullptr) {
-#pragma unroll
-              for (int j = 0; j < 32; ++j) {
-                const float bv = (cb + j < args.N) ? __bfloat162float(args.bias[cb + j]) : 0.f;
-                r[j] = __float_as_uint(__uint_as_float(r[j]) + bv);
-              }
-            }
-            if (args.alpha != 1.f) {
-#pragma unroll
-              for (int j = 0; j < 32; ++j) r[j] = __float_as_uint(__uint_as_float(r[j]) * args.alpha);
-            }
-            if (hh == 0) {
-              // the staging block may still be read by the store that used it last
-              if (etid == 0) tma_wait_group_read<C::EPI_BUFS - 1>();
-              named_bar_sync(bar_stage, 128);
-            }
-#pragma unroll
-            for (int j = 0; j < 4; ++j) {
-              uint4 v;
-              v.x = pack_bf16(__uint_as_float(r[8 * j + 0]), __uint_as_float(r[8 * j + 1]));
-              v.y = pack_bf16(__uint_as_float(r[8 * j + 2]), __uint_as_float(r[8 * j + 3]));
-              v.z = pack_bf16(__uint_as_float(r[8 * j + 4]), __uint_as_float(r[8 * j + 5]));
-              v.w = pack_bf16(__uint_as_float(r[8 * j + 6]), __uint_as_float(r[8 * j + 7]));
-              *reinterpret_cast<uint4*>(buf + sw128_offset(row, hh * 4 + j)) = v;
-            }
-          }
-          if (EPI == EPI_PUSH) {
-            // reduce-scatter by push: 128 threads copy the staged 128 x 128 B block into the
-            // owner's receive buffer with 16-byte stores (peer memory: plain st.global only)
-            named_bar_sync(bar_stage, 128);
-            if (m_sub < args.M) {
-              const int grow0 = args.push.row_offset + m_sub;
-              const int dest = grow0 / args.push.rows_per_rank;
-              const long drow0 = static_cast<long>(args.push.src_rank) * args.push.rows_per_rank +
-                                 (grow0 - dest * args.push.rows_per_rank);
-              push_block(buf, args.push.dest[dest] + drow0 * args.push.ld + col0, args.push.ld, etid,
-                         args.M - m_sub, args.N - col0);
-            }
-            if (C::EPI_BUFS == 1) named_bar_sync(bar_stage, 128);   // one block: all copies out before it is refilled
-          } else {
-            fence_proxy_async_smem();
-            named_bar_sync(bar_stage, 128);
-            if (etid == 0 && m_sub < args.M) {
-              if (add_into_c) tma_reduce_add_2d(&map_c, buf, col0, m_sub);
-              else tma_store_2d(&map_c, buf, col0, m_sub);
-              tma_commit_group();
-            }
-          }
-          ++buf_idx;
-        }
-        if (EPI == EPI_PUSH && m_sub < args.M) {
-          // this 128-row piece is on its way: count it, and publish the flag with the last one
-          __threadfence_system();
-          named_bar_sync(bar_stage, 128);
-          if (etid == 0) {
-            const int dest = (args.push.row_offset + m_sub) / args.push.rows_per_rank;
-            const unsigned done = atomicAdd(args.push.counters + dest, 1u) + 1u;
-            if (done == static_cast<unsigned>(args.push.tiles_per_dest)) {
-              args.push.counters[dest] = 0u;
-              __threadfence_system();
-              asm volatile("st.release.sys.global.u32 [%0], %1;" ::"l"(args.push.flag[dest]), "r"(args.push.epoch)
-                           : "memory");
-            }
-          }
-        }
-      }
+      drain_slot<EPI, BN, C::EPI_BUFS>(args, &map_c, taddr, tc.n0, m_sub, row, etid, bar_stage, epi, staged, add_into_c);
       tc_fence_before();
       __syncwarp();
       if (lane == 0) mbar_arrive(&tempty[slot]);
     }
-    if (etid == 0) tma_wait_group<0>();
+    if (lane == 0) tma_wait_group<0>();
   }
 
   // ------------------------------ teardown ------------------------------
@@ -761,13 +581,23 @@ static bool gemm_splits(const GemmCall& c, int* width, int* slices) {
   return gemm_split_plan(c, width, slices);
 }
 
+// Whether it goes to the two-CTA kernel (gemm_pair.cu): under the same condition, unless the switch for that kernel is on,
+// which is asked first.
+static bool gemm_pairs(const GemmCall& c, PairPlan* plan) {
+  const bool other = gemm::forced_tile_mode() != 0 || gemm::dynamic_tiles_mode() || gemm::split_k_mode() != 0 ||
+                     (gemm::tail_split_mode() != 0 && c.out_f32);
+  if (other && !gemm_pair_forced()) return false;
+  return gemm_pair_plan(c, plan);
+}
+
 int run_gemm(const GemmCall& c) {
   using namespace gemm;
   if (c.M <= 0 || c.N <= 0 || c.K <= 0) return fail("gemm: M, N, K must be positive");
   if ((c.lda % 8) || (c.ldb % 8)) return fail("gemm: lda and ldb must be multiples of 8 elements (16 bytes)");
   const bool needs_c = (c.epi != EPI_CE_STATS) && !c.push.enabled;
   if (needs_c && (c.ldc % (c.out_f32 ? 4 : 8))) return fail("gemm: ldc must be a multiple of 16 bytes");
-  if (gemm_pair_eligible(c)) return launch_gemm_pair(c);       // two-CTA 256 x 256 tiles (gemm_pair.cu)
+  PairPlan pair;
+  if (gemm_pairs(c, &pair) && gemm_pair_workspace(c, pair) <= c.workspace_bytes) return launch_gemm_pair(c, pair);
   int split_width = 0, split_slices = 0;
   if (gemm_splits(c, &split_width, &split_slices)) return launch_gemm_split(c, split_width, split_slices);
   const CUtensorMap* ma = c.a_mn ? get_tensor_map_2d(c.A, Elt::BF16, c.M, c.K, c.lda, 64, 64, true)
@@ -778,8 +608,8 @@ int run_gemm(const GemmCall& c) {
   if (!mb) return 1;
   const CUtensorMap* mc = ma;  // placeholder when no C tensor is written
   if (needs_c) {
-    mc = c.out_f32 ? get_tensor_map_2d(c.C, Elt::F32, c.N, c.M, c.ldc, 32, 128, true)
-                   : get_tensor_map_2d(c.C, Elt::BF16, c.N, c.M, c.ldc, 64, 128, true);
+    mc = c.out_f32 ? get_tensor_map_2d(c.C, Elt::F32, c.N, c.M, c.ldc, 32, 32, true)
+                   : get_tensor_map_2d(c.C, Elt::BF16, c.N, c.M, c.ldc, 64, 32, true);
     if (!mc) return 1;
   }
   GemmArgs a{};
@@ -942,15 +772,25 @@ int run_gemm(const GemmCall& c) {
 }  // namespace ctb
 
 // C ABI ------------------------------------------------------------------------------------
-// C[M,N] = alpha * A*B^T (+ bias) ; see the layout table at the top of this file.
+// C[M,N] = alpha * A*B^T (+ bias) ; see the layout table at the top of this file.  `workspace` (16-byte aligned) may be null:
+// with fewer bytes than ctb_gemm_workspace says, the product takes a kernel that needs none.
 CTB_API int ctb_gemm(const void* A, const void* B, void* C, int M, int N, int K, long lda, long ldb, long ldc,
                      int a_mn, int b_mn, int out_f32, int accumulate, float alpha, const void* bias, int max_ctas,
-                     void* stream) {
+                     void* workspace, long workspace_bytes, void* stream) {
   ctb::GemmCall c{};
+  c.workspace = workspace; c.workspace_bytes = workspace_bytes;
   c.A = A; c.B = B; c.C = C; c.M = M; c.N = N; c.K = K; c.lda = lda; c.ldb = ldb; c.ldc = ldc;
   c.a_mn = a_mn; c.b_mn = b_mn; c.out_f32 = out_f32; c.accumulate = accumulate; c.alpha = alpha; c.bias = bias;
   c.epi = ctb::EPI_STORE; c.max_ctas = max_ctas; c.stream = stream;
   return ctb::run_gemm(c);
+}
+
+// Bytes of workspace that the product's best kernel wants (16-byte aligned operands, no CTA limit, no gathered operand).
+CTB_API long ctb_gemm_workspace(int M, int N, int K, int a_mn, int out_f32, int accumulate) {
+  ctb::GemmCall c{};
+  c.M = M; c.N = N; c.K = K; c.a_mn = a_mn; c.out_f32 = out_f32; c.accumulate = accumulate; c.epi = ctb::EPI_STORE;
+  ctb::PairPlan plan;
+  return ctb::gemm_pairs(c, &plan) ? ctb::gemm_pair_workspace(c, plan) : 0;
 }
 
 // Same GEMM family whose B operand lives in a buffer that another kernel (the all-gather
@@ -996,12 +836,14 @@ CTB_API int ctb_gemm_push(const void* A, const void* B, int M, int N, int K, lon
 
 // Cut cross-entropy statistics: logits = hidden[rows,d] * head[vocab,d]^T are reduced per
 // 256-column slab to pmax/psum[slab][row]; target_logit[row] is written by the slab that
-// holds the row's target (rows with target < 0 are never written).
+// holds the row's target (rows with target < 0 are never written).  `gathered`: an operand lies in a gathered buffer, so
+// that the same kernel computes the logits however far the gather has come (here and in ctb_ce_dlogits).
 CTB_API int ctb_ce_stats(const void* hidden, const void* head, int rows, int vocab, int d, long ldh, long ldw,
                          const int* targets, float* pmax, float* psum, float* target_logit, const unsigned* flags,
                          long flag_chunk, long flag_base, unsigned epoch, const unsigned* a_flags, long a_flag_chunk,
-                         long a_flag_base, unsigned a_epoch, int m_rotate, void* stream) {
+                         long a_flag_base, unsigned a_epoch, int m_rotate, int gathered, void* stream) {
   ctb::GemmCall c{};
+  c.gathered = gathered;
   c.b_flags = flags; c.b_flag_chunk = flag_chunk; c.b_flag_base = flag_base; c.b_flag_epoch = epoch;
   c.a_flags = a_flags; c.a_flag_chunk = a_flag_chunk; c.a_flag_base = a_flag_base; c.a_flag_epoch = a_epoch;
   c.m_rotate = m_rotate;
@@ -1014,16 +856,17 @@ CTB_API int ctb_ce_stats(const void* hidden, const void* head, int rows, int voc
 // Cut cross-entropy backward slab: G[rows,vocab] = (exp(logits - lse[row]) - onehot) * coef[row], bf16.
 CTB_API int ctb_ce_dlogits(const void* hidden, const void* head, void* g, int rows, int vocab, int d, long ldh,
                            long ldw, long ldg, const int* targets, const float* lse, const float* coef,
-                           void* stream) {
+                           int gathered, void* stream) {
   ctb::GemmCall c{};
+  c.gathered = gathered;
   c.A = hidden; c.B = head; c.C = g; c.M = rows; c.N = vocab; c.K = d; c.lda = ldh; c.ldb = ldw; c.ldc = ldg;
   c.epi = ctb::EPI_CE_DLOGITS; c.stream = stream;
   c.ce_targets = targets; c.ce_lse = lse; c.ce_coef = coef;
   return ctb::run_gemm(c);
 }
 
-// Which kernel a plain product with a 16-byte aligned bf16 output takes: 1 and the tile width and number of K
-// slices of the cluster kernel, or 0 for the persistent kernel.
+// Which kernel a plain product with a 16-byte aligned bf16 output takes where the two-CTA kernel (ctb_gemm_pair_choice) does
+// not: 1 and the tile width and number of K slices of the cluster kernel, or 0 for the persistent kernel.
 CTB_API int ctb_gemm_split_choice(int M, int N, int K, int* width, int* slices) {
   ctb::GemmCall c{};
   c.M = M; c.N = N; c.K = K; c.alpha = 1.f; c.epi = ctb::EPI_STORE;

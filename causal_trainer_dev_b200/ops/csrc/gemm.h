@@ -98,19 +98,27 @@ struct GemmCall {
   const float* ce_lse = nullptr;
   const float* ce_coef = nullptr;
   GemmPush push{};
+  void* workspace = nullptr;   // fp32 partial tiles of a product whose K range is split (gemm_pair.cu)
+  long workspace_bytes = 0;
 };
 
 int run_gemm(const GemmCall& call);
 
-// Two-CTA variant (gemm_pair.cu): plain products on clusters of two CTAs with
-// tcgen05.mma.cta_group::2, selected by run_gemm when the mode is on (CTB_GEMM_PAIR=1 or
-// ctb_gemm_set_pair) and the call has no gathered operand, fused epilogue or bias.
-bool gemm_pair_eligible(const GemmCall& c);
-int launch_gemm_pair(const GemmCall& c);
+// Two-CTA kernel (gemm_pair.cu): 256 tm x 256 tiles on clusters of two CTAs with tcgen05.mma.cta_group::2.  The tiles
+// before `whole` are computed in one piece; the K range of each of the others is cut into `slices`, whose fp32 partial
+// tiles go to the call's workspace and are added up by a second kernel.  `band` is the number of row tiles that the walk
+// covers before it moves on.  The plan is false where another kernel is the better one.
+struct PairPlan {
+  int tm, whole, slices, band;
+};
+bool gemm_pair_plan(const GemmCall& c, PairPlan* plan);
+bool gemm_pair_forced();
+long gemm_pair_workspace(const GemmCall& c, const PairPlan& plan);
+int launch_gemm_pair(const GemmCall& c, const PairPlan& plan);
 
 // Products with too few output tiles to fill the GPU (gemm_split.cu): the K range of a tile cut over the
 // CTAs of a cluster.  The plan is false where the persistent kernel is the better one.
-bool gemm_split_plan(const GemmCall& c, int* width, int* splits);
+bool gemm_split_plan(const GemmCall& c, int* width, int* splits, double* cycles = nullptr);
 int launch_gemm_split(const GemmCall& c, int width, int splits);
 
 }  // namespace ctb

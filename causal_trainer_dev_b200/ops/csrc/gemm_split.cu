@@ -338,7 +338,7 @@ int dispatch(const GemmCall& c, const CUtensorMap* ma, const CUtensorMap* mb, co
 // kernel and 14000 here, where the slices are exchanged.  Clusters of 8, 4 and 2 leave some SMs of a 148-SM
 // part unused: 14, 32 and 72 of them run at a time.  Examples (us, persistent -> here): 64 x 1536 x 8960
 // 49 -> 15, 333 x 1536 x 32000 199 -> 60, 1000 x 1536 x 17920 107 -> 62; 2000 x 1536 x 17920 stays (112, 111).
-bool gemm_split_plan(const GemmCall& c, int* width, int* splits) {
+bool gemm_split_plan(const GemmCall& c, int* width, int* splits, double* estimate) {
   if (c.epi != EPI_STORE || c.accumulate || c.push.enabled || c.max_ctas > 0) return false;
   // a gathered operand: with flags only the persistent kernel will do, and without them (the pull was done
   // before the call) the product must come out the same
@@ -362,6 +362,7 @@ bool gemm_split_plan(const GemmCall& c, int* width, int* splits) {
         best = cycles;
         *width = bn;
         *splits = s;
+        if (estimate != nullptr) *estimate = cycles;
         found = true;
       }
     }

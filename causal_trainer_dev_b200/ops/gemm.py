@@ -55,6 +55,12 @@ def _source_of(t: torch.Tensor) -> FlagSource | None:
     return None
 
 
+def in_gathered_buffer(*operands: torch.Tensor) -> bool:
+    """Whether an operand lies in a gathered buffer.  Its products stay on one kernel whether or not the pull has completed:
+    how far it has come must not decide the order of their sums."""
+    return bool(_FLAG_SOURCES) and any(_source_of(t) is not None for t in operands)
+
+
 def flag_source_of(t: torch.Tensor) -> tuple[FlagSource, int] | None:
     src = _source_of(t)
     if src is None or (src.complete is not None and src.complete.query()):
@@ -124,9 +130,8 @@ def gemm(
         raise ValueError("out must be [M,N] bf16/fp32 with unit inner stride")
     if bias is not None and (bias.dtype != torch.bfloat16 or bias.numel() != n):
         raise ValueError("bias must be bf16 of length N")
-    if _FLAG_SOURCES and (_source_of(b) is not None or _source_of(a) is not None):
-        # (a finished pull needs no flags, but the same kernel: how far a pull has come must not decide the
-        # order of the sums)
+    if in_gathered_buffer(a, b):
+        # (a finished pull needs no flags, but the same kernel)
         hit, hit_a = flag_source_of(b), flag_source_of(a)
         n_rotate, m_rotate = _rotations(hit, hit_a, a, b, a_mn, b_mn, m, n)
         bf = _flag_args(hit)
@@ -140,10 +145,14 @@ def gemm(
         )
         _lib.check(code, "ctb_gemm_flagged")
         return out
-    code = _lib.lib().ctb_gemm(
+    f32 = out.dtype == torch.float32
+    L = _lib.lib()
+    size = 0 if max_ctas > 0 else L.ctb_gemm_workspace(m, n, k, bool(a_mn), f32, bool(accumulate))
+    work = torch.empty(size, dtype=torch.uint8, device=a.device) if size else None
+    code = L.ctb_gemm(
         a.data_ptr(), b.data_ptr(), out.data_ptr(), m, n, k, a.stride(0), b.stride(0), out.stride(0),
-        bool(a_mn), bool(b_mn), out.dtype == torch.float32, bool(accumulate), float(alpha),
-        None if bias is None else bias.data_ptr(), max_ctas, _lib.raw_stream(),
+        bool(a_mn), bool(b_mn), f32, bool(accumulate), float(alpha), None if bias is None else bias.data_ptr(), max_ctas,
+        None if work is None else work.data_ptr(), size, _lib.raw_stream(),
     )
     _lib.check(code, "ctb_gemm")
     return out

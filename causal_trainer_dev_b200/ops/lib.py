@@ -20,7 +20,8 @@ from .build import LIB_PATH
 # the ctypes types).
 _KINDS = {"p": ctypes.c_void_p, "i": ctypes.c_int, "l": ctypes.c_long, "u": ctypes.c_uint, "f": ctypes.c_float}
 _SIGNATURES = {
-    "ctb_gemm": "pppiiillliiiifpip",
+    "ctb_gemm": "pppiiillliiiifpi" "plp",
+    "ctb_gemm_workspace": "iiiiii",
     "ctb_rmsnorm_fwd": "ppppppiifp",
     "ctb_rmsnorm_bwd": "ppppppppiiiip",
     "ctb_rope": "pppliiiiiip",
@@ -45,6 +46,7 @@ def _load() -> ctypes.CDLL | None:
     lib.ctb_last_error.restype = ctypes.c_char_p
     for name, kinds in _SIGNATURES.items():
         getattr(lib, name).argtypes = [_KINDS[k] for k in kinds]
+    lib.ctb_gemm_workspace.restype = ctypes.c_long
     return lib
 
 
