@@ -30,9 +30,22 @@ from ..models.params import ModelParams, Unit, embed_layout
 from ..ops import attention as attn_ops
 from ..ops import cross_entropy as ce
 from ..ops import elementwise as ew
+from ..ops import gemm as gemm_ops
+from ..ops import layer as layer_ops
 from ..ops import lib as _lib
 from ..ops.gemm import gemm
 from . import losses
+
+# Largest scratch block of a layer that is issued as one library call per direction: up to here (about 700 tokens of a
+# 1536-wide model, 5000 of a 256-wide one) a layer's device time is no longer than the host time of its launches from Python
+# (0.4 ms).  Above, the launches hide under the device's work, and one block would hold every intermediate to the end
+LAYER_CALL_BYTES = 64 << 20
+
+
+def _unused_pool_bytes() -> int:
+    """Bytes that PyTorch's allocator has from the driver and that no tensor uses (0 before its first use)."""
+    stats = torch.cuda.memory_stats_as_nested_dict()
+    return stats["reserved_bytes"]["all"]["current"] - stats["allocated_bytes"]["all"]["current"] if stats else 0
 
 
 class LocalProvider:
@@ -268,6 +281,18 @@ class LayerwiseEngine:
             saved = dict(x=x, rstd1=rstd1, qkv=qkv, o=o, lse=lse, h=h, rstd2=rstd2, gu=gu, routing=routing)
         return h, mlp, saved
 
+    def _layer_calls(self, ctx: dict, resid: torch.Tensor) -> layer_ops.LayerCalls | None:
+        """The layers of this pass as one library call per direction, where that is the same schedule (plain local weights
+        and gradients, dense attention, no tiling) and the batch is small enough for the host time to matter."""
+        o, prov = self.options, self.provider
+        if (type(self) is not LayerwiseEngine or type(prov) is not LocalProvider or not self.train_base
+                or o.attention_options is not None or o.mlp_chunk_rows > 0 or self._wgrad_stream is not None
+                or gemm_ops._FLAG_SOURCES or resid.dtype != torch.bfloat16
+                or any(prov.params.units[f"layer.{i}"].data.dtype != torch.bfloat16 for i in range(self.cfg.num_hidden_layers))):
+            return None
+        calls = layer_ops.LayerCalls(self.cfg, ctx, prov.grad_dtype, o.train_norm)
+        return calls if calls.scratch_bytes <= LAYER_CALL_BYTES else None
+
     # ------------------------------------------------------------------ layer backward
     def _layer_backward(self, w: dict[str, torch.Tensor], g: dict[str, torch.Tensor], sv: dict, dout: torch.Tensor,
                         ctx: dict, accumulate: bool, li: int = 0) -> torch.Tensor:
@@ -341,6 +366,11 @@ class LayerwiseEngine:
         from .memory_plan import backward_working_set_bytes, layer_activation_bytes
 
         per_layer = layer_activation_bytes(cfg, tokens)
+        chunk = min(self.options.cut_chunk_rows, tokens)
+        if _unused_pool_bytes() >= cfg.num_hidden_layers * per_layer + backward_working_set_bytes(cfg, tokens, chunk):
+            # the allocator holds a whole pass already, and the reserve is for what it would have to ask the driver for.
+            # Asking the driver waits for its locks, on a shared host 0.8 to 9 ms (at times 90), the allocator 10 us
+            return cfg.num_hidden_layers
         free, _ = torch.cuda.mem_get_info()
         working_set = backward_working_set_bytes(cfg, tokens, self.options.cut_chunk_rows)
         budget = free - working_set - self.options.memory_reserve_bytes
@@ -402,15 +432,21 @@ class LayerwiseEngine:
         keep_layers = self._layers_to_keep(resid.shape[0])
         self.kept_layers = keep_layers
         group = max(1, self.options.remat_group_size)
+        calls = self._layer_calls(ctx, resid)
         for li in range(nl):
             unit = prov.acquire(f"layer.{li}", prefetch=f"layer.{li + 1}" if li + 1 < nl else "final")
             # the last layers are kept first: their activations are consumed soonest
             keep = li >= nl - keep_layers
             # a recomputed layer keeps its input; with remat groups only the first layer of a group does
             inputs.append((resid, branch) if (not keep and li % group == 0) else None)
-            resid, branch, sv = self._layer_forward(self._views(unit), resid, branch, ctx, li,
-                                                    save="keep" if keep else None)
-            kept.append(sv)
+            if calls is not None:
+                resid, branch, sv = calls.forward(unit, resid, branch)
+                self._count(layer_ops.FORWARD_LAUNCHES)
+                kept.append(sv if keep else None)
+            else:
+                resid, branch, sv = self._layer_forward(self._views(unit), resid, branch, ctx, li,
+                                                        save="keep" if keep else None)
+                kept.append(sv)
             prov.release(f"layer.{li}")
         self._mark("layers forward")
         # ---------------- head: final norm + cut cross-entropy ----------------
@@ -418,7 +454,7 @@ class LayerwiseEngine:
         fw = self._views(final)
         fg = self._views(final, prov.grad_buffer("final")) if self.train_base else dict.fromkeys(fw)
         y, rstd_f, xf = ew.rmsnorm_forward(resid, fw["norm"], cfg.rms_norm_eps, residual=branch)
-        targets, weights = losses.aligned_targets_and_weights(batch)
+        targets, weights = losses.device_targets_and_weights(batch)
         targets, weights = self.select_tokens(targets).reshape(-1), self.select_tokens(weights).reshape(-1)
         train_head = self.options.train_lm_head and self.train_base
         # Active-row compaction: with sparse supervision (assistant-only loss, MaskGIT targets) only
@@ -472,12 +508,19 @@ class LayerwiseEngine:
                     x = inputs[j + 1] = (r, br)
             # the embedding table is not read in the backward pass: nothing to prefetch for layer 0
             unit = prov.acquire(f"layer.{li}", prefetch=f"layer.{li - 1}" if li > 0 else None)
-            w = self._views(unit)
-            g = self._views(unit, prov.grad_buffer(f"layer.{li}")) if self.train_base else dict.fromkeys(w)
             layer_in = inputs.pop()
-            if saved is None:
-                _, _, saved = self._layer_forward(w, layer_in[0], layer_in[1], ctx, li, save="all")
-            dout = self._layer_backward(w, g, saved, dout, ctx, accumulate, li)
+            if calls is not None:
+                if saved is None:
+                    _, _, saved = calls.forward(unit, *layer_in)
+                    self._count(layer_ops.FORWARD_LAUNCHES)
+                dout = calls.backward(unit, prov.grad_buffer(f"layer.{li}"), saved, dout, accumulate)
+                self._count(layer_ops.BACKWARD_LAUNCHES)
+            else:
+                w = self._views(unit)
+                g = self._views(unit, prov.grad_buffer(f"layer.{li}")) if self.train_base else dict.fromkeys(w)
+                if saved is None:
+                    _, _, saved = self._layer_forward(w, layer_in[0], layer_in[1], ctx, li, save="all")
+                dout = self._layer_backward(w, g, saved, dout, ctx, accumulate, li)
             del saved, layer_in
             self._join_wgrads()
             prov.release(f"layer.{li}")

@@ -15,6 +15,7 @@ import torch
 
 from ..models.decoder import canonicalize_segment_ids
 from ..ops import cross_entropy as ce
+from ..ops import lib as _lib
 
 
 def shifted_targets_and_weights(
@@ -77,6 +78,27 @@ def aligned_targets_and_weights(batch: dict[str, torch.Tensor]) -> tuple[torch.T
     pad_t = torch.zeros_like(targets[:, :1])
     pad_w = torch.zeros_like(weights[:, :1])
     return torch.cat([targets, pad_t], dim=1), torch.cat([weights, pad_w], dim=1)
+
+
+def device_targets_and_weights(batch: dict[str, torch.Tensor]) -> tuple[torch.Tensor, torch.Tensor]:
+    """:func:`aligned_targets_and_weights` for the engines.  The shifted rule of a plain batch on a GPU is one kernel
+    (targets come as int32, which the loss kernels take); anything else goes through the tensor formulation."""
+    ids, mask, labels, loss = (batch.get(k) for k in ("input_ids", "attention_mask", "segment_ids", "loss_weights"))
+    given = [t for t in (ids, mask, labels, loss) if t is not None]
+    integers = (torch.int64, torch.int32)
+    if ("prediction_targets" in batch or "prediction_weights" in batch or ids.dim() != 2
+            or any(not t.is_cuda or t.shape != ids.shape or not t.is_contiguous() for t in given)
+            or ids.dtype not in integers or (mask is not None and mask.dtype not in (*integers, torch.bool, torch.uint8))
+            or (labels is not None and labels.dtype not in integers) or (loss is not None and loss.dtype != torch.float32)):
+        return aligned_targets_and_weights(batch)
+    targets = torch.empty(ids.shape, dtype=torch.int32, device=ids.device)
+    weights = torch.empty(ids.shape, dtype=torch.float32, device=ids.device)
+    size = lambda t: 0 if t is None else t.element_size()  # noqa: E731
+    at = lambda t: None if t is None else t.data_ptr()  # noqa: E731
+    code = _lib.lib().ctb_loss_targets(at(ids), size(ids), at(mask), size(mask), at(labels), size(labels), at(loss),
+                                       targets.data_ptr(), weights.data_ptr(), *ids.shape, -100, _lib.raw_stream())
+    _lib.check(code, "ctb_loss_targets")
+    return targets, weights
 
 
 def linear_cross_entropy(hidden: torch.Tensor, head: torch.Tensor, targets: torch.Tensor, weights: torch.Tensor, *,

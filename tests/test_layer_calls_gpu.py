@@ -1,0 +1,70 @@
+"""Layers issued as one library call per direction, and next-token targets from one kernel, against the same schedule
+launch by launch from Python and against the tensor formulation: the same bits."""
+import pytest
+import torch
+
+pytestmark = pytest.mark.gpu
+
+
+def _batch(rows, seq, vocab, gen):
+    ids = torch.randint(3, vocab, (rows, seq), generator=gen, device="cuda")
+    mask = torch.ones_like(ids)
+    mask[-1, seq - 77:] = 0
+    seg = torch.ones_like(ids)
+    seg[:, seq // 3:] = 2
+    return dict(input_ids=ids, attention_mask=mask, segment_ids=seg)
+
+
+@pytest.mark.parametrize("options", [{}, {"remat": "full"}, {"remat": "full", "remat_group_size": 2}, {"train_norm": False}])
+@pytest.mark.parametrize("bias,style,grad_dtype", [(False, "gpt-neox", torch.bfloat16), (True, "gpt-j", torch.float32)])
+def test_a_pass_gives_the_same_bits_either_way(cuda_lib, monkeypatch, options, bias, style, grad_dtype):
+    from causal_trainer_dev_b200.models.config import preset
+    from causal_trainer_dev_b200.models.params import ModelParams
+    from causal_trainer_dev_b200.training import engine as E
+
+    cfg = preset("tiny", num_hidden_layers=3, vocab_size=1000, attention_bias=bias, rope_style=style)
+    gen = torch.Generator(device="cuda").manual_seed(3)
+    batches = [_batch(2, 384, 1000, gen) for _ in range(2)]
+    results = []
+    for limit in (E.LAYER_CALL_BYTES, 0):
+        monkeypatch.setattr(E, "LAYER_CALL_BYTES", limit)
+        params = ModelParams.init_random(cfg, seed=1).to("cuda")
+        engine = E.LayerwiseEngine(cfg, E.LocalProvider(params, grad_dtype), E.EngineOptions(**options))
+        sums = [engine(b, 1e-2, first=i == 0) for i, b in enumerate(batches)]
+        calls = engine._layer_calls(engine._context(batches[0]), torch.empty(768, cfg.hidden_size, dtype=torch.bfloat16, device="cuda"))
+        assert (calls is not None) == (limit > 0)
+        results.append([x for s in sums for x in s] + [u.grad for u in params.units.values()])
+    for a, b in zip(*results):
+        assert torch.equal(a, b)
+    assert all(bool(torch.isfinite(g.float()).all()) for g in results[0][4:])
+    assert cuda_lib.device_status() == (0, 0, 0, 0)
+
+
+@pytest.mark.parametrize("id_dtype", [torch.int64, torch.int32])
+@pytest.mark.parametrize("mask_dtype", [torch.int64, torch.int32, torch.bool, None])
+@pytest.mark.parametrize("labels", [True, False])
+@pytest.mark.parametrize("loss", [True, False])
+def test_targets_from_one_kernel(cuda_lib, id_dtype, mask_dtype, labels, loss):
+    from causal_trainer_dev_b200.training import losses
+
+    gen = torch.Generator(device="cuda").manual_seed(5)
+    b, s = 3, 333
+    ids = torch.randint(0, 50, (b, s), generator=gen, device="cuda").to(id_dtype)
+    ids[0, 7] = -100
+    batch = {"input_ids": ids}
+    if mask_dtype is not None:
+        mask = torch.rand(b, s, generator=gen, device="cuda") < 0.8
+        batch["attention_mask"] = mask.to(mask_dtype)
+        if mask_dtype == torch.int64:
+            batch["attention_mask"][1, 5:9] = 2                   # only 1 is valid
+    if labels:
+        batch["segment_ids"] = torch.randint(0, 2, (b, s), generator=gen, device="cuda")
+    if loss:
+        batch["loss_weights"] = torch.randn(b, s, generator=gen, device="cuda")
+    want_t, want_w = losses.aligned_targets_and_weights(batch)
+    before = cuda_lib.launch_count()
+    got_t, got_w = losses.device_targets_and_weights(batch)
+    assert cuda_lib.launch_count() == before + 1 and got_t.dtype == torch.int32
+    assert torch.equal(got_t.long(), want_t) and torch.equal(got_w, want_w)
+    batch["prediction_targets"], batch["prediction_weights"] = ids.long().abs(), torch.ones(b, s, device="cuda")
+    assert torch.equal(losses.device_targets_and_weights(batch)[0], losses.aligned_targets_and_weights(batch)[0])
