@@ -95,7 +95,7 @@ def cut_ce_forward(hidden, head, targets, weights, grad_scale: float | torch.Ten
     code = L.ctb_ce_stats(_lib.ptr(hidden), _lib.ptr(head), rows, vocab, d, ctypes.c_long(hidden.stride(0)),
                           ctypes.c_long(head.stride(0)), _lib.ptr(tgt), _lib.ptr(pmax), _lib.ptr(psum),
                           _lib.ptr(tlogit), *_flag_args(hit), *_flag_args(hit_a), m_rotate,
-                          int(in_gathered_buffer(hidden, head)), _lib.stream_ptr())
+                          int(in_gathered_buffer(hidden, head)), None, ctypes.c_long(0), _lib.stream_ptr())
     _lib.check(code, "ctb_ce_stats")
     if exchange is not None:
         nll, wsum, lse, coef = exchange.ce_exchange(pmax, psum, slabs, tlogit, w, grad_scale)
@@ -162,6 +162,75 @@ def cut_ce_backward(hidden, head, targets, lse, coef, *, chunk_rows: int = 4096,
             gemm(g, h, a_mn=True, b_mn=True, out=dhead, accumulate=(dhead_accumulate or not first))  # dW += G^T H
         first = False
     return dhidden, dhead
+
+
+# From this width on the logits of a chunk are kept in fp32 between the statistics and the gradient (forward and backward
+# called as one): writing and reading an element again takes 8 bytes of memory, recomputing it 2 x width operations.
+# Forward and backward, computed twice and kept, us: 2048 rows x 32000 x 512 325 and 311, x 768 393 and 361, 333 x 32000 x 1536
+# 212 and 181, 8192 x 168384 x 1536 12700 and 11850, 4096 x 128256 x 4096 12700 and 10400.  Narrower ones are not measured.
+KEEP_LOGITS_WIDTH = 512
+
+
+def cut_ce_forward_backward(hidden, head, targets, weights, grad_scale: float | torch.Tensor = 1.0, *, chunk_rows: int = 4096,
+                            need_dhead: bool = True, dhead_out: torch.Tensor | None = None, dhead_accumulate: bool = False):
+    """:func:`cut_ce_forward` and :func:`cut_ce_backward` in one: ``(nll_sum, weight_sum, dhidden, dhead)``, the same bits.
+
+    Row chunk by row chunk, so a chunk's fp32 logits can wait for their gradient (which takes their place) instead of being
+    computed twice, where that is cheaper and there is memory for them."""
+    rows, d = hidden.shape
+    vocab = head.shape[0]
+    from .gemm import in_gathered_buffer
+
+    chunk_rows = min(chunk_rows, rows)
+    slab = None
+    if d >= KEEP_LOGITS_WIDTH and vocab % 8 == 0 and (chunk_rows == rows or chunk_rows % 32 == 0) and not in_gathered_buffer(hidden, head):
+        try:
+            slab = torch.empty((chunk_rows, vocab), dtype=torch.float32, device=hidden.device)
+        except torch.cuda.OutOfMemoryError:
+            slab = None
+    if slab is None:
+        nll, wsum, lse, coef = cut_ce_forward(hidden, head, targets, weights, grad_scale)
+        dhidden, dhead = cut_ce_backward(hidden, head, targets, lse, coef, chunk_rows=chunk_rows, need_dhead=need_dhead,
+                                         dhead_out=dhead_out, dhead_accumulate=dhead_accumulate)
+        return nll, wsum, dhidden, dhead
+    dev = hidden.device
+    scale_on_device = grad_scale if isinstance(grad_scale, torch.Tensor) else None
+    scale = 1.0 if scale_on_device is not None else grad_scale
+    slabs = (vocab + SLAB - 1) // SLAB
+    f32 = lambda *shape: torch.empty(shape, dtype=torch.float32, device=dev)  # noqa: E731
+    pmax, psum = f32(slabs, chunk_rows), f32(slabs, chunk_rows)
+    tlogit = torch.zeros(rows, dtype=torch.float32, device=dev)
+    lse, coef, bn, bw = f32(rows), f32(rows), f32((rows + 31) // 32), f32((rows + 31) // 32)
+    tgt = targets.to(torch.int32).contiguous()
+    w = weights.to(torch.float32).contiguous()
+    dhidden = torch.empty_like(hidden)
+    dhead = None
+    if need_dhead:
+        dhead = dhead_out if dhead_out is not None else torch.empty((vocab, d), dtype=torch.bfloat16, device=dev)
+    L, ln = _lib.lib(), ctypes.c_long
+    for start in range(0, rows, chunk_rows):
+        n = min(chunk_rows, rows - start)
+        part = slice(start, start + n)
+        blocks = slice(start // 32, (start + n + 31) // 32)
+        h = hidden[part]
+        code = L.ctb_ce_stats(_lib.ptr(h), _lib.ptr(head), n, vocab, d, ln(h.stride(0)), ln(head.stride(0)), _lib.ptr(tgt[part]),
+                              _lib.ptr(pmax), _lib.ptr(psum), _lib.ptr(tlogit[part]), None, ln(0), ln(0), ctypes.c_uint(0), None,
+                              ln(0), ln(0), ctypes.c_uint(0), 0, 0, _lib.ptr(slab), ln(vocab), _lib.stream_ptr())
+        _lib.check(code, "ctb_ce_stats")
+        code = L.ctb_ce_combine(_lib.ptr(pmax), _lib.ptr(psum), slabs, _lib.ptr(tlogit[part]), _lib.ptr(w[part]),
+                                ctypes.c_float(scale), _lib.ptr(lse[part]), _lib.ptr(coef[part]), _lib.ptr(bn[blocks]),
+                                _lib.ptr(bw[blocks]), n, _lib.stream_ptr())
+        _lib.check(code, "ctb_ce_combine")
+        if scale_on_device is not None:
+            coef[part].mul_(scale_on_device.reshape(()).to(coef.dtype))
+        code = L.ctb_kept_logits_gradient(_lib.ptr(slab), ln(vocab), n, vocab, _lib.ptr(tgt[part]), _lib.ptr(lse[part]),
+                                          _lib.ptr(coef[part]), _lib.stream_ptr())
+        _lib.check(code, "ctb_kept_logits_gradient")
+        g = slab.view(torch.bfloat16)[:n, :vocab]
+        gemm(g, head, b_mn=True, out=dhidden[part])                                                    # dH = G @ W
+        if need_dhead:
+            gemm(g, h, a_mn=True, b_mn=True, out=dhead, accumulate=dhead_accumulate or start > 0)       # dW += G^T H
+    return bn.sum(), bw.sum(), dhidden, dhead
 
 
 def logits_ce_forward_backward(hidden, head, targets, weights, grad_scale: float = 1.0, *, chunk_rows: int = 4096,

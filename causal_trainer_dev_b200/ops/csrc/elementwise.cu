@@ -741,6 +741,49 @@ logits_ce_backward_kernel(__nv_bfloat16* __restrict__ logits, long ld, int vocab
 }
 
 // ------------------------------------------------------------------------------------------
+// Gradients of kept fp32 logits, bf16, in the place of the logits: row r of the gradient begins where row r of the logits
+// does.  A block walks a row in chunks; chunk k is written over logits that chunk k / 2 held, which every thread has read
+// when it has passed the barrier of chunk k.  The expression is the one of the GEMM epilogue that recomputes the logits.
+// Bound by memory: 6 bytes an element.
+// ------------------------------------------------------------------------------------------
+__global__ void __launch_bounds__(256)
+kept_logits_gradient_kernel(float* __restrict__ logits, long ld, int vocab, const int* __restrict__ targets,
+                            const float* __restrict__ lse, const float* __restrict__ coef) {
+  const long row = blockIdx.x;
+  const float* x = logits + row * ld;
+  __nv_bfloat16* g = reinterpret_cast<__nv_bfloat16*>(logits + row * ld);
+  const float l = lse[row], c = coef[row];
+  const int t = targets[row];
+  const int chunks = (vocab + 2047) / 2048;
+  float4 a[2], next[2] = {};
+  auto load = [&](int k, float4 (&to)[2]) {
+    const int col = k * 2048 + threadIdx.x * 8;
+    if (col < vocab) {
+      to[0] = __ldcs(reinterpret_cast<const float4*>(x + col));
+      to[1] = __ldcs(reinterpret_cast<const float4*>(x + col) + 1);
+    }
+  };
+  load(0, next);
+  for (int k = 0; k < chunks; ++k) {
+    a[0] = next[0];
+    a[1] = next[1];
+    if (k + 1 < chunks) load(k + 1, next);
+    const int col = k * 2048 + threadIdx.x * 8;
+    float v[8] = {a[0].x, a[0].y, a[0].z, a[0].w, a[1].x, a[1].y, a[1].z, a[1].w};
+#pragma unroll
+    for (int e = 0; e < 8; ++e) {
+      float pv = __expf(v[e] - l);
+      if (col + e == t) pv -= 1.f;
+      v[e] = pv * c;
+    }
+    __syncthreads();
+    if (col < vocab)
+      *reinterpret_cast<uint4*>(g + col) = make_uint4(pack_bf16(v[0], v[1]), pack_bf16(v[2], v[3]), pack_bf16(v[4], v[5]),
+                                                      pack_bf16(v[6], v[7]));
+  }
+}
+
+// ------------------------------------------------------------------------------------------
 // Sum of squares (fp32) of a bf16 / fp32 vector into per-block partials.
 // ------------------------------------------------------------------------------------------
 // 16-byte loads, four in flight per thread (with one element per load: 3.0 TB/s on 872 MB of fp32); a
@@ -1249,6 +1292,16 @@ CTB_API int ctb_logits_ce_backward(void* logits, long ld, int rows, int vocab, c
   if (rows <= 0) return 0;
   logits_ce_backward_kernel<<<rows, 256, 0, static_cast<cudaStream_t>(stream)>>>(
       static_cast<__nv_bfloat16*>(logits), ld, vocab, targets, lse, coef);
+  CTB_CUDA_OK(cudaGetLastError());
+  return 0;
+}
+
+// The gradient of kept logits in their place (see the kernel): rows of ld fp32 elements become rows of 2 ld bf16 elements.
+CTB_API int ctb_kept_logits_gradient(float* logits, long ld, int rows, int vocab, const int* targets, const float* lse,
+                                     const float* coef, void* stream) {
+  if (ld % 8 || vocab % 8 || ld < vocab) return fail("kept_logits: rows must be whole vectors of eight");
+  if (rows <= 0) return 0;
+  kept_logits_gradient_kernel<<<rows, 256, 0, static_cast<cudaStream_t>(stream)>>>(logits, ld, vocab, targets, lse, coef);
   CTB_CUDA_OK(cudaGetLastError());
   return 0;
 }

@@ -594,7 +594,7 @@ int run_gemm(const GemmCall& c) {
   using namespace gemm;
   if (c.M <= 0 || c.N <= 0 || c.K <= 0) return fail("gemm: M, N, K must be positive");
   if ((c.lda % 8) || (c.ldb % 8)) return fail("gemm: lda and ldb must be multiples of 8 elements (16 bytes)");
-  const bool needs_c = (c.epi != EPI_CE_STATS) && !c.push.enabled;
+  const bool needs_c = (c.epi != EPI_CE_STATS || c.C != nullptr) && !c.push.enabled;
   if (needs_c && (c.ldc % (c.out_f32 ? 4 : 8))) return fail("gemm: ldc must be a multiple of 16 bytes");
   PairPlan pair;
   if (gemm_pairs(c, &pair) && gemm_pair_workspace(c, pair) <= c.workspace_bytes) return launch_gemm_pair(c, pair);
@@ -645,6 +645,7 @@ int run_gemm(const GemmCall& c) {
   a.ce_target_logit = c.ce_target_logit;
   a.ce_lse = c.ce_lse;
   a.ce_coef = c.ce_coef;
+  a.ce_keep = c.epi == EPI_CE_STATS && c.C != nullptr;
   a.push = c.push;
   const bool dynamic_tiles = dynamic_tiles_mode();
   a.dynamic_tiles = dynamic_tiles ? 1 : 0;
@@ -837,12 +838,15 @@ CTB_API int ctb_gemm_push(const void* A, const void* B, int M, int N, int K, lon
 // Cut cross-entropy statistics: logits = hidden[rows,d] * head[vocab,d]^T are reduced per
 // 256-column slab to pmax/psum[slab][row]; target_logit[row] is written by the slab that
 // holds the row's target (rows with target < 0 are never written).  `gathered`: an operand lies in a gathered buffer, so
-// that the same kernel computes the logits however far the gather has come (here and in ctb_ce_dlogits).
+// that the same kernel computes the logits however far the gather has come (here and in ctb_ce_dlogits).  `logits` (null: not
+// wanted): where the fp32 logits go, rows of ldl elements.
 CTB_API int ctb_ce_stats(const void* hidden, const void* head, int rows, int vocab, int d, long ldh, long ldw,
                          const int* targets, float* pmax, float* psum, float* target_logit, const unsigned* flags,
                          long flag_chunk, long flag_base, unsigned epoch, const unsigned* a_flags, long a_flag_chunk,
-                         long a_flag_base, unsigned a_epoch, int m_rotate, int gathered, void* stream) {
+                         long a_flag_base, unsigned a_epoch, int m_rotate, int gathered, float* logits, long ldl,
+                         void* stream) {
   ctb::GemmCall c{};
+  c.C = logits; c.ldc = ldl; c.out_f32 = 1;
   c.gathered = gathered;
   c.b_flags = flags; c.b_flag_chunk = flag_chunk; c.b_flag_base = flag_base; c.b_flag_epoch = epoch;
   c.a_flags = a_flags; c.a_flag_chunk = a_flag_chunk; c.a_flag_base = a_flag_base; c.a_flag_epoch = a_epoch;

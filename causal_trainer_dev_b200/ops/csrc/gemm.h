@@ -59,6 +59,7 @@ struct GemmArgs {
   float* ce_target_logit;
   const float* ce_lse;
   const float* ce_coef;
+  int ce_keep;           // statistics: the fp32 logits are stored too
   GemmPush push;
   int* tile_counter;     // [2]: next tile to claim, CTAs that stopped claiming (dynamic_tiles only)
   int dynamic_tiles;

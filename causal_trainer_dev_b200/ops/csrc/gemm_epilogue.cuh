@@ -119,7 +119,15 @@ __device__ __forceinline__ void drain_slot(const GemmArgs& args, const CUtensorM
           has_target = true;
         }
       }
-      if (c + 1 < blocks) tmem_ld32(taddr + (c + 1) * 32, r);
+      if (args.ce_keep) {
+        uint32_t w[32];
+#pragma unroll
+        for (int j = 0; j < 32; ++j) w[j] = __float_as_uint(v[j]);
+        if (c + 1 < blocks) tmem_ld32(taddr + (c + 1) * 32, r);
+        store_rows<BUFS>(w, stage, staged, lane, map_c, col0, y, live, false);      // (columns behind the matrix are cut off)
+      } else if (c + 1 < blocks) {
+        tmem_ld32(taddr + (c + 1) * 32, r);
+      }
       const float nmax = fmaxf(vmax, cmax);
       float s = 0.f;
 #pragma unroll

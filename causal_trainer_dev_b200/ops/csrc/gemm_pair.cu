@@ -477,6 +477,7 @@ int run(const GemmCall& c, const PairPlan& plan) {
   a.ce_target_logit = c.ce_target_logit;
   a.ce_lse = c.ce_lse;
   a.ce_coef = c.ce_coef;
+  a.ce_keep = c.epi == EPI_CE_STATS && c.C != nullptr;
   PairArgs w{};
   w.num_m = (c.M + 2 * TM * BM - 1) / (2 * TM * BM);
   w.num_n = (c.N + BN - 1) / BN;
@@ -487,7 +488,7 @@ int run(const GemmCall& c, const PairPlan& plan) {
   const int rest = w.num_m * w.num_n - w.whole;
   w.units = w.whole + rest * w.slices;
   const CUtensorMap* mc = ma;      // placeholder where no C tensor is written
-  if (c.epi != EPI_CE_STATS) {
+  if (c.epi != EPI_CE_STATS || c.C != nullptr) {
     mc = c.out_f32 ? get_tensor_map_2d(c.C, Elt::F32, c.N, c.M, c.ldc, 32, 32, true)
                    : get_tensor_map_2d(c.C, Elt::BF16, c.N, c.M, c.ldc, 64, 32, true);
     if (!mc) return 1;

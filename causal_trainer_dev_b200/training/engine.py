@@ -480,10 +480,9 @@ class LayerwiseEngine:
                 y, fw["lm_head"], targets, weights, grad_scale, chunk_rows=self.options.cut_chunk_rows,
                 need_dhead=train_head, dhead_out=fg["lm_head"] if train_head else None, dhead_accumulate=accumulate)
         else:
-            nll, wsum, lse, coef = ce.cut_ce_forward(y, fw["lm_head"], targets, weights, grad_scale)
-            dy, _ = ce.cut_ce_backward(y, fw["lm_head"], targets, lse, coef, chunk_rows=self.options.cut_chunk_rows,
-                                       need_dhead=train_head, dhead_out=fg["lm_head"] if train_head else None,
-                                       dhead_accumulate=accumulate)
+            nll, wsum, dy, _ = ce.cut_ce_forward_backward(
+                y, fw["lm_head"], targets, weights, grad_scale, chunk_rows=self.options.cut_chunk_rows,
+                need_dhead=train_head, dhead_out=fg["lm_head"] if train_head else None, dhead_accumulate=accumulate)
         self._count(4 + 3 * ((y.shape[0] + self.options.cut_chunk_rows - 1) // self.options.cut_chunk_rows))
         if active is not None:
             dy, y = ew.scatter_rows(dy, active, n_active_dev, full_rows), y_all     # rows without loss get zero gradient
