@@ -41,10 +41,11 @@ __device__ __forceinline__ void tmem_loaded(uint32_t (&r)[32]) {
 }
 
 // Stages one 128-byte row per lane in the warp's block and sends the block's 32 rows to (x, y) of `map`.  `stage` is the
-// warp's 4 KiB of the first of BUFS staging buffers.
+// warp's 4 KiB of the first of BUFS staging buffers.  Every block that is staged is stored: with two buffers the wait lets
+// the newest store go on reading, which is the other buffer's only if each of the last `staged` blocks sent one.
 template <int BUFS>
 __device__ __forceinline__ void store_rows(const uint32_t (&w)[32], uint8_t* stage, uint32_t& staged, int lane,
-                                           const CUtensorMap* map, int x, int y, bool live, bool add) {
+                                           const CUtensorMap* map, int x, int y, bool add) {
   uint8_t* buf = stage + (BUFS == 2 ? (staged & 1u) * EPI_BUF : 0u);
   if (lane == 0) tma_wait_group_read<BUFS - 1>();      // the block may still be read by the store that used it last
   __syncwarp();
@@ -53,7 +54,7 @@ __device__ __forceinline__ void store_rows(const uint32_t (&w)[32], uint8_t* sta
     *reinterpret_cast<uint4*>(buf + sw128_offset(lane, j)) = make_uint4(w[4 * j], w[4 * j + 1], w[4 * j + 2], w[4 * j + 3]);
   fence_proxy_async_smem();
   __syncwarp();
-  if (lane == 0 && live) {
+  if (lane == 0) {
     if (add) tma_reduce_add_2d(map, buf, x, y);
     else tma_store_2d(map, buf, x, y);
     tma_commit_group();
@@ -64,7 +65,7 @@ __device__ __forceinline__ void store_rows(const uint32_t (&w)[32], uint8_t* sta
 // fp32 columns [0, columns) of the COLS at `taddr`, times alpha, to rows y and columns x of `map`.
 template <int COLS, int BUFS>
 __device__ __forceinline__ void drain_f32(uint32_t taddr, float alpha, int columns, uint8_t* stage, uint32_t& staged, int lane,
-                                          const CUtensorMap* map, int x, int y, bool live, bool add) {
+                                          const CUtensorMap* map, int x, int y, bool add) {
   const int blocks = min(COLS / 32, (columns + 31) / 32);
   uint32_t r[32];
   tmem_ld32(taddr, r);
@@ -75,7 +76,7 @@ __device__ __forceinline__ void drain_f32(uint32_t taddr, float alpha, int colum
 #pragma unroll
     for (int j = 0; j < 32; ++j) w[j] = __float_as_uint(__uint_as_float(r[j]) * alpha);
     if (c + 1 < blocks) tmem_ld32(taddr + (c + 1) * 32, r);      // on its way while this block is staged
-    store_rows<BUFS>(w, stage, staged, lane, map, x + c * 32, y, live, add);
+    store_rows<BUFS>(w, stage, staged, lane, map, x + c * 32, y, add);
   }
 }
 
@@ -95,7 +96,9 @@ __device__ __forceinline__ void drain_slot(const GemmArgs& args, const CUtensorM
   const int lane = etid & 31, quad = etid >> 5;
   uint8_t* stage = epi + quad * 4096;
   const int y = m_sub + quad * 32;
-  const bool live = y < args.M;
+  // All rows of the warp may, too: it has nothing to store, and so must stage nothing (store_rows).  (In the push epilogue
+  // the four warps meet at barriers.)
+  if (EPI != EPI_PUSH && y >= args.M) return;
   if (EPI == EPI_CE_STATS) {
     // Online softmax statistics of this 256-column slab for one row per thread.
     const int target = (grow < args.M) ? args.ce_targets[grow] : -1;
@@ -124,7 +127,7 @@ __device__ __forceinline__ void drain_slot(const GemmArgs& args, const CUtensorM
 #pragma unroll
         for (int j = 0; j < 32; ++j) w[j] = __float_as_uint(v[j]);
         if (c + 1 < blocks) tmem_ld32(taddr + (c + 1) * 32, r);
-        store_rows<BUFS>(w, stage, staged, lane, map_c, col0, y, live, false);      // (columns behind the matrix are cut off)
+        store_rows<BUFS>(w, stage, staged, lane, map_c, col0, y, false);      // (columns behind the matrix are cut off)
       } else if (c + 1 < blocks) {
         tmem_ld32(taddr + (c + 1) * 32, r);
       }
@@ -142,7 +145,7 @@ __device__ __forceinline__ void drain_slot(const GemmArgs& args, const CUtensorM
       if (has_target) args.ce_target_logit[grow] = tlogit;
     }
   } else if (args.out_f32) {
-    drain_f32<COLS, BUFS>(taddr, args.alpha, args.N - n0, stage, staged, lane, map_c, n0, y, live, add_into_c);
+    drain_f32<COLS, BUFS>(taddr, args.alpha, args.N - n0, stage, staged, lane, map_c, n0, y, add_into_c);
   } else {
     float lse = 0.f, coef = 0.f;
     int target = -1;
@@ -191,7 +194,7 @@ __device__ __forceinline__ void drain_slot(const GemmArgs& args, const CUtensorM
         tmem_ld32(taddr + (c + 1) * 64 + 32, r[1]);
       }
       if (EPI != EPI_PUSH) {
-        store_rows<BUFS>(w, stage, staged, lane, map_c, col0, y, live, add_into_c);
+        store_rows<BUFS>(w, stage, staged, lane, map_c, col0, y, add_into_c);
       } else {
         // reduce-scatter by push: the warpgroup's 128 threads copy the staged 128 x 128 B block into the
         // owner's receive buffer with 16-byte stores (peer memory: plain st.global only)

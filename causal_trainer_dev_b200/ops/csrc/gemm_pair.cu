@@ -341,7 +341,7 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constan
       if (EPI == EPI_STORE && u.part >= 0) {
         // fp32 partial tile [256 TM][256] of the workspace
         const int y = (u.part * 2 * TM + slot_of * 2 + static_cast<int>(rank)) * BM + q * 32;
-        gemm::drain_f32<C::EPI_COLS, C::EPI_BUFS>(taddr, 1.f, C::EPI_COLS, epi + q * 4096, staged, lane, &map_part, col_of, y, true,
+        gemm::drain_f32<C::EPI_COLS, C::EPI_BUFS>(taddr, 1.f, C::EPI_COLS, epi + q * 4096, staged, lane, &map_part, col_of, y,
                                                   false);
       } else {
         gemm::drain_slot<EPI, C::EPI_COLS, C::EPI_BUFS>(args, &map_c, taddr, u.n0 + col_of, m_sub, row, etid, bar_stage, epi,
