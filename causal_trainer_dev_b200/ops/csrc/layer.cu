@@ -46,14 +46,25 @@ struct Weights {
   const char *ln1, *ln2, *qkv_w, *qkv_b, *o_w, *o_b, *gu_w, *gu_b, *down_w, *down_b;
 };
 
+// A block that is cut into pieces; `size` is what the caller holds (0 while the pieces are only counted).
 struct Block {
   char* base;
+  long size = 0;
   long used = 0;
+  bool holds = true;        // the caller's block holds every piece so far
   template <typename T>
   T* take(long count) {
     T* at = reinterpret_cast<T*>(base + used);
-    used += (count * static_cast<long>(sizeof(T)) + 255) / 256 * 256;
+    const long end = used + count * static_cast<long>(sizeof(T));
+    holds = holds && end <= size;
+    used = (end + 255) / 256 * 256;
     return at;
+  }
+  // The products' workspace: what a counted block asks for, what a real one has left.  A product that finds less than it
+  // asked for takes a kernel that needs none, so a switch that is turned between the two costs speed and nothing else.
+  char* take_rest(long wanted, long* bytes) {
+    *bytes = base == nullptr ? wanted : (size > used ? size - used : 0);
+    return take<char>(*bytes);
   }
 };
 
@@ -94,11 +105,13 @@ struct Forward {
     normed = b.take<bf16>(z.t * s.hidden);
     branch = b.take<bf16>(z.t * s.hidden);
     act = b.take<bf16>(z.t * s.inner);
-    work_bytes = most(most(ctb_gemm_workspace(t, static_cast<int>(z.w), s.hidden, 0, 0, 0),
-                           ctb_gemm_workspace(t, s.hidden, static_cast<int>(z.qw), 0, 0, 0)),
-                      most(ctb_gemm_workspace(t, 2 * s.inner, s.hidden, 0, 0, 0),
-                           ctb_gemm_workspace(t, s.hidden, s.inner, 0, 0, 0)));
-    work = b.take<char>(work_bytes);
+    long wanted = 0;
+    if (b.base == nullptr)
+      wanted = most(most(ctb_gemm_workspace(t, static_cast<int>(z.w), s.hidden, 0, 0, 0),
+                         ctb_gemm_workspace(t, s.hidden, static_cast<int>(z.qw), 0, 0, 0)),
+                    most(ctb_gemm_workspace(t, 2 * s.inner, s.hidden, 0, 0, 0),
+                         ctb_gemm_workspace(t, s.hidden, s.inner, 0, 0, 0)));
+    work = b.take_rest(wanted, &work_bytes);
   }
 };
 
@@ -124,14 +137,13 @@ struct Backward {
                                static_cast<long>(ctb_column_sum_parts(t, w)) * w));
     no_grad = b.take<float>(s.hidden);
     rstd = b.take<float>(z.t);
-    work_bytes = 0;
+    long wanted = 0;
     const int shapes[8][3] = {{t, s.inner, s.hidden}, {s.hidden, s.inner, t}, {t, s.hidden, 2 * s.inner},
                               {2 * s.inner, s.hidden, t}, {t, qw, s.hidden}, {s.hidden, qw, t},
                               {t, s.hidden, w}, {w, s.hidden, t}};
-    for (int i = 0; i < 8; ++i)
-      work_bytes = most(work_bytes, ctb_gemm_workspace(shapes[i][0], shapes[i][1], shapes[i][2], i % 2,
-                                                       i % 2 ? s.grad_f32 : 0, 0));
-    work = b.take<char>(work_bytes);
+    for (int i = 0; i < 8 && b.base == nullptr; ++i)
+      wanted = most(wanted, ctb_gemm_workspace(shapes[i][0], shapes[i][1], shapes[i][2], i % 2, i % 2 ? s.grad_f32 : 0, 0));
+    work = b.take_rest(wanted, &work_bytes);
   }
 };
 
@@ -160,7 +172,7 @@ int project_backward(const void* dy, const void* x, const void* w, void* dx, voi
 }  // namespace layer
 }  // namespace ctb
 
-// Bytes of the kept block, of the forward call's and of the backward call's scratch block.
+// Bytes of the kept block, of the forward call's and of the backward call's scratch block, with the GEMM switches as they are.
 CTB_API void ctb_layer_bytes(const ctb::layer::Shape* s, long* kept, long* forward, long* backward) {
   using namespace ctb::layer;
   Block k{nullptr}, f{nullptr}, b{nullptr};
@@ -174,15 +186,17 @@ CTB_API void ctb_layer_bytes(const ctb::layer::Shape* s, long* kept, long* forwa
 
 // h = x + attention branch and mlp, with x = resid + branch (branch null: x = resid, and nothing is kept in x's place).
 CTB_API int ctb_layer_forward(const ctb::layer::Shape* sp, const ctb::layer::Context* cx, const ctb::layer::Weights* w,
-                              const void* resid, const void* branch, void* kept, void* scratch, void* h, void* mlp,
-                              void* stream) {
+                              const void* resid, const void* branch, void* kept, long kept_bytes, void* scratch,
+                              long scratch_bytes, void* h, void* mlp, void* stream) {
   using namespace ctb::layer;
   const Shape& s = *sp;
   const Sizes z(s);
   const int t = static_cast<int>(z.t);
-  Block kb{static_cast<char*>(kept)}, sb{static_cast<char*>(scratch)};
+  if (kept == nullptr || scratch == nullptr) return ctb::fail("layer: no blocks");
+  Block kb{static_cast<char*>(kept), kept_bytes}, sb{static_cast<char*>(scratch), scratch_bytes};
   const Kept k(s, kb);
   const Forward f(s, sb);
+  if (!kb.holds || !sb.holds) return ctb::fail("layer: a block is too small (ctb_layer_bytes)");
   const void* x = branch != nullptr ? k.x : resid;
   CTB_TRY(ctb_rmsnorm_fwd(resid, branch, w->ln1, f.normed, branch != nullptr ? k.x : nullptr, k.rstd1, t, s.hidden, s.eps, stream));
   CTB_TRY(project(f.normed, w->qkv_w, w->qkv_b, k.qkv, z.t, s.hidden, z.w, f.work, f.work_bytes, stream));
@@ -201,14 +215,17 @@ CTB_API int ctb_layer_forward(const ctb::layer::Shape* sp, const ctb::layer::Con
 // not wanted).  `x` is the layer's input (resid where there was no branch).
 CTB_API int ctb_layer_backward(const ctb::layer::Shape* sp, const ctb::layer::Context* cx, const ctb::layer::Weights* w,
                                const ctb::layer::Weights* grads, int accumulate, const void* x_or_null, const void* h,
-                               const void* dout, void* kept, void* scratch, void* dx, void* stream) {
+                               const void* dout, void* kept, long kept_bytes, void* scratch, long scratch_bytes, void* dx,
+                               void* stream) {
   using namespace ctb::layer;
   const Shape& s = *sp;
   const Sizes z(s);
   const int t = static_cast<int>(z.t);
-  Block kb{static_cast<char*>(kept)}, sb{static_cast<char*>(scratch)};
+  if (kept == nullptr || scratch == nullptr) return ctb::fail("layer: no blocks");
+  Block kb{static_cast<char*>(kept), kept_bytes}, sb{static_cast<char*>(scratch), scratch_bytes};
   const Kept k(s, kb);
   const Backward b(s, sb);
+  if (!kb.holds || !sb.holds) return ctb::fail("layer: a block is too small (ctb_layer_bytes)");
   auto at = [](const char* p) { return const_cast<char*>(p); };
   const void* x = x_or_null != nullptr ? x_or_null : k.x;
   // the memory-bound intermediates are cheaper to rebuild than to hold (the inverse norms of the forward pass stay)

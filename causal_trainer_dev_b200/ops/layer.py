@@ -7,7 +7,6 @@ from __future__ import annotations
 
 import ctypes
 import math
-from functools import lru_cache
 
 import torch
 
@@ -31,10 +30,10 @@ class _Weights(ctypes.Structure):
     _fields_ = [(n, _P) for n in ("ln1", "ln2", "qkv_w", "qkv_b", "o_w", "o_b", "gu_w", "gu_b", "down_w", "down_b")]
 
 
-@lru_cache(maxsize=256)
 def _plan(batch: int, seq: int, hidden: int, q_heads: int, kv_heads: int, head_dim: int, inner: int, rotary_dim: int,
           rope_style: int, grad_f32: int, eps: float) -> tuple[_Shape, int, int, int]:
-    """The shape as the library takes it, and the bytes of its three blocks."""
+    """The shape as the library takes it, and the bytes of its three blocks.  (They follow the GEMM switches and the device of
+    the moment, and take 10 us a pass to ask for: not kept.)"""
     shape = _Shape(batch, seq, hidden, q_heads, kv_heads, head_dim, inner, rotary_dim, rope_style, grad_f32, eps,
                    1.0 / math.sqrt(head_dim))
     sizes = [ctypes.c_long() for _ in range(3)]
@@ -79,8 +78,8 @@ class LayerCalls:
         scratch = torch.empty(self._forward, dtype=torch.uint8, device=dev)
         code = _lib.lib().ctb_layer_forward(
             ctypes.byref(self._shape), ctypes.byref(self._context), ctypes.byref(_pointers(unit.layout, unit.data)),
-            resid.data_ptr(), None if branch is None else branch.data_ptr(), kept.data_ptr(), scratch.data_ptr(), h.data_ptr(),
-            mlp.data_ptr(), _lib.raw_stream())
+            resid.data_ptr(), None if branch is None else branch.data_ptr(), kept.data_ptr(), kept.numel(), scratch.data_ptr(),
+            scratch.numel(), h.data_ptr(), mlp.data_ptr(), _lib.raw_stream())
         _lib.check(code, "ctb_layer_forward", FORWARD_LAUNCHES)
         return h, mlp, (resid if branch is None else None, h, kept)
 
@@ -92,6 +91,7 @@ class LayerCalls:
         code = _lib.lib().ctb_layer_backward(
             ctypes.byref(self._shape), ctypes.byref(self._context), ctypes.byref(_pointers(unit.layout, unit.data)),
             ctypes.byref(_pointers(unit.layout, grads, self._no_grad)), accumulate, None if x is None else x.data_ptr(),
-            h.data_ptr(), dout.data_ptr(), kept.data_ptr(), scratch.data_ptr(), dx.data_ptr(), _lib.raw_stream())
+            h.data_ptr(), dout.data_ptr(), kept.data_ptr(), kept.numel(), scratch.data_ptr(), scratch.numel(), dx.data_ptr(),
+            _lib.raw_stream())
         _lib.check(code, "ctb_layer_backward", BACKWARD_LAUNCHES)
         return dx

@@ -30,8 +30,8 @@ _SIGNATURES = {
     "ctb_attn_bwd_stats": "pppppiiiillp",
     "ctb_attn_fwd_range": "pppppppppp" "iiiiiii" "llll" "flp",
     "ctb_attn_fwd_gathered": "pppppppppp" "iiiiiii" "llll" "f" "pllu" "lp",
-    "ctb_layer_forward": "pppppppppp",
-    "ctb_layer_backward": "ppppipppppp" "p",
+    "ctb_layer_forward": "pppppplplppp",
+    "ctb_layer_backward": "ppppippp" "plplpp",
     "ctb_loss_targets": "pipipipppiiip",
     "ctb_attn_bwd_range": "ppppppppppp" "ppppppppp" "iiiiiii" "llllllll" "flp",
 }

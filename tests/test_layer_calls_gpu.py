@@ -68,3 +68,29 @@ def test_targets_from_one_kernel(cuda_lib, id_dtype, mask_dtype, labels, loss):
     assert torch.equal(got_t.long(), want_t) and torch.equal(got_w, want_w)
     batch["prediction_targets"], batch["prediction_weights"] = ids.long().abs(), torch.ones(b, s, device="cuda")
     assert torch.equal(losses.device_targets_and_weights(batch)[0], losses.aligned_targets_and_weights(batch)[0])
+
+
+def test_a_switch_turned_between_the_passes(cuda_lib):
+    """Blocks are sized for the products' kernels of the moment: a pass with the two-CTA kernel off, one with it, and the
+    other way round, each the same bits as a pass of its own."""
+    from causal_trainer_dev_b200.models.config import preset
+    from causal_trainer_dev_b200.models.params import ModelParams
+    from causal_trainer_dev_b200.training import engine as E
+
+    cfg = preset("qwen2.5-1.5b-image", num_hidden_layers=1, vocab_size=1000)
+    batch = _batch(1, 384, 1000, torch.Generator(device="cuda").manual_seed(3))
+    set_pair = cuda_lib.lib().ctb_gemm_set_pair
+    before = set_pair(-1)
+    try:
+        seen = {}
+        for mode in (0, -1, 0, -1):
+            set_pair(mode)
+            params = ModelParams.init_random(cfg, seed=1).to("cuda")
+            engine = E.LayerwiseEngine(cfg, E.LocalProvider(params, torch.bfloat16))
+            sums = engine(batch, 1e-2, first=True)
+            assert engine._layer_calls(engine._context(batch), torch.empty(384, cfg.hidden_size, dtype=torch.bfloat16, device="cuda"))
+            got = [*sums, *(u.grad for u in params.units.values())]
+            assert all(torch.equal(a, b) for a, b in zip(seen.setdefault(mode, got), got))
+    finally:
+        set_pair(before)
+    assert cuda_lib.device_status() == (0, 0, 0, 0)
