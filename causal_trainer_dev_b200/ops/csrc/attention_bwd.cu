@@ -870,7 +870,7 @@ template <int D, int MODE>
 int prepare_bwd(const BwdCall& c, BwdMaps* maps, BwdArgs* args, int* items) {
   const bool grouped = c.grp.desc != nullptr;
   const int Sq = grouped ? c.gathered_rows : (c.Sq > 0 ? c.Sq : c.S);
-  auto make = [&](const void* base, int heads, long row_stride, int rows, int seq, int batches) -> const CUtensorMap* {
+  auto make = [&](const void* base, int heads, long row_stride, int rows, int seq, int batches) -> TensorMap {
     const uint64_t dims[4] = {static_cast<uint64_t>(D), static_cast<uint64_t>(heads), static_cast<uint64_t>(seq),
                               static_cast<uint64_t>(batches)};
     const uint64_t strides[3] = {static_cast<uint64_t>(D), static_cast<uint64_t>(row_stride),
@@ -882,13 +882,13 @@ int prepare_bwd(const BwdCall& c, BwdMaps* maps, BwdArgs* args, int* items) {
   // Resident operands use 128-row boxes, streamed operands 64-row boxes.
   // grouped: Q / dO / dQ are the gathered rows (one batch, one head)
   const int qh = grouped ? 1 : c.Hq, qb = grouped ? 1 : c.B;
-  const CUtensorMap* mq = make(c.q, qh, c.q_row_stride, DKV ? 64 : 128, Sq, qb);
-  const CUtensorMap* mk = make(c.k, c.Hkv, c.k_row_stride, DKV ? 128 : 64, c.S, c.B);
-  const CUtensorMap* mv = make(c.v, c.Hkv, c.v_row_stride, DKV ? 128 : 64, c.S, c.B);
-  const CUtensorMap* mdo = make(c.dout, qh, c.do_row_stride, DKV ? 64 : 128, Sq, qb);
-  const CUtensorMap* mo1 = DKV ? make(c.dv, c.Hkv, c.dv_row_stride, 128, c.S, c.B)
-                               : make(c.dq, qh, c.dq_row_stride, 128, Sq, qb);
-  const CUtensorMap* mo2 = DKV ? make(c.dk, c.Hkv, c.dk_row_stride, 128, c.S, c.B) : mo1;
+  const TensorMap mq = make(c.q, qh, c.q_row_stride, DKV ? 64 : 128, Sq, qb);
+  const TensorMap mk = make(c.k, c.Hkv, c.k_row_stride, DKV ? 128 : 64, c.S, c.B);
+  const TensorMap mv = make(c.v, c.Hkv, c.v_row_stride, DKV ? 128 : 64, c.S, c.B);
+  const TensorMap mdo = make(c.dout, qh, c.do_row_stride, DKV ? 64 : 128, Sq, qb);
+  const TensorMap mo1 = DKV ? make(c.dv, c.Hkv, c.dv_row_stride, 128, c.S, c.B)
+                            : make(c.dq, qh, c.dq_row_stride, 128, Sq, qb);
+  const TensorMap mo2 = DKV ? make(c.dk, c.Hkv, c.dk_row_stride, 128, c.S, c.B) : mo1;
   if (!mq || !mk || !mv || !mdo || !mo1 || !mo2) return 1;
   BwdArgs a{};
   a.B = c.B; a.S = c.S; a.Hq = c.Hq; a.Hkv = c.Hkv;
@@ -902,7 +902,7 @@ int prepare_bwd(const BwdCall& c, BwdMaps* maps, BwdArgs* args, int* items) {
   a.grp = c.grp;
   a.status = device_status();
   a.spin_budget = c.spin_budget > 0 ? c.spin_budget : CTB_SPIN_BUDGET;
-  *maps = BwdMaps{*mq, *mk, *mv, *mdo, *mo1, *mo2};
+  *maps = BwdMaps{mq.map, mk.map, mv.map, mdo.map, mo1.map, mo2.map};
   *args = a;
   *items = grouped ? c.ctas : (DKV ? c.B * c.Hkv * (c.S / 128) : c.B * c.Hq * (Sq / 128));
   return 0;

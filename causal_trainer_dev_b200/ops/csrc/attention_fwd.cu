@@ -703,10 +703,10 @@ int launch_fwd_as(const FwdCall& c) {
                           static_cast<uint64_t>(c.v_row_stride) * c.S};
   const uint64_t so[3] = {static_cast<uint64_t>(D), static_cast<uint64_t>(c.o_row_stride),
                           static_cast<uint64_t>(c.o_row_stride) * Sq};
-  const CUtensorMap* mq = get_tensor_map_4d(c.q, Elt::BF16, dq, sq, box, true);
-  const CUtensorMap* mk = get_tensor_map_4d(c.k, Elt::BF16, dk, sk, box, true);
-  const CUtensorMap* mv = get_tensor_map_4d(c.v, Elt::BF16, dk, sv, box, true);
-  const CUtensorMap* mo = get_tensor_map_4d(c.o, Elt::BF16, dq, so, box, true);
+  const TensorMap mq = get_tensor_map_4d(c.q, Elt::BF16, dq, sq, box, true);
+  const TensorMap mk = get_tensor_map_4d(c.k, Elt::BF16, dk, sk, box, true);
+  const TensorMap mv = get_tensor_map_4d(c.v, Elt::BF16, dk, sv, box, true);
+  const TensorMap mo = get_tensor_map_4d(c.o, Elt::BF16, dq, so, box, true);
   if (!mq || !mk || !mv || !mo) return 1;
   FwdArgs a{};
   a.B = c.B; a.S = c.S; a.Hq = grouped ? 1 : c.Hq; a.Hkv = grouped ? 1 : c.Hkv;
@@ -728,7 +728,7 @@ int launch_fwd_as(const FwdCall& c) {
     configured_dev = dev;
   }
   const int grid = grouped ? Sq / 256 : c.B * c.Hq * ((Sq + 255) / 256);
-  kern<<<grid, FWD_THREADS, L::BYTES, static_cast<cudaStream_t>(c.stream)>>>(*mq, *mk, *mv, *mo, a);
+  kern<<<grid, FWD_THREADS, L::BYTES, static_cast<cudaStream_t>(c.stream)>>>(mq.map, mk.map, mv.map, mo.map, a);
   CTB_CUDA_OK(cudaGetLastError());
   return 0;
 }

@@ -556,7 +556,7 @@ inline int* next_tile_counter() {
 }
 
 template <int TM, bool A_MN, bool B_MN, int EPI>
-int launch(const CUtensorMap* ma, const CUtensorMap* mb, const CUtensorMap* mc, const GemmArgs& args, int grid,
+int launch(const TensorMap& ma, const TensorMap& mb, const TensorMap& mc, const GemmArgs& args, int grid,
            cudaStream_t stream) {
   using C = Cfg<TM>;
   auto kern = gemm_kernel<TM, A_MN, B_MN, EPI>;
@@ -567,7 +567,7 @@ int launch(const CUtensorMap* ma, const CUtensorMap* mb, const CUtensorMap* mc, 
     CTB_CUDA_OK(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, C::SMEM_BYTES));
     configured_dev = dev;
   }
-  kern<<<grid, C::THREADS, C::SMEM_BYTES, stream>>>(*ma, *mb, *mc, args);
+  kern<<<grid, C::THREADS, C::SMEM_BYTES, stream>>>(ma.map, mb.map, mc.map, args);
   CTB_CUDA_OK(cudaGetLastError());
   return 0;
 }
@@ -600,13 +600,13 @@ int run_gemm(const GemmCall& c) {
   if (gemm_pairs(c, &pair) && gemm_pair_workspace(c, pair) <= c.workspace_bytes) return launch_gemm_pair(c, pair);
   int split_width = 0, split_slices = 0;
   if (gemm_splits(c, &split_width, &split_slices)) return launch_gemm_split(c, split_width, split_slices);
-  const CUtensorMap* ma = c.a_mn ? get_tensor_map_2d(c.A, Elt::BF16, c.M, c.K, c.lda, 64, 64, true)
-                                 : get_tensor_map_2d(c.A, Elt::BF16, c.K, c.M, c.lda, 64, BM, true);
+  const TensorMap ma = c.a_mn ? get_tensor_map_2d(c.A, Elt::BF16, c.M, c.K, c.lda, 64, 64, true)
+                             : get_tensor_map_2d(c.A, Elt::BF16, c.K, c.M, c.lda, 64, BM, true);
   if (!ma) return 1;
-  const CUtensorMap* mb = c.b_mn ? get_tensor_map_2d(c.B, Elt::BF16, c.N, c.K, c.ldb, 64, 64, true)
-                                 : get_tensor_map_2d(c.B, Elt::BF16, c.K, c.N, c.ldb, 64, BN, true);
+  const TensorMap mb = c.b_mn ? get_tensor_map_2d(c.B, Elt::BF16, c.N, c.K, c.ldb, 64, 64, true)
+                             : get_tensor_map_2d(c.B, Elt::BF16, c.K, c.N, c.ldb, 64, BN, true);
   if (!mb) return 1;
-  const CUtensorMap* mc = ma;  // placeholder when no C tensor is written
+  TensorMap mc = ma;  // placeholder when no C tensor is written
   if (needs_c) {
     mc = c.out_f32 ? get_tensor_map_2d(c.C, Elt::F32, c.N, c.M, c.ldc, 32, 32, true)
                    : get_tensor_map_2d(c.C, Elt::BF16, c.N, c.M, c.ldc, 64, 32, true);

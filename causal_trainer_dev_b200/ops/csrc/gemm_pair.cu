@@ -417,7 +417,7 @@ __global__ void __launch_bounds__(256) pair_reduce_kernel(const float* __restric
 }
 
 template <int TM, bool A_MN, bool B_MN, int EPI>
-int launch(const CUtensorMap* ma, const CUtensorMap* mb, const CUtensorMap* mc, const CUtensorMap* mp, const GemmArgs& a,
+int launch(const TensorMap& ma, const TensorMap& mb, const TensorMap& mc, const TensorMap& mp, const GemmArgs& a,
            const PairArgs& w, cudaStream_t s) {
   auto kern = gemm_pair_kernel<TM, A_MN, B_MN, EPI>;
   static int configured_dev = -1;
@@ -439,12 +439,12 @@ int launch(const CUtensorMap* ma, const CUtensorMap* mb, const CUtensorMap* mc, 
   attr[0].val.clusterDim.z = 1;
   cfg.attrs = attr;
   cfg.numAttrs = 1;
-  CTB_CUDA_OK(cudaLaunchKernelEx(&cfg, kern, *ma, *mb, *mc, *mp, a, w));
+  CTB_CUDA_OK(cudaLaunchKernelEx(&cfg, kern, ma.map, mb.map, mc.map, mp.map, a, w));
   return 0;
 }
 
 template <int TM, int EPI>
-int dispatch(const GemmCall& c, const CUtensorMap* ma, const CUtensorMap* mb, const CUtensorMap* mc, const CUtensorMap* mp,
+int dispatch(const GemmCall& c, const TensorMap& ma, const TensorMap& mb, const TensorMap& mc, const TensorMap& mp,
              const GemmArgs& a, const PairArgs& w) {
   cudaStream_t s = static_cast<cudaStream_t>(c.stream);
   if (!c.a_mn && !c.b_mn) return launch<TM, false, false, EPI>(ma, mb, mc, mp, a, w, s);
@@ -456,10 +456,10 @@ int dispatch(const GemmCall& c, const CUtensorMap* ma, const CUtensorMap* mb, co
 
 template <int TM>
 int run(const GemmCall& c, const PairPlan& plan) {
-  const CUtensorMap* ma = c.a_mn ? get_tensor_map_2d(c.A, Elt::BF16, c.M, c.K, c.lda, 64, 64, true)
-                                 : get_tensor_map_2d(c.A, Elt::BF16, c.K, c.M, c.lda, 64, 128, true);
-  const CUtensorMap* mb = c.b_mn ? get_tensor_map_2d(c.B, Elt::BF16, c.N, c.K, c.ldb, 64, 64, true)
-                                 : get_tensor_map_2d(c.B, Elt::BF16, c.K, c.N, c.ldb, 64, 128, true);
+  const TensorMap ma = c.a_mn ? get_tensor_map_2d(c.A, Elt::BF16, c.M, c.K, c.lda, 64, 64, true)
+                             : get_tensor_map_2d(c.A, Elt::BF16, c.K, c.M, c.lda, 64, 128, true);
+  const TensorMap mb = c.b_mn ? get_tensor_map_2d(c.B, Elt::BF16, c.N, c.K, c.ldb, 64, 64, true)
+                             : get_tensor_map_2d(c.B, Elt::BF16, c.K, c.N, c.ldb, 64, 128, true);
   if (!ma || !mb) return 1;
   GemmArgs a{};
   a.M = c.M;
@@ -487,13 +487,13 @@ int run(const GemmCall& c, const PairPlan& plan) {
   w.band = plan.band;
   const int rest = w.num_m * w.num_n - w.whole;
   w.units = w.whole + rest * w.slices;
-  const CUtensorMap* mc = ma;      // placeholder where no C tensor is written
+  TensorMap mc = ma;      // placeholder where no C tensor is written
   if (c.epi != EPI_CE_STATS || c.C != nullptr) {
     mc = c.out_f32 ? get_tensor_map_2d(c.C, Elt::F32, c.N, c.M, c.ldc, 32, 32, true)
                    : get_tensor_map_2d(c.C, Elt::BF16, c.N, c.M, c.ldc, 64, 32, true);
     if (!mc) return 1;
   }
-  const CUtensorMap* mp = ma;
+  TensorMap mp = ma;
   if (rest > 0) {
     mp = get_tensor_map_2d(c.workspace, Elt::F32, BN, static_cast<uint64_t>(rest) * w.slices * 2 * TM * BM, BN, 32, 32, true);
     if (!mp) return 1;

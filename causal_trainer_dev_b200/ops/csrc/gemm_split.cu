@@ -296,7 +296,7 @@ gemm_split_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_consta
 }
 
 template <int BN, bool A_MN, bool B_MN>
-int launch(const CUtensorMap* ma, const CUtensorMap* mb, const SplitArgs& a, int tiles, cudaStream_t s) {
+int launch(const TensorMap& ma, const TensorMap& mb, const SplitArgs& a, int tiles, cudaStream_t s) {
   auto kern = gemm_split_kernel<BN, A_MN, B_MN>;
   static int configured_dev = -1;
   int dev = 0;
@@ -317,12 +317,12 @@ int launch(const CUtensorMap* ma, const CUtensorMap* mb, const SplitArgs& a, int
   attr[0].val.clusterDim.z = 1;
   cfg.attrs = attr;
   cfg.numAttrs = 1;
-  CTB_CUDA_OK(cudaLaunchKernelEx(&cfg, kern, *ma, *mb, a));
+  CTB_CUDA_OK(cudaLaunchKernelEx(&cfg, kern, ma.map, mb.map, a));
   return 0;
 }
 
 template <int BN>
-int dispatch(const GemmCall& c, const CUtensorMap* ma, const CUtensorMap* mb, const SplitArgs& a, int tiles) {
+int dispatch(const GemmCall& c, const TensorMap& ma, const TensorMap& mb, const SplitArgs& a, int tiles) {
   cudaStream_t s = static_cast<cudaStream_t>(c.stream);
   if (!c.a_mn && !c.b_mn) return launch<BN, false, false>(ma, mb, a, tiles, s);
   if (!c.a_mn && c.b_mn) return launch<BN, false, true>(ma, mb, a, tiles, s);
@@ -371,11 +371,11 @@ bool gemm_split_plan(const GemmCall& c, int* width, int* splits, double* estimat
 }
 
 int launch_gemm_split(const GemmCall& c, int width, int splits) {
-  const CUtensorMap* ma = c.a_mn ? get_tensor_map_2d(c.A, Elt::BF16, c.M, c.K, c.lda, 64, 64, true)
-                                 : get_tensor_map_2d(c.A, Elt::BF16, c.K, c.M, c.lda, 64, 128, true);
+  const TensorMap ma = c.a_mn ? get_tensor_map_2d(c.A, Elt::BF16, c.M, c.K, c.lda, 64, 64, true)
+                             : get_tensor_map_2d(c.A, Elt::BF16, c.K, c.M, c.lda, 64, 128, true);
   if (!ma) return 1;
-  const CUtensorMap* mb = c.b_mn ? get_tensor_map_2d(c.B, Elt::BF16, c.N, c.K, c.ldb, 64, 64, true)
-                                 : get_tensor_map_2d(c.B, Elt::BF16, c.K, c.N, c.ldb, 64, width, true);
+  const TensorMap mb = c.b_mn ? get_tensor_map_2d(c.B, Elt::BF16, c.N, c.K, c.ldb, 64, 64, true)
+                             : get_tensor_map_2d(c.B, Elt::BF16, c.K, c.N, c.ldb, 64, width, true);
   if (!mb) return 1;
   gemm3::SplitArgs a{};
   a.M = c.M; a.N = c.N; a.K = c.K;

@@ -51,17 +51,23 @@ struct MapKeyHash {
 };
 
 std::mutex g_map_mutex;
-std::unordered_map<MapKey, CUtensorMap*, MapKeyHash> g_maps;
+std::unordered_map<MapKey, CUtensorMap, MapKeyHash> g_maps;
+size_t g_map_limit = 65536;      // maps are 128 bytes, but addresses change as the allocator reuses memory
 
-const CUtensorMap* lookup_or_encode(const MapKey& key, const void* base, Elt elt, uint32_t rank, const uint64_t* dims,
-                                    const uint64_t* strides_elems, const uint32_t* box, bool swizzle128) {
+TensorMap lookup_or_encode(const MapKey& key, const void* base, Elt elt, uint32_t rank, const uint64_t* dims,
+                           const uint64_t* strides_elems, const uint32_t* box, bool swizzle128) {
   std::lock_guard<std::mutex> lock(g_map_mutex);
+  TensorMap out;
   auto it = g_maps.find(key);
-  if (it != g_maps.end()) return it->second;
+  if (it != g_maps.end()) {
+    out.map = it->second;
+    out.ok = true;
+    return out;
+  }
   EncodeFn fn = encode_fn();
   if (fn == nullptr) {
     set_error("cuTensorMapEncodeTiled is not available from this driver");
-    return nullptr;
+    return out;
   }
   const uint64_t esize = (elt == Elt::BF16) ? 2 : 4;
   cuuint64_t gdims[4];
@@ -73,29 +79,25 @@ const CUtensorMap* lookup_or_encode(const MapKey& key, const void* base, Elt elt
     gbox[i] = box[i];
   }
   for (uint32_t i = 0; i + 1 < rank; ++i) gstrides[i] = strides_elems[i] * esize;
-  auto* map = new CUtensorMap;
-  CUresult r = fn(map, elt == Elt::BF16 ? CU_TENSOR_MAP_DATA_TYPE_BFLOAT16 : CU_TENSOR_MAP_DATA_TYPE_FLOAT32, rank,
+  CUresult r = fn(&out.map, elt == Elt::BF16 ? CU_TENSOR_MAP_DATA_TYPE_BFLOAT16 : CU_TENSOR_MAP_DATA_TYPE_FLOAT32, rank,
                   const_cast<void*>(base), gdims, gstrides, gbox, estr, CU_TENSOR_MAP_INTERLEAVE_NONE,
                   swizzle128 ? CU_TENSOR_MAP_SWIZZLE_128B : CU_TENSOR_MAP_SWIZZLE_NONE,
                   CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
   if (r != CUDA_SUCCESS) {
-    delete map;
     set_error("cuTensorMapEncodeTiled failed with code " + std::to_string(static_cast<int>(r)) +
               " (base must be 16-byte aligned, strides multiples of 16 bytes)");
-    return nullptr;
+    return out;
   }
-  if (g_maps.size() > 65536) {  // bound the cache; maps are tiny but pointers churn under allocator reuse
-    for (auto& kv : g_maps) delete kv.second;
-    g_maps.clear();
-  }
-  g_maps.emplace(key, map);
-  return map;
+  if (g_maps.size() >= g_map_limit) g_maps.clear();
+  g_maps.emplace(key, out.map);
+  out.ok = true;
+  return out;
 }
 
 }  // namespace
 
-const CUtensorMap* get_tensor_map_2d(const void* base, Elt elt, uint64_t inner, uint64_t outer, uint64_t row_stride,
-                                     uint32_t box_inner, uint32_t box_outer, bool swizzle128) {
+TensorMap get_tensor_map_2d(const void* base, Elt elt, uint64_t inner, uint64_t outer, uint64_t row_stride,
+                            uint32_t box_inner, uint32_t box_outer, bool swizzle128) {
   MapKey key{};
   key.v[0] = reinterpret_cast<uint64_t>(base);
   key.v[1] = static_cast<uint64_t>(elt) | (2ull << 8) | (swizzle128 ? 1ull << 16 : 0);
@@ -113,30 +115,8 @@ const CUtensorMap* get_tensor_map_2d(const void* base, Elt elt, uint64_t inner, 
   return lookup_or_encode(key, base, elt, 2, dims, strides, box, swizzle128);
 }
 
-const CUtensorMap* get_tensor_map_3d(const void* base, Elt elt, uint64_t d0, uint64_t d1, uint64_t d2, uint64_t s1,
-                                     uint64_t s2, uint32_t b0, uint32_t b1, uint32_t b2, bool swizzle128) {
-  MapKey key{};
-  key.v[0] = reinterpret_cast<uint64_t>(base);
-  key.v[1] = static_cast<uint64_t>(elt) | (3ull << 8) | (swizzle128 ? 1ull << 16 : 0);
-  key.v[2] = d0;
-  key.v[3] = d1;
-  key.v[4] = d2;
-  key.v[5] = s1;
-  key.v[6] = s2;
-  key.v[7] = b0;
-  key.v[8] = b1;
-  key.v[9] = b2;
-  int dev = 0;
-  cudaGetDevice(&dev);
-  key.v[10] = static_cast<uint64_t>(dev);
-  uint64_t dims[3] = {d0, d1, d2};
-  uint64_t strides[2] = {s1, s2};
-  uint32_t box[3] = {b0, b1, b2};
-  return lookup_or_encode(key, base, elt, 3, dims, strides, box, swizzle128);
-}
-
-const CUtensorMap* get_tensor_map_4d(const void* base, Elt elt, const uint64_t dims[4], const uint64_t strides[3],
-                                     const uint32_t box[4], bool swizzle128) {
+TensorMap get_tensor_map_4d(const void* base, Elt elt, const uint64_t dims[4], const uint64_t strides[3],
+                            const uint32_t box[4], bool swizzle128) {
   MapKey key{};
   key.v[0] = reinterpret_cast<uint64_t>(base);
   key.v[1] = static_cast<uint64_t>(elt) | (4ull << 8) | (swizzle128 ? 1ull << 16 : 0);
@@ -182,6 +162,14 @@ int sm_count() {
 }  // namespace ctb
 
 CTB_API const char* ctb_last_error() { return ctb::g_last_error.c_str(); }
+
+// Tensor maps that are kept at most (at least one).  Returns the limit before.
+CTB_API long ctb_tensor_map_limit(long limit) {
+  std::lock_guard<std::mutex> lock(ctb::g_map_mutex);
+  const long before = static_cast<long>(ctb::g_map_limit);
+  ctb::g_map_limit = limit < 1 ? 1 : static_cast<size_t>(limit);
+  return before;
+}
 
 // Copies the device status word to `out[4]` (code, block, detail0, detail1) and clears it.
 // Synchronises the given stream first.

@@ -28,19 +28,23 @@ int fail(const std::string& msg);  // sets the message, returns a non-zero code
 
 enum class Elt : int { BF16 = 0, F32 = 1 };
 
+// A copy of an encoded tensor map.  The cache drops its own when it is full, at any later lookup of this or of another
+// thread, and a launch needs several: so it hands out no pointers.
+struct TensorMap {
+  CUtensorMap map{};
+  bool ok = false;
+  explicit operator bool() const { return ok; }
+};
+
 // Encodes (or fetches from cache) a tiled tensor map over a row-major 2-D view.
 //   inner/outer: extents in elements; row_stride: elements between rows;
 //   box_inner/box_outer: tile; swizzle128: 128-byte swizzle or none.
-// Returns nullptr and sets the error message on failure.
-const CUtensorMap* get_tensor_map_2d(const void* base, Elt elt, uint64_t inner, uint64_t outer, uint64_t row_stride,
-                                     uint32_t box_inner, uint32_t box_outer, bool swizzle128);
-// 3-D variant: dims {d0 (contiguous), d1, d2} with element strides s1, s2.
-const CUtensorMap* get_tensor_map_3d(const void* base, Elt elt, uint64_t d0, uint64_t d1, uint64_t d2, uint64_t s1,
-                                     uint64_t s2, uint32_t b0, uint32_t b1, uint32_t b2, bool swizzle128);
-
+// Not ok, with the error message set, on failure.
+TensorMap get_tensor_map_2d(const void* base, Elt elt, uint64_t inner, uint64_t outer, uint64_t row_stride,
+                            uint32_t box_inner, uint32_t box_outer, bool swizzle128);
 // 4-D variant used by attention: dims {d0 (contiguous), d1, d2, d3}, element strides s1..s3.
-const CUtensorMap* get_tensor_map_4d(const void* base, Elt elt, const uint64_t dims[4], const uint64_t strides[3],
-                                     const uint32_t box[4], bool swizzle128);
+TensorMap get_tensor_map_4d(const void* base, Elt elt, const uint64_t dims[4], const uint64_t strides[3],
+                            const uint32_t box[4], bool swizzle128);
 
 // Per-device status word in device memory (allocated on first use).
 DeviceStatus* device_status();
