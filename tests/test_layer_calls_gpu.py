@@ -77,7 +77,7 @@ def test_a_switch_turned_between_the_passes(cuda_lib):
     from causal_trainer_dev_b200.models.params import ModelParams
     from causal_trainer_dev_b200.training import engine as E
 
-    cfg = preset("qwen2.5-1.5b-image", num_hidden_layers=1, vocab_size=1000)
+    cfg = preset("qwen2.5-1.5b-image", num_hidden_layers=1, vocab_size=1000, pad_token_id=0, eos_token_id=2)
     batch = _batch(1, 384, 1000, torch.Generator(device="cuda").manual_seed(3))
     set_pair = cuda_lib.lib().ctb_gemm_set_pair
     before = set_pair(-1)
