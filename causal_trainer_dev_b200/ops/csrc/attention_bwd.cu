@@ -503,13 +503,13 @@ __device__ __forceinline__ bool bwd_compute(const BwdShared& sh, const BwdMaps& 
     const uint32_t dp_at = sh.tmem_base + T::DP + lane_off + 32 * wg;
     if (DKV) {
       // (the statistics were written by bulk copies: these waits make them visible to the thread)
-      if (!mbar_wait(&sh.y1_full[at.y1_slot], at.y1_phase, sh.abort_flag, sh.st, SITE_B_CW_S, sh.budget) ||
-          !mbar_wait(&sh.y2_full[at.y2_slot()], at.y2_phase(), sh.abort_flag, sh.st, SITE_B_CW_S, sh.budget)) {
+      if (!mbar_wait_warp(&sh.y1_full[at.y1_slot], at.y1_phase, sh.abort_flag, sh.st, SITE_B_CW_S, sh.budget) ||
+          !mbar_wait_warp(&sh.y2_full[at.y2_slot()], at.y2_phase(), sh.abort_flag, sh.st, SITE_B_CW_S, sh.budget)) {
         ok = false;
         break;
       }
     }
-    if (!mbar_wait(&sh.s_full[u], (at.s_phase >> u) & 1u, sh.abort_flag, sh.st, SITE_B_CW_S, sh.budget)) {
+    if (!mbar_wait_warp(&sh.s_full[u], (at.s_phase >> u) & 1u, sh.abort_flag, sh.st, SITE_B_CW_S, sh.budget)) {
       ok = false;
       break;
     }
@@ -564,7 +564,7 @@ __device__ __forceinline__ bool bwd_compute(const BwdShared& sh, const BwdMaps& 
     };
     if (warp_all) probabilities(std::false_type{});
     else probabilities(std::true_type{});
-    if (!mbar_wait(sh.dp_full, at.iterations & 1u, sh.abort_flag, sh.st, SITE_B_CW_S, sh.budget)) {
+    if (!mbar_wait_warp(sh.dp_full, at.iterations & 1u, sh.abort_flag, sh.st, SITE_B_CW_S, sh.budget)) {
       ok = false;
       break;
     }
@@ -613,14 +613,14 @@ __device__ __forceinline__ bool bwd_compute(const BwdShared& sh, const BwdMaps& 
   const bool writes = DKV || (u == 0);
   // ---- epilogue: accumulators -> bf16 -> staging -> TMA store ----
   if (ok && n_iter > 0) {
-    ok = mbar_wait(sh.acc_full, at.items & 1u, sh.abort_flag, sh.st, SITE_B_CW_ACC, sh.budget);
+    ok = mbar_wait_warp(sh.acc_full, at.items & 1u, sh.abort_flag, sh.st, SITE_B_CW_ACC, sh.budget);
     tc_fence_after();
   }
   // pair 0 stages in the Y1 slot, pair 1 in the Y2 slot that the producer leaves to the epilogue
   const uint32_t slot = u == 0 ? at.y1_slot : at.y2_slot();
   if (ok && writes)
-    ok = mbar_wait(u == 0 ? &sh.y1_full[slot] : &sh.y2_full[slot], u == 0 ? at.y1_phase : at.y2_phase(), sh.abort_flag, sh.st,
-                   SITE_B_CW_ACC, sh.budget);
+    ok = mbar_wait_warp(u == 0 ? &sh.y1_full[slot] : &sh.y2_full[slot], u == 0 ? at.y1_phase : at.y2_phase(), sh.abort_flag,
+                        sh.st, SITE_B_CW_ACC, sh.budget);
   const bool any_bad = named_bar_or(2 + u, 256, !ok);
   if (!any_bad && writes) {
     // DKV: warpgroup 0 stores dV, warpgroup 1 stores dK (scaled); DQ: warpgroup 0 stores dQ (scaled).
@@ -848,7 +848,13 @@ attn_bwd_kernel(const __grid_constant__ BwdMaps dkv_maps, const __grid_constant_
     }
   } else if (warp >= 4) {
     BwdWalk at;
-    while (take(w)) {
+    while (true) {
+      if (!take(w)) {
+        // no more work; or this warp gave up on an item that another warp of the pair of warpgroups has, which waits for
+        // this vote
+        named_bar_or(2 + ((warp >> 2) - 1) % 2, 256, true);
+        break;
+      }
       bool ok = true;
       if (MODES != MODE_DQ && w.mode == MODE_DKV) ok = bwd_compute<D, MODE_DKV>(sh, dkv_maps, dkv, w, at);
       else if (MODES != MODE_DKV) ok = bwd_compute<D, MODE_DQ>(sh, dq_maps, dq, w, at);
@@ -859,6 +865,7 @@ attn_bwd_kernel(const __grid_constant__ BwdMaps dkv_maps, const __grid_constant_
 
   tc_fence_before();
   __syncthreads();
+  if (*sh.abort_flag) wait_out_copies();      // (nobody sets it any more)
   if (warp == 1) {
     tc_fence_after();
     tmem_dealloc(sh.tmem_base, 512);

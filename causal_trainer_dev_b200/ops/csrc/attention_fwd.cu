@@ -409,12 +409,14 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constant
           }
         }
         for (int i = 0; ok && i < nmax; ++i) {
-          if (!mbar_wait_warp(&kv_full[slot], phase, abort_flag, st, SITE_F_MMA_KV, budget)) break;
+          ok = mbar_wait_warp(&kv_full[slot], phase, abort_flag, st, SITE_F_MMA_KV, budget);
+          if (!ok) break;
           const uint32_t vslot = slot;
           next_slot();
           const bool has_next = (i + 1 < nmax);
           if (has_next) {
-            if (!mbar_wait_warp(&kv_full[slot], phase, abort_flag, st, SITE_F_MMA_KV, budget)) break;
+            ok = mbar_wait_warp(&kv_full[slot], phase, abort_flag, st, SITE_F_MMA_KV, budget);
+            if (!ok) break;
             kslot = slot;
             next_slot();
           }
@@ -477,7 +479,12 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constant
     uint32_t sph = 0, pv = 0;              // parity of the scores, products so far
     uint32_t slot = 0;                     // KV ring
     uint32_t left = 0;                     // bit s: parity of the times that slot s was left to a tile
-    while (take()) {
+    while (true) {
+      if (!take()) {
+        // no more work; or this warp gave up on an item that another warp of the tile has, which waits for this vote
+        named_bar_or(2 + t, 128, true);
+        break;
+      }
       const int n_mine = t == 0 ? w.n[0] : w.n[1];
       const int s_mine = t == 0 ? w.s[0] : w.s[1];
       const bool tile_valid = (w.valid >> t) & 1;
@@ -512,7 +519,7 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constant
           none = !v0 && !v1;
         }
         const bool all = !none && (c_lo <= 0) && (c_hi >= 127) && v0 && v1;
-        if (!mbar_wait(&s_full[t], sph, abort_flag, st, SITE_F_SM_S, budget)) {
+        if (!mbar_wait_warp(&s_full[t], sph, abort_flag, st, SITE_F_SM_S, budget)) {      // (votes of the warp follow)
           ok = false;
           break;
         }
@@ -619,7 +626,7 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constant
       // ---- finalize ----
       if (ok && n_mine > 0) {
         pv += static_cast<uint32_t>(n_mine - s_mine);
-        ok = mbar_wait(&pv_done[t], (pv - 1u) & 1u, abort_flag, st, SITE_F_SM_PV, budget);
+        ok = mbar_wait_warp(&pv_done[t], (pv - 1u) & 1u, abort_flag, st, SITE_F_SM_PV, budget);
         tc_fence_after();
       }
       // tile t stages in the t-th of the slots that the producer leaves to O
@@ -627,7 +634,7 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constant
       const uint32_t first = (slot + static_cast<uint32_t>(2 * max(w.n[0], w.n[1]))) % KV_SLOTS;
       const uint32_t second = first + 1 < KV_SLOTS ? first + 1 : 0;
       slot = t == 0 ? first : second;
-      ok = ok && mbar_wait(&o_slot[slot], (left >> slot) & 1u, abort_flag, st, SITE_F_SM_PV, budget);
+      ok = ok && mbar_wait_warp(&o_slot[slot], (left >> slot) & 1u, abort_flag, st, SITE_F_SM_PV, budget);
       left ^= (1u << first) | (1u << second);
       uint8_t* obuf = smem + L::OFF_KV + slot * L::QT;
       const bool any_bad = named_bar_or(2 + t, 128, !ok);
@@ -678,6 +685,7 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constant
 
   tc_fence_before();
   __syncthreads();
+  if (*abort_flag) wait_out_copies();      // (nobody sets it any more)
   if (warp == 1) {
     tc_fence_after();
     tmem_dealloc(tmem_base, 512);

@@ -116,6 +116,12 @@ __device__ __forceinline__ bool mbar_wait_warp(uint64_t* bar, uint32_t parity, v
                                                DeviceStatus* st, unsigned code, long long budget = CTB_SPIN_BUDGET) {
   return __all_sync(0xffffffffu, mbar_wait(bar, parity, abort_flag, st, code, budget));
 }
+// After a wait that gave up: the time that copies of this CTA still in flight can take at the very most (1 ms).  Their
+// barriers may be among those that never completed, so there is no phase to wait for.
+__device__ __forceinline__ void wait_out_copies() {
+  const long long t0 = clock64();
+  while (clock64() - t0 < 2000000ll) __nanosleep(1000);
+}
 __device__ __forceinline__ void mbar_expect_tx_if(uint32_t on, uint64_t* bar, uint32_t bytes) {
   asm volatile(
       "{\n\t.reg .pred q;\n\tsetp.ne.b32 q, %2, 0;\n\t"
