@@ -171,28 +171,36 @@ def cut_ce_backward(hidden, head, targets, lse, coef, *, chunk_rows: int = 4096,
 KEEP_LOGITS_WIDTH = 512
 
 
+def keeps_logits(rows: int, vocab: int, width: int, chunk_rows: int) -> bool:
+    """Whether :func:`cut_ce_forward_backward` keeps the logits of a chunk (in plain, not in gathered buffers): then its slab
+    holds 4 bytes for each, otherwise 2."""
+    chunk_rows = min(chunk_rows, rows)
+    return rows > 0 and width >= KEEP_LOGITS_WIDTH and vocab % 8 == 0 and (chunk_rows == rows or chunk_rows % 32 == 0)
+
+
 def cut_ce_forward_backward(hidden, head, targets, weights, grad_scale: float | torch.Tensor = 1.0, *, chunk_rows: int = 4096,
-                            need_dhead: bool = True, dhead_out: torch.Tensor | None = None, dhead_accumulate: bool = False):
+                            need_dhead: bool = True, dhead_out: torch.Tensor | None = None, dhead_accumulate: bool = False,
+                            keep_logits: bool = True):
     """:func:`cut_ce_forward` and :func:`cut_ce_backward` in one: ``(nll_sum, weight_sum, dhidden, dhead)``, the same bits.
 
     Row chunk by row chunk, so a chunk's fp32 logits can wait for their gradient (which takes their place) instead of being
-    computed twice, where that is cheaper and there is memory for them."""
+    computed twice, where that is cheaper (:func:`keeps_logits`).  ``keep_logits=False``: the caller has no memory for them
+    (chunk_rows x vocab x 4 bytes).  Their slab is the last that is allocated: where it finds no memory, half of it has to do,
+    and while it lives nothing is allocated that could not do without."""
     rows, d = hidden.shape
     vocab = head.shape[0]
     from .gemm import in_gathered_buffer
 
     chunk_rows = min(chunk_rows, rows)
-    slab = None
-    if d >= KEEP_LOGITS_WIDTH and vocab % 8 == 0 and (chunk_rows == rows or chunk_rows % 32 == 0) and not in_gathered_buffer(hidden, head):
-        try:
-            slab = torch.empty((chunk_rows, vocab), dtype=torch.float32, device=hidden.device)
-        except torch.cuda.OutOfMemoryError:
-            slab = None
-    if slab is None:
+
+    def twice():
         nll, wsum, lse, coef = cut_ce_forward(hidden, head, targets, weights, grad_scale)
         dhidden, dhead = cut_ce_backward(hidden, head, targets, lse, coef, chunk_rows=chunk_rows, need_dhead=need_dhead,
                                          dhead_out=dhead_out, dhead_accumulate=dhead_accumulate)
         return nll, wsum, dhidden, dhead
+
+    if not keep_logits or not keeps_logits(rows, vocab, d, chunk_rows) or in_gathered_buffer(hidden, head):
+        return twice()
     dev = hidden.device
     scale_on_device = grad_scale if isinstance(grad_scale, torch.Tensor) else None
     scale = 1.0 if scale_on_device is not None else grad_scale
@@ -207,6 +215,13 @@ def cut_ce_forward_backward(hidden, head, targets, weights, grad_scale: float | 
     dhead = None
     if need_dhead:
         dhead = dhead_out if dhead_out is not None else torch.empty((vocab, d), dtype=torch.bfloat16, device=dev)
+    try:
+        slab = f32(chunk_rows, vocab)
+    except torch.cuda.OutOfMemoryError:
+        slab = None
+    if slab is None:
+        del pmax, psum, dhidden, dhead
+        return twice()
     L, ln = _lib.lib(), ctypes.c_long
     for start in range(0, rows, chunk_rows):
         n = min(chunk_rows, rows - start)

@@ -103,6 +103,9 @@ class EngineOptions:
 class LayerwiseEngine:
     """Gradient producer (see ``training.steps.GradientProducer``) running on the CUDA kernels."""
 
+    provider = None                # set by __init__
+    _room_for_logits = True        # the loss chunk may keep its fp32 logits (set with the activation policy)
+
     def __init__(self, cfg: ModelConfig, provider, options: EngineOptions | None = None):
         _lib.require_gpu_lib()
         self.cfg = cfg
@@ -363,20 +366,23 @@ class LayerwiseEngine:
             return 0
         if mode == "none":
             return cfg.num_hidden_layers
-        from .memory_plan import backward_working_set_bytes, layer_activation_bytes
+        from .memory_plan import backward_working_set_bytes, head_logit_bytes, layer_activation_bytes
 
-        per_layer = layer_activation_bytes(cfg, tokens)
-        chunk = min(self.options.cut_chunk_rows, tokens)
-        if _unused_pool_bytes() >= cfg.num_hidden_layers * per_layer + backward_working_set_bytes(cfg, tokens, chunk):
+        per_layer, chunk = layer_activation_bytes(cfg, tokens), self.options.cut_chunk_rows
+        local = type(self.provider) is LocalProvider
+        logit = head_logit_bytes(cfg, tokens, chunk) if local and self.options.loss_backend == "cut" else 2
+        self._room_for_logits = True
+        if _unused_pool_bytes() >= cfg.num_hidden_layers * per_layer + backward_working_set_bytes(cfg, tokens, min(chunk, tokens), logit):
             # the allocator holds a whole pass already, and the reserve is for what it would have to ask the driver for.
             # Asking the driver waits for its locks, on a shared host 0.8 to 9 ms (at times 90), the allocator 10 us
             return cfg.num_hidden_layers
         free, _ = torch.cuda.mem_get_info()
-        working_set = backward_working_set_bytes(cfg, tokens, self.options.cut_chunk_rows)
-        budget = free - working_set - self.options.memory_reserve_bytes
+        budget = free - backward_working_set_bytes(cfg, tokens, chunk, logit) - self.options.memory_reserve_bytes
         if budget < cfg.num_hidden_layers * per_layer:
             # what the allocator holds without using it counts too (asking takes 0.1 ms: only where it matters)
             budget += torch.cuda.memory_reserved() - torch.cuda.memory_allocated()
+        # (with nothing to spare the loss computes its logits twice, in half of the slab)
+        self._room_for_logits = budget >= 0
         return max(0, min(cfg.num_hidden_layers, int(budget // per_layer)))
 
     # ------------------------------------------------------------------ step context
@@ -482,7 +488,8 @@ class LayerwiseEngine:
         else:
             nll, wsum, dy, _ = ce.cut_ce_forward_backward(
                 y, fw["lm_head"], targets, weights, grad_scale, chunk_rows=self.options.cut_chunk_rows,
-                need_dhead=train_head, dhead_out=fg["lm_head"] if train_head else None, dhead_accumulate=accumulate)
+                need_dhead=train_head, dhead_out=fg["lm_head"] if train_head else None, dhead_accumulate=accumulate,
+                keep_logits=self._room_for_logits)
         self._count(4 + 3 * ((y.shape[0] + self.options.cut_chunk_rows - 1) // self.options.cut_chunk_rows))
         if active is not None:
             dy, y = ew.scatter_rows(dy, active, n_active_dev, full_rows), y_all     # rows without loss get zero gradient

@@ -53,9 +53,18 @@ def layer_activation_bytes(cfg: ModelConfig, tokens: int) -> int:
             + tokens * 12 * cfg.num_attention_heads)
 
 
-def backward_working_set_bytes(cfg: ModelConfig, tokens: int, cut_chunk_rows: int) -> int:
-    """Transient buffers of one layer's backward pass plus the loss chunk (bf16 logits slab)."""
-    return tokens * 2 * (6 * cfg.intermediate_size + 8 * cfg.hidden_size) + cut_chunk_rows * cfg.vocab_size * 2
+def backward_working_set_bytes(cfg: ModelConfig, tokens: int, cut_chunk_rows: int, logit_bytes: int = 2) -> int:
+    """Transient buffers of one layer's backward pass plus the loss chunk: a slab of ``logit_bytes`` a logit (2: the gradients
+    in bf16; 4: the logits kept in fp32 for them, see :func:`head_logit_bytes`)."""
+    return (tokens * 2 * (6 * cfg.intermediate_size + 8 * cfg.hidden_size)
+            + cut_chunk_rows * cfg.vocab_size * logit_bytes)
+
+
+def head_logit_bytes(cfg: ModelConfig, tokens: int, cut_chunk_rows: int) -> int:
+    """Bytes a logit that the loss chunk of a head in a plain local buffer holds."""
+    from ..ops.cross_entropy import keeps_logits
+
+    return 4 if keeps_logits(tokens, cfg.vocab_size, cfg.hidden_size, cut_chunk_rows) else 2
 
 
 def _local_config(cfg: ModelConfig, tp: int) -> ModelConfig:
@@ -93,7 +102,8 @@ def plan(cfg: ModelConfig, *, seq_len: int, micro_rows: int, lattice: Lattice = 
     tokens_full = micro_rows * seq_local                                    # all tokens of the rank's rows (its sp slice)
     tokens_rows = tokens_full // lattice.tp                                 # row-sharded over tp between projections
     per_layer = layer_activation_bytes(local, tokens_full)
-    working = backward_working_set_bytes(local, tokens_full, cut_chunk_rows)
+    working = backward_working_set_bytes(local, tokens_full, cut_chunk_rows,
+                                         2 if sharded else head_logit_bytes(local, tokens_full, cut_chunk_rows))
     out["attention_metadata"] = micro_rows * seq_len * 4 * 9 + micro_rows * (seq_len // 128) * 4 * 8
     out["rotary_table"] = 2 * micro_rows * seq_local * local.rotary_dim * 4 // 2
     if lattice.sp > 1:

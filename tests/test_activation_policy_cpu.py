@@ -1,0 +1,51 @@
+"""How many layers keep their activations: the loss chunk at its size."""
+import torch
+
+from causal_trainer_dev_b200.models.config import preset
+from causal_trainer_dev_b200.training import engine as E
+from causal_trainer_dev_b200.training.memory_plan import (Lattice, backward_working_set_bytes, head_logit_bytes,
+                                                          layer_activation_bytes, plan)
+
+TOKENS = 16384
+
+
+def _engine(cls=E.LayerwiseEngine, local=True, **options):
+    engine = cls.__new__(cls)
+    engine.cfg, engine.options = preset("llama3-8b"), E.EngineOptions(**options)
+    engine.provider = E.LocalProvider.__new__(E.LocalProvider) if local else object()
+    return engine
+
+
+def _memory(monkeypatch, free, unused=0):
+    def driver():
+        if free is None:
+            raise AssertionError("the driver was asked")
+        return free, 0
+
+    monkeypatch.setattr(torch.cuda, "mem_get_info", driver)
+    monkeypatch.setattr(torch.cuda, "memory_reserved", lambda: unused)
+    monkeypatch.setattr(torch.cuda, "memory_allocated", lambda: 0)
+    monkeypatch.setattr(E, "_unused_pool_bytes", lambda: unused)
+
+
+def test_kept_logits_take_four_bytes():
+    cfg = preset("llama3-8b")
+    assert head_logit_bytes(cfg, TOKENS, 4096) == 4 and head_logit_bytes(preset("tiny"), 512, 4096) == 2
+    assert head_logit_bytes(cfg, TOKENS, 100) == 2 and head_logit_bytes(cfg, 100, 4096) == 4       # chunks of whole blocks
+    two, four = (backward_working_set_bytes(cfg, TOKENS, 4096, n) for n in (2, 4))
+    assert four - two == 4096 * 128256 * 2
+    alone = plan(cfg, seq_len=4096, micro_rows=4)
+    assert alone["backward_working_set"] == four
+    assert plan(cfg, seq_len=4096, micro_rows=4, lattice=Lattice(2))["backward_working_set"] == two    # a gathered head
+
+
+def test_policy_counts_the_slab_that_the_loss_allocates(monkeypatch):
+    cfg = preset("llama3-8b")
+    per_layer = layer_activation_bytes(cfg, TOKENS)
+    for engine, logit in ((_engine(), 4), (_engine(local=False), 2), (_engine(loss_backend="logits"), 2)):
+        working = backward_working_set_bytes(cfg, TOKENS, 4096, logit)
+        for spare in (0, per_layer - 1):
+            _memory(monkeypatch, working + engine.options.memory_reserve_bytes + 5 * per_layer + spare)
+            assert engine._layers_to_keep(TOKENS) == 5 and engine._room_for_logits
+        _memory(monkeypatch, working + engine.options.memory_reserve_bytes - 1)
+        assert engine._layers_to_keep(TOKENS) == 0 and not engine._room_for_logits

@@ -37,3 +37,30 @@ def test_a_vocabulary_that_the_two_refuse(cuda_lib):
     hidden, head = (torch.zeros(n, 1024, dtype=torch.bfloat16, device="cuda") for n in (64, 1001))
     with pytest.raises(cuda_lib.KernelError, match="16 bytes"):
         ce.cut_ce_forward_backward(hidden, head, torch.zeros(64, dtype=torch.long, device="cuda"), torch.ones(64, device="cuda"))
+
+
+@pytest.mark.parametrize("how", ["no memory", "not wanted"])
+def test_without_memory_for_the_logits(cuda_lib, monkeypatch, how):
+    """The slab that is refused, or not asked for: the two calls, and no slab of four bytes a logit."""
+    from causal_trainer_dev_b200.ops import cross_entropy as ce
+
+    gen = torch.Generator(device="cuda").manual_seed(1)
+    hidden = torch.randn(300, 1024, generator=gen, device="cuda").bfloat16()
+    head = (torch.randn(4104, 1024, generator=gen, device="cuda") * 0.05).bfloat16()
+    targets = torch.randint(0, 4104, (300,), generator=gen, device="cuda")
+    weights = torch.ones(300, device="cuda")
+    want = ce.cut_ce_forward_backward(hidden, head, targets, weights, 1e-2, chunk_rows=128)
+    empty, asked = torch.empty, []
+
+    def refuse(*args, **kw):
+        shape = args[0] if len(args) == 1 and not isinstance(args[0], int) else args
+        if tuple(shape) == (128, 4104) and kw.get("dtype") == torch.float32:
+            asked.append(shape)
+            raise torch.cuda.OutOfMemoryError("refused by the test")
+        return empty(*args, **kw)
+
+    monkeypatch.setattr(torch, "empty", refuse)
+    got = ce.cut_ce_forward_backward(hidden, head, targets, weights, 1e-2, chunk_rows=128, keep_logits=how == "no memory")
+    assert len(asked) == (how == "no memory")
+    assert all(torch.equal(a, b) for a, b in zip(got, want))
+    assert cuda_lib.device_status() == (0, 0, 0, 0)
