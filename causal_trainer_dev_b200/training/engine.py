@@ -43,9 +43,11 @@ LAYER_CALL_BYTES = 64 << 20
 
 
 def _unused_pool_bytes() -> int:
-    """Bytes that PyTorch's allocator has from the driver and that no tensor uses (0 before its first use)."""
+    """Bytes that PyTorch's allocator has from the driver in segments that no tensor lies in, and so could give back (0 before
+    its first use): what is left beside the tensors of a segment may be in pieces too small for anything."""
     stats = torch.cuda.memory_stats_as_nested_dict()
-    return stats["reserved_bytes"]["all"]["current"] - stats["allocated_bytes"]["all"]["current"] if stats else 0
+    now = lambda key: stats[key]["all"]["current"]  # noqa: E731
+    return now("reserved_bytes") - now("allocated_bytes") - now("inactive_split_bytes") if stats else 0
 
 
 class LocalProvider:
@@ -372,9 +374,11 @@ class LayerwiseEngine:
         local = type(self.provider) is LocalProvider
         logit = head_logit_bytes(cfg, tokens, chunk) if local and self.options.loss_backend == "cut" else 2
         self._room_for_logits = True
-        if _unused_pool_bytes() >= cfg.num_hidden_layers * per_layer + backward_working_set_bytes(cfg, tokens, min(chunk, tokens), logit):
-            # the allocator holds a whole pass already, and the reserve is for what it would have to ask the driver for.
-            # Asking the driver waits for its locks, on a shared host 0.8 to 9 ms (at times 90), the allocator 10 us
+        if (local and type(self) is LayerwiseEngine and _unused_pool_bytes() >= cfg.num_hidden_layers * per_layer
+                + backward_working_set_bytes(cfg, tokens, min(chunk, tokens), logit)):
+            # the allocator could give back a whole pass already, so this one takes nothing more from the driver, which is what
+            # the reserve is for.  Asking the driver waits for its locks, on a shared host 0.8 to 9 ms (at times 90), the
+            # allocator 10 us.  (One replica only: ranks that share layers take the same decision, below.)
             return cfg.num_hidden_layers
         free, _ = torch.cuda.mem_get_info()
         budget = free - backward_working_set_bytes(cfg, tokens, chunk, logit) - self.options.memory_reserve_bytes

@@ -1,4 +1,5 @@
-"""How many layers keep their activations: the loss chunk at its size."""
+"""How many layers keep their activations: the loss chunk at its size, the allocator's own memory."""
+import pytest
 import torch
 
 from causal_trainer_dev_b200.models.config import preset
@@ -49,3 +50,35 @@ def test_policy_counts_the_slab_that_the_loss_allocates(monkeypatch):
             assert engine._layers_to_keep(TOKENS) == 5 and engine._room_for_logits
         _memory(monkeypatch, working + engine.options.memory_reserve_bytes - 1)
         assert engine._layers_to_keep(TOKENS) == 0 and not engine._room_for_logits
+
+
+def test_a_whole_pass_in_the_allocator_needs_no_question(monkeypatch):
+    cfg = preset("llama3-8b")
+    need = cfg.num_hidden_layers * layer_activation_bytes(cfg, TOKENS) + backward_working_set_bytes(cfg, TOKENS, 4096, 4)
+    _memory(monkeypatch, None, need)
+    engine = _engine()
+    engine._room_for_logits = False
+    assert engine._layers_to_keep(TOKENS) == cfg.num_hidden_layers and engine._room_for_logits
+    _memory(monkeypatch, 0, need - 1)                       # less: the reserve counts
+    assert 0 < engine._layers_to_keep(TOKENS) < cfg.num_hidden_layers
+
+
+@pytest.mark.parametrize("which", ["provider", "subclass"])
+def test_only_one_replica_answers_from_the_allocator_alone(monkeypatch, which):
+    class Other(E.LayerwiseEngine):
+        pass
+
+    cfg = preset("llama3-8b")
+    need = cfg.num_hidden_layers * layer_activation_bytes(cfg, TOKENS) + backward_working_set_bytes(cfg, TOKENS, 4096, 4)
+    _memory(monkeypatch, 0, need)
+    engine = _engine(local=False) if which == "provider" else _engine(Other)
+    assert engine._layers_to_keep(TOKENS) < cfg.num_hidden_layers
+
+
+def test_pieces_of_segments_in_use_do_not_count(monkeypatch):
+    current = lambda n: {"all": {"current": n}}  # noqa: E731
+    stats = dict(reserved_bytes=current(1000), allocated_bytes=current(300), inactive_split_bytes=current(450))
+    monkeypatch.setattr(torch.cuda, "memory_stats_as_nested_dict", lambda: stats)
+    assert E._unused_pool_bytes() == 250
+    monkeypatch.setattr(torch.cuda, "memory_stats_as_nested_dict", dict)
+    assert E._unused_pool_bytes() == 0
