@@ -387,7 +387,27 @@ class LayerwiseEngine:
             budget += torch.cuda.memory_reserved() - torch.cuda.memory_allocated()
         # (with nothing to spare the loss computes its logits twice, in half of the slab)
         self._room_for_logits = budget >= 0
-        return max(0, min(cfg.num_hidden_layers, int(budget // per_layer)))
+        return self._least(max(0, min(cfg.num_hidden_layers, int(budget // per_layer))))
+
+    def _recompute_groups(self) -> tuple:
+        """Process groups whose ranks take part in the recomputation of a layer."""
+        # (a rebuilt group of layers gathers weights that are gathered again afterwards; our own pull kernels take no
+        # part of the other ranks, an NCCL all-gather does)
+        sharded = self.options.remat_group_size > 1 and not getattr(self.provider, "fused", True)
+        return (self.provider.group,) if sharded else ()
+
+    def _least(self, count: int) -> int:
+        """The smallest count of the ranks that recompute together: each sees its own free memory, and ranks that recomputed
+        different layers would wait for one another in different collectives.  Reading it back waits for this rank's stream."""
+        import torch.distributed as dist
+
+        for group in self._recompute_groups():
+            if dist.get_world_size(group) > 1:
+                gloo = dist.get_backend(group) == "gloo"
+                least = torch.tensor([count], device="cpu" if gloo else torch.device("cuda", torch.cuda.current_device()))
+                dist.all_reduce(least, op=dist.ReduceOp.MIN, group=group)
+                count = int(least)
+        return count
 
     # ------------------------------------------------------------------ step context
     def _context(self, batch: dict[str, torch.Tensor]) -> dict:

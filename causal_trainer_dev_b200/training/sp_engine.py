@@ -117,6 +117,9 @@ class SequenceParallelAttention:
         ctx.update(seq=n, seq_full=s, q_ranges=self.token_ranges(s))
         return ctx
 
+    def _recompute_groups(self) -> tuple:
+        return (*super()._recompute_groups(), self.sp_group)
+
     def _uses_moba(self, li: int, seq: int, longest: int | None = None) -> bool:
         return False
 

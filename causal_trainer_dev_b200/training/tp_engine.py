@@ -68,6 +68,9 @@ class TpLayerwiseEngine(LayerwiseEngine):
         # `tokens` counts this rank's rows; the kept tensors are mostly full-row, local-width
         return super()._layers_to_keep(tokens * self.tp_world)
 
+    def _recompute_groups(self) -> tuple:
+        return (*super()._recompute_groups(), self.tp_group)
+
     # ------------------------------------------------------------------ layer forward
     def _layer_forward(self, w, resid, branch, ctx, li, save):
         cfg = self.cfg

@@ -1,4 +1,10 @@
-"""How many layers keep their activations: the loss chunk at its size, the allocator's own memory."""
+"""How many layers keep their activations: the loss chunk at its size, the allocator's own memory, and one answer for the ranks
+that recompute together."""
+import os
+import subprocess
+import sys
+from pathlib import Path
+
 import pytest
 import torch
 
@@ -7,6 +13,7 @@ from causal_trainer_dev_b200.training import engine as E
 from causal_trainer_dev_b200.training.memory_plan import (Lattice, backward_working_set_bytes, head_logit_bytes,
                                                           layer_activation_bytes, plan)
 
+ROOT = Path(__file__).resolve().parents[1]
 TOKENS = 16384
 
 
@@ -82,3 +89,53 @@ def test_pieces_of_segments_in_use_do_not_count(monkeypatch):
     assert E._unused_pool_bytes() == 250
     monkeypatch.setattr(torch.cuda, "memory_stats_as_nested_dict", dict)
     assert E._unused_pool_bytes() == 0
+
+
+WORKER = r'''
+import sys
+import torch
+import torch.distributed as dist
+sys.path.insert(0, sys.argv[1])
+from causal_trainer_dev_b200.models.config import preset
+from causal_trainer_dev_b200.training import engine as E
+from causal_trainer_dev_b200.training.memory_plan import backward_working_set_bytes, layer_activation_bytes
+from causal_trainer_dev_b200.training.sp_engine import SpLayerwiseEngine
+from causal_trainer_dev_b200.training.tp_engine import TpLayerwiseEngine
+
+dist.init_process_group("gloo")
+rank, group = dist.get_rank(), dist.group.WORLD
+cfg = preset("llama3-8b")
+
+
+class Sharded:
+    fused, group = False, group
+
+
+for cls, options in ((TpLayerwiseEngine, {}), (SpLayerwiseEngine, {}), (E.LayerwiseEngine, dict(remat_group_size=2))):
+    engine = cls.__new__(cls)
+    engine.cfg, engine.options, engine.provider = cfg, E.EngineOptions(**options), Sharded()
+    engine.tp_group = engine.sp_group = group
+    engine.tp_world = 1
+    tokens = 16384
+    per_layer = layer_activation_bytes(cfg, tokens)
+    base = backward_working_set_bytes(cfg, tokens, 4096) + engine.options.memory_reserve_bytes + per_layer // 2
+    torch.cuda.mem_get_info = lambda: (base + (7 + 3 * rank) * per_layer, 0)      # this rank alone: 7 or 10 layers
+    torch.cuda.memory_reserved = torch.cuda.memory_allocated = lambda: 0
+    assert engine._layers_to_keep(tokens) == 7, (cls, rank)
+    engine.options.remat = "none"
+    assert engine._layers_to_keep(tokens) == cfg.num_hidden_layers
+engine.options.remat, engine.options.remat_group_size = "auto", 1
+assert engine._layers_to_keep(tokens) == 7 + 3 * rank                             # nothing is recomputed together
+print("DONE", rank)
+dist.destroy_process_group()
+'''
+
+
+def test_ranks_that_recompute_together_keep_the_same_layers(tmp_path):
+    script = tmp_path / "worker.py"
+    script.write_text(WORKER)
+    env = {**os.environ, "OMP_NUM_THREADS": "1", "CUDA_VISIBLE_DEVICES": ""}
+    out = subprocess.run([sys.executable, "-m", "torch.distributed.run", "--standalone", "--local-addr", "127.0.0.1",
+                          "--nproc-per-node", "2", str(script), str(ROOT)], capture_output=True, text=True, env=env, timeout=300)
+    assert out.returncode == 0, out.stdout + out.stderr
+    assert out.stdout.count("DONE") == 2
