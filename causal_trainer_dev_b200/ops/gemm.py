@@ -148,7 +148,12 @@ def gemm(
     f32 = out.dtype == torch.float32
     L = _lib.lib()
     size = 0 if max_ctas > 0 else L.ctb_gemm_workspace(m, n, k, bool(a_mn), f32, bool(accumulate))
-    work = torch.empty(size, dtype=torch.uint8, device=a.device) if size else None
+    work = None
+    if size:
+        try:
+            work = torch.empty(size, dtype=torch.uint8, device=a.device)
+        except torch.cuda.OutOfMemoryError:
+            size = 0                              # the product takes a kernel that needs none
     code = L.ctb_gemm(
         a.data_ptr(), b.data_ptr(), out.data_ptr(), m, n, k, a.stride(0), b.stride(0), out.stride(0),
         bool(a_mn), bool(b_mn), f32, bool(accumulate), float(alpha), None if bias is None else bias.data_ptr(), max_ctas,
