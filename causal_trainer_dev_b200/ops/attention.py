@@ -204,12 +204,12 @@ def flash_attention_forward(
               _at(meta.start), meta.kv_lo.data_ptr(), meta.kv_hi.data_ptr(), b, s, sq, q_offset, hq, hkv, d,
               _row_stride(q), _row_stride(k), _row_stride(v), _row_stride(out), float(scale))
     if kv_flags is None:
-        code = _lib.lib().ctb_attn_fwd_range(*common, spin_budget, _lib.raw_stream())
+        code = _lib.lib().ctb_attn_fwd_range(*common, int(spin_budget), _lib.raw_stream())
         _lib.check(code, "ctb_attn_fwd_range")
     else:
         flags, chunk, row_elems, epoch = kv_flags
-        code = _lib.lib().ctb_attn_fwd_gathered(*common, flags.data_ptr(), chunk, row_elems, epoch, spin_budget,
-                                                _lib.raw_stream())
+        code = _lib.lib().ctb_attn_fwd_gathered(*common, flags.data_ptr(), int(chunk), int(row_elems), int(epoch),
+                                                int(spin_budget), _lib.raw_stream())
         _lib.check(code, "ctb_attn_fwd_gathered")
     return out, lse
 
@@ -223,7 +223,8 @@ def flash_attention_backward(
     """dQ (query-tile-owned work items) and dK/dV (key-tile-owned ones, group reduced in TMEM), in one launch.
 
     With a query range (``q_offset``, ``Sq < S``) dK / dV are this rank's partial sums over its
-    queries, for all ``S`` keys.
+    queries, for all ``S`` keys.  ``stats`` are used in the place of ``lse``.  ``dq`` may take the place of ``q`` or ``dout``
+    (then dK / dV are a launch of their own, before it); no other output may share memory with an input but ``out``.
     """
     b, sq, hq, d = q.shape
     s = k.shape[1]
@@ -241,12 +242,13 @@ def flash_attention_backward(
     dk = torch.empty((b, s, hkv, d), dtype=torch.bfloat16, device=q.device) if dk is None else dk
     dv = torch.empty((b, s, hkv, d), dtype=torch.bfloat16, device=q.device) if dv is None else dv
     code = _lib.lib().ctb_attn_bwd_range(
-        q.data_ptr(), k.data_ptr(), v.data_ptr(), out.data_ptr() if stats is None else None, dout.data_ptr(), lse.data_ptr(),
+        q.data_ptr(), k.data_ptr(), v.data_ptr(), out.data_ptr() if stats is None else None, dout.data_ptr(),
+        lse.data_ptr() if stats is None else None,
         dq.data_ptr(), dk.data_ptr(), dv.data_ptr(), neg_lse2, neg_delta, meta.seg.data_ptr(),
         _at(meta.lim), meta.kv_lo.data_ptr(), meta.kv_hi.data_ptr(), meta.q_lo.data_ptr(), meta.q_hi.data_ptr(),
         _at(meta.start), _at(meta.end), _at(meta.first_q), b, s, sq, q_offset, hq, hkv, d, _row_stride(q), _row_stride(k),
-        _row_stride(v), out_stride, dout_stride, _row_stride(dq), _row_stride(dk), _row_stride(dv), float(scale), spin_budget,
-        _lib.raw_stream())
+        _row_stride(v), out_stride, dout_stride, _row_stride(dq), _row_stride(dk), _row_stride(dv), float(scale),
+        int(spin_budget), _lib.raw_stream())
     _lib.check(code, "ctb_attn_bwd_range", 1 if stats is not None else 2)
     return dq, dk, dv
 

@@ -134,7 +134,7 @@ struct BwdCall {
   const int* seg; const int* lim; const int* kv_lo; const int* kv_hi; const int* q_lo; const int* q_hi;
   const int* run_start; const int* run_end; const int* first_q;
   int B, S, Hq, Hkv;
-  int Sq = 0, q_off = 0;
+  int Sq = 0, q_off = 0, D = 0;
   long q_row_stride, k_row_stride, v_row_stride, do_row_stride, dq_row_stride, dk_row_stride, dv_row_stride;
   float scale;
   long long spin_budget;

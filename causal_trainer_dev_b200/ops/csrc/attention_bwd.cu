@@ -957,6 +957,29 @@ int launch_bwd_both(const BwdCall& dkv, const BwdCall& dq) {
   return launch_items<D, MODE_BOTH>(dkv_maps, dq_maps, dkv_args, dq_args, dkv_items, dq_items, dkv.stream);
 }
 
+// Whether dQ shares memory with what the dK / dV items read of the queries (whole ranges: strided views that interleave
+// count as sharing).
+inline bool dq_over_inputs(const BwdCall& c) {
+  const long rows = static_cast<long>(c.B) * c.Sq, width = static_cast<long>(c.Hq) * c.D;
+  auto range = [&](const void* p, long row_stride, uintptr_t* from) {
+    *from = reinterpret_cast<uintptr_t>(p);
+    return *from + 2 * static_cast<uintptr_t>((rows - 1) * row_stride + width);
+  };
+  uintptr_t dq, q, dout;
+  const uintptr_t dq_end = range(c.dq, c.dq_row_stride, &dq), q_end = range(c.q, c.q_row_stride, &q),
+                  dout_end = range(c.dout, c.do_row_stride, &dout);
+  return (dq < q_end && q < dq_end) || (dq < dout_end && dout < dq_end);
+}
+
+// dQ in the place of Q or dO: a dQ item replaces rows that no other dQ item reads, but dK / dV items do, so these come
+// first, in a launch of their own.
+template <int D>
+int launch_bwd_dense(const BwdCall& c) {
+  if (!dq_over_inputs(c)) return launch_bwd_both<D>(c, c);
+  const int rc = launch_bwd<D, MODE_DKV>(c);
+  return rc != 0 ? rc : launch_bwd<D, MODE_DQ>(c);
+}
+
 }  // namespace attn
 }  // namespace ctb
 
@@ -982,11 +1005,11 @@ CTB_API int ctb_attn_bwd_range(const void* q, const void* k, const void* v, cons
   c.q = q; c.k = k; c.v = v; c.dout = dout; c.dq = dq; c.dk = dk; c.dv = dv; c.neg_lse2 = neg_lse2; c.neg_delta = neg_delta;
   c.seg = seg; c.lim = lim; c.kv_lo = kv_lo; c.kv_hi = kv_hi; c.q_lo = q_lo; c.q_hi = q_hi;
   c.run_start = run_start; c.run_end = run_end; c.first_q = first_q;
-  c.B = B; c.S = S; c.Sq = Sq; c.q_off = q_off; c.Hq = Hq; c.Hkv = Hkv;
+  c.B = B; c.S = S; c.Sq = Sq; c.q_off = q_off; c.Hq = Hq; c.Hkv = Hkv; c.D = D;
   c.q_row_stride = q_rs; c.k_row_stride = k_rs; c.v_row_stride = v_rs; c.do_row_stride = do_rs;
   c.dq_row_stride = dq_rs; c.dk_row_stride = dk_rs; c.dv_row_stride = dv_rs;
   c.scale = scale; c.spin_budget = spin_budget; c.stream = stream;
-  return D == 128 ? ctb::attn::launch_bwd_both<128>(c, c) : ctb::attn::launch_bwd_both<64>(c, c);
+  return D == 128 ? ctb::attn::launch_bwd_dense<128>(c) : ctb::attn::launch_bwd_dense<64>(c);
 }
 
 // Block-sparse (MoBA) backward: `it_off` has one entry per CTA plus one, in grid order
