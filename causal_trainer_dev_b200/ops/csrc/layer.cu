@@ -43,7 +43,7 @@ struct Context {
   const int *seg, *lim, *start, *end, *first_q, *kv_lo, *kv_hi, *q_lo, *q_hi;
 };
 struct Weights {
-  const char *ln1, *ln2, *qkv_w, *qkv_b, *o_w, *o_b, *gu_w, *gu_b, *down_w, *down_b;
+  const char *ln1, *ln2, *qkv_w, *qkv_b, *o_w, *gu_w, *down_w;      // (qkv_b may be null)
 };
 
 // A block that is cut into pieces; `size` is what the caller holds (0 while the pieces are only counted).
@@ -204,11 +204,11 @@ CTB_API int ctb_layer_forward(const ctb::layer::Shape* sp, const ctb::layer::Con
   CTB_TRY(ctb_attn_fwd_range(k.qkv, k.qkv + z.qw, k.qkv + z.qw + z.kvw, k.o, k.lse, cx->seg, cx->lim, cx->start, cx->kv_lo,
                              cx->kv_hi, s.batch, s.seq, s.seq, 0, s.q_heads, s.kv_heads, s.head_dim, z.w, z.w, z.w, z.qw, s.scale,
                              0, stream));
-  CTB_TRY(project(k.o, w->o_w, w->o_b, f.branch, z.t, z.qw, s.hidden, f.work, f.work_bytes, stream));
+  CTB_TRY(project(k.o, w->o_w, nullptr, f.branch, z.t, z.qw, s.hidden, f.work, f.work_bytes, stream));
   CTB_TRY(ctb_rmsnorm_fwd(x, f.branch, w->ln2, f.normed, h, k.rstd2, t, s.hidden, s.eps, stream));
-  CTB_TRY(project(f.normed, w->gu_w, w->gu_b, k.gu, z.t, s.hidden, 2l * s.inner, f.work, f.work_bytes, stream));
+  CTB_TRY(project(f.normed, w->gu_w, nullptr, k.gu, z.t, s.hidden, 2l * s.inner, f.work, f.work_bytes, stream));
   CTB_TRY(ctb_swiglu_fwd(k.gu, f.act, z.t, s.inner, stream));
-  return project(f.act, w->down_w, w->down_b, mlp, z.t, s.inner, s.hidden, f.work, f.work_bytes, stream);
+  return project(f.act, w->down_w, nullptr, mlp, z.t, s.inner, s.hidden, f.work, f.work_bytes, stream);
 }
 
 // Gradient dx of the layer's input from the gradient dout of its output h + mlp; the weight gradients go where `g` says (null:

@@ -27,7 +27,17 @@ class _Context(ctypes.Structure):
 
 
 class _Weights(ctypes.Structure):
-    _fields_ = [(n, _P) for n in ("ln1", "ln2", "qkv_w", "qkv_b", "o_w", "o_b", "gu_w", "gu_b", "down_w", "down_b")]
+    _fields_ = [(n, _P) for n in ("ln1", "ln2", "qkv_w", "qkv_b", "o_w", "gu_w", "down_w")]
+
+
+_SEGMENTS = {name for name, _ in _Weights._fields_}
+
+
+def takes(layout) -> bool:
+    """Whether the library's layer has all that a unit of this layout has, and trains it: the schedule in ``csrc/layer.cu`` is
+    written for these segments (``qkv_b`` may be missing)."""
+    names = {seg.name for seg in layout.segments}
+    return names <= _SEGMENTS and names | {"qkv_b"} == _SEGMENTS
 
 
 def _plan(batch: int, seq: int, hidden: int, q_heads: int, kv_heads: int, head_dim: int, inner: int, rotary_dim: int,

@@ -292,8 +292,10 @@ class LayerwiseEngine:
         o, prov = self.options, self.provider
         if (type(self) is not LayerwiseEngine or type(prov) is not LocalProvider or not self.train_base
                 or o.attention_options is not None or o.mlp_chunk_rows > 0 or self._wgrad_stream is not None
-                or gemm_ops._FLAG_SOURCES or resid.dtype != torch.bfloat16
-                or any(prov.params.units[f"layer.{i}"].data.dtype != torch.bfloat16 for i in range(self.cfg.num_hidden_layers))):
+                or gemm_ops._FLAG_SOURCES or resid.dtype != torch.bfloat16):
+            return None
+        units = [prov.params.units[f"layer.{i}"] for i in range(self.cfg.num_hidden_layers)]
+        if any(u.data.dtype != torch.bfloat16 or not layer_ops.takes(u.layout) for u in units):
             return None
         calls = layer_ops.LayerCalls(self.cfg, ctx, prov.grad_dtype, o.train_norm)
         return calls if calls.scratch_bytes <= LAYER_CALL_BYTES else None

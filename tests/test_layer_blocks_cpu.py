@@ -47,3 +47,15 @@ def test_a_block_that_is_too_small_is_refused(pair_switch, kept_short, scratch_s
                                 low(backward, scratch_short), at, None) == 1
     assert "too small" in L.ctb_last_error().decode()
     assert L.ctb_layer_forward(ctypes.byref(shape), c, w, at, None, None, 0, at, forward, at, at, None) == 1
+
+
+def test_only_the_segments_that_the_library_trains():
+    from causal_trainer_dev_b200.models import params
+    from causal_trainer_dev_b200.models.config import preset
+
+    for bias in (False, True):
+        assert layer.takes(params.layer_layout(preset("tiny", attention_bias=bias), 0))
+    entries = [("ln1", (64,)), ("ln2", (64,)), ("qkv_w", (192, 64)), ("o_w", (64, 64)), ("gu_w", (256, 64)), ("down_w", (64, 128))]
+    assert layer.takes(params._layout("layer.0", entries))
+    assert not layer.takes(params._layout("layer.0", [*entries, ("o_b", (64,))]))       # a bias that it would leave out
+    assert not layer.takes(params._layout("layer.0", entries[1:]))
