@@ -666,6 +666,18 @@ CTB_API int ctb_gemm_pair_choice(int M, int N, int K, int out_f32, int accumulat
   return 1;
 }
 
+// The same for the products of the loss: the statistics of the logits (kept or not), or with `gradients` their gradients.
+CTB_API int ctb_ce_pair_choice(int rows, int vocab, int d, int gradients, int* form) {
+  ctb::GemmCall c{};
+  c.M = rows; c.N = vocab; c.K = d;
+  c.epi = gradients ? ctb::EPI_CE_DLOGITS : ctb::EPI_CE_STATS;
+  c.out_f32 = gradients ? 0 : 1;
+  ctb::PairPlan p;
+  if (!ctb::gemm_pair_plan(c, &p)) return 0;
+  form[0] = p.tm; form[1] = p.whole; form[2] = p.slices; form[3] = p.band;
+  return 1;
+}
+
 // The two-CTA kernel with a given plan, whatever the choice by size would be: for tests of every form that the plan may
 // choose and for measurements of it.
 CTB_API int ctb_gemm_pair(const void* A, const void* B, void* C, int M, int N, int K, long lda, long ldb, long ldc,

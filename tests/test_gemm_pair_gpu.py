@@ -66,10 +66,17 @@ def test_every_form(cuda_lib, tm, m, n, k, whole, slices, band, a_mn, b_mn):
     assert cuda_lib.device_status() == (0, 0, 0, 0)
 
 
-@pytest.mark.parametrize("rows,vocab,d", [(1000, 32000, 1536), (300, 20000, 520), (4000, 5000, 256)])
-def test_loss_epilogues_on_two_ctas(cuda_lib, rows, vocab, d):
+@pytest.mark.parametrize("rows,vocab,d,tm", [
+    (1000, 32000, 1536, 1), (4000, 5000, 256, 1), (1, 4912, 720, 1),
+    (516, 7976, 400, 2), (894, 7376, 896, 2), (452, 12400, 1328, 2), (1052, 4256, 408, 2), (2184, 2120, 400, 2),
+    (300, 20000, 520, None)])                     # None: the one-CTA kernel by size, too
+def test_loss_epilogues_on_two_ctas(cuda_lib, rows, vocab, d, tm):
     from causal_trainer_dev_b200.ops import cross_entropy as ce
 
+    form = (ctypes.c_int * 4)()
+    for gradients in (0, 1):
+        taken = cuda_lib.lib().ctb_ce_pair_choice(rows, vocab, d, gradients, form)
+        assert (form[0] if taken else None) == tm
     hidden, head = _bf16(rows, d, seed=1), _bf16(vocab, d, seed=2, scale=0.05)
     gen = torch.Generator(device="cuda").manual_seed(3)
     targets = torch.randint(0, vocab, (rows,), generator=gen, device="cuda")

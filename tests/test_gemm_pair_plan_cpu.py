@@ -53,6 +53,22 @@ def test_the_choice_does_not_depend_on_the_calls_before_it():
     assert forward[0] is not None and forward[1] is not None and forward[2] is None
 
 
+def test_the_loss_products_choose_whole_tiles():
+    """Their epilogues see whole logits: no K slices.  Both tile heights occur."""
+    lib = ctypes.CDLL(str(LIB_PATH))
+    rng, form, seen = random.Random(2), (ctypes.c_int * 4)(), set()
+    for _ in range(3000):
+        rows, vocab, d = rng.randint(1, 4096), 8 * rng.randint(100, 16000), 8 * rng.randint(16, 512)
+        for gradients in (0, 1):
+            if lib.ctb_ce_pair_choice(rows, vocab, d, gradients, form):
+                tm, whole, slices, band = form
+                assert whole == -(-rows // (256 * tm)) * -(-vocab // 256) and slices == 1 and band >= 1
+                seen.add((gradients, tm))
+            else:
+                seen.add((gradients, None))
+    assert seen == {(g, tm) for g in (0, 1) for tm in (1, 2, None)}
+
+
 def test_the_mode_switch_turns_the_choice_off_and_on():
     lib = ctypes.CDLL(str(LIB_PATH))
     before = lib.ctb_gemm_set_pair(0)

@@ -39,11 +39,16 @@ def test_warps_without_rows_leave_the_staging_alone(cuda_lib, one_cta, m, k, dty
     assert cuda_lib.device_status() == (0, 0, 0, 0)
 
 
-@pytest.mark.parametrize("rows,vocab,d", [(333, 32000, 64), (33, 64008, 512), (200, 40000, 128), (1100, 32000, 512)])
-def test_kept_logits_and_their_gradients(cuda_lib, rows, vocab, d):
+@pytest.mark.parametrize("rows,vocab,d,tm", [
+    (333, 32000, 64, None), (33, 64008, 512, None), (200, 40000, 128, None),                     # one CTA
+    (1100, 32000, 512, 1), (4000, 5000, 256, 1), (516, 7976, 400, 2), (1052, 4256, 408, 2)])     # two, 256 or 512 rows
+def test_kept_logits_and_their_gradients(cuda_lib, rows, vocab, d, tm):
     """The loss epilogues, on the kernel that the sizes choose."""
     import ctypes
 
+    form = (ctypes.c_int * 4)()
+    for gradients in (0, 1):
+        assert (form[0] if cuda_lib.lib().ctb_ce_pair_choice(rows, vocab, d, gradients, form) else None) == tm
     gen = torch.Generator(device="cuda").manual_seed(rows)
     hidden = torch.randn(rows, d, generator=gen, device="cuda").bfloat16()
     head = (torch.randn(vocab, d, generator=gen, device="cuda") * 0.05).bfloat16()

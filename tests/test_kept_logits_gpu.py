@@ -7,7 +7,8 @@ pytestmark = pytest.mark.gpu
 
 
 @pytest.mark.parametrize("rows,vocab,d,chunk", [(1, 8, 1024, 4096), (333, 4104, 1024, 128), (700, 2048, 1032, 256), (260, 2056, 1024, 4096),
-                                                (600, 20008, 1536, 512), (129, 4104, 512, 64), (129, 4104, 504, 64)])
+                                                (600, 20008, 1536, 512), (129, 4104, 512, 64), (129, 4104, 504, 64),
+                                                (894, 7376, 896, 4096), (904, 12400, 1328, 452)])      # two CTAs, 512 rows
 @pytest.mark.parametrize("on_device,accumulate", [(False, False), (True, True)])
 def test_one_call_is_the_two(cuda_lib, rows, vocab, d, chunk, on_device, accumulate):
     from causal_trainer_dev_b200.ops import cross_entropy as ce
