@@ -63,7 +63,7 @@ template <int D>
 struct FwdSmem {
   static constexpr int HALVES = D / 64;
   static constexpr int QT = HALVES * 16384;        // one 128-row Q / K / V tile
-  static constexpr int OFF_Q = 0;                  // two Q tiles; each doubles as the staging tile of its O
+  static constexpr int OFF_Q = 0;                  // two Q tiles (O is staged in slots of the K / V ring)
   static constexpr int OFF_KV = 2 * QT;
   static constexpr int OFF_BAR = OFF_KV + KV_SLOTS * QT;
   static constexpr int OFF_ITEMS = OFF_BAR + 320;  // answer of the work request, two work items
@@ -749,26 +749,9 @@ int launch_fwd(const FwdCall& c) {
 }  // namespace attn
 }  // namespace ctb
 
-// q/k/v/o are [B, S, H, D] views with arbitrary row stride (elements between consecutive
-// tokens), so the packed QKV projection output is read in place.  lse is [B, Hq, S] fp32.
-CTB_API int ctb_attn_fwd(const void* q, const void* k, const void* v, void* o, float* lse, const int* seg,
-                         const int* lim, const int* row_start, const int* kv_lo, const int* kv_hi, int B,
-                         int S, int Hq, int Hkv, int D, long q_row_stride, long k_row_stride, long v_row_stride,
-                         long o_row_stride, float scale, long long spin_budget, void* stream) {
-  if (S % 128) return ctb::fail("attention: sequence length must be a multiple of 128");
-  if (Hq % Hkv) return ctb::fail("attention: Hq must be a multiple of Hkv");
-  ctb::attn::FwdCall c{};
-  c.q = q; c.k = k; c.v = v; c.o = o; c.lse = lse; c.seg = seg; c.lim = lim; c.row_start = row_start; c.kv_lo = kv_lo; c.kv_hi = kv_hi;
-  c.B = B; c.S = S; c.Hq = Hq; c.Hkv = Hkv;
-  c.q_row_stride = q_row_stride; c.k_row_stride = k_row_stride; c.v_row_stride = v_row_stride;
-  c.o_row_stride = o_row_stride; c.scale = scale; c.spin_budget = spin_budget; c.stream = stream;
-  if (D == 128) return ctb::attn::launch_fwd<128>(c);
-  if (D == 64) return ctb::attn::launch_fwd<64>(c);
-  return ctb::fail("attention: head_dim must be 64 or 128");
-}
-
-// Sequence-parallel forward: q / o hold the Sq queries [q_off, q_off + Sq) of every row, k / v all
-// S keys; lse is [B, Hq, Sq].  q_off and Sq must be multiples of 128.
+// q/k/v/o are [B, S, H, D] views with arbitrary row stride (elements between consecutive tokens), so the packed QKV
+// projection output is read in place.  q / o hold the Sq queries [q_off, q_off + Sq) of every row (all of them: q_off 0,
+// Sq = S; fewer under sequence parallelism), k / v all S keys; lse is [B, Hq, Sq] fp32.  q_off and Sq are multiples of 128.
 CTB_API int ctb_attn_fwd_range(const void* q, const void* k, const void* v, void* o, float* lse, const int* seg,
                                const int* lim, const int* row_start, const int* kv_lo, const int* kv_hi,
                                int B, int S, int Sq, int q_off, int Hq, int Hkv, int D, long q_row_stride,
