@@ -117,9 +117,15 @@ bool gemm_pair_forced();
 long gemm_pair_workspace(const GemmCall& c, const PairPlan& plan);
 int launch_gemm_pair(const GemmCall& c, const PairPlan& plan);
 
+// Cost of a plan of the kernel below, by the estimate that it is chosen by: cycles, and k-blocks of the busiest cluster's CTAs.
+struct SplitCost {
+  double cycles;
+  long k_blocks;
+};
+
 // Products with too few output tiles to fill the GPU (gemm_split.cu): the K range of a tile cut over the
 // CTAs of a cluster.  The plan is false where the persistent kernel is the better one.
-bool gemm_split_plan(const GemmCall& c, int* width, int* splits, double* cycles = nullptr);
+bool gemm_split_plan(const GemmCall& c, int* width, int* splits, SplitCost* cost = nullptr);
 int launch_gemm_split(const GemmCall& c, int width, int splits);
 
 }  // namespace ctb

@@ -565,8 +565,11 @@ double one_cta_time(const GemmCall& c, int sms) {
   GemmCall sizes{};      // (of the sizes alone: the choice must not depend on which call came first)
   sizes.M = c.M; sizes.N = c.N; sizes.K = c.K; sizes.epi = c.epi; sizes.accumulate = c.accumulate;
   int width, slices;
-  double cycles = 0.0;
-  if (gemm_split_plan(sizes, &width, &slices, &cycles)) return 0.76 + 1.131 * cycles / 1.8e3;
+  SplitCost cost;
+  // 128-wide tiles: 0.28 us a k-block, not the 0.39 that the choice of the slices charges for both widths (240 products of 1
+  // to 1400 tokens, 17 % rms; 35 x 256 x 32000 19 us, where 37 were expected and the two-CTA form took 29)
+  if (gemm_split_plan(sizes, &width, &slices, &cost))
+    return width == 128 ? 6.9 + 0.284 * cost.k_blocks : 0.76 + 1.131 * cost.cycles / 1.8e3;
   const long num_k = div_up(c.K, 64);
   const int tm = div_up(c.M, 256) * div_up(c.N, 256) >= 2l * sms ? 2 : 1;
   const long tiles = div_up(c.M, 128 * tm) * div_up(c.N, 256), rounds = div_up(tiles, sms);
@@ -588,7 +591,10 @@ long gemm_pair_workspace(const GemmCall& c, const PairPlan& p) {
 }
 
 // Over the products of the fit the choice makes them 1.044 times as fast in the geometric mean, almost none more than 3 %
-// slower than on the one-CTA kernels (the runs of one form differ by about 2 %).
+// slower than on the one-CTA kernels (the runs of one form differ by about 2 %).  Over 1568 others, of 1 to 16384 tokens with
+// operands out of memory, not run for long: 1.030 times, 10 of them more than 3 % (and half a microsecond) slower; it was 1.018 and
+// 93 before the gain had to be 0.8 us, which is what the estimates of two short forms differ by without a reason (128 x 256 x
+// 512: 7.9 us on one CTA and 8.6 on two, expected the other way round), and before the estimate of 128-wide slices above.
 bool gemm_pair_plan(const GemmCall& c, PairPlan* plan) {
   using namespace gemm2;
   const int mode = pair_mode();
@@ -617,7 +623,8 @@ bool gemm_pair_plan(const GemmCall& c, PairPlan* plan) {
                      static_cast<unsigned>(form)) % 128u];
   if (at.form != form || at.m != c.M || at.n != c.N || at.k != c.K) {
     at = Known{c.M, c.N, c.K, form, 0, plain};
-    double best = 0.99 * one_cta_time(c, sms);
+    const double other = one_cta_time(c, sms);
+    double best = std::min(0.99 * other, other - 0.8);
     auto consider = [&](const PairPlan& p) {
       const double t = pair_time(c, p, pairs);
       if (t >= best) return;

@@ -338,7 +338,7 @@ int dispatch(const GemmCall& c, const TensorMap& ma, const TensorMap& mb, const 
 // kernel and 14000 here, where the slices are exchanged.  Clusters of 8, 4 and 2 leave some SMs of a 148-SM
 // part unused: 14, 32 and 72 of them run at a time.  Examples (us, persistent -> here): 64 x 1536 x 8960
 // 49 -> 15, 333 x 1536 x 32000 199 -> 60, 1000 x 1536 x 17920 107 -> 62; 2000 x 1536 x 17920 stays (112, 111).
-bool gemm_split_plan(const GemmCall& c, int* width, int* splits, double* estimate) {
+bool gemm_split_plan(const GemmCall& c, int* width, int* splits, SplitCost* cost) {
   if (c.epi != EPI_STORE || c.accumulate || c.push.enabled || c.max_ctas > 0) return false;
   // a gathered operand: with flags only the persistent kernel will do, and without them (the pull was done
   // before the call) the product must come out the same
@@ -357,12 +357,13 @@ bool gemm_split_plan(const GemmCall& c, int* width, int* splits, double* estimat
       const long at_once = s == 2 ? sms * 72 / 148 : (s == 4 ? sms * 32 / 148 : sms * 14 / 148);
       if (at_once < 1) break;
       const long waves = (t + at_once - 1) / at_once;
-      const double cycles = waves * (static_cast<double>((num_k + s - 1) / s) * 700.0 + 14000.0);
+      const long slice = (num_k + s - 1) / s;
+      const double cycles = waves * (static_cast<double>(slice) * 700.0 + 14000.0);
       if (cycles < best) {
         best = cycles;
         *width = bn;
         *splits = s;
-        if (estimate != nullptr) *estimate = cycles;
+        if (cost != nullptr) *cost = SplitCost{cycles, waves * slice};
         found = true;
       }
     }
