@@ -597,7 +597,11 @@ int run_gemm(const GemmCall& c) {
   const bool needs_c = (c.epi != EPI_CE_STATS || c.C != nullptr) && !c.push.enabled;
   if (needs_c && (c.ldc % (c.out_f32 ? 4 : 8))) return fail("gemm: ldc must be a multiple of 16 bytes");
   PairPlan pair;
-  if (gemm_pairs(c, &pair) && gemm_pair_workspace(c, pair) <= c.workspace_bytes) return launch_gemm_pair(c, pair);
+  if (gemm_pairs(c, &pair)) {
+    const long wanted = gemm_pair_workspace(c, pair);      // (whole pieces of 64 KiB)
+    if (wanted <= std::max(0l, c.workspace_bytes)) return launch_gemm_pair(c, pair);
+    if (c.workspace_bytes < 0) return static_cast<int>(-(wanted >> 16));
+  }
   int split_width = 0, split_slices = 0;
   if (gemm_splits(c, &split_width, &split_slices)) return launch_gemm_split(c, split_width, split_slices);
   const TensorMap ma = c.a_mn ? get_tensor_map_2d(c.A, Elt::BF16, c.M, c.K, c.lda, 64, 64, true)
@@ -774,7 +778,8 @@ int run_gemm(const GemmCall& c) {
 
 // C ABI ------------------------------------------------------------------------------------
 // C[M,N] = alpha * A*B^T (+ bias) ; see the layout table at the top of this file.  `workspace` (16-byte aligned) may be null:
-// with fewer bytes than ctb_gemm_workspace says, the product takes a kernel that needs none.
+// with fewer bytes than ctb_gemm_workspace says, the product takes a kernel that needs none.  With -1 bytes the caller asks
+// first: a product that wants a workspace is not launched, and the call returns minus its size in pieces of 64 KiB.
 CTB_API int ctb_gemm(const void* A, const void* B, void* C, int M, int N, int K, long lda, long ldb, long ldc,
                      int a_mn, int b_mn, int out_f32, int accumulate, float alpha, const void* bias, int max_ctas,
                      void* workspace, long workspace_bytes, void* stream) {

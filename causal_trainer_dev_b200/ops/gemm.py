@@ -147,18 +147,15 @@ def gemm(
         return out
     f32 = out.dtype == torch.float32
     L = _lib.lib()
-    size = 0 if max_ctas > 0 else L.ctb_gemm_workspace(m, n, k, bool(a_mn), f32, bool(accumulate))
-    work = None
-    if size:
+    args = (a.data_ptr(), b.data_ptr(), out.data_ptr(), m, n, k, a.stride(0), b.stride(0), out.stride(0),
+            bool(a_mn), bool(b_mn), f32, bool(accumulate), float(alpha), None if bias is None else bias.data_ptr(), max_ctas)
+    code = L.ctb_gemm(*args, None, -1, _lib.raw_stream())      # few products want a workspace: one call for the others
+    if code < 0:
         try:
-            work = torch.empty(size, dtype=torch.uint8, device=a.device)
+            work, size = torch.empty(-code << 16, dtype=torch.uint8, device=a.device), -code << 16
         except torch.cuda.OutOfMemoryError:
-            size = 0                              # the product takes a kernel that needs none
-    code = L.ctb_gemm(
-        a.data_ptr(), b.data_ptr(), out.data_ptr(), m, n, k, a.stride(0), b.stride(0), out.stride(0),
-        bool(a_mn), bool(b_mn), f32, bool(accumulate), float(alpha), None if bias is None else bias.data_ptr(), max_ctas,
-        None if work is None else work.data_ptr(), size, _lib.raw_stream(),
-    )
+            work, size = None, 0                               # the product takes a kernel that needs none
+        code = L.ctb_gemm(*args, None if work is None else work.data_ptr(), size, _lib.raw_stream())
     _lib.check(code, "ctb_gemm")
     return out
 
