@@ -591,10 +591,10 @@ long gemm_pair_workspace(const GemmCall& c, const PairPlan& p) {
 }
 
 // Over the products of the fit the choice makes them 1.044 times as fast in the geometric mean, almost none more than 3 %
-// slower than on the one-CTA kernels (the runs of one form differ by about 2 %).  Over 1568 others, of 1 to 16384 tokens with
-// operands out of memory, not run for long: 1.030 times, 10 of them more than 3 % (and half a microsecond) slower; it was 1.018 and
-// 93 before the gain had to be 0.8 us, which is what the estimates of two short forms differ by without a reason (128 x 256 x
-// 512: 7.9 us on one CTA and 8.6 on two, expected the other way round), and before the estimate of 128-wide slices above.
+// slower than on the one-CTA kernels (the runs of one form differ by about 2 %).  Over 1614 others, of 1 to 16384 tokens, with
+// operands out of memory and not run for long: 1.031 times, and 6 of the 1042 that take less than 40 us more than 3 % (and half a
+// microsecond) slower.  It was 40 before the gain of a short product had to be 0.8 us, which is what the estimates of two
+// short forms differ by without a reason (128 x 256 x 512: 7.9 us on one CTA and 8.6 on two, expected the other way round).
 bool gemm_pair_plan(const GemmCall& c, PairPlan* plan) {
   using namespace gemm2;
   const int mode = pair_mode();
@@ -624,7 +624,7 @@ bool gemm_pair_plan(const GemmCall& c, PairPlan* plan) {
   if (at.form != form || at.m != c.M || at.n != c.N || at.k != c.K) {
     at = Known{c.M, c.N, c.K, form, 0, plain};
     const double other = one_cta_time(c, sms);
-    double best = std::min(0.99 * other, other - 0.8);
+    double best = other < 16.0 ? other - 0.8 : 0.99 * other;
     auto consider = [&](const PairPlan& p) {
       const double t = pair_time(c, p, pairs);
       if (t >= best) return;
