@@ -468,7 +468,8 @@ gemm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ C
       tc_fence_after();
       const uint32_t taddr = tmem_base + slot * BN + (static_cast<uint32_t>(q * 32) << 16);
       const int m_sub = tc.m0 + wg * BM;     // first row of this warpgroup's sub-tile
-      drain_slot<EPI, BN, C::EPI_BUFS>(args, &map_c, taddr, tc.n0, m_sub, row, etid, bar_stage, epi, staged, add_into_c);
+      drain_slot<EPI, BN, C::EPI_BUFS, TM == 1 && EPI != EPI_PUSH>(args, &map_c, taddr, tc.n0, m_sub, row, etid, bar_stage, epi,
+                                                                   staged, add_into_c);
       tc_fence_before();
       __syncwarp();
       if (lane == 0) mbar_arrive(&tempty[slot]);
@@ -610,12 +611,6 @@ int run_gemm(const GemmCall& c) {
   const TensorMap mb = c.b_mn ? get_tensor_map_2d(c.B, Elt::BF16, c.N, c.K, c.ldb, 64, 64, true)
                              : get_tensor_map_2d(c.B, Elt::BF16, c.K, c.N, c.ldb, 64, BN, true);
   if (!mb) return 1;
-  TensorMap mc = ma;  // placeholder when no C tensor is written
-  if (needs_c) {
-    mc = c.out_f32 ? get_tensor_map_2d(c.C, Elt::F32, c.N, c.M, c.ldc, 32, 32, true)
-                   : get_tensor_map_2d(c.C, Elt::BF16, c.N, c.M, c.ldc, 64, 32, true);
-    if (!mc) return 1;
-  }
   GemmArgs a{};
   a.M = c.M;
   a.N = c.N;
@@ -753,6 +748,12 @@ int run_gemm(const GemmCall& c) {
         tiles = full + tail * ts;
       }
     }
+  }
+  TensorMap mc = ma;  // placeholder when no C tensor is written
+  if (needs_c) {
+    mc = c.out_f32 ? get_tensor_map_2d(c.C, Elt::F32, c.N, c.M, c.ldc, 32, 32, true)
+                   : get_tensor_map_2d(c.C, Elt::BF16, c.N, c.M, c.ldc, 64, tm == 1 ? 128 : 32, true);
+    if (!mc) return 1;
   }
   int grid = std::min(tiles, c.max_ctas > 0 ? c.max_ctas : sm_count());
 #define CTB_DISPATCH_TM(TMV, AM, BMN)                                                       \

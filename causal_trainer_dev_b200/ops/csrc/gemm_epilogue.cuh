@@ -43,18 +43,24 @@ __device__ __forceinline__ void tmem_loaded(uint32_t (&r)[32]) {
 // Stages one 128-byte row per lane in the warp's block and sends the block's 32 rows to (x, y) of `map`.  `stage` is the
 // warp's 4 KiB of the first of BUFS staging buffers.  Every block that is staged is stored: with two buffers the wait lets
 // the newest store go on reading, which is the other buffer's only if each of the last `staged` blocks sent one.
-template <int BUFS>
+//
+// WIDE: the warpgroup's four blocks leave as one box of 128 rows, between barriers `bar` of its own.  For bf16 tiles of 128 rows:
+// a short product is bound by its stores, and four times as many cost it a tenth (4608 x 3584 x 263 17.7 us, wide 16.3).  In
+// fp32, or with 256 rows a tile, the barriers cost more (6144 x 4096 x 367 in fp32 33.0, wide 38.6).
+template <int BUFS, bool WIDE = false>
 __device__ __forceinline__ void store_rows(const uint32_t (&w)[32], uint8_t* stage, uint32_t& staged, int lane,
-                                           const CUtensorMap* map, int x, int y, bool add) {
+                                           const CUtensorMap* map, int x, int y, bool add, bool first = true, uint32_t bar = 0) {
   uint8_t* buf = stage + (BUFS == 2 ? (staged & 1u) * EPI_BUF : 0u);
-  if (lane == 0) tma_wait_group_read<BUFS - 1>();      // the block may still be read by the store that used it last
-  __syncwarp();
+  if (lane == 0 && first) tma_wait_group_read<BUFS - 1>();      // the block may still be read by the store that used it last
+  if (WIDE) named_bar_sync(bar, 128);
+  else __syncwarp();
 #pragma unroll
   for (int j = 0; j < 8; ++j)
     *reinterpret_cast<uint4*>(buf + sw128_offset(lane, j)) = make_uint4(w[4 * j], w[4 * j + 1], w[4 * j + 2], w[4 * j + 3]);
   fence_proxy_async_smem();
-  __syncwarp();
-  if (lane == 0) {
+  if (WIDE) named_bar_sync(bar, 128);
+  else __syncwarp();
+  if (lane == 0 && first) {
     if (add) tma_reduce_add_2d(map, buf, x, y);
     else tma_store_2d(map, buf, x, y);
     tma_commit_group();
@@ -86,8 +92,8 @@ __device__ __forceinline__ void drain_f32(uint32_t taddr, float alpha, int colum
 //
 // Each warp stages and stores its own 32 rows, without a barrier of the warpgroup, and the next columns are loaded while these
 // are staged: 650 cycles for 64 columns (the copy out of shared memory of the block before last), 1050 with 128-row
-// blocks and two barriers for each.
-template <int EPI, int COLS, int BUFS>
+// blocks and two barriers for each.  WIDE: bf16 blocks of 128 rows (store_rows; `map_c` then has boxes of 128 rows).
+template <int EPI, int COLS, int BUFS, bool WIDE = false>
 __device__ __forceinline__ void drain_slot(const GemmArgs& args, const CUtensorMap* map_c, uint32_t taddr, int n0, int m_sub,
                                            int row, int etid, uint32_t bar_stage, uint8_t* epi, uint32_t& staged,
                                            bool add_into_c) {
@@ -96,47 +102,73 @@ __device__ __forceinline__ void drain_slot(const GemmArgs& args, const CUtensorM
   const int lane = etid & 31, quad = etid >> 5;
   uint8_t* stage = epi + quad * 4096;
   const int y = m_sub + quad * 32;
-  // All rows of the warp may, too: it has nothing to store, and so must stage nothing (store_rows).  (In the push epilogue
-  // the four warps meet at barriers.)
-  if (EPI != EPI_PUSH && y >= args.M) return;
+  // All rows of the warp may, too: it has nothing to store, and so must stage nothing (store_rows).
+  // (In the push epilogue and with wide blocks, whose tiles have no 128 rows without one, the four warps meet at barriers.)
+  const bool wide = WIDE && EPI != EPI_CE_STATS && !args.out_f32;
+  if (EPI != EPI_PUSH && !wide && y >= args.M) return;
   if (EPI == EPI_CE_STATS) {
     // Online softmax statistics of this 256-column slab for one row per thread.
     const int target = (grow < args.M) ? args.ce_targets[grow] : -1;
     float vmax = -INFINITY, vsum = 0.f, tlogit = 0.f;
     bool has_target = false;
     const int blocks = min(COLS / 32, (args.N - n0 + 31) / 32);
-    uint32_t r[32];
-    tmem_ld32(taddr, r);
+    if (!args.ce_keep) {
+      // (a loop of its own: with the copy and the early load of the next one the short statistics take a tenth longer, 1100 x
+      // 32000 x 512 68 us, here 62)
 #pragma unroll 1
-    for (int c = 0; c < blocks; ++c) {
-      const int col0 = n0 + c * 32;
-      float v[32];
-      float cmax = -INFINITY;
-      tmem_loaded(r);
+      for (int c = 0; c < blocks; ++c) {
+        const int col0 = n0 + c * 32;
+        uint32_t r[32];
+        tmem_ld32(taddr + c * 32, r);
+        tmem_ld_wait();
+        float cmax = -INFINITY;
 #pragma unroll
-      for (int j = 0; j < 32; ++j) {
-        v[j] = (col0 + j < args.N) ? __uint_as_float(r[j]) : -INFINITY;
-        cmax = fmaxf(cmax, v[j]);
-        if (col0 + j == target) {
-          tlogit = v[j];
-          has_target = true;
+        for (int j = 0; j < 32; ++j) {
+          const float v = (col0 + j < args.N) ? __uint_as_float(r[j]) : -INFINITY;
+          r[j] = __float_as_uint(v);
+          cmax = fmaxf(cmax, v);
+          if (col0 + j == target) {
+            tlogit = v;
+            has_target = true;
+          }
         }
+        const float nmax = fmaxf(vmax, cmax);
+        float s = 0.f;
+#pragma unroll
+        for (int j = 0; j < 32; ++j) s += __expf(__uint_as_float(r[j]) - nmax);
+        vsum = vsum * __expf(vmax - nmax) + s;
+        vmax = nmax;
       }
-      if (args.ce_keep) {
+    } else {
+      uint32_t r[32];
+      tmem_ld32(taddr, r);
+#pragma unroll 1
+      for (int c = 0; c < blocks; ++c) {
+        const int col0 = n0 + c * 32;
+        float v[32];
+        float cmax = -INFINITY;
+        tmem_loaded(r);
+#pragma unroll
+        for (int j = 0; j < 32; ++j) {
+          v[j] = (col0 + j < args.N) ? __uint_as_float(r[j]) : -INFINITY;
+          cmax = fmaxf(cmax, v[j]);
+          if (col0 + j == target) {
+            tlogit = v[j];
+            has_target = true;
+          }
+        }
         uint32_t w[32];
 #pragma unroll
         for (int j = 0; j < 32; ++j) w[j] = __float_as_uint(v[j]);
         if (c + 1 < blocks) tmem_ld32(taddr + (c + 1) * 32, r);
         store_rows<BUFS>(w, stage, staged, lane, map_c, col0, y, false);      // (columns behind the matrix are cut off)
-      } else if (c + 1 < blocks) {
-        tmem_ld32(taddr + (c + 1) * 32, r);
-      }
-      const float nmax = fmaxf(vmax, cmax);
-      float s = 0.f;
+        const float nmax = fmaxf(vmax, cmax);
+        float s = 0.f;
 #pragma unroll
-      for (int j = 0; j < 32; ++j) s += __expf(v[j] - nmax);
-      vsum = vsum * __expf(vmax - nmax) + s;
-      vmax = nmax;
+        for (int j = 0; j < 32; ++j) s += __expf(v[j] - nmax);
+        vsum = vsum * __expf(vmax - nmax) + s;
+        vmax = nmax;
+      }
     }
     if (grow < args.M) {
       const int slab = n0 / BN;
@@ -194,7 +226,7 @@ __device__ __forceinline__ void drain_slot(const GemmArgs& args, const CUtensorM
         tmem_ld32(taddr + (c + 1) * 64 + 32, r[1]);
       }
       if (EPI != EPI_PUSH) {
-        store_rows<BUFS>(w, stage, staged, lane, map_c, col0, y, add_into_c);
+        store_rows<BUFS, WIDE>(w, stage, staged, lane, map_c, col0, WIDE ? m_sub : y, add_into_c, !WIDE || quad == 0, bar_stage);
       } else {
         // reduce-scatter by push: the warpgroup's 128 threads copy the staged 128 x 128 B block into the
         // owner's receive buffer with 16-byte stores (peer memory: plain st.global only)
