@@ -42,12 +42,14 @@ from . import losses
 LAYER_CALL_BYTES = 64 << 20
 
 
-def _unused_pool_bytes() -> int:
-    """Bytes that PyTorch's allocator has from the driver in segments that no tensor lies in, and so could give back (0 before
-    its first use): what is left beside the tensors of a segment may be in pieces too small for anything."""
+# What tensors that a caller keeps from pass to pass (losses, say) may take before the activation policy looks again.
+POOL_DRIFT_BYTES = 32 << 20
+
+
+def _pool_bytes() -> tuple[int, int]:
+    """Bytes that PyTorch's allocator has from the driver, and those of them that tensors use (10 us)."""
     stats = torch.cuda.memory_stats_as_nested_dict()
-    now = lambda key: stats[key]["all"]["current"]  # noqa: E731
-    return now("reserved_bytes") - now("allocated_bytes") - now("inactive_split_bytes") if stats else 0
+    return (stats["reserved_bytes"]["all"]["current"], stats["allocated_bytes"]["all"]["current"]) if stats else (0, 0)
 
 
 class LocalProvider:
@@ -115,6 +117,7 @@ class LayerwiseEngine:
         self.options = options or EngineOptions()
         self.launches = 0
         self.kept_layers = 0
+        self._decided: dict[tuple, tuple[int, int, int, bool]] = {}     # see _layers_to_keep
         self.train_base = True                   # False: base weights frozen, no gradient buffers (LoRA)
         self.marks: list[tuple[str, torch.cuda.Event]] | None = None   # phase boundaries (benchmarks/step_phases.py)
         self._inv_freq: torch.Tensor | None = None
@@ -375,13 +378,17 @@ class LayerwiseEngine:
         per_layer, chunk = layer_activation_bytes(cfg, tokens), self.options.cut_chunk_rows
         local = type(self.provider) is LocalProvider
         logit = head_logit_bytes(cfg, tokens, chunk) if local and self.options.loss_backend == "cut" else 2
-        self._room_for_logits = True
-        if (local and type(self) is LayerwiseEngine and _unused_pool_bytes() >= cfg.num_hidden_layers * per_layer
-                + backward_working_set_bytes(cfg, tokens, min(chunk, tokens), logit)):
-            # the allocator could give back a whole pass already, so this one takes nothing more from the driver, which is what
-            # the reserve is for.  Asking the driver waits for its locks, on a shared host 0.8 to 9 ms (at times 90), the
-            # allocator 10 us.  (One replica only: ranks that share layers take the same decision, below.)
-            return cfg.num_hidden_layers
+        # Asking the driver waits for its locks, on a shared host 0.1 to 9 ms (at times 90).  An earlier pass of this size that
+        # began with as much reserved and allocated has shown that what was decided then fits into what the allocator has:
+        # had it taken more from the driver, more would be reserved now.  (One replica only: ranks that share layers decide
+        # together, below.)
+        size = (tokens, chunk, logit, self.options.memory_reserve_bytes)
+        reserved, allocated = _pool_bytes() if local and type(self) is LayerwiseEngine else (0, 0)
+        if reserved > 0 and size in self._decided:
+            then, least, count, room = self._decided[size]
+            if then == reserved and allocated <= least + POOL_DRIFT_BYTES:
+                self._room_for_logits = room
+                return count
         free, _ = torch.cuda.mem_get_info()
         budget = free - backward_working_set_bytes(cfg, tokens, chunk, logit) - self.options.memory_reserve_bytes
         if budget < cfg.num_hidden_layers * per_layer:
@@ -389,7 +396,12 @@ class LayerwiseEngine:
             budget += torch.cuda.memory_reserved() - torch.cuda.memory_allocated()
         # (with nothing to spare the loss computes its logits twice, in half of the slab)
         self._room_for_logits = budget >= 0
-        return self._least(max(0, min(cfg.num_hidden_layers, int(budget // per_layer))))
+        count = self._least(max(0, min(cfg.num_hidden_layers, int(budget // per_layer))))
+        if reserved > 0:
+            if len(self._decided) >= 64:
+                self._decided.clear()
+            self._decided[size] = (reserved, allocated, count, self._room_for_logits)
+        return count
 
     def _recompute_groups(self) -> tuple:
         """Process groups whose ranks take part in the recomputation of a layer."""

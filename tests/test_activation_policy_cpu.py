@@ -21,19 +21,21 @@ def _engine(cls=E.LayerwiseEngine, local=True, **options):
     engine = cls.__new__(cls)
     engine.cfg, engine.options = preset("llama3-8b"), E.EngineOptions(**options)
     engine.provider = E.LocalProvider.__new__(E.LocalProvider) if local else object()
+    engine._decided = {}
     return engine
 
 
-def _memory(monkeypatch, free, unused=0):
+def _memory(monkeypatch, free, pool=(0, 0)):
+    """The driver's free bytes (None: it must not be asked) and what the allocator has reserved and allocated."""
     def driver():
         if free is None:
             raise AssertionError("the driver was asked")
         return free, 0
 
     monkeypatch.setattr(torch.cuda, "mem_get_info", driver)
-    monkeypatch.setattr(torch.cuda, "memory_reserved", lambda: unused)
-    monkeypatch.setattr(torch.cuda, "memory_allocated", lambda: 0)
-    monkeypatch.setattr(E, "_unused_pool_bytes", lambda: unused)
+    monkeypatch.setattr(torch.cuda, "memory_reserved", lambda: pool[0])
+    monkeypatch.setattr(torch.cuda, "memory_allocated", lambda: pool[1])
+    monkeypatch.setattr(E, "_pool_bytes", lambda: pool)
 
 
 def test_kept_logits_take_four_bytes():
@@ -59,36 +61,70 @@ def test_policy_counts_the_slab_that_the_loss_allocates(monkeypatch):
         assert engine._layers_to_keep(TOKENS) == 0 and not engine._room_for_logits
 
 
-def test_a_whole_pass_in_the_allocator_needs_no_question(monkeypatch):
+def _free_for(layers, pool=(0, 0)):
     cfg = preset("llama3-8b")
-    need = cfg.num_hidden_layers * layer_activation_bytes(cfg, TOKENS) + backward_working_set_bytes(cfg, TOKENS, 4096, 4)
-    _memory(monkeypatch, None, need)
-    engine = _engine()
-    engine._room_for_logits = False
-    assert engine._layers_to_keep(TOKENS) == cfg.num_hidden_layers and engine._room_for_logits
-    _memory(monkeypatch, 0, need - 1)                       # less: the reserve counts
-    assert 0 < engine._layers_to_keep(TOKENS) < cfg.num_hidden_layers
+    return (backward_working_set_bytes(cfg, TOKENS, 4096, 4) + E.EngineOptions().memory_reserve_bytes
+            + layers * layer_activation_bytes(cfg, TOKENS) - (pool[0] - pool[1]))
 
 
-@pytest.mark.parametrize("which", ["provider", "subclass"])
-def test_only_one_replica_answers_from_the_allocator_alone(monkeypatch, which):
+def test_a_pass_that_has_fitted_is_not_asked_for_again(monkeypatch):
+    gb, engine = 1 << 30, _engine()
+    for layers, used, room in ((5, 20 * gb, True), (0, 21 * gb, False)):
+        pool = (30 * gb, used)
+        _memory(monkeypatch, _free_for(layers, pool) - (not room), pool)
+        assert engine._layers_to_keep(TOKENS) == layers and engine._room_for_logits == room
+        engine._room_for_logits = not room
+        for later in (pool, (30 * gb, used - gb), (30 * gb, used + E.POOL_DRIFT_BYTES)):
+            _memory(monkeypatch, None, later)
+            assert engine._layers_to_keep(TOKENS) == layers and engine._room_for_logits == room
+        engine._decided.clear()
+
+
+def test_another_state_of_the_allocator_or_another_size_asks(monkeypatch):
+    gb, engine = 1 << 30, _engine()
+    pool = (30 * gb, 20 * gb)
+    _memory(monkeypatch, _free_for(5, pool), pool)
+    assert engine._layers_to_keep(TOKENS) == 5
+    for later in ((30 * gb + 1, 20 * gb), (30 * gb - 1, 20 * gb)):
+        _memory(monkeypatch, _free_for(3, later), later)
+        assert engine._layers_to_keep(TOKENS) == 3
+        _memory(monkeypatch, _free_for(5, pool), pool)
+        assert engine._layers_to_keep(TOKENS) == 5
+    later = (30 * gb, 20 * gb + E.POOL_DRIFT_BYTES + 1)
+    _memory(monkeypatch, _free_for(3, later), later)
+    assert engine._layers_to_keep(TOKENS) == 3
+    pool = later
+    _memory(monkeypatch, None, pool)
+    for change in (lambda e: e._layers_to_keep(TOKENS - 128), lambda e: (setattr(e.options, "memory_reserve_bytes", gb), e._layers_to_keep(TOKENS))):
+        with pytest.raises(AssertionError, match="driver was asked"):
+            change(engine)
+    for tokens in range(128, 128 * 200, 128):                    # the memory of decisions is bounded
+        _memory(monkeypatch, _free_for(5, pool), pool)
+        engine._layers_to_keep(tokens)
+    assert len(engine._decided) <= 64
+
+
+@pytest.mark.parametrize("which", ["provider", "subclass", "empty"])
+def test_only_one_replica_remembers(monkeypatch, which):
     class Other(E.LayerwiseEngine):
         pass
 
-    cfg = preset("llama3-8b")
-    need = cfg.num_hidden_layers * layer_activation_bytes(cfg, TOKENS) + backward_working_set_bytes(cfg, TOKENS, 4096, 4)
-    _memory(monkeypatch, 0, need)
-    engine = _engine(local=False) if which == "provider" else _engine(Other)
-    assert engine._layers_to_keep(TOKENS) < cfg.num_hidden_layers
+    pool = (0, 0) if which == "empty" else (30 << 30, 20 << 30)
+    engine = _engine(Other) if which == "subclass" else _engine(local=which != "provider")
+    _memory(monkeypatch, _free_for(5, pool), pool)
+    engine._layers_to_keep(TOKENS)
+    _memory(monkeypatch, None, pool)
+    with pytest.raises(AssertionError, match="driver was asked"):
+        engine._layers_to_keep(TOKENS)
 
 
-def test_pieces_of_segments_in_use_do_not_count(monkeypatch):
+def test_what_the_allocator_says(monkeypatch):
     current = lambda n: {"all": {"current": n}}  # noqa: E731
-    stats = dict(reserved_bytes=current(1000), allocated_bytes=current(300), inactive_split_bytes=current(450))
+    stats = dict(reserved_bytes=current(1000), allocated_bytes=current(300))
     monkeypatch.setattr(torch.cuda, "memory_stats_as_nested_dict", lambda: stats)
-    assert E._unused_pool_bytes() == 250
+    assert E._pool_bytes() == (1000, 300)
     monkeypatch.setattr(torch.cuda, "memory_stats_as_nested_dict", dict)
-    assert E._unused_pool_bytes() == 0
+    assert E._pool_bytes() == (0, 0)
 
 
 WORKER = r'''
