@@ -5,12 +5,16 @@
 //   C[M,N] = alpha * A * B^T   and the epilogues of gemm_epilogue.cuh, the four operand layouts of gemm.cu
 //
 // What it is for.  An SM takes at most 64 bytes a clock from L2.  A k-block of a one-CTA 128 x 256 tile is
-// 48 KB for 516 cycles of tensor core, so that tile runs at two thirds of the tensor rate at best (measured:
-// 63 B / clk / SM and 66 % tensor activity on 1000 x 17920 x 1536).  Here a k-block is 32 KB for the same 516
-// cycles (490 cycles a k-block measured).  Long products run under the power cap, where bytes cost clock: the taller
-// tile reads less of B, and bands of 16 row tiles re-read B from memory half as often.  Sustained, one-CTA kernels and here,
-// us: 16384 x 28672 x 4096 2875 and 2756, 4096 x 14336 x 16384 1473 and 1398, 4096 x 4096 x 128256 3742 and 3158,
-// 8192 x 1536 x 17920 408 and 344, 8192 x 17920 x 1536 384 and 350.
+// 48 KB for 516 cycles of tensor core, so that tile runs at two thirds of the tensor rate at best (1000 x 17920 x 1536, counters:
+// 661 MB from L2, 61 bytes a clock and SM while it works, the tensor pipe active for 65 % of it).  Here a k-block is 32 KB for the
+// same 516 cycles (440 MB, 75 %).  Long products run under the power cap, where bytes cost clock: the taller tile reads less
+// of B, and bands of 16 row tiles re-read B from memory half as often.  One-CTA kernels and here, the two in turn for 4 s in
+// blocks of 20 ms, medians in us with the tenth and ninetieth hundredths: 16384 x 28672 x 4096 3090 (2972..3176) and 2768
+// (2686..2877), 16384 x 14336 x 4096 of a gradient 1533 (1499..1606) and 1390 (1365..1447), 4096 x 14336 x 16384 1587 (1517..1624) and
+// 1398 (1313..1441), 28672 x 4096 x 16384 3088 (2953..3219) and 2902 (2789..3222), 4096 x 4096 x 128256 4306 (4233..4424) and 3293
+// (3247..3401), 8192 x 1536 x 17920 412 (404..425) and 349 (343..358), 8192 x 17920 x 1536 423 (385..453) and 340 (323..382), 1000 x 17920 x
+// 1536 58 (57..59) and 51 (51..52).  16384 x 4096 x 14336 and x 28672 stay on one CTA.  Of that little is left in a whole pass over
+// an 8B MLP, whose products warm the chip for one another: 14.20 ms before there was this choice, 14.09 with it.
 //
 // Tiles of a wave that would be nearly empty, or all of them where they are fewer than the pairs of SMs, may be cut
 // along K into slices that leave fp32 partial tiles in a workspace; a second kernel adds them in the order of the slices, so
