@@ -111,7 +111,9 @@ __device__ __forceinline__ uint32_t elect_one() {
 __device__ __forceinline__ int uniform_warp_index() {
   return __shfl_sync(0xffffffffu, static_cast<int>(threadIdx.x >> 5), 0);
 }
-// mbar_wait by all lanes of a converged warp, which learn the same answer.
+// mbar_wait by all lanes of a converged warp, which learn the same answer: lanes that left alone would be missed by the votes
+// that follow, and the uniform branch is faster than the vote costs (attention, forward and backward: 1 %, a row of 1536 to 8192
+// tokens backward 6 to 10 %).
 __device__ __forceinline__ bool mbar_wait_warp(uint64_t* bar, uint32_t parity, volatile uint32_t* abort_flag,
                                                DeviceStatus* st, unsigned code, long long budget = CTB_SPIN_BUDGET) {
   return __all_sync(0xffffffffu, mbar_wait(bar, parity, abort_flag, st, code, budget));
