@@ -392,15 +392,21 @@ __global__ void rope_table_kernel(const int* __restrict__ pos, const float* __re
 // SwiGLU on the packed projection gu[T][2f] = [gate | up]:  h = silu(gate) * up.
 // Backward writes d(gate|up) in the same packed layout.
 // ------------------------------------------------------------------------------------------
+// sigmoid(x) = 1 / (1 + e) for x >= 0 and e / (1 + e) below, e = exp(-|x|): the denominator stays in (1, 2], where the
+// reciprocal needs no care for range, and nothing overflows, so gates below -88.7 keep what is left of their activation.
+// One Newton step brings the approximate reciprocal to half an ulp (and a little).  The IEEE quotient x / (1 + exp(-x)),
+// which this replaces, bound the forward kernel by its instructions (279 us at 16384 x 14336); a fast division returns zero
+// for denominators above 2^126, gates between -88.7 and -87.4.
+__device__ __forceinline__ float reciprocal_1_to_2(float d) {
+  float r;
+  asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(d));
+  return fmaf(r, fmaf(-d, r, 1.f), r);
+}
+
 // A thread takes every gridDim * blockDim-th 16-byte vector of h and steps its row along instead of dividing for
 // it, so no thread idles whatever the width (a column per thread and rows over blockIdx.y left 224 of 256 idle at
 // f = 256: 100000 x 256 82 us forward where this takes 36).  The forward kernel keeps two vectors in flight where
-// a thread has ten or more (16384 x 14336: 279 us against 300; 333 x 8960: 5.7 against 5.1), the backward kernel one (389 us
-// against 465 with two, for their 92 registers).
-// The quotient of the sigmoid is the correctly rounded one: the fast division takes 228 and 371 us at 16384 x 14336
-// where this takes 279 and 389, but returns zero for denominators above 2^126, i.e. for gates between -88.7 and
-// -87.4.  So the forward kernel is bound by the instructions of that division (1.41 GB at 5.0 TB/s), the
-// backward one by memory (6.0 TB/s).
+// a thread has ten or more, the backward kernel one.  Both are bound by memory; the grids are chosen where they are launched.
 struct SwigluWalk {
   long i, total, stride;      // vector of h; number of them; step
   long row_at, row_step;      // (row of i) * nvec: the gate vector of i is i + row_at, its up vector nvec further
@@ -451,7 +457,8 @@ swiglu_fwd_kernel(const __nv_bfloat16* __restrict__ gu, __nv_bfloat16* __restric
         unpack8(uv[k], u);
 #pragma unroll
         for (int e = 0; e < 8; ++e) {
-          const float act = __bfloat162float(__float2bfloat16(g[e] / (1.f + __expf(-g[e]))));
+          const float x = __expf(-fabsf(g[e]));
+          const float act = __bfloat162float(__float2bfloat16((g[e] < 0.f ? g[e] * x : g[e]) * reciprocal_1_to_2(1.f + x)));
           o[e] = act * u[e];
         }
         reinterpret_cast<uint4*>(h)[to[k]] = pack8(o);
@@ -472,7 +479,8 @@ swiglu_bwd_kernel(const __nv_bfloat16* __restrict__ gu, const __nv_bfloat16* __r
     unpack8(dv, d);
 #pragma unroll
     for (int e = 0; e < 8; ++e) {
-      const float sg = 1.f / (1.f + __expf(-g[e]));
+      const float x = __expf(-fabsf(g[e]));
+      const float sg = (g[e] < 0.f ? x : 1.f) * reciprocal_1_to_2(1.f + x);
       const float act = g[e] * sg;
       du[e] = d[e] * act;
       dg[e] = d[e] * u[e] * sg * (1.f + g[e] * (1.f - sg));
@@ -1192,11 +1200,17 @@ CTB_API int ctb_rope(void* x, const float* cosv, const float* sinv, long row_str
   return 0;
 }
 
+// Calls that move more than L2 holds (126 MB) stream through HBM, and there the backward kernel's two reads of a row, one of
+// dh and two writes go best with half the threads an SM can hold, the forward kernel's with twice as many blocks as fit at
+// once.  Blocks an SM, us: backward 16384 x 14336 2: 493, 4: 362 (6.5 TB/s), 6: 426, 8: 427, 16: 388; 8192 x 8960 4: 116, 8: 134;
+// out of L2 1000 x 8960 4: 13.0, 8: 11.9; 3000 x 3584 17.7 and 15.4.  Forward 16384 x 14336 4: 225, 8: 232, 16: 221 (6.4 TB/s).
+// Before, with the quotient, 388 and 278 us.
+constexpr long SWIGLU_STREAMED = 128l << 20;
 CTB_API int ctb_swiglu_fwd(const void* gu, void* h, long T, int f, void* stream) {
   if (f % 8) return fail("swiglu: intermediate size must be a multiple of 8");
   if (T <= 0 || f <= 0) return 0;
   const long total = T * (f / 8);
-  const int grid = grid_for(total, 256);
+  const int grid = grid_for(total, 256, 6 * T * f > SWIGLU_STREAMED ? 16 : 8);
   auto kern = total >= 10l * 256 * grid ? swiglu_fwd_kernel<2> : swiglu_fwd_kernel<1>;
   kern<<<grid, 256, 0, static_cast<cudaStream_t>(stream)>>>(
       static_cast<const __nv_bfloat16*>(gu), static_cast<__nv_bfloat16*>(h), T, f);
@@ -1207,7 +1221,7 @@ CTB_API int ctb_swiglu_fwd(const void* gu, void* h, long T, int f, void* stream)
 CTB_API int ctb_swiglu_bwd(const void* gu, const void* dh, void* dgu, long T, int f, void* stream) {
   if (f % 8) return fail("swiglu: intermediate size must be a multiple of 8");
   if (T <= 0 || f <= 0) return 0;
-  swiglu_bwd_kernel<<<grid_for(T * (f / 8), 256), 256, 0, static_cast<cudaStream_t>(stream)>>>(
+  swiglu_bwd_kernel<<<grid_for(T * (f / 8), 256, 10 * T * f > SWIGLU_STREAMED ? 4 : 8), 256, 0, static_cast<cudaStream_t>(stream)>>>(
       static_cast<const __nv_bfloat16*>(gu), static_cast<const __nv_bfloat16*>(dh), static_cast<__nv_bfloat16*>(dgu),
       T, f);
   CTB_CUDA_OK(cudaGetLastError());

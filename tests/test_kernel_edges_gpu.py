@@ -163,6 +163,25 @@ def test_swiglu_of_large_negative_gates(cuda_lib):
     assert near(dgate, gd.grad, 1) and near(dup, ud.grad, 1)
 
 
+@pytest.mark.parametrize("t", [1497, 1499, 2496, 2497, 4099])      # 128 MiB of traffic: backward above 1497 rows, forward above 2496
+def test_swiglu_grids_beyond_l2(cuda_lib, t):
+    """Calls on both sides of the sizes where the grids change; gates down to where exp(gate) leaves the normal range."""
+    from causal_trainer_dev_b200.ops import elementwise as E
+
+    f = 8960
+    gu, dh = _bf16(t, 2 * f, seed=t, scale=4.0), _bf16(t, f, seed=2)
+    gu[-1, :40] = -torch.arange(80, 120).bfloat16()
+    gd = gu.double().requires_grad_()
+    want = torch.nn.functional.silu(gd[:, :f]) * gd[:, f:]
+    want.backward(dh.double())
+    got, dgu = E.swiglu_forward(gu), E.swiglu_backward(gu, dh)
+    assert _rel(got, want) < 2 * BF16 and _rel(dgu, gd.grad) < BF16
+    # exp(-102) has 2 bits left in fp32, and below 1e-40 so has bf16
+    small = (want[-1, :40].abs() > 1e-36) | (want[-1, :40] == 0)
+    near = (got[-1, :40].double() - want[-1, :40]).abs() <= (2 * BF16 + 2e-5) * want[-1, :40].abs()
+    assert bool((near | ~small).all()) and not bool(got.isnan().any()) and not bool(dgu.isnan().any())
+
+
 @pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float32])
 @pytest.mark.parametrize("n,offset", [(1, 0), (7, 0), (4099, 0), (4099, 1), (1 << 20, 0), ((1 << 20) + 5, 3)])
 def test_sum_of_squares_tails_and_alignment(cuda_lib, dtype, n, offset):
