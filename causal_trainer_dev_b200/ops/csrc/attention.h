@@ -82,6 +82,7 @@ struct FwdArgs {
   SparseArgs sp;
   GroupArgs grp;
   KvFlags kvf;
+  int chained;         // see launch_chained
 };
 
 struct FwdCall {
@@ -98,6 +99,10 @@ struct FwdCall {
   int gathered_rows = 0;     // grouped: capacity of the gathered row space (a multiple of 256)
   KvFlags kvf{};
 };
+
+// Whether a call is chained to the launch before it (launch_chained): by what it reads of Q and writes of O, a long way below
+// the sizes that take CHAINED_BYTES of time.
+inline bool chained_rows(long rows, int heads, int D) { return 8 * rows * heads * D <= CHAINED_BYTES; }
 
 enum : int { MODE_DKV = 0, MODE_DQ = 1, MODE_BOTH = 2 };
 
@@ -125,6 +130,7 @@ struct BwdArgs {
   long long spin_budget;
   SparseArgs sp;
   GroupArgs grp;
+  int chained;              // see launch_chained
 };
 
 struct BwdCall {

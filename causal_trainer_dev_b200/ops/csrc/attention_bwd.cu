@@ -758,6 +758,7 @@ attn_bwd_kernel(const __grid_constant__ BwdMaps dkv_maps, const __grid_constant_
       mbar_fence_init();
     }
     __syncwarp();
+    wait_for_predecessor();
     w = resolve(static_cast<int>(blockIdx.x));
     // the resident tiles are on their way while TMEM is allocated (with Q in the forward kernel, a layer's forward
     // and backward: 8.00 -> 7.77 ms on one document of 32768 tokens, 1096 -> 1047 us on 8 image rows of 4096)
@@ -775,6 +776,8 @@ attn_bwd_kernel(const __grid_constant__ BwdMaps dkv_maps, const __grid_constant_
   __syncthreads();
   tc_fence_after();
   sh.tmem_base = *tmem_slot;
+  if (any.chained) let_successor_start();
+  wait_for_predecessor();
 
   // the next work item, for the roles that are told of it
   uint32_t turn = 0;
@@ -907,6 +910,7 @@ int prepare_bwd(const BwdCall& c, BwdMaps* maps, BwdArgs* args, int* items) {
   a.neg_lse2 = c.neg_lse2; a.neg_delta = c.neg_delta;
   a.sp = c.sp;
   a.grp = c.grp;
+  a.chained = !grouped && c.sp.it_list == nullptr && chained_rows(static_cast<long>(c.B) * Sq, c.Hq, D);
   a.status = device_status();
   a.spin_budget = c.spin_budget > 0 ? c.spin_budget : CTB_SPIN_BUDGET;
   *maps = BwdMaps{mq.map, mk.map, mv.map, mdo.map, mo1.map, mo2.map};
@@ -928,9 +932,8 @@ int launch_items(const BwdMaps& dkv_maps, const BwdMaps& dq_maps, const BwdArgs&
     CTB_CUDA_OK(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, BwdSmem<D>::BYTES));
     configured_dev = dev;
   }
-  kern<<<items, BWD_THREADS, BwdSmem<D>::BYTES, static_cast<cudaStream_t>(stream)>>>(dkv_maps, dq_maps, dkv, dq,
-                                                                                   max(dkv_items, 0));
-  CTB_CUDA_OK(cudaGetLastError());
+  CTB_CUDA_OK(launch_chained((MODES == MODE_DQ ? dq : dkv).chained != 0, kern, items, BWD_THREADS, BwdSmem<D>::BYTES, stream, 0,
+                             dkv_maps, dq_maps, dkv, dq, max(dkv_items, 0)));
   return 0;
 }
 

@@ -234,6 +234,7 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constant
       mbar_fence_init();
     }
     __syncwarp();
+    wait_for_predecessor();
     w = fwd_item<SPARSE>(args, static_cast<int>(blockIdx.x));
     if (w.state == 0 && max(w.n[0], w.n[1]) > 0) load_q(elect_one(), w);      // on its way while TMEM is allocated
   }
@@ -245,6 +246,8 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constant
   __syncthreads();
   tc_fence_after();
   const uint32_t tmem_base = *tmem_slot;
+  if (args.chained) let_successor_start();
+  wait_for_predecessor();
   auto tmem_s_of = [&](int t) -> uint32_t { return tmem_base + static_cast<uint32_t>(t) * 128u; };
   auto tmem_o_of = [&](int t) -> uint32_t { return tmem_base + 256u + static_cast<uint32_t>(t) * D; };
 
@@ -725,6 +728,7 @@ int launch_fwd_as(const FwdCall& c) {
   a.sp = c.sp;
   a.grp = c.grp;
   a.kvf = c.kvf;
+  a.chained = !grouped && c.sp.it_list == nullptr && c.kvf.flags == nullptr && chained_rows(static_cast<long>(c.B) * Sq, c.Hq, D);
   a.status = device_status();
   a.spin_budget = c.spin_budget > 0 ? c.spin_budget : CTB_SPIN_BUDGET;
   auto kern = attn_fwd_kernel<D, SPARSE>;
@@ -736,8 +740,7 @@ int launch_fwd_as(const FwdCall& c) {
     configured_dev = dev;
   }
   const int grid = grouped ? Sq / 256 : c.B * c.Hq * ((Sq + 255) / 256);
-  kern<<<grid, FWD_THREADS, L::BYTES, static_cast<cudaStream_t>(c.stream)>>>(mq.map, mk.map, mv.map, mo.map, a);
-  CTB_CUDA_OK(cudaGetLastError());
+  CTB_CUDA_OK(launch_chained(a.chained != 0, kern, grid, FWD_THREADS, L::BYTES, c.stream, 0, mq.map, mk.map, mv.map, mo.map, a));
   return 0;
 }
 

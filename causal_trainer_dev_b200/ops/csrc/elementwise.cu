@@ -67,6 +67,8 @@ __global__ void __launch_bounds__(NORM_THREADS)
 rmsnorm_fwd_kernel(const __nv_bfloat16* __restrict__ x, const __nv_bfloat16* __restrict__ residual,
                    const __nv_bfloat16* __restrict__ w, __nv_bfloat16* __restrict__ y,
                    __nv_bfloat16* __restrict__ h_out, float* __restrict__ rstd_out, int rows, int d, float eps) {
+  let_successor_start();
+  wait_for_predecessor();
   __shared__ float scratch[33];
   const int nvec = d / 8;
   for (int row = blockIdx.x; row < rows; row += gridDim.x) {
@@ -127,6 +129,8 @@ rmsnorm_bwd_kernel(const __nv_bfloat16* __restrict__ dy, const __nv_bfloat16* __
                    const __nv_bfloat16* __restrict__ w, const float* __restrict__ rstd,
                    const __nv_bfloat16* __restrict__ dres, __nv_bfloat16* __restrict__ dx,
                    float* __restrict__ dw_partial, int rows, int d) {
+  let_successor_start();
+  wait_for_predecessor();
   constexpr int WARPS = NORM_THREADS / 32;
   constexpr bool AHEAD = NV <= 2;
   constexpr bool HOLD = NV <= 4;          // w and the residual gradient in registers (else read where they are used)
@@ -229,6 +233,8 @@ constexpr int DW_WARPS = 8;
 __global__ void __launch_bounds__(DW_WARPS * 32)
 rmsnorm_dw_reduce_kernel(const float* __restrict__ partial, int parts, int d, void* __restrict__ dw, int out_f32,
                          int accumulate) {
+  let_successor_start();
+  wait_for_predecessor();
   __shared__ float sums[DW_WARPS][32];
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   const int c = blockIdx.x * 32 + lane;
@@ -257,6 +263,8 @@ rmsnorm_dw_reduce_kernel(const float* __restrict__ partial, int parts, int d, vo
 // twice the matrix in between.
 __global__ void __launch_bounds__(256)
 column_sum_kernel(const __nv_bfloat16* __restrict__ x, long ld, int rows, int n, float* __restrict__ partial) {
+  let_successor_start();
+  wait_for_predecessor();
   __shared__ float sums[8][256 + 8];
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   const int c = blockIdx.x * 256 + lane * 8;
@@ -294,6 +302,8 @@ column_sum_kernel(const __nv_bfloat16* __restrict__ x, long ld, int rows, int n,
 __global__ void rope_kernel(__nv_bfloat16* __restrict__ x, const float* __restrict__ cosv,
                             const float* __restrict__ sinv, long row_stride, int T, int heads, int D, int rot,
                             int style, float sign) {
+  let_successor_start();
+  wait_for_predecessor();
   const int half = rot / 2;
   const long total = static_cast<long>(T) * heads * half;
   for (long i = blockIdx.x * static_cast<long>(blockDim.x) + threadIdx.x; i < total;
@@ -323,6 +333,8 @@ template <int STYLE, bool SHARED>
 __global__ void __launch_bounds__(256)
 rope_vec_kernel(__nv_bfloat16* __restrict__ x, const float* __restrict__ cosv, const float* __restrict__ sinv,
                 long row_stride, int T, int heads, int D, int rot, float sign, int share) {
+  let_successor_start();
+  wait_for_predecessor();
   constexpr int N = STYLE == 0 ? 4 : 8;          // angles per lane
   const int half = rot / 2;
   const int per_head = half / N;                 // lanes per head (<= 32)
@@ -435,6 +447,8 @@ struct SwigluWalk {
 template <int AHEAD>      // vectors in flight
 __global__ void __launch_bounds__(256)
 swiglu_fwd_kernel(const __nv_bfloat16* __restrict__ gu, __nv_bfloat16* __restrict__ h, long T, int f) {
+  let_successor_start();
+  wait_for_predecessor();
   const uint4* src = reinterpret_cast<const uint4*>(gu);
   SwigluWalk w(T, f);
   while (w.i < w.total) {
@@ -468,6 +482,8 @@ swiglu_fwd_kernel(const __nv_bfloat16* __restrict__ gu, __nv_bfloat16* __restric
 __global__ void __launch_bounds__(256)
 swiglu_bwd_kernel(const __nv_bfloat16* __restrict__ gu, const __nv_bfloat16* __restrict__ dh,
                   __nv_bfloat16* __restrict__ dgu, long T, int f) {
+  let_successor_start();
+  wait_for_predecessor();
   const uint4* src = reinterpret_cast<const uint4*>(gu);
   uint4* dst = reinterpret_cast<uint4*>(dgu);
   for (SwigluWalk w(T, f); w.i < w.total; w.step()) {
@@ -541,6 +557,8 @@ __global__ void attn_delta_kernel(const __nv_bfloat16* __restrict__ o, const __n
 __global__ void attn_bwd_stats_kernel(const __nv_bfloat16* __restrict__ o, const __nv_bfloat16* __restrict__ dout,
                                       const float* __restrict__ lse, float* __restrict__ neg_lse2,
                                       float* __restrict__ neg_delta, int B, int S, int H, int D, long o_rs, long do_rs) {
+  let_successor_start();
+  wait_for_predecessor();
   const long warp_id = (blockIdx.x * static_cast<long>(blockDim.x) + threadIdx.x) >> 5;
   const int lane = threadIdx.x & 31;
   const long total = static_cast<long>(B) * S * H;
@@ -576,6 +594,8 @@ __global__ void __launch_bounds__(256)
 attn_bwd_stats_vec_kernel(const __nv_bfloat16* __restrict__ o, const __nv_bfloat16* __restrict__ dout,
                           const float* __restrict__ lse, float* __restrict__ neg_lse2,
                           float* __restrict__ neg_delta, int S, int H, long tokens, long o_rs, long do_rs) {
+  let_successor_start();
+  wait_for_predecessor();
   constexpr int LANES = D / 8;                   // lanes per (token, head) row
   constexpr int ROWS = 256 / LANES;              // rows per pass of the block
   constexpr int PASSES = STAT_TOKENS * STAT_HEADS / ROWS;
@@ -622,6 +642,8 @@ ce_combine_kernel(const float* __restrict__ pmax, const float* __restrict__ psum
                   const float* __restrict__ target_logit, const float* __restrict__ weights, float grad_scale,
                   float* __restrict__ lse, float* __restrict__ coef, float* __restrict__ block_nll,
                   float* __restrict__ block_w, int rows) {
+  let_successor_start();
+  wait_for_predecessor();
   __shared__ float part[CE_WARPS][CE_ROWS];
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   const int row = blockIdx.x * CE_ROWS + lane;
@@ -1095,12 +1117,13 @@ CTB_API int ctb_rmsnorm_fwd(const void* x, const void* residual, const void* w, 
   if (d % 8 || d > NORM_MAXV * NORM_THREADS * 8) return fail("rmsnorm: hidden size must be a multiple of 8, <= 16384");
   if (residual && !h_out) return fail("rmsnorm: residual given without h_out");
   const int grid = rows < sm_count() * 8 ? rows : sm_count() * 8;
+  const bool chained = (residual ? 8l : 4l) * rows * d <= CHAINED_BYTES;
   const int nv = (d / 8 + NORM_THREADS - 1) / NORM_THREADS;
 #define CTB_NORM_FWD(NV)                                                                                         \
-  rmsnorm_fwd_kernel<NV><<<grid, NORM_THREADS, 0, static_cast<cudaStream_t>(stream)>>>(                          \
+  CTB_CUDA_OK(launch_chained(chained, rmsnorm_fwd_kernel<NV>, grid, NORM_THREADS, 0, stream, 0,                  \
       static_cast<const __nv_bfloat16*>(x), static_cast<const __nv_bfloat16*>(residual),                         \
       static_cast<const __nv_bfloat16*>(w), static_cast<__nv_bfloat16*>(y), static_cast<__nv_bfloat16*>(h_out),  \
-      rstd, rows, d, eps)
+      rstd, rows, d, eps))
   if (nv <= 1) CTB_NORM_FWD(1);
   else if (nv <= 2) CTB_NORM_FWD(2);
   else if (nv <= 4) CTB_NORM_FWD(4);
@@ -1123,12 +1146,13 @@ CTB_API int ctb_rmsnorm_bwd(const void* dy, const void* x, const void* w, const 
   if (d % 8 || d > NORM_MAXV * NORM_THREADS * 8) return fail("rmsnorm: hidden size must be a multiple of 8, <= 16384");
   const int parts = ctb_rmsnorm_bwd_parts(rows);
   cudaStream_t s = static_cast<cudaStream_t>(stream);
+  const bool chained = 8l * rows * d <= CHAINED_BYTES;
   const int nv = (d / 8 + NORM_THREADS - 1) / NORM_THREADS;
 #define CTB_NORM_BWD(NV)                                                                       \
-  rmsnorm_bwd_kernel<NV><<<parts, NORM_THREADS, 0, s>>>(                                       \
+  CTB_CUDA_OK(launch_chained(chained, rmsnorm_bwd_kernel<NV>, parts, NORM_THREADS, 0, s, 0,    \
       static_cast<const __nv_bfloat16*>(dy), static_cast<const __nv_bfloat16*>(x),             \
       static_cast<const __nv_bfloat16*>(w), rstd, static_cast<const __nv_bfloat16*>(dres),     \
-      static_cast<__nv_bfloat16*>(dx), dw_partial, rows, d)
+      static_cast<__nv_bfloat16*>(dx), dw_partial, rows, d))
   if (nv <= 1) CTB_NORM_BWD(1);
   else if (nv <= 2) CTB_NORM_BWD(2);
   else if (nv <= 4) CTB_NORM_BWD(4);
@@ -1136,8 +1160,8 @@ CTB_API int ctb_rmsnorm_bwd(const void* dy, const void* x, const void* w, const 
 #undef CTB_NORM_BWD
   CTB_CUDA_OK(cudaGetLastError());
   if (dw != nullptr) {
-    rmsnorm_dw_reduce_kernel<<<(d + 31) / 32, DW_WARPS * 32, 0, s>>>(dw_partial, parts, d, dw, dw_f32, dw_accumulate);
-    CTB_CUDA_OK(cudaGetLastError());
+    CTB_CUDA_OK(launch_chained(chained, rmsnorm_dw_reduce_kernel, (d + 31) / 32, DW_WARPS * 32, 0, s, 0, dw_partial, parts, d, dw,
+                               dw_f32, dw_accumulate));
   }
   return 0;
 }
@@ -1156,10 +1180,11 @@ CTB_API int ctb_column_sum(const void* x, long ld, int rows, int n, float* parti
   if (n <= 0) return 0;
   cudaStream_t s = static_cast<cudaStream_t>(stream);
   const int parts = ctb_column_sum_parts(rows, n);
-  column_sum_kernel<<<dim3((n + 255) / 256, parts), 256, 0, s>>>(static_cast<const __nv_bfloat16*>(x), ld, rows, n, partial);
-  CTB_CUDA_OK(cudaGetLastError());
-  rmsnorm_dw_reduce_kernel<<<(n + 31) / 32, DW_WARPS * 32, 0, s>>>(partial, parts, n, out, out_f32, accumulate);
-  CTB_CUDA_OK(cudaGetLastError());
+  const bool chained = 2l * rows * n <= CHAINED_BYTES;
+  CTB_CUDA_OK(launch_chained(chained, column_sum_kernel, dim3((n + 255) / 256, parts), 256, 0, s, 0,
+                             static_cast<const __nv_bfloat16*>(x), ld, rows, n, partial));
+  CTB_CUDA_OK(launch_chained(chained, rmsnorm_dw_reduce_kernel, (n + 31) / 32, DW_WARPS * 32, 0, s, 0, partial, parts, n, out,
+                             out_f32, accumulate));
   return 0;
 }
 
@@ -1179,6 +1204,7 @@ CTB_API int ctb_rope(void* x, const float* cosv, const float* sinv, long row_str
   // long for the number of tokens), is no faster than a thread per pair (us, pair and vector: 8192 tokens, 4 lanes of a warp
   // 3.2 and 4.0; 2048 tokens, 8 lanes 2.7 and 2.4; 333 tokens, 4 heads of 128 2.2 and 2.0; 128 tokens, 10 heads of 128 2.3 and
   // 2.5, 40 heads 3.7 and 2.6).
+  const bool chained = 4l * T * heads * rot <= CHAINED_BYTES;
   const int angles = style == 0 ? 4 : 8;
   const int per_head = rot / 2 / angles;
   if (rot % (2 * angles) == 0 && per_head >= 1 && per_head <= 32 && D % 8 == 0 && row_stride % 8 == 0 &&
@@ -1189,14 +1215,14 @@ CTB_API int ctb_rope(void* x, const float* cosv, const float* sinv, long row_str
     while (share < 3 && (2 << share) <= walk && (static_cast<long>(T) << share) < sm_count() * 8l) ++share;
     auto kern = style == 0 ? (share ? rope_vec_kernel<0, true> : rope_vec_kernel<0, false>)
                            : (share ? rope_vec_kernel<1, true> : rope_vec_kernel<1, false>);
-    kern<<<grid_for((static_cast<long>(T) << share) * 32, 256), 256, 0, static_cast<cudaStream_t>(stream)>>>(
-        static_cast<__nv_bfloat16*>(x), cosv, sinv, row_stride, T, heads, D, rot, inverse ? -1.f : 1.f, share);
-    CTB_CUDA_OK(cudaGetLastError());
+    CTB_CUDA_OK(launch_chained(chained, kern, grid_for((static_cast<long>(T) << share) * 32, 256), 256, 0, stream, 0,
+                               static_cast<__nv_bfloat16*>(x), cosv, sinv, row_stride, T, heads, D, rot, inverse ? -1.f : 1.f,
+                               share));
     return 0;
   }
-  rope_kernel<<<grid_for(static_cast<long>(T) * heads * (rot / 2), 256), 256, 0, static_cast<cudaStream_t>(stream)>>>(
-      static_cast<__nv_bfloat16*>(x), cosv, sinv, row_stride, T, heads, D, rot, style, inverse ? -1.f : 1.f);
-  CTB_CUDA_OK(cudaGetLastError());
+  CTB_CUDA_OK(launch_chained(chained, rope_kernel, grid_for(static_cast<long>(T) * heads * (rot / 2), 256), 256, 0, stream, 0,
+                             static_cast<__nv_bfloat16*>(x), cosv, sinv, row_stride, T, heads, D, rot, style,
+                             inverse ? -1.f : 1.f));
   return 0;
 }
 
@@ -1212,19 +1238,18 @@ CTB_API int ctb_swiglu_fwd(const void* gu, void* h, long T, int f, void* stream)
   const long total = T * (f / 8);
   const int grid = grid_for(total, 256, 6 * T * f > SWIGLU_STREAMED ? 16 : 8);
   auto kern = total >= 10l * 256 * grid ? swiglu_fwd_kernel<2> : swiglu_fwd_kernel<1>;
-  kern<<<grid, 256, 0, static_cast<cudaStream_t>(stream)>>>(
-      static_cast<const __nv_bfloat16*>(gu), static_cast<__nv_bfloat16*>(h), T, f);
-  CTB_CUDA_OK(cudaGetLastError());
+  CTB_CUDA_OK(launch_chained(6 * T * f <= CHAINED_BYTES, kern, grid, 256, 0, stream, 0, static_cast<const __nv_bfloat16*>(gu),
+                             static_cast<__nv_bfloat16*>(h), T, f));
   return 0;
 }
 
 CTB_API int ctb_swiglu_bwd(const void* gu, const void* dh, void* dgu, long T, int f, void* stream) {
   if (f % 8) return fail("swiglu: intermediate size must be a multiple of 8");
   if (T <= 0 || f <= 0) return 0;
-  swiglu_bwd_kernel<<<grid_for(T * (f / 8), 256, 10 * T * f > SWIGLU_STREAMED ? 4 : 8), 256, 0, static_cast<cudaStream_t>(stream)>>>(
-      static_cast<const __nv_bfloat16*>(gu), static_cast<const __nv_bfloat16*>(dh), static_cast<__nv_bfloat16*>(dgu),
-      T, f);
-  CTB_CUDA_OK(cudaGetLastError());
+  CTB_CUDA_OK(launch_chained(10 * T * f <= CHAINED_BYTES, swiglu_bwd_kernel,
+                             grid_for(T * (f / 8), 256, 10 * T * f > SWIGLU_STREAMED ? 4 : 8), 256, 0, stream, 0,
+                             static_cast<const __nv_bfloat16*>(gu), static_cast<const __nv_bfloat16*>(dh),
+                             static_cast<__nv_bfloat16*>(dgu), T, f));
   return 0;
 }
 
@@ -1259,23 +1284,21 @@ CTB_API int ctb_attn_bwd_stats(const void* o, const void* dout, const float* lse
   const long tokens = static_cast<long>(B) * S;
   const bool wide = (D == 64 || D == 128) && o_rs % 8 == 0 && do_rs % 8 == 0 && tokens * H >= 192l * D &&
                     (reinterpret_cast<uintptr_t>(o) | reinterpret_cast<uintptr_t>(dout)) % 16 == 0;
+  const bool chained = 4 * tokens * H * D <= CHAINED_BYTES;
   const int head_blocks = (H + STAT_HEADS - 1) / STAT_HEADS;
   if (wide && head_blocks <= 65535) {
     const dim3 grid(static_cast<unsigned>((tokens + STAT_TOKENS - 1) / STAT_TOKENS), head_blocks);
     auto kern = D == 128 ? attn_bwd_stats_vec_kernel<128> : attn_bwd_stats_vec_kernel<64>;
-    kern<<<grid, 256, 0, static_cast<cudaStream_t>(stream)>>>(
-        static_cast<const __nv_bfloat16*>(o), static_cast<const __nv_bfloat16*>(dout), lse, neg_lse2, neg_delta, S, H,
-        tokens, o_rs, do_rs);
-    CTB_CUDA_OK(cudaGetLastError());
+    CTB_CUDA_OK(launch_chained(chained, kern, grid, 256, 0, stream, 0, static_cast<const __nv_bfloat16*>(o),
+                               static_cast<const __nv_bfloat16*>(dout), lse, neg_lse2, neg_delta, S, H, tokens, o_rs, do_rs));
     return 0;
   }
   const long warps = static_cast<long>(B) * S * H;
   const int threads = 256;
   const long blocks = (warps * 32 + threads - 1) / threads;
-  attn_bwd_stats_kernel<<<static_cast<unsigned>(blocks), threads, 0, static_cast<cudaStream_t>(stream)>>>(
-      static_cast<const __nv_bfloat16*>(o), static_cast<const __nv_bfloat16*>(dout), lse, neg_lse2, neg_delta, B, S, H,
-      D, o_rs, do_rs);
-  CTB_CUDA_OK(cudaGetLastError());
+  CTB_CUDA_OK(launch_chained(chained, attn_bwd_stats_kernel, static_cast<unsigned>(blocks), threads, 0, stream, 0,
+                             static_cast<const __nv_bfloat16*>(o), static_cast<const __nv_bfloat16*>(dout), lse, neg_lse2,
+                             neg_delta, B, S, H, D, o_rs, do_rs));
   return 0;
 }
 
@@ -1283,9 +1306,9 @@ CTB_API int ctb_attn_bwd_stats(const void* o, const void* dout, const float* lse
 CTB_API int ctb_ce_combine(const float* pmax, const float* psum, int slabs, const float* target_logit,
                            const float* weights, float grad_scale, float* lse, float* coef, float* block_nll,
                            float* block_w, int rows, void* stream) {
-  ce_combine_kernel<<<(rows + CE_ROWS - 1) / CE_ROWS, CE_ROWS * CE_WARPS, 0, static_cast<cudaStream_t>(stream)>>>(
-      pmax, psum, slabs, target_logit, weights, grad_scale, lse, coef, block_nll, block_w, rows);
-  CTB_CUDA_OK(cudaGetLastError());
+  CTB_CUDA_OK(launch_chained(8l * rows * slabs <= CHAINED_BYTES, ce_combine_kernel, (rows + CE_ROWS - 1) / CE_ROWS,
+                             CE_ROWS * CE_WARPS, 0, stream, 0, pmax, psum, slabs, target_logit, weights, grad_scale, lse, coef,
+                             block_nll, block_w, rows));
   return 0;
 }
 

@@ -205,6 +205,8 @@ gemm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ C
   __syncthreads();
   tc_fence_after();
   const uint32_t tmem_base = *tmem_slot;
+  if (args.chained) let_successor_start();
+  wait_for_predecessor();
 
   if (warp == 0) {
     // ------------------------------ TMA producer ------------------------------
@@ -568,8 +570,7 @@ int launch(const TensorMap& ma, const TensorMap& mb, const TensorMap& mc, const 
     CTB_CUDA_OK(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, C::SMEM_BYTES));
     configured_dev = dev;
   }
-  kern<<<grid, C::THREADS, C::SMEM_BYTES, stream>>>(ma.map, mb.map, mc.map, args);
-  CTB_CUDA_OK(cudaGetLastError());
+  CTB_CUDA_OK(launch_chained(args.chained != 0, kern, grid, C::THREADS, C::SMEM_BYTES, stream, 0, ma.map, mb.map, mc.map, args));
   return 0;
 }
 
@@ -621,6 +622,7 @@ int run_gemm(const GemmCall& c) {
   a.bias = static_cast<const __nv_bfloat16*>(c.bias);
   a.status = device_status();
   a.spin_budget = c.spin_budget > 0 ? c.spin_budget : CTB_SPIN_BUDGET;
+  a.chained = chained_call(c);
   a.b_flags = c.b_flags;
   a.b_flag_chunk = c.b_flag_chunk > 0 ? c.b_flag_chunk : 1;
   a.b_flag_base = c.b_flag_base;

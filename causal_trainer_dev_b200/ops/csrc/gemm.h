@@ -63,6 +63,7 @@ struct GemmArgs {
   GemmPush push;
   int* tile_counter;     // [2]: next tile to claim, CTAs that stopped claiming (dynamic_tiles only)
   int dynamic_tiles;
+  int chained;           // a short product of plain operands: see launch_chained
 };
 
 // Host-side call description.
@@ -104,6 +105,13 @@ struct GemmCall {
 };
 
 int run_gemm(const GemmCall& call);
+
+// Nothing that waits for another launch on this GPU or for a peer is chained: a successor that is resident already could hold
+// what the other launch needs.
+inline bool chained_call(const GemmCall& c) {
+  return !c.gathered && c.b_flags == nullptr && c.a_flags == nullptr && !c.push.enabled &&
+         2. * c.M * c.N * c.K <= CHAINED_FLOPS;
+}
 
 // Two-CTA kernel (gemm_pair.cu): 256 tm x 256 tiles on clusters of two CTAs with tcgen05.mma.cta_group::2.  The tiles
 // before `whole` are computed in one piece; the K range of each of the others is cut into `slices`, whose fp32 partial

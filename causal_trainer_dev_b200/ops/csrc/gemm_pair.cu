@@ -216,6 +216,8 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constan
   cluster_sync();                    // both CTAs' barriers exist before either signals the other
   tc_fence_after();
   const uint32_t tmem_base = *tmem_slot;
+  if (args.chained) let_successor_start();
+  wait_for_predecessor();
 
   if (warp == 0) {
     // ------------------------------ TMA producer (both CTAs) ------------------------------
@@ -374,6 +376,8 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constan
 template <int TM, bool F32>
 __global__ void __launch_bounds__(256) pair_reduce_kernel(const float* __restrict__ part, const GemmArgs args, const PairArgs walk,
                                                           void* out, long ldc) {
+  if (args.chained) let_successor_start();
+  wait_for_predecessor();
   constexpr int ROWS = 2 * TM * BM;
   const int rest = walk.num_m * walk.num_n - walk.whole;
   const int tile = blockIdx.x / (ROWS / 8);
@@ -431,19 +435,8 @@ int launch(const TensorMap& ma, const TensorMap& mb, const TensorMap& mc, const 
     CTB_CUDA_OK(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, Cfg<TM, EPI>::SMEM_BYTES));
     configured_dev = dev;
   }
-  cudaLaunchConfig_t cfg = {};
-  cfg.gridDim = dim3(static_cast<unsigned>(2 * std::min(w.units, sm_count() / 2)), 1, 1);
-  cfg.blockDim = dim3(Cfg<TM, EPI>::THREADS, 1, 1);
-  cfg.dynamicSmemBytes = Cfg<TM, EPI>::SMEM_BYTES;
-  cfg.stream = s;
-  cudaLaunchAttribute attr[1];
-  attr[0].id = cudaLaunchAttributeClusterDimension;
-  attr[0].val.clusterDim.x = 2;
-  attr[0].val.clusterDim.y = 1;
-  attr[0].val.clusterDim.z = 1;
-  cfg.attrs = attr;
-  cfg.numAttrs = 1;
-  CTB_CUDA_OK(cudaLaunchKernelEx(&cfg, kern, ma.map, mb.map, mc.map, mp.map, a, w));
+  CTB_CUDA_OK(launch_chained(a.chained != 0, kern, 2 * std::min(w.units, sm_count() / 2), Cfg<TM, EPI>::THREADS,
+                             Cfg<TM, EPI>::SMEM_BYTES, s, 2, ma.map, mb.map, mc.map, mp.map, a, w));
   return 0;
 }
 
@@ -466,6 +459,7 @@ int run(const GemmCall& c, const PairPlan& plan) {
                              : get_tensor_map_2d(c.B, Elt::BF16, c.K, c.N, c.ldb, 64, 128, true);
   if (!ma || !mb) return 1;
   GemmArgs a{};
+  a.chained = chained_call(c);
   a.M = c.M;
   a.N = c.N;
   a.K = c.K;
@@ -511,10 +505,9 @@ int run(const GemmCall& c, const PairPlan& plan) {
   }
   if (rc != 0 || rest == 0) return rc;
   const dim3 grid(static_cast<unsigned>(rest * (2 * TM * BM / 8)));
-  cudaStream_t s = static_cast<cudaStream_t>(c.stream);
-  if (c.out_f32) pair_reduce_kernel<TM, true><<<grid, 256, 0, s>>>(static_cast<const float*>(c.workspace), a, w, c.C, c.ldc);
-  else pair_reduce_kernel<TM, false><<<grid, 256, 0, s>>>(static_cast<const float*>(c.workspace), a, w, c.C, c.ldc);
-  CTB_CUDA_OK(cudaGetLastError());
+  auto reduce = c.out_f32 ? pair_reduce_kernel<TM, true> : pair_reduce_kernel<TM, false>;
+  CTB_CUDA_OK(launch_chained(a.chained != 0, reduce, grid, 256, 0, c.stream, 0, static_cast<const float*>(c.workspace), a, w, c.C,
+                             c.ldc));
   return 0;
 }
 

@@ -56,6 +56,7 @@ struct SplitArgs {
   long ldc;
   DeviceStatus* status;
   long long spin_budget;
+  int chained;           // see launch_chained
 };
 
 __device__ __forceinline__ uint32_t cluster_rank() {
@@ -124,6 +125,8 @@ gemm_split_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_consta
   __syncthreads();
   tc_fence_after();
   const uint32_t tmem_base = *tmem_slot;
+  if (args.chained) let_successor_start();
+  wait_for_predecessor();
 
   if (warp == 0) {
     {
@@ -305,19 +308,7 @@ int launch(const TensorMap& ma, const TensorMap& mb, const SplitArgs& a, int til
     CTB_CUDA_OK(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, Cfg<BN>::BYTES));
     configured_dev = dev;
   }
-  cudaLaunchConfig_t cfg = {};
-  cfg.gridDim = dim3(static_cast<unsigned>(tiles * a.splits), 1, 1);
-  cfg.blockDim = dim3(THREADS, 1, 1);
-  cfg.dynamicSmemBytes = Cfg<BN>::BYTES;
-  cfg.stream = s;
-  cudaLaunchAttribute attr[1];
-  attr[0].id = cudaLaunchAttributeClusterDimension;
-  attr[0].val.clusterDim.x = static_cast<unsigned>(a.splits);
-  attr[0].val.clusterDim.y = 1;
-  attr[0].val.clusterDim.z = 1;
-  cfg.attrs = attr;
-  cfg.numAttrs = 1;
-  CTB_CUDA_OK(cudaLaunchKernelEx(&cfg, kern, ma.map, mb.map, a));
+  CTB_CUDA_OK(launch_chained(a.chained != 0, kern, tiles * a.splits, THREADS, Cfg<BN>::BYTES, s, a.splits, ma.map, mb.map, a));
   return 0;
 }
 
@@ -381,6 +372,7 @@ int launch_gemm_split(const GemmCall& c, int width, int splits) {
   gemm3::SplitArgs a{};
   a.M = c.M; a.N = c.N; a.K = c.K;
   a.splits = splits;
+  a.chained = chained_call(c);
   a.out_f32 = c.out_f32;
   a.alpha = c.alpha;
   a.bias = static_cast<const __nv_bfloat16*>(c.bias);

@@ -51,4 +51,34 @@ DeviceStatus* device_status();
 
 int sm_count();
 
+// Programmatic dependent launch: with `chained` the kernel's CTAs may start, set up and wait (wait_for_predecessor) while the
+// launch before it in the stream still runs, if that one lets them (let_successor_start).  Only calls that are short on both
+// sides are chained.
+constexpr long CHAINED_BYTES = 64l << 20;       // moved by a memory-bound kernel
+constexpr double CHAINED_FLOPS = 6e10;          // of a product
+template <typename... P, typename... A>
+cudaError_t launch_chained(bool chained, void (*kern)(P...), dim3 grid, dim3 block, size_t smem, void* stream, int cluster,
+                           const A&... args) {
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = grid;
+  cfg.blockDim = block;
+  cfg.dynamicSmemBytes = smem;
+  cfg.stream = static_cast<cudaStream_t>(stream);
+  cudaLaunchAttribute attr[2];
+  if (cluster > 0) {
+    attr[0].id = cudaLaunchAttributeClusterDimension;
+    attr[0].val.clusterDim.x = static_cast<unsigned>(cluster);
+    attr[0].val.clusterDim.y = 1;
+    attr[0].val.clusterDim.z = 1;
+    cfg.numAttrs = 1;
+  }
+  if (chained) {
+    attr[cfg.numAttrs].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attr[cfg.numAttrs].val.programmaticStreamSerializationAllowed = 1;
+    ++cfg.numAttrs;
+  }
+  cfg.attrs = attr;
+  return cudaLaunchKernelEx(&cfg, kern, static_cast<P>(args)...);
+}
+
 }  // namespace ctb

@@ -248,6 +248,16 @@ __device__ __forceinline__ void tma_wait_group() {
 }
 
 // ---------------------------------------------------------------------------------------
+// Programmatic dependent launch (see launch_chained in host_common.h)
+// ---------------------------------------------------------------------------------------
+// Every thread, before anything that the launches before this one write or read is touched; nothing to wait for in a launch
+// that was not chained.
+__device__ __forceinline__ void wait_for_predecessor() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
+// The launch behind this one may start when all CTAs have said so.  Not before a CTA has the TMEM that it allocates: a
+// successor that took it would wait for this launch to end.
+__device__ __forceinline__ void let_successor_start() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
+
+// ---------------------------------------------------------------------------------------
 // Cluster launch control: a CTA takes over a work item (CTA) of its grid that has not started
 // ---------------------------------------------------------------------------------------
 // Asks for one; the 16-byte answer is credited to `bar`.  Not to be asked again after a refusal.
