@@ -241,6 +241,14 @@ def flash_attention_backward(
     dq = torch.empty((b, sq, hq, d), dtype=torch.bfloat16, device=q.device) if dq is None else dq
     dk = torch.empty((b, s, hkv, d), dtype=torch.bfloat16, device=q.device) if dk is None else dk
     dv = torch.empty((b, s, hkv, d), dtype=torch.bfloat16, device=q.device) if dv is None else dv
+    # partial sums of dK / dV where the key tiles are too few for the GPU; without memory for them they are computed in one piece
+    wanted = _lib.lib().ctb_attn_bwd_workspace(b, s, sq, hq, hkv, d)
+    work = None
+    if wanted:
+        try:
+            work = torch.empty(wanted, dtype=torch.uint8, device=q.device)
+        except torch.cuda.OutOfMemoryError:
+            wanted = 0
     code = _lib.lib().ctb_attn_bwd_range(
         q.data_ptr(), k.data_ptr(), v.data_ptr(), out.data_ptr() if stats is None else None, dout.data_ptr(),
         lse.data_ptr() if stats is None else None,
@@ -248,8 +256,8 @@ def flash_attention_backward(
         _at(meta.lim), meta.kv_lo.data_ptr(), meta.kv_hi.data_ptr(), meta.q_lo.data_ptr(), meta.q_hi.data_ptr(),
         _at(meta.start), _at(meta.end), _at(meta.first_q), b, s, sq, q_offset, hq, hkv, d, _row_stride(q), _row_stride(k),
         _row_stride(v), out_stride, dout_stride, _row_stride(dq), _row_stride(dk), _row_stride(dv), float(scale),
-        int(spin_budget), _lib.raw_stream())
-    _lib.check(code, "ctb_attn_bwd_range", 1 if stats is not None else 2)
+        int(spin_budget), _at(work), wanted, _lib.raw_stream())
+    _lib.check(code, "ctb_attn_bwd_range", (1 if stats is not None else 2) + (work is not None))
     return dq, dk, dv
 
 

@@ -100,9 +100,10 @@ struct FwdCall {
   KvFlags kvf{};
 };
 
-// Whether a call is chained to the launch before it (launch_chained): by what it reads of Q and writes of O, a long way below
-// the sizes that take CHAINED_BYTES of time.
-inline bool chained_rows(long rows, int heads, int D) { return 8 * rows * heads * D <= CHAINED_BYTES; }
+// Whether a call is chained to the launch before it (launch_chained): up to 2 MB of Q.  From there on nothing is gained (4
+// rows of 1024 tokens, 32 / 8 heads, forward and backward 180 us either way) and a call of a few items an SM can lose (one row of 2048,
+// 32 / 8 heads, documents of 500, backward: 58 us, chained 66).
+inline bool chained_rows(long rows, int heads, int D) { return 2 * rows * heads * D <= 2l << 20; }
 
 enum : int { MODE_DKV = 0, MODE_DQ = 1, MODE_BOTH = 2 };
 
@@ -131,6 +132,8 @@ struct BwdArgs {
   SparseArgs sp;
   GroupArgs grp;
   int chained;              // see launch_chained
+  int parts;                // dK/dV: work items per key tile (> 1: see dkv_parts_used)
+  float* partial;           // [item][part][dV, dK][D / 4][128 keys][4]
 };
 
 struct BwdCall {
@@ -149,6 +152,8 @@ struct BwdCall {
   GroupArgs grp{};
   int gathered_rows = 0;     // grouped: capacity of the gathered row space
   int ctas = 0;              // grouped: CTAs to launch (one per descriptor)
+  int parts = 1;             // work items per key tile of dK/dV, with `partial` to hold their sums
+  float* partial = nullptr;
 };
 
 // First entry and length of the work list of CTA `item`.

@@ -97,10 +97,24 @@ struct alignas(16) BwdItem {
   int y_n64;         // their number (per head)
   int y_base;        // grouped: first row (DKV) or key (DQ) of the streamed operand
   int n_entry;       // 64-row blocks to visit
-  int list;          // block-sparse: offset of the item's entries in it_list
-  int pad;
+  int list;          // block-sparse: offset of the item's entries in it_list;  dK/dV in parts: index of its partial tiles,
+                     // -1: the whole tile
+  int first;         // dK/dV in parts: first entry of this one
 };
 static_assert(sizeof(BwdItem) == 48, "three 16-byte reads");
+
+// Of the `parts` work items that a launch has for a key tile, as many have work as leave each eight iterations (two entries
+// each); one alone stores its results as if there were no others.
+__device__ __forceinline__ int dkv_parts_used(const BwdArgs& args, int n_entry) { return max(1, min(args.parts, n_entry / 16)); }
+
+// The 64-row query blocks that see the key tile kb of row b: [first, first + count).  Only the queries this rank holds,
+// [q_off, q_off + Sq), are walked.
+__device__ __forceinline__ void dkv_queries(const BwdArgs& args, int b, int kb, int& first, int& count) {
+  const int at = b * (args.S / 128) + kb;
+  const int qlo = max(args.q_lo[at], args.q_off), qhi = min(args.q_hi[at], args.q_off + args.Sq);
+  first = qlo / 64;
+  count = qhi > qlo ? (qhi + 63) / 64 - first : 0;
+}
 
 template <int MODE>
 __device__ __forceinline__ BwdItem bwd_item(const BwdArgs& args, const int cta) {
@@ -111,7 +125,7 @@ __device__ __forceinline__ BwdItem bwd_item(const BwdArgs& args, const int cta) 
   w.mode = MODE;
   w.y_base = 0;
   w.list = 0;
-  w.pad = 0;
+  w.first = 0;
   if (args.grp.desc != nullptr) {
     // grouped MoBA (see GroupArgs): gathered rows of one group against the keys of its block, no masks.
     // X = the item's resident tile: 128 keys of the block (dK/dV) or 128 gathered rows (dQ);
@@ -129,20 +143,24 @@ __device__ __forceinline__ BwdItem bwd_item(const BwdArgs& args, const int cta) 
     if (gd.w <= 0) w.mode = -2;                        // unused capacity: nothing is written
     return w;
   }
-  int idx = cta;
+  int idx = DKV && args.parts > 1 ? cta / args.parts : cta;
   if (DKV) {
     w.head = idx % args.Hkv;      // kv head
     idx /= args.Hkv;
     w.b = idx % args.B;
     const int kb = idx / args.B;  // ascending: key blocks near the start see the most queries
     w.x0 = kb * 128;
-    // only the queries this rank holds, [q_off, q_off + Sq), are walked
-    const int qlo = max(args.q_lo[w.b * nb128 + kb], args.q_off);
-    const int qhi = min(args.q_hi[w.b * nb128 + kb], args.q_off + args.Sq);
-    w.y_lo64 = qlo / 64;
-    w.y_n64 = qhi > qlo ? (qhi + 63) / 64 - w.y_lo64 : 0;
+    dkv_queries(args, w.b, kb, w.y_lo64, w.y_n64);
     w.n_entry = w.y_n64 * group;
     w.hkv = w.head;
+    if (args.parts > 1) {
+      // whole iterations (two entries) to every part that has work
+      const int part = cta % args.parts, used = dkv_parts_used(args, w.n_entry), all = w.n_entry;
+      if (part >= used) w.mode = -2;
+      w.first = all * part / used & ~1;
+      w.n_entry = (part + 1 < used ? all * (part + 1) / used & ~1 : all) - w.first;
+      w.list = used > 1 ? cta : -1;
+    }
   } else {
     w.head = idx % args.Hq;       // query head
     idx /= args.Hq;
@@ -168,6 +186,7 @@ template <int MODE>
 __device__ __forceinline__ void bwd_entry(const BwdArgs& args, const BwdItem& w, int e, int& block, int& head) {
   const bool sparse = args.sp.it_list != nullptr;
   const int entry = sparse ? __ldg(args.sp.it_list + w.list + e) : 0;
+  e += w.first;
   block = sparse ? (entry & 0xffffff) : w.y_lo64 + e % w.y_n64;
   if (args.grp.desc != nullptr) head = 0;
   else if (MODE == MODE_DQ) head = w.head;
@@ -442,7 +461,7 @@ __device__ __forceinline__ bool bwd_compute(const BwdShared& sh, const BwdMaps& 
       ++walk_head;
     }
   };
-  if (!sparse && n_entry > 0) advance(mine);
+  if (!sparse && n_entry > 0) advance(w.first + mine);
   for (int it = 0; it < n_iter; ++it) {
     const int entry_at = 2 * it + mine;
     const bool real = entry_at < n_entry;
@@ -622,7 +641,26 @@ __device__ __forceinline__ bool bwd_compute(const BwdShared& sh, const BwdMaps& 
     ok = mbar_wait_warp(u == 0 ? &sh.y1_full[slot] : &sh.y2_full[slot], u == 0 ? at.y1_phase : at.y2_phase(), sh.abort_flag,
                         sh.st, SITE_B_CW_ACC, sh.budget);
   const bool any_bad = named_bar_or(2 + u, 256, !ok);
-  if (!any_bad && writes) {
+  if (!any_bad && DKV && args.parts > 1 && w.list >= 0) {
+    // one of several work items of its key tile: fp32, as the accumulators hold them, 512 bytes of 32 keys at a time
+    float4* to = reinterpret_cast<float4*>(args.partial) + (static_cast<size_t>(w.list) * 2 + u) * (D / 4) * 128 + r;
+    const uint32_t acc = sh.tmem_base + (u == 1 ? T::ACC2 : T::ACC1);
+#pragma unroll 1
+    for (int c = half * (D / 64); c < (half + 1) * (D / 64); ++c) {
+      uint32_t rr[32];
+      if (n_iter > 0) {
+        tmem_ld32(acc + lane_off + c * 32, rr);
+        tmem_ld_wait();
+      } else {
+#pragma unroll
+        for (int e = 0; e < 32; ++e) rr[e] = 0u;
+      }
+#pragma unroll
+      for (int jj = 0; jj < 8; ++jj)
+        to[(c * 8 + jj) * 128] = make_float4(__uint_as_float(rr[jj * 4]), __uint_as_float(rr[jj * 4 + 1]),
+                                             __uint_as_float(rr[jj * 4 + 2]), __uint_as_float(rr[jj * 4 + 3]));
+    }
+  } else if (!any_bad && writes) {
     // DKV: warpgroup 0 stores dV, warpgroup 1 stores dK (scaled); DQ: warpgroup 0 stores dQ (scaled).
     const uint32_t acc = sh.tmem_base + ((DKV && u == 1) ? T::ACC2 : T::ACC1);
     const float mul = (DKV && u == 0) ? 1.f : args.scale;
@@ -678,6 +716,46 @@ __device__ __forceinline__ bool bwd_compute(const BwdShared& sh, const BwdMaps& 
   at.next_y1();
   if (DKV) ++at.y2;
   return !any_bad;
+}
+
+// dK and dV of key tiles that several work items share: the sums of their parts in the order of the parts (so the same bits
+// whatever the timing), scaled and rounded once.  A block takes 32 channels of one gradient of one tile, a thread one key.
+// Bound by the reads, out of L2.
+template <int D>
+__global__ void __launch_bounds__(128) attn_bwd_sum_kernel(const BwdArgs args, __nv_bfloat16* __restrict__ dk, long dk_rs,
+                                                           __nv_bfloat16* __restrict__ dv, long dv_rs) {
+  let_successor_start();
+  wait_for_predecessor();
+  constexpr int CHUNKS = D / 32;
+  const int chunk = blockIdx.x % CHUNKS, u = blockIdx.x / CHUNKS % 2, item = blockIdx.x / (2 * CHUNKS), r = threadIdx.x;
+  const int head = item % args.Hkv, b = item / args.Hkv % args.B, kb = item / args.Hkv / args.B;
+  int first, count;
+  dkv_queries(args, b, kb, first, count);
+  const int used = dkv_parts_used(args, count * (args.Hq / args.Hkv));
+  if (used == 1) return;                     // stored by its one work item
+  const float4* from = reinterpret_cast<const float4*>(args.partial) +
+                       (static_cast<size_t>(item) * args.parts * 2 + u) * (D / 4) * 128 + chunk * 8 * 128 + r;
+  float4 sum[8];
+#pragma unroll
+  for (int j = 0; j < 8; ++j) sum[j] = __ldcs(from + j * 128);
+  for (int p = 1; p < used; ++p) {
+    from += 2 * (D / 4) * 128;
+#pragma unroll
+    for (int j = 0; j < 8; ++j) {
+      const float4 v = __ldcs(from + j * 128);
+      sum[j].x += v.x;
+      sum[j].y += v.y;
+      sum[j].z += v.z;
+      sum[j].w += v.w;
+    }
+  }
+  const float mul = u == 0 ? 1.f : args.scale;
+  uint4* to = reinterpret_cast<uint4*>((u == 0 ? dv : dk) + (static_cast<long>(b) * args.S + kb * 128 + r) * (u == 0 ? dv_rs : dk_rs) +
+                                       head * D + chunk * 32);
+#pragma unroll
+  for (int j = 0; j < 8; j += 2)
+    to[j / 2] = make_uint4(pack_bf16(sum[j].x * mul, sum[j].y * mul), pack_bf16(sum[j].z * mul, sum[j].w * mul),
+                           pack_bf16(sum[j + 1].x * mul, sum[j + 1].y * mul), pack_bf16(sum[j + 1].z * mul, sum[j + 1].w * mul));
 }
 
 // MODES: MODE_DKV, MODE_DQ, or MODE_BOTH: work items [0, dkv_items) of the first kind, then those of the second.
@@ -776,7 +854,6 @@ attn_bwd_kernel(const __grid_constant__ BwdMaps dkv_maps, const __grid_constant_
   __syncthreads();
   tc_fence_after();
   sh.tmem_base = *tmem_slot;
-  if (any.chained) let_successor_start();
   wait_for_predecessor();
 
   // the next work item, for the roles that are told of it
@@ -837,6 +914,8 @@ attn_bwd_kernel(const __grid_constant__ BwdMaps dkv_maps, const __grid_constant_
       if (cta >= 0) w = resolve(cta);
       else w.mode = -1;
     }
+    // not at the start: the successor's blocks would crowd on the SMs that run out of work first
+    if (any.chained) let_successor_start();
   } else if (warp == 1) {
     const uint32_t on = elect_one();
     BwdWalk at;
@@ -913,9 +992,11 @@ int prepare_bwd(const BwdCall& c, BwdMaps* maps, BwdArgs* args, int* items) {
   a.chained = !grouped && c.sp.it_list == nullptr && chained_rows(static_cast<long>(c.B) * Sq, c.Hq, D);
   a.status = device_status();
   a.spin_budget = c.spin_budget > 0 ? c.spin_budget : CTB_SPIN_BUDGET;
+  a.parts = DKV && c.partial != nullptr ? c.parts : 1;
+  a.partial = c.partial;
   *maps = BwdMaps{mq.map, mk.map, mv.map, mdo.map, mo1.map, mo2.map};
   *args = a;
-  *items = grouped ? c.ctas : (DKV ? c.B * c.Hkv * (c.S / 128) : c.B * c.Hq * (Sq / 128));
+  *items = grouped ? c.ctas : (DKV ? c.B * c.Hkv * (c.S / 128) * a.parts : c.B * c.Hq * (Sq / 128));
   return 0;
 }
 
@@ -978,24 +1059,72 @@ inline bool dq_over_inputs(const BwdCall& c) {
 // first, in a launch of their own.
 template <int D>
 int launch_bwd_dense(const BwdCall& c) {
-  if (!dq_over_inputs(c)) return launch_bwd_both<D>(c, c);
-  const int rc = launch_bwd<D, MODE_DKV>(c);
-  return rc != 0 ? rc : launch_bwd<D, MODE_DQ>(c);
+  int rc;
+  if (dq_over_inputs(c)) {
+    rc = launch_bwd<D, MODE_DKV>(c);
+    if (rc == 0) rc = launch_bwd<D, MODE_DQ>(c);
+  } else {
+    rc = launch_bwd_both<D>(c, c);
+  }
+  if (rc != 0 || c.partial == nullptr) return rc;
+  BwdArgs a{};
+  a.B = c.B; a.S = c.S; a.Hq = c.Hq; a.Hkv = c.Hkv;
+  a.Sq = c.Sq; a.q_off = c.q_off;
+  a.q_lo = c.q_lo; a.q_hi = c.q_hi;
+  a.scale = c.scale;
+  a.parts = c.parts;
+  a.partial = c.partial;
+  CTB_CUDA_OK(launch_chained(chained_rows(static_cast<long>(c.B) * c.Sq, c.Hq, D), attn_bwd_sum_kernel<D>,
+                             c.B * c.Hkv * (c.S / 128) * 2 * (D / 32), 128, 0, c.stream, 0, a,
+                             static_cast<__nv_bfloat16*>(c.dk), c.dk_row_stride, static_cast<__nv_bfloat16*>(c.dv),
+                             c.dv_row_stride));
+  return 0;
+}
+
+// Work items per key tile of dK/dV.  A key tile's item walks the queries of its whole group of heads, so a call with few
+// key tiles (short rows, few kv heads) ends with a few SMs on the long ones of them: one row of 2048 tokens, 14 / 2 heads, has 32,
+// and the longest is 112 iterations where an SM has 29 of the whole call.  The estimate (cycles) takes the rows for whole
+// documents: an iteration of dK/dV 2615 and of dQ 2047, the start and end of an item 10000 and 8000, of a further part with its
+// fp32 tiles 12000, the sum of the parts 8000.  Rows of short documents then lose little, because a part without eight
+// iterations of its own has no work.
+inline int dkv_parts(int B, int S, int Sq, int Hq, int Hkv) {
+  const double tiles = static_cast<double>(B) * Hkv * (S / 128), rows = static_cast<double>(B) * Hq * (Sq / 128);
+  const double longest = static_cast<double>(Hq / Hkv) * (Sq / 128), seen = (Sq / 128 + 1) / 2.;
+  const double all = tiles * (longest / 2 * 2615 + 10000) + rows * (seen * 2047 + 8000), sms = sm_count();
+  const double whole = max(longest * 2615 + 10000, all / sms);
+  int best = 1;
+  double least = 0.83 * whole;
+  for (int p = 2; p <= 8 && longest >= 8 * p; ++p) {
+    const double t = max(longest / p * 2615 + 10000, (all + tiles * (p - 1) * 12000) / sms) + 8000;
+    if (t < least) {
+      least = t;
+      best = p;
+    }
+  }
+  return best;
 }
 
 }  // namespace attn
 }  // namespace ctb
 
+// Bytes that a backward pass of these sizes would like for partial sums of dK/dV (see dkv_parts), 0: none.
+CTB_API long ctb_attn_bwd_workspace(int B, int S, int Sq, int Hq, int Hkv, int D) {
+  if (B <= 0 || S <= 0 || Sq <= 0 || Hkv <= 0 || Hq % Hkv || (D != 64 && D != 128)) return 0;
+  const int parts = ctb::attn::dkv_parts(B, S, Sq, Hq, Hkv);
+  return parts > 1 ? static_cast<long>(B) * Hkv * (S / 128) * parts * 2 * 128 * D * 4 : 0;
+}
+
 // Whole backward of the queries [q_off, q_off + Sq) of every row (all of them: q_off 0, Sq = S): q / out / dout / dq, lse,
 // neg_lse2 and neg_delta hold those queries; k / v / dk / dv cover all S keys (with fewer queries dk / dv are partial sums).
 // The statistics are computed from out and lse first, unless out is null: then the caller hands them in.
+// With less workspace than ctb_attn_bwd_workspace says, dK/dV of a key tile are one work item each, however few there are.
 CTB_API int ctb_attn_bwd_range(const void* q, const void* k, const void* v, const void* out, const void* dout,
                                const float* lse, void* dq, void* dk, void* dv, float* neg_lse2, float* neg_delta,
                                const int* seg, const int* lim, const int* kv_lo, const int* kv_hi, const int* q_lo,
                                const int* q_hi, const int* run_start, const int* run_end, const int* first_q, int B, int S,
                                int Sq, int q_off, int Hq, int Hkv, int D, long q_rs, long k_rs, long v_rs, long o_rs,
                                long do_rs, long dq_rs, long dk_rs, long dv_rs, float scale, long long spin_budget,
-                               void* stream) {
+                               void* workspace, long workspace_bytes, void* stream) {
   if (S % 128 || Sq % 128 || q_off % 128 || q_off < 0 || q_off + Sq > S)
     return ctb::fail("attention: S, Sq and q_off must be multiples of 128 with q_off + Sq <= S");
   if (Hq % Hkv) return ctb::fail("attention: Hq must be a multiple of Hkv");
@@ -1012,6 +1141,12 @@ CTB_API int ctb_attn_bwd_range(const void* q, const void* k, const void* v, cons
   c.q_row_stride = q_rs; c.k_row_stride = k_rs; c.v_row_stride = v_rs; c.do_row_stride = do_rs;
   c.dq_row_stride = dq_rs; c.dk_row_stride = dk_rs; c.dv_row_stride = dv_rs;
   c.scale = scale; c.spin_budget = spin_budget; c.stream = stream;
+  const long wanted = ctb_attn_bwd_workspace(B, S, Sq, Hq, Hkv, D);
+  if (wanted > 0 && workspace != nullptr && workspace_bytes >= wanted && reinterpret_cast<uintptr_t>(workspace) % 16 == 0 &&
+      ((reinterpret_cast<uintptr_t>(dk) | reinterpret_cast<uintptr_t>(dv)) % 16 == 0 && dk_rs % 8 == 0 && dv_rs % 8 == 0)) {
+    c.parts = ctb::attn::dkv_parts(B, S, Sq, Hq, Hkv);
+    c.partial = static_cast<float*>(workspace);
+  }
   return D == 128 ? ctb::attn::launch_bwd_dense<128>(c) : ctb::attn::launch_bwd_dense<64>(c);
 }
 

@@ -246,7 +246,6 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constant
   __syncthreads();
   tc_fence_after();
   const uint32_t tmem_base = *tmem_slot;
-  if (args.chained) let_successor_start();
   wait_for_predecessor();
   auto tmem_s_of = [&](int t) -> uint32_t { return tmem_base + static_cast<uint32_t>(t) * 128u; };
   auto tmem_o_of = [&](int t) -> uint32_t { return tmem_base + 256u + static_cast<uint32_t>(t) * D; };
@@ -367,6 +366,8 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constant
       if (cta >= 0) w = fwd_item<SPARSE>(args, cta);
       else w.state = -1;
     }
+    // not at the start: the successor's blocks would crowd on the SMs that run out of work first
+    if (args.chained) let_successor_start();
   } else if (warp == 1) {
     // ------------------------------ MMA issuer ------------------------------
     const uint32_t on = elect_one();            // the whole warp walks, one lane issues

@@ -12,7 +12,7 @@
 // src/causal_trainer/training/optimizer.py:42-75).
 #include <cuda_bf16.h>
 
-#include "host_common.h"
+#include "attention.h"
 
 namespace ctb {
 namespace ew {
@@ -1284,7 +1284,7 @@ CTB_API int ctb_attn_bwd_stats(const void* o, const void* dout, const float* lse
   const long tokens = static_cast<long>(B) * S;
   const bool wide = (D == 64 || D == 128) && o_rs % 8 == 0 && do_rs % 8 == 0 && tokens * H >= 192l * D &&
                     (reinterpret_cast<uintptr_t>(o) | reinterpret_cast<uintptr_t>(dout)) % 16 == 0;
-  const bool chained = 4 * tokens * H * D <= CHAINED_BYTES;
+  const bool chained = attn::chained_rows(tokens, H, D);
   const int head_blocks = (H + STAT_HEADS - 1) / STAT_HEADS;
   if (wide && head_blocks <= 65535) {
     const dim3 grid(static_cast<unsigned>((tokens + STAT_TOKENS - 1) / STAT_TOKENS), head_blocks);

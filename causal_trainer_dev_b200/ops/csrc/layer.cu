@@ -28,7 +28,8 @@ CTB_API int ctb_attn_fwd_range(const void*, const void*, const void*, void*, flo
 CTB_API int ctb_attn_bwd_range(const void*, const void*, const void*, const void*, const void*, const float*, void*, void*,
                                void*, float*, float*, const int*, const int*, const int*, const int*, const int*, const int*,
                                const int*, const int*, const int*, int, int, int, int, int, int, int, long, long, long, long,
-                               long, long, long, long, float, long long, void*);
+                               long, long, long, long, float, long long, void*, long, void*);
+CTB_API long ctb_attn_bwd_workspace(int, int, int, int, int, int);
 
 namespace ctb {
 namespace layer {
@@ -118,6 +119,8 @@ struct Forward {
 struct Backward {
   bf16 *act, *n1, *n2, *dact, *dgu, *dn, *dh, *dout_o, *dqkv;
   float *stats, *parts, *no_grad, *rstd;
+  char* dkv;
+  long dkv_bytes;
   char* work;
   long work_bytes;
   Backward(const Shape& s, Block& b) {
@@ -137,6 +140,8 @@ struct Backward {
                                static_cast<long>(ctb_column_sum_parts(t, w)) * w));
     no_grad = b.take<float>(s.hidden);
     rstd = b.take<float>(z.t);
+    dkv_bytes = ctb_attn_bwd_workspace(s.batch, s.seq, s.seq, s.q_heads, s.kv_heads, s.head_dim);
+    dkv = b.take<char>(dkv_bytes);
     long wanted = 0;
     const int shapes[8][3] = {{t, s.inner, s.hidden}, {s.hidden, s.inner, t}, {t, s.hidden, 2 * s.inner},
                               {2 * s.inner, s.hidden, t}, {t, qw, s.hidden}, {s.hidden, qw, t},
@@ -247,7 +252,7 @@ CTB_API int ctb_layer_backward(const ctb::layer::Shape* sp, const ctb::layer::Co
   CTB_TRY(ctb_attn_bwd_range(k.qkv, k.qkv + z.qw, k.qkv + z.qw + z.kvw, k.o, b.dout_o, k.lse, b.dqkv, b.dqkv + z.qw,
                              b.dqkv + z.qw + z.kvw, b.stats, b.stats + z.t * s.q_heads, cx->seg, cx->lim, cx->kv_lo, cx->kv_hi,
                              cx->q_lo, cx->q_hi, cx->start, cx->end, cx->first_q, s.batch, s.seq, s.seq, 0, s.q_heads, s.kv_heads,
-                             s.head_dim, z.w, z.w, z.w, z.qw, z.qw, z.w, z.w, z.w, s.scale, 0, stream));
+                             s.head_dim, z.w, z.w, z.w, z.qw, z.qw, z.w, z.w, z.w, s.scale, 0, b.dkv, b.dkv_bytes, stream));
   CTB_TRY(ctb_rope(b.dqkv, cx->cosine, cx->sine, z.w, t, s.q_heads + s.kv_heads, s.head_dim, s.rotary_dim, s.rope_style, 1, stream));
   CTB_TRY(project_backward(b.dqkv, b.n1, w->qkv_w, b.dn, at(grads->qkv_w), z.t, s.hidden, z.w, s.grad_f32, accumulate, b.work,
                            b.work_bytes, stream));

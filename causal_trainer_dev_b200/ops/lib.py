@@ -33,7 +33,8 @@ _SIGNATURES = {
     "ctb_layer_forward": "pppppplplppp",
     "ctb_layer_backward": "ppppippp" "plplpp",
     "ctb_loss_targets": "pipipipppiiip",
-    "ctb_attn_bwd_range": "ppppppppppp" "ppppppppp" "iiiiiii" "llllllll" "flp",
+    "ctb_attn_bwd_range": "ppppppppppp" "ppppppppp" "iiiiiii" "llllllll" "fl" "plp",
+    "ctb_attn_bwd_workspace": "iiiiii",
 }
 
 
@@ -50,6 +51,7 @@ def _load() -> ctypes.CDLL | None:
     for name, kinds in _SIGNATURES.items():
         getattr(lib, name).argtypes = [_KINDS[k] for k in kinds]
     lib.ctb_gemm_workspace.restype = ctypes.c_long
+    lib.ctb_attn_bwd_workspace.restype = ctypes.c_long
     return lib
 
 
