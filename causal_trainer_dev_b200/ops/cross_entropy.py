@@ -64,6 +64,34 @@ def chunked_cross_entropy(hidden, head, targets, weights, token_budget: int = 40
     return total, weights.float().sum()
 
 
+def _target_words(targets: torch.Tensor) -> tuple[torch.Tensor, int]:
+    """Target ids as the kernels read them: 32-bit words, every one (step 1) or, of 64-bit ids, the low one of two (step 2)."""
+    if targets.dtype == torch.int64 and targets.is_contiguous():
+        return targets, 2
+    return targets.to(torch.int32).contiguous(), 1
+
+
+def _device_scale(grad_scale, device) -> tuple[float, torch.Tensor | None]:
+    """A factor of the gradients as (number, one fp32 element on the device or None)."""
+    if not isinstance(grad_scale, torch.Tensor):
+        return grad_scale, None
+    return 1.0, grad_scale.reshape(()).to(device=device, dtype=torch.float32)
+
+
+def _combine(L, pmax, psum, slabs, tlogit, tgt, step, vocab, w, scale, device_scale, lse, coef, bn, bw, rows):
+    code = L.ctb_ce_combine(_lib.ptr(pmax), _lib.ptr(psum), slabs, _lib.ptr(tlogit), _lib.ptr(tgt), step, vocab, _lib.ptr(w),
+                            ctypes.c_float(scale), _lib.ptr(device_scale), _lib.ptr(lse), _lib.ptr(coef), _lib.ptr(bn),
+                            _lib.ptr(bw), rows, _lib.stream_ptr())
+    _lib.check(code, "ctb_ce_combine")
+
+
+def _sums(L, bn, bw) -> tuple[torch.Tensor, torch.Tensor]:
+    nll, wsum = (torch.empty((), dtype=torch.float32, device=bn.device) for _ in range(2))
+    code = L.ctb_ce_sums(_lib.ptr(bn), _lib.ptr(bw), bn.numel(), _lib.ptr(nll), _lib.ptr(wsum), _lib.stream_ptr())
+    _lib.check(code, "ctb_ce_sums")
+    return nll, wsum
+
+
 def cut_ce_forward(hidden, head, targets, weights, grad_scale: float | torch.Tensor = 1.0, exchange=None):
     """Returns (nll_sum, weight_sum, lse, coef); coef = weights * grad_scale for the backward.
 
@@ -78,13 +106,12 @@ def cut_ce_forward(hidden, head, targets, weights, grad_scale: float | torch.Ten
     vocab = head.shape[0]
     slabs = (vocab + SLAB - 1) // SLAB
     dev = hidden.device
-    scale_on_device = grad_scale if isinstance(grad_scale, torch.Tensor) else None
-    if scale_on_device is not None:
-        grad_scale = 1.0
+    grad_scale, device_scale = _device_scale(grad_scale, dev)
     pmax = torch.empty((slabs, rows), dtype=torch.float32, device=dev)
     psum = torch.empty((slabs, rows), dtype=torch.float32, device=dev)
-    tlogit = torch.zeros(rows, dtype=torch.float32, device=dev)
-    tgt = targets.to(torch.int32).contiguous()
+    # (an exchange adds the ranks' target logits up: zero where a rank has none)
+    tlogit = (torch.empty if exchange is None else torch.zeros)(rows, dtype=torch.float32, device=dev)
+    tgt, step = _target_words(targets)
     w = weights.to(torch.float32).contiguous()
     L = _lib.lib()
     from .gemm import _FLAG_SOURCES, _flag_args, _rotations, flag_source_of, in_gathered_buffer
@@ -92,28 +119,23 @@ def cut_ce_forward(hidden, head, targets, weights, grad_scale: float | torch.Ten
     hit = flag_source_of(head) if _FLAG_SOURCES else None
     hit_a = flag_source_of(hidden) if _FLAG_SOURCES else None
     _, m_rotate = _rotations(None, hit_a, hidden, head, False, False, rows, vocab)
-    code = L.ctb_ce_stats(_lib.ptr(hidden), _lib.ptr(head), rows, vocab, d, ctypes.c_long(hidden.stride(0)),
-                          ctypes.c_long(head.stride(0)), _lib.ptr(tgt), _lib.ptr(pmax), _lib.ptr(psum),
+    code = L.ctb_ce_stats_step(_lib.ptr(hidden), _lib.ptr(head), rows, vocab, d, ctypes.c_long(hidden.stride(0)),
+                          ctypes.c_long(head.stride(0)), _lib.ptr(tgt), step, _lib.ptr(pmax), _lib.ptr(psum),
                           _lib.ptr(tlogit), *_flag_args(hit), *_flag_args(hit_a), m_rotate,
                           int(in_gathered_buffer(hidden, head)), None, ctypes.c_long(0), _lib.stream_ptr())
     _lib.check(code, "ctb_ce_stats")
     if exchange is not None:
         nll, wsum, lse, coef = exchange.ce_exchange(pmax, psum, slabs, tlogit, w, grad_scale)
-        if scale_on_device is not None:
-            coef.mul_(scale_on_device.reshape(()).to(coef.dtype))
+        if device_scale is not None:
+            coef.mul_(device_scale)
         return nll, wsum, lse, coef
     lse = torch.empty(rows, dtype=torch.float32, device=dev)
     coef = torch.empty(rows, dtype=torch.float32, device=dev)
     nblk = (rows + 31) // 32          # partial sums of 32 rows each (csrc/elementwise.cu: CE_ROWS)
     bn = torch.empty(nblk, dtype=torch.float32, device=dev)
     bw = torch.empty(nblk, dtype=torch.float32, device=dev)
-    code = L.ctb_ce_combine(_lib.ptr(pmax), _lib.ptr(psum), slabs, _lib.ptr(tlogit), _lib.ptr(w),
-                            ctypes.c_float(grad_scale), _lib.ptr(lse), _lib.ptr(coef), _lib.ptr(bn), _lib.ptr(bw),
-                            rows, _lib.stream_ptr())
-    _lib.check(code, "ctb_ce_combine")
-    if scale_on_device is not None:
-        coef.mul_(scale_on_device.reshape(()).to(coef.dtype))
-    return bn.sum(), bw.sum(), lse, coef
+    _combine(L, pmax, psum, slabs, tlogit, tgt, step, vocab, w, grad_scale, device_scale, lse, coef, bn, bw, rows)
+    return *_sums(L, bn, bw), lse, coef
 
 
 def cut_ce_backward(hidden, head, targets, lse, coef, *, chunk_rows: int = 4096, need_dhead: bool = True,
@@ -126,7 +148,7 @@ def cut_ce_backward(hidden, head, targets, lse, coef, *, chunk_rows: int = 4096,
     rows, d = hidden.shape
     vocab = head.shape[0]
     dev = hidden.device
-    tgt = targets.to(torch.int32).contiguous()
+    tgt, step = _target_words(targets)
     dhidden = torch.empty_like(hidden) if push is None else None
     dhead = None
     if need_dhead:
@@ -146,9 +168,9 @@ def cut_ce_backward(hidden, head, targets, lse, coef, *, chunk_rows: int = 4096,
         n = min(chunk_rows, rows - start)
         h = hidden[start:start + n]
         g = slab[:n]
-        code = L.ctb_ce_dlogits(_lib.ptr(h), _lib.ptr(head), _lib.ptr(g), n, vocab, d, ctypes.c_long(h.stride(0)),
+        code = L.ctb_ce_dlogits_step(_lib.ptr(h), _lib.ptr(head), _lib.ptr(g), n, vocab, d, ctypes.c_long(h.stride(0)),
                                 ctypes.c_long(head.stride(0)), ctypes.c_long(g.stride(0)),
-                                _lib.ptr(tgt[start:start + n]), _lib.ptr(lse[start:start + n]),
+                                _lib.ptr(tgt[start:start + n]), step, _lib.ptr(lse[start:start + n]),
                                 _lib.ptr(coef[start:start + n]), gathered, _lib.stream_ptr())
         _lib.check(code, "ctb_ce_dlogits")
         if push is None:
@@ -202,14 +224,13 @@ def cut_ce_forward_backward(hidden, head, targets, weights, grad_scale: float | 
     if not keep_logits or not keeps_logits(rows, vocab, d, chunk_rows) or in_gathered_buffer(hidden, head):
         return twice()
     dev = hidden.device
-    scale_on_device = grad_scale if isinstance(grad_scale, torch.Tensor) else None
-    scale = 1.0 if scale_on_device is not None else grad_scale
+    scale, device_scale = _device_scale(grad_scale, dev)
     slabs = (vocab + SLAB - 1) // SLAB
     f32 = lambda *shape: torch.empty(shape, dtype=torch.float32, device=dev)  # noqa: E731
     pmax, psum = f32(slabs, chunk_rows), f32(slabs, chunk_rows)
-    tlogit = torch.zeros(rows, dtype=torch.float32, device=dev)
+    tlogit = f32(rows)
     lse, coef, bn, bw = f32(rows), f32(rows), f32((rows + 31) // 32), f32((rows + 31) // 32)
-    tgt = targets.to(torch.int32).contiguous()
+    tgt, step = _target_words(targets)
     w = weights.to(torch.float32).contiguous()
     dhidden = torch.empty_like(hidden)
     dhead = None
@@ -228,24 +249,20 @@ def cut_ce_forward_backward(hidden, head, targets, weights, grad_scale: float | 
         part = slice(start, start + n)
         blocks = slice(start // 32, (start + n + 31) // 32)
         h = hidden[part]
-        code = L.ctb_ce_stats(_lib.ptr(h), _lib.ptr(head), n, vocab, d, ln(h.stride(0)), ln(head.stride(0)), _lib.ptr(tgt[part]),
-                              _lib.ptr(pmax), _lib.ptr(psum), _lib.ptr(tlogit[part]), None, ln(0), ln(0), ctypes.c_uint(0), None,
+        code = L.ctb_ce_stats_step(_lib.ptr(h), _lib.ptr(head), n, vocab, d, ln(h.stride(0)), ln(head.stride(0)), _lib.ptr(tgt[part]),
+                              step, _lib.ptr(pmax), _lib.ptr(psum), _lib.ptr(tlogit[part]), None, ln(0), ln(0), ctypes.c_uint(0), None,
                               ln(0), ln(0), ctypes.c_uint(0), 0, 0, _lib.ptr(slab), ln(vocab), _lib.stream_ptr())
         _lib.check(code, "ctb_ce_stats")
-        code = L.ctb_ce_combine(_lib.ptr(pmax), _lib.ptr(psum), slabs, _lib.ptr(tlogit[part]), _lib.ptr(w[part]),
-                                ctypes.c_float(scale), _lib.ptr(lse[part]), _lib.ptr(coef[part]), _lib.ptr(bn[blocks]),
-                                _lib.ptr(bw[blocks]), n, _lib.stream_ptr())
-        _lib.check(code, "ctb_ce_combine")
-        if scale_on_device is not None:
-            coef[part].mul_(scale_on_device.reshape(()).to(coef.dtype))
-        code = L.ctb_kept_logits_gradient(_lib.ptr(slab), ln(vocab), n, vocab, _lib.ptr(tgt[part]), _lib.ptr(lse[part]),
+        _combine(L, pmax, psum, slabs, tlogit[part], tgt[part], step, vocab, w[part], scale, device_scale, lse[part], coef[part],
+                 bn[blocks], bw[blocks], n)
+        code = L.ctb_kept_logits_gradient(_lib.ptr(slab), ln(vocab), n, vocab, _lib.ptr(tgt[part]), step, _lib.ptr(lse[part]),
                                           _lib.ptr(coef[part]), _lib.stream_ptr())
         _lib.check(code, "ctb_kept_logits_gradient")
         g = slab.view(torch.bfloat16)[:n, :vocab]
         gemm(g, head, b_mn=True, out=dhidden[part])                                                    # dH = G @ W
         if need_dhead:
             gemm(g, h, a_mn=True, b_mn=True, out=dhead, accumulate=dhead_accumulate or start > 0)       # dW += G^T H
-    return bn.sum(), bw.sum(), dhidden, dhead
+    return *_sums(L, bn, bw), dhidden, dhead
 
 
 def logits_ce_forward_backward(hidden, head, targets, weights, grad_scale: float = 1.0, *, chunk_rows: int = 4096,

@@ -639,7 +639,8 @@ attn_bwd_stats_vec_kernel(const __nv_bfloat16* __restrict__ o, const __nv_bfloat
 constexpr int CE_ROWS = 32, CE_WARPS = 8;
 __global__ void __launch_bounds__(CE_ROWS * CE_WARPS)
 ce_combine_kernel(const float* __restrict__ pmax, const float* __restrict__ psum, int slabs,
-                  const float* __restrict__ target_logit, const float* __restrict__ weights, float grad_scale,
+                  const float* __restrict__ target_logit, const int* __restrict__ targets, int target_step, int vocab,
+                  const float* __restrict__ weights, float grad_scale, const float* __restrict__ scale,
                   float* __restrict__ lse, float* __restrict__ coef, float* __restrict__ block_nll,
                   float* __restrict__ block_w, int rows) {
   let_successor_start();
@@ -677,14 +678,37 @@ ce_combine_kernel(const float* __restrict__ pmax, const float* __restrict__ psum
     const float l = m + logf(acc);
     lse[row] = l;
     w = weights[row];
-    coef[row] = w * grad_scale;
-    nll = (w != 0.f) ? (l - target_logit[row]) * w : 0.f;
+    coef[row] = w * grad_scale * (scale != nullptr ? *scale : 1.f);
+    // (the statistics write the logit of a target that is in the vocabulary, and nothing else)
+    const int t = targets[static_cast<long>(row) * target_step];
+    nll = (w != 0.f) ? (l - (t >= 0 && t < vocab ? target_logit[row] : 0.f)) * w : 0.f;
   }
   nll = warp_sum(nll);
   w = warp_sum(w);
   if (lane == 0) {
     block_nll[blockIdx.x] = nll;
     block_w[blockIdx.x] = w;
+  }
+}
+
+// Sums of the blocks' partial sums, in a fixed order: one block, both sums (two reductions of the framework took 3.5 us each and
+// a launch gap, this 2 behind the combine that it is chained to).
+__global__ void __launch_bounds__(256)
+ce_sums_kernel(const float* __restrict__ block_nll, const float* __restrict__ block_w, int blocks, float* __restrict__ nll,
+               float* __restrict__ w) {
+  let_successor_start();
+  wait_for_predecessor();
+  __shared__ float scratch[33];
+  float a = 0.f, b = 0.f;
+  for (int i = threadIdx.x; i < blocks; i += 256) {
+    a += __ldg(block_nll + i);
+    b += __ldg(block_w + i);
+  }
+  a = block_sum(a, scratch);
+  b = block_sum(b, scratch);
+  if (threadIdx.x == 0) {
+    *nll = a;
+    *w = b;
   }
 }
 
@@ -777,13 +801,15 @@ logits_ce_backward_kernel(__nv_bfloat16* __restrict__ logits, long ld, int vocab
 // Bound by memory: 6 bytes an element.
 // ------------------------------------------------------------------------------------------
 __global__ void __launch_bounds__(256)
-kept_logits_gradient_kernel(float* __restrict__ logits, long ld, int vocab, const int* __restrict__ targets,
+kept_logits_gradient_kernel(float* __restrict__ logits, long ld, int vocab, const int* __restrict__ targets, int target_step,
                             const float* __restrict__ lse, const float* __restrict__ coef) {
+  let_successor_start();
+  wait_for_predecessor();
   const long row = blockIdx.x;
   const float* x = logits + row * ld;
   __nv_bfloat16* g = reinterpret_cast<__nv_bfloat16*>(logits + row * ld);
   const float l = lse[row], c = coef[row];
-  const int t = targets[row];
+  const int t = targets[row * target_step];
   const int chunks = (vocab + 2047) / 2048;
   float4 a[2], next[2] = {};
   auto load = [&](int k, float4 (&to)[2]) {
@@ -1302,13 +1328,19 @@ CTB_API int ctb_attn_bwd_stats(const void* o, const void* dout, const float* lse
   return 0;
 }
 
-// block_nll / block_w must hold ceil(rows / 32) floats each.
-CTB_API int ctb_ce_combine(const float* pmax, const float* psum, int slabs, const float* target_logit,
-                           const float* weights, float grad_scale, float* lse, float* coef, float* block_nll,
-                           float* block_w, int rows, void* stream) {
+// block_nll / block_w must hold ceil(rows / 32) floats each; ctb_ce_sums adds them up.  coef = weights * grad_scale * *scale (scale
+// may be null).  target_step: see ctb_ce_stats_step; the logit of a row whose target is outside [0, vocab) counts as 0.
+CTB_API int ctb_ce_combine(const float* pmax, const float* psum, int slabs, const float* target_logit, const int* targets,
+                           int target_step, int vocab, const float* weights, float grad_scale, const float* scale, float* lse,
+                           float* coef, float* block_nll, float* block_w, int rows, void* stream) {
   CTB_CUDA_OK(launch_chained(8l * rows * slabs <= CHAINED_BYTES, ce_combine_kernel, (rows + CE_ROWS - 1) / CE_ROWS,
-                             CE_ROWS * CE_WARPS, 0, stream, 0, pmax, psum, slabs, target_logit, weights, grad_scale, lse, coef,
-                             block_nll, block_w, rows));
+                             CE_ROWS * CE_WARPS, 0, stream, 0, pmax, psum, slabs, target_logit, targets, target_step, vocab,
+                             weights, grad_scale, scale, lse, coef, block_nll, block_w, rows));
+  return 0;
+}
+
+CTB_API int ctb_ce_sums(const float* block_nll, const float* block_w, int blocks, float* nll, float* w, void* stream) {
+  CTB_CUDA_OK(launch_chained(true, ce_sums_kernel, 1, 256, 0, stream, 0, block_nll, block_w, blocks, nll, w));
   return 0;
 }
 
@@ -1334,12 +1366,12 @@ CTB_API int ctb_logits_ce_backward(void* logits, long ld, int rows, int vocab, c
 }
 
 // The gradient of kept logits in their place (see the kernel): rows of ld fp32 elements become rows of 2 ld bf16 elements.
-CTB_API int ctb_kept_logits_gradient(float* logits, long ld, int rows, int vocab, const int* targets, const float* lse,
-                                     const float* coef, void* stream) {
+CTB_API int ctb_kept_logits_gradient(float* logits, long ld, int rows, int vocab, const int* targets, int target_step,
+                                     const float* lse, const float* coef, void* stream) {
   if (ld % 8 || vocab % 8 || ld < vocab) return fail("kept_logits: rows must be whole vectors of eight");
   if (rows <= 0) return 0;
-  kept_logits_gradient_kernel<<<rows, 256, 0, static_cast<cudaStream_t>(stream)>>>(logits, ld, vocab, targets, lse, coef);
-  CTB_CUDA_OK(cudaGetLastError());
+  CTB_CUDA_OK(launch_chained(6l * rows * vocab <= CHAINED_BYTES, kept_logits_gradient_kernel, rows, 256, 0, stream, 0, logits, ld,
+                             vocab, targets, target_step, lse, coef));
   return 0;
 }
 

@@ -54,6 +54,7 @@ struct GemmArgs {
   long a_flag_base;
   unsigned a_flag_epoch;
   const int* ce_targets;
+  int ce_target_step;    // words from one target to the next: 2 for 64-bit ids, of which the low word is read
   float* ce_max;
   float* ce_sum;
   float* ce_target_logit;
@@ -94,6 +95,7 @@ struct GemmCall {
   int gathered = 0;       // an operand lies in a gathered buffer (its flags may be left out once the pull is done)
   long long spin_budget = 0;
   const int* ce_targets = nullptr;
+  int ce_target_step = 1;
   float* ce_max = nullptr;
   float* ce_sum = nullptr;
   float* ce_target_logit = nullptr;

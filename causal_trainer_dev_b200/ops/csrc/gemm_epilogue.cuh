@@ -108,7 +108,7 @@ __device__ __forceinline__ void drain_slot(const GemmArgs& args, const CUtensorM
   if (EPI != EPI_PUSH && !wide && y >= args.M) return;
   if (EPI == EPI_CE_STATS) {
     // Online softmax statistics of this 256-column slab for one row per thread.
-    const int target = (grow < args.M) ? args.ce_targets[grow] : -1;
+    const int target = (grow < args.M) ? args.ce_targets[static_cast<long>(grow) * args.ce_target_step] : -1;
     float vmax = -INFINITY, vsum = 0.f, tlogit = 0.f;
     bool has_target = false;
     const int blocks = min(COLS / 32, (args.N - n0 + 31) / 32);
@@ -184,7 +184,7 @@ __device__ __forceinline__ void drain_slot(const GemmArgs& args, const CUtensorM
     if (EPI == EPI_CE_DLOGITS && grow < args.M) {
       lse = args.ce_lse[grow];
       coef = args.ce_coef[grow];
-      target = args.ce_targets[grow];
+      target = args.ce_targets[static_cast<long>(grow) * args.ce_target_step];
     }
     const int blocks = min(COLS / 64, (args.N - n0 + 63) / 64);
     uint32_t r[2][32];

@@ -470,6 +470,7 @@ int run(const GemmCall& c, const PairPlan& plan) {
   a.status = device_status();
   a.spin_budget = c.spin_budget > 0 ? c.spin_budget : CTB_SPIN_BUDGET;
   a.ce_targets = c.ce_targets;
+  a.ce_target_step = c.ce_target_step;
   a.ce_max = c.ce_max;
   a.ce_sum = c.ce_sum;
   a.ce_target_logit = c.ce_target_logit;
