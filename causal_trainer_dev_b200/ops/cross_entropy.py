@@ -78,18 +78,39 @@ def _device_scale(grad_scale, device) -> tuple[float, torch.Tensor | None]:
     return 1.0, grad_scale.reshape(()).to(device=device, dtype=torch.float32)
 
 
-def _combine(L, pmax, psum, slabs, tlogit, tgt, step, vocab, w, scale, device_scale, lse, coef, bn, bw, rows):
-    code = L.ctb_ce_combine(_lib.ptr(pmax), _lib.ptr(psum), slabs, _lib.ptr(tlogit), _lib.ptr(tgt), step, vocab, _lib.ptr(w),
-                            ctypes.c_float(scale), _lib.ptr(device_scale), _lib.ptr(lse), _lib.ptr(coef), _lib.ptr(bn),
-                            _lib.ptr(bw), rows, _lib.stream_ptr())
+class _Scratch:
+    """fp32 pieces of one allocation by their addresses (an allocation each costs more host time than a launch); it holds them
+    while it lives."""
+
+    def __init__(self, device, **counts: int):
+        self.device = device
+        self._whole = torch.empty(sum(counts.values()), dtype=torch.float32, device=device)
+        at = self._whole.data_ptr()
+        for name, count in counts.items():
+            setattr(self, name, at)
+            at += 4 * count
+
+
+def _combine(L, work: _Scratch, slabs, tgt, step, vocab, w, scale, device_scale, lse, coef, start, rows):
+    """Row statistics of the rows [start, start + rows) of a call (``work``: the slabs of these rows alone)."""
+    p = ctypes.c_void_p
+    code = L.ctb_ce_combine(p(work.pmax), p(work.psum), slabs, p(work.tlogit + 4 * start), p(tgt.data_ptr() + 4 * step * start),
+                            step, vocab, p(w.data_ptr() + 4 * start), ctypes.c_float(scale), _lib.ptr(device_scale),
+                            p(lse + 4 * start), p(coef + 4 * start), p(work.bn + start // 32 * 4), p(work.bw + start // 32 * 4),
+                            rows, _lib.stream_ptr())
     _lib.check(code, "ctb_ce_combine")
 
 
-def _sums(L, bn, bw) -> tuple[torch.Tensor, torch.Tensor]:
-    nll, wsum = (torch.empty((), dtype=torch.float32, device=bn.device) for _ in range(2))
-    code = L.ctb_ce_sums(_lib.ptr(bn), _lib.ptr(bw), bn.numel(), _lib.ptr(nll), _lib.ptr(wsum), _lib.stream_ptr())
+def _sums(L, work: _Scratch, rows: int) -> tuple[torch.Tensor, torch.Tensor]:
+    nll, wsum = (torch.empty((), dtype=torch.float32, device=work.device) for _ in range(2))
+    code = L.ctb_ce_sums(ctypes.c_void_p(work.bn), ctypes.c_void_p(work.bw), _row_blocks(rows), _lib.ptr(nll), _lib.ptr(wsum),
+                         _lib.stream_ptr())
     _lib.check(code, "ctb_ce_sums")
     return nll, wsum
+
+
+def _row_blocks(rows: int) -> int:
+    return (rows + 31) // 32          # partial sums of 32 rows each (csrc/elementwise.cu: CE_ROWS)
 
 
 def cut_ce_forward(hidden, head, targets, weights, grad_scale: float | torch.Tensor = 1.0, exchange=None):
@@ -107,10 +128,15 @@ def cut_ce_forward(hidden, head, targets, weights, grad_scale: float | torch.Ten
     slabs = (vocab + SLAB - 1) // SLAB
     dev = hidden.device
     grad_scale, device_scale = _device_scale(grad_scale, dev)
-    pmax = torch.empty((slabs, rows), dtype=torch.float32, device=dev)
-    psum = torch.empty((slabs, rows), dtype=torch.float32, device=dev)
-    # (an exchange adds the ranks' target logits up: zero where a rank has none)
-    tlogit = (torch.empty if exchange is None else torch.zeros)(rows, dtype=torch.float32, device=dev)
+    p = ctypes.c_void_p
+    if exchange is None:
+        work = _Scratch(dev, pmax=slabs * rows, psum=slabs * rows, tlogit=rows, bn=_row_blocks(rows), bw=_row_blocks(rows))
+        parts = p(work.pmax), p(work.psum), p(work.tlogit)
+    else:
+        pmax, psum = (torch.empty((slabs, rows), dtype=torch.float32, device=dev) for _ in range(2))
+        # (the exchange adds the ranks' target logits up: zero where a rank has none)
+        tlogit = torch.zeros(rows, dtype=torch.float32, device=dev)
+        parts = _lib.ptr(pmax), _lib.ptr(psum), _lib.ptr(tlogit)
     tgt, step = _target_words(targets)
     w = weights.to(torch.float32).contiguous()
     L = _lib.lib()
@@ -120,9 +146,8 @@ def cut_ce_forward(hidden, head, targets, weights, grad_scale: float | torch.Ten
     hit_a = flag_source_of(hidden) if _FLAG_SOURCES else None
     _, m_rotate = _rotations(None, hit_a, hidden, head, False, False, rows, vocab)
     code = L.ctb_ce_stats_step(_lib.ptr(hidden), _lib.ptr(head), rows, vocab, d, ctypes.c_long(hidden.stride(0)),
-                          ctypes.c_long(head.stride(0)), _lib.ptr(tgt), step, _lib.ptr(pmax), _lib.ptr(psum),
-                          _lib.ptr(tlogit), *_flag_args(hit), *_flag_args(hit_a), m_rotate,
-                          int(in_gathered_buffer(hidden, head)), None, ctypes.c_long(0), _lib.stream_ptr())
+                               ctypes.c_long(head.stride(0)), _lib.ptr(tgt), step, *parts, *_flag_args(hit), *_flag_args(hit_a),
+                               m_rotate, int(in_gathered_buffer(hidden, head)), None, ctypes.c_long(0), _lib.stream_ptr())
     _lib.check(code, "ctb_ce_stats")
     if exchange is not None:
         nll, wsum, lse, coef = exchange.ce_exchange(pmax, psum, slabs, tlogit, w, grad_scale)
@@ -131,11 +156,8 @@ def cut_ce_forward(hidden, head, targets, weights, grad_scale: float | torch.Ten
         return nll, wsum, lse, coef
     lse = torch.empty(rows, dtype=torch.float32, device=dev)
     coef = torch.empty(rows, dtype=torch.float32, device=dev)
-    nblk = (rows + 31) // 32          # partial sums of 32 rows each (csrc/elementwise.cu: CE_ROWS)
-    bn = torch.empty(nblk, dtype=torch.float32, device=dev)
-    bw = torch.empty(nblk, dtype=torch.float32, device=dev)
-    _combine(L, pmax, psum, slabs, tlogit, tgt, step, vocab, w, grad_scale, device_scale, lse, coef, bn, bw, rows)
-    return *_sums(L, bn, bw), lse, coef
+    _combine(L, work, slabs, tgt, step, vocab, w, grad_scale, device_scale, lse.data_ptr(), coef.data_ptr(), 0, rows)
+    return *_sums(L, work, rows), lse, coef
 
 
 def cut_ce_backward(hidden, head, targets, lse, coef, *, chunk_rows: int = 4096, need_dhead: bool = True,
@@ -226,10 +248,8 @@ def cut_ce_forward_backward(hidden, head, targets, weights, grad_scale: float | 
     dev = hidden.device
     scale, device_scale = _device_scale(grad_scale, dev)
     slabs = (vocab + SLAB - 1) // SLAB
-    f32 = lambda *shape: torch.empty(shape, dtype=torch.float32, device=dev)  # noqa: E731
-    pmax, psum = f32(slabs, chunk_rows), f32(slabs, chunk_rows)
-    tlogit = f32(rows)
-    lse, coef, bn, bw = f32(rows), f32(rows), f32((rows + 31) // 32), f32((rows + 31) // 32)
+    work = _Scratch(dev, pmax=slabs * chunk_rows, psum=slabs * chunk_rows, tlogit=rows, lse=rows, coef=rows,
+                    bn=_row_blocks(rows), bw=_row_blocks(rows))
     tgt, step = _target_words(targets)
     w = weights.to(torch.float32).contiguous()
     dhidden = torch.empty_like(hidden)
@@ -237,32 +257,32 @@ def cut_ce_forward_backward(hidden, head, targets, weights, grad_scale: float | 
     if need_dhead:
         dhead = dhead_out if dhead_out is not None else torch.empty((vocab, d), dtype=torch.bfloat16, device=dev)
     try:
-        slab = f32(chunk_rows, vocab)
+        slab = torch.empty((chunk_rows, vocab), dtype=torch.float32, device=dev)
     except torch.cuda.OutOfMemoryError:
         slab = None
     if slab is None:
-        del pmax, psum, dhidden, dhead
+        del work, dhidden, dhead
         return twice()
-    L, ln = _lib.lib(), ctypes.c_long
+    L, ln, p = _lib.lib(), ctypes.c_long, ctypes.c_void_p
     for start in range(0, rows, chunk_rows):
         n = min(chunk_rows, rows - start)
         part = slice(start, start + n)
-        blocks = slice(start // 32, (start + n + 31) // 32)
         h = hidden[part]
-        code = L.ctb_ce_stats_step(_lib.ptr(h), _lib.ptr(head), n, vocab, d, ln(h.stride(0)), ln(head.stride(0)), _lib.ptr(tgt[part]),
-                              step, _lib.ptr(pmax), _lib.ptr(psum), _lib.ptr(tlogit[part]), None, ln(0), ln(0), ctypes.c_uint(0), None,
-                              ln(0), ln(0), ctypes.c_uint(0), 0, 0, _lib.ptr(slab), ln(vocab), _lib.stream_ptr())
+        ids = p(tgt.data_ptr() + 4 * step * start)
+        code = L.ctb_ce_stats_step(_lib.ptr(h), _lib.ptr(head), n, vocab, d, ln(h.stride(0)), ln(head.stride(0)), ids,
+                                   step, p(work.pmax), p(work.psum), p(work.tlogit + 4 * start), None, ln(0), ln(0),
+                                   ctypes.c_uint(0), None, ln(0), ln(0), ctypes.c_uint(0), 0, 0, _lib.ptr(slab), ln(vocab),
+                                   _lib.stream_ptr())
         _lib.check(code, "ctb_ce_stats")
-        _combine(L, pmax, psum, slabs, tlogit[part], tgt[part], step, vocab, w[part], scale, device_scale, lse[part], coef[part],
-                 bn[blocks], bw[blocks], n)
-        code = L.ctb_kept_logits_gradient(_lib.ptr(slab), ln(vocab), n, vocab, _lib.ptr(tgt[part]), step, _lib.ptr(lse[part]),
-                                          _lib.ptr(coef[part]), _lib.stream_ptr())
+        _combine(L, work, slabs, tgt, step, vocab, w, scale, device_scale, work.lse, work.coef, start, n)
+        code = L.ctb_kept_logits_gradient(_lib.ptr(slab), ln(vocab), n, vocab, ids, step, p(work.lse + 4 * start),
+                                          p(work.coef + 4 * start), _lib.stream_ptr())
         _lib.check(code, "ctb_kept_logits_gradient")
         g = slab.view(torch.bfloat16)[:n, :vocab]
         gemm(g, head, b_mn=True, out=dhidden[part])                                                    # dH = G @ W
         if need_dhead:
             gemm(g, h, a_mn=True, b_mn=True, out=dhead, accumulate=dhead_accumulate or start > 0)       # dW += G^T H
-    return *_sums(L, bn, bw), dhidden, dhead
+    return *_sums(L, work, rows), dhidden, dhead
 
 
 def logits_ce_forward_backward(hidden, head, targets, weights, grad_scale: float = 1.0, *, chunk_rows: int = 4096,
