@@ -405,15 +405,58 @@ __global__ void rope_table_kernel(const int* __restrict__ pos, const float* __re
 // SwiGLU on the packed projection gu[T][2f] = [gate | up]:  h = silu(gate) * up.
 // Backward writes d(gate|up) in the same packed layout.
 // ------------------------------------------------------------------------------------------
-// sigmoid(x) = 1 / (1 + e) for x >= 0 and e / (1 + e) below, e = exp(-|x|): the denominator stays in (1, 2], where the
-// reciprocal needs no care for range, and nothing overflows, so gates below -88.7 keep what is left of their activation.
-// One Newton step brings the approximate reciprocal to half an ulp (and a little).  The IEEE quotient x / (1 + exp(-x)),
-// which this replaces, bound the forward kernel by its instructions (279 us at 16384 x 14336); a fast division returns zero
-// for denominators above 2^126, gates between -88.7 and -87.4.
-__device__ __forceinline__ float reciprocal_1_to_2(float d) {
+// n / d for d = 1 + exp(-g), g below 87 in size, and finite n: an approximate reciprocal, a Newton step, and the quotient corrected
+// by its own remainder, which rounds it correctly (for every bf16 gate the bits of the IEEE division, but for the sign of a
+// zero) without that division's range reduction.  The division bound the forward kernel by its instructions (279 us at 16384 x
+// 14336); a fast one returns zero for denominators above 2^126, gates between -88.7 and -87.4.  A vector with a larger gate
+// divides, in a function of its own: inlined it costs the others their registers (260 us).
+__device__ __forceinline__ float quotient_in_range(float n, float d) {
   float r;
   asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(d));
-  return fmaf(r, fmaf(-d, r, 1.f), r);
+  r = fmaf(r, fmaf(-d, r, 1.f), r);
+  const float q = n * r;
+  return fmaf(fmaf(-q, d, n), r, q);
+}
+// Whether all eight gates are below 87 (0x42ae) in size, as bf16 bit patterns.
+__device__ __forceinline__ bool gates_in_range(const uint4& gates) {
+  const unsigned m = __vmaxu2(__vmaxu2(gates.x & 0x7fff7fffu, gates.y & 0x7fff7fffu),
+                              __vmaxu2(gates.z & 0x7fff7fffu, gates.w & 0x7fff7fffu));
+  return (m & 0xffffu) < 0x42aeu && (m >> 16) < 0x42aeu;
+}
+template <bool PLAIN>
+__device__ __forceinline__ uint4 swiglu_vector(const uint4& gates, const uint4& ups) {
+  float g[8], u[8], o[8];
+  unpack8(gates, g);
+  unpack8(ups, u);
+#pragma unroll
+  for (int e = 0; e < 8; ++e) {
+    const float d = 1.f + __expf(-g[e]);
+    o[e] = __bfloat162float(__float2bfloat16(PLAIN ? quotient_in_range(g[e], d) : g[e] / d)) * u[e];
+  }
+  return pack8(o);
+}
+struct GateUp {
+  uint4 gate, up;
+};
+template <bool PLAIN>
+__device__ __forceinline__ GateUp swiglu_gradient(const uint4& gates, const uint4& ups, const uint4& grads) {
+  float g[8], u[8], d[8], dg[8], du[8];
+  unpack8(gates, g);
+  unpack8(ups, u);
+  unpack8(grads, d);
+#pragma unroll
+  for (int e = 0; e < 8; ++e) {
+    const float den = 1.f + __expf(-g[e]);
+    const float sg = PLAIN ? quotient_in_range(1.f, den) : 1.f / den;
+    const float act = g[e] * sg;
+    du[e] = d[e] * act;
+    dg[e] = d[e] * u[e] * sg * (1.f + g[e] * (1.f - sg));
+  }
+  return {pack8(dg), pack8(du)};
+}
+__device__ __noinline__ uint4 swiglu_vector_of_any(uint4 gates, uint4 ups) { return swiglu_vector<false>(gates, ups); }
+__device__ __noinline__ GateUp swiglu_gradient_of_any(uint4 gates, uint4 ups, uint4 grads) {
+  return swiglu_gradient<false>(gates, ups, grads);
 }
 
 // A thread takes every gridDim * blockDim-th 16-byte vector of h and steps its row along instead of dividing for
@@ -467,16 +510,8 @@ swiglu_fwd_kernel(const __nv_bfloat16* __restrict__ gu, __nv_bfloat16* __restric
 #pragma unroll
     for (int k = 0; k < AHEAD; ++k)
       if (to[k] < w.total) {
-        float g[8], u[8], o[8];
-        unpack8(gv[k], g);
-        unpack8(uv[k], u);
-#pragma unroll
-        for (int e = 0; e < 8; ++e) {
-          const float x = __expf(-fabsf(g[e]));
-          const float act = __bfloat162float(__float2bfloat16((g[e] < 0.f ? g[e] * x : g[e]) * reciprocal_1_to_2(1.f + x)));
-          o[e] = act * u[e];
-        }
-        reinterpret_cast<uint4*>(h)[to[k]] = pack8(o);
+        reinterpret_cast<uint4*>(h)[to[k]] =
+            gates_in_range(gv[k]) ? swiglu_vector<true>(gv[k], uv[k]) : swiglu_vector_of_any(gv[k], uv[k]);
       }
   }
 }
@@ -490,20 +525,9 @@ swiglu_bwd_kernel(const __nv_bfloat16* __restrict__ gu, const __nv_bfloat16* __r
   for (SwigluWalk w(T, f); w.i < w.total; w.step()) {
     const long at = w.i + w.row_at;
     const uint4 gv = src[at], uv = src[at + w.nvec], dv = reinterpret_cast<const uint4*>(dh)[w.i];
-    float g[8], u[8], d[8], dg[8], du[8];
-    unpack8(gv, g);
-    unpack8(uv, u);
-    unpack8(dv, d);
-#pragma unroll
-    for (int e = 0; e < 8; ++e) {
-      const float x = __expf(-fabsf(g[e]));
-      const float sg = (g[e] < 0.f ? x : 1.f) * reciprocal_1_to_2(1.f + x);
-      const float act = g[e] * sg;
-      du[e] = d[e] * act;
-      dg[e] = d[e] * u[e] * sg * (1.f + g[e] * (1.f - sg));
-    }
-    dst[at] = pack8(dg);
-    dst[at + w.nvec] = pack8(du);
+    const GateUp r = gates_in_range(gv) ? swiglu_gradient<true>(gv, uv, dv) : swiglu_gradient_of_any(gv, uv, dv);
+    dst[at] = r.gate;
+    dst[at + w.nvec] = r.up;
   }
 }
 
@@ -1253,11 +1277,10 @@ CTB_API int ctb_rope(void* x, const float* cosv, const float* sinv, long row_str
   return 0;
 }
 
-// Calls that move more than L2 holds (126 MB) stream through HBM, and there the backward kernel's two reads of a row, one of
-// dh and two writes go best with half the threads an SM can hold, the forward kernel's with twice as many blocks as fit at
-// once.  Blocks an SM, us: backward 16384 x 14336 2: 493, 4: 362 (6.5 TB/s), 6: 426, 8: 427, 16: 388; 8192 x 8960 4: 116, 8: 134;
-// out of L2 1000 x 8960 4: 13.0, 8: 11.9; 3000 x 3584 17.7 and 15.4.  Forward 16384 x 14336 4: 225, 8: 232, 16: 221 (6.4 TB/s).
-// Before, with the quotient, 388 and 278 us.
+// Blocks an SM.  Calls that move more than L2 holds (126 MB) stream through HBM and go best with several times as many blocks as
+// fit at once, backward 24 (us: 16384 x 14336 8: 398, 16: 374, 24: 363 (6.5 TB/s); 8192 x 8960 122, 116, 111), forward 16 (8: 234,
+// 16: 231 (6.1 TB/s); 8192 x 8960 79 and 77); others lose by it (1000 x 8960 backward 8: 12.6, 24: 13.3).  Before, with the
+// quotient and 8 blocks, 388 and 278 us.
 constexpr long SWIGLU_STREAMED = 128l << 20;
 CTB_API int ctb_swiglu_fwd(const void* gu, void* h, long T, int f, void* stream) {
   if (f % 8) return fail("swiglu: intermediate size must be a multiple of 8");
@@ -1274,7 +1297,7 @@ CTB_API int ctb_swiglu_bwd(const void* gu, const void* dh, void* dgu, long T, in
   if (f % 8) return fail("swiglu: intermediate size must be a multiple of 8");
   if (T <= 0 || f <= 0) return 0;
   CTB_CUDA_OK(launch_chained(10 * T * f <= CHAINED_BYTES, swiglu_bwd_kernel,
-                             grid_for(T * (f / 8), 256, 10 * T * f > SWIGLU_STREAMED ? 4 : 8), 256, 0, stream, 0,
+                             grid_for(T * (f / 8), 256, 10 * T * f > SWIGLU_STREAMED ? 24 : 8), 256, 0, stream, 0,
                              static_cast<const __nv_bfloat16*>(gu), static_cast<const __nv_bfloat16*>(dh),
                              static_cast<__nv_bfloat16*>(dgu), T, f));
   return 0;

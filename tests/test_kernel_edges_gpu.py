@@ -165,21 +165,22 @@ def test_swiglu_of_large_negative_gates(cuda_lib):
 
 @pytest.mark.parametrize("t", [1497, 1499, 2496, 2497, 4099])      # 128 MiB of traffic: backward above 1497 rows, forward above 2496
 def test_swiglu_grids_beyond_l2(cuda_lib, t):
-    """Calls on both sides of the sizes where the grids change; gates down to where exp(gate) leaves the normal range."""
+    """Calls on both sides of the sizes where the grids change; vectors with gates whose exponential leaves the range of the short
+    division beside others (below -88.7 it is infinite in fp32 and the result zero, as in the long one)."""
     from causal_trainer_dev_b200.ops import elementwise as E
 
     f = 8960
     gu, dh = _bf16(t, 2 * f, seed=t, scale=4.0), _bf16(t, f, seed=2)
-    gu[-1, :40] = -torch.arange(80, 120).bfloat16()
+    gu[-1, :40:2] = -torch.arange(70, 90).bfloat16()
+    gu[-1, f:f + 40] = 3.0                                   # (products that bf16 holds to its full precision)
     gd = gu.double().requires_grad_()
     want = torch.nn.functional.silu(gd[:, :f]) * gd[:, f:]
     want.backward(dh.double())
     got, dgu = E.swiglu_forward(gu), E.swiglu_backward(gu, dh)
     assert _rel(got, want) < 2 * BF16 and _rel(dgu, gd.grad) < BF16
-    # exp(-102) has 2 bits left in fp32, and below 1e-40 so has bf16
-    small = (want[-1, :40].abs() > 1e-36) | (want[-1, :40] == 0)
+    # element by element, where the gate is above -88.7: silu is rounded before the product, __expf is off by 1.3e-5 at 88
     near = (got[-1, :40].double() - want[-1, :40]).abs() <= (2 * BF16 + 2e-5) * want[-1, :40].abs()
-    assert bool((near | ~small).all()) and not bool(got.isnan().any()) and not bool(dgu.isnan().any())
+    assert bool((near | (gu[-1, :40] < -88.6)).all()) and not bool(got.isnan().any()) and not bool(dgu.isnan().any())
 
 
 @pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float32])
