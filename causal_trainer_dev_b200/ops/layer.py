@@ -78,7 +78,10 @@ class LayerCalls:
 
     @property
     def scratch_bytes(self) -> int:
-        return max(self._forward, self._backward)
+        """Of the larger call, without the partial sums of dK / dV: they take their time from the device's, not from the host's."""
+        s = self._shape
+        sums = _lib.lib().ctb_attn_bwd_workspace(s.batch, s.seq, s.seq, s.q_heads, s.kv_heads, s.head_dim)
+        return max(self._forward, self._backward - sums)
 
     def forward(self, unit, resid: torch.Tensor, branch: torch.Tensor | None) -> tuple[torch.Tensor, torch.Tensor, tuple]:
         """Returns (h, mlp, what :meth:`backward` needs)."""
