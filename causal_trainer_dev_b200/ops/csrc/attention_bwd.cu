@@ -116,7 +116,9 @@ __device__ __forceinline__ void dkv_queries(const BwdArgs& args, int b, int kb, 
   count = qhi > qlo ? (qhi + 63) / 64 - first : 0;
 }
 
-template <int MODE>
+// (PARTS here and below: the launch has several work items per key tile.  A kernel of its own, because what it adds to the loops and
+// the epilogue costs a long call half a percent)
+template <int MODE, bool PARTS>
 __device__ __forceinline__ BwdItem bwd_item(const BwdArgs& args, const int cta) {
   constexpr bool DKV = (MODE == MODE_DKV);
   const int group = args.Hq / args.Hkv;
@@ -143,7 +145,7 @@ __device__ __forceinline__ BwdItem bwd_item(const BwdArgs& args, const int cta) 
     if (gd.w <= 0) w.mode = -2;                        // unused capacity: nothing is written
     return w;
   }
-  int idx = DKV && args.parts > 1 ? cta / args.parts : cta;
+  int idx = DKV && PARTS ? cta / args.parts : cta;
   if (DKV) {
     w.head = idx % args.Hkv;      // kv head
     idx /= args.Hkv;
@@ -153,7 +155,7 @@ __device__ __forceinline__ BwdItem bwd_item(const BwdArgs& args, const int cta) 
     dkv_queries(args, w.b, kb, w.y_lo64, w.y_n64);
     w.n_entry = w.y_n64 * group;
     w.hkv = w.head;
-    if (args.parts > 1) {
+    if (PARTS) {
       // whole iterations (two entries) to every part that has work
       const int part = cta % args.parts, used = dkv_parts_used(args, w.n_entry), all = w.n_entry;
       if (part >= used) w.mode = -2;
@@ -182,11 +184,11 @@ __device__ __forceinline__ BwdItem bwd_item(const BwdArgs& args, const int cta) 
 
 // entry -> (64-row block of the streamed operand, query head).  Iteration i holds entries 2i and
 // 2i + 1 in the two halves of its tile; an odd last half repeats the last entry, fully masked.
-template <int MODE>
+template <int MODE, bool PARTS>
 __device__ __forceinline__ void bwd_entry(const BwdArgs& args, const BwdItem& w, int e, int& block, int& head) {
   const bool sparse = args.sp.it_list != nullptr;
   const int entry = sparse ? __ldg(args.sp.it_list + w.list + e) : 0;
-  e += w.first;
+  if (PARTS) e += w.first;
   block = sparse ? (entry & 0xffffff) : w.y_lo64 + e % w.y_n64;
   if (args.grp.desc != nullptr) head = 0;
   else if (MODE == MODE_DQ) head = w.head;
@@ -250,7 +252,7 @@ __device__ __forceinline__ void bwd_load_x(uint32_t on, const BwdShared& sh, con
 // ------------------------------ producer ------------------------------
 // The streamed tiles of an item, then the ring slots that its epilogue stages its results in: a slot whose full barrier
 // completes without a copy belongs to the epilogue, which frees it when the results have left.
-template <int D, int MODE>
+template <int D, int MODE, bool PARTS>
 __device__ __forceinline__ bool bwd_produce(uint32_t on, const BwdShared& sh, const BwdMaps& maps, const BwdArgs& args,
                                             const BwdItem& w, BwdWalk& at) {
   using L = BwdSmem<D>;
@@ -266,7 +268,7 @@ __device__ __forceinline__ bool bwd_produce(uint32_t on, const BwdShared& sh, co
 #pragma unroll
     for (int q = 0; q < 2; ++q) {              // the two 64-row halves of the tile
       int block;
-      bwd_entry<MODE>(args, w, min(2 * it + q, w.n_entry - 1), block, yh[q]);
+      bwd_entry<MODE, PARTS>(args, w, min(2 * it + q, w.n_entry - 1), block, yh[q]);
       if (!DKV) yh[q] = w.hkv;
       y0[q] = w.y_base + block * 64 - (DKV ? args.q_off : 0);   // streamed queries are stored locally
       stat[q] = grouped ? static_cast<size_t>(y0[q])
@@ -406,7 +408,7 @@ __device__ __forceinline__ bool bwd_issue(uint32_t on, const BwdShared& sh, cons
 // ------------------------------ compute warpgroups ------------------------------
 // Four compute warpgroups work on every iteration together: warpgroup wg takes columns
 // [32 wg, 32 wg + 32) of the tile, i.e. 32 columns of entry 2 it + wg / 2.
-template <int D, int MODE>
+template <int D, int MODE, bool PARTS>
 __device__ __forceinline__ bool bwd_compute(const BwdShared& sh, const BwdMaps& maps, const BwdArgs& args, const BwdItem& w,
                                             BwdWalk& at) {
   using L = BwdSmem<D>;
@@ -461,7 +463,7 @@ __device__ __forceinline__ bool bwd_compute(const BwdShared& sh, const BwdMaps& 
       ++walk_head;
     }
   };
-  if (!sparse && n_entry > 0) advance(w.first + mine);
+  if (!sparse && n_entry > 0) advance(PARTS ? w.first + mine : mine);
   for (int it = 0; it < n_iter; ++it) {
     const int entry_at = 2 * it + mine;
     const bool real = entry_at < n_entry;
@@ -641,7 +643,7 @@ __device__ __forceinline__ bool bwd_compute(const BwdShared& sh, const BwdMaps& 
     ok = mbar_wait_warp(u == 0 ? &sh.y1_full[slot] : &sh.y2_full[slot], u == 0 ? at.y1_phase : at.y2_phase(), sh.abort_flag,
                         sh.st, SITE_B_CW_ACC, sh.budget);
   const bool any_bad = named_bar_or(2 + u, 256, !ok);
-  if (!any_bad && DKV && args.parts > 1 && w.list >= 0) {
+  if (!any_bad && DKV && PARTS && w.list >= 0) {
     // one of several work items of its key tile: fp32, as the accumulators hold them, 512 bytes of 32 keys at a time
     float4* to = reinterpret_cast<float4*>(args.partial) + (static_cast<size_t>(w.list) * 2 + u) * (D / 4) * 128 + r;
     const uint32_t acc = sh.tmem_base + (u == 1 ? T::ACC2 : T::ACC1);
@@ -765,7 +767,7 @@ __global__ void __launch_bounds__(128) attn_bwd_sum_kernel(const BwdArgs args, _
 // its start, its first copies and its last stores one after the other (about 7000 cycles, a quarter of the dQ item of a
 // packed row).  The next item is requested when the last copies of the current one are issued, not earlier: an item
 // that waits behind a long one could have run elsewhere.
-template <int D, int MODES>
+template <int D, int MODES, bool PARTS>
 __global__ void __launch_bounds__(BWD_THREADS, 1)
 attn_bwd_kernel(const __grid_constant__ BwdMaps dkv_maps, const __grid_constant__ BwdMaps dq_maps,
                 const __grid_constant__ BwdArgs dkv, const __grid_constant__ BwdArgs dq, const int dkv_items) {
@@ -804,8 +806,8 @@ attn_bwd_kernel(const __grid_constant__ BwdMaps dkv_maps, const __grid_constant_
   const int lane = threadIdx.x & 31;
 
   auto resolve = [&](int cta) -> BwdItem {
-    if (MODES == MODE_DKV || (MODES == MODE_BOTH && cta < dkv_items)) return bwd_item<MODE_DKV>(dkv, cta);
-    return bwd_item<MODE_DQ>(dq, MODES == MODE_BOTH ? cta - dkv_items : cta);
+    if (MODES == MODE_DKV || (MODES == MODE_BOTH && cta < dkv_items)) return bwd_item<MODE_DKV, PARTS>(dkv, cta);
+    return bwd_item<MODE_DQ, false>(dq, MODES == MODE_BOTH ? cta - dkv_items : cta);
   };
   BwdItem w;
   if (threadIdx.x < 32) {
@@ -897,8 +899,8 @@ attn_bwd_kernel(const __grid_constant__ BwdMaps dkv_maps, const __grid_constant_
           }
           ++at.items;
         }
-        if (MODES != MODE_DQ && w.mode == MODE_DKV) ok = bwd_produce<D, MODE_DKV>(on, sh, dkv_maps, dkv, w, at);
-        else if (MODES != MODE_DKV) ok = bwd_produce<D, MODE_DQ>(on, sh, dq_maps, dq, w, at);
+        if (MODES != MODE_DQ && w.mode == MODE_DKV) ok = bwd_produce<D, MODE_DKV, PARTS>(on, sh, dkv_maps, dkv, w, at);
+        else if (MODES != MODE_DKV) ok = bwd_produce<D, MODE_DQ, false>(on, sh, dq_maps, dq, w, at);
         if (!ok) break;
       }
       loaded = false;
@@ -938,8 +940,8 @@ attn_bwd_kernel(const __grid_constant__ BwdMaps dkv_maps, const __grid_constant_
         break;
       }
       bool ok = true;
-      if (MODES != MODE_DQ && w.mode == MODE_DKV) ok = bwd_compute<D, MODE_DKV>(sh, dkv_maps, dkv, w, at);
-      else if (MODES != MODE_DKV) ok = bwd_compute<D, MODE_DQ>(sh, dq_maps, dq, w, at);
+      if (MODES != MODE_DQ && w.mode == MODE_DKV) ok = bwd_compute<D, MODE_DKV, PARTS>(sh, dkv_maps, dkv, w, at);
+      else if (MODES != MODE_DKV) ok = bwd_compute<D, MODE_DQ, false>(sh, dq_maps, dq, w, at);
       if (!ok) break;
     }
     tma_wait_group<0>();
@@ -1000,12 +1002,12 @@ int prepare_bwd(const BwdCall& c, BwdMaps* maps, BwdArgs* args, int* items) {
   return 0;
 }
 
-template <int D, int MODES>
-int launch_items(const BwdMaps& dkv_maps, const BwdMaps& dq_maps, const BwdArgs& dkv, const BwdArgs& dq, int dkv_items,
+template <int D, int MODES, bool PARTS>
+int launch_items_as(const BwdMaps& dkv_maps, const BwdMaps& dq_maps, const BwdArgs& dkv, const BwdArgs& dq, int dkv_items,
                  int dq_items, void* stream) {
   const int items = max(dkv_items, 0) + max(dq_items, 0);
   if (items == 0) return 0;
-  auto kern = attn_bwd_kernel<D, MODES>;
+  auto kern = attn_bwd_kernel<D, MODES, PARTS>;
   static int configured_dev = -1;
   int dev = 0;
   cudaGetDevice(&dev);
@@ -1016,6 +1018,14 @@ int launch_items(const BwdMaps& dkv_maps, const BwdMaps& dq_maps, const BwdArgs&
   CTB_CUDA_OK(launch_chained((MODES == MODE_DQ ? dq : dkv).chained != 0, kern, items, BWD_THREADS, BwdSmem<D>::BYTES, stream, 0,
                              dkv_maps, dq_maps, dkv, dq, max(dkv_items, 0)));
   return 0;
+}
+
+template <int D, int MODES>
+int launch_items(const BwdMaps& dkv_maps, const BwdMaps& dq_maps, const BwdArgs& dkv, const BwdArgs& dq, int dkv_items,
+                 int dq_items, void* stream) {
+  if (MODES != MODE_DQ && dkv.parts > 1)
+    return launch_items_as<D, MODES == MODE_DQ ? MODE_DKV : MODES, true>(dkv_maps, dq_maps, dkv, dq, dkv_items, dq_items, stream);
+  return launch_items_as<D, MODES, false>(dkv_maps, dq_maps, dkv, dq, dkv_items, dq_items, stream);
 }
 
 template <int D, int MODE>
