@@ -721,14 +721,14 @@ __device__ __forceinline__ bool bwd_compute(const BwdShared& sh, const BwdMaps& 
 }
 
 // dK and dV of key tiles that several work items share: the sums of their parts in the order of the parts (so the same bits
-// whatever the timing), scaled and rounded once.  A block takes 32 channels of one gradient of one tile, a thread one key.
+// whatever the timing), scaled and rounded once.  A block takes 16 channels of one gradient of one tile, a thread one key.
 // Bound by the reads, out of L2.
 template <int D>
 __global__ void __launch_bounds__(128) attn_bwd_sum_kernel(const BwdArgs args, __nv_bfloat16* __restrict__ dk, long dk_rs,
                                                            __nv_bfloat16* __restrict__ dv, long dv_rs) {
   let_successor_start();
   wait_for_predecessor();
-  constexpr int CHUNKS = D / 32;
+  constexpr int CHUNKS = D / 16;
   const int chunk = blockIdx.x % CHUNKS, u = blockIdx.x / CHUNKS % 2, item = blockIdx.x / (2 * CHUNKS), r = threadIdx.x;
   const int head = item % args.Hkv, b = item / args.Hkv % args.B, kb = item / args.Hkv / args.B;
   int first, count;
@@ -736,14 +736,15 @@ __global__ void __launch_bounds__(128) attn_bwd_sum_kernel(const BwdArgs args, _
   const int used = dkv_parts_used(args, count * (args.Hq / args.Hkv));
   if (used == 1) return;                     // stored by its one work item
   const float4* from = reinterpret_cast<const float4*>(args.partial) +
-                       (static_cast<size_t>(item) * args.parts * 2 + u) * (D / 4) * 128 + chunk * 8 * 128 + r;
-  float4 sum[8];
+                       (static_cast<size_t>(item) * args.parts * 2 + u) * (D / 4) * 128 + chunk * 4 * 128 + r;
+  float4 sum[4];
 #pragma unroll
-  for (int j = 0; j < 8; ++j) sum[j] = __ldcs(from + j * 128);
+  for (int j = 0; j < 4; ++j) sum[j] = __ldcs(from + j * 128);
+#pragma unroll 4
   for (int p = 1; p < used; ++p) {
     from += 2 * (D / 4) * 128;
 #pragma unroll
-    for (int j = 0; j < 8; ++j) {
+    for (int j = 0; j < 4; ++j) {
       const float4 v = __ldcs(from + j * 128);
       sum[j].x += v.x;
       sum[j].y += v.y;
@@ -753,9 +754,9 @@ __global__ void __launch_bounds__(128) attn_bwd_sum_kernel(const BwdArgs args, _
   }
   const float mul = u == 0 ? 1.f : args.scale;
   uint4* to = reinterpret_cast<uint4*>((u == 0 ? dv : dk) + (static_cast<long>(b) * args.S + kb * 128 + r) * (u == 0 ? dv_rs : dk_rs) +
-                                       head * D + chunk * 32);
+                                       head * D + chunk * 16);
 #pragma unroll
-  for (int j = 0; j < 8; j += 2)
+  for (int j = 0; j < 4; j += 2)
     to[j / 2] = make_uint4(pack_bf16(sum[j].x * mul, sum[j].y * mul), pack_bf16(sum[j].z * mul, sum[j].w * mul),
                            pack_bf16(sum[j + 1].x * mul, sum[j + 1].y * mul), pack_bf16(sum[j + 1].z * mul, sum[j + 1].w * mul));
 }
@@ -1085,7 +1086,7 @@ int launch_bwd_dense(const BwdCall& c) {
   a.parts = c.parts;
   a.partial = c.partial;
   CTB_CUDA_OK(launch_chained(chained_rows(static_cast<long>(c.B) * c.Sq, c.Hq, D), attn_bwd_sum_kernel<D>,
-                             c.B * c.Hkv * (c.S / 128) * 2 * (D / 32), 128, 0, c.stream, 0, a,
+                             c.B * c.Hkv * (c.S / 128) * 2 * (D / 16), 128, 0, c.stream, 0, a,
                              static_cast<__nv_bfloat16*>(c.dk), c.dk_row_stride, static_cast<__nv_bfloat16*>(c.dv),
                              c.dv_row_stride));
   return 0;
