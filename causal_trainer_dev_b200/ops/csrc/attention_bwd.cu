@@ -103,9 +103,10 @@ struct alignas(16) BwdItem {
 };
 static_assert(sizeof(BwdItem) == 48, "three 16-byte reads");
 
-// Of the `parts` work items that a launch has for a key tile, as many have work as leave each eight iterations (two entries
-// each); one alone stores its results as if there were no others.
-__device__ __forceinline__ int dkv_parts_used(const BwdArgs& args, int n_entry) { return max(1, min(args.parts, n_entry / 16)); }
+// Of the `parts` work items that a launch has for a key tile, as many have work as leave each two iterations (two entries
+// each); one alone stores its results as if there were no others.  (us, with eight, four and two iterations: 512 tokens 8 / 2
+// heads 26.7, 17.6, 17.5; 2 x 512 12 / 2 31.7, 25.6, 23.1; 1024 12 / 2 in documents of 200 34.9, 23.5, 22.5.)
+__device__ __forceinline__ int dkv_parts_used(const BwdArgs& args, int n_entry) { return max(1, min(args.parts, n_entry / 4)); }
 
 // The 64-row query blocks that see the key tile kb of row b: [first, first + count).  Only the queries this rank holds,
 // [q_off, q_off + Sq), are walked.
@@ -1096,8 +1097,9 @@ int launch_bwd_dense(const BwdCall& c) {
 // key tiles (short rows, few kv heads) ends with a few SMs on the long ones of them: one row of 2048 tokens, 14 / 2 heads, has 32,
 // and the longest is 112 iterations where an SM has 29 of the whole call.  The estimate (cycles) takes the rows for whole
 // documents: an iteration of dK/dV 2615 and of dQ 2047, the start and end of an item 10000 and 8000, of a further part with its
-// fp32 tiles 12000, the sum of the parts 8000.  Rows of short documents then lose little, because a part without eight
-// iterations of its own has no work.
+// fp32 tiles 12000, the sum of the parts 8000.  Rows of short documents lose little by that, because a part without two
+// iterations of its own has no work (4 rows of 512 in documents of 128, 8 / 2 heads, 18.3 us uncut, 22.1; of 1024 in documents of 200, 12 /
+// 2 heads, 32.5 and 22.5).
 inline int dkv_parts(int B, int S, int Sq, int Hq, int Hkv) {
   const double tiles = static_cast<double>(B) * Hkv * (S / 128), rows = static_cast<double>(B) * Hq * (Sq / 128);
   const double longest = static_cast<double>(Hq / Hkv) * (Sq / 128), seen = (Sq / 128 + 1) / 2.;
@@ -1105,7 +1107,7 @@ inline int dkv_parts(int B, int S, int Sq, int Hq, int Hkv) {
   const double whole = max(longest * 2615 + 10000, all / sms);
   int best = 1;
   double least = 0.83 * whole;
-  for (int p = 2; p <= 8 && longest >= 8 * p; ++p) {
+  for (int p = 2; p <= 16 && longest >= 2 * p; ++p) {
     const double t = max(longest / p * 2615 + 10000, (all + tiles * (p - 1) * 12000) / sms) + 8000;
     if (t < least) {
       least = t;

@@ -20,7 +20,7 @@ def _segments(kind, b, s):
     at = torch.arange(s).repeat(b, 1)
     if kind == "one":
         seg = torch.ones(b, s)
-    elif kind == "short":                       # no tile has enough queries for two items
+    elif kind == "short":                       # a tile sees two or three 64-row blocks a head
         seg = at // 40 + 1
     elif kind == "uneven":                      # tiles with one, with several and with the most items, odd numbers of blocks
         seg = (at >= 70).int() + (at >= 200).int() + (at >= 3 * s // 4 - 9).int() + 1
@@ -30,7 +30,7 @@ def _segments(kind, b, s):
 
 
 @pytest.mark.parametrize("kind", ["one", "short", "uneven", "padded"])
-@pytest.mark.parametrize("b,s,hq,hkv,d", [(1, 1152, 14, 2, 128), (1, 2048, 4, 1, 64), (2, 640, 12, 2, 128)])
+@pytest.mark.parametrize("b,s,hq,hkv,d", [(1, 1152, 14, 2, 128), (1, 2048, 4, 1, 64), (2, 640, 12, 2, 128), (1, 1024, 2, 1, 64)])
 def test_key_tiles_in_parts(cuda_lib, monkeypatch, kind, b, s, hq, hkv, d):
     from causal_trainer_dev_b200.ops import attention as A
 
@@ -68,8 +68,8 @@ def test_key_tiles_in_parts(cuda_lib, monkeypatch, kind, b, s, hq, hkv, d):
     assert torch.equal(first[0], whole[0]) and torch.equal(part[0], whole_part[0])
     for got, want in ((first[1], whole[1]), (first[2], whole[2]), (part[1], whole_part[1]), (part[2], whole_part[2])):
         assert _rel(got, want) < 2 * BF16           # two roundings to bf16 of sums in another order
-        if kind == "short":
-            assert torch.equal(got, want)           # one item a tile, whatever the launch has room for
+        if kind == "short" and hq == 2 * hkv:       # at most three blocks a head: less than two items' work
+            assert torch.equal(got, want)
     group, i = hq // hkv, b - 1
     qd, kd, vd = (t[i].double().requires_grad_() for t in (q, k, v))
     score = torch.einsum("qhd,khd->hqk", qd, kd.repeat_interleave(group, 1)) / math.sqrt(d)
