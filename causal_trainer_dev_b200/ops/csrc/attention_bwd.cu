@@ -736,17 +736,17 @@ __global__ void __launch_bounds__(128) attn_bwd_sum_kernel(const BwdArgs args, _
   dkv_queries(args, b, kb, first, count);
   const int used = dkv_parts_used(args, count * (args.Hq / args.Hkv));
   if (used == 1) return;                     // stored by its one work item
-  const float4* from = reinterpret_cast<const float4*>(args.partial) +
-                       (static_cast<size_t>(item) * args.parts * 2 + u) * (D / 4) * 128 + chunk * 4 * 128 + r;
+  const float* from = args.partial +
+                      ((static_cast<size_t>(item) * args.parts * 2 + u) * (D / 4) * 128 + chunk * 4 * 128 + r) * 4;
   float4 sum[4];
 #pragma unroll
-  for (int j = 0; j < 4; ++j) sum[j] = __ldcs(from + j * 128);
+  for (int j = 0; j < 4; ++j) sum[j] = load_streamed(from + j * 512);
 #pragma unroll 4
   for (int p = 1; p < used; ++p) {
-    from += 2 * (D / 4) * 128;
+    from += 2 * D * 128;
 #pragma unroll
     for (int j = 0; j < 4; ++j) {
-      const float4 v = __ldcs(from + j * 128);
+      const float4 v = load_streamed(from + j * 512);
       sum[j].x += v.x;
       sum[j].y += v.y;
       sum[j].z += v.z;

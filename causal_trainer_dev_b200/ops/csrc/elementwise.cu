@@ -64,8 +64,8 @@ __device__ __forceinline__ float block_sum(float v, float* scratch) {
 // ------------------------------------------------------------------------------------------
 template <int NV>
 __global__ void __launch_bounds__(NORM_THREADS)
-rmsnorm_fwd_kernel(const __nv_bfloat16* __restrict__ x, const __nv_bfloat16* __restrict__ residual,
-                   const __nv_bfloat16* __restrict__ w, __nv_bfloat16* __restrict__ y,
+rmsnorm_fwd_kernel(const __nv_bfloat16* x, const __nv_bfloat16* residual,
+                   const __nv_bfloat16* w, __nv_bfloat16* __restrict__ y,
                    __nv_bfloat16* __restrict__ h_out, float* __restrict__ rstd_out, int rows, int d, float eps) {
   let_successor_start();
   wait_for_predecessor();
@@ -125,9 +125,9 @@ rmsnorm_fwd_kernel(const __nv_bfloat16* __restrict__ x, const __nv_bfloat16* __r
 // before and now: d = 4096 217 and 112; 8192, one CTA per SM for its 179 registers, 384 and 249; 16384 1297 and 832.
 template <int NV>
 __global__ void __launch_bounds__(NORM_THREADS)
-rmsnorm_bwd_kernel(const __nv_bfloat16* __restrict__ dy, const __nv_bfloat16* __restrict__ x,
-                   const __nv_bfloat16* __restrict__ w, const float* __restrict__ rstd,
-                   const __nv_bfloat16* __restrict__ dres, __nv_bfloat16* __restrict__ dx,
+rmsnorm_bwd_kernel(const __nv_bfloat16* dy, const __nv_bfloat16* x,
+                   const __nv_bfloat16* w, const float* rstd,
+                   const __nv_bfloat16* dres, __nv_bfloat16* __restrict__ dx,
                    float* __restrict__ dw_partial, int rows, int d) {
   let_successor_start();
   wait_for_predecessor();
@@ -183,7 +183,7 @@ rmsnorm_bwd_kernel(const __nv_bfloat16* __restrict__ dy, const __nv_bfloat16* __
       unpack8(dy_now[i], a);
       unpack8(x_now[i], b);
       const int v = threadIdx.x + i * NORM_THREADS;
-      unpack8(HOLD ? wv[i] : (v < nvec ? __ldg(reinterpret_cast<const uint4*>(w) + v) : zero), c);
+      unpack8(HOLD ? wv[i] : (v < nvec ? reinterpret_cast<const uint4*>(w)[v] : zero), c);
 #pragma unroll
       for (int e = 0; e < 8; ++e) {
         const float xh = b[e] * r_now;
@@ -205,7 +205,7 @@ rmsnorm_bwd_kernel(const __nv_bfloat16* __restrict__ dy, const __nv_bfloat16* __
         float a[8], b[8], c[8], r[8], o[8];
         unpack8(dy_now[i], a);
         unpack8(x_now[i], b);
-        unpack8(HOLD ? wv[i] : __ldg(reinterpret_cast<const uint4*>(w) + v), c);
+        unpack8(HOLD ? wv[i] : reinterpret_cast<const uint4*>(w)[v], c);
         if (!HOLD && dres) res_now[i] = reinterpret_cast<const uint4*>(dres)[static_cast<size_t>(row) * nvec + v];
         unpack8(res_now[i], r);
 #pragma unroll
@@ -232,7 +232,7 @@ rmsnorm_bwd_kernel(const __nv_bfloat16* __restrict__ dy, const __nv_bfloat16* __
 // 32 the whole backward norm of 512 x 256 takes 6.8 us for 4.8, of 1000 x 1536 9.1 for 7.3, of 8192 x 1536 29.0 for 27.0.
 constexpr int DW_WARPS = 32;
 __global__ void __launch_bounds__(DW_WARPS * 32)
-rmsnorm_dw_reduce_kernel(const float* __restrict__ partial, int parts, int d, void* __restrict__ dw, int out_f32,
+rmsnorm_dw_reduce_kernel(const float* partial, int parts, int d, void* __restrict__ dw, int out_f32,
                          int accumulate) {
   let_successor_start();
   wait_for_predecessor();
@@ -242,7 +242,7 @@ rmsnorm_dw_reduce_kernel(const float* __restrict__ partial, int parts, int d, vo
   float s = 0.f;
   if (c < d) {
 #pragma unroll 8
-    for (int p = warp; p < parts; p += DW_WARPS) s += __ldg(partial + static_cast<size_t>(p) * d + c);
+    for (int p = warp; p < parts; p += DW_WARPS) s += partial[static_cast<size_t>(p) * d + c];
   }
   sums[warp][lane] = s;
   __syncthreads();
@@ -263,7 +263,7 @@ rmsnorm_dw_reduce_kernel(const float* __restrict__ partial, int parts, int d, vo
 // rows a CTA and four in flight a warp; the cast to fp32 and the strided sum that did this wrote and read
 // twice the matrix in between.
 __global__ void __launch_bounds__(256)
-column_sum_kernel(const __nv_bfloat16* __restrict__ x, long ld, int rows, int n, float* __restrict__ partial) {
+column_sum_kernel(const __nv_bfloat16* x, long ld, int rows, int n, float* __restrict__ partial) {
   let_successor_start();
   wait_for_predecessor();
   __shared__ float sums[8][256 + 8];
@@ -276,7 +276,7 @@ column_sum_kernel(const __nv_bfloat16* __restrict__ x, long ld, int rows, int n,
 #pragma unroll 4
     for (int r = blockIdx.y * 8 + warp; r < rows; r += step) {
       float f[8];
-      unpack8(__ldg(reinterpret_cast<const uint4*>(x + static_cast<long>(r) * ld + c)), f);
+      unpack8(*reinterpret_cast<const uint4*>(x + static_cast<long>(r) * ld + c), f);
 #pragma unroll
       for (int e = 0; e < 8; ++e) acc[e] += f[e];
     }
@@ -300,8 +300,8 @@ column_sum_kernel(const __nv_bfloat16* __restrict__ x, long ld, int rows, int n,
 //   style 0 = gpt-j (adjacent pairs), 1 = gpt-neox (half split).  sign=-1 applies the
 //   inverse rotation (the backward pass).
 // ------------------------------------------------------------------------------------------
-__global__ void rope_kernel(__nv_bfloat16* __restrict__ x, const float* __restrict__ cosv,
-                            const float* __restrict__ sinv, long row_stride, int T, int heads, int D, int rot,
+__global__ void rope_kernel(__nv_bfloat16* __restrict__ x, const float* cosv,
+                            const float* sinv, long row_stride, int T, int heads, int D, int rot,
                             int style, float sign) {
   let_successor_start();
   wait_for_predecessor();
@@ -332,7 +332,7 @@ __global__ void rope_kernel(__nv_bfloat16* __restrict__ x, const float* __restri
 //   gpt-neox: a lane holds channels [8 p, 8 p + 8) of both halves;  gpt-j: four adjacent pairs.
 template <int STYLE, bool SHARED>
 __global__ void __launch_bounds__(256)
-rope_vec_kernel(__nv_bfloat16* __restrict__ x, const float* __restrict__ cosv, const float* __restrict__ sinv,
+rope_vec_kernel(__nv_bfloat16* __restrict__ x, const float* cosv, const float* sinv,
                 long row_stride, int T, int heads, int D, int rot, float sign, int share) {
   let_successor_start();
   wait_for_predecessor();
@@ -351,8 +351,8 @@ rope_vec_kernel(__nv_bfloat16* __restrict__ x, const float* __restrict__ cosv, c
     float c[N], s[N];
 #pragma unroll
     for (int e = 0; e < N; e += 4) {
-      *reinterpret_cast<float4*>(c + e) = __ldg(reinterpret_cast<const float4*>(cosv + t * half + p * N + e));
-      *reinterpret_cast<float4*>(s + e) = __ldg(reinterpret_cast<const float4*>(sinv + t * half + p * N + e));
+      *reinterpret_cast<float4*>(c + e) = *reinterpret_cast<const float4*>(cosv + t * half + p * N + e);
+      *reinterpret_cast<float4*>(s + e) = *reinterpret_cast<const float4*>(sinv + t * half + p * N + e);
     }
 #pragma unroll
     for (int e = 0; e < N; ++e) s[e] *= sign;
@@ -490,7 +490,7 @@ struct SwigluWalk {
 };
 template <int AHEAD>      // vectors in flight
 __global__ void __launch_bounds__(256)
-swiglu_fwd_kernel(const __nv_bfloat16* __restrict__ gu, __nv_bfloat16* __restrict__ h, long T, int f) {
+swiglu_fwd_kernel(const __nv_bfloat16* gu, __nv_bfloat16* __restrict__ h, long T, int f) {
   let_successor_start();
   wait_for_predecessor();
   const uint4* src = reinterpret_cast<const uint4*>(gu);
@@ -516,7 +516,7 @@ swiglu_fwd_kernel(const __nv_bfloat16* __restrict__ gu, __nv_bfloat16* __restric
   }
 }
 __global__ void __launch_bounds__(256)
-swiglu_bwd_kernel(const __nv_bfloat16* __restrict__ gu, const __nv_bfloat16* __restrict__ dh,
+swiglu_bwd_kernel(const __nv_bfloat16* gu, const __nv_bfloat16* dh,
                   __nv_bfloat16* __restrict__ dgu, long T, int f) {
   let_successor_start();
   wait_for_predecessor();
@@ -579,8 +579,8 @@ __global__ void attn_delta_kernel(const __nv_bfloat16* __restrict__ o, const __n
 //   neg_delta[b][h][s] = -sum_d O dO        neg_lse2[b][h][s] = -lse[b][h][s] * log2(e)
 // (one warp per (token, head)), so the inner loops use packed fma / add without a negation.
 // ------------------------------------------------------------------------------------------
-__global__ void attn_bwd_stats_kernel(const __nv_bfloat16* __restrict__ o, const __nv_bfloat16* __restrict__ dout,
-                                      const float* __restrict__ lse, float* __restrict__ neg_lse2,
+__global__ void attn_bwd_stats_kernel(const __nv_bfloat16* o, const __nv_bfloat16* dout,
+                                      const float* lse, float* __restrict__ neg_lse2,
                                       float* __restrict__ neg_delta, int B, int S, int H, int D, long o_rs, long do_rs) {
   let_successor_start();
   wait_for_predecessor();
@@ -616,8 +616,8 @@ __global__ void attn_bwd_stats_kernel(const __nv_bfloat16* __restrict__ o, const
 constexpr int STAT_TOKENS = 32;
 template <int D, int STAT_HEADS>
 __global__ void __launch_bounds__(256)
-attn_bwd_stats_vec_kernel(const __nv_bfloat16* __restrict__ o, const __nv_bfloat16* __restrict__ dout,
-                          const float* __restrict__ lse, float* __restrict__ neg_lse2,
+attn_bwd_stats_vec_kernel(const __nv_bfloat16* o, const __nv_bfloat16* dout,
+                          const float* lse, float* __restrict__ neg_lse2,
                           float* __restrict__ neg_delta, int S, int H, long tokens, long o_rs, long do_rs) {
   let_successor_start();
   wait_for_predecessor();
@@ -635,8 +635,8 @@ attn_bwd_stats_vec_kernel(const __nv_bfloat16* __restrict__ o, const __nv_bfloat
     if (t0 + tl < tokens && h0 + hl < H) {
       const long at = static_cast<long>(h0 + hl) * D + c;
       float a[8], b[8];
-      unpack8(__ldg(reinterpret_cast<const uint4*>(o + (t0 + tl) * o_rs + at)), a);
-      unpack8(__ldg(reinterpret_cast<const uint4*>(dout + (t0 + tl) * do_rs + at)), b);
+      unpack8(*reinterpret_cast<const uint4*>(o + (t0 + tl) * o_rs + at), a);
+      unpack8(*reinterpret_cast<const uint4*>(dout + (t0 + tl) * do_rs + at), b);
 #pragma unroll
       for (int e = 0; e < 8; ++e) acc += a[e] * b[e];
     }
@@ -663,9 +663,9 @@ attn_bwd_stats_vec_kernel(const __nv_bfloat16* __restrict__ o, const __nv_bfloat
 // 2 x 501 loads (129 us).
 constexpr int CE_ROWS = 32, CE_WARPS = 8;
 __global__ void __launch_bounds__(CE_ROWS * CE_WARPS)
-ce_combine_kernel(const float* __restrict__ pmax, const float* __restrict__ psum, int slabs,
-                  const float* __restrict__ target_logit, const int* __restrict__ targets, int target_step, int vocab,
-                  const float* __restrict__ weights, float grad_scale, const float* __restrict__ scale,
+ce_combine_kernel(const float* pmax, const float* psum, int slabs,
+                  const float* target_logit, const int* targets, int target_step, int vocab,
+                  const float* weights, float grad_scale, const float* scale,
                   float* __restrict__ lse, float* __restrict__ coef, float* __restrict__ block_nll,
                   float* __restrict__ block_w, int rows) {
   let_successor_start();
@@ -677,7 +677,7 @@ ce_combine_kernel(const float* __restrict__ pmax, const float* __restrict__ psum
   float m = -INFINITY;
   if (live) {
 #pragma unroll 8
-    for (int s = warp; s < slabs; s += CE_WARPS) m = fmaxf(m, __ldg(pmax + static_cast<size_t>(s) * rows + row));
+    for (int s = warp; s < slabs; s += CE_WARPS) m = fmaxf(m, pmax[static_cast<size_t>(s) * rows + row]);
   }
   part[warp][lane] = m;
   __syncthreads();
@@ -688,7 +688,7 @@ ce_combine_kernel(const float* __restrict__ pmax, const float* __restrict__ psum
 #pragma unroll 8
     for (int s = warp; s < slabs; s += CE_WARPS) {
       const size_t i = static_cast<size_t>(s) * rows + row;
-      acc += __ldg(psum + i) * __expf(__ldg(pmax + i) - m);
+      acc += psum[i] * __expf(pmax[i] - m);
     }
   }
   __syncthreads();
@@ -719,15 +719,15 @@ ce_combine_kernel(const float* __restrict__ pmax, const float* __restrict__ psum
 // Sums of the blocks' partial sums, in a fixed order: one block, both sums (two reductions of the framework took 3.5 us each and
 // a launch gap, this 2 behind the combine that it is chained to).
 __global__ void __launch_bounds__(256)
-ce_sums_kernel(const float* __restrict__ block_nll, const float* __restrict__ block_w, int blocks, float* __restrict__ nll,
+ce_sums_kernel(const float* block_nll, const float* block_w, int blocks, float* __restrict__ nll,
                float* __restrict__ w) {
   let_successor_start();
   wait_for_predecessor();
   __shared__ float scratch[33];
   float a = 0.f, b = 0.f;
   for (int i = threadIdx.x; i < blocks; i += 256) {
-    a += __ldg(block_nll + i);
-    b += __ldg(block_w + i);
+    a += block_nll[i];
+    b += block_w[i];
   }
   a = block_sum(a, scratch);
   b = block_sum(b, scratch);
@@ -826,8 +826,8 @@ logits_ce_backward_kernel(__nv_bfloat16* __restrict__ logits, long ld, int vocab
 // Bound by memory: 6 bytes an element.
 // ------------------------------------------------------------------------------------------
 __global__ void __launch_bounds__(256)
-kept_logits_gradient_kernel(float* __restrict__ logits, long ld, int vocab, const int* __restrict__ targets, int target_step,
-                            const float* __restrict__ lse, const float* __restrict__ coef) {
+kept_logits_gradient_kernel(float* __restrict__ logits, long ld, int vocab, const int* targets, int target_step,
+                            const float* lse, const float* coef) {
   let_successor_start();
   wait_for_predecessor();
   const long row = blockIdx.x;
@@ -840,8 +840,8 @@ kept_logits_gradient_kernel(float* __restrict__ logits, long ld, int vocab, cons
   auto load = [&](int k, float4 (&to)[2]) {
     const int col = k * 2048 + threadIdx.x * 8;
     if (col < vocab) {
-      to[0] = __ldcs(reinterpret_cast<const float4*>(x + col));
-      to[1] = __ldcs(reinterpret_cast<const float4*>(x + col) + 1);
+      to[0] = load_streamed(x + col);
+      to[1] = load_streamed(x + col + 4);
     }
   };
   load(0, next);

@@ -374,7 +374,7 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constan
 
 // Sum of the partial tiles in slice order, a warp per row of a tile, eight columns a thread.
 template <int TM, bool F32>
-__global__ void __launch_bounds__(256) pair_reduce_kernel(const float* __restrict__ part, const GemmArgs args, const PairArgs walk,
+__global__ void __launch_bounds__(256) pair_reduce_kernel(const float* part, const GemmArgs args, const PairArgs walk,
                                                           void* out, long ldc) {
   if (args.chained) let_successor_start();
   wait_for_predecessor();
@@ -386,11 +386,11 @@ __global__ void __launch_bounds__(256) pair_reduce_kernel(const float* __restric
   const Unit u = map_unit<TM>(walk.whole + tile, walk);
   const int m = u.m0 + row, n = u.n0 + col;
   if (m >= args.M || n >= args.N) return;
-  const float4* from = reinterpret_cast<const float4*>(part + (static_cast<size_t>(tile) * ROWS + row) * BN + col);
-  const size_t step = static_cast<size_t>(rest) * ROWS * BN / 4;
-  float4 lo = __ldcs(from), hi = __ldcs(from + 1);
+  const float* from = part + (static_cast<size_t>(tile) * ROWS + row) * BN + col;
+  const size_t step = static_cast<size_t>(rest) * ROWS * BN;
+  float4 lo = load_streamed(from), hi = load_streamed(from + 4);
   for (int s = 1; s < walk.slices; ++s) {
-    const float4 a = __ldcs(from + s * step), b = __ldcs(from + s * step + 1);
+    const float4 a = load_streamed(from + s * step), b = load_streamed(from + s * step + 4);
     lo.x += a.x; lo.y += a.y; lo.z += a.z; lo.w += a.w;
     hi.x += b.x; hi.y += b.y; hi.z += b.z; hi.w += b.w;
   }

@@ -252,10 +252,22 @@ __device__ __forceinline__ void tma_wait_group() {
 // ---------------------------------------------------------------------------------------
 // Every thread, before anything that the launches before this one write or read is touched; nothing to wait for in a launch
 // that was not chained.
+//
+// A kernel that may be chained reads whatever a launch before it may have written, its weights and tables too, by ordinary loads
+// through pointers that are not const __restrict__, or by load_streamed.  The read-only loads that __ldg and const __restrict__
+// stand for promise that the memory does not change while the kernel runs, and this kernel runs while its predecessor still
+// writes: no wait orders them, and the compiler may move them ahead of it.  (The other cache intrinsics are no better: nothing
+// keeps the compiler from moving them.)  tests/test_chained_kernels.py checks the sources for it.
 __device__ __forceinline__ void wait_for_predecessor() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
 // The launch behind this one may start when all CTAs have said so.  Not before a CTA has the TMEM that it allocates: a
 // successor that took it would wait for this launch to end.
 __device__ __forceinline__ void let_successor_start() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
+// 16 bytes that are read once, kept behind the wait.
+__device__ __forceinline__ float4 load_streamed(const float* at) {
+  float4 v;
+  asm volatile("ld.global.cs.v4.f32 {%0, %1, %2, %3}, [%4];" : "=f"(v.x), "=f"(v.y), "=f"(v.z), "=f"(v.w) : "l"(at) : "memory");
+  return v;
+}
 
 // ---------------------------------------------------------------------------------------
 // Cluster launch control: a CTA takes over a work item (CTA) of its grid that has not started

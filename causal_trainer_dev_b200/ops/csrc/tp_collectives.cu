@@ -464,7 +464,7 @@ embedding_backward_kernel(const int* __restrict__ sorted_ids, const int* __restr
 // ------------------------------------------------------------------------------------------
 constexpr int SORT_MOST = 2048;
 __global__ void __launch_bounds__(1024)
-sort_ids_kernel(const int* __restrict__ ids, int words, int count, int slots, int* __restrict__ sorted_ids,
+sort_ids_kernel(const int* ids, int words, int count, int slots, int* __restrict__ sorted_ids,
                 int* __restrict__ perm) {
   let_successor_start();
   wait_for_predecessor();
