@@ -133,6 +133,7 @@ struct BwdArgs {
   GroupArgs grp;
   int chained;              // see launch_chained
   int parts;                // dK/dV: work items per key tile (> 1: see dkv_parts_used)
+  int least;                // entries that each of them has at least
   float* partial;           // [item][part][dV, dK][D / 4][128 keys][4]
 };
 
@@ -153,6 +154,7 @@ struct BwdCall {
   int gathered_rows = 0;     // grouped: capacity of the gathered row space
   int ctas = 0;              // grouped: CTAs to launch (one per descriptor)
   int parts = 1;             // work items per key tile of dK/dV, with `partial` to hold their sums
+  int least = 4;             // entries that each of them has at least
   float* partial = nullptr;
 };
 

@@ -103,10 +103,11 @@ struct alignas(16) BwdItem {
 };
 static_assert(sizeof(BwdItem) == 48, "three 16-byte reads");
 
-// Of the `parts` work items that a launch has for a key tile, as many have work as leave each two iterations (two entries
-// each); one alone stores its results as if there were no others.  (us, with eight, four and two iterations: 512 tokens 8 / 2
-// heads 26.7, 17.6, 17.5; 2 x 512 12 / 2 31.7, 25.6, 23.1; 1024 12 / 2 in documents of 200 34.9, 23.5, 22.5.)
-__device__ __forceinline__ int dkv_parts_used(const BwdArgs& args, int n_entry) { return max(1, min(args.parts, n_entry / 4)); }
+// Of the `parts` work items that a launch has for a key tile, as many have work as leave each `least` entries (see dkv_least);
+// one alone stores its results as if there were no others.
+__device__ __forceinline__ int dkv_parts_used(const BwdArgs& args, int n_entry) {
+  return max(1, min(args.parts, n_entry / args.least));
+}
 
 // The 64-row query blocks that see the key tile kb of row b: [first, first + count).  Only the queries this rank holds,
 // [q_off, q_off + Sq), are walked.
@@ -146,7 +147,10 @@ __device__ __forceinline__ BwdItem bwd_item(const BwdArgs& args, const int cta) 
     if (gd.w <= 0) w.mode = -2;                        // unused capacity: nothing is written
     return w;
   }
-  int idx = DKV && PARTS ? cta / args.parts : cta;
+  // The first part of every key tile, then the second ones, ...: side by side, the parts that have no work in a call of short documents
+  // came ahead of tiles and dQ items that do (2 rows of 2048 in documents of 200, 14 / 2 heads, 65.6 us, in this order 46.8).
+  const int tiles = args.Hkv * args.B * nb128;
+  int idx = DKV && PARTS ? cta % tiles : cta;
   if (DKV) {
     w.head = idx % args.Hkv;      // kv head
     idx /= args.Hkv;
@@ -158,11 +162,11 @@ __device__ __forceinline__ BwdItem bwd_item(const BwdArgs& args, const int cta) 
     w.hkv = w.head;
     if (PARTS) {
       // whole iterations (two entries) to every part that has work
-      const int part = cta % args.parts, used = dkv_parts_used(args, w.n_entry), all = w.n_entry;
+      const int part = cta / tiles, used = dkv_parts_used(args, w.n_entry), all = w.n_entry;
       if (part >= used) w.mode = -2;
       w.first = all * part / used & ~1;
       w.n_entry = (part + 1 < used ? all * (part + 1) / used & ~1 : all) - w.first;
-      w.list = used > 1 ? cta : -1;
+      w.list = used > 1 ? cta % tiles * args.parts + part : -1;
     }
   } else {
     w.head = idx % args.Hq;       // query head
@@ -997,6 +1001,7 @@ int prepare_bwd(const BwdCall& c, BwdMaps* maps, BwdArgs* args, int* items) {
   a.status = device_status();
   a.spin_budget = c.spin_budget > 0 ? c.spin_budget : CTB_SPIN_BUDGET;
   a.parts = DKV && c.partial != nullptr ? c.parts : 1;
+  a.least = c.least;
   a.partial = c.partial;
   *maps = BwdMaps{mq.map, mk.map, mv.map, mdo.map, mo1.map, mo2.map};
   *args = a;
@@ -1085,6 +1090,7 @@ int launch_bwd_dense(const BwdCall& c) {
   a.q_lo = c.q_lo; a.q_hi = c.q_hi;
   a.scale = c.scale;
   a.parts = c.parts;
+  a.least = c.least;
   a.partial = c.partial;
   CTB_CUDA_OK(launch_chained(chained_rows(static_cast<long>(c.B) * c.Sq, c.Hq, D), attn_bwd_sum_kernel<D>,
                              c.B * c.Hkv * (c.S / 128) * 2 * (D / 16), 128, 0, c.stream, 0, a,
@@ -1097,9 +1103,12 @@ int launch_bwd_dense(const BwdCall& c) {
 // key tiles (short rows, few kv heads) ends with a few SMs on the long ones of them: one row of 2048 tokens, 14 / 2 heads, has 32,
 // and the longest is 112 iterations where an SM has 29 of the whole call.  The estimate (cycles) takes the rows for whole
 // documents: an iteration of dK/dV 2615 and of dQ 2047, the start and end of an item 10000 and 8000, of a further part with its
-// fp32 tiles 12000, the sum of the parts 8000.  Rows of short documents lose little by that, because a part without two
-// iterations of its own has no work (4 rows of 512 in documents of 128, 8 / 2 heads, 18.3 us uncut, 22.1; of 1024 in documents of 200, 12 /
-// 2 heads, 32.5 and 22.5).
+// fp32 tiles 12000, the sum of the parts 8000.  Rows of short documents, whose tiles stay whole or nearly so (dkv_least), pay for
+// that: the launch of the sums and the parts without work are 2 to 5 us.  Backward, us, uncut and so: 2 rows of 2048, 14 / 2 heads,
+// one document 176.9, 101.2, documents of 350 59.5, 52.8, of 128 31.0, 35.7; 4 rows of 512, 8 / 2 heads, 34.8, 25.7, of 200 27.0, 24.2,
+// of 128 18.4, 20.4; 1 row of 1024, 28 / 4 heads, of 200 37.8, 29.6.  What did not mend it: the sums by the last part of a tile to
+// finish (one SM reads them all: 5 to 8 us a cut tile), a compact list of the items made by every CTA with the sums at its end
+// (the sums in the compute warps' loop spill registers: 6 to 12 us).
 inline int dkv_parts(int B, int S, int Sq, int Hq, int Hkv) {
   const double tiles = static_cast<double>(B) * Hkv * (S / 128), rows = static_cast<double>(B) * Hq * (Sq / 128);
   const double longest = static_cast<double>(Hq / Hkv) * (Sq / 128), seen = (Sq / 128 + 1) / 2.;
@@ -1116,6 +1125,13 @@ inline int dkv_parts(int B, int S, int Sq, int Hq, int Hkv) {
   }
   return best;
 }
+
+// Entries that a part of a key tile has at least: half of what the parts of the longest tile of one document have, and two iterations
+// (two entries each).  Cut finer, rows of short documents with tiles enough for the GPU pay for the ends of their items (backward,
+// us, without parts, with two iterations and with this: 2 rows of 2048, 14 / 2 heads, documents of 128 30.6, 48.1, 35.9; 1 row, 28 /
+// 4 heads, of 200 41.0, 50.6, 44.1).  Parts twice as long lose where tiles are few (1 row of 2048, 14 / 2 heads, documents of 350 47.2,
+// here 35.2, uncut 53.8).
+inline int dkv_least(int Sq, int Hq, int Hkv, int parts) { return max(4, Hq / Hkv * (Sq / 128) / 2 / parts); }
 
 }  // namespace attn
 }  // namespace ctb
@@ -1158,6 +1174,7 @@ CTB_API int ctb_attn_bwd_range(const void* q, const void* k, const void* v, cons
   if (wanted > 0 && workspace != nullptr && workspace_bytes >= wanted && reinterpret_cast<uintptr_t>(workspace) % 16 == 0 &&
       ((reinterpret_cast<uintptr_t>(dk) | reinterpret_cast<uintptr_t>(dv)) % 16 == 0 && dk_rs % 8 == 0 && dv_rs % 8 == 0)) {
     c.parts = ctb::attn::dkv_parts(B, S, Sq, Hq, Hkv);
+    c.least = ctb::attn::dkv_least(Sq, Hq, Hkv, c.parts);
     c.partial = static_cast<float*>(workspace);
   }
   return D == 128 ? ctb::attn::launch_bwd_dense<128>(c) : ctb::attn::launch_bwd_dense<64>(c);

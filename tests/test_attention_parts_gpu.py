@@ -78,3 +78,22 @@ def test_key_tiles_in_parts(cuda_lib, monkeypatch, kind, b, s, hq, hkv, d):
     torch.einsum("hqk,khd->qhd", p, vd.repeat_interleave(group, 1)).backward(do[i].double())
     for got, want in zip(first, (qd.grad, kd.grad, vd.grad)):
         assert _rel(got[i], want) < 3 * BF16
+
+
+@pytest.mark.parametrize("b,s,hq,hkv,d,docs", [(2, 2048, 14, 2, 128, 128), (1, 4096, 8, 2, 128, 128), (1, 4096, 8, 2, 64, 64)])
+def test_tiles_of_short_documents_stay_whole(cuda_lib, monkeypatch, b, s, hq, hkv, d, docs):
+    """Rows that would be cut as one document, but whose documents leave no part the work it has to have at least: the bits of
+    the uncut call."""
+    from causal_trainer_dev_b200.ops import attention as A
+
+    assert cuda_lib.lib().ctb_attn_bwd_workspace(b, s, s, hq, hkv, d) > 0
+    gen = torch.Generator(device="cuda").manual_seed(4)
+    q, do = (torch.randn(b, s, hq, d, generator=gen, device="cuda").bfloat16() for _ in range(2))
+    k, v = (torch.randn(b, s, hkv, d, generator=gen, device="cuda").bfloat16() for _ in range(2))
+    meta = A.build_attention_meta((torch.arange(s, device="cuda") // docs + 1).int().repeat(b, 1))
+    o, lse = A.flash_attention_forward(q, k, v, meta)
+    got = A.flash_attention_backward(q, k, v, o, do, lse, meta)
+    monkeypatch.setattr(cuda_lib.lib(), "ctb_attn_bwd_workspace", lambda *a: 0)
+    want = A.flash_attention_backward(q, k, v, o, do, lse, meta)
+    assert all(torch.equal(x, y) for x, y in zip(got, want))
+    assert cuda_lib.device_status() == (0, 0, 0, 0)
