@@ -191,6 +191,20 @@ rmsnorm_bwd_kernel(const __nv_bfloat16* dy, const __nv_bfloat16* x,
         dw_acc[i][e] += a[e] * xh;
       }
     }
+    // (not held: w and the residual gradient are read two vectors ahead, because they could not pass the barrier and the stores)
+    uint4 w_at[3], r_at[3];
+    auto fetch_wide = [&](int i) {
+      const int v = threadIdx.x + i * NORM_THREADS;
+      r_at[i % 3] = zero;
+      if (v < nvec) {
+        w_at[i % 3] = reinterpret_cast<const uint4*>(w)[v];
+        if (dres) r_at[i % 3] = reinterpret_cast<const uint4*>(dres)[static_cast<size_t>(row) * nvec + v];
+      }
+    };
+    if (!HOLD) {
+      fetch_wide(0);
+      fetch_wide(1);
+    }
     dot = warp_sum(dot);
     if ((threadIdx.x & 31) == 0) sums[parity][threadIdx.x >> 5] = dot;
     __syncthreads();
@@ -201,13 +215,13 @@ rmsnorm_bwd_kernel(const __nv_bfloat16* dy, const __nv_bfloat16* x,
 #pragma unroll
     for (int i = 0; i < NV; ++i) {
       const int v = threadIdx.x + i * NORM_THREADS;
+      if (!HOLD && i + 2 < NV) fetch_wide(i + 2);
       if (v < nvec) {
         float a[8], b[8], c[8], r[8], o[8];
         unpack8(dy_now[i], a);
         unpack8(x_now[i], b);
-        unpack8(HOLD ? wv[i] : reinterpret_cast<const uint4*>(w)[v], c);
-        if (!HOLD && dres) res_now[i] = reinterpret_cast<const uint4*>(dres)[static_cast<size_t>(row) * nvec + v];
-        unpack8(res_now[i], r);
+        unpack8(HOLD ? wv[i] : w_at[i % 3], c);
+        unpack8(HOLD ? res_now[i] : r_at[i % 3], r);
 #pragma unroll
         for (int e = 0; e < 8; ++e) o[e] = r_now * (a[e] * c[e] - b[e] * r_now * mean) + r[e];
         reinterpret_cast<uint4*>(dx + static_cast<size_t>(row) * d)[v] = pack8(o);
@@ -260,12 +274,14 @@ rmsnorm_dw_reduce_kernel(const float* partial, int parts, int d, void* __restric
 
 // Column sums of a bf16 matrix (the gradient of a projection's bias) into per-CTA partial rows, which
 // rmsnorm_dw_reduce_kernel adds up.  Bound by reading the matrix once: a warp reads 512 bytes of a row, eight
-// rows a CTA and four in flight a warp; the cast to fp32 and the strided sum that did this wrote and read
+// rows a CTA, and the next four rows a warp are on their way while four are added (8192 x 2048 6.7 us; in a loop that the compiler
+// unrolls by four 11.9, four at a time 10.2); the cast to fp32 and the strided sum that did this wrote and read
 // twice the matrix in between.
 __global__ void __launch_bounds__(256)
 column_sum_kernel(const __nv_bfloat16* x, long ld, int rows, int n, float* __restrict__ partial) {
   let_successor_start();
   wait_for_predecessor();
+  constexpr int AHEAD = 4;                       // rows; the loads of as many more are in flight behind them
   __shared__ float sums[8][256 + 8];
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   const int c = blockIdx.x * 256 + lane * 8;
@@ -273,12 +289,30 @@ column_sum_kernel(const __nv_bfloat16* x, long ld, int rows, int n, float* __res
   const int step = gridDim.y * 8;
   float acc[8] = {0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f};
   if (live) {
-#pragma unroll 4
-    for (int r = blockIdx.y * 8 + warp; r < rows; r += step) {
-      float f[8];
-      unpack8(*reinterpret_cast<const uint4*>(x + static_cast<long>(r) * ld + c), f);
+    uint4 raw[2][AHEAD];
+    auto load = [&](int r, uint4 (&to)[AHEAD]) {
 #pragma unroll
-      for (int e = 0; e < 8; ++e) acc[e] += f[e];
+      for (int k = 0; k < AHEAD; ++k) {
+        to[k] = make_uint4(0u, 0u, 0u, 0u);
+        if (r + k * step < rows) to[k] = *reinterpret_cast<const uint4*>(x + static_cast<long>(r + k * step) * ld + c);
+      }
+    };
+    auto add = [&](const uint4 (&from)[AHEAD]) {
+#pragma unroll
+      for (int k = 0; k < AHEAD; ++k) {
+        float f[8];
+        unpack8(from[k], f);
+#pragma unroll
+        for (int e = 0; e < 8; ++e) acc[e] += f[e];
+      }
+    };
+    int r = blockIdx.y * 8 + warp;
+    load(r, raw[0]);
+    while (r < rows) {
+      load(r += AHEAD * step, raw[1]);
+      add(raw[0]);
+      load(r += AHEAD * step, raw[0]);
+      add(raw[1]);
     }
   }
 #pragma unroll
@@ -610,11 +644,13 @@ __global__ void attn_bwd_stats_kernel(const __nv_bfloat16* o, const __nv_bfloat1
 // The same for D = 64 or 128 and 16-byte aligned rows.  Bound by reading O and dO once.  The kernel
 // above reads 4 bytes per lane and access and stores one float per warp, S floats apart; here a
 // group of D / 8 lanes reads a (token, head) row as 16-byte vectors, a block takes STAT_TOKENS tokens
-// x 8 heads (2 KiB contiguous per token at D = 128; 4 heads where their number is not a multiple of 8, so that no half of a
-// block idles: 8 rows of 4096 tokens, 12 heads 54 -> 38 us) and turns the sums round in shared memory, so that
-// lse is read and both statistics are written 128 bytes at a time.
-constexpr int STAT_TOKENS = 32;
-template <int D, int STAT_HEADS>
+// x STAT_HEADS heads (1 KiB contiguous per token at D = 128) and turns the sums round in shared memory, so that
+// lse is read and both statistics are written 128 bytes at a time.  With 8 heads a block (us; 4 heads behind it): 8 rows of 4096 tokens,
+// 12 heads 43.8, 37.5; 1 of 4096, 28 heads 9.9, 8.3; 4 of 1024, 32 heads 10.0, 9.1; 1 of 32768, 8 heads 27.3, 28.3.
+// The loads of four passes are issued before the sums of the first: left to the compiler, which may not move ordinary loads over the
+// stores of the sums, 1 of 4096, 28 heads took 11.5.
+constexpr int STAT_TOKENS = 32, STAT_HEADS = 4;
+template <int D>
 __global__ void __launch_bounds__(256)
 attn_bwd_stats_vec_kernel(const __nv_bfloat16* o, const __nv_bfloat16* dout,
                           const float* lse, float* __restrict__ neg_lse2,
@@ -628,21 +664,32 @@ attn_bwd_stats_vec_kernel(const __nv_bfloat16* o, const __nv_bfloat16* dout,
   const long t0 = static_cast<long>(blockIdx.x) * STAT_TOKENS;
   const int h0 = blockIdx.y * STAT_HEADS;
   const int sub = threadIdx.x / LANES, c = (threadIdx.x % LANES) * 8;
-#pragma unroll 4
-  for (int p = 0; p < PASSES; ++p) {
-    const int row = p * ROWS + sub, hl = row % STAT_HEADS, tl = row / STAT_HEADS;
-    float acc = 0.f;
-    if (t0 + tl < tokens && h0 + hl < H) {
-      const long at = static_cast<long>(h0 + hl) * D + c;
-      float a[8], b[8];
-      unpack8(*reinterpret_cast<const uint4*>(o + (t0 + tl) * o_rs + at), a);
-      unpack8(*reinterpret_cast<const uint4*>(dout + (t0 + tl) * do_rs + at), b);
+  constexpr int AHEAD = 4;
+  static_assert(PASSES % AHEAD == 0, "whole groups of passes");
+  for (int p0 = 0; p0 < PASSES; p0 += AHEAD) {
+    uint4 av[AHEAD], bv[AHEAD];
 #pragma unroll
-      for (int e = 0; e < 8; ++e) acc += a[e] * b[e];
+    for (int p = 0; p < AHEAD; ++p) {
+      const int row = (p0 + p) * ROWS + sub, hl = row % STAT_HEADS, tl = row / STAT_HEADS;
+      av[p] = bv[p] = make_uint4(0u, 0u, 0u, 0u);
+      if (t0 + tl < tokens && h0 + hl < H) {
+        const long at = static_cast<long>(h0 + hl) * D + c;
+        av[p] = *reinterpret_cast<const uint4*>(o + (t0 + tl) * o_rs + at);
+        bv[p] = *reinterpret_cast<const uint4*>(dout + (t0 + tl) * do_rs + at);
+      }
     }
 #pragma unroll
-    for (int m = LANES / 2; m > 0; m >>= 1) acc += __shfl_xor_sync(0xffffffffu, acc, m);
-    if (c == 0) sums[hl][tl] = acc;
+    for (int p = 0; p < AHEAD; ++p) {
+      const int row = (p0 + p) * ROWS + sub;
+      float a[8], b[8], acc = 0.f;
+      unpack8(av[p], a);
+      unpack8(bv[p], b);
+#pragma unroll
+      for (int e = 0; e < 8; ++e) acc += a[e] * b[e];
+#pragma unroll
+      for (int m = LANES / 2; m > 0; m >>= 1) acc += __shfl_xor_sync(0xffffffffu, acc, m);
+      if (c == 0) sums[row % STAT_HEADS][row / STAT_HEADS] = acc;
+    }
   }
   __syncthreads();
   const int hl = threadIdx.x >> 5, tl = threadIdx.x & 31;
@@ -1329,20 +1376,18 @@ CTB_API int ctb_attn_delta(const void* o, const void* dout, float* delta, int B,
 CTB_API int ctb_attn_bwd_stats(const void* o, const void* dout, const float* lse, float* neg_lse2, float* neg_delta,
                                int B, int S, int H, int D, long o_rs, long do_rs, void* stream) {
   // 16-byte rows of the two head sizes the flash kernels take, and enough of them: a block of the wide kernel takes
-  // 256 rows one after the other, 4.0 us at D = 64 and 6.4 at D = 128 however few there are, where a warp per row
-  // (below) takes 2.0 and grows with the rows.  They meet at 192 D rows (us, warp per row and wide: D = 64 8192 rows
-  // 3.5 and 4.0, 12288 rows 4.2 and 4.0, 16384 rows 5.0 and 4.1; D = 128 16384 rows 5.3 and 6.5, 24576 rows 7.0
-  // and 6.6, 32768 rows 8.6 and 6.9).
+  // 128 rows one after the other, 2.3 us at D = 64 and 3.4 at D = 128 however few there are, where a warp per row
+  // (below) takes 1.8 and grows with the rows.  They meet at 80 D rows (us, warp per row and wide: D = 64 4096 rows
+  // 2.5 and 2.4, 8192 rows 3.1 and 2.4, 16384 rows 4.8 and 2.5; D = 128 8192 rows 3.2 and 3.7, 12288 rows 4.6
+  // and 4.0, 16384 rows 5.4 and 4.0).
   const long tokens = static_cast<long>(B) * S;
-  const bool wide = (D == 64 || D == 128) && o_rs % 8 == 0 && do_rs % 8 == 0 && tokens * H >= 192l * D &&
+  const bool wide = (D == 64 || D == 128) && o_rs % 8 == 0 && do_rs % 8 == 0 && tokens * H >= 80l * D &&
                     (reinterpret_cast<uintptr_t>(o) | reinterpret_cast<uintptr_t>(dout)) % 16 == 0;
   const bool chained = attn::chained_rows(tokens, H, D);
-  const int heads = H % 8 != 0 && H % 4 == 0 ? 4 : 8;
-  const int head_blocks = (H + heads - 1) / heads;
+  const int head_blocks = (H + STAT_HEADS - 1) / STAT_HEADS;
   if (wide && head_blocks <= 65535) {
     const dim3 grid(static_cast<unsigned>((tokens + STAT_TOKENS - 1) / STAT_TOKENS), head_blocks);
-    auto kern = heads == 8 ? (D == 128 ? attn_bwd_stats_vec_kernel<128, 8> : attn_bwd_stats_vec_kernel<64, 8>)
-                           : (D == 128 ? attn_bwd_stats_vec_kernel<128, 4> : attn_bwd_stats_vec_kernel<64, 4>);
+    auto kern = D == 128 ? attn_bwd_stats_vec_kernel<128> : attn_bwd_stats_vec_kernel<64>;
     CTB_CUDA_OK(launch_chained(chained, kern, grid, 256, 0, stream, 0, static_cast<const __nv_bfloat16*>(o),
                                static_cast<const __nv_bfloat16*>(dout), lse, neg_lse2, neg_delta, S, H, tokens, o_rs, do_rs));
     return 0;
