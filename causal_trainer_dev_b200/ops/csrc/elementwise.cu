@@ -1217,7 +1217,9 @@ CTB_API int ctb_rmsnorm_fwd(const void* x, const void* residual, const void* w, 
   if (d % 8 || d > NORM_MAXV * NORM_THREADS * 8) return fail("rmsnorm: hidden size must be a multiple of 8, <= 16384");
   if (residual && !h_out) return fail("rmsnorm: residual given without h_out");
   const int grid = rows < sm_count() * 8 ? rows : sm_count() * 8;
-  const bool chained = (residual ? 8l : 4l) * rows * d <= CHAINED_BYTES;
+  // (half of CHAINED_BYTES: us, chained and not, 64 x 4096 2.3 and 2.6, 1000 x 1536 3.3 and 3.7; 4096 x 4096 14.5 and 13.1, with
+  // a residual 2000 x 4096 12.0 and 11.2)
+  const bool chained = (residual ? 8l : 4l) * rows * d <= CHAINED_BYTES / 2;
   const int nv = (d / 8 + NORM_THREADS - 1) / NORM_THREADS;
 #define CTB_NORM_FWD(NV)                                                                                         \
   CTB_CUDA_OK(launch_chained(chained, rmsnorm_fwd_kernel<NV>, grid, NORM_THREADS, 0, stream, 0,                  \
@@ -1304,7 +1306,9 @@ CTB_API int ctb_rope(void* x, const float* cosv, const float* sinv, long row_str
   // long for the number of tokens), is no faster than a thread per pair (us, pair and vector: 8192 tokens, 4 lanes of a warp
   // 3.2 and 4.0; 2048 tokens, 8 lanes 2.7 and 2.4; 333 tokens, 4 heads of 128 2.2 and 2.0; 128 tokens, 10 heads of 128 2.3 and
   // 2.5, 40 heads 3.7 and 2.6).
-  const bool chained = 4l * T * heads * rot <= CHAINED_BYTES;
+  // (2 MB and not CHAINED_BYTES: us, chained and not, 512 tokens, 6 heads of 64 1.9 and 2.0; 512, 14 heads of 128 2.6 and 2.3; 2000, 14 heads
+  // 5.8 and 4.4; 1000, 40 heads 5.6 and 4.1)
+  const bool chained = 4l * T * heads * rot <= 2l << 20;
   const int angles = style == 0 ? 4 : 8;
   const int per_head = rot / 2 / angles;
   if (rot % (2 * angles) == 0 && per_head >= 1 && per_head <= 32 && D % 8 == 0 && row_stride % 8 == 0 &&
