@@ -439,11 +439,16 @@ __global__ void rope_table_kernel(const int* __restrict__ pos, const float* __re
 // SwiGLU on the packed projection gu[T][2f] = [gate | up]:  h = silu(gate) * up.
 // Backward writes d(gate|up) in the same packed layout.
 // ------------------------------------------------------------------------------------------
-// n / d for d = 1 + exp(-g), g below 87 in size, and finite n: an approximate reciprocal, a Newton step, and the quotient corrected
-// by its own remainder, which rounds it correctly (for every bf16 gate the bits of the IEEE division, but for the sign of a
-// zero) without that division's range reduction.  The division bound the forward kernel by its instructions (279 us at 16384 x
-// 14336); a fast one returns zero for denominators above 2^126, gates between -88.7 and -87.4.  A vector with a larger gate
-// divides, in a function of its own: inlined it costs the others their registers (260 us).
+// n / d for d = 1 + exp(-g), g below 87 in size, and |n| <= 87, by Markstein's method (P. W. Markstein, Computation of elementary
+// functions on the IBM RISC System/6000 processor, IBM J. Res. Dev. 34, 1990): a reciprocal refined by a Newton step, a quotient
+// of it, and that quotient corrected by its remainder.  Why it holds here: 1 <= d < 2^126, so that the reciprocal is a normal
+// number; after the step it is within half an ulp and a little of 1 / d (the approximate one is within 2^-23, the step squares that), the
+// quotient within an ulp of n / d, and the remainder of such a quotient is a number that the fused multiply-add gives exactly.  The sum
+// before its one rounding is within 2^-46 of n / d, so only a quotient that close to the middle of two fp32 numbers could come out as the
+// other one.  tests/test_kernel_edges_gpu.py compares all gates of bf16 with the division: no result differs, but for the sign of a zero.
+// The division bound the forward kernel by its instructions (279 us at 16384 x 14336, so 231); a fast one returns zero for
+// denominators above 2^126, gates between -88.7 and -87.4.  A vector with a larger gate, or one that is not a number, divides, in a
+// function of its own: inlined it costs the others their registers (260 us).
 __device__ __forceinline__ float quotient_in_range(float n, float d) {
   float r;
   asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(d));

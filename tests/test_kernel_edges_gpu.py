@@ -164,6 +164,48 @@ def test_swiglu_of_large_negative_gates(cuda_lib):
     assert near(dgate, gd.grad, 1) and near(dup, ud.grad, 1)
 
 
+def test_swiglu_quotient_of_every_gate(cuda_lib):
+    """All 65536 gates of bf16, among themselves (vectors of gates below 87 take the corrected quotient) and each in a vector with a
+    gate of 88 (which divides): the same results, but for the sign of a zero, with several factors forward and backward."""
+    from causal_trainer_dev_b200.ops import elementwise as E
+
+    gates = torch.arange(-2 ** 15, 2 ** 15, device="cuda").to(torch.int16).view(torch.bfloat16)
+    small = gates[gates.abs() < 87]
+    large = gates[~(gates.abs() < 87)]                         # infinities and what is not a number among them
+    assert small.numel() > 34000 and small.numel() % 4 == large.numel() % 4 == 0
+    gen = torch.Generator(device="cuda").manual_seed(9)
+    for turn in range(24):
+        up, dh = (torch.randn(gates.numel(), generator=gen, device="cuda").bfloat16() for _ in range(2))
+        if turn == 0:
+            up, dh = torch.ones_like(up), torch.ones_like(dh)
+
+        def run(g, u, d):                                      # rows of 512 gates and their factors
+            rows = -(-g.numel() // 512)
+            def block(x, fill):
+                out = torch.full((rows * 512,), fill, dtype=torch.bfloat16, device="cuda")
+                out[:x.numel()] = x
+                return out.view(rows, 512)
+            gu = torch.cat([block(g, 0.5), block(u, 1.0)], dim=1)
+            h, dgu = E.swiglu_forward(gu), E.swiglu_backward(gu, block(d, 1.0))
+            return [x.reshape(-1)[:g.numel()] for x in (h, dgu[:, :512], dgu[:, 512:])]
+
+        n = small.numel()
+        short = run(small, up[:n], dh[:n])
+        wide = lambda x, fill: torch.cat([x.view(-1, 4), torch.full_like(x.view(-1, 4), fill)], 1).reshape(-1)  # noqa: E731
+        long = [x.view(-1, 8)[:, :4].reshape(-1) for x in run(wide(small, 88.0), wide(up[:n], 1.0), wide(dh[:n], 1.0))]
+        for a, b in zip(short, long):
+            assert torch.equal(a, b) and not bool(a.isnan().any())
+        # a large gate leaves the others of its vector alone, and is itself what it is alone
+        m = large.numel()
+        mixed = torch.stack([large.view(-1, 4), small[-m:].view(-1, 4)], 2).reshape(-1)
+        factor = lambda x: torch.stack([x[:m].view(-1, 4), x[n - m:n].view(-1, 4)], 2).reshape(-1)  # noqa: E731
+        got = run(mixed, factor(up), factor(dh))
+        alone = run(large, up[:m], dh[:m])
+        for a, b, c in zip(got, alone, short):
+            a = a.view(-1, 4, 2)
+            assert torch.equal(a[:, :, 1].reshape(-1), c[n - m:]) and torch.equal(a[:, :, 0].reshape(-1).nan_to_num(7.0), b.nan_to_num(7.0))
+
+
 @pytest.mark.parametrize("t", [1497, 1499, 2496, 2497, 4099])      # 128 MiB of traffic: backward above 1497 rows, forward above 2496
 def test_swiglu_grids_beyond_l2(cuda_lib, t):
     """Calls on both sides of the sizes where the grids change; vectors with gates whose exponential leaves the range of the short
