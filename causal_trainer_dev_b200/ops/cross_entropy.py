@@ -72,9 +72,12 @@ def _target_words(targets: torch.Tensor) -> tuple[torch.Tensor, int]:
 
 
 def _device_scale(grad_scale, device) -> tuple[float, torch.Tensor | None]:
-    """A factor of the gradients as (number, one fp32 element on the device or None)."""
+    """A factor of the gradients as (number, one fp32 element on the device or None).  A tensor on the host is a number: a copy
+    to the device would wait for the stream, and cannot be captured."""
     if not isinstance(grad_scale, torch.Tensor):
         return grad_scale, None
+    if grad_scale.device.type == "cpu":
+        return grad_scale.reshape(()).to(torch.float32).item(), None
     return 1.0, grad_scale.reshape(()).to(device=device, dtype=torch.float32)
 
 
