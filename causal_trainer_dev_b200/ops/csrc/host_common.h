@@ -79,7 +79,9 @@ cudaError_t launch_chained(bool chained, void (*kern)(P...), dim3 grid, dim3 blo
     ++cfg.numAttrs;
   }
   cfg.attrs = attr;
-  return cudaLaunchKernelEx(&cfg, kern, static_cast<P>(args)...);
+  const cudaError_t e = cudaLaunchKernelEx(&cfg, kern, static_cast<P>(args)...);
+  if (e != cudaSuccess) (void)cudaGetLastError();      // a refused launch is the caller's to report, not the next launch's to meet
+  return e;
 }
 
 }  // namespace ctb

@@ -156,3 +156,14 @@ def test_the_bits_of_a_sequence_that_the_host_waits_in(cuda_lib):
 
     captured([])
     captured([other])
+
+
+def test_a_refused_launch_leaves_no_error_behind(cuda_lib):
+    """An empty grid is refused; whoever launches next, the framework's own kernels among them, must not be told of it."""
+    from causal_trainer_dev_b200.ops import elementwise as E
+
+    x, w = torch.empty(0, 256, device="cuda", dtype=torch.bfloat16), torch.ones(256, device="cuda", dtype=torch.bfloat16)
+    for _ in range(2):
+        with pytest.raises(cuda_lib.KernelError):
+            E.rmsnorm_forward(x, w, 1e-5)
+        assert float(torch.ones(300, device="cuda").cumsum(0)[-1]) == 300
