@@ -244,7 +244,8 @@ def flash_attention_backward(
     dq = torch.empty(b, sq, hq, d, dtype=torch.bfloat16, device=dev) if dq is None else dq
     dk = torch.empty(b, s, hkv, d, dtype=torch.bfloat16, device=dev) if dk is None else dk
     dv = torch.empty(b, s, hkv, d, dtype=torch.bfloat16, device=dev) if dv is None else dv
-    # partial sums of dK / dV where the key tiles are too few for the GPU; without memory for them they are computed in one piece
+    # partial sums of dK / dV where the key tiles are too few for the GPU; without memory for them they are computed in one piece,
+    # fp32 sums in another order: where memory runs out, the last bits of dK / dV are those of the uncut call
     # (an item of up to four iterations of 128 queries costs less than the sum of its parts: the smallest calls need not ask)
     wanted = _lib.lib().ctb_attn_bwd_workspace(b, s, sq, hq, hkv, d) if hq // hkv * sq > 512 else 0
     work = None

@@ -37,6 +37,7 @@ namespace layer {
 // Mirrored by ops/layer.py (same order, same types).
 struct Shape {
   int batch, seq, hidden, q_heads, kv_heads, head_dim, inner, rotary_dim, rope_style, grad_f32;
+  int whole_tiles;      // no room in the backward call's block for partial sums of dK / dV (ctb_attn_bwd_workspace)
   float eps, scale;
 };
 struct Context {
@@ -140,7 +141,7 @@ struct Backward {
                                static_cast<long>(ctb_column_sum_parts(t, w)) * w));
     no_grad = b.take<float>(s.hidden);
     rstd = b.take<float>(z.t);
-    dkv_bytes = ctb_attn_bwd_workspace(s.batch, s.seq, s.seq, s.q_heads, s.kv_heads, s.head_dim);
+    dkv_bytes = s.whole_tiles ? 0 : ctb_attn_bwd_workspace(s.batch, s.seq, s.seq, s.q_heads, s.kv_heads, s.head_dim);
     dkv = b.take<char>(dkv_bytes);
     long wanted = 0;
     const int shapes[8][3] = {{t, s.inner, s.hidden}, {s.hidden, s.inner, t}, {t, s.hidden, 2 * s.inner},

@@ -18,7 +18,7 @@ FORWARD_LAUNCHES, BACKWARD_LAUNCHES = 9, 22
 
 class _Shape(ctypes.Structure):
     _fields_ = [(n, ctypes.c_int) for n in ("batch", "seq", "hidden", "q_heads", "kv_heads", "head_dim", "inner",
-                                            "rotary_dim", "rope_style", "grad_f32")]
+                                            "rotary_dim", "rope_style", "grad_f32", "whole_tiles")]
     _fields_ += [("eps", ctypes.c_float), ("scale", ctypes.c_float)]
 
 
@@ -44,7 +44,7 @@ def _plan(batch: int, seq: int, hidden: int, q_heads: int, kv_heads: int, head_d
           rope_style: int, grad_f32: int, eps: float) -> tuple[_Shape, int, int, int]:
     """The shape as the library takes it, and the bytes of its three blocks.  (They follow the GEMM switches and the device of
     the moment, and take 10 us a pass to ask for: not kept.)"""
-    shape = _Shape(batch, seq, hidden, q_heads, kv_heads, head_dim, inner, rotary_dim, rope_style, grad_f32, eps,
+    shape = _Shape(batch, seq, hidden, q_heads, kv_heads, head_dim, inner, rotary_dim, rope_style, grad_f32, 0, eps,
                    1.0 / math.sqrt(head_dim))
     sizes = [ctypes.c_long() for _ in range(3)]
     _lib.lib().ctb_layer_bytes(ctypes.byref(shape), *(ctypes.byref(x) for x in sizes))
@@ -75,13 +75,19 @@ class LayerCalls:
         self._context = _Context(ctx["cos"].data_ptr(), ctx["sin"].data_ptr(), *(at(t) for t in (
             meta.seg, meta.lim, meta.start, meta.end, meta.first_q, meta.kv_lo, meta.kv_hi, meta.q_lo, meta.q_hi)))
         self._no_grad = () if train_norm else ("ln1", "ln2")
+        s = self._shape
+        # (pieces of the block are whole 256 bytes)
+        self._sums = -(-_lib.lib().ctb_attn_bwd_workspace(s.batch, s.seq, s.seq, s.q_heads, s.kv_heads, s.head_dim) // 256) * 256
 
     @property
     def scratch_bytes(self) -> int:
         """Of the larger call, without the partial sums of dK / dV: they take their time from the device's, not from the host's."""
-        s = self._shape
-        sums = _lib.lib().ctb_attn_bwd_workspace(s.batch, s.seq, s.seq, s.q_heads, s.kv_heads, s.head_dim)
-        return max(self._forward, self._backward - sums)
+        return max(self._forward, self._backward - self._sums)
+
+    @property
+    def backward_launches(self) -> int:
+        """Kernels of a backward call; the partial sums of dK / dV are added by one more."""
+        return BACKWARD_LAUNCHES + (self._sums > 0)
 
     def forward(self, unit, resid: torch.Tensor, branch: torch.Tensor | None) -> tuple[torch.Tensor, torch.Tensor, tuple]:
         """Returns (h, mlp, what :meth:`backward` needs)."""
@@ -100,11 +106,19 @@ class LayerCalls:
         """Gradient of the layer's input; the weight gradients go into ``grads``, which is laid out as the unit."""
         x, h, kept = saved
         dx = torch.empty_like(dout)
-        scratch = torch.empty(self._backward, dtype=torch.uint8, device=dout.device)
+        try:
+            scratch = torch.empty(self._backward, dtype=torch.uint8, device=dout.device)
+        except torch.cuda.OutOfMemoryError:
+            if self._sums == 0:
+                raise
+            # without the partial sums: key tiles in one piece each, here and in the layers that follow (dK / dV are then sums in
+            # another order, as in ops.attention)
+            self._shape.whole_tiles, self._backward, self._sums = 1, self._backward - self._sums, 0
+            scratch = torch.empty(self._backward, dtype=torch.uint8, device=dout.device)
         code = _lib.lib().ctb_layer_backward(
             ctypes.byref(self._shape), ctypes.byref(self._context), ctypes.byref(_pointers(unit.layout, unit.data)),
             ctypes.byref(_pointers(unit.layout, grads, self._no_grad)), accumulate, None if x is None else x.data_ptr(),
             h.data_ptr(), dout.data_ptr(), kept.data_ptr(), kept.numel(), scratch.data_ptr(), scratch.numel(), dx.data_ptr(),
             _lib.raw_stream())
-        _lib.check(code, "ctb_layer_backward", BACKWARD_LAUNCHES)
+        _lib.check(code, "ctb_layer_backward", self.backward_launches)
         return dx

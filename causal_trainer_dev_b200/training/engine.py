@@ -36,9 +36,9 @@ from ..ops import lib as _lib
 from ..ops.gemm import gemm
 from . import losses
 
-# Largest scratch block of a layer that is issued as one library call per direction: up to here (about 700 tokens of a
-# 1536-wide model, 5000 of a 256-wide one) a layer's device time is no longer than the host time of its launches from Python
-# (0.4 ms).  Above, the launches hide under the device's work, and one block would hold every intermediate to the end
+# Largest scratch block, but for the partial sums of dK / dV, of a layer that is issued as one library call per direction: up to
+# here (about 700 tokens of a 1536-wide model, 5000 of a 256-wide one) a layer's device time is no longer than the host time of its
+# launches from Python (0.4 ms).  Above, the launches hide under the device's work, and one block would hold every intermediate to the end
 LAYER_CALL_BYTES = 64 << 20
 
 
@@ -558,7 +558,7 @@ class LayerwiseEngine:
                     _, _, saved = calls.forward(unit, *layer_in)
                     self._count(layer_ops.FORWARD_LAUNCHES)
                 dout = calls.backward(unit, prov.grad_buffer(f"layer.{li}"), saved, dout, accumulate)
-                self._count(layer_ops.BACKWARD_LAUNCHES)
+                self._count(calls.backward_launches)
             else:
                 w = self._views(unit)
                 g = self._views(unit, prov.grad_buffer(f"layer.{li}")) if self.train_base else dict.fromkeys(w)

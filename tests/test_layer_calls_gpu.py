@@ -94,3 +94,49 @@ def test_a_switch_turned_between_the_passes(cuda_lib):
     finally:
         set_pair(before)
     assert cuda_lib.device_status() == (0, 0, 0, 0)
+
+
+def test_a_pass_without_room_for_partial_sums(cuda_lib, monkeypatch):
+    """A backward block that cannot be had is asked for again without the partial sums of dK / dV: the bits of the schedule from
+    Python without them, and two roundings of the results with them."""
+    from causal_trainer_dev_b200.models.config import preset
+    from causal_trainer_dev_b200.models.params import ModelParams
+    from causal_trainer_dev_b200.training import engine as E
+
+    cfg = preset("tiny", num_hidden_layers=2, vocab_size=1000)
+    lib, heads = cuda_lib.lib(), (cfg.num_attention_heads, cfg.num_key_value_heads, cfg.head_dim)
+    assert lib.ctb_attn_bwd_workspace(1, 1024, 1024, *heads) > 0
+    gen = torch.Generator(device="cuda").manual_seed(3)
+    ids = torch.randint(3, 1000, (1, 1024), generator=gen, device="cuda")
+    batch = dict(input_ids=ids, attention_mask=torch.ones_like(ids), segment_ids=torch.ones_like(ids))
+    seen, real = [], torch.empty
+
+    def run(refuse):
+        params = ModelParams.init_random(cfg, seed=1).to("cuda")
+        engine = E.LayerwiseEngine(cfg, E.LocalProvider(params, torch.bfloat16))
+        calls = engine._layer_calls(engine._context(batch), real(1024, cfg.hidden_size, dtype=torch.bfloat16, device="cuda"))
+
+        def empty(*size, **how):
+            if size == (calls._backward,):
+                seen.append(size)
+                raise torch.cuda.OutOfMemoryError("no memory for the block")
+            return real(*size, **how)
+
+        with monkeypatch.context() as m:
+            if refuse:
+                m.setattr(torch, "empty", empty)
+            sums = engine(batch, 1e-2, first=True)
+        return [*sums, *(u.grad for u in params.units.values())], calls
+
+    with_sums, calls = run(False)
+    assert calls.backward_launches == 23 and not seen
+    without, _ = run(True)
+    assert len(seen) == 1                                   # the second layer asks for what there is
+    monkeypatch.setattr(E, "LAYER_CALL_BYTES", 0)
+    monkeypatch.setattr(lib, "ctb_attn_bwd_workspace", lambda *a: 0)
+    python, calls = run(False)
+    assert calls is None and all(torch.equal(a, b) for a, b in zip(without, python))
+    assert not all(torch.equal(a, b) for a, b in zip(without, with_sums))
+    for a, b in zip(without, with_sums):
+        assert ((a.double() - b.double()).norm() <= 2.0 ** -6 * b.double().norm()).item()      # bf16 roundings of two layers
+    assert cuda_lib.device_status() == (0, 0, 0, 0)
