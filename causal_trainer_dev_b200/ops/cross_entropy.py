@@ -148,9 +148,9 @@ def cut_ce_forward(hidden, head, targets, weights, grad_scale: float | torch.Ten
     hit = flag_source_of(head) if _FLAG_SOURCES else None
     hit_a = flag_source_of(hidden) if _FLAG_SOURCES else None
     _, m_rotate = _rotations(None, hit_a, hidden, head, False, False, rows, vocab)
-    code = L.ctb_ce_stats_step(_lib.ptr(hidden), _lib.ptr(head), rows, vocab, d, ctypes.c_long(hidden.stride(0)),
-                               ctypes.c_long(head.stride(0)), _lib.ptr(tgt), step, *parts, *_flag_args(hit), *_flag_args(hit_a),
-                               m_rotate, int(in_gathered_buffer(hidden, head)), None, ctypes.c_long(0), _lib.stream_ptr())
+    code = L.ctb_ce_stats(_lib.ptr(hidden), _lib.ptr(head), rows, vocab, d, ctypes.c_long(hidden.stride(0)),
+                          ctypes.c_long(head.stride(0)), _lib.ptr(tgt), step, *parts, *_flag_args(hit), *_flag_args(hit_a),
+                          m_rotate, int(in_gathered_buffer(hidden, head)), None, ctypes.c_long(0), _lib.stream_ptr())
     _lib.check(code, "ctb_ce_stats")
     if exchange is not None:
         nll, wsum, lse, coef = exchange.ce_exchange(pmax, psum, slabs, tlogit, w, grad_scale)
@@ -193,7 +193,7 @@ def cut_ce_backward(hidden, head, targets, lse, coef, *, chunk_rows: int = 4096,
         n = min(chunk_rows, rows - start)
         h = hidden[start:start + n]
         g = slab[:n]
-        code = L.ctb_ce_dlogits_step(_lib.ptr(h), _lib.ptr(head), _lib.ptr(g), n, vocab, d, ctypes.c_long(h.stride(0)),
+        code = L.ctb_ce_dlogits(_lib.ptr(h), _lib.ptr(head), _lib.ptr(g), n, vocab, d, ctypes.c_long(h.stride(0)),
                                 ctypes.c_long(head.stride(0)), ctypes.c_long(g.stride(0)),
                                 _lib.ptr(tgt[start:start + n]), step, _lib.ptr(lse[start:start + n]),
                                 _lib.ptr(coef[start:start + n]), gathered, _lib.stream_ptr())
@@ -272,10 +272,9 @@ def cut_ce_forward_backward(hidden, head, targets, weights, grad_scale: float | 
         part = slice(start, start + n)
         h = hidden[part]
         ids = p(tgt.data_ptr() + 4 * step * start)
-        code = L.ctb_ce_stats_step(_lib.ptr(h), _lib.ptr(head), n, vocab, d, ln(h.stride(0)), ln(head.stride(0)), ids,
-                                   step, p(work.pmax), p(work.psum), p(work.tlogit + 4 * start), None, ln(0), ln(0),
-                                   ctypes.c_uint(0), None, ln(0), ln(0), ctypes.c_uint(0), 0, 0, _lib.ptr(slab), ln(vocab),
-                                   _lib.stream_ptr())
+        code = L.ctb_ce_stats(_lib.ptr(h), _lib.ptr(head), n, vocab, d, ln(h.stride(0)), ln(head.stride(0)), ids, step,
+                              p(work.pmax), p(work.psum), p(work.tlogit + 4 * start), None, ln(0), ln(0), ctypes.c_uint(0), None,
+                              ln(0), ln(0), ctypes.c_uint(0), 0, 0, _lib.ptr(slab), ln(vocab), _lib.stream_ptr())
         _lib.check(code, "ctb_ce_stats")
         _combine(L, work, slabs, tgt, step, vocab, w, scale, device_scale, work.lse, work.coef, start, n)
         code = L.ctb_kept_logits_gradient(_lib.ptr(slab), ln(vocab), n, vocab, ids, step, p(work.lse + 4 * start),

@@ -1418,7 +1418,7 @@ CTB_API int ctb_attn_bwd_stats(const void* o, const void* dout, const float* lse
 }
 
 // block_nll / block_w must hold ceil(rows / 32) floats each; ctb_ce_sums adds them up.  coef = weights * grad_scale * *scale (scale
-// may be null).  target_step: see ctb_ce_stats_step; the logit of a row whose target is outside [0, vocab) counts as 0.
+// may be null).  target_step: see ctb_ce_stats; the logit of a row whose target is outside [0, vocab) counts as 0.
 CTB_API int ctb_ce_combine(const float* pmax, const float* psum, int slabs, const float* target_logit, const int* targets,
                            int target_step, int vocab, const float* weights, float grad_scale, const float* scale, float* lse,
                            float* coef, float* block_nll, float* block_w, int rows, void* stream) {

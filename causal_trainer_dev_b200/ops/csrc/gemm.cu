@@ -850,11 +850,11 @@ CTB_API int ctb_gemm_push(const void* A, const void* B, int M, int N, int K, lon
 // that the same kernel computes the logits however far the gather has come (here and in ctb_ce_dlogits).  `logits` (null: not
 // wanted): where the fp32 logits go, rows of ldl elements.
 // The targets may be 64-bit ids: target_step words lie from one to the next (1 or 2) and the low one is read.
-CTB_API int ctb_ce_stats_step(const void* hidden, const void* head, int rows, int vocab, int d, long ldh, long ldw,
-                              const int* targets, int target_step, float* pmax, float* psum, float* target_logit,
-                              const unsigned* flags, long flag_chunk, long flag_base, unsigned epoch, const unsigned* a_flags,
-                              long a_flag_chunk, long a_flag_base, unsigned a_epoch, int m_rotate, int gathered, float* logits,
-                              long ldl, void* stream) {
+CTB_API int ctb_ce_stats(const void* hidden, const void* head, int rows, int vocab, int d, long ldh, long ldw,
+                         const int* targets, int target_step, float* pmax, float* psum, float* target_logit,
+                         const unsigned* flags, long flag_chunk, long flag_base, unsigned epoch, const unsigned* a_flags,
+                         long a_flag_chunk, long a_flag_base, unsigned a_epoch, int m_rotate, int gathered, float* logits,
+                         long ldl, void* stream) {
   ctb::GemmCall c{};
   c.C = logits; c.ldc = ldl; c.out_f32 = 1;
   c.gathered = gathered;
@@ -867,19 +867,11 @@ CTB_API int ctb_ce_stats_step(const void* hidden, const void* head, int rows, in
   c.ce_max = pmax; c.ce_sum = psum; c.ce_target_logit = target_logit;
   return ctb::run_gemm(c);
 }
-CTB_API int ctb_ce_stats(const void* hidden, const void* head, int rows, int vocab, int d, long ldh, long ldw,
-                         const int* targets, float* pmax, float* psum, float* target_logit, const unsigned* flags,
-                         long flag_chunk, long flag_base, unsigned epoch, const unsigned* a_flags, long a_flag_chunk,
-                         long a_flag_base, unsigned a_epoch, int m_rotate, int gathered, float* logits, long ldl,
-                         void* stream) {
-  return ctb_ce_stats_step(hidden, head, rows, vocab, d, ldh, ldw, targets, 1, pmax, psum, target_logit, flags, flag_chunk,
-                           flag_base, epoch, a_flags, a_flag_chunk, a_flag_base, a_epoch, m_rotate, gathered, logits, ldl, stream);
-}
 
 // Cut cross-entropy backward slab: G[rows,vocab] = (exp(logits - lse[row]) - onehot) * coef[row], bf16.
-CTB_API int ctb_ce_dlogits_step(const void* hidden, const void* head, void* g, int rows, int vocab, int d, long ldh,
-                                long ldw, long ldg, const int* targets, int target_step, const float* lse, const float* coef,
-                                int gathered, void* stream) {
+CTB_API int ctb_ce_dlogits(const void* hidden, const void* head, void* g, int rows, int vocab, int d, long ldh,
+                           long ldw, long ldg, const int* targets, int target_step, const float* lse, const float* coef,
+                           int gathered, void* stream) {
   ctb::GemmCall c{};
   c.gathered = gathered;
   c.A = hidden; c.B = head; c.C = g; c.M = rows; c.N = vocab; c.K = d; c.lda = ldh; c.ldb = ldw; c.ldc = ldg;
@@ -887,11 +879,6 @@ CTB_API int ctb_ce_dlogits_step(const void* hidden, const void* head, void* g, i
   c.ce_targets = targets; c.ce_target_step = target_step;
   c.ce_lse = lse; c.ce_coef = coef;
   return ctb::run_gemm(c);
-}
-CTB_API int ctb_ce_dlogits(const void* hidden, const void* head, void* g, int rows, int vocab, int d, long ldh,
-                           long ldw, long ldg, const int* targets, const float* lse, const float* coef,
-                           int gathered, void* stream) {
-  return ctb_ce_dlogits_step(hidden, head, g, rows, vocab, d, ldh, ldw, ldg, targets, 1, lse, coef, gathered, stream);
 }
 
 // Which kernel a plain product with a 16-byte aligned bf16 output takes where the two-CTA kernel (ctb_gemm_pair_choice) does

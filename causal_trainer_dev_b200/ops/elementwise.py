@@ -184,8 +184,8 @@ def embedding_backward(ids: torch.Tensor, dout: torch.Tensor, grad: torch.Tensor
         order = torch.sort(flat.to(torch.int32), stable=True)
         ordered, perm = order.values, order.indices.to(torch.int32)
     code = L.ctb_embedding_backward(_lib.ptr(ordered), _lib.ptr(perm), _l(flat.numel()), _lib.ptr(dout),
-                                             _lib.ptr(grad), int(grad.dtype == torch.float32), dout.shape[1], vocab_lo,
-                                             grad.shape[0], pad_id, _lib.stream_ptr())
+                                    _lib.ptr(grad), int(grad.dtype == torch.float32), dout.shape[1], vocab_lo,
+                                    grad.shape[0], pad_id, _lib.stream_ptr())
     _lib.check(code, "ctb_embedding_backward")
 
 

@@ -39,10 +39,11 @@ def test_warps_without_rows_leave_the_staging_alone(cuda_lib, one_cta, m, k, dty
     assert cuda_lib.device_status() == (0, 0, 0, 0)
 
 
+@pytest.mark.parametrize("ids", [torch.int32, torch.int64])
 @pytest.mark.parametrize("rows,vocab,d,tm", [
     (333, 32000, 64, None), (33, 64008, 512, None), (200, 40000, 128, None),                     # one CTA
     (1100, 32000, 512, 1), (4000, 5000, 256, 1), (644, 6216, 584, 2), (2077, 2064, 608, 2)])     # two, 256 or 512 rows
-def test_kept_logits_and_their_gradients(cuda_lib, rows, vocab, d, tm):
+def test_kept_logits_and_their_gradients(cuda_lib, rows, vocab, d, tm, ids):
     """The loss epilogues, on the kernel that the sizes choose."""
     import ctypes
 
@@ -52,7 +53,8 @@ def test_kept_logits_and_their_gradients(cuda_lib, rows, vocab, d, tm):
     gen = torch.Generator(device="cuda").manual_seed(rows)
     hidden = torch.randn(rows, d, generator=gen, device="cuda").bfloat16()
     head = (torch.randn(vocab, d, generator=gen, device="cuda") * 0.05).bfloat16()
-    targets = torch.randint(0, vocab, (rows,), generator=gen, device="cuda", dtype=torch.int32)
+    targets = torch.randint(0, vocab, (rows,), generator=gen, device="cuda", dtype=ids)
+    step = targets.element_size() // 4
     p, ln, slabs = cuda_lib.ptr, ctypes.c_long, -(-vocab // 256)
     none = (None, ln(0), ln(0), ctypes.c_uint(0))
     want = hidden.double() @ head.double().t()
@@ -61,14 +63,14 @@ def test_kept_logits_and_their_gradients(cuda_lib, rows, vocab, d, tm):
     for _ in range(3):
         pmax, psum = (torch.empty(slabs, rows, device="cuda") for _ in range(2))
         at_target, logits = torch.zeros(rows, device="cuda"), torch.full((rows + 2, vocab), 7.0, device="cuda")
-        assert cuda_lib.lib().ctb_ce_stats(p(hidden), p(head), rows, vocab, d, ln(d), ln(d), p(targets), p(pmax), p(psum),
-                                           p(at_target), *none, *none, 0, 0, p(logits), ln(vocab), cuda_lib.stream_ptr()) == 0
+        assert cuda_lib.lib().ctb_ce_stats(p(hidden), p(head), rows, vocab, d, ln(d), ln(d), p(targets), step, p(pmax),
+                                           p(psum), p(at_target), *none, *none, 0, 0, p(logits), ln(vocab), cuda_lib.stream_ptr()) == 0
         assert bool(((logits[:rows].double() - want).abs() <= size + 2.0 ** -23 * want.abs()).all())
         assert bool((logits[rows:] == 7).all())
         assert torch.equal(at_target, logits[:rows].gather(1, targets.long()[:, None])[:, 0])
         g = torch.full((rows + 2, vocab), 7.0, device="cuda", dtype=torch.bfloat16)
         coef = torch.ones(rows, device="cuda")
-        assert cuda_lib.lib().ctb_ce_dlogits(p(hidden), p(head), p(g), rows, vocab, d, ln(d), ln(d), ln(vocab), p(targets),
+        assert cuda_lib.lib().ctb_ce_dlogits(p(hidden), p(head), p(g), rows, vocab, d, ln(d), ln(d), ln(vocab), p(targets), step,
                                              p(lse.float()), p(coef), 0, cuda_lib.stream_ptr()) == 0
         prob = (want - lse[:, None]).exp()
         exact = prob.clone()
