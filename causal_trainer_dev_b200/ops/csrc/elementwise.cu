@@ -1393,11 +1393,12 @@ CTB_API int ctb_attn_bwd_stats(const void* o, const void* dout, const float* lse
                                int B, int S, int H, int D, long o_rs, long do_rs, void* stream) {
   // 16-byte rows of the two head sizes the flash kernels take, and enough of them: a block of the wide kernel takes
   // 128 rows one after the other, 2.3 us at D = 64 and 3.4 at D = 128 however few there are, where a warp per row
-  // (below) takes 1.8 and grows with the rows.  They meet at 80 D rows (us, warp per row and wide: D = 64 4096 rows
+  // (below) takes 1.8 and grows with the rows.  They meet at 64 to 80 D rows (us, warp per row and wide: D = 64 4096 rows
   // 2.5 and 2.4, 8192 rows 3.1 and 2.4, 16384 rows 4.8 and 2.5; D = 128 8192 rows 3.2 and 3.7, 12288 rows 4.6
-  // and 4.0, 16384 rows 5.4 and 4.0).
+  // and 4.0, 16384 rows 5.4 and 4.0).  The line stays at 192 D, where 8 heads a block met the warp per row, because the two add
+  // in different orders: the last bits of a call do not change with it.
   const long tokens = static_cast<long>(B) * S;
-  const bool wide = (D == 64 || D == 128) && o_rs % 8 == 0 && do_rs % 8 == 0 && tokens * H >= 80l * D &&
+  const bool wide = (D == 64 || D == 128) && o_rs % 8 == 0 && do_rs % 8 == 0 && tokens * H >= 192l * D &&
                     (reinterpret_cast<uintptr_t>(o) | reinterpret_cast<uintptr_t>(dout)) % 16 == 0;
   const bool chained = attn::chained_rows(tokens, H, D);
   const int head_blocks = (H + STAT_HEADS - 1) / STAT_HEADS;

@@ -84,7 +84,7 @@ def test_a_nan_key_reaches_every_query_that_sees_it(cuda_lib, d, key):
 @pytest.mark.parametrize("shape", [(1, 1, 1), (2, 33, 3), (1, 128, 28), (2, 6149, 1), (3, 4099, 3), (1, 945, 26), (1, 3001, 9),
                                    (1, 2051, 12), (3, 2049, 4), (1, 945, 28), (1, 1027, 31), (1, 427, 12)])
 def test_attention_backward_statistics(cuda_lib, d, shape):
-    """A warp per row below 80 d rows (and for other head sizes), above it blocks of 32 tokens and 4 heads, cut off."""
+    """A warp per row below 192 d rows (and for other head sizes), above it blocks of 32 tokens and 4 heads, cut off."""
     from causal_trainer_dev_b200.ops import elementwise as E
 
     b, s, h = shape
