@@ -456,11 +456,14 @@ __device__ __forceinline__ float quotient_in_range(float n, float d) {
   const float q = n * r;
   return fmaf(fmaf(-q, d, n), r, q);
 }
-// Whether all eight gates are below 87 (0x42ae) in size, as bf16 bit patterns.
+// Whether the eight gates of every lane that has come here are below 87 (0x42ae) in size, as bf16 bit patterns.  One answer for the
+// warp: with lanes apart it runs both quotients one after the other (1000 x 8960 in a sequence, gates of size 39, forward and
+// backward: 23.4 and 24.1 us, where the division alone took 16.8 and 17.7; so 1.04 and 1.09 of the division's time, of gates of size 20
+// 0.81 and 0.95).
 __device__ __forceinline__ bool gates_in_range(const uint4& gates) {
   const unsigned m = __vmaxu2(__vmaxu2(gates.x & 0x7fff7fffu, gates.y & 0x7fff7fffu),
                               __vmaxu2(gates.z & 0x7fff7fffu, gates.w & 0x7fff7fffu));
-  return (m & 0xffffu) < 0x42aeu && (m >> 16) < 0x42aeu;
+  return __all_sync(__activemask(), (m & 0xffffu) < 0x42aeu && (m >> 16) < 0x42aeu);
 }
 template <bool PLAIN>
 __device__ __forceinline__ uint4 swiglu_vector(const uint4& gates, const uint4& ups) {
