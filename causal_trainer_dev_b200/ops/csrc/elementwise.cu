@@ -1268,8 +1268,11 @@ CTB_API int ctb_rmsnorm_bwd(const void* dy, const void* x, const void* w, const 
   cudaStream_t s = static_cast<cudaStream_t>(stream);
   const bool chained = 8l * rows * d <= CHAINED_BYTES;
   const int nv = (d / 8 + NORM_THREADS - 1) / NORM_THREADS;
+  // Rows of up to 2048: three blocks fit an SM where two are launched for each, and started early they crowd (us, chained and not: 1000 x
+  // 1536 7.3 and 7.0, 2000 x 1536 9.5 and 8.8, 4096 x 1536 14.7 and 12.7); wider ones have no room to (1000 x 4096 8.9 and 9.1, 700
+  // x 8192 13.3 and 14.1).  Below 2 MB it is the launch that counts (512 x 256 4.6, unchained 5.5).
 #define CTB_NORM_BWD(NV)                                                                       \
-  CTB_CUDA_OK(launch_chained(chained, rmsnorm_bwd_kernel<NV>, parts, NORM_THREADS, 0, s, 0,    \
+  CTB_CUDA_OK(launch_chained(chained && (NV > 1 || 8l * rows * d <= 2l << 20), rmsnorm_bwd_kernel<NV>, parts, NORM_THREADS, 0, s, 0, \
       static_cast<const __nv_bfloat16*>(dy), static_cast<const __nv_bfloat16*>(x),             \
       static_cast<const __nv_bfloat16*>(w), rstd, static_cast<const __nv_bfloat16*>(dres),     \
       static_cast<__nv_bfloat16*>(dx), dw_partial, rows, d))

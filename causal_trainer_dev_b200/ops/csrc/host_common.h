@@ -55,6 +55,9 @@ int sm_count();
 // launch before it in the stream still runs, if that one lets them (let_successor_start).  Only short calls are chained: there
 // the 2 us between two launches count (two rows of 256 tokens, attention 36.5 -> 34.1 us; an MLP on 1000 rows of 1536 / 8960 299 ->
 // 284; a head on 333 rows 221 -> 215); with 512 MB and 4e11 for the limits longer sequences took 0.96 to 1.15 of their time.
+// These two are the most that anything chains at.  A kernel whose blocks are fewer than fit at once loses by an early start, because
+// they crowd on the SMs that have room first: rotary embedding, norms, attention and the gradient of kept logits have lines of
+// their own where they are launched.
 constexpr long CHAINED_BYTES = 64l << 20;       // moved by a memory-bound kernel
 constexpr double CHAINED_FLOPS = 6e10;          // of a product
 template <typename... P, typename... A>
