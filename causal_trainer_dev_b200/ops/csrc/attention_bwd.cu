@@ -1104,11 +1104,11 @@ int launch_bwd_dense(const BwdCall& c) {
 // and the longest is 112 iterations where an SM has 29 of the whole call.  The estimate (cycles) takes the rows for whole
 // documents: an iteration of dK/dV 2615 and of dQ 2047, the start and end of an item 10000 and 8000, of a further part with its
 // fp32 tiles 12000, the sum of the parts 8000.  Rows of short documents, whose tiles stay whole or nearly so (dkv_least), pay for
-// that: the launch of the sums and the parts without work are 2 to 5 us.  Backward, us, uncut and so: 2 rows of 2048, 14 / 2 heads,
-// one document 176.9, 101.2, documents of 350 59.5, 52.8, of 128 31.0, 35.7; 4 rows of 512, 8 / 2 heads, 34.8, 25.7, of 200 27.0, 24.2,
-// of 128 18.4, 20.4; 1 row of 1024, 28 / 4 heads, of 200 37.8, 29.6.  What did not mend it: the sums by the last part of a tile to
-// finish (one SM reads them all: 5 to 8 us a cut tile), a compact list of the items made by every CTA with the sums at its end
-// (the sums in the compute warps' loop spill registers: 6 to 12 us).
+// that: the launch of the sums and the parts without work are 2 to 3 us.  Backward, us, uncut and so: 2 rows of 2048, 14 / 2 heads,
+// one document 170.4, 95.3, documents of 350 54.4, 48.2, of 200 41.0, 43.5, of 128 28.9, 31.8; 4 rows of 512, 8 / 2 heads, 34.9, 25.8, of
+// 200 26.7, 24.2, of 128 18.2, 20.2; 1 row of 1024, 28 / 4 heads, of 200 37.2, 29.5.  What did not mend it: the sums by the last part of
+// a tile to finish (one SM reads them all: 5 to 8 us a cut tile), a compact list of the items made by every CTA with the sums at its
+// end (the sums in the compute warps' loop spill registers: 6 to 12 us).
 inline int dkv_parts(int B, int S, int Sq, int Hq, int Hkv) {
   const double tiles = static_cast<double>(B) * Hkv * (S / 128), rows = static_cast<double>(B) * Hq * (Sq / 128);
   const double longest = static_cast<double>(Hq / Hkv) * (Sq / 128), seen = (Sq / 128 + 1) / 2.;
