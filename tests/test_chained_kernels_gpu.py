@@ -167,3 +167,60 @@ def test_a_refused_launch_leaves_no_error_behind(cuda_lib):
         with pytest.raises(cuda_lib.KernelError):
             E.rmsnorm_forward(x, w, 1e-5)
         assert float(torch.ones(300, device="cuda").cumsum(0)[-1]) == 300
+
+
+@pytest.mark.parametrize("captured", [False, True])
+def test_an_event_between_two_launches_is_waited_for(cuda_lib, captured):
+    """The kernel before a chained one lets its successor start at once; what the chained one reads comes from another stream,
+    whose event its own stream waits for in between, and is still being written."""
+    from causal_trainer_dev_b200.ops import elementwise as E
+    from causal_trainer_dev_b200.ops import lib as L
+    from causal_trainer_dev_b200.ops.gemm import gemm
+
+    gen = torch.Generator(device="cuda").manual_seed(8)
+    gate_up, w = _randn(gen, WIDE, 2 * F), _randn(gen, F)
+    weight, short = _randn(gen, 256, F, scale=0.02), _randn(gen, 512, 2 * F)
+    wide, act = torch.empty(WIDE, F, dtype=torch.bfloat16, device="cuda"), torch.empty(512, F, dtype=torch.bfloat16, device="cuda")
+    tail = wide[WIDE - 512:]
+    main, other = torch.cuda.Stream(), torch.cuda.Stream()
+
+    def into(gu, out, rows):
+        L.check(L.lib().ctb_swiglu_fwd(gu.data_ptr(), out.data_ptr(), rows, F, L.raw_stream()), "ctb_swiglu_fwd")
+
+    def calls(s):
+        other.wait_stream(s)
+        with torch.cuda.stream(other):
+            into(gate_up, wide, WIDE)                                  # about 80 us
+        into(short, act, 512)                                          # lets its successor in, and is over long before
+        s.wait_stream(other)
+        normed, rstd, _ = E.rmsnorm_forward(tail, w, 1e-5)
+        # the same in front of a product (operands by bulk copies)
+        other.wait_stream(s)
+        with torch.cuda.stream(other):
+            torch.mul(wide, 2.0, out=wide)
+        into(short, act, 512)
+        s.wait_stream(other)
+        return normed, rstd, gemm(tail, weight)
+
+    wide.fill_(3.0)
+    into(gate_up, wide, WIDE)
+    torch.cuda.synchronize()
+    want = list(E.rmsnorm_forward(tail, w, 1e-5)[:2])
+    wide.mul_(2.0)
+    want.append(gemm(tail, weight))
+    torch.cuda.synchronize()
+    if captured:
+        graph = torch.cuda.CUDAGraph()
+        with torch.cuda.graph(graph, stream=main):
+            got = calls(main)
+    for _ in range(5):
+        wide.fill_(3.0)
+        torch.cuda.synchronize()
+        if captured:
+            graph.replay()
+        else:
+            with torch.cuda.stream(main):
+                got = calls(main)
+        torch.cuda.synchronize()
+        assert all(torch.equal(a, b) for a, b in zip(got, want))
+    assert cuda_lib.device_status() == (0, 0, 0, 0)
