@@ -50,19 +50,12 @@ def rmsnorm_forward(x, w, eps, residual=None, out=None):
     return y, rstd, h
 
 
-_norm_scratch: dict[tuple[int, int], torch.Tensor] = {}
-
-
 def rmsnorm_backward(dy, x, w, rstd, dres=None, dw_out=None, dw_accumulate=False, dx_out=None):
     """Returns (dx, dw).  ``dx`` includes ``dres`` when given (the residual branch gradient)."""
     rows, d = x.shape
     L = _lib.lib()
-    parts = L.ctb_rmsnorm_bwd_parts(rows)
-    key = (x.device.index or 0, parts * d)
-    scratch = _norm_scratch.get(key)
-    if scratch is None:
-        scratch = torch.empty(parts * d, dtype=torch.float32, device=x.device)
-        _norm_scratch[key] = scratch
+    # partial rows of this call alone: calls on several streams, or captured, must not meet in them
+    scratch = torch.empty(L.ctb_rmsnorm_bwd_parts(rows) * d, dtype=torch.float32, device=x.device)
     dx = torch.empty_like(x) if dx_out is None else dx_out
     if dw_out is None:
         dw_out = torch.empty(d, dtype=torch.float32, device=x.device)

@@ -157,3 +157,25 @@ def test_active_row_compaction_is_stable_and_round_trips(cuda_lib):
     assert torch.equal(back, expect)                     # padding slots did not overwrite row 0
     none, _, n0 = E.active_rows(torch.zeros(300, device="cuda"))
     assert n0 == 0 and none.numel() == 0
+
+
+def test_norm_backward_on_two_streams_at_once(cuda_lib):
+    """Calls of one shape share nothing: weight gradients on two streams are those of the same calls one after the other."""
+    from causal_trainer_dev_b200.ops import elementwise as E
+
+    gen = torch.Generator(device="cuda").manual_seed(2)
+    rows, d = 8192, 1536
+    x, dy = ([torch.randn(rows, d, generator=gen, device="cuda").bfloat16() for _ in range(2)] for _ in range(2))
+    w = torch.randn(d, generator=gen, device="cuda").bfloat16()
+    rstd = [E.rmsnorm_forward(t, w, 1e-5)[1] for t in x]
+    want = [E.rmsnorm_backward(dy[i], x[i], w, rstd[i]) for i in range(2)]
+    torch.cuda.synchronize()
+    streams = [torch.cuda.Stream() for _ in range(2)]
+    got = [[], []]
+    for _ in range(20):
+        for i in range(2):
+            with torch.cuda.stream(streams[i]):
+                got[i].append(E.rmsnorm_backward(dy[i], x[i], w, rstd[i]))
+    torch.cuda.synchronize()
+    for i in range(2):
+        assert all(torch.equal(a, b) for pair in got[i] for a, b in zip(pair, want[i]))
