@@ -445,8 +445,8 @@ __global__ void rope_table_kernel(const int* __restrict__ pos, const float* __re
 // number; after the step it is within half an ulp and a little of 1 / d (the approximate one is within 2^-23, the step squares that), the
 // quotient within an ulp of n / d, and the remainder of such a quotient is a number that the fused multiply-add gives exactly.  The sum
 // before its one rounding is within 2^-46 of n / d, so only a quotient that close to the middle of two fp32 numbers could come out as the
-// other one.  tests/test_kernel_edges_gpu.py compares all gates of bf16 with the division: no result differs, but for the sign of a zero.
-// The division bound the forward kernel by its instructions (279 us at 16384 x 14336, so 231); a fast one returns zero for
+// other one.  tests/test_kernel_edges_gpu.py compares all gates of bf16 with the division: no result differs.
+// The division bound the forward kernel by its instructions (280 us at 16384 x 14336, so 234); a fast one returns zero for
 // denominators above 2^126, gates between -88.7 and -87.4.  A vector with a larger gate, or one that is not a number, divides, in a
 // function of its own: inlined it costs the others their registers (260 us).
 __device__ __forceinline__ float quotient_in_range(float n, float d) {
@@ -470,10 +470,17 @@ __device__ __forceinline__ uint4 swiglu_vector(const uint4& gates, const uint4& 
   float g[8], u[8], o[8];
   unpack8(gates, g);
   unpack8(ups, u);
+  const unsigned words[4] = {gates.x, gates.y, gates.z, gates.w};
 #pragma unroll
-  for (int e = 0; e < 8; ++e) {
-    const float d = 1.f + __expf(-g[e]);
-    o[e] = __bfloat162float(__float2bfloat16(PLAIN ? quotient_in_range(g[e], d) : g[e] / d)) * u[e];
+  for (int i = 0; i < 4; ++i) {
+    const float d0 = 1.f + __expf(-g[2 * i]), d1 = 1.f + __expf(-g[2 * i + 1]);
+    __nv_bfloat162 act = PLAIN ? __floats2bfloat162_rn(quotient_in_range(g[2 * i], d0), quotient_in_range(g[2 * i + 1], d1))
+                               : __floats2bfloat162_rn(g[2 * i] / d0, g[2 * i + 1] / d1);
+    // (the corrected quotient of -0 is +0)
+    if (PLAIN) *reinterpret_cast<unsigned*>(&act) |= words[i] & 0x80008000u;
+    const float2 a = __bfloat1622float2(act);
+    o[2 * i] = a.x * u[2 * i];
+    o[2 * i + 1] = a.y * u[2 * i + 1];
   }
   return pack8(o);
 }

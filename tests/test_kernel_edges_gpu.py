@@ -166,7 +166,7 @@ def test_swiglu_of_large_negative_gates(cuda_lib):
 
 def test_swiglu_quotient_of_every_gate(cuda_lib):
     """All 65536 gates of bf16, among themselves (vectors of gates below 87 take the corrected quotient) and each in a vector with a
-    gate of 88 (which divides): the same results, but for the sign of a zero, with several factors forward and backward."""
+    gate of 88 (which divides): the same bits, with several factors forward and backward."""
     from causal_trainer_dev_b200.ops import elementwise as E
 
     gates = torch.arange(-2 ** 15, 2 ** 15, device="cuda").to(torch.int16).view(torch.bfloat16)
@@ -194,7 +194,7 @@ def test_swiglu_quotient_of_every_gate(cuda_lib):
         wide = lambda x, fill: torch.cat([x.view(-1, 4), torch.full_like(x.view(-1, 4), fill)], 1).reshape(-1)  # noqa: E731
         long = [x.view(-1, 8)[:, :4].reshape(-1) for x in run(wide(small, 88.0), wide(up[:n], 1.0), wide(dh[:n], 1.0))]
         for a, b in zip(short, long):
-            assert torch.equal(a, b) and not bool(a.isnan().any())
+            assert torch.equal(a.view(torch.int16), b.view(torch.int16)) and not bool(a.isnan().any())
         # a large gate leaves the others of its vector alone, and is itself what it is alone
         m = large.numel()
         mixed = torch.stack([large.view(-1, 4), small[-m:].view(-1, 4)], 2).reshape(-1)
